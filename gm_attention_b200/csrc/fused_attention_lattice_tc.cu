@@ -632,12 +632,14 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? (MODE == TC_BWD_S ? 3
     }
     if constexpr (PASS_S) {
       float* ds = stats(buf);
-      for (int idx = threadIdx.x; idx < 2 * n_rows; idx += THREADS) {
+      // every row a step can read, zeros beyond the window: its weights are zero there, and zero times whatever an earlier
+      // kernel left in shared memory need not be
+      for (int idx = threadIdx.x; idx < 2 * TN_ROWS; idx += THREADS) {
         const int pl = idx >> 1, which = idx & 1;
         int lon = lon0 + pl;
         if (lon >= a.nlon) lon %= a.nlon;
         const int64_t nn = ((int64_t)z * a.nlon + lon) * a.H + h;
-        cp_async4(ds + 2 * pl + which, (which ? a.delta : a.lse) + nn, 4);
+        cp_async4(ds + 2 * pl + which, (which ? a.delta : a.lse) + nn, pl < n_rows ? 4 : 0);
       }
     }
     cp_async_commit();

@@ -221,6 +221,25 @@ def test_tensor_core_backward_bf16(case):
         assert torch.equal(a, a2), name
 
 
+def test_tensor_core_backward_ignores_stale_shared_memory():
+    """A step of 16 staged positions may start inside a window and end beyond it: the rows beyond carry weight zero, and
+    whatever an earlier kernel left in shared memory (here NaN, on every SM) must not reach the sums."""
+    from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
+
+    batch = TMA_CASE[6]
+    c = make_case(*TMA_CASE[:5], dtype=np.float32, window=TMA_CASE[5])
+    _, lat = tables_for(c)
+    Q, K, V, G = (torch.from_numpy(x).bfloat16().cuda() for x in seeded((batch * c.n_nodes, c.width), 58, np.float32, 4))
+    out, lse = lattice_attention_forward(Q, K, V, lat, tensor_cores=True)
+    poison = torch.full_like(Q, float("nan"))
+    for _ in range(4):  # the fp32-arithmetic and the tensor-core kernel stage these rows over most of an SM's shared memory
+        for tensor_cores in (False, True):
+            lattice_attention_forward(poison, poison, poison, lat, tensor_cores=tensor_cores)
+        lattice_attention_backward(poison, poison, poison, poison, poison, torch.full_like(lse, float("nan")), lat, tensor_cores=True)
+        for name, got in zip(("dq", "dk", "dv"), lattice_attention_backward(G, Q, K, V, out, lse, lat, tensor_cores=True)):
+            assert bool(torch.isfinite(got.float()).all()), name
+
+
 def test_tma_staging_equals_per_thread_staging(monkeypatch):
     """The two staging paths of the tensor-core kernels (TMA tensor copies; per-thread cp.async) feed the same
     arithmetic: results are bit-identical, and no wait on a copy barrier ever ran out."""
