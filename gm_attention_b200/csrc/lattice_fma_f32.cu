@@ -1,0 +1,10 @@
+// float32 instantiations of the fp32-arithmetic lattice attention kernels.
+#include "lattice_fma.cuh"
+
+namespace gmb {
+namespace lat {
+int lattice_pass_f32(int mode, LatArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
+  return lattice_pass<float>(mode, a, n_order_rows, batch, stream);
+}
+}  // namespace lat
+}  // namespace gmb
