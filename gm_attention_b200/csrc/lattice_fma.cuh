@@ -24,7 +24,10 @@
 // Ragged heads (copies not a multiple of C) are padded with zeros there, so every layout runs the same inner loop.
 // The forward has one buffer (its 128 owners x 2 fields fill it; three CTAs per SM overlap copy and compute), the
 // backward passes two.  On 128 x 256, batch 4, 4 heads of 8 x (m <= 3), float32, the layer's training pass measured
-// 13.06 ms with staging by a loop of dependent loads and 4 / 8 lanes per owner; figures for this form are at the launch.
+// 13.06 ms with staging by a loop of dependent loads and 4 / 8 lanes per owner, and 6.2 ms in this form (1.7 + 2.1 + 2.4).
+// Issue slots are 42 % busy: two or three CTAs of 4 warps are what registers and shared memory allow, and 7 to 9 steps per
+// stage on the equatorial rows leave the barriers and the copies' latency visible (64-thread CTAs, twice the lanes with
+// half the copies, and equal stages of a wide window measured the same or slower).
 //
 // Small problems: PARTS lanes share an owner's neighbours (r = part, part + PARTS, ...) and merge their softmax states /
 // sums at the end, so that a polar row's few hundred neighbours are not one lane's serial chain.
@@ -89,7 +92,9 @@ struct Tile {
   // registers of state per lane decide how many CTAs share an SM (65536 / 128 threads: 4 at 128, 3 at 168, 2 at 255)
   static constexpr int SLICE = C * (1 + 2 * NCF);
   static constexpr int STATE = (MODE == MODE_FWD ? 4 : MODE == MODE_BWD_T ? 3 : 4) * SLICE + (MODE == MODE_FWD ? 1 : 2) * SLICE;
-  static constexpr int CTAS = STATE <= 72 ? 4 : STATE <= 124 ? 3 : 2;
+  // (pass T at 8 x (m <= 3): 202 registers, two CTAs 2.20 ms; held to 168, three CTAs 2.10 ms; the forward held to 168 loses:
+  // 1.72 against 2.09 ms, pass S too: 2.38 against 3.57 ms)
+  static constexpr int CTAS = STATE <= 72 ? 4 : STATE <= (MODE == MODE_BWD_T ? 140 : 124) ? 3 : 2;
   static __device__ __forceinline__ int idx(int p) { return TT == 2 ? (p >> 1) + (p & 1) * HALF : p; }
 };
 
