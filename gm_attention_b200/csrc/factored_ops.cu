@@ -9,17 +9,22 @@
 // before the write, rows n -> 0 keep the real part.
 //
 // Forward: one CTA per source node (the caller's grouping order / group_ptr /
-// group_source), Z(j) staged once in shared memory, one thread per edge of the
-// source with h~ in registers; all threads read the same Z address at the same
-// time (broadcast).  The packed width 2 wc + wr is bounded only by shared memory
-// (the reference stops at 320).
+// group_source), Z(j) staged once in shared memory, the source's edges in tiles of
+// 64.  The packed width 2 wc + wr is bounded only by shared memory (the reference
+// stops at 320).
+//
+// The edges of a source are scattered over the target-major edge list, so their records (h, both phase rows, rho; the
+// gradient row in the backward) are copied into shared memory element by element, consecutive threads taking consecutive
+// elements of one edge: read by the edge's own thread straight from global memory, each of the ~60 loads of the forward
+// touched 32 lines.  128 x 256 lattice, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4}, trunk 16, float32: forward
+// 1.40 -> 1.36 ms, backward 4.64 -> 2.56 ms.
 //
 // Backward: one CTA per source again, so dZ(j) needs no atomics.  Edges are taken
-// in tiles of 32; each lane of the first warp... every thread of the tile builds its
-// edge's packed row W(e) = scale * G conj(F) and h~(e) in shared memory, then the CTA
-// forms dh(e, t) = <W(e), Z_t(j)> (one thread per (edge, t)) and accumulates
-// dZ(t, c) += h~_t(e) W_c(e) with patches of 4 (fp32) / 2 (fp64) consecutive columns of one t
-// owned by fixed threads in registers; both read shared memory 16 bytes at a time.
+// in tiles; the CTA builds its edges' packed rows W(e) = scale * G conj(F) in shared
+// memory, then forms dh(e, t) = <W(e), Z_t(j)> and dZ(t, c) += h~_t(e) W_c(e).  Both are small matrix products whose
+// bound is shared-memory bandwidth, so both run on register tiles: 2 edges x 4 t over 4 columns per step for dh (6
+// 16-byte reads for 32 multiply-adds), 5 t x 4 columns over 4 edges per step for dZ (9 reads for 80), the latter owned by
+// fixed threads for the whole source.
 #include "common.cuh"
 
 namespace gmb {
@@ -28,8 +33,9 @@ namespace {
 constexpr int FMAX_K = 20;
 constexpr int FDESC = 8;
 constexpr int FTHREADS = 128;
-constexpr int TILE = 32;           // edges per backward tile
-constexpr int MAX_OWNED = 64;      // (t, c) pairs a thread can own in the backward: K * C <= 64 * 256
+constexpr int MAX_TILE = 64;       // edges per tile, at most (a power of two; less where shared memory is short)
+constexpr int MAX_OWNED = 64;      // K * C <= 64 * 128 in the backward
+constexpr int TP = 5;              // rows t of a dZ patch (4 columns wide)
 
 template <typename T>
 struct FArgs {
@@ -46,132 +52,248 @@ struct FArgs {
   T *dh, *dzc, *dzr, *dweights;
 };
 
-// The block's per-edge factor (factored.h:118-144).
+// An edge's record in shared memory: angular phases (n_f, 2), transport phases (n_f, 2), rho; odd pitch.
+inline int record_pitch(int n_f) { return 4 * n_f + 1; }
+
+// One element global -> shared, asynchronously.
 template <typename T>
-__device__ __forceinline__ void block_factor(const FArgs<T>& a, int64_t e, const int32_t* d, T& fr, T& fi) {
+__device__ __forceinline__ void copy_async(T* dst, const T* src) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(addr), "l"(src), "n"((int)sizeof(T)) : "memory");
+}
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// f(le, w) for every edge le < n of a tile and every element w < width of its row: consecutive threads on consecutive
+// elements, one division per thread and call (a division per element cost as much as the rows' arithmetic)
+template <typename F>
+__device__ __forceinline__ void for_rows(int n, int width, const F& f) {
+  if (width <= 0) return;
+  const int per = max(FTHREADS / width, 1), le0 = (int)threadIdx.x / width;
+  if (width <= FTHREADS) {
+    const int w = (int)threadIdx.x - le0 * width;
+    if (le0 < per)
+      for (int le = le0; le < n; le += per) f(le, w);
+  } else {
+    for (int le = 0; le < n; ++le)
+      for (int w = threadIdx.x; w < width; w += FTHREADS) f(le, w);
+  }
+}
+
+// dst[le][w] = src[row_s[le] * width + w]
+template <typename T>
+__device__ __forceinline__ void stage_rows(T* dst, int pitch, const T* src, int width, int n, const int64_t* row_s) {
+  for_rows(n, width, [&](int le, int w) { copy_async(dst + le * pitch + w, src + row_s[le] * width + w); });
+}
+
+// The records of n edges (edges_s: their indices)
+template <typename T>
+__device__ __forceinline__ void stage_records(const FArgs<T>& a, const int64_t* edges_s, int n, T* rec) {
+  const int w = 2 * a.n_f, pitch = 2 * w + 1;
+  stage_rows(rec, pitch, a.angular, w, n, edges_s);
+  stage_rows(rec + w, pitch, a.transport, w, n, edges_s);
+  stage_rows(rec + 2 * w, pitch, a.rho, 1, n, edges_s);
+}
+
+// The block's per-edge factor (factored.h:118-144), from the edge's record.
+template <typename T>
+__device__ __forceinline__ void block_factor(const T* rec, int n_f, const int32_t* d, T& fr, T& fi) {
   fr = T(1);
   fi = T(0);
   const int ang = d[3], trn = d[4], power = d[5];
   if (ang != 0) {
     const int o = ang < 0 ? -ang : ang;
-    const T pr = a.angular[(e * a.n_f + o) * 2], pi = ang < 0 ? -a.angular[(e * a.n_f + o) * 2 + 1] : a.angular[(e * a.n_f + o) * 2 + 1];
+    const T pr = rec[2 * o], pi = ang < 0 ? -rec[2 * o + 1] : rec[2 * o + 1];
     const T nr = fr * pr - fi * pi, ni = fr * pi + fi * pr;
     fr = nr;
     fi = ni;
   }
   if (trn != 0) {
     const int o = trn < 0 ? -trn : trn;
-    const T pr = a.transport[(e * a.n_f + o) * 2], pi = trn < 0 ? -a.transport[(e * a.n_f + o) * 2 + 1] : a.transport[(e * a.n_f + o) * 2 + 1];
+    const T* t = rec + 2 * n_f;
+    const T pr = t[2 * o], pi = trn < 0 ? -t[2 * o + 1] : t[2 * o + 1];
     const T nr = fr * pr - fi * pi, ni = fr * pi + fi * pr;
     fr = nr;
     fi = ni;
   }
-  const T r = a.rho[e];
+  const T r = rec[4 * n_f];
   T s = T(1);
   for (int x = 0; x < power; ++x) s *= r;
   fr *= s;
   fi *= s;
 }
 
-// Z(j) of one node into shared memory: zc (k, wc, 2) then zr (k, wr).
+// Z(j) of one node into shared memory: row t = [zc (wc, 2) | zr (wr)], `pitch` elements apart; asynchronous.
 template <typename T>
-__device__ __forceinline__ void stage_node(const FArgs<T>& a, int64_t j, T* zc_s, T* zr_s) {
-  const int nc = a.k * a.wc * 2, nr = a.k * a.wr;
-  for (int x = threadIdx.x; x < nc; x += blockDim.x) zc_s[x] = a.zc[j * nc + x];
-  for (int x = threadIdx.x; x < nr; x += blockDim.x) zr_s[x] = a.zr[j * nr + x];
+__device__ __forceinline__ void stage_node(const FArgs<T>& a, int64_t j, T* z_s, int pitch) {
+  const int wc2 = 2 * a.wc;
+  const T* zc = a.zc + j * a.k * wc2;
+  const T* zr = a.zr + j * a.k * a.wr;
+  for_rows(a.k, wc2, [&](int t, int c) { copy_async(z_s + t * pitch + c, zc + t * wc2 + c); });
+  for_rows(a.k, a.wr, [&](int t, int c) { copy_async(z_s + t * pitch + wc2 + c, zr + t * a.wr + c); });
 }
 
-// KT: the trunk width + 1 when it is known at compile time (17: the reference's default radial trunk), 0 = any k <= FMAX_K
-template <typename T, int KT>
-__global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, int pitch) {
-  constexpr int KMAX = KT ? KT : FMAX_K;
+template <typename T> struct Vec4 { T v[4]; };
+template <typename T>
+__device__ __forceinline__ Vec4<T> load4(const T* p) {  // 16-byte aligned
+  Vec4<T> r;
+  if constexpr (sizeof(T) == 4) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    r.v[0] = q.x; r.v[1] = q.y; r.v[2] = q.z; r.v[3] = q.w;
+  } else {
+    const double2 q0 = *reinterpret_cast<const double2*>(p), q1 = *reinterpret_cast<const double2*>(p + 2);
+    r.v[0] = q0.x; r.v[1] = q0.y; r.v[2] = q1.x; r.v[3] = q1.y;
+  }
+  return r;
+}
+
+template <typename T>
+__device__ __forceinline__ void store4(T* p, const T (&v)[4]) {  // 16-byte aligned
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+  } else {
+    *reinterpret_cast<double2*>(p) = make_double2(v[0], v[1]);
+    *reinterpret_cast<double2*>(p + 2) = make_double2(v[2], v[3]);
+  }
+}
+
+// Forward, per tile of a source's edges: U(c, e) = sum_t h~_t(e) Z_t(c) as a matrix product in register tiles of 4 edges x
+// 4 packed columns (two 16-byte reads for 16 multiply-adds), the blocks' factors F(b, e), then a thread per (edge, output
+// column) adds up its blocks.  Everything indexed by edge has the edge fastest, so a warp's 32 edges read one line.
+// (A thread per edge that walked the blocks with all of Z broadcast measured 1.40 ms, 1.62 with staged records; this form
+// 1.36.  What is left is issue: a third of the instructions are multiply-adds, the rest mostly the factors' phases and powers.)
+template <typename T>
+struct ForwardLayout {  // shared memory, in elements of T
+  int tile, pitch, cols, e_pitch, rec_pitch, row_pitch;
+  int z, h, u, f, rec, total;
+  __host__ __device__ ForwardLayout(int k, int C, int n_f, int n_blocks, int d_out, int tile_) {
+    tile = tile_;
+    cols = (C + 3) / 4 * 4;
+    pitch = cols;
+    e_pitch = tile + 4;
+    rec_pitch = 4 * n_f + 1;
+    row_pitch = d_out | 1;
+    z = 0;
+    h = z + k * pitch;
+    u = h + k * e_pitch;
+    f = u + cols * e_pitch;
+    rec = f + 2 * n_blocks * tile;  // the records; the finished rows afterwards
+    total = (rec + tile * (rec_pitch > row_pitch ? rec_pitch : row_pitch) + 3) / 4 * 4;
+  }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, int tile) {
   extern __shared__ __align__(16) unsigned char raw[];
-  T* zc_s = reinterpret_cast<T*>(raw);
-  T* zr_s = zc_s + a.k * a.wc * 2;
-  // every thread builds its edge's row in shared memory (odd pitch: no bank conflicts); the warp then writes its 32 rows
-  // to global memory one row per store instruction (contiguous) instead of 32 scattered elements per instruction
-  T* row = zr_s + ((a.k * a.wr + 3) / 4) * 4 + (size_t)threadIdx.x * pitch;
-  const int lane = threadIdx.x & 31;
+  __shared__ int64_t edges_s[MAX_TILE];
+  __shared__ int n_out_s;
+  const int wc2 = 2 * a.wc, C = wc2 + a.wr;
+  const ForwardLayout<T> L(a.k, C, a.n_f, a.n_blocks, a.d_out, tile);
+  T* base_s = reinterpret_cast<T*>(raw);
+  T* z_s = base_s + L.z;      // (k, pitch)
+  T* h_s = base_s + L.h;      // (k, e_pitch): h~ transposed
+  T* u_s = base_s + L.u;      // (cols, e_pitch)
+  T* f_s = base_s + L.f;      // (n_blocks, 2, tile)
+  T* rec_s = base_s + L.rec;  // (tile, rec_pitch), then rows (tile, row_pitch)
+  int4* block_s = reinterpret_cast<int4*>(base_s + L.total);            // (n_blocks): U row 0, F row (-1: none), columns
+  int4* out_s = block_s + a.n_blocks;                                   // (<= d_out): first block, blocks, column, output column (~: real)
+  int32_t* desc_s = reinterpret_cast<int32_t*>(out_s + a.d_out);        // (n_blocks, FDESC)
+  for (int x = threadIdx.x; x < L.rec; x += FTHREADS) base_s[x] = T(0);  // padding columns and edges beyond a tile stay finite
+  for (int x = threadIdx.x; x < a.n_blocks * FDESC; x += FTHREADS) desc_s[x] = a.desc[x];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    // blocks are sorted by output offset; blocks of one offset add into the same columns
+    int n = 0;
+    for (int b = 0; b < a.n_blocks;) {
+      int last = b + 1;
+      while (last < a.n_blocks && desc_s[last * FDESC + 6] == desc_s[b * FDESC + 6]) ++last;
+      const int32_t* d = desc_s + b * FDESC;
+      const bool real_column = d[0] == 0 || d[7] != 0;
+      for (int c = 0; c < d[2] && n < a.d_out; ++c, ++n) out_s[n] = make_int4(b, last, c, real_column ? ~(d[6] + c) : d[6] + 2 * c);
+      b = last;
+    }
+    n_out_s = n;
+  }
+  if ((int)threadIdx.x < a.n_blocks) {
+    for (int b = threadIdx.x; b < a.n_blocks; b += FTHREADS) {
+      const int32_t* d = desc_s + b * FDESC;
+      block_s[b] = d[0] == 0 ? make_int4((wc2 + d[1]) * L.e_pitch, -1, d[2], 0) : make_int4(2 * d[1] * L.e_pitch, 2 * b * tile, d[2], 0);
+    }
+  }
+  const int le = threadIdx.x & (tile - 1), sub = threadIdx.x / tile, subs = FTHREADS / tile;
   for (int64_t grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
     const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
     __syncthreads();
-    stage_node(a, j, zc_s, zr_s);
-    __syncthreads();
-    for (int64_t x0 = first; x0 < last; x0 += blockDim.x) {  // x0: uniform, so that whole warps take part in the row hand-over
-      const int64_t x = x0 + threadIdx.x;
-      const bool mine = x < last;
-      const int64_t e = mine ? a.order[x] : -1;
-      if (mine) {
-        T hh[KMAX];
-        hh[0] = T(1);
+    stage_node(a, j, z_s, L.pitch);
+    for (int64_t x0 = first; x0 < last; x0 += tile) {
+      const int n_tile = (int)min((int64_t)tile, last - x0);
+      __syncthreads();
+      if ((int)threadIdx.x < n_tile) edges_s[threadIdx.x] = a.order[x0 + threadIdx.x];
+      __syncthreads();
+      for_rows(n_tile, a.k - 1, [&](int e, int t) { copy_async(h_s + (t + 1) * L.e_pitch + e, a.h + edges_s[e] * (a.k - 1) + t); });
+      stage_records(a, edges_s, n_tile, rec_s);
+      if ((int)threadIdx.x < tile) h_s[threadIdx.x] = T(1);
+      copy_wait();
+      __syncthreads();
+      const int eqs = (n_tile + 3) / 4;
+      for (int x = threadIdx.x; x < eqs * (L.cols / 4); x += FTHREADS) {
+        const int cq = x / eqs, e0 = 4 * (x - cq * eqs);
+        const T* zp = z_s + 4 * cq;
+        const T* hp = h_s + e0;
+        T acc[4][4];
 #pragma unroll
-        for (int t = 1; t < KMAX; ++t) hh[t] = (KT || t < a.k) ? a.h[e * (a.k - 1) + t - 1] : T(0);
-        // Blocks are sorted by output offset; blocks of one offset add into the same columns.  The
-        // first block of a group writes, the following ones add to the edge's row.
-        int open_offset = -1;
-        for (int b = 0; b < a.n_blocks; ++b) {
-          const int32_t* d = a.desc + b * FDESC;
-          const int kind = d[0], zoff = d[1], bm = d[2], ooff = d[6];
-          const bool take_real = d[7] != 0;
-          const bool first_of_group = ooff != open_offset;
-          open_offset = ooff;
-          if (kind == 0) {
-            for (int c = 0; c < bm; ++c) {
-              T s = T(0);
+        for (int c = 0; c < 4; ++c)
 #pragma unroll
-              for (int t = 0; t < KMAX; ++t)
-                if (KT || t < a.k) s += hh[t] * zr_s[t * a.wr + zoff + c];
-              row[ooff + c] = first_of_group ? s : row[ooff + c] + s;
-            }
-            continue;
-          }
+          for (int e = 0; e < 4; ++e) acc[c][e] = T(0);
+#pragma unroll 4
+        for (int t = 0; t < a.k; ++t) {
+          const Vec4<T> zv = load4(zp + t * L.pitch), hv = load4(hp + t * L.e_pitch);
+#pragma unroll
+          for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[c][e] += hv.v[e] * zv.v[c];
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) store4(u_s + (4 * cq + c) * L.e_pitch + e0, acc[c]);
+      }
+      if (le < n_tile)
+        for (int b = sub; b < a.n_blocks; b += subs) {
+          if (desc_s[b * FDESC] == 0) continue;
           T fr, fi;
-          block_factor(a, e, d, fr, fi);
-          auto emit = [&](int c, T ur, T ui) {
-            const T vr = fr * ur - fi * ui, vi = fr * ui + fi * ur;
-            if (take_real) {
-              row[ooff + c] = first_of_group ? vr : row[ooff + c] + vr;
-            } else {
-              row[ooff + 2 * c] = first_of_group ? vr : row[ooff + 2 * c] + vr;
-              row[ooff + 2 * c + 1] = first_of_group ? vi : row[ooff + 2 * c + 1] + vi;
+          block_factor(rec_s + le * L.rec_pitch, a.n_f, desc_s + b * FDESC, fr, fi);
+          f_s[2 * b * tile + le] = fr;
+          f_s[(2 * b + 1) * tile + le] = fi;
+        }
+      __syncthreads();
+      T* row = rec_s + le * L.row_pitch;
+      if (le < n_tile)
+        for (int n = sub; n < n_out_s; n += subs) {
+          const int4 o = out_s[n];
+          const int c = o.z;
+          T vr = T(0), vi = T(0);
+          for (int b = o.x; b < o.y; ++b) {
+            const int4 at = block_s[b];
+            if (c >= at.z) continue;
+            if (at.y < 0) {
+              vr += u_s[at.x + c * L.e_pitch + le];
+              continue;
             }
-          };
-          int c = 0;
-          if (sizeof(T) == 4 && (a.wc % 2) == 0 && (zoff % 2) == 0) {
-            // two complex columns per 16-byte shared-memory load: (re, im, re, im) of columns c, c + 1 for one t
-            for (; c + 2 <= bm; c += 2) {
-              T ur0 = T(0), ui0 = T(0), ur1 = T(0), ui1 = T(0);
-#pragma unroll
-              for (int t = 0; t < KMAX; ++t)
-                if (KT || t < a.k) {
-                  const float4 z = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(zc_s) + (t * a.wc + zoff + c) * 2);
-                  ur0 += hh[t] * (T)z.x; ui0 += hh[t] * (T)z.y;
-                  ur1 += hh[t] * (T)z.z; ui1 += hh[t] * (T)z.w;
-                }
-              emit(c, ur0, ui0);
-              emit(c + 1, ur1, ui1);
-            }
+            const T* u = u_s + at.x + 2 * c * L.e_pitch + le;
+            const T* f = f_s + at.y + le;
+            const T ur = u[0], ui = u[L.e_pitch], fr = f[0], fi = f[tile];
+            vr += fr * ur;
+            vr -= fi * ui;
+            vi += fr * ui;
+            vi += fi * ur;
           }
-          for (; c < bm; ++c) {
-            T ur = T(0), ui = T(0);
-#pragma unroll
-            for (int t = 0; t < KMAX; ++t)
-              if (KT || t < a.k) {
-                ur += hh[t] * zc_s[(t * a.wc + zoff + c) * 2];
-                ui += hh[t] * zc_s[(t * a.wc + zoff + c) * 2 + 1];
-              }
-            emit(c, ur, ui);
+          if (o.w < 0) {
+            row[~o.w] = vr;
+          } else {
+            row[o.w] = vr;
+            row[o.w + 1] = vi;
           }
         }
-      }
-      __syncwarp();
-      const T* warp_rows = row - (size_t)lane * pitch;
-      for (int r = 0; r < 32; ++r) {
-        const int64_t e_r = __shfl_sync(0xffffffffu, e, r);
-        if (e_r < 0) break;  // lanes take consecutive x: the first idle lane ends the warp's rows
-        for (int c = lane; c < a.d_out; c += 32) a.out[e_r * a.d_out + c] = warp_rows[(size_t)r * pitch + c];
-      }
-      __syncwarp();
+      __syncthreads();
+      for_rows(n_tile, a.d_out, [&](int e, int c) { a.out[edges_s[e] * a.d_out + c] = rec_s[e * L.row_pitch + c]; });
     }
   }
 }
@@ -191,116 +313,184 @@ __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict
   }
 }
 
-// Backward.  C = 2 wc + wr packed columns, CP = C rounded up to a whole number of 16-byte vectors (the padding
-// columns of Z and W stay zero), so that both small products run on 16-byte shared-memory loads:
-//   dh(e, t)   = <W(e), Z_t>           one thread per (edge, t), V columns per pair of loads
-//   dZ(t, c)  += h~_t(e) W_c(e)        a thread owns patches of V consecutive columns of one t, in registers
+// Backward.  C = 2 wc + wr packed columns; the rows of Z, W lie at `pitch` >= C elements: a multiple of 4 (16-byte vectors)
+// that is an odd number of them (rows of neighbouring edges on different banks); padding columns stay zero.
 template <typename T>
-__global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a, int C, int CP) {
-  constexpr int V = 16 / sizeof(T);
-  constexpr int MAX_PATCH = MAX_OWNED / V;
+struct BackwardLayout {  // shared memory, in elements of T
+  int pitch, quads, tgroups, h_pitch, rec_pitch, g_pitch, tile;
+  int z, w, h, rec, g, scale, total;
+  __host__ __device__ BackwardLayout(int k, int C, int n_f, int d_out, int tile_) {
+    const int vecs = (C + 3) / 4;
+    tile = tile_;
+    pitch = 4 * (vecs | 1);
+    quads = (k - 1 + 3) / 4;           // groups of 4 trunk rows t = 1 ..
+    tgroups = (k + TP - 1) / TP;
+    h_pitch = tile + 4;                // h~ transposed: (t, edge)
+    rec_pitch = 4 * n_f + 1;
+    g_pitch = d_out | 1;
+    z = 0;
+    const int z_rows = 1 + 4 * quads;
+    w = z + z_rows * pitch;
+    h = w + tile * pitch;
+    rec = h + tgroups * TP * h_pitch;
+    g = rec + tile * rec_pitch;
+    scale = g + tile * g_pitch;
+    total = scale + tile;
+  }
+};
+
+// NP: dZ patches per thread and pass over the source's edges (wider kernels take several passes)
+template <typename T, int NP>
+__global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a, int C, int tile) {
   extern __shared__ __align__(16) unsigned char raw[];
-  const int K = a.k;
-  T* z_s = reinterpret_cast<T*>(raw);  // (K, CP): packed per t as [zc (wc, 2) | zr (wr) | 0]
-  T* w_s = z_s + K * CP;               // (TILE, CP)
-  T* h_s = w_s + TILE * CP;            // (TILE, K)
-  const int wc2 = 2 * a.wc, patches = K * (CP / V);
-  for (int x = threadIdx.x; x < TILE * CP; x += blockDim.x) w_s[x] = T(0);  // the padding columns are never written again
+  __shared__ int64_t edges_s[MAX_TILE], g_rows_s[MAX_TILE];  // the tile's edges, and the rows of g that reach them
+  const BackwardLayout<T> L(a.k, C, a.n_f, a.d_out, tile);
+  const int K = a.k, wc2 = 2 * a.wc, pitch = L.pitch;
+  T* base_s = reinterpret_cast<T*>(raw);
+  T* z_s = base_s + L.z;      // (1 + 4 quads, pitch): packed per t as [zc (wc, 2) | zr (wr) | 0]
+  T* w_s = base_s + L.w;      // (tile, pitch)
+  T* h_s = base_s + L.h;      // (TP tgroups, h_pitch)
+  T* rec_s = base_s + L.rec;  // (tile, rec_pitch)
+  T* g_s = base_s + L.g;      // (tile, g_pitch): the edge's output-gradient row
+  T* scale_s = base_s + L.scale;
+  for (int x = threadIdx.x; x < L.rec; x += FTHREADS) base_s[x] = T(0);  // padding rows and columns are never written again
+  const int col_quads = (C + 3) / 4, patches = L.tgroups * col_quads;
+  const int passes = (patches + NP * FTHREADS - 1) / (NP * FTHREADS);
   for (int64_t grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
     const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
     __syncthreads();
-    for (int x = threadIdx.x; x < K * CP; x += blockDim.x) {
-      const int t = x / CP, c = x - t * CP;
-      z_s[x] = c < wc2 ? a.zc[(j * K + t) * wc2 + c] : (c < C ? a.zr[(j * K + t) * a.wr + (c - wc2)] : T(0));
-    }
-    T acc[MAX_PATCH][V];
+    stage_node(a, j, z_s, pitch);
+    for (int pass = 0; pass < passes; ++pass) {
+      T acc[NP][TP][4];
 #pragma unroll
-    for (int o = 0; o < MAX_PATCH; ++o)
+      for (int o = 0; o < NP; ++o)
 #pragma unroll
-      for (int v = 0; v < V; ++v) acc[o][v] = T(0);
-    for (int64_t base = first; base < last; base += TILE) {
-      const int n_tile = (int)min((int64_t)TILE, last - base);
-      __syncthreads();
-      // build W(e) and h~(e): threads split (edge, block) pairs
-      for (int x = threadIdx.x; x < n_tile * a.n_blocks; x += blockDim.x) {
-        const int le = x / a.n_blocks, b = x - le * a.n_blocks;
-        const int64_t e = a.order[base + le];
-        const int32_t* d = a.desc + b * FDESC;
-        const int kind = d[0], zoff = d[1], bm = d[2], ooff = d[6];
-        const bool take_real = d[7] != 0;
-        const T scale = a.weights ? a.weights[e] : T(1);
-        const T* g = a.target ? a.g + a.target[e] * a.d_out : a.g + e * a.d_out;
-        T* w = w_s + le * CP;
-        if (kind == 0) {
-          for (int c = 0; c < bm; ++c) w[wc2 + zoff + c] = scale * g[ooff + c];
-        } else {
-          T fr, fi;
-          block_factor(a, e, d, fr, fi);
-          for (int c = 0; c < bm; ++c) {
-            const T gr = scale * (take_real ? g[ooff + c] : g[ooff + 2 * c]);
-            const T gi = take_real ? T(0) : scale * g[ooff + 2 * c + 1];
-            w[(zoff + c) * 2] = gr * fr + gi * fi;  // W = G conj(F)
-            w[(zoff + c) * 2 + 1] = gi * fr - gr * fi;
+        for (int t = 0; t < TP; ++t)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) acc[o][t][v] = T(0);
+      for (int64_t base = first; base < last; base += tile) {
+        const int n_tile = (int)min((int64_t)tile, last - base);
+        __syncthreads();
+        if ((int)threadIdx.x < n_tile) {
+          const int64_t e = a.order[base + threadIdx.x];
+          edges_s[threadIdx.x] = e;
+          g_rows_s[threadIdx.x] = a.target ? a.target[e] : e;
+        }
+        __syncthreads();
+        stage_records(a, edges_s, n_tile, rec_s);
+        stage_rows(g_s, L.g_pitch, a.g, a.d_out, n_tile, g_rows_s);
+        for_rows(n_tile, K - 1, [&](int le, int t) { copy_async(h_s + (t + 1) * L.h_pitch + le, a.h + edges_s[le] * (K - 1) + t); });
+        // edges beyond the tile's end (their h~ multiplies whatever W rows an earlier tile left): zero
+        for (int x = threadIdx.x; x < (tile - n_tile) * K; x += FTHREADS) h_s[(x % K) * L.h_pitch + n_tile + x / K] = T(0);
+        if ((int)threadIdx.x < n_tile) {
+          h_s[threadIdx.x] = T(1);
+          scale_s[threadIdx.x] = a.weights ? a.weights[edges_s[threadIdx.x]] : T(1);
+        }
+        // rows of W beyond the tile's end: zero as well, a non-finite leftover must not meet that zero
+        for (int x = threadIdx.x; x < (tile - n_tile) * pitch; x += FTHREADS) w_s[n_tile * pitch + x] = T(0);
+        copy_wait();
+        __syncthreads();
+        // W(e): a warp takes 32 edges of one block
+        const int le = threadIdx.x & (tile - 1);
+        for (int b = threadIdx.x / tile; b < a.n_blocks && le < n_tile; b += FTHREADS / tile) {
+          const int32_t* d = a.desc + b * FDESC;
+          const int kind = d[0], zoff = d[1], bm = d[2], ooff = d[6];
+          const bool take_real = d[7] != 0;
+          const T scale = scale_s[le];
+          const T* g = g_s + le * L.g_pitch + ooff;
+          T* w = w_s + le * pitch;
+          if (kind == 0) {
+            for (int c = 0; c < bm; ++c) w[wc2 + zoff + c] = scale * g[c];
+          } else {
+            T fr, fi;
+            block_factor(rec_s + le * L.rec_pitch, a.n_f, d, fr, fi);
+            for (int c = 0; c < bm; ++c) {
+              const T gr = scale * (take_real ? g[c] : g[2 * c]);
+              const T gi = take_real ? T(0) : scale * g[2 * c + 1];
+              w[(zoff + c) * 2] = gr * fr + gi * fi;  // W = G conj(F)
+              w[(zoff + c) * 2 + 1] = gi * fr - gr * fi;
+            }
+          }
+        }
+        if (a.dweights && pass == 0) {  // dweights_e = <g_i, row_e>: eight lanes per edge
+          const int sub = threadIdx.x & 7;
+          for (int l0 = 0; l0 < n_tile; l0 += FTHREADS / 8) {
+            const int le = l0 + (threadIdx.x >> 3);
+            T s = T(0);
+            if (le < n_tile)
+              for (int c = sub; c < a.d_out; c += 8) s += g_s[le * L.g_pitch + c] * a.rows[edges_s[le] * a.d_out + c];
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (le < n_tile && sub == 0) a.dweights[edges_s[le]] = s;
+          }
+        }
+        __syncthreads();
+        if (pass == 0) {  // dh(e, t) = <W(e), Z_t>, t >= 1: edges le, le + tile / 2 and four t per thread
+          const int half = tile / 2;
+          for (int x = threadIdx.x; x < half * L.quads; x += FTHREADS) {
+            const int le = x / L.quads, t0 = 1 + 4 * (x - le * L.quads);
+            const T* w0 = w_s + le * pitch;
+            const T* w1 = w0 + half * pitch;
+            const T* z = z_s + t0 * pitch;
+            T s0[4] = {T(0), T(0), T(0), T(0)}, s1[4] = {T(0), T(0), T(0), T(0)};
+            for (int c = 0; c < 4 * col_quads; c += 4) {
+              const Vec4<T> v0 = load4(w0 + c), v1 = load4(w1 + c);
+#pragma unroll
+              for (int t = 0; t < 4; ++t) {
+                const Vec4<T> zv = load4(z + t * pitch + c);
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                  s0[t] += v0.v[v] * zv.v[v];
+                  s1[t] += v1.v[v] * zv.v[v];
+                }
+              }
+            }
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+              if (t0 + t >= K) break;
+              if (le < n_tile) a.dh[edges_s[le] * (K - 1) + t0 + t - 1] = s0[t];
+              if (le + half < n_tile) a.dh[edges_s[le + half] * (K - 1) + t0 + t - 1] = s1[t];
+            }
+          }
+        }
+        // dZ(t, c) += h~_t(e) W_c(e): patch x stays with this thread through the pass
+#pragma unroll
+        for (int o = 0; o < NP; ++o) {
+          const int x = threadIdx.x + (pass * NP + o) * FTHREADS;
+          if (x < patches) {
+            const int tg = x / col_quads, c = 4 * (x - tg * col_quads);
+            const T* hr = h_s + tg * TP * L.h_pitch;
+            for (int le = 0; le < n_tile; le += 4) {
+              Vec4<T> wv[4];
+#pragma unroll
+              for (int u = 0; u < 4; ++u) wv[u] = load4(w_s + (le + u) * pitch + c);
+#pragma unroll
+              for (int t = 0; t < TP; ++t) {
+                const Vec4<T> hv = load4(hr + t * L.h_pitch + le);
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+#pragma unroll
+                  for (int v = 0; v < 4; ++v) acc[o][t][v] += hv.v[u] * wv[u].v[v];
+              }
+            }
           }
         }
       }
-      for (int x = threadIdx.x; x < n_tile * K; x += blockDim.x) {
-        const int le = x / K, t = x - le * K;
-        const int64_t e = a.order[base + le];
-        h_s[le * K + t] = t == 0 ? T(1) : a.h[e * (K - 1) + t - 1];
-      }
-      if (a.dweights) {  // dweights_e = <g_i, row_e>
-        for (int le = threadIdx.x; le < n_tile; le += blockDim.x) {
-          const int64_t e = a.order[base + le];
-          const T* g = a.g + a.target[e] * a.d_out;
-          T s = T(0);
-          for (int c = 0; c < a.d_out; ++c) s += g[c] * a.rows[e * a.d_out + c];
-          a.dweights[e] = s;
-        }
-      }
-      __syncthreads();
-      // dh(e, t) = <W(e), Z_t>, t >= 1
-      for (int x = threadIdx.x; x < n_tile * (K - 1); x += blockDim.x) {
-        const int le = x / (K - 1), t = x - le * (K - 1) + 1;
-        const T* w = w_s + le * CP;
-        const T* z = z_s + t * CP;
-        T s = T(0);
-        for (int c = 0; c < CP; c += V) {
-          T wv[V], zv[V];
-          *reinterpret_cast<uint4*>(wv) = *reinterpret_cast<const uint4*>(w + c);
-          *reinterpret_cast<uint4*>(zv) = *reinterpret_cast<const uint4*>(z + c);
 #pragma unroll
-          for (int v = 0; v < V; ++v) s += wv[v] * zv[v];
-        }
-        a.dh[a.order[base + le] * (K - 1) + t - 1] = s;
-      }
-      // dZ(t, c) += h~_t(e) W_c(e): patch x = threadIdx.x + o * blockDim.x stays with this thread
+      for (int o = 0; o < NP; ++o) {
+        const int x = threadIdx.x + (pass * NP + o) * FTHREADS;
+        if (x >= patches) continue;
+        const int tg = x / col_quads, c0 = 4 * (x - tg * col_quads);
 #pragma unroll
-      for (int o = 0; o < MAX_PATCH; ++o) {
-        const int x = threadIdx.x + o * FTHREADS;
-        if (x < patches) {
-          const int t = x / (CP / V), c = (x - t * (CP / V)) * V;
-          for (int le = 0; le < n_tile; ++le) {
-            const T hv = h_s[le * K + t];
-            T wv[V];
-            *reinterpret_cast<uint4*>(wv) = *reinterpret_cast<const uint4*>(w_s + le * CP + c);
+        for (int t = 0; t < TP; ++t)
 #pragma unroll
-            for (int v = 0; v < V; ++v) acc[o][v] += hv * wv[v];
+          for (int v = 0; v < 4; ++v) {
+            const int64_t tt = tg * TP + t;
+            const int c = c0 + v;
+            if (tt >= K) continue;
+            if (c < wc2) a.dzc[(j * K + tt) * wc2 + c] = acc[o][t][v];
+            else if (c < C) a.dzr[(j * K + tt) * a.wr + (c - wc2)] = acc[o][t][v];
           }
-        }
-      }
-    }
-#pragma unroll
-    for (int o = 0; o < MAX_PATCH; ++o) {
-      const int x = threadIdx.x + o * FTHREADS;
-      if (x < patches) {
-        const int t = x / (CP / V), c0 = (x - t * (CP / V)) * V;
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-          const int c = c0 + v;
-          if (c < wc2) a.dzc[(j * K + t) * wc2 + c] = acc[o][v];
-          else if (c < C) a.dzr[(j * K + t) * a.wr + (c - wc2)] = acc[o][v];
-        }
       }
     }
   }
@@ -338,14 +528,16 @@ extern "C" int gm_factored_forward(const void* h, const void* zc, const void* zr
     a.h = (const T*)h; a.zc = (const T*)zc; a.zr = (const T*)zr; a.angular = (const T*)angular; a.transport = (const T*)transport;
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.out = (T*)out;
-    const int pitch = d_out | 1;  // per-thread output rows in shared memory, odd pitch
-    const size_t smem = ((size_t)k * 2 * wc + ((size_t)k * wr + 3) / 4 * 4 + (size_t)FTHREADS * pitch) * sizeof(T);
-    int st = k == 17 ? allow_smem(factored_forward_kernel<T, 17>, smem, "gm_factored_forward")
-                     : allow_smem(factored_forward_kernel<T, 0>, smem, "gm_factored_forward");
+    const int C = 2 * wc + wr;
+    const size_t extra = (size_t)(n_blocks * FDESC) * sizeof(int32_t) + (size_t)(n_blocks + d_out) * sizeof(int4);
+    // 64 edges per tile; fewer where the packed width or the phase tables leave no room for them
+    int tile = MAX_TILE;
+    while (tile > 8 && ForwardLayout<T>(k, C, n_f, n_blocks, d_out, tile).total * sizeof(T) + extra > 200 * 1024) tile /= 2;
+    const size_t smem = ForwardLayout<T>(k, C, n_f, n_blocks, d_out, tile).total * sizeof(T) + extra;
+    int st = allow_smem(factored_forward_kernel<T>, smem, "gm_factored_forward");
     if (st != GM_OK) return st;
-    const unsigned blocks = (unsigned)(n_groups < (1 << 20) ? n_groups : (1 << 20));
-    if (k == 17) factored_forward_kernel<T, 17><<<blocks, FTHREADS, smem, (cudaStream_t)stream>>>(a, pitch);
-    else factored_forward_kernel<T, 0><<<blocks, FTHREADS, smem, (cudaStream_t)stream>>>(a, pitch);
+    const int64_t cap = (int64_t)sm_count() * 16;  // the CTAs stride the sources: the column list is built once per CTA
+    factored_forward_kernel<T><<<(unsigned)(n_groups < cap ? n_groups : cap), FTHREADS, smem, (cudaStream_t)stream>>>(a, tile);
     return launch_status("gm_factored_forward");
   };
   return dtype == GM_F32 ? run(float()) : run(double());
@@ -386,13 +578,19 @@ extern "C" int gm_factored_backward(const void* g, const int64_t* target, const 
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.g = (const T*)g; a.target = target; a.weights = aggregated ? (const T*)weights : nullptr; a.rows = aggregated ? (const T*)rows : nullptr;
     a.dh = (T*)dh; a.dzc = (T*)dzc; a.dzr = (T*)dzr; a.dweights = aggregated ? (T*)dweights : nullptr;
-    const int V = 16 / (int)sizeof(T), CP = (C + V - 1) / V * V;  // packed columns padded to whole 16-byte vectors
-    const size_t smem = ((size_t)k * CP + (size_t)TILE * CP + (size_t)TILE * k) * sizeof(T);
-    int st = allow_smem(factored_backward_kernel<T>, smem, "gm_factored_backward");
-    if (st != GM_OK) return st;
+    // 64 edges per tile; fewer where the packed width is so large that 64 rows of it do not fit shared memory
+    int tile = MAX_TILE;
+    while (tile > 8 && BackwardLayout<T>(k, C, n_f, d_out, tile).total * sizeof(T) > 200 * 1024) tile /= 2;
+    const BackwardLayout<T> L(k, C, n_f, d_out, tile);
+    const size_t smem = (size_t)L.total * sizeof(T);
     const unsigned blocks = (unsigned)(n_groups < (1 << 20) ? n_groups : (1 << 20));
-    factored_backward_kernel<T><<<blocks, FTHREADS, smem, (cudaStream_t)stream>>>(a, C, CP);
-    return launch_status("gm_factored_backward");
+    auto go = [&](auto kernel) {
+      int st = allow_smem(kernel, smem, "gm_factored_backward");
+      if (st != GM_OK) return st;
+      kernel<<<blocks, FTHREADS, smem, (cudaStream_t)stream>>>(a, C, tile);
+      return launch_status("gm_factored_backward");
+    };
+    return L.tgroups * ((C + 3) / 4) <= FTHREADS ? go(factored_backward_kernel<T, 1>) : go(factored_backward_kernel<T, 2>);
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }

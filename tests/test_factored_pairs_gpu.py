@@ -12,7 +12,7 @@ import numpy as np
 import pytest
 import torch
 
-from tests.helpers import assert_close, cuda, make_case, seeded
+from tests.helpers import assert_close, cuda, make_case, rel_err, seeded
 
 pytestmark = pytest.mark.gpu
 
@@ -136,6 +136,62 @@ def test_factored_autograd_functions():
     grads_b = torch.autograd.grad((want * g).sum(), (H, ZC, ZR, W))
     for a, b in zip(grads_a, grads_b):
         assert torch.allclose(a, b, rtol=1e-9, atol=1e-10)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("type_in, type_out, k, degrees", [
+    ({0: 1}, {0: 3}, 1, [1, 2]),                                        # no trunk, no complex block
+    ({0: 2, 1: 2}, {0: 2, 1: 3}, 2, [64, 65, 0, 63]),                   # tile of 64 edges: exact, one more, one less; a source without edges
+    ({1: 3}, {0: 5, 2: 5}, 6, [3, 130]),                                # no scalar block; k - 1 = 5 is no multiple of 4
+    ({0: 8, 1: 8, 2: 8}, {0: 4, 1: 4, 2: 4}, 17, [92, 7, 129]),
+    ({0: 2, 1: 2, 2: 2}, {0: 8, 1: 8, 2: 8}, 20, [66, 31]),             # 200 packed columns: two dZ patches per thread
+    ({0: 2, 1: 2, 2: 2, 3: 2}, {0: 9, 1: 9, 2: 9, 3: 9}, 17, [70, 5]),  # 441 packed columns: smaller tiles in float64
+    ({0: 2, 1: 2, 2: 2}, {0: 25, 1: 25, 2: 25}, 11, [33]),              # 625 packed columns: several passes over the edges
+])
+def test_factored_against_plain_sums(type_in, type_out, k, degrees, dtype):
+    """Rows and all gradients against the op's definition written with torch in float64: float64 to 1e-10, float32 to
+    2e-6 of each tensor's magnitude (sums of at most 130 edges x 441 columns of O(1) terms)."""
+    from gm_attention_b200.fields import FieldType
+    from gm_attention_b200.nn import fused_factored as ff
+
+    blocks, powers = blocks_for(type_in, type_out)
+    p = ff.plan_blocks(blocks, FieldType(type_out), powers)
+    n_f, n = 8, len(degrees)
+    rng = np.random.default_rng(5)
+    source = rng.permutation(np.repeat(np.arange(n), degrees))
+    e = source.shape[0]
+    h, zc, zr, g = (rng.standard_normal(shape).astype(dtype) for shape in ((e, k - 1), (n, k, p.wc, 2), (n, k, p.wr), (e, p.d_out)))
+    phase = np.exp(1j * rng.uniform(0, 6.28, (2, e, 1)) * np.arange(n_f))
+    angular, transport = (np.stack([x.real, x.imag], -1).astype(dtype) for x in phase)
+    rho = rng.uniform(0.1, 1.0, e).astype(dtype)
+    # the definition
+    H, ZC, ZR = (torch.from_numpy(x.astype(np.float64)).requires_grad_(True) for x in (h, zc, zr))
+    src = torch.from_numpy(source)
+    A, T = (torch.view_as_complex(torch.from_numpy(x.astype(np.float64))) for x in (angular, transport))
+    hh = torch.cat([torch.ones(e, 1, dtype=torch.float64), H], 1)
+    uc, ur = torch.einsum("et,etcx->ecx", hh, ZC[src]), torch.einsum("et,etc->ec", hh, ZR[src])
+    order = lambda table, o: table[:, o] if o >= 0 else table[:, -o].conj()
+    want = torch.zeros(e, p.d_out, dtype=torch.float64)
+    for b in p.blocks:
+        if b.kind == 0:
+            part = ur[:, b.z_offset:b.z_offset + b.b_m]
+        else:
+            factor = order(A, b.angular) * order(T, b.transport) * torch.from_numpy(rho.astype(np.float64)) ** b.power
+            z = factor[:, None] * torch.view_as_complex(uc[:, b.z_offset:b.z_offset + b.b_m].contiguous())
+            part = z.real if b.take_real else torch.view_as_real(z).reshape(e, -1)
+        want = want + torch.nn.functional.pad(part, (b.out_offset, p.d_out - b.out_offset - part.shape[1]))
+    grads = torch.autograd.grad((want * torch.from_numpy(g.astype(np.float64))).sum(), (H, ZC, ZR), allow_unused=True)
+    # the op
+    desc = np.array([b.row() for b in p.blocks], np.int32).reshape(-1, 8)
+    groups = [x.cuda() for x in ff.source_groups(src)]
+    leaves = [cuda(x).requires_grad_(True) for x in (h, zc, zr)]
+    rows = ff.Factored.apply(*leaves, *(cuda(x) for x in (angular, transport, rho, desc, source)), *groups, p.d_out, p.max_bm)
+    got = torch.autograd.grad(rows, leaves, cuda(g))
+    tolerance = 1e-10 if dtype == np.float64 else 2e-6
+    for name, a, b in zip(("rows", "dh", "dzc", "dzr"), (rows.detach(), *got), (want.detach(), *grads)):
+        if b is None or b.numel() == 0:
+            continue
+        assert rel_err(a.cpu().numpy(), b.numpy()) < tolerance, name
 
 
 PAIR_CASES = [
