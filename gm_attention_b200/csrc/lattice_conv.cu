@@ -19,7 +19,8 @@
 // one item -- a complex copy, or a pair of scalar channels -- so a warp reads 32 neighbouring items of a node as one
 // 128-byte line; it keeps 8 longitudes x 2 samples of accumulators in registers and slides a register window of 8
 // source longitudes (apply) or 8 target longitudes (table_grad) past them, so every loaded value is used for 8 x 4
-// multiply-adds and nothing is staged in shared memory.  Results do not depend on the launch geometry: no atomics.
+// multiply-adds without shared memory.  apply has a second form that stages both operands and packs the arithmetic, taken
+// wherever a stage fits.  Results do not depend on the launch geometry: no atomics.
 #include "common.cuh"
 
 namespace gmb {
@@ -174,6 +175,211 @@ __global__ void __launch_bounds__(THREADS, 3) conv_apply_kernel(const ConvArgs a
   }
 }
 
+// ------------------------------------------------------------------------------------------------------- apply, staged
+// The same sums with the window's sources and table entries brought to shared memory first.  A CTA covers G tiles of 8
+// longitudes (thread = tile x item); a stage holds up to SO offsets of one window: their table entries, read once per CTA
+// instead of once per tile, and the 8 G + SO - 1 source positions of NB samples they meet.  The copies of the next stage
+// (cp.async, 16 bytes where the field's rows allow) run while the current one is consumed, so a window's first sources are
+// not waited for, and the inner loop has no addresses to form.
+//
+// The arithmetic is packed: fma.rn.f32x2 on the targets (l, l + 4), whose sources (t, t + 4) form a register pair; moving
+// one offset on renames three of the four pairs and rebuilds the fourth from its own upper half and the new source, so the
+// window costs one move per value.  Per offset, copy and NB samples 16 NB packed multiply-adds stand against about 8 moves
+// (the matrix, duplicated into pairs) and 6 NB of loads, conversions and window moves.  Same order of operations per
+// output as conv_apply_kernel: bit-identical results.  256 x 512, radius 4 pi / 256, batch 4, 64 x (m <= 2), bf16: 7.92 ms
+// with conv_apply_kernel, 4.51 in this form (FMA pipe about 40 % busy, 10 warps' barriers and the per-stage set-up beside
+// it); 45 x 88, batch 3, 32 x (m <= 2), float32: 220 us before, 128 now.
+struct StagedShape {
+  int tiles, so, threads, stage_bytes, pos_bytes;  // G, SO, G * n_items, bytes of a stage, bytes of one node's row
+  int vec16;                                       // rows and bases are multiples of 16 bytes
+};
+
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
+  if constexpr (BYTES == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(addr), "l"(src) : "memory");
+  else asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(addr), "l"(src), "n"(BYTES) : "memory");
+}
+template <typename S> __device__ __forceinline__ float2 shared_pair(const unsigned char* p) {
+  if constexpr (sizeof(S) == 4) return *reinterpret_cast<const float2*>(p);
+  else return Pair<__nv_bfloat16>::unpack(*reinterpret_cast<const unsigned*>(p));
+}
+// `bytes` consecutive bytes of a cyclic row of row_bytes, from byte `at` on, into shared memory
+template <int BYTES>
+__device__ __forceinline__ void copy_cyclic(unsigned char* dst, const unsigned char* row, int at, int bytes, int row_bytes, int threads) {
+  for (int u = threadIdx.x * BYTES; u < bytes; u += threads * BYTES) {
+    int o = at + u;
+    while (o >= row_bytes) o -= row_bytes;
+    copy_async<BYTES>(dst + u, row + o);
+  }
+}
+
+// KIND 0: complex copies (2 x 2 matrices), 1: pairs of scalar channels.  One stage's offsets for one thread.
+template <typename S, int NB, int KIND>
+__device__ __forceinline__ void consume_stage(const unsigned char* table, int entry_bytes, const unsigned char* pos, int pos_bytes, int sample_bytes,
+                                              int n, bool transpose, unsigned long long (&ax)[4][NB], unsigned long long (&ay)[4][NB]) {
+  unsigned long long px[4][NB], py[4][NB];  // slot (d + j) & 3: sources (d + j, d + j + 4)
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    float2 v[7];
+#pragma unroll
+    for (int t = 0; t < 7; ++t) v[t] = shared_pair<S>(pos + b * sample_bytes + t * pos_bytes);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      px[j][b] = pack2(v[j].x, v[j + 4].x);
+      py[j][b] = pack2(v[j].y, v[j + 4].y);
+    }
+    // the first step turns slot 3 into (source 3, source 7): as after every step, the lower half comes from the upper one
+    px[3][b] = pack2(0.f, v[3].x);
+    py[3][b] = pack2(0.f, v[3].y);
+  }
+  pos += 7 * pos_bytes;
+  for (int d0 = 0; d0 < n; d0 += 4) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (d0 + u >= n) break;
+      // source d + 7 completes the pair (d + 3, d + 7): its lower half is the upper half of the pair that left the window
+#pragma unroll
+      for (int b = 0; b < NB; ++b) {
+        const float2 v = shared_pair<S>(pos + b * sample_bytes);
+        px[(u + 3) & 3][b] = pack2(unpack2(px[(u + 3) & 3][b]).y, v.x);
+        py[(u + 3) & 3][b] = pack2(unpack2(py[(u + 3) & 3][b]).y, v.y);
+      }
+      pos += pos_bytes;
+      if constexpr (KIND == 0) {
+        const float4 m = *reinterpret_cast<const float4*>(table);
+        const float my = transpose ? m.z : m.y, mz = transpose ? m.y : m.z;
+        const unsigned long long m00 = pack2(m.x, m.x), m01 = pack2(my, my), m10 = pack2(mz, mz), m11 = pack2(m.w, m.w);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            const unsigned long long x = px[(u + j) & 3][b], y = py[(u + j) & 3][b];
+            ax[j][b] = fma2(m00, x, fma2(m01, y, ax[j][b]));
+            ay[j][b] = fma2(m10, x, fma2(m11, y, ay[j][b]));
+          }
+      } else {  // two independent scalar channels: no cross terms, so a non-finite value stays in its channel
+        const float2 m = *reinterpret_cast<const float2*>(table);
+        const unsigned long long m0 = pack2(m.x, m.x), m1 = pack2(m.y, m.y);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            ax[j][b] = fma2(m0, px[(u + j) & 3][b], ax[j][b]);
+            ay[j][b] = fma2(m1, py[(u + j) & 3][b], ay[j][b]);
+          }
+      }
+      table += entry_bytes;
+    }
+  }
+}
+
+constexpr int STAGED_THREADS = 320;
+
+template <typename S, int NB>
+__global__ void __launch_bounds__(STAGED_THREADS, 2) conv_apply_staged_kernel(const ConvArgs a, const StagedShape sh) {
+  extern __shared__ __align__(16) unsigned char stage_smem[];
+  const int row = a.order[blockIdx.y];
+  const int l0 = blockIdx.x * 8 * sh.tiles;
+  const int b0 = blockIdx.z * NB;
+  const int nb = min(NB, a.batch - b0);
+  const int span = 2 * a.halo + 1;
+  const int row_bytes = a.nlon * sh.pos_bytes, entry_bytes = 4 * a.table_width;
+  const size_t sample = (size_t)a.rows * row_bytes;
+  const unsigned char* x = static_cast<const unsigned char*>(a.x) + b0 * sample;
+  const int tile = threadIdx.x / a.n_items, item = threadIdx.x - tile * a.n_items;
+  const int kind = a.items[3 * item], col = a.items[3 * item + 1], fcol = a.items[3 * item + 2];
+  const int most_pos = 8 * sh.tiles + sh.so - 1, sample_bytes = most_pos * sh.pos_bytes;
+  const int table_at = (NB * sample_bytes + 15) / 16 * 16;
+
+  // stages: offsets [d, d + n) of window c of this row
+  struct Stage { int c, d, n, cnt; };
+  auto first_of = [&](int c) {
+    for (; c < span; ++c) {
+      const int j = row + c - a.halo;
+      if (j < 0 || j >= a.rows) continue;
+      const int cnt = a.win_cnt[row * span + c];
+      if (cnt > 0) return Stage{c, 0, min(sh.so, cnt), cnt};
+    }
+    return Stage{span, 0, 0, 0};
+  };
+  auto next_of = [&](const Stage& s) {
+    const int d = s.d + s.n;
+    return d < s.cnt ? Stage{s.c, d, min(sh.so, s.cnt - d), s.cnt} : first_of(s.c + 1);
+  };
+  auto issue = [&](int buf, const Stage& s) {
+    unsigned char* dst = stage_smem + (size_t)buf * sh.stage_bytes;
+    const int j = row + s.c - a.halo, w = row * span + s.c;
+    int p = l0 + a.win_lo[w] + s.d;
+    while (p < 0) p += a.nlon;
+    while (p >= a.nlon) p -= a.nlon;
+    const int at = p * sh.pos_bytes, bytes = (8 * sh.tiles + s.n - 1) * sh.pos_bytes;
+    for (int b = 0; b < nb; ++b) {
+      const unsigned char* src = x + b * sample + (size_t)j * row_bytes;
+      if (sh.vec16) copy_cyclic<16>(dst + b * sample_bytes, src, at, bytes, row_bytes, sh.threads);
+      else copy_cyclic<4>(dst + b * sample_bytes, src, at, bytes, row_bytes, sh.threads);
+    }
+    const unsigned char* entries = reinterpret_cast<const unsigned char*>(a.table) + (size_t)(a.win_off[w] + s.d) * entry_bytes;
+    for (int u = threadIdx.x * 16; u < s.n * entry_bytes; u += sh.threads * 16) copy_async<16>(dst + table_at + u, entries + u);
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+
+  unsigned long long ax[4][NB], ay[4][NB];  // targets (j, j + 4)
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) ax[j][b] = ay[j][b] = 0ull;
+
+  Stage cur = first_of(0);
+  if (cur.c < span) issue(0, cur);
+  int buf = 0;
+  while (cur.c < span) {
+    const Stage nxt = next_of(cur);
+    if (nxt.c < span) {
+      issue(buf ^ 1, nxt);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const unsigned char* st = stage_smem + (size_t)buf * sh.stage_bytes;
+    const unsigned char* pos = st + 8 * tile * sh.pos_bytes + col * (int)sizeof(S);
+    const unsigned char* table = st + table_at + 4 * fcol;
+    if (kind == 0) consume_stage<S, NB, 0>(table, entry_bytes, pos, sh.pos_bytes, sample_bytes, cur.n, a.transpose != 0, ax, ay);
+    else consume_stage<S, NB, 1>(table, entry_bytes, pos, sh.pos_bytes, sample_bytes, cur.n, false, ax, ay);
+    __syncthreads();
+    cur = nxt;
+    buf ^= 1;
+  }
+  S* y = static_cast<S*>(a.y) + ((size_t)b0 * a.rows + row) * a.nlon * a.width + col;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      const float2 vx = unpack2(ax[j][b]), vy = unpack2(ay[j][b]);
+      const int l = l0 + 8 * tile + j;
+      if (b >= nb || l >= a.nlon) continue;  // nlon is a multiple of 8: a tile is whole or absent
+      S* at = y + b * (size_t)a.rows * a.nlon * a.width + (size_t)l * a.width;
+      Pair<S>::store(at, make_float2(vx.x, vy.x));
+      Pair<S>::store(at + (size_t)4 * a.width, make_float2(vx.y, vy.y));
+    }
+}
+
 // ----------------------------------------------------------------------------------------------------------- table_grad
 // One CTA: one window (target row, source row) and 8 consecutive offsets d0 .. d0 + 7 of it; it walks once around the
 // source row.  Step u brings the source at longitude u + lo + d0; offset d0 + k pairs it with the target u - k (cyclic),
@@ -259,6 +465,36 @@ __global__ void __launch_bounds__(THREADS, 3) conv_table_grad_kernel(const ConvA
   }
 }
 
+// Tiles, offsets per stage and samples per thread of the staged apply kernel; returns the samples, 0 where it cannot run.
+// Two samples and two CTAs of 320 threads per SM (102 registers) measured 4.5 ms against 4.7 for four samples and one CTA,
+// 5.8 to 6.0 for CTAs of one tile (256 x 512, batch 4, 64 x (m <= 2), bf16).  A stage should hold the equator's windows
+// whole: where half of the shared memory holds fewer than 8 offsets (float32 rows of 320 columns: 3) a CTA takes all of it.
+// Tiles: as many as 320 threads take, fewer while the launch has less than two CTAs per SM (a small lattice waits for
+// its polar rows' chains of offsets).
+int staged_shape(const ConvArgs& a, int elem, int n_order, StagedShape& sh) {
+  if (a.n_items > STAGED_THREADS) return 0;
+  sh.pos_bytes = a.width * elem;
+  if ((int64_t)a.nlon * sh.pos_bytes > (1ll << 28)) return 0;  // offsets within a row are 32-bit
+  const uintptr_t base = reinterpret_cast<uintptr_t>(a.x);
+  sh.vec16 = sh.pos_bytes % 16 == 0 && base % 16 == 0;
+  const int nb = a.batch >= 2 ? 2 : 1;
+  sh.tiles = max(1, min(STAGED_THREADS / a.n_items, a.nlon / 8));
+  const int64_t want = 2 * (int64_t)sm_count();
+  auto ctas = [&]() { return (int64_t)n_order * ((a.nlon / 8 + sh.tiles - 1) / sh.tiles) * ((a.batch + nb - 1) / nb); };
+  while (ctas() < want && sh.tiles > 1) sh.tiles = (sh.tiles + 1) / 2;
+  sh.threads = sh.tiles * a.n_items;
+  for (const int budget : {55 * 1024, 110 * 1024})  // of the two buffers' one
+    for (sh.so = 16; sh.so >= (budget < 64 * 1024 ? 8 : 1); --sh.so) {
+      const int64_t pos = ((int64_t)nb * (8 * sh.tiles + sh.so - 1) * sh.pos_bytes + 15) / 16 * 16;
+      const int64_t bytes = pos + (int64_t)sh.so * a.table_width * 4;
+      if (bytes <= budget) {
+        sh.stage_bytes = (int)bytes;
+        return nb;
+      }
+    }
+  return 0;
+}
+
 int check_common(const char* what, const void* x, const float* table, const int* items, int n_items, const int* win_cnt, const int* win_lo,
                  const int* win_off, int rows, int nlon, int batch, int width, int halo, int table_width, int dtype) {
   GM_REQUIRE(dtype == GM_F32 || dtype == GM_BF16, GM_ERR_UNSUPPORTED, "%s: node fields are float32 or bfloat16", what);
@@ -291,19 +527,36 @@ extern "C" int gm_lattice_conv_apply(const void* x, const float* table, const in
   a.x = x; a.table = table; a.items = items; a.win_cnt = win_cnt; a.win_lo = win_lo; a.win_off = win_off; a.order = order; a.y = y;
   a.n_items = n_items; a.rows = rows; a.nlon = nlon; a.batch = batch; a.width = width; a.halo = halo; a.table_width = table_width;
   a.transpose = transpose;
-  const int threads = min(THREADS, (n_items + 31) / 32 * 32);
-  // 32 accumulators + a window of as many sources + 4 steps in flight stay under 128 registers: three CTAs per SM (four
-  // samples x 8 targets measured one CTA per SM and half the speed)
-  // (16 targets x 1 sample per thread -- the same registers -- measured the same 8.05 ms in bf16 and 4 % slower in float32)
-  const int nb = batch >= 2 ? 2 : 1, tl = LON;
-  GM_REQUIRE((batch + nb - 1) / nb <= 65535, GM_ERR_LIMIT, "gm_lattice_conv_apply: batch too large");
-  dim3 grid(nlon / tl, n_order, (batch + nb - 1) / nb);
   cudaStream_t cs = (cudaStream_t)stream;
+  const int elem = dtype == GM_F32 ? 4 : 2;
+  StagedShape sh{};
+  const int nb = staged_shape(a, elem, n_order, sh);
+  if (nb > 0) {
+    const size_t smem = 2 * (size_t)sh.stage_bytes;
+    const dim3 grid((nlon / 8 + sh.tiles - 1) / sh.tiles, n_order, (batch + nb - 1) / nb);
+    GM_REQUIRE(grid.z <= 65535, GM_ERR_LIMIT, "gm_lattice_conv_apply: batch too large");
+    auto go = [&](auto kernel) {
+      const int st = allow_smem(kernel, smem, "gm_lattice_conv_apply");
+      if (st != GM_OK) return st;
+      kernel<<<grid, sh.threads, smem, cs>>>(a, sh);
+      return launch_status("gm_lattice_conv_apply");
+    };
+    auto pick = [&](auto tag) {
+      using S = decltype(tag);
+      return nb == 2 ? go(conv_apply_staged_kernel<S, 2>) : go(conv_apply_staged_kernel<S, 1>);
+    };
+    return dtype == GM_F32 ? pick(float()) : pick(__nv_bfloat16());
+  }
+  // what a stage cannot hold: more items than a CTA has threads, or rows so wide that 8 + 1 positions outgrow shared memory
+  const int threads = min(THREADS, (n_items + 31) / 32 * 32);
+  const int pair = batch >= 2 ? 2 : 1;
+  GM_REQUIRE((batch + pair - 1) / pair <= 65535, GM_ERR_LIMIT, "gm_lattice_conv_apply: batch too large");
+  dim3 grid(nlon / LON, n_order, (batch + pair - 1) / pair);
 #define GM_APPLY(S, NB) conv_apply_kernel<S, NB, LON><<<grid, threads, 0, cs>>>(a)
   if (dtype == GM_F32) {
-    if (nb == 2) GM_APPLY(float, 2); else GM_APPLY(float, 1);
+    if (pair == 2) GM_APPLY(float, 2); else GM_APPLY(float, 1);
   } else {
-    if (nb == 2) GM_APPLY(__nv_bfloat16, 2); else GM_APPLY(__nv_bfloat16, 1);
+    if (pair == 2) GM_APPLY(__nv_bfloat16, 2); else GM_APPLY(__nv_bfloat16, 1);
   }
 #undef GM_APPLY
   return launch_status("gm_lattice_conv_apply");

@@ -126,6 +126,41 @@ def test_only_true_neighbours_are_touched():
 
 # ----------------------------------------------------------------------------- 256 x 512, radius 4 pi / 256, batch 4
 
+@pytest.mark.parametrize("storage", ["f32", "bf16"])
+@pytest.mark.parametrize("nlat, nlon, reach, head, batch", [
+    (6, 8, 1.5, {0: 2, 1: 1}, 1),                    # one tile; windows of whole rows; stages longer than the row
+    (6, 24, 2.0, {0: 10, 1: 10}, 3),                 # node rows of 60 / 120 bytes: 4-byte copies; an odd batch
+    (5, 144, 1.6, {0: 6, 1: 5, 2: 5}, 2),            # tiles beyond the last longitude, windows of several stages
+    (4, 32, 1.2, {0: 64, 1: 64, 2: 64}, 2),          # 160 items: two tiles fill 320 threads
+    (4, 16, 1.2, {0: 130, 1: 130, 2: 130}, 1),       # 325 items: more than a CTA has threads, the kernel without stages
+])
+def test_apply_against_the_host_loops(nlat, nlon, reach, head, batch, storage):
+    """Both forms of the apply kernel, forward and transposed, against numpy loops in float64 on the same (rounded) field:
+    at most ~300 products per output, 1e-5 of the largest in float32; one rounding to bf16 (2^-9) on top in bf16."""
+    from types import SimpleNamespace
+
+    from gm_attention_b200.nn.lattice_depthwise import _apply, conv_tables
+    from tests.test_lattice_depthwise_cpu import _apply_on_the_host
+
+    c = make_case(nlat, nlon, reach * math.pi / nlat, head, 1, dtype=np.float32)
+    geometry = SimpleNamespace(transport=cuda(c.transport), angular=cuda(c.angular), rho=cuda(c.rho), bias=cuda(c.bias), inside=cuda(c.inside),
+                               row_ptr=cuda(c.row_ptr), source=cuda(c.source))
+    t = conv_tables(geometry, cuda(c.rho * np.float32(c.radius)), cuda(c.weights), descriptor_rows(c.head_type, 1), nlat, nlon)
+    lat = t.lattice
+    table, = seeded((t.n_entries, t.table_width), 61, np.float32)
+    x = torch.from_numpy(seeded((batch * c.n_nodes, c.width), 62, np.float32)[0]).to(torch.bfloat16 if storage == "bf16" else torch.float32)
+    items = t.items.cpu().numpy().tolist()
+    sample = slice((batch - 1) * c.n_nodes, batch * c.n_nodes)
+    for transposed in (False, True):
+        windows = (lat.t_win_cnt, lat.t_win_lo, lat.t_win_off) if transposed else (lat.win_cnt, lat.win_lo, lat.win_off)
+        used = table[lat.t_entry.cpu().numpy()] if transposed else table
+        want = _apply_on_the_host(x[sample].double().numpy(), used.astype(np.float64), *(w.cpu().numpy() for w in windows), items, nlat, nlon, lat.halo,
+                                  transposed)
+        got = _apply(x.cuda(), cuda(used), t, transposed)[sample].float().cpu().numpy()
+        atol = 1e-5 * np.abs(want).max()
+        assert_close(got, want, 2.0 ** -8 if storage == "bf16" else 1e-5, atol, "transposed" if transposed else "forward")
+
+
 NLAT, NLON, BATCH, COPIES = 256, 512, 4, 64
 HEAD = {0: COPIES, 1: COPIES, 2: COPIES}
 RADIUS = 4 * math.pi / NLAT
