@@ -117,8 +117,9 @@ template <typename T, int R, int NF>
 __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArgs<T> a) {
   constexpr int FN = NF ? NF : MAX_F;
   const int lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= a.n_nodes) return;
+  const int64_t x = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (x >= a.n_nodes) return;
+  const int64_t i = from_both_ends(x, a.n_nodes);
   const int L = 32 / a.H, h = lane / L, s = lane % L;
   int col[FN][R], order[FN];
   T qr[FN][R], qi[FN][R];
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
     if (a.inside[e] && lw > m) m = lw;
     if (s == 0) a.alpha[e * a.H + h] = lw;
   };
-  constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together
+  constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together (8: 0.96 ms against 0.88)
   int64_t e = e0;
   for (; e + U <= e1; e += U) {
     const T* k_j[U];
@@ -274,7 +275,8 @@ __global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
   __syncthreads();
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   constexpr int U = 4;
-  for (int64_t i = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); i < a.n_nodes; i += (int64_t)gridDim.x * warps) {
+  for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
+    const int64_t i = from_both_ends(x, a.n_nodes);
     const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
     T total_of_lane = T(0);  // lane h < H ends up with sum_e alpha[e, h] dalpha[e, h]
     for (int h = 0; h < a.H; ++h) {
@@ -384,7 +386,8 @@ __global__ void conv_forward_kernel(ConvArgs<T> a) {
   int n_real = 0;  // items are in column order: the scalar block (frequency 0) first
   while (n_real < n_items && items_s[n_real].order == 0) ++n_real;
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int64_t i = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); i < a.n_nodes; i += (int64_t)gridDim.x * warps) {
+  for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
+    const int64_t i = from_both_ends(x, a.n_nodes);
     const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
     for (int t0 = 0; t0 < n_real; t0 += 32) {
       if (t0 + lane >= n_real) continue;
@@ -465,7 +468,8 @@ __global__ void conv_backward_kernel(ConvArgs<T> a) {
   int n_real = 0;
   while (n_real < n_items && items_s[n_real].order == 0) ++n_real;
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int64_t i = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); i < a.n_nodes; i += (int64_t)gridDim.x * warps) {
+  for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
+    const int64_t i = from_both_ends(x, a.n_nodes);
     const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
     for (int t0 = 0; t0 < n_real; t0 += 32) {
       if (t0 + lane >= n_real) continue;

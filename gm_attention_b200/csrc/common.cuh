@@ -71,6 +71,11 @@ __device__ __forceinline__ float gm_log(float x) { return logf(x); }
 __device__ __forceinline__ double gm_log(double x) { return log(x); }
 template <typename T> __device__ __forceinline__ T neg_inf() { return -(T)INFINITY; }
 
+// The x-th of n items taken from both ends of the list in turn: 0, n - 1, 1, n - 2, ...  On a lattice the nodes of large
+// degree are the polar rows, at the two ends of the node list; in plain order the last of them start when everything else
+// is done, and the launch ends in their serial chains of several hundred edges.
+__device__ __forceinline__ int64_t from_both_ends(int64_t x, int64_t n) { return x & 1 ? n - 1 - (x >> 1) : x >> 1; }
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

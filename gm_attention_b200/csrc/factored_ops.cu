@@ -220,7 +220,8 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, 
     }
   }
   const int le = threadIdx.x & (tile - 1), sub = threadIdx.x / tile, subs = FTHREADS / tile;
-  for (int64_t grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
+  for (int64_t g0 = blockIdx.x; g0 < a.n_groups; g0 += gridDim.x) {
+    const int64_t grp = from_both_ends(g0, a.n_groups);
     const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
     __syncthreads();
     stage_node(a, j, z_s, L.pitch);
@@ -303,8 +304,9 @@ template <typename T>
 __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict__ weights, const int64_t* __restrict__ row_ptr,
                                  int64_t n_targets, int d_out, T* __restrict__ out) {
   const int lane = threadIdx.x & 31;
-  const int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (i >= n_targets) return;
+  const int64_t x = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (x >= n_targets) return;
+  const int64_t i = from_both_ends(x, n_targets);
   const int64_t e0 = row_ptr[i], e1 = row_ptr[i + 1];
   for (int c = lane; c < d_out; c += 32) {
     T acc = T(0);
@@ -356,7 +358,8 @@ __global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a,
   for (int x = threadIdx.x; x < L.rec; x += FTHREADS) base_s[x] = T(0);  // padding rows and columns are never written again
   const int col_quads = (C + 3) / 4, patches = L.tgroups * col_quads;
   const int passes = (patches + NP * FTHREADS - 1) / (NP * FTHREADS);
-  for (int64_t grp = blockIdx.x; grp < a.n_groups; grp += gridDim.x) {
+  for (int64_t g0 = blockIdx.x; g0 < a.n_groups; g0 += gridDim.x) {
+    const int64_t grp = from_both_ends(g0, a.n_groups);
     const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
     __syncthreads();
     stage_node(a, j, z_s, pitch);
