@@ -43,6 +43,8 @@ SIGNATURES: dict[str, list[Any]] = {
     "gm_factored_backward": [_P] * 15 + [_L, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
     "gm_pairs_forward": [_P] * 8 + [_L, _I, _I, _I, _I, _I, _P],
     "gm_pairs_backward": [_P] * 11 + [_L, _I, _I, _I, _I, _I, _P],
+    "gm_node_products_forward": [_P] * 6 + [_L] + [_I] * 6 + [_P] * 3,
+    "gm_node_products_backward": [_P] * 8 + [_L] + [_I] * 9 + [_P] * 4,
     "gm_lattice_attention_tc_wait_expired": [_P],
     "gm_lattice_attention_forward_tc4": [_P] * 8 + [_I, _P, _I, _I, _I, _L, _I, _I, _I, _I, _I, _D, _P, _P, _P],
     "gm_lattice_attention_backward_tc4_passes": [_P] * 11 + [_I] + [_P] * 5 + [_I, _P, _I, _I, _I, _L, _I, _I, _I, _I, _I, _D, _P, _P, _P, _P, _I, _P],

@@ -17,6 +17,11 @@ coefficient-major slab of the coefficient gradient written), then the readout
 weight / bias gradients as ONE product of the coefficient gradient with
 ``[hidden | 1]``, summed over blocks of 16 384 edges like the reference's
 ``_blocked_weight_gradient`` (``nn/kernels.py:49-64``).
+
+``forward_general`` on a NODE-level field takes the factored form instead: an edge's phases commute with the sum over the
+input copies, so ``M(e) (pre u~)`` is a phase times ``sum_t h~_t(e) Z_t(source(e))`` with ``Z_t = W_t x`` formed once per node
+(:class:`NodeProducts`) -- ``a`` times fewer multiply-adds per edge, no per-edge coefficient gradients, and the readout's
+gradient a sum over nodes.  Edge-level fields, and anything :func:`_factored_inputs` does not recognise, take the pair terms.
 """
 
 from __future__ import annotations
@@ -206,6 +211,131 @@ class _FusedPairs(torch.autograd.Function):
         return (grad_hidden, grad_cw, grad_cb, grad_rw, grad_rb, None, None, None, *grad_vectors)
 
 
+# ----------------------------------------------------------------------------- node-level fields: the factored form
+
+#: nodes per partial sum of the readout's gradient
+NODE_CHUNK = 128
+
+
+class NodeProducts(torch.autograd.Function):
+    """``(x (N, D), complex / real readout) -> zc (N, k, wc, 2), zr (N, k, wr)``: every block's ``Z_t = M_t x~``."""
+
+    @staticmethod
+    def forward(ctx: Any, x: Tensor, cw: Tensor | None, cb: Tensor | None, rw: Tensor | None, rb: Tensor | None,  # type: ignore[override]
+                desc: Tensor, k: int, wc: int, wr: int) -> tuple[Tensor, Tensor]:
+        from gm_attention_b200 import _lib
+
+        x, cw, cb, rw, rb = (None if t is None else t.contiguous() for t in (x, cw, cb, rw, rb))
+        zc, zr = x.new_empty(x.shape[0], k, wc, 2), x.new_empty(x.shape[0], k, wr)
+        with torch.cuda.device(x.device):
+            _lib.call("gm_node_products_forward", *(_lib.ptr(t) for t in (x, cw, cb, rw, rb, desc)), x.shape[0], desc.shape[0], x.shape[1], k, wc, wr,
+                      _lib.dtype_code(x.dtype), _lib.ptr(zc), _lib.ptr(zr), _lib.stream(x.device))
+        ctx.save_for_backward(x, cw, cb, rw, rb, desc)
+        return zc, zr
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx: Any, dzc: Tensor, dzr: Tensor) -> tuple[Any, ...]:  # type: ignore[override]
+        from gm_attention_b200 import _lib
+
+        x, cw, cb, rw, rb, desc = ctx.saved_tensors
+        dzc, dzr = dzc.contiguous(), dzr.contiguous()
+        k, wc, wr = dzc.shape[1], dzc.shape[2], dzr.shape[2]
+        chunks = -(-x.shape[0] // NODE_CHUNK)
+        rows = [0 if w is None else w.shape[0] for w in (cw, rw)]
+        dx = torch.empty_like(x)
+        parts = [x.new_zeros(chunks, r, k) for r in rows]
+        with torch.cuda.device(x.device):
+            _lib.call("gm_node_products_backward", *(_lib.ptr(t) for t in (x, cw, cb, rw, rb, desc, dzc, dzr)), x.shape[0], desc.shape[0], x.shape[1],
+                      k, wc, wr, *rows, NODE_CHUNK, _lib.dtype_code(x.dtype), _lib.ptr(dx), _lib.ptr(parts[0]), _lib.ptr(parts[1]),
+                      _lib.stream(x.device))
+        grads: list[Tensor | None] = []
+        for part, w, b in ((parts[0], cw, cb), (parts[1], rw, rb)):
+            total = None if w is None else part.sum(0)
+            grads += [None if total is None else total[:, 1:], None if b is None else total[:, 0]]  # type: ignore[index]
+        return (dx, *grads, None, None, None, None)
+
+
+def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]]]:
+    """The factored plan of the kernel's terms and the descriptor rows of their node products (cached on the kernel)."""
+    cached = kernel.__dict__.get("_fused_node_blocks")
+    if cached is not None:
+        return cached  # type: ignore[no-any-return]
+    from gm_attention_b200.nn import fused_factored
+
+    p = fused_factored.plan_blocks([(t.n, t.m, t.role) for t in terms], kernel.field_type_out,
+                                   {(t.n, t.m, t.role): t.power for t in terms if t.power is not None})
+    offsets, at = {}, 0
+    for n in kernel.field_type_in.frequencies:
+        offsets[n] = at
+        at += kernel.field_type_in.multiplicity(n) * (1 if n == 0 else 2)
+    by_block = {(t.n, t.m, t.role): t for t in terms}
+    rows = []
+    for b in p.blocks:
+        t = by_block[b.block]
+        operand = 0 if t.flags & U_REAL else (2 if t.flags & CONJ_U else 1)
+        rows.append([b.kind, b.z_offset, t.b, t.a, offsets[t.n], operand, t.rows.start, 0])
+    kernel.__dict__["_fused_node_blocks"] = (p, rows)
+    return p, rows
+
+
+def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term]) -> tuple | None:
+    """What the factored form needs of this call, or ``None`` where the pair terms serve it: an edge-level or mixed field,
+    fewer than 4 edges per node (the node products would not be repaid), phase tables that are not plain per-edge
+    ``angular_phases`` / ``transport_phases`` of one width or that want gradients, sizes beyond the factored kernels."""
+    frequencies = list(kernel.field_type_in.frequencies)
+    values = [x[n] for n in frequencies]
+    nodes = {int(v.shape[0]) for v in values}
+    n_edges = int(edges.n_edges)
+    if hidden.device.type != "cuda" or hidden.dtype not in (torch.float32, torch.float64) or len(nodes) != 1 or not terms:
+        return None
+    n_nodes = nodes.pop()
+    if n_nodes == n_edges or n_nodes == 0 or n_edges < 4 * n_nodes:
+        return None
+    angular, transport = getattr(edges, "angular_phases", None), getattr(edges, "transport_phases", None)
+    if angular is None or transport is None or not hasattr(edges, "edge_index") or angular.shape != transport.shape:
+        return None
+    if angular.dtype != _complex_of(hidden.dtype) or transport.dtype != angular.dtype or angular.requires_grad or transport.requires_grad:
+        return None
+    if any(v.device != hidden.device or (v.real if v.is_complex() else v).dtype != hidden.dtype for v in (*values, angular, transport)):
+        return None
+    from gm_attention_b200.nn import fused_factored as ff
+
+    p, rows = _node_blocks(kernel, terms)
+    k = hidden.shape[1] + 1
+    if k > ff.MAX_K or p.d_out > ff.MAX_OUT or p.max_bm > ff.MAX_BM or k * (-(-(2 * p.wc + p.wr) // 4) * 4) > ff.MAX_KC:
+        return None
+    if max((max(abs(b.angular), abs(b.transport)) for b in p.blocks), default=0) >= angular.shape[1]:
+        return None
+    return p, rows, values, angular, transport, n_nodes
+
+
+def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tuple) -> Any:
+    from gm_attention_b200.nn import fused_factored as ff
+
+    p, rows, values, angular, transport, n_nodes = found
+    device, dtype = hidden.device, hidden.dtype
+    flat = [(torch.view_as_real(v) if v.is_complex() else v).reshape(n_nodes, -1) for v in values]
+    packed = flat[0] if len(flat) == 1 else torch.cat(flat, 1)
+    tables = kernel.__dict__.setdefault("_fused_node_descriptors", {})
+    if str(device) not in tables:
+        tables[str(device)] = (torch.tensor(rows, dtype=torch.int32, device=device).reshape(-1, 8),
+                               torch.tensor([b.row() for b in p.blocks], dtype=torch.int32, device=device).reshape(-1, 8))
+    node_desc, desc = tables[str(device)]
+    params = [q for head in (kernel.complex_head, kernel.real_head) for q in ((None, None) if head is None else (head.weight, head.bias))]
+    zc, zr = NodeProducts.apply(packed, *params, node_desc, hidden.shape[1] + 1, p.wc, p.wr)
+    powers = [b.power for b in p.blocks]
+    rho = kernel._radial_powers(edges.distances)[:, 1].detach().to(dtype).contiguous() if max(powers, default=0) else hidden.new_ones(hidden.shape[0])
+    source = edges.source_index.contiguous()
+    order, group_ptr, group_source = ff.groups_for(edges, source)
+    out = ff.Factored.apply(hidden, zc, zr, torch.view_as_real(angular.contiguous()), torch.view_as_real(transport.contiguous()), rho, desc, source,
+                            order, group_ptr, group_source, p.d_out, p.max_bm)
+    slices = kernel.field_type_out.slices()
+    orders = sorted(kernel.field_type_out.frequencies, key=lambda m: slices[m].start)
+    parts = dict(zip(orders, out.split([slices[m].stop - slices[m].start for m in orders], 1), strict=True))
+    return {m: parts[m].contiguous() if m == 0 else parts[m].contiguous().reshape(hidden.shape[0], -1, 2) for m in kernel.field_type_out.frequencies}
+
+
 # ----------------------------------------------------------------------------- driver entry
 
 def _trunk_output(kernel: Any, distances: Tensor) -> Tensor:
@@ -243,6 +373,10 @@ def forward_general(kernel: Any, x: Any, edges: Any) -> Any:
     terms = plan(kernel)
     with torch.profiler.record_function("gm::kernel/radial"):
         hidden = _trunk_output(kernel, edges.distances)
+    found = _factored_inputs(kernel, x, edges, hidden, terms)
+    if found is not None:
+        with torch.profiler.record_function("gm::kernel/pairs"):
+            return type(x)(kernel.field_type_out, _forward_factored(kernel, x, edges, hidden, found))
     in_frequencies, out_frequencies = list(kernel.field_type_in.frequencies), list(kernel.field_type_out.frequencies)
     with torch.profiler.record_function("gm::transport"):
         vectors = _transported_vectors(x, edges, in_frequencies)

@@ -274,6 +274,27 @@ int gm_pairs_backward(const void* hidden, const void* weight, const void* bias, 
                       int a, int b, int trunk, int flags, int dtype, void* stream);
 
 /* ------------------------------------------------------------------------
+ * Node-side products of a steerable kernel's readout with a node field, in the
+ * packing gm_factored_* read: Z_{t,b}(j) = sum_a M_t[b, a] x~_n(j)[a], M_0 the
+ * readout's bias, M_t its weight column t - 1 (t < k), x~ = x or conj(x).
+ *   x      (n_nodes, din) packed node field
+ *   cw, cb (crows, k - 1), (crows) complex readout: row r + 2 (b a_n + a) real, + 1 imaginary part; rw, rb real
+ *          readout: row r + b a_n + a; a bias may be NULL (zero)
+ *   desc   (n_blocks, 8) int32: complex block (else real), first Z column, b, a_n, offset in x, operand (0 real,
+ *          1 complex, 2 conjugate), first readout row, 0
+ *   zc, zr (n_nodes, k, wc, 2), (n_nodes, k, wr): every column a block names is written
+ *   dx (n_nodes, din) written; dcw (ceil(n_nodes / chunk), crows, k), drw (.., rrows, k): per-chunk sums of the
+ *   readout's gradient, the bias in column 0; rows no block names are left untouched
+ * dtype: GM_F32 or GM_F64.
+ * ------------------------------------------------------------------------ */
+int gm_node_products_forward(const void* x, const void* cw, const void* cb, const void* rw, const void* rb, const int32_t* desc,
+                             int64_t n_nodes, int n_blocks, int din, int k, int wc, int wr, int dtype, void* zc, void* zr, void* stream);
+
+int gm_node_products_backward(const void* x, const void* cw, const void* cb, const void* rw, const void* rb, const int32_t* desc,
+                              const void* dzc, const void* dzr, int64_t n_nodes, int n_blocks, int din, int k, int wc, int wr, int crows,
+                              int rrows, int chunk, int dtype, void* dx, void* dcw, void* drw, void* stream);
+
+/* ------------------------------------------------------------------------
  * Tensor-core variants of the lattice fast path for bf16 node fields (same
  * tables, same results within bf16 rounding of the attention weights): the
  * per-frequency Gram blocks and the (alpha o tau) V sums run as m16n8k16 bf16

@@ -313,3 +313,52 @@ def test_pairs_driver_matches_the_pair_loop(field_in, field_out, bias, dtype):
         assert float((y_fused[m] - y_plain[m]).abs().max()) <= tol_y * scale, m
     for a, b in zip(g_fused, g_plain):
         assert float((a - b).abs().max()) <= tol_g * max(1.0, float(b.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("field_in, field_out, trunk, bias", [
+    ({0: 3, 1: 5}, {0: 3, 1: 2, 2: 1}, 5, True),       # odd scalar block before complex ones, a trunk that is no multiple of 4
+    ({0: 8, 1: 8, 2: 8}, {0: 4, 1: 4, 2: 4}, 16, True),
+    ({0: 16, 1: 16}, {0: 8, 1: 8}, 16, False),
+    ({1: 2}, {0: 2}, 1, True),                          # complex readout only
+    ({0: 3}, {0: 2}, 16, True),                         # real readout only
+])
+def test_node_level_field_equals_the_pair_terms(monkeypatch, field_in, field_out, trunk, bias, dtype):
+    """The factored form of ``forward_general`` against the pair terms on the same call: outputs (contiguous, as before) and
+    every gradient; a node field that is a strided view takes it too, the same field gathered onto the edges takes the pair
+    terms.  float64 1e-11; float32 4e-6 of each tensor's magnitude (sums over ~2 000 edges in another order)."""
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=dtype)
+    kernel = StandInKernel(field_in, field_out, cutoff, trunk=trunk, bias=bias, dtype=dtype).to(dev)
+    generator = torch.Generator().manual_seed(7)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, generator=generator, dtype=dtype).to(dev).requires_grad_(True)
+    taken = []
+    recognise = fp._factored_inputs
+    monkeypatch.setattr(fp, "_factored_inputs", lambda *a: taken.append(recognise(*a)) or taken[-1])
+
+    def run(values):
+        out = fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, values), edges).coefficients
+        assert all(v.is_contiguous() for v in out.values())
+        g = torch.Generator().manual_seed(8)
+        loss = sum((v * torch.randn(*v.shape, generator=g, dtype=dtype).to(dev)).sum() for v in out.values())
+        return [*(v.detach() for v in out.values()), *torch.autograd.grad(loss, [flat, *kernel.parameters()])]
+
+    node = run(flat)
+    assert taken[-1] is not None
+    strided = run(torch.cat([flat, flat], 1)[:, :flat.shape[1]])
+    assert taken[-1] is not None
+    edge = run(flat.index_select(0, edges.source_index))
+    assert taken[-1] is None
+    monkeypatch.setattr(fp, "_factored_inputs", lambda *a: None)
+    terms = run(flat)
+    bound = 1e-11 if dtype == torch.float64 else 4e-6
+    for got in (node, strided, edge):
+        for a, b in zip(got, terms):
+            assert a.shape == b.shape and rel_err(a.cpu().numpy(), b.cpu().numpy()) < bound
