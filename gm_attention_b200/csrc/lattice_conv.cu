@@ -465,6 +465,54 @@ __global__ void __launch_bounds__(THREADS, 3) conv_table_grad_kernel(const ConvA
   }
 }
 
+// ----------------------------------------------------------------------------------------------------------------- fold
+// An entry's coefficients -> its row of the table, and back (gm_attention_b200/nn/lattice_depthwise.py: fold writes the same in
+// tensor algebra, about 35 launches forward and 50 backward over the entries' complex temporaries): scalar factors times
+// the weight w; per complex copy a = w tau A, b = w omega conj(tau) B and the real 2 x 2 matrix of z -> a z + b conj(z).
+// One CTA per entry, a thread per column: bound by reading the coefficients and writing the table once each (45 x 88, batch
+// 3, 32 x (m <= 2): 4.7 us each way; the pass 1.87 -> 0.72 ms, 134 -> 35 launches, of which the host was the bound).
+struct FoldArgs {
+  const float *rc, *cc, *weights;
+  const float2 *tau, *omega;  // (entries, nf)
+  const int* items;           // (n_complex, 3): coefficient column of A, of B, frequency index
+  const float* dtable;
+  float *table, *drc, *dcc;
+  int a0, padded, width, n_complex, nf, table_width;
+};
+
+__device__ __forceinline__ float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+
+template <bool BACKWARD>
+__global__ void __launch_bounds__(128) conv_fold_kernel(const FoldArgs a) {
+  const size_t e = blockIdx.x;
+  const float w = a.weights[e];
+  for (int x = threadIdx.x; x < a.padded + a.n_complex; x += 128) {
+    if (x < a.padded) {
+      if constexpr (BACKWARD) {
+        if (x < a.a0 && a.drc) a.drc[e * a.a0 + x] = w * a.dtable[e * a.table_width + x];
+      } else {
+        a.table[e * a.table_width + x] = x < a.a0 ? w * a.rc[e * a.a0 + x] : 0.f;
+      }
+      continue;
+    }
+    const int c = x - a.padded, at_a = a.items[3 * c], at_b = a.items[3 * c + 1], f = a.items[3 * c + 2];
+    const float2 tau = a.tau[e * a.nf + f], omega = a.omega[e * a.nf + f];
+    const float2 fa = make_float2(w * tau.x, w * tau.y);
+    const float2 ot = cmul(omega, make_float2(tau.x, -tau.y)), fb = make_float2(w * ot.x, w * ot.y);
+    const size_t ca = e * a.width + at_a, cb = e * a.width + at_b, out = e * a.table_width + a.padded + 4 * c;
+    if constexpr (BACKWARD) {
+      const float4 d = *reinterpret_cast<const float4*>(a.dtable + out);
+      const float2 da = cmul(make_float2(fa.x, -fa.y), make_float2(d.x + d.w, d.z - d.y));
+      const float2 db = cmul(make_float2(fb.x, -fb.y), make_float2(d.x - d.w, d.y + d.z));
+      a.dcc[ca] = da.x; a.dcc[ca + 1] = da.y;
+      a.dcc[cb] = db.x; a.dcc[cb + 1] = db.y;
+    } else {
+      const float2 va = cmul(fa, make_float2(a.cc[ca], a.cc[ca + 1])), vb = cmul(fb, make_float2(a.cc[cb], a.cc[cb + 1]));
+      *reinterpret_cast<float4*>(a.table + out) = make_float4(va.x + vb.x, vb.y - va.y, va.y + vb.y, va.x - vb.x);
+    }
+  }
+}
+
 // Tiles, offsets per stage and samples per thread of the staged apply kernel; returns the samples, 0 where it cannot run.
 // Two samples and two CTAs of 320 threads per SM (102 registers) measured 4.5 ms against 4.7 for four samples and one CTA,
 // 5.8 to 6.0 for CTAs of one tile (256 x 512, batch 4, 64 x (m <= 2), bf16).  A stage should hold the equator's windows
@@ -587,4 +635,25 @@ extern "C" int gm_lattice_conv_table_grad(const void* g, const void* x, const in
   }
 #undef GM_GRAD
   return launch_status("gm_lattice_conv_table_grad");
+}
+
+// The table of per-entry coefficients (dtable null: forward, writes table) or the coefficients' gradients from the table's
+// (writes drc, dcc).  rc (entries, a0), cc (entries, width), weights (entries), tau / omega (entries, nf, 2), items
+// (n_complex, 3) as conv_fold_kernel reads them; table_width = a0 rounded up to 4, plus 4 per complex copy.
+extern "C" int gm_lattice_conv_fold(const float* rc, const float* cc, const float* weights, const float* tau, const float* omega,
+                                    const int32_t* items, const float* dtable, int64_t entries, int a0, int width, int n_complex, int nf,
+                                    float* table, float* drc, float* dcc, void* stream) {
+  if (entries == 0) return GM_OK;
+  const int padded = (a0 + 3) / 4 * 4;
+  GM_REQUIRE(entries > 0 && entries < (int64_t)1 << 31 && a0 >= 0 && width >= 0 && n_complex >= 0 && nf >= 0, GM_ERR_ARGUMENT, "gm_lattice_conv_fold: bad sizes");
+  GM_REQUIRE(weights && (n_complex == 0 || (tau && omega && items)), GM_ERR_ARGUMENT, "gm_lattice_conv_fold: null pointer");
+  GM_REQUIRE(dtable ? (a0 == 0 || drc) && (n_complex == 0 || dcc) : table && (a0 == 0 || rc) && (n_complex == 0 || cc), GM_ERR_ARGUMENT,
+             "gm_lattice_conv_fold: null pointer");
+  GM_REQUIRE(reinterpret_cast<uintptr_t>(table) % 16 == 0 && reinterpret_cast<uintptr_t>(dtable) % 16 == 0 && reinterpret_cast<uintptr_t>(tau) % 8 == 0 &&
+                 reinterpret_cast<uintptr_t>(omega) % 8 == 0, GM_ERR_ARGUMENT, "gm_lattice_conv_fold: misaligned table or phases");
+  FoldArgs a{rc, cc, weights, reinterpret_cast<const float2*>(tau), reinterpret_cast<const float2*>(omega), items, dtable, table, drc, dcc,
+             a0, padded, width, n_complex, nf, padded + 4 * n_complex};
+  if (dtable) conv_fold_kernel<true><<<(unsigned)entries, 128, 0, (cudaStream_t)stream>>>(a);
+  else conv_fold_kernel<false><<<(unsigned)entries, 128, 0, (cudaStream_t)stream>>>(a);
+  return launch_status("gm_lattice_conv_fold");
 }

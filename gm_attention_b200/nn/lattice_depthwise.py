@@ -48,6 +48,7 @@ class ConvTables:
     weights: Tensor  # (entries,) aggregation weight of the entry's edges
     tau: Tensor  # (entries, complex frequencies) complex64: transport phase of order n
     omega: Tensor  # (entries, complex frequencies) complex64: (r / cutoff)^{2n} e^{2 i n phi}
+    fold_items: Tensor | None = None  # (complex copies, 3) int32: columns of A and B among the coefficients, frequency index
 
     @property
     def n_entries(self) -> int:
@@ -74,6 +75,7 @@ def conv_tables(geometry: Any, distances: Tensor, weights: Tensor, rows: Sequenc
         for c in range(copies):
             items.append((0, flat + 2 * c, column))
             column += 4
+    fold_items = [(offset + 2 * c, offset + 2 * (copies + c), index) for index, (_, copies, _, offset, _) in enumerate(complex_rows) for c in range(copies)]
     device = edge.device
     cnt = lat.win_cnt.cpu().numpy().reshape(-1)
     blocks = [(w, d) for w in np.flatnonzero(cnt > 0) for d in range(0, int(cnt[w]), OFFSETS_PER_BLOCK)]
@@ -90,7 +92,8 @@ def conv_tables(geometry: Any, distances: Tensor, weights: Tensor, rows: Sequenc
     return ConvTables(lat, rows, a_0, sum(4 * r[1] for r in complex_rows), column,
                       torch.tensor(items, dtype=torch.int32, device=device).reshape(-1, 3),
                       torch.tensor(blocks, dtype=torch.int32, device=device).reshape(-1, 2),
-                      distances.index_select(0, edge).float(), weights.index_select(0, edge).float(), stack(tau), stack(omega))
+                      distances.index_select(0, edge).float(), weights.index_select(0, edge).float(), stack(tau), stack(omega),
+                      torch.tensor(fold_items, dtype=torch.int32, device=device).reshape(-1, 3))
 
 
 def fold(real_coefficients: Tensor | None, complex_coefficients: Tensor | None, t: ConvTables) -> Tensor:
@@ -117,6 +120,51 @@ def fold(real_coefficients: Tensor | None, complex_coefficients: Tensor | None, 
         parts.append(torch.stack([a.real + b.real, b.imag - a.imag, a.imag + b.imag, a.real - b.real], -1).reshape(-1, 4 * copies))
         index += 1
     return torch.cat(parts, 1).contiguous()
+
+
+class FoldTable(torch.autograd.Function):
+    """:func:`fold` as one launch each way, differentiable in the coefficients."""
+
+    @staticmethod
+    def forward(ctx: Any, rc: Tensor | None, cc: Tensor | None, t: ConvTables) -> Tensor:
+        rc, cc = (None if c is None else c.contiguous() for c in (rc, cc))
+        ctx.tables, ctx.shapes = t, (None if rc is None else rc.shape, None if cc is None else cc.shape)
+        table = torch.empty((t.n_entries, t.table_width), dtype=torch.float32, device=t.weights.device)
+        _fold_call(t, rc, cc, None, table, None, None)
+        return table
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx: Any, grad: Tensor) -> tuple:  # type: ignore[override]
+        grad = grad.contiguous()
+        drc, dcc = (None if s is None else grad.new_empty(s) for s in ctx.shapes)
+        _fold_call(ctx.tables, None, None, grad, None, drc, dcc)
+        return drc, dcc, None
+
+
+def _fold_call(t: ConvTables, rc: Tensor | None, cc: Tensor | None, dtable: Tensor | None, table: Tensor | None, drc: Tensor | None,
+               dcc: Tensor | None) -> None:
+    device = t.weights.device
+    with torch.cuda.device(device):
+        _lib.call("gm_lattice_conv_fold", _lib.ptr(rc), _lib.ptr(cc), _lib.ptr(t.weights), _lib.ptr(t.tau), _lib.ptr(t.omega), _lib.ptr(t.fold_items),
+                  _lib.ptr(dtable), t.n_entries, t.a_0, t.complex_width, t.fold_items.shape[0], t.tau.shape[1], _lib.ptr(table), _lib.ptr(drc),
+                  _lib.ptr(dcc), _lib.stream(device))
+
+
+def _fold(rc: Tensor | None, cc: Tensor | None, t: ConvTables) -> Tensor:
+    """The table through :class:`FoldTable` where its layout is what the kernel reads (float32 phases and weights that want
+    no gradient, coefficients of exactly the layer's widths on the same GPU), through :func:`fold` otherwise."""
+    n = t.n_entries
+    constants = (t.weights, t.tau, t.omega)
+    fits = (t.fold_items is not None and t.weights.is_cuda and n > 0 and not any(c.requires_grad for c in constants)
+            and all(c.is_contiguous() and not c.is_conj() for c in constants) and t.weights.dtype == torch.float32
+            and t.tau.dtype == t.omega.dtype == torch.complex64 and 4 * t.fold_items.shape[0] == t.complex_width
+            and t.table_width == -(-t.a_0 // 4) * 4 + t.complex_width
+            and (t.a_0 == 0 or (rc is not None and rc.shape == (n, t.a_0) and rc.device == t.weights.device))
+            and (t.complex_width == 0 or (cc is not None and cc.shape == (n, t.complex_width) and cc.device == t.weights.device)))
+    if not fits or any(c is not None and c.is_complex() for c in (rc, cc)):
+        return fold(rc, cc, t)
+    return FoldTable.apply(rc.float() if t.a_0 else None, cc.float() if t.complex_width else None, t)  # type: ignore[no-any-return,union-attr]
 
 
 def _apply(x: Tensor, table: Tensor, t: ConvTables, transposed: bool) -> Tensor:
@@ -173,7 +221,7 @@ class LatticeDepthwise(torch.autograd.Function):
 
 def lattice_depthwise(v: Tensor, real_coefficients: Tensor | None, complex_coefficients: Tensor | None, tables: ConvTables) -> Tensor:
     """The depthwise convolution of the flat field ``v (batch * nodes, D)`` under per-ENTRY coefficients."""
-    return LatticeDepthwise.apply(v.contiguous(), fold(real_coefficients, complex_coefficients, tables), tables)  # type: ignore[no-any-return]
+    return LatticeDepthwise.apply(v.contiguous(), _fold(real_coefficients, complex_coefficients, tables), tables)  # type: ignore[no-any-return]
 
 
 class RadialCoefficients(nn.Module):

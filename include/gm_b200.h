@@ -458,6 +458,13 @@ int gm_lattice_conv_apply(const void* x, const float* table, const int32_t* item
 int gm_lattice_conv_table_grad(const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt,
                                const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows,
                                int nlon, int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream);
+/* gm_lattice_conv_fold: an entry's coefficients rc (entries, a0), cc (entries, width), weight and phases tau, omega
+ * (entries, nf, 2) -> its table row: w rc, zeros up to a multiple of 4, then per complex copy the matrix [[a, b], [c, d]]
+ * of z -> w (A tau z + omega B conj(tau z)); items (n_complex, 3) int32: columns of A and B in cc, frequency index.  With
+ * dtable != NULL the gradients instead: drc, dcc from dtable (table is not read; table_width = padded a0 + 4 n_complex). */
+int gm_lattice_conv_fold(const float* rc, const float* cc, const float* weights, const float* tau, const float* omega, const int32_t* items,
+                         const float* dtable, int64_t entries, int a0, int width, int n_complex, int nf, float* table, float* drc, float* dcc,
+                         void* stream);
 
 /* ---------------------------------------------------------------------------
  * Halo exchange through peer memory (machines whose GPUs can map each other's

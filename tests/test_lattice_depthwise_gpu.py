@@ -161,6 +161,28 @@ def test_apply_against_the_host_loops(nlat, nlon, reach, head, batch, storage):
         assert_close(got, want, 2.0 ** -8 if storage == "bf16" else 1e-5, atol, "transposed" if transposed else "forward")
 
 
+@pytest.mark.parametrize("head", [{0: 2, 1: 1}, {0: 6, 1: 5, 2: 7}, {1: 3}, {0: 130, 1: 130}, {0: 4}])
+def test_fold_kernel_equals_the_tensor_algebra(head):
+    """One launch each way against :func:`fold` and its autograd gradients: a handful of float32 products per value, 2e-6 of
+    the largest; float64 coefficients are rounded first, as :func:`fold` does."""
+    from types import SimpleNamespace
+
+    from gm_attention_b200.nn.lattice_depthwise import _fold, conv_tables, fold
+
+    c = make_case(6, 16, 1.7 * math.pi / 6, head, 1, dtype=np.float32)
+    geometry = SimpleNamespace(transport=cuda(c.transport), angular=cuda(c.angular), rho=cuda(c.rho), bias=cuda(c.bias), inside=cuda(c.inside),
+                               row_ptr=cuda(c.row_ptr), source=cuda(c.source))
+    t = conv_tables(geometry, cuda(c.rho * np.float32(c.radius)), cuda(c.weights), descriptor_rows(c.head_type, 1), 6, 16)
+    for dtype in (np.float32, np.float64):
+        coefficients = [cuda(seeded((t.n_entries, w), 63 + w, dtype)[0]).requires_grad_(True) if w else None for w in (t.a_0, t.complex_width)]
+        leaves = [x for x in coefficients if x is not None]
+        got, want = _fold(*coefficients, t), fold(*coefficients, t)
+        assert "FoldTable" in type(got.grad_fn).__name__ and got.shape == want.shape and got.is_contiguous()
+        g = cuda(seeded(tuple(got.shape), 64, np.float32)[0])
+        for name, a, b in zip(("table", "first", "second"), (got, *torch.autograd.grad(got, leaves, g)), (want, *torch.autograd.grad(want, leaves, g))):
+            assert a.dtype == b.dtype and rel_err(a.detach().cpu().numpy(), b.detach().cpu().numpy()) < 2e-6, name
+
+
 NLAT, NLON, BATCH, COPIES = 256, 512, 4, 64
 HEAD = {0: COPIES, 1: COPIES, 2: COPIES}
 RADIUS = 4 * math.pi / NLAT
