@@ -466,6 +466,10 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? (MODE == TC_BWD_S ? 3
   }
   if (!a.use_tma)  // per-thread staging leaves rows beyond a window and padding columns untouched: they must be finite
     for (int x = threadIdx.x; x < 2 * buf_bytes / 16; x += THREADS) reinterpret_cast<uint4*>(smem_raw)[x] = make_uint4(0, 0, 0, 0);
+  // a step of 16 rows may end beyond the window: the weights there are zero, and zero times whatever an earlier kernel left
+  // in the statistics' slots need not be
+  if constexpr (PASS_S)
+    for (int x = threadIdx.x; x < 4 * TN_ROWS; x += THREADS) stats(x & 1)[x >> 1] = 0.f;
   if (threadIdx.x == 0) {
     failed_s = 0;
     mbar_init(&copy_bar[0], 1);
@@ -632,14 +636,12 @@ __global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? (MODE == TC_BWD_S ? 3
     }
     if constexpr (PASS_S) {
       float* ds = stats(buf);
-      // every row a step can read, zeros beyond the window: its weights are zero there, and zero times whatever an earlier
-      // kernel left in shared memory need not be
-      for (int idx = threadIdx.x; idx < 2 * TN_ROWS; idx += THREADS) {
+      for (int idx = threadIdx.x; idx < 2 * n_rows; idx += THREADS) {
         const int pl = idx >> 1, which = idx & 1;
         int lon = lon0 + pl;
         if (lon >= a.nlon) lon %= a.nlon;
         const int64_t nn = ((int64_t)z * a.nlon + lon) * a.H + h;
-        cp_async4(ds + 2 * pl + which, (which ? a.delta : a.lse) + nn, pl < n_rows ? 4 : 0);
+        cp_async4(ds + 2 * pl + which, (which ? a.delta : a.lse) + nn, 4);
       }
     }
     cp_async_commit();
