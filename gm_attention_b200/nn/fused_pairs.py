@@ -274,9 +274,19 @@ def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]]]:
     for b in p.blocks:
         t = by_block[b.block]
         operand = 0 if t.flags & U_REAL else (2 if t.flags & CONJ_U else 1)
-        rows.append([b.kind, b.z_offset, t.b, t.a, offsets[t.n], operand, t.rows.start, 0])
+        rows.append([b.kind, b.z_offset, t.b, t.a, offsets[t.n], operand, t.rows.start or 0, 0])
     kernel.__dict__["_fused_node_blocks"] = (p, rows)
     return p, rows
+
+
+def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
+    """Whether an earlier call left the kernel's descriptors on the device and grouped these edges by source."""
+    from gm_attention_b200.nn import fused_attention
+    from gm_attention_b200.nn import fused_factored as ff
+
+    registered = fused_attention.chunk_of(edges)
+    parent, first, last = registered if registered is not None else (edges, 0, int(edges.n_edges))
+    return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.group_key(parent, first, last) in ff._GROUPS
 
 
 def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term]) -> tuple | None:
@@ -307,6 +317,8 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
         return None
     if max((max(abs(b.angular), abs(b.transport)) for b in p.blocks), default=0) >= angular.shape[1]:
         return None
+    if torch.cuda.is_current_stream_capturing() and not _prepared(kernel, edges, hidden.device):
+        return None  # grouping the edges by source and uploading the descriptors synchronise: not while a graph is captured
     return p, rows, values, angular, transport, n_nodes
 
 

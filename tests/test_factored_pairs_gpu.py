@@ -362,3 +362,40 @@ def test_node_level_field_equals_the_pair_terms(monkeypatch, field_in, field_out
     for got in (node, strided, edge):
         for a, b in zip(got, terms):
             assert a.shape == b.shape and rel_err(a.cpu().numpy(), b.cpu().numpy()) < bound
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_pair_driver_under_capture(monkeypatch, warm):
+    """A graph captures ``forward_general`` on an edge set it has never seen (pair terms: grouping the edges would
+    synchronise) and on one an eager call has grouped (factored form); replayed, both give the eager result."""
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(8, 18, dev)
+    cutoff = 1.9 * math.pi / 8
+    make = lambda: compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32)
+    seen, fresh = make(), make()
+    kernel = StandInKernel({0: 3, 1: 2}, {0: 2, 1: 2}, cutoff, trunk=8, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    taken = []
+    recognise = fp._factored_inputs
+    monkeypatch.setattr(fp, "_factored_inputs", lambda *a: taken.append(recognise(*a)) or taken[-1])
+    run = lambda edges: fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, flat), edges).coefficients
+    with torch.no_grad():
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            want = run(seen)
+            run(seen)
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = run(seen if warm else fresh)
+        assert (taken[-1] is not None) == warm
+        graph.replay()
+        torch.cuda.synchronize()
+    for m in want:
+        assert rel_err(out[m].cpu().numpy(), want[m].cpu().numpy()) < 4e-6
