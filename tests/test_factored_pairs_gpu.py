@@ -194,6 +194,40 @@ def test_factored_against_plain_sums(type_in, type_out, k, degrees, dtype):
         assert rel_err(a.cpu().numpy(), b.numpy()) < tolerance, name
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_factored_sources_without_edges(dtype):
+    """A grouping that lists every node, most of them with an empty run between two full ones (more runs than the forward
+    has CTAs, so that a CTA meets both), gives the rows and gradients of the grouping without them, bit for bit: an empty
+    run leaves no copy behind that the next source's could race with, and its node's gradient is zero."""
+    from gm_attention_b200.fields import FieldType
+    from gm_attention_b200.nn import fused_factored as ff
+
+    blocks, powers = blocks_for({0: 2, 1: 2}, {0: 2, 1: 3})
+    p = ff.plan_blocks(blocks, FieldType({0: 2, 1: 3}), powers)
+    n, k, n_f = 9000, 6, 4
+    degrees = np.where(np.arange(n) % 3 == 1, 1 + np.arange(n) % 5, 0)
+    rng = np.random.default_rng(9)
+    source = rng.permutation(np.repeat(np.arange(n), degrees))
+    e = source.shape[0]
+    draw = lambda *shape: cuda(rng.standard_normal(shape).astype(dtype))
+    h, zc, zr, angular, transport, rho = draw(e, k - 1), draw(n, k, p.wc, 2), draw(n, k, p.wr), draw(e, n_f, 2), draw(e, n_f, 2), draw(e)
+    desc, src = cuda(np.array([b.row() for b in p.blocks], np.int32)), cuda(source)
+    args = (h, zc, zr, angular, transport, rho, desc, src)
+    order, group_ptr, group_source = ff.source_groups(src)
+    every_ptr = torch.zeros(n + 1, dtype=torch.long, device=src.device)
+    every_ptr[1:] = torch.cumsum(torch.bincount(src, minlength=n), 0)
+    every = (order, every_ptr, torch.arange(n, device=src.device))
+    assert group_source.shape[0] < n
+    ext, g = ff.extension(True), draw(e, p.d_out)
+    rows = ext.forward(*args, order, group_ptr, group_source, p.d_out, p.max_bm)
+    grads = ext.backward(g, *args, order, group_ptr, group_source)
+    assert torch.equal(ext.forward(*args, *every, p.d_out, p.max_bm), rows)
+    for got, want in zip(ext.backward(g, *args, *every), grads):
+        assert torch.equal(got, want)
+    empty = torch.from_numpy(degrees == 0).to(src.device)
+    assert bool((grads[1][empty] == 0).all()) and bool((grads[2][empty] == 0).all())
+
+
 PAIR_CASES = [
     (3, 2, 5, 2 | 8),          # real block: U_REAL | OUT_REAL
     (4, 8, 16, 1 | 2),         # 0 -> m: MATRIX_COMPLEX | U_REAL
