@@ -139,29 +139,50 @@ def _pack(p: Plan, products: dict) -> tuple[Tensor, Tensor]:
     return zc, zr
 
 
-_GROUPS: OrderedDict[tuple, tuple[Any, tuple[Tensor, Tensor, Tensor]]] = OrderedDict()
+@dataclass(frozen=True)
+class Grouping:
+    """An edge set's edges grouped by source, and the range of its sources."""
+
+    groups: tuple[Tensor, Tensor, Tensor]  # order, group_ptr, group_source
+    lowest: int
+    highest: int
+
+    def require_nodes(self, n_nodes: int) -> tuple[Tensor, Tensor, Tensor]:
+        """The groups, for kernels that index ``n_nodes`` rows by source: refused where a source has no row."""
+        if self.lowest < 0 or self.highest >= n_nodes:
+            raise RuntimeError(f"gm_factored: the edges' sources are {self.lowest} .. {self.highest}, the node field has {n_nodes} rows")
+        return self.groups
+
+
+_GROUPS: OrderedDict[tuple, tuple[Any, Grouping]] = OrderedDict()
 GROUP_CACHE_SIZE = 512
+
+
+def grouping(source_index: Tensor, key: tuple | None = None, owner: Tensor | None = None) -> Grouping:
+    """:func:`source_groups` with the sources' range, read once where the groups are built."""
+    if key is not None and key in _GROUPS:
+        held, found = _GROUPS[key]
+        alive = owner is None if held is None else (held() is not None and held() is owner)
+        if alive and found.groups[0].device == source_index.device:
+            _GROUPS.move_to_end(key)
+            return found
+    order = torch.argsort(source_index, stable=True)
+    group_source, counts = torch.unique_consecutive(source_index[order], return_counts=True)
+    group_ptr = torch.zeros(group_source.shape[0] + 1, dtype=torch.long, device=source_index.device)
+    group_ptr[1:] = torch.cumsum(counts, 0)
+    lowest, highest = torch.stack((group_source[0], group_source[-1])).tolist() if group_source.shape[0] else (0, -1)
+    built = Grouping((order.contiguous(), group_ptr.contiguous(), group_source.contiguous()), lowest, highest)
+    if key is not None:
+        _GROUPS[key] = (None if owner is None else weakref.ref(owner), built)
+        while len(_GROUPS) > GROUP_CACHE_SIZE:
+            _GROUPS.popitem(last=False)
+    return built
 
 
 def source_groups(source_index: Tensor, key: tuple | None = None, owner: Tensor | None = None) -> tuple[Tensor, Tensor, Tensor]:
     """``(order, group_ptr, group_source)``: the edges stably sorted by source, each source's
     half-open run in that order, and the sources; cached under ``key`` (tied to ``owner`` while it lives)."""
-    if key is not None and key in _GROUPS:
-        held, groups = _GROUPS[key]
-        alive = owner is None if held is None else (held() is not None and held() is owner)
-        if alive and groups[0].device == source_index.device:
-            _GROUPS.move_to_end(key)
-            return groups
-    order = torch.argsort(source_index, stable=True)
-    group_source, counts = torch.unique_consecutive(source_index[order], return_counts=True)
-    group_ptr = torch.zeros(group_source.shape[0] + 1, dtype=torch.long, device=source_index.device)
-    group_ptr[1:] = torch.cumsum(counts, 0)
-    groups = (order.contiguous(), group_ptr.contiguous(), group_source.contiguous())
-    if key is not None:
-        _GROUPS[key] = (None if owner is None else weakref.ref(owner), groups)
-        while len(_GROUPS) > GROUP_CACHE_SIZE:
-            _GROUPS.popitem(last=False)
-    return groups
+    return grouping(source_index, key, owner).groups
 
 
 def group_key(parent: Any, first: int, last: int) -> tuple:
@@ -256,12 +277,16 @@ def inputs(kernel: Any, x: Any, edges: Any, products: dict | None) -> Inputs:
     return Inputs(h.contiguous(), zc, zr, angular, transport, rho, descriptors(kernel, h.device), edges.source_index.contiguous(), p)
 
 
-def groups_for(edges: Any, source: Tensor) -> tuple[Tensor, Tensor, Tensor]:
+def grouping_for(edges: Any, source: Tensor) -> Grouping:
     from gm_attention_b200.nn import fused_attention
 
     registered = fused_attention.chunk_of(edges)
     parent, first, last = registered if registered is not None else (edges, 0, int(edges.n_edges))
-    return source_groups(source, group_key(parent, first, last), owner=parent.edge_index)
+    return grouping(source, group_key(parent, first, last), owner=parent.edge_index)
+
+
+def groups_for(edges: Any, source: Tensor) -> tuple[Tensor, Tensor, Tensor]:
+    return grouping_for(edges, source).groups
 
 
 def _wrap_output(kernel: Any, flat: Tensor) -> Any:
@@ -271,7 +296,7 @@ def _wrap_output(kernel: Any, flat: Tensor) -> Any:
 
 def forward(kernel: Any, x: Any, edges: Any, products: dict | None = None, groups: tuple[Tensor, Tensor, Tensor] | None = None) -> Any:
     i = inputs(kernel, x, edges, products)
-    order, group_ptr, group_source = groups_for(edges, i.source) if groups is None else groups
+    order, group_ptr, group_source = grouping_for(edges, i.source).require_nodes(i.zc.shape[0]) if groups is None else groups
     flat = Factored.apply(i.h, i.zc, i.zr, i.angular, i.transport, i.rho, i.desc, i.source, order, group_ptr, group_source, i.plan.d_out,
                           i.plan.max_bm)
     return _wrap_output(kernel, flat)
@@ -280,7 +305,7 @@ def forward(kernel: Any, x: Any, edges: Any, products: dict | None = None, group
 def forward_aggregated(kernel: Any, x: Any, edges: Any, weights: Tensor, products: dict | None = None,
                        groups: tuple[Tensor, Tensor, Tensor] | None = None) -> Any:
     i = inputs(kernel, x, edges, products)
-    order, group_ptr, group_source = groups_for(edges, i.source) if groups is None else groups
+    order, group_ptr, group_source = grouping_for(edges, i.source).require_nodes(i.zc.shape[0]) if groups is None else groups
     flat = FactoredAggregate.apply(i.h, i.zc, i.zr, weights.to(i.h.dtype).contiguous(), i.angular, i.transport, i.rho, i.desc, i.source,
                                    edges.target_index.contiguous(), edges.row_ptr.contiguous(), order, group_ptr, group_source,
                                    i.plan.d_out, i.plan.max_bm)

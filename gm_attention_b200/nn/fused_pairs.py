@@ -339,7 +339,7 @@ def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tu
     powers = [b.power for b in p.blocks]
     rho = kernel._radial_powers(edges.distances)[:, 1].detach().to(dtype).contiguous() if max(powers, default=0) else hidden.new_ones(hidden.shape[0])
     source = edges.source_index.contiguous()
-    order, group_ptr, group_source = ff.groups_for(edges, source)
+    order, group_ptr, group_source = ff.grouping_for(edges, source).require_nodes(n_nodes)
     out = ff.Factored.apply(hidden, zc, zr, torch.view_as_real(angular.contiguous()), torch.view_as_real(transport.contiguous()), rho, desc, source,
                             order, group_ptr, group_source, p.d_out, p.max_bm)
     slices = kernel.field_type_out.slices()

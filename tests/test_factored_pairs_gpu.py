@@ -433,3 +433,37 @@ def test_pair_driver_under_capture(monkeypatch, warm):
         torch.cuda.synchronize()
     for m in want:
         assert rel_err(out[m].cpu().numpy(), want[m].cpu().numpy()) < 4e-6
+
+
+def test_node_field_with_too_few_rows_is_refused():
+    """A field shorter than the edges' largest source + 1 is an error on the host, from the pair driver and from the
+    factored drivers; one row per source is enough, and rows beyond the sources are read by nobody."""
+    from types import SimpleNamespace
+
+    from gm_attention_b200.fields import FeatureField, FieldType
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_factored as ff
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32)
+    kernel = StandInKernel({0: 2, 1: 2}, {0: 2, 1: 2}, cutoff, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes + 5, kernel.field_type_in.dimension, device=dev)
+    general = lambda n: fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, flat[:n]), edges).coefficients
+    want = general(lattice.n_nodes)
+    for m, values in general(lattice.n_nodes + 5).items():
+        assert torch.equal(values, want[m])
+    with pytest.raises(RuntimeError, match="the node field has"):
+        general(lattice.n_nodes - 1)
+    blocks, powers = blocks_for({0: 2, 1: 2}, {0: 2, 1: 2})
+    factored = SimpleNamespace(field_type_out=FieldType({0: 2, 1: 2}), _pair_powers=powers, _blocks=lambda: blocks, radial_basis=SimpleNamespace(cutoff=cutoff),
+                               _trunk_hidden=lambda e: torch.ones(e.n_edges, 3, device=dev))
+    products = lambda n: {b: torch.ones(n, 4, 2, device=dev, dtype=torch.float32 if b[2] == "real" else torch.complex64) for b in blocks}
+    weights = torch.ones(edges.n_edges, device=dev)
+    for call in (lambda n: ff.forward(factored, None, edges, products(n)), lambda n: ff.forward_aggregated(factored, None, edges, weights, products(n))):
+        assert call(lattice.n_nodes).isfinite().all()
+        with pytest.raises(RuntimeError, match="the node field has"):
+            call(lattice.n_nodes - 1)

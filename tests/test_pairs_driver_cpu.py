@@ -89,3 +89,19 @@ def test_plan_order_and_node_level_fields(reference_modules, monkeypatch):
     monkeypatch.setattr(fp, "GRADIENT_BLOCK_ROWS", 7)
     gk, op = torch.randn(6, 40, dtype=torch.float64), torch.randn(40, 5, dtype=torch.float64)
     torch.testing.assert_close(fp._coefficient_product(gk, op), gk @ op, atol=1e-12, rtol=0)
+
+
+def test_sources_beyond_the_node_field_are_refused():
+    """The grouping knows the range of its sources; what reads a node field through it refuses one with too few rows."""
+    from gm_attention_b200.nn import fused_factored as ff
+
+    edges, _ = cpu_edges()
+    found = ff.grouping_for(edges, edges.source_index)
+    assert (found.lowest, found.highest) == (int(edges.source_index.min()), int(edges.source_index.max()))
+    assert found.require_nodes(found.highest + 1) is found.groups
+    with pytest.raises(RuntimeError, match="the node field has"):
+        found.require_nodes(found.highest)
+    with pytest.raises(RuntimeError, match="the node field has"):
+        ff.grouping(torch.tensor([3, -1, 2])).require_nodes(4)
+    empty = ff.grouping(torch.zeros(0, dtype=torch.long))
+    assert [t.shape[0] for t in empty.require_nodes(0)] == [0, 1, 0]
