@@ -185,8 +185,14 @@ def source_groups(source_index: Tensor, key: tuple | None = None, owner: Tensor 
     return grouping(source_index, key, owner).groups
 
 
-def group_key(parent: Any, first: int, last: int) -> tuple:
-    return (id(parent), parent.edge_index.data_ptr(), int(parent.n_edges), int(first), int(last))
+def version(indices: Tensor) -> int:
+    """The tensor's write counter, which every in-place write through torch raises (-1: an inference tensor has none)."""
+    return -1 if indices.is_inference() else indices._version
+
+
+def group_key(parent: Any, first: int, last: int, source: Tensor) -> tuple:
+    """Edges ``first .. last`` of ``parent`` as they are now: indices written over in place are another edge set."""
+    return (id(parent), parent.edge_index.data_ptr(), int(parent.n_edges), int(first), int(last), version(parent.edge_index), version(source))
 
 
 def enabled(kernel: Any, x: Any, edges: Any) -> bool:
@@ -282,7 +288,7 @@ def grouping_for(edges: Any, source: Tensor) -> Grouping:
 
     registered = fused_attention.chunk_of(edges)
     parent, first, last = registered if registered is not None else (edges, 0, int(edges.n_edges))
-    return grouping(source, group_key(parent, first, last), owner=parent.edge_index)
+    return grouping(source, group_key(parent, first, last, edges.source_index), owner=parent.edge_index)
 
 
 def groups_for(edges: Any, source: Tensor) -> tuple[Tensor, Tensor, Tensor]:

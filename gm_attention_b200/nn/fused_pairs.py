@@ -286,7 +286,7 @@ def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
 
     registered = fused_attention.chunk_of(edges)
     parent, first, last = registered if registered is not None else (edges, 0, int(edges.n_edges))
-    return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.group_key(parent, first, last) in ff._GROUPS
+    return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.group_key(parent, first, last, edges.source_index) in ff._GROUPS
 
 
 def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term]) -> tuple | None:
@@ -297,6 +297,8 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     values = [x[n] for n in frequencies]
     nodes = {int(v.shape[0]) for v in values}
     n_edges = int(edges.n_edges)
+    from gm_attention_b200.nn import fused_factored as ff
+
     if hidden.device.type != "cuda" or hidden.dtype not in (torch.float32, torch.float64) or len(nodes) != 1 or not terms:
         return None
     n_nodes = nodes.pop()
@@ -305,12 +307,13 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     angular, transport = getattr(edges, "angular_phases", None), getattr(edges, "transport_phases", None)
     if angular is None or transport is None or not hasattr(edges, "edge_index") or angular.shape != transport.shape:
         return None
+    source = edges.source_index
+    if ff.version(source) < 0 or source.untyped_storage().data_ptr() != edges.edge_index.untyped_storage().data_ptr():
+        return None  # other indices could not be told by the key of their grouping: inference tensors, sources kept apart from edge_index
     if angular.dtype != _complex_of(hidden.dtype) or transport.dtype != angular.dtype or angular.requires_grad or transport.requires_grad:
         return None
     if any(v.device != hidden.device or (v.real if v.is_complex() else v).dtype != hidden.dtype for v in (*values, angular, transport)):
         return None
-    from gm_attention_b200.nn import fused_factored as ff
-
     p, rows = _node_blocks(kernel, terms)
     k = hidden.shape[1] + 1
     if k > ff.MAX_K or p.d_out > ff.MAX_OUT or p.max_bm > ff.MAX_BM or k * (-(-(2 * p.wc + p.wr) // 4) * 4) > ff.MAX_KC:

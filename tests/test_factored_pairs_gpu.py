@@ -467,3 +467,34 @@ def test_node_field_with_too_few_rows_is_refused():
         assert call(lattice.n_nodes).isfinite().all()
         with pytest.raises(RuntimeError, match="the node field has"):
             call(lattice.n_nodes - 1)
+
+
+def test_node_level_field_after_the_edges_were_overwritten(monkeypatch):
+    """``forward_general`` reads the indices as they are at the call: an ``edge_index`` overwritten in place, and a
+    ``source_index`` kept apart from it and replaced, give what the pair terms give for the new sources."""
+    from types import SimpleNamespace
+
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float64)
+    kernel = StandInKernel({0: 2, 1: 2}, {0: 2, 1: 2}, cutoff).to(dev)
+    x = FeatureField.from_flat(kernel.field_type_in, torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev, dtype=torch.float64))
+    apart = SimpleNamespace(**{name: getattr(edges, name) for name in ("edge_index", "n_edges", "row_ptr", "distances", "angular_phases", "transport_phases",
+                                                                       "max_frequency", "angular_harmonic", "transport_harmonic")})
+    apart.source_index = edges.source_index.clone()
+    for _ in range(2):
+        for e in (edges, apart):
+            got = fp.forward_general(kernel, x, e).coefficients
+            with monkeypatch.context() as patch:
+                patch.setattr(fp, "_factored_inputs", lambda *a: None)
+                want = fp.forward_general(kernel, x, e).coefficients
+            for m in want:
+                assert rel_err(got[m].detach().cpu().numpy(), want[m].detach().cpu().numpy()) < 1e-11
+        edges.edge_index[1] = edges.edge_index[1].flip(0)
+        apart.source_index = apart.source_index.roll(11)

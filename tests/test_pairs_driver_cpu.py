@@ -105,3 +105,24 @@ def test_sources_beyond_the_node_field_are_refused():
         ff.grouping(torch.tensor([3, -1, 2])).require_nodes(4)
     empty = ff.grouping(torch.zeros(0, dtype=torch.long))
     assert [t.shape[0] for t in empty.require_nodes(0)] == [0, 1, 0]
+
+
+def test_grouping_follows_indices_written_in_place():
+    """An edge set whose indices are overwritten in place is grouped anew, whether it is written through ``edge_index`` or
+    through a view of it, and so is a registered chunk; unchanged indices keep their grouping."""
+    from gm_attention_b200.nn import fused_attention
+    from gm_attention_b200.nn import fused_factored as ff
+
+    edges, _ = cpu_edges()
+    order_of = lambda e: ff.groups_for(e, e.source_index)[0]
+    first = order_of(edges)
+    assert order_of(edges) is first
+    edges.edge_index[1] = edges.edge_index[1].flip(0)
+    assert torch.equal(order_of(edges), torch.argsort(edges.source_index, stable=True)) and not torch.equal(order_of(edges), first)
+    edges.source_index.copy_(edges.source_index.roll(7))
+    assert torch.equal(order_of(edges), torch.argsort(edges.source_index, stable=True))
+    chunk, lo, hi = edges.target_range(3, 9)
+    fused_attention.register_chunk(chunk, edges, lo, hi)
+    assert order_of(chunk) is order_of(chunk)
+    chunk.edge_index[1] = chunk.edge_index[1].flip(0)
+    assert torch.equal(order_of(chunk), torch.argsort(chunk.source_index, stable=True))
