@@ -158,14 +158,25 @@ _GROUPS: OrderedDict[tuple, tuple[Any, Grouping]] = OrderedDict()
 GROUP_CACHE_SIZE = 512
 
 
+def _cached(key: tuple, owner: Tensor | None, device: torch.device) -> Grouping | None:
+    """The grouping kept under ``key``, if the owner it was built for is alive and the one asking; a dead owner's is dropped."""
+    if key not in _GROUPS:
+        return None
+    held, found = _GROUPS[key]
+    if held is not None and held() is None:
+        del _GROUPS[key]
+        return None
+    if (None if held is None else held()) is not owner or found.groups[0].device != device:
+        return None
+    _GROUPS.move_to_end(key)
+    return found
+
+
 def grouping(source_index: Tensor, key: tuple | None = None, owner: Tensor | None = None) -> Grouping:
     """:func:`source_groups` with the sources' range, read once where the groups are built."""
-    if key is not None and key in _GROUPS:
-        held, found = _GROUPS[key]
-        alive = owner is None if held is None else (held() is not None and held() is owner)
-        if alive and found.groups[0].device == source_index.device:
-            _GROUPS.move_to_end(key)
-            return found
+    found = None if key is None else _cached(key, owner, source_index.device)
+    if found is not None:
+        return found
     order = torch.argsort(source_index, stable=True)
     group_source, counts = torch.unique_consecutive(source_index[order], return_counts=True)
     group_ptr = torch.zeros(group_source.shape[0] + 1, dtype=torch.long, device=source_index.device)
@@ -283,12 +294,22 @@ def inputs(kernel: Any, x: Any, edges: Any, products: dict | None) -> Inputs:
     return Inputs(h.contiguous(), zc, zr, angular, transport, rho, descriptors(kernel, h.device), edges.source_index.contiguous(), p)
 
 
-def grouping_for(edges: Any, source: Tensor) -> Grouping:
+def _slot(edges: Any) -> tuple[tuple, Tensor]:
+    """Key and owner of the edge set's grouping (a registered chunk's: its parent's edges first .. last)."""
     from gm_attention_b200.nn import fused_attention
 
     registered = fused_attention.chunk_of(edges)
     parent, first, last = registered if registered is not None else (edges, 0, int(edges.n_edges))
-    return grouping(source, group_key(parent, first, last, edges.source_index), owner=parent.edge_index)
+    return group_key(parent, first, last, edges.source_index), parent.edge_index
+
+
+def grouping_for(edges: Any, source: Tensor) -> Grouping:
+    return grouping(source, *_slot(edges))
+
+
+def cached_grouping(edges: Any, device: torch.device) -> Grouping | None:
+    """What :func:`grouping_for` would return without building anything, else ``None``."""
+    return _cached(*_slot(edges), device)
 
 
 def groups_for(edges: Any, source: Tensor) -> tuple[Tensor, Tensor, Tensor]:

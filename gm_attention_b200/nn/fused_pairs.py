@@ -281,12 +281,9 @@ def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]]]:
 
 def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
     """Whether an earlier call left the kernel's descriptors on the device and grouped these edges by source."""
-    from gm_attention_b200.nn import fused_attention
     from gm_attention_b200.nn import fused_factored as ff
 
-    registered = fused_attention.chunk_of(edges)
-    parent, first, last = registered if registered is not None else (edges, 0, int(edges.n_edges))
-    return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.group_key(parent, first, last, edges.source_index) in ff._GROUPS
+    return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.cached_grouping(edges, device) is not None
 
 
 def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term]) -> tuple | None:

@@ -498,3 +498,46 @@ def test_node_level_field_after_the_edges_were_overwritten(monkeypatch):
                 assert rel_err(got[m].detach().cpu().numpy(), want[m].detach().cpu().numpy()) < 1e-11
         edges.edge_index[1] = edges.edge_index[1].flip(0)
         apart.source_index = apart.source_index.roll(11)
+
+
+def test_pair_driver_under_capture_beside_a_dead_edge_set(monkeypatch):
+    """An entry left by a freed edge set under the key of a new one does not count as that set's grouping: under capture
+    the call takes the pair terms, as on any edge set it has not seen, instead of building groups inside the graph."""
+    import weakref
+
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_factored as ff
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(8, 18, dev)
+    cutoff = 1.9 * math.pi / 8
+    seen, fresh = (compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32) for _ in range(2))
+    kernel = StandInKernel({0: 3, 1: 2}, {0: 2, 1: 2}, cutoff, trunk=8, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    run = lambda edges: fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, flat), edges).coefficients
+    taken = []
+    recognise = fp._factored_inputs
+    monkeypatch.setattr(fp, "_factored_inputs", lambda *a: taken.append(recognise(*a)) or taken[-1])
+    with torch.no_grad():
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            want = run(seen)
+            with monkeypatch.context() as patch:  # the pair terms once, so that the library behind torch's products is set up
+                patch.setattr(fp, "_factored_inputs", lambda *a: None)
+                run(seen)
+        torch.cuda.current_stream().wait_stream(side)
+        gone = torch.zeros(3)
+        ff._GROUPS[ff._slot(fresh)[0]] = (weakref.ref(gone), ff.grouping_for(seen, seen.source_index))
+        del gone
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = run(fresh)
+        assert taken[-1] is None
+        graph.replay()
+        torch.cuda.synchronize()
+    for m in want:
+        assert rel_err(out[m].cpu().numpy(), want[m].cpu().numpy()) < 4e-6

@@ -126,3 +126,27 @@ def test_grouping_follows_indices_written_in_place():
     assert order_of(chunk) is order_of(chunk)
     chunk.edge_index[1] = chunk.edge_index[1].flip(0)
     assert torch.equal(order_of(chunk), torch.argsort(chunk.source_index, stable=True))
+
+
+def test_a_dead_edge_sets_grouping_is_nobodys():
+    """An entry whose edge set is gone is not found under the key of the set that took its id and address, neither by the
+    query nor by the builder, and is dropped."""
+    import weakref
+
+    from gm_attention_b200.nn import fused_factored as ff
+
+    edges, _ = cpu_edges()
+    device = edges.source_index.device
+    assert ff.cached_grouping(edges, device) is None
+    gone = torch.zeros(3)
+    reference = weakref.ref(gone)
+    del gone
+    key, _ = ff._slot(edges)
+    stale = ff.Grouping(ff.source_groups(edges.source_index.flip(0)), 0, 39)
+    ff._GROUPS[key] = (reference, stale)
+    assert ff.cached_grouping(edges, device) is None and key not in ff._GROUPS
+    ff._GROUPS[key] = (reference, stale)
+    found = ff.grouping_for(edges, edges.source_index)
+    assert found is not stale and torch.equal(found.groups[0], torch.argsort(edges.source_index, stable=True))
+    assert ff.cached_grouping(edges, device) is found
+    assert ff._cached(key, None, device) is None and ff._cached(key, edges.row_ptr, device) is None and key in ff._GROUPS
