@@ -19,6 +19,7 @@ from __future__ import annotations
 
 import functools
 import os
+import threading
 import weakref
 from collections import OrderedDict
 from dataclasses import dataclass
@@ -154,22 +155,45 @@ class Grouping:
         return self.groups
 
 
-_GROUPS: OrderedDict[tuple, tuple[Any, Grouping]] = OrderedDict()
+@dataclass
+class _Kept:
+    held: Any  # weak reference to the owner, None where there is none
+    found: Grouping
+    captured: bool = False  # a graph reads these groups by address
+
+
+_GROUPS: OrderedDict[tuple, _Kept] = OrderedDict()
 GROUP_CACHE_SIZE = 512
+_GROUPS_LOCK = threading.Lock()
 
 
 def _cached(key: tuple, owner: Tensor | None, device: torch.device) -> Grouping | None:
-    """The grouping kept under ``key``, if the owner it was built for is alive and the one asking; a dead owner's is dropped."""
-    if key not in _GROUPS:
-        return None
-    held, found = _GROUPS[key]
-    if held is not None and held() is None:
-        del _GROUPS[key]
-        return None
-    if (None if held is None else held()) is not owner or found.groups[0].device != device:
-        return None
-    _GROUPS.move_to_end(key)
-    return found
+    """The grouping kept under ``key``, if the owner it was built for is alive and the one asking; a dead owner's is dropped.
+    One handed out while a graph is captured stays for as long as its owner lives, however many others are built."""
+    with _GROUPS_LOCK:
+        kept = _GROUPS.get(key)
+        if kept is None:
+            return None
+        if kept.held is not None and kept.held() is None:
+            del _GROUPS[key]
+            return None
+        if (None if kept.held is None else kept.held()) is not owner or kept.found.groups[0].device != device:
+            return None
+        _GROUPS.move_to_end(key)
+        if device.type == "cuda" and torch.cuda.is_current_stream_capturing():
+            kept.captured = True
+        return kept.found
+
+
+def _keep(key: tuple, owner: Tensor | None, built: Grouping) -> None:
+    """``built`` under ``key``; beyond GROUP_CACHE_SIZE entries the least recently used go, but for those a graph reads."""
+    with _GROUPS_LOCK:
+        for gone in [k for k, kept in _GROUPS.items() if kept.held is not None and kept.held() is None]:
+            del _GROUPS[gone]
+        _GROUPS[key] = _Kept(None if owner is None else weakref.ref(owner), built)
+        loose = [k for k, kept in _GROUPS.items() if not kept.captured]
+        for old in loose[:max(len(loose) - GROUP_CACHE_SIZE, 0)]:
+            del _GROUPS[old]
 
 
 def grouping(source_index: Tensor, key: tuple | None = None, owner: Tensor | None = None) -> Grouping:
@@ -184,9 +208,7 @@ def grouping(source_index: Tensor, key: tuple | None = None, owner: Tensor | Non
     lowest, highest = torch.stack((group_source[0], group_source[-1])).tolist() if group_source.shape[0] else (0, -1)
     built = Grouping((order.contiguous(), group_ptr.contiguous(), group_source.contiguous()), lowest, highest)
     if key is not None:
-        _GROUPS[key] = (None if owner is None else weakref.ref(owner), built)
-        while len(_GROUPS) > GROUP_CACHE_SIZE:
-            _GROUPS.popitem(last=False)
+        _keep(key, owner, built)
     return built
 
 

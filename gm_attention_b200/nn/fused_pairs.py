@@ -305,8 +305,9 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     if angular is None or transport is None or not hasattr(edges, "edge_index") or angular.shape != transport.shape:
         return None
     source = edges.source_index
-    if ff.version(source) < 0 or source.untyped_storage().data_ptr() != edges.edge_index.untyped_storage().data_ptr():
-        return None  # other indices could not be told by the key of their grouping: inference tensors, sources kept apart from edge_index
+    if edges.edge_index is not edges.edge_index or ff.version(source) < 0 or source.untyped_storage().data_ptr() != edges.edge_index.untyped_storage().data_ptr():
+        return None  # no grouping to keep, or one whose key could not tell other indices: an edge_index formed on every access,
+        # inference tensors, sources kept apart from edge_index
     if angular.dtype != _complex_of(hidden.dtype) or transport.dtype != angular.dtype or angular.requires_grad or transport.requires_grad:
         return None
     if any(v.device != hidden.device or (v.real if v.is_complex() else v).dtype != hidden.dtype for v in (*values, angular, transport)):

@@ -531,7 +531,7 @@ def test_pair_driver_under_capture_beside_a_dead_edge_set(monkeypatch):
                 run(seen)
         torch.cuda.current_stream().wait_stream(side)
         gone = torch.zeros(3)
-        ff._GROUPS[ff._slot(fresh)[0]] = (weakref.ref(gone), ff.grouping_for(seen, seen.source_index))
+        ff._GROUPS[ff._slot(fresh)[0]] = ff._Kept(weakref.ref(gone), ff.grouping_for(seen, seen.source_index))
         del gone
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
@@ -541,3 +541,42 @@ def test_pair_driver_under_capture_beside_a_dead_edge_set(monkeypatch):
         torch.cuda.synchronize()
     for m in want:
         assert rel_err(out[m].cpu().numpy(), want[m].cpu().numpy()) < 4e-6
+
+
+def test_captured_pair_driver_outlives_the_grouping_cache(monkeypatch):
+    """A graph that captured the factored form replays the eager result after other edge sets have filled the cache of
+    groupings several times over: the groups it reads by address stay while the edge set lives."""
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_factored as ff
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(8, 18, dev)
+    cutoff = 1.9 * math.pi / 8
+    make = lambda: compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32)
+    seen = make()
+    kernel = StandInKernel({0: 3, 1: 2}, {0: 2, 1: 2}, cutoff, trunk=8, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    run = lambda edges: fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, flat), edges).coefficients
+    monkeypatch.setattr(ff, "GROUP_CACHE_SIZE", 2)
+    with torch.no_grad():
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            want = {m: v.clone() for m, v in run(seen).items()}
+        torch.cuda.current_stream().wait_stream(side)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = run(seen)
+        entry = ff._GROUPS[ff._slot(seen)[0]]
+        assert entry.captured
+        others = [make() for _ in range(8)]
+        for e in others:
+            ff.grouping_for(e, e.source_index)
+        assert ff._GROUPS[ff._slot(seen)[0]] is entry and len(ff._GROUPS) <= 3 + sum(kept.captured for kept in ff._GROUPS.values())
+        graph.replay()
+        torch.cuda.synchronize()
+    for m in want:
+        assert torch.equal(out[m], want[m])

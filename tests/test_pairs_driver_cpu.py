@@ -143,10 +143,30 @@ def test_a_dead_edge_sets_grouping_is_nobodys():
     del gone
     key, _ = ff._slot(edges)
     stale = ff.Grouping(ff.source_groups(edges.source_index.flip(0)), 0, 39)
-    ff._GROUPS[key] = (reference, stale)
+    ff._GROUPS[key] = ff._Kept(reference, stale)
     assert ff.cached_grouping(edges, device) is None and key not in ff._GROUPS
-    ff._GROUPS[key] = (reference, stale)
+    ff._GROUPS[key] = ff._Kept(reference, stale)
     found = ff.grouping_for(edges, edges.source_index)
     assert found is not stale and torch.equal(found.groups[0], torch.argsort(edges.source_index, stable=True))
     assert ff.cached_grouping(edges, device) is found
     assert ff._cached(key, None, device) is None and ff._cached(key, edges.row_ptr, device) is None and key in ff._GROUPS
+
+
+def test_groupings_read_by_a_graph_outlive_the_cache(monkeypatch):
+    """A grouping handed out during a capture is kept until its edge set goes, past any number of others; the rest are
+    bounded, least recently used first, and dead edge sets' entries go when one is added."""
+    from gm_attention_b200.nn import fused_factored as ff
+
+    monkeypatch.setattr(ff, "_GROUPS", type(ff._GROUPS)())
+    monkeypatch.setattr(ff, "GROUP_CACHE_SIZE", 3)
+    sets = [cpu_edges()[0] for _ in range(6)]
+    find = lambda e: ff.grouping_for(e, e.source_index)
+    captured = find(sets[0])
+    ff._GROUPS[ff._slot(sets[0])[0]].captured = True
+    built = [find(e) for e in sets[1:]]
+    assert len(ff._GROUPS) == 4 and find(sets[0]) is captured
+    assert [find(e) is b for e, b in zip(sets[3:], built[2:])] == [True] * 3
+    assert ff.cached_grouping(sets[1], sets[1].source_index.device) is None
+    del sets[0]
+    find(sets[0])
+    assert len(ff._GROUPS) == 3 and not any(kept.captured for kept in ff._GROUPS.values())
