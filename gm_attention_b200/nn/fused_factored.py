@@ -159,6 +159,7 @@ class Grouping:
 class _Kept:
     held: Any  # weak reference to the owner, None where there is none
     found: Grouping
+    stream: Any  # where the groups were built, None on the CPU
     captured: bool = False  # a graph reads these groups by address
 
 
@@ -169,7 +170,8 @@ _GROUPS_LOCK = threading.Lock()
 
 def _cached(key: tuple, owner: Tensor | None, device: torch.device) -> Grouping | None:
     """The grouping kept under ``key``, if the owner it was built for is alive and the one asking; a dead owner's is dropped.
-    One handed out while a graph is captured stays for as long as its owner lives, however many others are built."""
+    One handed out while a graph is captured stays for as long as its owner lives, however many others are built; one
+    handed to another stream than it was built on is not given back to the allocator before that stream is done with it."""
     with _GROUPS_LOCK:
         kept = _GROUPS.get(key)
         if kept is None:
@@ -180,8 +182,13 @@ def _cached(key: tuple, owner: Tensor | None, device: torch.device) -> Grouping 
         if (None if kept.held is None else kept.held()) is not owner or kept.found.groups[0].device != device:
             return None
         _GROUPS.move_to_end(key)
-        if device.type == "cuda" and torch.cuda.is_current_stream_capturing():
-            kept.captured = True
+        if kept.stream is not None:
+            stream = torch.cuda.current_stream(device)
+            if torch.cuda.is_current_stream_capturing():
+                kept.captured = kept.held is not None
+            elif stream != kept.stream:
+                for t in kept.found.groups:
+                    t.record_stream(stream)
         return kept.found
 
 
@@ -190,7 +197,8 @@ def _keep(key: tuple, owner: Tensor | None, built: Grouping) -> None:
     with _GROUPS_LOCK:
         for gone in [k for k, kept in _GROUPS.items() if kept.held is not None and kept.held() is None]:
             del _GROUPS[gone]
-        _GROUPS[key] = _Kept(None if owner is None else weakref.ref(owner), built)
+        device = built.groups[0].device
+        _GROUPS[key] = _Kept(None if owner is None else weakref.ref(owner), built, torch.cuda.current_stream(device) if device.type == "cuda" else None)
         loose = [k for k, kept in _GROUPS.items() if not kept.captured]
         for old in loose[:max(len(loose) - GROUP_CACHE_SIZE, 0)]:
             del _GROUPS[old]
@@ -205,6 +213,7 @@ def grouping(source_index: Tensor, key: tuple | None = None, owner: Tensor | Non
     group_source, counts = torch.unique_consecutive(source_index[order], return_counts=True)
     group_ptr = torch.zeros(group_source.shape[0] + 1, dtype=torch.long, device=source_index.device)
     group_ptr[1:] = torch.cumsum(counts, 0)
+    # read last: the host waits for the groups here, so whatever stream asks for them later finds them written
     lowest, highest = torch.stack((group_source[0], group_source[-1])).tolist() if group_source.shape[0] else (0, -1)
     built = Grouping((order.contiguous(), group_ptr.contiguous(), group_source.contiguous()), lowest, highest)
     if key is not None:

@@ -531,7 +531,7 @@ def test_pair_driver_under_capture_beside_a_dead_edge_set(monkeypatch):
                 run(seen)
         torch.cuda.current_stream().wait_stream(side)
         gone = torch.zeros(3)
-        ff._GROUPS[ff._slot(fresh)[0]] = ff._Kept(weakref.ref(gone), ff.grouping_for(seen, seen.source_index))
+        ff._GROUPS[ff._slot(fresh)[0]] = ff._Kept(weakref.ref(gone), ff.grouping_for(seen, seen.source_index), torch.cuda.current_stream())
         del gone
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
@@ -580,3 +580,41 @@ def test_captured_pair_driver_outlives_the_grouping_cache(monkeypatch):
         torch.cuda.synchronize()
     for m in want:
         assert torch.equal(out[m], want[m])
+
+
+def test_grouping_shared_between_streams(monkeypatch):
+    """Groups built at the end of one stream's queue are complete for a call on another stream, without an order between
+    the two; and groups that are dropped while that stream still waits to read them are not handed out again."""
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_factored as ff
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(16, 40, dev)
+    cutoff = 1.9 * math.pi / 16
+    edges, same = (compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32) for _ in range(2))
+    kernel = StandInKernel({0: 3, 1: 2}, {0: 2, 1: 2}, cutoff, trunk=8, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    run = lambda e: fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, flat), e).coefficients
+    with torch.no_grad():
+        want = run(same)
+        torch.cuda.synchronize()
+        first, second = torch.cuda.Stream(), torch.cuda.Stream()
+        with torch.cuda.stream(first):
+            torch.cuda._sleep(100_000_000)
+            found = ff.grouping_for(edges, edges.source_index)
+        with torch.cuda.stream(second):
+            out = run(edges)
+            torch.cuda._sleep(100_000_000)
+            late = run(edges)
+        shapes = [t.shape for t in found.groups]
+        del found
+        del ff._GROUPS[ff._slot(edges)[0]]
+        with torch.cuda.stream(first):  # zeros are harmless groups, and not these
+            again = [torch.zeros(s, dtype=torch.long, device=dev) for s in shapes for _ in range(3)]
+        torch.cuda.synchronize()
+    assert again
+    for m in want:
+        assert torch.equal(out[m], want[m]) and torch.equal(late[m], want[m])

@@ -143,9 +143,9 @@ def test_a_dead_edge_sets_grouping_is_nobodys():
     del gone
     key, _ = ff._slot(edges)
     stale = ff.Grouping(ff.source_groups(edges.source_index.flip(0)), 0, 39)
-    ff._GROUPS[key] = ff._Kept(reference, stale)
+    ff._GROUPS[key] = ff._Kept(reference, stale, None)
     assert ff.cached_grouping(edges, device) is None and key not in ff._GROUPS
-    ff._GROUPS[key] = ff._Kept(reference, stale)
+    ff._GROUPS[key] = ff._Kept(reference, stale, None)
     found = ff.grouping_for(edges, edges.source_index)
     assert found is not stale and torch.equal(found.groups[0], torch.argsort(edges.source_index, stable=True))
     assert ff.cached_grouping(edges, device) is found
