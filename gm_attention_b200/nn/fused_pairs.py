@@ -328,7 +328,8 @@ def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tu
 
     p, rows, values, angular, transport, n_nodes = found
     device, dtype = hidden.device, hidden.dtype
-    flat = [(torch.view_as_real(v) if v.is_complex() else v).reshape(n_nodes, -1) for v in values]
+    # the kernels read memory: conjugations and signs that torch has put off are carried out first
+    flat = [(torch.view_as_real(v.resolve_conj()) if v.is_complex() else v.resolve_neg()).reshape(n_nodes, -1) for v in values]
     packed = flat[0] if len(flat) == 1 else torch.cat(flat, 1)
     tables = kernel.__dict__.setdefault("_fused_node_descriptors", {})
     if str(device) not in tables:
@@ -341,7 +342,7 @@ def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tu
     rho = kernel._radial_powers(edges.distances)[:, 1].detach().to(dtype).contiguous() if max(powers, default=0) else hidden.new_ones(hidden.shape[0])
     source = edges.source_index.contiguous()
     order, group_ptr, group_source = ff.grouping_for(edges, source).require_nodes(n_nodes)
-    out = ff.Factored.apply(hidden, zc, zr, torch.view_as_real(angular.contiguous()), torch.view_as_real(transport.contiguous()), rho, desc, source,
+    out = ff.Factored.apply(hidden, zc, zr, *(torch.view_as_real(t.resolve_conj().contiguous()) for t in (angular, transport)), rho, desc, source,
                             order, group_ptr, group_source, p.d_out, p.max_bm)
     slices = kernel.field_type_out.slices()
     orders = sorted(kernel.field_type_out.frequencies, key=lambda m: slices[m].start)

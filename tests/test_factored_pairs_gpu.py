@@ -618,3 +618,45 @@ def test_grouping_shared_between_streams(monkeypatch):
     assert again
     for m in want:
         assert torch.equal(out[m], want[m]) and torch.equal(late[m], want[m])
+
+
+class _Field:
+    """A field of any coefficients, complex ones among them."""
+
+    def __init__(self, field_type, coefficients):
+        self.field_type, self.coefficients = field_type, coefficients
+
+    def __getitem__(self, frequency):
+        return self.coefficients[frequency]
+
+
+def test_node_level_field_with_lazy_conjugates(monkeypatch):
+    """Complex coefficients and phase tables that are conjugate views, and real ones with a pending sign, give the factored
+    form the values the pair terms see.  float64, 1e-11."""
+    import dataclasses
+
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    plain = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float64)
+    lazy = dataclasses.replace(plain, angular_phases=plain.angular_phases.conj(), transport_phases=plain.transport_phases.conj())
+    kernel = StandInKernel({0: 2, 1: 3, 2: 1}, {0: 2, 1: 2}, cutoff).to(dev)
+    draw = lambda a: torch.randn(lattice.n_nodes, a, dtype=torch.complex128, device=dev, requires_grad=True)
+    z0, z1, z2 = draw(2), draw(3), draw(1)
+    for edges in (plain, lazy):
+        results = []
+        for factored in (True, False):
+            values = {0: z0.conj().imag, 1: z1.conj(), 2: torch.view_as_real(z2)}
+            assert values[0].is_neg() and values[1].is_conj()
+            with monkeypatch.context() as patch:
+                if not factored:
+                    patch.setattr(fp, "_factored_inputs", lambda *a: None)
+                out = fp.forward_general(kernel, _Field(kernel.field_type_in, values), edges).coefficients
+            loss = sum((v * torch.linspace(-1.0, 1.0, v.numel(), dtype=v.dtype, device=dev).reshape(v.shape)).sum() for v in out.values())
+            results.append([*out.values(), *(torch.view_as_real(g.resolve_conj()) for g in torch.autograd.grad(loss, [z0, z1, z2]))])
+        for a, b in zip(*results):
+            assert rel_err(a.detach().cpu().numpy(), b.detach().cpu().numpy()) < 1e-11
