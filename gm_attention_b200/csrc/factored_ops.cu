@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, 
   for (int64_t g0 = blockIdx.x; g0 < a.n_groups; g0 += gridDim.x) {
     const int64_t grp = from_both_ends(g0, a.n_groups);
     const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
-    if (first == last) continue;  // a source without edges has no row, and no tile below would wait for its copies
+    copy_wait();  // where the source before had no edges, no tile waited for its copies, and these go to the same place
     __syncthreads();
     stage_node(a, j, z_s, L.pitch);
     for (int64_t x0 = first; x0 < last; x0 += tile) {
@@ -362,8 +362,9 @@ __global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a,
   for (int64_t g0 = blockIdx.x; g0 < a.n_groups; g0 += gridDim.x) {
     const int64_t grp = from_both_ends(g0, a.n_groups);
     const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
+    copy_wait();  // as in the forward
     __syncthreads();
-    if (first < last) stage_node(a, j, z_s, pitch);  // waited for in the first tile; a source without edges has none and gets zeros
+    stage_node(a, j, z_s, pitch);
     for (int pass = 0; pass < passes; ++pass) {
       T acc[NP][TP][4];
 #pragma unroll
