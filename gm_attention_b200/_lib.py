@@ -41,6 +41,8 @@ SIGNATURES: dict[str, list[Any]] = {
     "gm_factored_forward": [_P] * 11 + [_L, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "gm_factored_aggregate": [_P, _P, _P, _L, _L, _I, _I, _P, _P],
     "gm_factored_backward": [_P] * 15 + [_L, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
+    "gm_factored_forward_scaled": [_P] * 6 + [_I] + [_P] * 5 + [_L, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "gm_factored_backward_scaled": [_P] * 10 + [_I] + [_P] * 5 + [_L, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P, _P, _P, _P],
     "gm_pairs_forward": [_P] * 8 + [_L, _I, _I, _I, _I, _I, _P],
     "gm_pairs_backward": [_P] * 11 + [_L, _I, _I, _I, _I, _I, _P],
     "gm_node_products_forward": [_P] * 6 + [_L] + [_I] * 6 + [_P] * 3,

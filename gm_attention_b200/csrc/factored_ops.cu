@@ -41,6 +41,7 @@ template <typename T>
 struct FArgs {
   int64_t n_edges, n_groups;
   int k, wc, wr, n_f, n_blocks, d_out;
+  int n_scales;  // 0: rho (n_edges), a block's scale is a power of it; else (SCALED) rho (n_edges, n_scales), its scale a column of it
   const T *h, *zc, *zr, *angular, *transport, *rho;
   const int32_t* desc;
   const int64_t *source, *order, *group_ptr, *group_source;
@@ -52,8 +53,8 @@ struct FArgs {
   T *dh, *dzc, *dzr, *dweights;
 };
 
-// An edge's record in shared memory: angular phases (n_f, 2), transport phases (n_f, 2), rho; odd pitch.
-inline int record_pitch(int n_f) { return 4 * n_f + 1; }
+// An edge's record in shared memory: angular phases (n_f, 2), transport phases (n_f, 2), rho or the scales; odd pitch.
+__host__ __device__ inline int record_pitch(int n_f, int n_scales) { return n_scales ? (4 * n_f + n_scales) | 1 : 4 * n_f + 1; }
 
 // One element global -> shared, asynchronously.
 template <typename T>
@@ -86,16 +87,16 @@ __device__ __forceinline__ void stage_rows(T* dst, int pitch, const T* src, int 
 }
 
 // The records of n edges (edges_s: their indices)
-template <typename T>
+template <bool SCALED, typename T>
 __device__ __forceinline__ void stage_records(const FArgs<T>& a, const int64_t* edges_s, int n, T* rec) {
-  const int w = 2 * a.n_f, pitch = 2 * w + 1;
+  const int w = 2 * a.n_f, pitch = record_pitch(a.n_f, SCALED ? a.n_scales : 0);
   stage_rows(rec, pitch, a.angular, w, n, edges_s);
   stage_rows(rec + w, pitch, a.transport, w, n, edges_s);
-  stage_rows(rec + 2 * w, pitch, a.rho, 1, n, edges_s);
+  stage_rows(rec + 2 * w, pitch, a.rho, SCALED ? a.n_scales : 1, n, edges_s);
 }
 
-// The block's per-edge factor (factored.h:118-144), from the edge's record.
-template <typename T>
+// The block's per-edge factor (factored.h:118-144), from the edge's record; SCALED: "power" names a scale.
+template <bool SCALED, typename T>
 __device__ __forceinline__ void block_factor(const T* rec, int n_f, const int32_t* d, T& fr, T& fi) {
   fr = T(1);
   fi = T(0);
@@ -115,9 +116,13 @@ __device__ __forceinline__ void block_factor(const T* rec, int n_f, const int32_
     fr = nr;
     fi = ni;
   }
-  const T r = rec[4 * n_f];
   T s = T(1);
-  for (int x = 0; x < power; ++x) s *= r;
+  if constexpr (SCALED) {
+    s = rec[4 * n_f + power];
+  } else {
+    const T r = rec[4 * n_f];
+    for (int x = 0; x < power; ++x) s *= r;
+  }
   fr *= s;
   fi *= s;
 }
@@ -165,12 +170,12 @@ template <typename T>
 struct ForwardLayout {  // shared memory, in elements of T
   int tile, pitch, cols, e_pitch, rec_pitch, row_pitch;
   int z, h, u, f, rec, total;
-  __host__ __device__ ForwardLayout(int k, int C, int n_f, int n_blocks, int d_out, int tile_) {
+  __host__ __device__ ForwardLayout(int k, int C, int n_f, int n_scales, int n_blocks, int d_out, int tile_) {
     tile = tile_;
     cols = (C + 3) / 4 * 4;
     pitch = cols;
     e_pitch = tile + 4;
-    rec_pitch = 4 * n_f + 1;
+    rec_pitch = record_pitch(n_f, n_scales);
     row_pitch = d_out | 1;
     z = 0;
     h = z + k * pitch;
@@ -181,13 +186,13 @@ struct ForwardLayout {  // shared memory, in elements of T
   }
 };
 
-template <typename T>
+template <typename T, bool SCALED>
 __global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, int tile) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int64_t edges_s[MAX_TILE];
   __shared__ int n_out_s;
   const int wc2 = 2 * a.wc, C = wc2 + a.wr;
-  const ForwardLayout<T> L(a.k, C, a.n_f, a.n_blocks, a.d_out, tile);
+  const ForwardLayout<T> L(a.k, C, a.n_f, SCALED ? a.n_scales : 0, a.n_blocks, a.d_out, tile);
   T* base_s = reinterpret_cast<T*>(raw);
   T* z_s = base_s + L.z;      // (k, pitch)
   T* h_s = base_s + L.h;      // (k, e_pitch): h~ transposed
@@ -232,7 +237,7 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, 
       if ((int)threadIdx.x < n_tile) edges_s[threadIdx.x] = a.order[x0 + threadIdx.x];
       __syncthreads();
       for_rows(n_tile, a.k - 1, [&](int e, int t) { copy_async(h_s + (t + 1) * L.e_pitch + e, a.h + edges_s[e] * (a.k - 1) + t); });
-      stage_records(a, edges_s, n_tile, rec_s);
+      stage_records<SCALED>(a, edges_s, n_tile, rec_s);
       if ((int)threadIdx.x < tile) h_s[threadIdx.x] = T(1);
       copy_wait();
       __syncthreads();
@@ -261,7 +266,7 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, 
         for (int b = sub; b < a.n_blocks; b += subs) {
           if (desc_s[b * FDESC] == 0) continue;
           T fr, fi;
-          block_factor(rec_s + le * L.rec_pitch, a.n_f, desc_s + b * FDESC, fr, fi);
+          block_factor<SCALED>(rec_s + le * L.rec_pitch, a.n_f, desc_s + b * FDESC, fr, fi);
           f_s[2 * b * tile + le] = fr;
           f_s[(2 * b + 1) * tile + le] = fi;
         }
@@ -322,14 +327,14 @@ template <typename T>
 struct BackwardLayout {  // shared memory, in elements of T
   int pitch, quads, tgroups, h_pitch, rec_pitch, g_pitch, tile;
   int z, w, h, rec, g, scale, total;
-  __host__ __device__ BackwardLayout(int k, int C, int n_f, int d_out, int tile_) {
+  __host__ __device__ BackwardLayout(int k, int C, int n_f, int n_scales, int d_out, int tile_) {
     const int vecs = (C + 3) / 4;
     tile = tile_;
     pitch = 4 * (vecs | 1);
     quads = (k - 1 + 3) / 4;           // groups of 4 trunk rows t = 1 ..
     tgroups = (k + TP - 1) / TP;
     h_pitch = tile + 4;                // h~ transposed: (t, edge)
-    rec_pitch = 4 * n_f + 1;
+    rec_pitch = record_pitch(n_f, n_scales);
     g_pitch = d_out | 1;
     z = 0;
     const int z_rows = 1 + 4 * quads;
@@ -343,11 +348,13 @@ struct BackwardLayout {  // shared memory, in elements of T
 };
 
 // NP: dZ patches per thread and pass over the source's edges (wider kernels take several passes)
-template <typename T, int NP>
-__global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a, int C, int tile) {
+// (float64 with one patch: four CTAs' registers suffice without spills; left to itself the compiler took 168 for the SCALED form
+// and 64 x 128, {2, 2} -> {2, 2}, trunk 8 went from 233 to 291 us)
+template <typename T, int NP, bool SCALED>
+__global__ void __launch_bounds__(FTHREADS, (SCALED && sizeof(T) == 8 && NP == 1 ? 4 : 0)) factored_backward_kernel(FArgs<T> a, int C, int tile) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int64_t edges_s[MAX_TILE], g_rows_s[MAX_TILE];  // the tile's edges, and the rows of g that reach them
-  const BackwardLayout<T> L(a.k, C, a.n_f, a.d_out, tile);
+  const BackwardLayout<T> L(a.k, C, a.n_f, SCALED ? a.n_scales : 0, a.d_out, tile);
   const int K = a.k, wc2 = 2 * a.wc, pitch = L.pitch;
   T* base_s = reinterpret_cast<T*>(raw);
   T* z_s = base_s + L.z;      // (1 + 4 quads, pitch): packed per t as [zc (wc, 2) | zr (wr) | 0]
@@ -382,7 +389,7 @@ __global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a,
           g_rows_s[threadIdx.x] = a.target ? a.target[e] : e;
         }
         __syncthreads();
-        stage_records(a, edges_s, n_tile, rec_s);
+        stage_records<SCALED>(a, edges_s, n_tile, rec_s);
         stage_rows(g_s, L.g_pitch, a.g, a.d_out, n_tile, g_rows_s);
         for_rows(n_tile, K - 1, [&](int le, int t) { copy_async(h_s + (t + 1) * L.h_pitch + le, a.h + edges_s[le] * (K - 1) + t); });
         // edges beyond the tile's end (their h~ multiplies whatever W rows an earlier tile left): zero
@@ -408,7 +415,7 @@ __global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a,
             for (int c = 0; c < bm; ++c) w[wc2 + zoff + c] = scale * g[c];
           } else {
             T fr, fi;
-            block_factor(rec_s + le * L.rec_pitch, a.n_f, d, fr, fi);
+            block_factor<SCALED>(rec_s + le * L.rec_pitch, a.n_f, d, fr, fi);
             for (int c = 0; c < bm; ++c) {
               const T gr = scale * (take_real ? g[c] : g[2 * c]);
               const T gi = take_real ? T(0) : scale * g[2 * c + 1];
@@ -503,7 +510,8 @@ __global__ void __launch_bounds__(FTHREADS) factored_backward_kernel(FArgs<T> a,
 
 int check_factored(const void* h, const void* zc, const void* zr, const void* angular, const void* transport, const void* rho,
                    const int32_t* desc, const int64_t* source, int64_t n_edges, int k, int wc, int wr, int n_f, int n_blocks, int d_out,
-                   int dtype) {
+                   int n_scales, int dtype) {
+  GM_REQUIRE(n_scales >= 0, GM_ERR_ARGUMENT, "gm_factored: negative n_scales");
   GM_REQUIRE(n_edges >= 0 && wc >= 0 && wr >= 0 && n_f >= 1 && n_blocks >= 0, GM_ERR_ARGUMENT, "gm_factored: bad sizes");
   GM_REQUIRE(k >= 1 && k <= FMAX_K, GM_ERR_ARGUMENT, "gm_factored: k exceeds MAX_K");
   GM_REQUIRE(d_out >= 1 && d_out <= 128, GM_ERR_ARGUMENT, "gm_factored: d_out must be in [1, MAX_OUT]");
@@ -523,13 +531,21 @@ extern "C" int gm_factored_forward(const void* h, const void* zc, const void* zr
                                    const void* rho, const int32_t* desc, const int64_t* source, const int64_t* order,
                                    const int64_t* group_ptr, const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k,
                                    int wc, int wr, int n_f, int n_blocks, int d_out, int dtype, void* out, void* stream) {
-  int status = check_factored(h, zc, zr, angular, transport, rho, desc, source, n_edges, k, wc, wr, n_f, n_blocks, d_out, dtype);
+  return gm_factored_forward_scaled(h, zc, zr, angular, transport, rho, 0, desc, source, order, group_ptr, group_source, n_edges, n_groups, k,
+                                    wc, wr, n_f, n_blocks, d_out, dtype, out, stream);
+}
+
+extern "C" int gm_factored_forward_scaled(const void* h, const void* zc, const void* zr, const void* angular, const void* transport,
+                                          const void* rho, int n_scales, const int32_t* desc, const int64_t* source, const int64_t* order,
+                                          const int64_t* group_ptr, const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k,
+                                          int wc, int wr, int n_f, int n_blocks, int d_out, int dtype, void* out, void* stream) {
+  int status = check_factored(h, zc, zr, angular, transport, rho, desc, source, n_edges, k, wc, wr, n_f, n_blocks, d_out, n_scales, dtype);
   if (status != GM_OK || n_edges == 0) return status;
   GM_REQUIRE(order && group_ptr && group_source && out && n_groups >= 1, GM_ERR_ARGUMENT, "gm_factored_forward: null grouping / output");
   auto run = [&](auto tag) {
     using T = decltype(tag);
     FArgs<T> a{};
-    a.n_edges = n_edges; a.n_groups = n_groups; a.k = k; a.wc = wc; a.wr = wr; a.n_f = n_f; a.n_blocks = n_blocks; a.d_out = d_out;
+    a.n_edges = n_edges; a.n_groups = n_groups; a.k = k; a.wc = wc; a.wr = wr; a.n_f = n_f; a.n_blocks = n_blocks; a.d_out = d_out; a.n_scales = n_scales;
     a.h = (const T*)h; a.zc = (const T*)zc; a.zr = (const T*)zr; a.angular = (const T*)angular; a.transport = (const T*)transport;
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.out = (T*)out;
@@ -537,13 +553,15 @@ extern "C" int gm_factored_forward(const void* h, const void* zc, const void* zr
     const size_t extra = (size_t)(n_blocks * FDESC) * sizeof(int32_t) + (size_t)(n_blocks + d_out) * sizeof(int4);
     // 64 edges per tile; fewer where the packed width or the phase tables leave no room for them
     int tile = MAX_TILE;
-    while (tile > 8 && ForwardLayout<T>(k, C, n_f, n_blocks, d_out, tile).total * sizeof(T) + extra > 200 * 1024) tile /= 2;
-    const size_t smem = ForwardLayout<T>(k, C, n_f, n_blocks, d_out, tile).total * sizeof(T) + extra;
-    int st = allow_smem(factored_forward_kernel<T>, smem, "gm_factored_forward");
-    if (st != GM_OK) return st;
+    while (tile > 8 && ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra > 200 * 1024) tile /= 2;
+    const size_t smem = ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra;
     const int64_t cap = (int64_t)sm_count() * 16;  // the CTAs stride the sources: the column list is built once per CTA
-    factored_forward_kernel<T><<<(unsigned)(n_groups < cap ? n_groups : cap), FTHREADS, smem, (cudaStream_t)stream>>>(a, tile);
-    return launch_status("gm_factored_forward");
+    auto go = [&](auto kernel) {
+      const int st = allow_smem(kernel, smem, "gm_factored_forward");
+      if (st == GM_OK) kernel<<<(unsigned)(n_groups < cap ? n_groups : cap), FTHREADS, smem, (cudaStream_t)stream>>>(a, tile);
+      return st == GM_OK ? launch_status("gm_factored_forward") : st;
+    };
+    return n_scales ? go(factored_forward_kernel<T, true>) : go(factored_forward_kernel<T, false>);
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }
@@ -567,7 +585,16 @@ extern "C" int gm_factored_backward(const void* g, const int64_t* target, const 
                                     const int32_t* desc, const int64_t* source, const int64_t* order, const int64_t* group_ptr,
                                     const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k, int wc, int wr, int n_f,
                                     int n_blocks, int d_out, int dtype, void* dh, void* dzc, void* dzr, void* dweights, void* stream) {
-  int status = check_factored(h, zc, zr, angular, transport, rho, desc, source, n_edges, k, wc, wr, n_f, n_blocks, d_out, dtype);
+  return gm_factored_backward_scaled(g, target, weights, rows, h, zc, zr, angular, transport, rho, 0, desc, source, order, group_ptr, group_source,
+                                     n_edges, n_groups, k, wc, wr, n_f, n_blocks, d_out, dtype, dh, dzc, dzr, dweights, stream);
+}
+
+extern "C" int gm_factored_backward_scaled(const void* g, const int64_t* target, const void* weights, const void* rows, const void* h,
+                                           const void* zc, const void* zr, const void* angular, const void* transport, const void* rho, int n_scales,
+                                           const int32_t* desc, const int64_t* source, const int64_t* order, const int64_t* group_ptr,
+                                           const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k, int wc, int wr, int n_f,
+                                           int n_blocks, int d_out, int dtype, void* dh, void* dzc, void* dzr, void* dweights, void* stream) {
+  int status = check_factored(h, zc, zr, angular, transport, rho, desc, source, n_edges, k, wc, wr, n_f, n_blocks, d_out, n_scales, dtype);
   if (status != GM_OK || n_edges == 0) return status;
   GM_REQUIRE(g && order && group_ptr && group_source && n_groups >= 1, GM_ERR_ARGUMENT, "gm_factored_backward: null pointer");
   GM_REQUIRE((dh || k == 1) && (dzc || wc == 0) && (dzr || wr == 0), GM_ERR_ARGUMENT, "gm_factored_backward: null output");
@@ -578,15 +605,15 @@ extern "C" int gm_factored_backward(const void* g, const int64_t* target, const 
   auto run = [&](auto tag) {
     using T = decltype(tag);
     FArgs<T> a{};
-    a.n_edges = n_edges; a.n_groups = n_groups; a.k = k; a.wc = wc; a.wr = wr; a.n_f = n_f; a.n_blocks = n_blocks; a.d_out = d_out;
+    a.n_edges = n_edges; a.n_groups = n_groups; a.k = k; a.wc = wc; a.wr = wr; a.n_f = n_f; a.n_blocks = n_blocks; a.d_out = d_out; a.n_scales = n_scales;
     a.h = (const T*)h; a.zc = (const T*)zc; a.zr = (const T*)zr; a.angular = (const T*)angular; a.transport = (const T*)transport;
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.g = (const T*)g; a.target = target; a.weights = aggregated ? (const T*)weights : nullptr; a.rows = aggregated ? (const T*)rows : nullptr;
     a.dh = (T*)dh; a.dzc = (T*)dzc; a.dzr = (T*)dzr; a.dweights = aggregated ? (T*)dweights : nullptr;
     // 64 edges per tile; fewer where the packed width is so large that 64 rows of it do not fit shared memory
     int tile = MAX_TILE;
-    while (tile > 8 && BackwardLayout<T>(k, C, n_f, d_out, tile).total * sizeof(T) > 200 * 1024) tile /= 2;
-    const BackwardLayout<T> L(k, C, n_f, d_out, tile);
+    while (tile > 8 && BackwardLayout<T>(k, C, n_f, n_scales, d_out, tile).total * sizeof(T) > 200 * 1024) tile /= 2;
+    const BackwardLayout<T> L(k, C, n_f, n_scales, d_out, tile);
     const size_t smem = (size_t)L.total * sizeof(T);
     const unsigned blocks = (unsigned)(n_groups < (1 << 20) ? n_groups : (1 << 20));
     auto go = [&](auto kernel) {
@@ -595,7 +622,9 @@ extern "C" int gm_factored_backward(const void* g, const int64_t* target, const 
       kernel<<<blocks, FTHREADS, smem, (cudaStream_t)stream>>>(a, C, tile);
       return launch_status("gm_factored_backward");
     };
-    return L.tgroups * ((C + 3) / 4) <= FTHREADS ? go(factored_backward_kernel<T, 1>) : go(factored_backward_kernel<T, 2>);
+    const bool one = L.tgroups * ((C + 3) / 4) <= FTHREADS;
+    if (n_scales) return one ? go(factored_backward_kernel<T, 1, true>) : go(factored_backward_kernel<T, 2, true>);
+    return one ? go(factored_backward_kernel<T, 1, false>) : go(factored_backward_kernel<T, 2, false>);
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }

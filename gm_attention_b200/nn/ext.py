@@ -166,13 +166,16 @@ def _fcheck(condition: bool, message: str) -> None:
 
 
 class FactoredExtension:
-    """``forward``, ``aggregate``, ``backward``, ``backward_aggregated``."""
+    """``forward``, ``aggregate``, ``backward``, ``backward_aggregated``.
+
+    ``scales=True``: ``rho`` is a table ``(n_edges, n_scales)`` and a complex block's power names the column that
+    multiplies its phases, in place of a power of ``rho (n_edges,)``."""
 
     with_cuda = True
 
     @staticmethod
     def _check_common(h: Tensor, zc: Tensor, zr: Tensor, angular: Tensor, transport: Tensor, rho: Tensor, desc: Tensor, source: Tensor,
-                      d_out: int) -> None:
+                      d_out: int, scales: bool) -> None:
         _fcheck(h.dim() == 2 and h.is_contiguous(), "h must be a contiguous (n_edges, k - 1) tensor")
         _fcheck(zc.dim() == 4 and zc.size(3) == 2 and zc.is_contiguous(), "zc must be a contiguous (n_nodes, k, wc, 2) tensor")
         _fcheck(zr.dim() == 3 and zr.is_contiguous(), "zr must be a contiguous (n_nodes, k, wr) tensor")
@@ -181,7 +184,8 @@ class FactoredExtension:
         _fcheck(angular.dim() == 3 and angular.size(2) == 2 and angular.is_contiguous() and angular.size(0) == h.size(0),
                 "angular must be a contiguous (n_edges, n_f, 2) tensor")
         _fcheck(transport.shape == angular.shape and transport.is_contiguous(), "transport must match angular")
-        _fcheck(rho.dim() == 1 and rho.is_contiguous() and rho.size(0) == h.size(0), "rho must be a contiguous (n_edges,) tensor")
+        _fcheck(rho.dim() == 1 + scales and rho.is_contiguous() and rho.size(0) == h.size(0),
+                "rho must be a contiguous (n_edges, n_scales) tensor" if scales else "rho must be a contiguous (n_edges,) tensor")
         _fcheck(desc.dim() == 2 and desc.size(1) == FDESC and desc.dtype == torch.int32 and desc.is_contiguous(),
                 "desc must be a contiguous int32 (n_blocks, 8) tensor")
         _fcheck(source.dim() == 1 and source.size(0) == h.size(0) and source.dtype == torch.int64 and source.is_contiguous(),
@@ -199,16 +203,16 @@ class FactoredExtension:
         return (h.size(0), group_source.size(0), h.size(1) + 1, zc.size(2), zr.size(2), angular.size(1), desc.size(0))
 
     def forward(self, h: Tensor, zc: Tensor, zr: Tensor, angular: Tensor, transport: Tensor, rho: Tensor, desc: Tensor, source: Tensor,
-                order: Tensor, group_ptr: Tensor, group_source: Tensor, d_out: int, max_bm: int) -> Tensor:
-        self._check_common(h, zc, zr, angular, transport, rho, desc, source, d_out)
+                order: Tensor, group_ptr: Tensor, group_source: Tensor, d_out: int, max_bm: int, scales: bool = False) -> Tensor:
+        self._check_common(h, zc, zr, angular, transport, rho, desc, source, d_out, scales)
         out = torch.empty((h.size(0), d_out), dtype=h.dtype, device=h.device)
         _fcheck(1 <= max_bm <= MAX_BM, "max_bm must be in [1, MAX_BM]")
         if h.size(0) == 0:
             return out
         device = _lib.require_cuda(h, order, group_ptr, group_source)
         with torch.cuda.device(device):
-            _lib.call("gm_factored_forward", _lib.ptr(h), _lib.ptr(zc), _lib.ptr(zr), _lib.ptr(angular), _lib.ptr(transport), _lib.ptr(rho),
-                      _lib.ptr(desc), _lib.ptr(source), _lib.ptr(order.contiguous()), _lib.ptr(group_ptr.contiguous()),
+            _lib.call("gm_factored_forward_scaled", _lib.ptr(h), _lib.ptr(zc), _lib.ptr(zr), _lib.ptr(angular), _lib.ptr(transport), _lib.ptr(rho),
+                      rho.size(1) if scales else 0, _lib.ptr(desc), _lib.ptr(source), _lib.ptr(order.contiguous()), _lib.ptr(group_ptr.contiguous()),
                       _lib.ptr(group_source.contiguous()), *self._sizes(h, zc, zr, angular, desc, group_source), int(d_out),
                       _lib.dtype_code(h.dtype), _lib.ptr(out), _lib.stream(device))
         return out
@@ -233,10 +237,10 @@ class FactoredExtension:
 
     def _backward(self, g: Tensor, target: Tensor | None, weights: Tensor | None, rows: Tensor | None, h: Tensor, zc: Tensor, zr: Tensor,
                   angular: Tensor, transport: Tensor, rho: Tensor, desc: Tensor, source: Tensor, order: Tensor, group_ptr: Tensor,
-                  group_source: Tensor) -> list[Tensor]:
+                  group_source: Tensor, scales: bool = False) -> list[Tensor]:
         _fcheck(g.dim() == 2 and g.is_contiguous() and g.dtype == h.dtype and g.device == h.device,
                 "g must be a contiguous (rows, d_out) tensor in h's dtype")
-        self._check_common(h, zc, zr, angular, transport, rho, desc, source, g.size(1))
+        self._check_common(h, zc, zr, angular, transport, rho, desc, source, g.size(1), scales)
         aggregated = target is not None and target.numel() > 0
         if aggregated:
             _fcheck(target.dim() == 1 and target.size(0) == h.size(0) and target.dtype == torch.int64 and target.is_contiguous()
@@ -255,16 +259,17 @@ class FactoredExtension:
             return [dh, dzc, dzr, dweights]
         device = _lib.require_cuda(h, g, order, group_ptr, group_source)
         with torch.cuda.device(device):
-            _lib.call("gm_factored_backward", _lib.ptr(g), _lib.ptr(target) if aggregated else None, _lib.ptr(weights) if aggregated else None,
+            _lib.call("gm_factored_backward_scaled", _lib.ptr(g), _lib.ptr(target) if aggregated else None, _lib.ptr(weights) if aggregated else None,
                       _lib.ptr(rows) if aggregated else None, _lib.ptr(h), _lib.ptr(zc), _lib.ptr(zr), _lib.ptr(angular), _lib.ptr(transport),
-                      _lib.ptr(rho), _lib.ptr(desc), _lib.ptr(source), _lib.ptr(order.contiguous()), _lib.ptr(group_ptr.contiguous()),
+                      _lib.ptr(rho), rho.size(1) if scales else 0, _lib.ptr(desc), _lib.ptr(source), _lib.ptr(order.contiguous()),
+                      _lib.ptr(group_ptr.contiguous()),
                       _lib.ptr(group_source.contiguous()), *self._sizes(h, zc, zr, angular, desc, group_source), g.size(1),
                       _lib.dtype_code(h.dtype), _lib.ptr(dh), _lib.ptr(dzc), _lib.ptr(dzr), _lib.ptr(dweights), _lib.stream(device))
         return [dh, dzc, dzr, dweights]
 
     def backward(self, g: Tensor, h: Tensor, zc: Tensor, zr: Tensor, angular: Tensor, transport: Tensor, rho: Tensor, desc: Tensor,
-                 source: Tensor, order: Tensor, group_ptr: Tensor, group_source: Tensor) -> list[Tensor]:
-        return self._backward(g, None, None, None, h, zc, zr, angular, transport, rho, desc, source, order, group_ptr, group_source)[:3]
+                 source: Tensor, order: Tensor, group_ptr: Tensor, group_source: Tensor, scales: bool = False) -> list[Tensor]:
+        return self._backward(g, None, None, None, h, zc, zr, angular, transport, rho, desc, source, order, group_ptr, group_source, scales)[:3]
 
     def backward_aggregated(self, g: Tensor, target: Tensor, weights: Tensor, rows: Tensor, h: Tensor, zc: Tensor, zr: Tensor,
                             angular: Tensor, transport: Tensor, rho: Tensor, desc: Tensor, source: Tensor, order: Tensor,

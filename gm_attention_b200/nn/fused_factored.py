@@ -253,13 +253,15 @@ def enabled(kernel: Any, x: Any, edges: Any) -> bool:
 
 
 class Factored(torch.autograd.Function):
-    """Rows ``(E, d_out)`` of the factored kernel, differentiable in ``(h, zc, zr)``."""
+    """Rows ``(E, d_out)`` of the factored kernel, differentiable in ``(h, zc, zr)``.  ``scales``: ``rho`` is a table
+    ``(E, n_scales)`` whose columns the descriptors' powers name."""
 
     @staticmethod
     def forward(ctx: Any, h: Tensor, zc: Tensor, zr: Tensor, angular: Tensor, transport: Tensor, rho: Tensor, desc: Tensor, source: Tensor,
-                order: Tensor, group_ptr: Tensor, group_source: Tensor, d_out: int, max_bm: int) -> Tensor:
+                order: Tensor, group_ptr: Tensor, group_source: Tensor, d_out: int, max_bm: int, scales: bool = False) -> Tensor:
         with torch.profiler.record_function("gm::kernel/pairs"):
-            out = extension(True).forward(h, zc, zr, angular, transport, rho, desc, source, order, group_ptr, group_source, d_out, max_bm)
+            out = extension(True).forward(h, zc, zr, angular, transport, rho, desc, source, order, group_ptr, group_source, d_out, max_bm, scales)
+        ctx.scales = scales
         ctx.save_for_backward(h, zc, zr, angular, transport, rho, desc, source, order, group_ptr, group_source)
         return out  # type: ignore[no-any-return]
 
@@ -267,8 +269,8 @@ class Factored(torch.autograd.Function):
     @torch.autograd.function.once_differentiable
     def backward(ctx: Any, grad_out: Tensor) -> tuple:  # type: ignore[override]
         with torch.profiler.record_function("gm::kernel/pairs_backward"):
-            dh, dzc, dzr = extension(True).backward(grad_out.contiguous(), *ctx.saved_tensors)
-        return (dh, dzc, dzr) + (None,) * 10
+            dh, dzc, dzr = extension(True).backward(grad_out.contiguous(), *ctx.saved_tensors, ctx.scales)
+        return (dh, dzc, dzr) + (None,) * 11
 
 
 class FactoredAggregate(torch.autograd.Function):

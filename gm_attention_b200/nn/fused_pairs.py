@@ -286,7 +286,7 @@ def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
     return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.cached_grouping(edges, device) is not None
 
 
-def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term]) -> tuple | None:
+def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term], table: Tensor | None) -> tuple | None:
     """What the factored form needs of this call, or ``None`` where the pair terms serve it: an edge-level or mixed field,
     fewer than 4 edges per node (the node products would not be repaid), phase tables that are not plain per-edge
     ``angular_phases`` / ``transport_phases`` of one width or that want gradients, sizes beyond the factored kernels."""
@@ -318,16 +318,20 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
         return None
     if max((max(abs(b.angular), abs(b.transport)) for b in p.blocks), default=0) >= angular.shape[1]:
         return None
+    scales = hidden.new_ones(n_edges, 1) if table is None else table.detach()  # table None: no block has a scale
+    powers = [b.power for b in p.blocks]
+    if scales.dim() != 2 or scales.shape[0] != n_edges or min(powers) < 0 or max(powers) >= scales.shape[1] or scales.dtype != hidden.dtype or scales.device != hidden.device:
+        return None
     if torch.cuda.is_current_stream_capturing() and not _prepared(kernel, edges, hidden.device):
         return None  # grouping the edges by source and uploading the descriptors synchronise: not while a graph is captured
-    return p, rows, values, angular, transport, n_nodes
+    return p, rows, values, angular, transport, scales, n_nodes
 
 
 def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tuple) -> Any:
     from gm_attention_b200.nn import fused_factored as ff
 
-    p, rows, values, angular, transport, n_nodes = found
-    device, dtype = hidden.device, hidden.dtype
+    p, rows, values, angular, transport, scales, n_nodes = found
+    device = hidden.device
     # the kernels read memory: conjugations and signs that torch has put off are carried out first
     flat = [(torch.view_as_real(v.resolve_conj()) if v.is_complex() else v.resolve_neg()).reshape(n_nodes, -1) for v in values]
     packed = flat[0] if len(flat) == 1 else torch.cat(flat, 1)
@@ -338,12 +342,10 @@ def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tu
     node_desc, desc = tables[str(device)]
     params = [q for head in (kernel.complex_head, kernel.real_head) for q in ((None, None) if head is None else (head.weight, head.bias))]
     zc, zr = NodeProducts.apply(packed, *params, node_desc, hidden.shape[1] + 1, p.wc, p.wr)
-    powers = [b.power for b in p.blocks]
-    rho = kernel._radial_powers(edges.distances)[:, 1].detach().to(dtype).contiguous() if max(powers, default=0) else hidden.new_ones(hidden.shape[0])
     source = edges.source_index.contiguous()
     order, group_ptr, group_source = ff.grouping_for(edges, source).require_nodes(n_nodes)
-    out = ff.Factored.apply(hidden, zc, zr, *(torch.view_as_real(t.resolve_conj().contiguous()) for t in (angular, transport)), rho, desc, source,
-                            order, group_ptr, group_source, p.d_out, p.max_bm)
+    out = ff.Factored.apply(hidden, zc, zr, *(torch.view_as_real(t.resolve_conj().contiguous()) for t in (angular, transport)), scales.resolve_neg().contiguous(),
+                            desc, source, order, group_ptr, group_source, p.d_out, p.max_bm, True)
     slices = kernel.field_type_out.slices()
     orders = sorted(kernel.field_type_out.frequencies, key=lambda m: slices[m].start)
     parts = dict(zip(orders, out.split([slices[m].stop - slices[m].start for m in orders], 1), strict=True))
@@ -387,7 +389,9 @@ def forward_general(kernel: Any, x: Any, edges: Any) -> Any:
     terms = plan(kernel)
     with torch.profiler.record_function("gm::kernel/radial"):
         hidden = _trunk_output(kernel, edges.distances)
-    found = _factored_inputs(kernel, x, edges, hidden, terms)
+    powers = sorted({t.power for t in terms if t.power is not None})
+    table = kernel._radial_powers(edges.distances) if powers else None
+    found = _factored_inputs(kernel, x, edges, hidden, terms, table)
     if found is not None:
         with torch.profiler.record_function("gm::kernel/pairs"):
             return type(x)(kernel.field_type_out, _forward_factored(kernel, x, edges, hidden, found))
@@ -395,9 +399,7 @@ def forward_general(kernel: Any, x: Any, edges: Any) -> Any:
     with torch.profiler.record_function("gm::transport"):
         vectors = _transported_vectors(x, edges, in_frequencies)
     orders = sorted({o for t in terms for o in (t.pre_order, t.post_order) if o is not None})
-    powers = sorted({t.power for t in terms if t.power is not None})
     phases = tuple(edges.angular_harmonic(o).contiguous() for o in orders)
-    table = kernel._radial_powers(edges.distances) if powers else None
     scales = tuple(table[:, p].contiguous() for p in powers)
     where_order, where_power = {o: i for i, o in enumerate(orders)}, {p: i for i, p in enumerate(powers)}
     meta = {

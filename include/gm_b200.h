@@ -252,6 +252,19 @@ int gm_factored_backward(const void* g, const int64_t* target, const void* weigh
                          const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k, int wc, int wr, int n_f,
                          int n_blocks, int d_out, int dtype, void* dh, void* dzc, void* dzr, void* dweights, void* stream);
 
+/* The same with a table of scales in place of the powers: rho (n_edges, n_scales), and a complex block's "power" names the
+ * column (< n_scales) that multiplies its phases; n_scales = 0 is the form above. */
+int gm_factored_forward_scaled(const void* h, const void* zc, const void* zr, const void* angular, const void* transport,
+                               const void* rho, int n_scales, const int32_t* desc, const int64_t* source, const int64_t* order,
+                               const int64_t* group_ptr, const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k, int wc,
+                               int wr, int n_f, int n_blocks, int d_out, int dtype, void* out, void* stream);
+
+int gm_factored_backward_scaled(const void* g, const int64_t* target, const void* weights, const void* rows, const void* h,
+                                const void* zc, const void* zr, const void* angular, const void* transport, const void* rho, int n_scales,
+                                const int32_t* desc, const int64_t* source, const int64_t* order, const int64_t* group_ptr,
+                                const int64_t* group_source, int64_t n_edges, int64_t n_groups, int k, int wc, int wr, int n_f,
+                                int n_blocks, int d_out, int dtype, void* dh, void* dzc, void* dzr, void* dweights, void* stream);
+
 /* ------------------------------------------------------------------------
  * Pair term of the general steerable kernel (drop-in for the reference
  * extension's forward / backward: pairs_cpu.cpp:88-136, arithmetic
