@@ -261,9 +261,11 @@ def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]]]:
     cached = kernel.__dict__.get("_fused_node_blocks")
     if cached is not None:
         return cached  # type: ignore[no-any-return]
+    from gm_attention_b200.fields import FieldType
     from gm_attention_b200.nn import fused_factored
 
-    p = fused_factored.plan_blocks([(t.n, t.m, t.role) for t in terms], kernel.field_type_out,
+    # the rows' layout is this route's own: what the kernel's field type is asked is what the pair terms ask
+    p = fused_factored.plan_blocks([(t.n, t.m, t.role) for t in terms], FieldType({t.m: t.b for t in terms}),
                                    {(t.n, t.m, t.role): t.power for t in terms if t.power is not None})
     offsets, at = {}, 0
     for n in kernel.field_type_in.frequencies:
@@ -302,7 +304,7 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     if n_nodes == n_edges or n_nodes == 0 or n_edges < 4 * n_nodes:
         return None
     angular, transport = getattr(edges, "angular_phases", None), getattr(edges, "transport_phases", None)
-    if angular is None or transport is None or not hasattr(edges, "edge_index") or angular.shape != transport.shape:
+    if angular is None or transport is None or angular.shape != transport.shape or any(not hasattr(edges, x) for x in ("edge_index", "row_ptr")):
         return None
     source = edges.source_index
     if edges.edge_index is not edges.edge_index or ff.version(source) < 0 or source.untyped_storage().data_ptr() != edges.edge_index.untyped_storage().data_ptr():
@@ -346,9 +348,8 @@ def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tu
     order, group_ptr, group_source = ff.grouping_for(edges, source).require_nodes(n_nodes)
     out = ff.Factored.apply(hidden, zc, zr, *(torch.view_as_real(t.resolve_conj().contiguous()) for t in (angular, transport)), scales.resolve_neg().contiguous(),
                             desc, source, order, group_ptr, group_source, p.d_out, p.max_bm, True)
-    slices = kernel.field_type_out.slices()
-    orders = sorted(kernel.field_type_out.frequencies, key=lambda m: slices[m].start)
-    parts = dict(zip(orders, out.split([slices[m].stop - slices[m].start for m in orders], 1), strict=True))
+    widths = {m: kernel.field_type_out.multiplicity(m) * (2 if m else 1) for m in sorted(kernel.field_type_out.frequencies)}
+    parts = dict(zip(widths, out.split(list(widths.values()), 1), strict=True))
     return {m: parts[m].contiguous() if m == 0 else parts[m].contiguous().reshape(hidden.shape[0], -1, 2) for m in kernel.field_type_out.frequencies}
 
 

@@ -689,3 +689,36 @@ def test_node_level_field_uses_the_kernels_radial_table(monkeypatch, dtype):
     assert taken[0] is not None
     for a, b in zip(*results):
         assert rel_err(a.detach().cpu().numpy(), b.detach().cpu().numpy()) < (1e-11 if dtype == torch.float64 else 4e-6)
+
+
+def test_node_level_field_on_a_callers_own_types(monkeypatch):
+    """An edge set without ``row_ptr`` takes the pair terms; field types that know their frequencies and multiplicities
+    only, in any order, take the factored form.  float64, 1e-11 against the pair terms."""
+    from types import SimpleNamespace
+
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float64)
+    names = ("edge_index", "source_index", "n_edges", "distances", "angular_phases", "transport_phases", "max_frequency", "angular_harmonic",
+             "transport_harmonic")
+    bare = SimpleNamespace(**{name: getattr(edges, name) for name in names})
+    kernel = StandInKernel({0: 2, 1: 3}, {0: 2, 1: 1, 2: 2}, cutoff).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev, dtype=torch.float64)
+    coefficients = FeatureField.from_flat(kernel.field_type_in, flat).coefficients
+    multiplicity = {2: 2, 0: 2, 1: 1}
+    kernel.field_type_out = SimpleNamespace(frequencies=tuple(multiplicity), multiplicity=multiplicity.__getitem__)
+    taken = []
+    recognise = fp._factored_inputs
+    monkeypatch.setattr(fp, "_factored_inputs", lambda *a: taken.append(recognise(*a)) or taken[-1])
+    with torch.no_grad():
+        results = [fp.forward_general(kernel, _Field(kernel.field_type_in, coefficients), e).coefficients for e in (edges, bare)]
+    assert [found is not None for found in taken] == [True, False]
+    assert list(results[0]) == list(results[1]) == [2, 0, 1]
+    for m in multiplicity:
+        assert rel_err(results[0][m].cpu().numpy(), results[1][m].cpu().numpy()) < 1e-11
