@@ -215,6 +215,8 @@ class _FusedPairs(torch.autograd.Function):
 
 #: nodes per partial sum of the readout's gradient
 NODE_CHUNK = 128
+#: widest packed node field gm_node_products_* take (its rows are staged in shared memory)
+MAX_NODE_WIDTH = 2048
 
 
 class NodeProducts(torch.autograd.Function):
@@ -313,6 +315,11 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     if angular.dtype != _complex_of(hidden.dtype) or transport.dtype != angular.dtype or angular.requires_grad or transport.requires_grad:
         return None
     if any(v.device != hidden.device or (v.real if v.is_complex() else v).dtype != hidden.dtype for v in (*values, angular, transport)):
+        return None
+    # the pair terms' own bounds: what they refuse is refused on any graph
+    if not 1 <= hidden.shape[1] <= MAX_TRUNK or any(not (1 <= t.a <= MAX_MULT and 1 <= t.b <= MAX_MULT) for t in terms):
+        return None
+    if sum(kernel.field_type_in.multiplicity(n) * (2 if n else 1) for n in frequencies) > MAX_NODE_WIDTH:
         return None
     p, rows = _node_blocks(kernel, terms)
     k = hidden.shape[1] + 1

@@ -722,3 +722,42 @@ def test_node_level_field_on_a_callers_own_types(monkeypatch):
     assert list(results[0]) == list(results[1]) == [2, 0, 1]
     for m in multiplicity:
         assert rel_err(results[0][m].cpu().numpy(), results[1][m].cpu().numpy()) < 1e-11
+
+
+@pytest.mark.parametrize("field_in, field_out, trunk", [({0: 2, 1: 2}, {0: 2, 1: 2}, 17), ({0: 17}, {0: 2}, 8), ({0: 2, 1: 2}, {1: 17}, 8)])
+def test_pair_driver_bounds_do_not_depend_on_the_graph(field_in, field_out, trunk):
+    """Trunks above 16 and multiplicities above 16 are refused for a node-level field as for the same field on the edges."""
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32)
+    kernel = StandInKernel(field_in, field_out, cutoff, trunk=trunk, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    for values in (flat, flat[edges.source_index]):
+        with pytest.raises(RuntimeError, match="must be in 1..16"):
+            fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, values), edges)
+
+
+def test_wide_node_field_takes_the_pair_terms():
+    """A packed input beyond what the node products stage (2048 columns) is served by the pair terms, bit for bit the
+    result on the gathered field."""
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(6, 14, dev)
+    cutoff = 1.9 * math.pi / 6
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=70, dtype=torch.float32)
+    kernel = StandInKernel({n: 16 for n in range(67)}, {0: 1}, cutoff, trunk=2, dtype=torch.float32).to(dev)
+    assert kernel.field_type_in.dimension > fp.MAX_NODE_WIDTH and edges.n_edges >= 4 * lattice.n_nodes
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    with torch.no_grad():
+        node, edge = (fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, v), edges)[0] for v in (flat, flat[edges.source_index]))
+    assert torch.equal(node, edge)
