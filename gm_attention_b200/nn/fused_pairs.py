@@ -258,9 +258,10 @@ class NodeProducts(torch.autograd.Function):
         return (dx, *grads, None, None, None, None)
 
 
-def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]]]:
-    """The factored plan of the kernel's terms and the descriptor rows of their node products (cached on the kernel)."""
-    cached = kernel.__dict__.get("_fused_node_blocks")
+def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]], dict[bool, int] | None]:
+    """The factored plan of the kernel's terms, the descriptor rows of their node products, and the readout rows they read
+    of the real (True) and complex (False) head -- ``None`` where a term's rows are no plain run (cached on the kernel)."""
+    cached = kernel.__dict__.get("_fused_node_plan")
     if cached is not None:
         return cached  # type: ignore[no-any-return]
     from gm_attention_b200.fields import FieldType
@@ -279,8 +280,40 @@ def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]]]:
         t = by_block[b.block]
         operand = 0 if t.flags & U_REAL else (2 if t.flags & CONJ_U else 1)
         rows.append([b.kind, b.z_offset, t.b, t.a, offsets[t.n], operand, t.rows.start or 0, 0])
-    kernel.__dict__["_fused_node_blocks"] = (p, rows)
-    return p, rows
+    needed: dict[bool, int] | None = {}
+    for t in terms:
+        start, width = t.rows.start or 0, t.a * t.b * (2 if t.flags & MATRIX_COMPLEX else 1)
+        if needed is None or start < 0 or t.rows.stop != start + width or t.rows.step not in (None, 1):
+            needed = None
+        else:
+            needed[t.real_head] = max(needed.get(t.real_head, 0), start + width)
+    kernel.__dict__["_fused_node_plan"] = (p, rows, needed)
+    return p, rows, needed
+
+
+def _readouts_fit(kernel: Any, needed: dict[bool, int] | None, hidden: Tensor) -> bool:
+    """Whether both heads hold, in the trunk's dtype and place, the rows their terms read."""
+    if needed is None:
+        return False
+    for real, rows in needed.items():
+        head = kernel.real_head if real else kernel.complex_head
+        weight, bias = getattr(head, "weight", None), getattr(head, "bias", None)
+        if weight is None or weight.dim() != 2 or weight.shape[0] < rows or weight.shape[1] != hidden.shape[1]:
+            return False
+        if bias is not None and bias.shape != weight.shape[:1]:
+            return False
+        if any(t.dtype != hidden.dtype or t.device != hidden.device for t in (weight, bias) if t is not None):
+            return False
+    return True
+
+
+def _field_fits(kernel: Any, frequencies: list[int], values: list[Tensor], n_nodes: int) -> bool:
+    """Whether the coefficients are ``(N, a_0)`` reals and ``(N, a_n)`` complex numbers or ``(N, a_n, 2)`` pairs."""
+    for n, v in zip(frequencies, values, strict=True):
+        pairs = () if n == 0 or v.is_complex() else (2,)
+        if (n == 0 and v.is_complex()) or v.shape != (n_nodes, kernel.field_type_in.multiplicity(n), *pairs):
+            return False
+    return True
 
 
 def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
@@ -300,7 +333,7 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     n_edges = int(edges.n_edges)
     from gm_attention_b200.nn import fused_factored as ff
 
-    if hidden.device.type != "cuda" or hidden.dtype not in (torch.float32, torch.float64) or len(nodes) != 1 or not terms:
+    if hidden.device.type != "cuda" or hidden.dtype not in (torch.float32, torch.float64) or hidden.dim() != 2 or len(nodes) != 1 or not terms:
         return None
     n_nodes = nodes.pop()
     if n_nodes == n_edges or n_nodes == 0 or n_edges < 4 * n_nodes:
@@ -321,7 +354,13 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
         return None
     if sum(kernel.field_type_in.multiplicity(n) * (2 if n else 1) for n in frequencies) > MAX_NODE_WIDTH:
         return None
-    p, rows = _node_blocks(kernel, terms)
+    if not _field_fits(kernel, frequencies, values, n_nodes) or angular.dim() != 2 or len({n_edges, *(t.shape[0] for t in (hidden, angular, source))}) != 1:
+        return None
+    if source.dim() != 1 or source.dtype != torch.int64 or source.device != hidden.device:
+        return None
+    p, rows, needed = _node_blocks(kernel, terms)
+    if not _readouts_fit(kernel, needed, hidden):
+        return None
     k = hidden.shape[1] + 1
     if k > ff.MAX_K or p.d_out > ff.MAX_OUT or p.max_bm > ff.MAX_BM or k * (-(-(2 * p.wc + p.wr) // 4) * 4) > ff.MAX_KC:
         return None

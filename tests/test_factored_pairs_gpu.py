@@ -761,3 +761,48 @@ def test_wide_node_field_takes_the_pair_terms():
     with torch.no_grad():
         node, edge = (fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, v), edges)[0] for v in (flat, flat[edges.source_index]))
     assert torch.equal(node, edge)
+
+
+def test_node_level_route_only_for_tensors_its_kernels_can_read(monkeypatch):
+    """What the route's kernels would read out of range or as other numbers does not take it: readouts with missing rows
+    or columns, of another dtype or place, a field of another shape than the input type's, tables of another length,
+    32-bit sources.  (Judged on the tensors alone: nothing is launched.)"""
+    import dataclasses
+    from types import SimpleNamespace
+
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32)
+    x = FeatureField.from_flat(StandInKernel({0: 2, 1: 3}, {0: 2, 1: 1}, cutoff).field_type_in, torch.randn(lattice.n_nodes, 8, device=dev)).coefficients
+
+    def takes(values=x, over=edges, spoil=None):
+        kernel = StandInKernel({0: 2, 1: 3}, {0: 2, 1: 1}, cutoff, dtype=torch.float32).to(dev)
+        if spoil is not None:
+            spoil(kernel)
+        hidden = fp._trunk_output(kernel, edges.distances)
+        return fp._factored_inputs(kernel, values, over, hidden, fp.plan(kernel), kernel._radial_powers(edges.distances)) is not None
+
+    def replace(head, **parts):
+        def spoil(kernel):
+            old = getattr(kernel, head)
+            del kernel._modules[head]
+            setattr(kernel, head, SimpleNamespace(weight=parts.get("weight", lambda w: w)(old.weight), bias=parts.get("bias", lambda b: b)(old.bias)))
+        return spoil
+
+    assert takes() and takes(spoil=replace("real_head")) and takes(spoil=replace("complex_head", bias=lambda b: None))
+    for head in ("real_head", "complex_head"):
+        for parts in ({"weight": lambda w: w[:-1]}, {"weight": lambda w: w[:, :-1]}, {"weight": lambda w: w.double()}, {"weight": lambda w: w.cpu()},
+                      {"bias": lambda b: b[:-1]}, {"bias": lambda b: b.double()}, {"bias": lambda b: b.cpu()}):
+            assert not takes(spoil=replace(head, **parts)), (head, parts)
+    for values in ({0: x[0][:, :1], 1: x[1]}, {0: x[0], 1: x[1][:, :2]}, {0: x[0], 1: x[1].flatten(1)}, {0: x[0][:-1], 1: x[1]},
+                   {0: torch.complex(x[0], x[0]), 1: x[1]}, {0: x[0].double(), 1: x[1].double()}):
+        assert not takes(values=values)
+    short = {name: getattr(edges, name)[:-1] for name in ("angular_phases", "transport_phases")}
+    assert not takes(over=dataclasses.replace(edges, **short))
+    assert not takes(over=dataclasses.replace(edges, edge_index=edges.edge_index.int()))
