@@ -307,6 +307,14 @@ def _readouts_fit(kernel: Any, needed: dict[bool, int] | None, hidden: Tensor) -
     return True
 
 
+def _products_repaid(n_nodes: int, n_edges: int) -> bool:
+    """Whether a node's products serve enough edges.  Forward and backward, float32, trunk 16, ms as factored form / pair
+    terms: {16, 16} -> {8, 8} on 30 000 nodes 3.53 / 2.71 at 4.9 edges per node, 3.63 / 3.63 at 8.6, 3.81 / 5.95 at 17 (the
+    products bound the factored form there); {2, 2} -> {8, 8} 1.97 / 1.90 at 6.8, 2.20 / 2.64 at 17.  Up to 8 192 nodes both
+    wait for their launches, of which the factored form has fewer: 1.32 / 1.42 at 2.6, 1.33 / 1.73 at 4.8."""
+    return n_edges >= (4 if n_nodes <= 8192 else 10) * n_nodes
+
+
 def _field_fits(kernel: Any, frequencies: list[int], values: list[Tensor], n_nodes: int) -> bool:
     """Whether the coefficients are ``(N, a_0)`` reals and ``(N, a_n)`` complex numbers or ``(N, a_n, 2)`` pairs."""
     for n, v in zip(frequencies, values, strict=True):
@@ -325,7 +333,7 @@ def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
 
 def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term], table: Tensor | None) -> tuple | None:
     """What the factored form needs of this call, or ``None`` where the pair terms serve it: an edge-level or mixed field,
-    fewer than 4 edges per node (the node products would not be repaid), phase tables that are not plain per-edge
+    too few edges per node (:func:`_products_repaid`), phase tables that are not plain per-edge
     ``angular_phases`` / ``transport_phases`` of one width or that want gradients, sizes beyond the factored kernels."""
     frequencies = list(kernel.field_type_in.frequencies)
     values = [x[n] for n in frequencies]
@@ -336,7 +344,7 @@ def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: lis
     if hidden.device.type != "cuda" or hidden.dtype not in (torch.float32, torch.float64) or hidden.dim() != 2 or len(nodes) != 1 or not terms:
         return None
     n_nodes = nodes.pop()
-    if n_nodes == n_edges or n_nodes == 0 or n_edges < 4 * n_nodes:
+    if n_nodes == n_edges or n_nodes == 0 or not _products_repaid(n_nodes, n_edges):
         return None
     angular, transport = getattr(edges, "angular_phases", None), getattr(edges, "transport_phases", None)
     if angular is None or transport is None or angular.shape != transport.shape or any(not hasattr(edges, x) for x in ("edge_index", "row_ptr")):

@@ -170,3 +170,11 @@ def test_groupings_read_by_a_graph_outlive_the_cache(monkeypatch):
     del sets[0]
     find(sets[0])
     assert len(ff._GROUPS) == 3 and not any(kept.captured for kept in ff._GROUPS.values())
+
+
+@pytest.mark.parametrize("n_nodes, n_edges, repaid", [(100, 399, False), (100, 400, True), (8192, 4 * 8192, True), (8193, 4 * 8193, False),
+                                                      (30000, 299_999, False), (30000, 300_000, True)])
+def test_where_the_node_products_are_repaid(n_nodes, n_edges, repaid):
+    from gm_attention_b200.nn import fused_pairs as fp
+
+    assert fp._products_repaid(n_nodes, n_edges) is repaid
