@@ -364,7 +364,8 @@ __global__ void __launch_bounds__(FTHREADS, (SCALED && sizeof(T) == 8 && NP == 1
   T* g_s = base_s + L.g;      // (tile, g_pitch): the edge's output-gradient row
   T* scale_s = base_s + L.scale;
   for (int x = threadIdx.x; x < L.rec; x += FTHREADS) base_s[x] = T(0);  // padding rows and columns are never written again
-  const int col_quads = (C + 3) / 4, patches = L.tgroups * col_quads;
+  // (C = 0: one quad of padding, so that dh and dweights are written)
+  const int col_quads = (max(C, 1) + 3) / 4, patches = L.tgroups * col_quads;
   const int passes = (patches + NP * FTHREADS - 1) / (NP * FTHREADS);
   for (int64_t g0 = blockIdx.x; g0 < a.n_groups; g0 += gridDim.x) {
     const int64_t grp = from_both_ends(g0, a.n_groups);

@@ -228,6 +228,27 @@ def test_factored_sources_without_edges(dtype):
     assert bool((grads[1][empty] == 0).all()) and bool((grads[2][empty] == 0).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_factored_backward_without_columns(dtype):
+    """Blocks of no columns: dh is zero and dweights = <g, row>, whatever the memory held."""
+    from gm_attention_b200.nn import fused_factored as ff
+
+    dev = torch.device("cuda", 0)
+    draw = lambda *shape: torch.randn(*shape, dtype=dtype, device=dev)
+    n, e, k, d_out = 5, 37, 4, 3
+    source, target = torch.arange(e, device=dev) % n, torch.arange(e, device=dev) // 8
+    desc = torch.tensor([[1, 0, 0, 1, 1, 1, 0, 0]], dtype=torch.int32, device=dev)
+    args = (draw(e, k - 1), draw(n, k, 0, 2), draw(n, k, 0), draw(e, 2, 2), draw(e, 2, 2), draw(e), desc, source)
+    g, weights, rows = draw(e, d_out), draw(e), draw(e, d_out)
+    del draw
+    for _ in range(2):  # the second call's outputs come from memory the first one left non-zero
+        scrap = [torch.full((e, k - 1), 7.0, dtype=dtype, device=dev), torch.full((e,), 7.0, dtype=dtype, device=dev)]
+        del scrap
+        dh, _, _, dweights = ff.extension(True).backward_aggregated(g, target, weights, rows, *args, *ff.source_groups(source))
+        assert bool((dh == 0).all())
+        torch.testing.assert_close(dweights, (g[target] * rows).sum(1), rtol=1e-5, atol=1e-6)
+
+
 PAIR_CASES = [
     (3, 2, 5, 2 | 8),          # real block: U_REAL | OUT_REAL
     (4, 8, 16, 1 | 2),         # 0 -> m: MATRIX_COMPLEX | U_REAL
