@@ -11,13 +11,13 @@
 // Forward: one CTA per source node (the caller's grouping order / group_ptr /
 // group_source), Z(j) staged once in shared memory, the source's edges in tiles of
 // 64.  The packed width 2 wc + wr is bounded only by shared memory (the reference
-// stops at 320).
+// stops at 320); what the tiles cannot hold has a form of its own.
 //
 // The edges of a source are scattered over the target-major edge list, so their records (h, both phase rows, rho; the
 // gradient row in the backward) are copied into shared memory element by element, consecutive threads taking consecutive
 // elements of one edge: read by the edge's own thread straight from global memory, each of the ~60 loads of the forward
-// touched 32 lines.  128 x 256 lattice, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4}, trunk 16, float32: forward
-// 1.40 -> 1.36 ms, backward 4.64 -> 2.56 ms.
+// touched 32 lines.  With the register tiles below, on 128 x 256, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4},
+// trunk 16, float32: forward 1.40 -> 1.36 ms, backward 4.64 -> 2.56; sources taken from both ends of the list: 1.30, 2.48.
 //
 // Backward: one CTA per source again, so dZ(j) needs no atomics.  Edges are taken
 // in tiles; the CTA builds its edges' packed rows W(e) = scale * G conj(F) in shared
@@ -35,6 +35,7 @@ constexpr int FDESC = 8;
 constexpr int FTHREADS = 128;
 constexpr int MAX_TILE = 64;       // edges per tile, at most (a power of two; less where shared memory is short)
 constexpr int MAX_OWNED = 64;      // K * C <= 64 * 128 in the backward
+constexpr size_t FSMEM_MOST = 224 * 1024;  // dynamic shared memory a CTA may ask for, beside the static arrays
 constexpr int TP = 5;              // rows t of a dZ patch (4 columns wide)
 
 template <typename T>
@@ -126,6 +127,38 @@ __device__ __forceinline__ void block_factor(const T* rec, int n_f, const int32_
   fr *= s;
   fi *= s;
 }
+// ... from the tables themselves.  (Its own body: one over pointers to the three parts, or over accessors, cost the staged
+// kernels registers and 1 to 6 %.)
+template <bool SCALED, typename T>
+__device__ __forceinline__ void table_factor(const FArgs<T>& a, int64_t e, const int32_t* d, T& fr, T& fi) {
+  const T *angular = a.angular + e * a.n_f * 2, *t = a.transport + e * a.n_f * 2, *scale = a.rho + e * (SCALED ? a.n_scales : 1);
+  fr = T(1);
+  fi = T(0);
+  const int ang = d[3], trn = d[4], power = d[5];
+  if (ang != 0) {
+    const int o = ang < 0 ? -ang : ang;
+    const T pr = angular[2 * o], pi = ang < 0 ? -angular[2 * o + 1] : angular[2 * o + 1];
+    const T nr = fr * pr - fi * pi, ni = fr * pi + fi * pr;
+    fr = nr;
+    fi = ni;
+  }
+  if (trn != 0) {
+    const int o = trn < 0 ? -trn : trn;
+    const T pr = t[2 * o], pi = trn < 0 ? -t[2 * o + 1] : t[2 * o + 1];
+    const T nr = fr * pr - fi * pi, ni = fr * pi + fi * pr;
+    fr = nr;
+    fi = ni;
+  }
+  T s = T(1);
+  if constexpr (SCALED) {
+    s = scale[power];
+  } else {
+    const T r = scale[0];
+    for (int x = 0; x < power; ++x) s *= r;
+  }
+  fr *= s;
+  fi *= s;
+}
 
 // Z(j) of one node into shared memory: row t = [zc (wc, 2) | zr (wr)], `pitch` elements apart; asynchronous.
 template <typename T>
@@ -164,8 +197,8 @@ __device__ __forceinline__ void store4(T* p, const T (&v)[4]) {  // 16-byte alig
 // Forward, per tile of a source's edges: U(c, e) = sum_t h~_t(e) Z_t(c) as a matrix product in register tiles of 4 edges x
 // 4 packed columns (two 16-byte reads for 16 multiply-adds), the blocks' factors F(b, e), then a thread per (edge, output
 // column) adds up its blocks.  Everything indexed by edge has the edge fastest, so a warp's 32 edges read one line.
-// (A thread per edge that walked the blocks with all of Z broadcast measured 1.40 ms, 1.62 with staged records; this form
-// 1.36.  What is left is issue: a third of the instructions are multiply-adds, the rest mostly the factors' phases and powers.)
+// (A thread per edge that walked the blocks with all of Z broadcast measured 1.40 ms, 1.62 with staged records alone; this
+// form 1.36.)
 template <typename T>
 struct ForwardLayout {  // shared memory, in elements of T
   int tile, pitch, cols, e_pitch, rec_pitch, row_pitch;
@@ -305,6 +338,76 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_kernel(FArgs<T> a, 
   }
 }
 
+// The forward where the tiled form does not fit: packed rows of thousands of columns over a short trunk (k = 1: 4 460 in
+// float32; U takes more room than Z there), phase tables of hundreds of orders.  A thread per edge walks the blocks, all
+// threads reading the same address of Z(j); phases come straight from the tables.  571 us against 312 for the tiled form on
+// 64 x 128, radius 3 pi / 64, 13 blocks to {4, 4, 4}, trunk 16, float32, so only what that form cannot hold comes here.
+template <typename T, bool SCALED>
+__global__ void __launch_bounds__(FTHREADS) factored_forward_wide_kernel(FArgs<T> a, int pitch) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  const int wc2 = 2 * a.wc, nc = a.k * wc2, nr = a.k * a.wr;
+  T* zc_s = reinterpret_cast<T*>(raw);  // (k, wc, 2)
+  T* zr_s = zc_s + nc;                  // (k, wr)
+  T* rows_s = zr_s + (nr + 3) / 4 * 4;  // (FTHREADS, pitch)
+  T* row = rows_s + (size_t)threadIdx.x * pitch;
+  for (int64_t g0 = blockIdx.x; g0 < a.n_groups; g0 += gridDim.x) {
+    const int64_t grp = from_both_ends(g0, a.n_groups);
+    const int64_t j = a.group_source[grp], first = a.group_ptr[grp], last = a.group_ptr[grp + 1];
+    if (first == last) continue;
+    __syncthreads();
+    for (int x = threadIdx.x; x < nc; x += FTHREADS) zc_s[x] = a.zc[j * nc + x];
+    for (int x = threadIdx.x; x < nr; x += FTHREADS) zr_s[x] = a.zr[j * nr + x];
+    __syncthreads();
+    for (int64_t x0 = first; x0 < last; x0 += FTHREADS) {
+      const int n = (int)min((int64_t)FTHREADS, last - x0);
+      if ((int)threadIdx.x < n) {
+        const int64_t e = a.order[x0 + threadIdx.x];
+        T hh[FMAX_K];
+        hh[0] = T(1);
+#pragma unroll
+        for (int t = 1; t < FMAX_K; ++t) hh[t] = t < a.k ? a.h[e * (a.k - 1) + t - 1] : T(0);
+        for (int c = 0; c < a.d_out; ++c) row[c] = T(0);
+        for (int b = 0; b < a.n_blocks; ++b) {
+          const int32_t* d = a.desc + b * FDESC;
+          const int zoff = d[1], bm = d[2];
+          T* out = row + d[6];
+          if (d[0] == 0) {
+            for (int c = 0; c < bm; ++c) {
+              T s = T(0);
+#pragma unroll
+              for (int t = 0; t < FMAX_K; ++t)
+                if (t < a.k) s += hh[t] * zr_s[t * a.wr + zoff + c];
+              out[c] += s;
+            }
+            continue;
+          }
+          T fr, fi;
+          table_factor<SCALED>(a, e, d, fr, fi);
+          for (int c = 0; c < bm; ++c) {
+            T ur = T(0), ui = T(0);
+#pragma unroll
+            for (int t = 0; t < FMAX_K; ++t)
+              if (t < a.k) {
+                ur += hh[t] * zc_s[t * wc2 + 2 * (zoff + c)];
+                ui += hh[t] * zc_s[t * wc2 + 2 * (zoff + c) + 1];
+              }
+            const T vr = fr * ur - fi * ui, vi = fr * ui + fi * ur;
+            if (d[7] != 0) {
+              out[c] += vr;
+            } else {
+              out[2 * c] += vr;
+              out[2 * c + 1] += vi;
+            }
+          }
+        }
+      }
+      __syncthreads();
+      for_rows(n, a.d_out, [&](int r, int c) { a.out[a.order[x0 + r] * a.d_out + c] = rows_s[r * pitch + c]; });
+      __syncthreads();
+    }
+  }
+}
+
 // out_i = sum over the target's edges of w_e * row_e  (factored.h:337-347): a warp per target, lanes over columns.
 template <typename T>
 __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict__ weights, const int64_t* __restrict__ row_ptr,
@@ -327,14 +430,14 @@ template <typename T>
 struct BackwardLayout {  // shared memory, in elements of T
   int pitch, quads, tgroups, h_pitch, rec_pitch, g_pitch, tile;
   int z, w, h, rec, g, scale, total;
-  __host__ __device__ BackwardLayout(int k, int C, int n_f, int n_scales, int d_out, int tile_) {
+  __host__ __device__ BackwardLayout(int k, int C, int n_f, int n_scales, int d_out, int tile_, bool staged) {
     const int vecs = (C + 3) / 4;
     tile = tile_;
     pitch = 4 * (vecs | 1);
     quads = (k - 1 + 3) / 4;           // groups of 4 trunk rows t = 1 ..
     tgroups = (k + TP - 1) / TP;
     h_pitch = tile + 4;                // h~ transposed: (t, edge)
-    rec_pitch = record_pitch(n_f, n_scales);
+    rec_pitch = staged ? record_pitch(n_f, n_scales) : 0;
     g_pitch = d_out | 1;
     z = 0;
     const int z_rows = 1 + 4 * quads;
@@ -347,14 +450,15 @@ struct BackwardLayout {  // shared memory, in elements of T
   }
 };
 
-// NP: dZ patches per thread and pass over the source's edges (wider kernels take several passes)
+// NP: dZ patches per thread and pass over the source's edges (wider kernels take several passes).  STAGED: the edges'
+// records go through shared memory; phase tables of hundreds of orders leave no room for them and are read where they are.
 // (float64 with one patch: four CTAs' registers suffice without spills; left to itself the compiler took 168 for the SCALED form
 // and 64 x 128, {2, 2} -> {2, 2}, trunk 8 went from 233 to 291 us)
-template <typename T, int NP, bool SCALED>
+template <typename T, int NP, bool STAGED, bool SCALED>
 __global__ void __launch_bounds__(FTHREADS, (SCALED && sizeof(T) == 8 && NP == 1 ? 4 : 0)) factored_backward_kernel(FArgs<T> a, int C, int tile) {
   extern __shared__ __align__(16) unsigned char raw[];
   __shared__ int64_t edges_s[MAX_TILE], g_rows_s[MAX_TILE];  // the tile's edges, and the rows of g that reach them
-  const BackwardLayout<T> L(a.k, C, a.n_f, SCALED ? a.n_scales : 0, a.d_out, tile);
+  const BackwardLayout<T> L(a.k, C, a.n_f, SCALED ? a.n_scales : 0, a.d_out, tile, STAGED);
   const int K = a.k, wc2 = 2 * a.wc, pitch = L.pitch;
   T* base_s = reinterpret_cast<T*>(raw);
   T* z_s = base_s + L.z;      // (1 + 4 quads, pitch): packed per t as [zc (wc, 2) | zr (wr) | 0]
@@ -390,7 +494,7 @@ __global__ void __launch_bounds__(FTHREADS, (SCALED && sizeof(T) == 8 && NP == 1
           g_rows_s[threadIdx.x] = a.target ? a.target[e] : e;
         }
         __syncthreads();
-        stage_records<SCALED>(a, edges_s, n_tile, rec_s);
+        if constexpr (STAGED) stage_records<SCALED>(a, edges_s, n_tile, rec_s);
         stage_rows(g_s, L.g_pitch, a.g, a.d_out, n_tile, g_rows_s);
         for_rows(n_tile, K - 1, [&](int le, int t) { copy_async(h_s + (t + 1) * L.h_pitch + le, a.h + edges_s[le] * (K - 1) + t); });
         // edges beyond the tile's end (their h~ multiplies whatever W rows an earlier tile left): zero
@@ -416,7 +520,8 @@ __global__ void __launch_bounds__(FTHREADS, (SCALED && sizeof(T) == 8 && NP == 1
             for (int c = 0; c < bm; ++c) w[wc2 + zoff + c] = scale * g[c];
           } else {
             T fr, fi;
-            block_factor<SCALED>(rec_s + le * L.rec_pitch, a.n_f, d, fr, fi);
+            if constexpr (STAGED) block_factor<SCALED>(rec_s + le * L.rec_pitch, a.n_f, d, fr, fi);
+            else table_factor<SCALED>(a, edges_s[le], d, fr, fi);
             for (int c = 0; c < bm; ++c) {
               const T gr = scale * (take_real ? g[c] : g[2 * c]);
               const T gi = take_real ? T(0) : scale * g[2 * c + 1];
@@ -555,14 +660,20 @@ extern "C" int gm_factored_forward_scaled(const void* h, const void* zc, const v
     // 64 edges per tile; fewer where the packed width or the phase tables leave no room for them
     int tile = MAX_TILE;
     while (tile > 8 && ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra > 200 * 1024) tile /= 2;
-    const size_t smem = ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra;
+    size_t smem = ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra;
     const int64_t cap = (int64_t)sm_count() * 16;  // the CTAs stride the sources: the column list is built once per CTA
-    auto go = [&](auto kernel) {
+    const unsigned blocks = (unsigned)(n_groups < cap ? n_groups : cap);
+    auto go = [&](auto kernel, int x) {
       const int st = allow_smem(kernel, smem, "gm_factored_forward");
-      if (st == GM_OK) kernel<<<(unsigned)(n_groups < cap ? n_groups : cap), FTHREADS, smem, (cudaStream_t)stream>>>(a, tile);
+      if (st == GM_OK) kernel<<<blocks, FTHREADS, smem, (cudaStream_t)stream>>>(a, x);
       return st == GM_OK ? launch_status("gm_factored_forward") : st;
     };
-    return n_scales ? go(factored_forward_kernel<T, true>) : go(factored_forward_kernel<T, false>);
+    if (smem > FSMEM_MOST) {
+      const int pitch = d_out | 1;  // odd: no bank conflicts between the threads' rows
+      smem = ((size_t)k * 2 * wc + ((size_t)k * wr + 3) / 4 * 4 + (size_t)FTHREADS * pitch) * sizeof(T);
+      return n_scales ? go(factored_forward_wide_kernel<T, true>, pitch) : go(factored_forward_wide_kernel<T, false>, pitch);
+    }
+    return n_scales ? go(factored_forward_kernel<T, true>, tile) : go(factored_forward_kernel<T, false>, tile);
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }
@@ -613,8 +724,10 @@ extern "C" int gm_factored_backward_scaled(const void* g, const int64_t* target,
     a.dh = (T*)dh; a.dzc = (T*)dzc; a.dzr = (T*)dzr; a.dweights = aggregated ? (T*)dweights : nullptr;
     // 64 edges per tile; fewer where the packed width is so large that 64 rows of it do not fit shared memory
     int tile = MAX_TILE;
-    while (tile > 8 && BackwardLayout<T>(k, C, n_f, n_scales, d_out, tile).total * sizeof(T) > 200 * 1024) tile /= 2;
-    const BackwardLayout<T> L(k, C, n_f, n_scales, d_out, tile);
+    auto layout = [&](bool staged) { return BackwardLayout<T>(k, C, n_f, n_scales, d_out, tile, staged); };
+    while (tile > 8 && layout(true).total * sizeof(T) > 200 * 1024) tile /= 2;
+    const bool staged = layout(true).total * sizeof(T) <= FSMEM_MOST;
+    const BackwardLayout<T> L = layout(staged);
     const size_t smem = (size_t)L.total * sizeof(T);
     const unsigned blocks = (unsigned)(n_groups < (1 << 20) ? n_groups : (1 << 20));
     auto go = [&](auto kernel) {
@@ -624,8 +737,12 @@ extern "C" int gm_factored_backward_scaled(const void* g, const int64_t* target,
       return launch_status("gm_factored_backward");
     };
     const bool one = L.tgroups * ((C + 3) / 4) <= FTHREADS;
-    if (n_scales) return one ? go(factored_backward_kernel<T, 1, true>) : go(factored_backward_kernel<T, 2, true>);
-    return one ? go(factored_backward_kernel<T, 1, false>) : go(factored_backward_kernel<T, 2, false>);
+    auto form = [&](auto scaled) {
+      constexpr bool SC = decltype(scaled)::value;
+      if (staged) return one ? go(factored_backward_kernel<T, 1, true, SC>) : go(factored_backward_kernel<T, 2, true, SC>);
+      return one ? go(factored_backward_kernel<T, 1, false, SC>) : go(factored_backward_kernel<T, 2, false, SC>);
+    };
+    return n_scales ? form(std::true_type{}) : form(std::false_type{});
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }

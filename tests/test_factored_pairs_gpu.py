@@ -249,6 +249,39 @@ def test_factored_backward_without_columns(dtype):
         torch.testing.assert_close(dweights, (g[target] * rows).sum(1), rtol=1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("k, blocks, n_f, backward", [
+    (1, 127, 4, False),   # 8 128 packed columns without a trunk
+    (2, 63, 4, False),    # 4 032 over a trunk of one
+    (4, 32, 4, False),    # 2 048 over a trunk of three: the tiled form holds the float32 one only
+    (5, 2, 2000, True),   # phase tables of 2 000 orders, most of them unused
+])
+def test_factored_sizes_beyond_the_tiled_kernels(k, blocks, n_f, backward, dtype):
+    """Rows (and gradients, where the backward's own buffers fit) of sizes whose tiles outgrow shared memory, against the
+    numpy restatement: float64 1e-10, float32 1e-5 of each tensor's magnitude (sums of up to 127 blocks x 4 terms)."""
+    from gm_attention_b200.nn import fused_factored as ff
+    from oracle import ops_np
+
+    rng = np.random.default_rng(11)
+    width, n, e = 32, 3, 150
+    desc = np.array([[1, width * i, width, (i % 3) + n_f - 4, -(i % 2), i % 4, 0, 0] for i in range(blocks)], np.int32)
+    draw = lambda *shape: rng.standard_normal(shape).astype(dtype)
+    h, zc, zr, rho, g = draw(e, k - 1), draw(n, k, width * blocks, 2), draw(n, k, 0), rng.uniform(0.1, 1.0, e).astype(dtype), draw(e, 2 * width)
+    phase = np.exp(1j * rng.uniform(0, 6.28, (2, e, 1)) * np.arange(n_f))
+    angular, transport = (np.stack([x.real, x.imag], -1).astype(dtype) for x in phase)
+    source = rng.integers(0, n, e)
+    args = (h, zc, zr, angular, transport, rho, desc, source)
+    groups = ff.source_groups(cuda(source))
+    ext = ff.extension(True)
+    bound = 1e-10 if dtype == np.float64 else 1e-5
+    wide = [x.astype(np.float64) if x.dtype == np.float32 else x for x in args]
+    rows = ext.forward(*map(cuda, args), *groups, 2 * width, width)
+    assert rel_err(rows.cpu().numpy(), ops_np.factored_forward(*wide, 2 * width)) < bound
+    if backward:
+        for got, want in zip(ext.backward(cuda(g), *map(cuda, args), *groups), ops_np.factored_backward(g.astype(np.float64), *wide)):
+            assert got.numel() == 0 or rel_err(got.cpu().numpy(), want) < bound
+
+
 PAIR_CASES = [
     (3, 2, 5, 2 | 8),          # real block: U_REAL | OUT_REAL
     (4, 8, 16, 1 | 2),         # 0 -> m: MATRIX_COMPLEX | U_REAL
