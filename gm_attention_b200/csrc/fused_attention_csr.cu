@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
       const C* tau = a.transport + e * a.orders * 2;
       C part = C(0), dpart = C(0);
       C tkr[NS], tki[NS];
-  #pragma unroll
+#pragma unroll
       for (int t = 0; t < NS; ++t) {
         tkr[t] = tki[t] = C(0);
         if (col[t] >= 0) {
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
       const C ds = a.scale * p * (dpart - delta);
       A* dk_j = dk + j * a.D;
       A* dv_j = dv + j * a.D;
-  #pragma unroll
+#pragma unroll
       for (int t = 0; t < NS; ++t) {
         if (col[t] >= 0) {
           const int n = a.plan.order[t];
@@ -284,7 +284,10 @@ __global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
       }
     }
   };
-  if (pairs_aligned<S, NS>(a, col, a.k, a.v)) walk(std::true_type{});
+  // 16 slots of float64 leave no registers for two walks in one kernel (988 bytes of spill stores against 420; 4 236 us
+  // against 4 115 on 6 000 points, batch 2, 8 heads of 16 x (m <= 3); at 8 slots the vector form wins, 1 817 against 1 837)
+  if constexpr (std::is_same<S, double>::value && NS > 8) walk(std::false_type{});
+  else if (pairs_aligned<S, NS>(a, col, a.k, a.v)) walk(std::true_type{});
   else walk(std::false_type{});
   S* dq_i = a.dq + (base + i) * a.D;
 #pragma unroll
