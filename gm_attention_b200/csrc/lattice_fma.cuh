@@ -94,7 +94,11 @@ struct Tile {
   static constexpr int STATE = (MODE == MODE_FWD ? 4 : MODE == MODE_BWD_T ? 3 : 4) * SLICE + (MODE == MODE_FWD ? 1 : 2) * SLICE;
   // (pass T at 8 x (m <= 3): 202 registers, two CTAs 2.20 ms; held to 168, three CTAs 2.10 ms; the forward held to 168 loses:
   // 1.72 against 2.09 ms, pass S too: 2.38 against 3.57 ms)
-  static constexpr int CTAS = STATE <= 72 ? 4 : STATE <= (MODE == MODE_BWD_T ? 140 : 124) ? 3 : 2;
+  static constexpr int BY_STATE = STATE <= 72 ? 4 : STATE <= (MODE == MODE_BWD_T ? 140 : 124) ? 3 : 2;
+  // ... and no more than shared memory admits (228 KB per SM; 1.5 KB of a CTA's are the system's and the row pairs'):
+  // registers held down for a CTA that cannot come would only cost
+  static constexpr int BY_SMEM = 228 * 1024 / (NBUF * STAGE + 1536);
+  static constexpr int CTAS = BY_STATE < BY_SMEM ? BY_STATE : BY_SMEM;
   static __device__ __forceinline__ int idx(int p) { return TT == 2 ? (p >> 1) + (p & 1) * HALF : p; }
 };
 
