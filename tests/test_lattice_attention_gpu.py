@@ -56,27 +56,41 @@ def test_lattice_matches_oracle_float32(case):
         assert_close(a.cpu().numpy(), b, 1e-5, 1e-5 * max(1.0, np.abs(b).max()), name)
 
 
-@pytest.mark.parametrize("head", [{0: 1}, {0: 16, 1: 2}, {1: 3, 2: 3, 3: 3, 4: 3}, {0: 5, 1: 5, 2: 5}, {0: 7, 1: 7}, {0: 9, 1: 9, 2: 9},
-                                  {0: 13, 1: 13}, {0: 16, 1: 16, 2: 16, 3: 16, 4: 16}])
-@pytest.mark.parametrize("shape", [(6, 14, 2.0, 1, 1), (4, 320, 1.6, 2, 4)])
+# one head layout or more per tile: (copies per lane, lanes per owner) follow the larger multiplicity, then the number of frequencies
+LAYOUTS = [
+    {0: 1}, {0: 4, 1: 3, 2: 3}, {0: 2, 1: 4, 2: 4, 3: 4}, {1: 3, 2: 3, 3: 3, 4: 3},               # 4 x 1
+    {0: 6, 1: 5}, {0: 5, 1: 5, 2: 5}, {1: 6, 2: 6, 3: 6}, {0: 5, 1: 6, 2: 6, 3: 6, 4: 6},          # 3 x 2
+    {0: 7, 1: 7}, {0: 8, 1: 7, 2: 7}, {0: 7, 1: 8, 2: 8, 3: 8}, {1: 7, 2: 7, 3: 7, 4: 7},          # 4 x 2
+    {0: 12, 1: 11}, {0: 9, 1: 9, 2: 9}, {0: 10, 1: 9, 2: 9, 3: 9}, {1: 12, 2: 12, 3: 12, 4: 12},   # 3 x 4
+    {0: 16, 1: 2}, {0: 13, 1: 13}, {0: 15, 1: 14, 2: 14}, {0: 16, 1: 13, 2: 13, 3: 13}, {0: 16, 1: 16, 2: 16, 3: 16, 4: 16},  # 4 x 4
+]
+
+
+@pytest.mark.parametrize("head", LAYOUTS)
+@pytest.mark.parametrize("shape", [(6, 14, 2.0, 1, 1), (4, 320, 1.6, 2, 4), (4, 320, 1.6, 2, 32)])
 def test_lattice_float32_layouts(head, shape):
-    """Every (copies per lane, lanes per owner, frequencies) tile, ragged runs padded with zeros; one shape whose neighbours
-    are split over eight lanes and whose tile outgrows the lattice row, one (82 k to 330 k owners x lanes) with none to two
-    lanes per owner, several stages per window and a tile remainder.  Float32 against the oracle on the float32 tables,
-    tolerances as above."""
+    """Every (copies per lane, lanes per owner, frequencies) tile, ragged runs padded with zeros, on three shapes: one whose
+    neighbours are split over eight lanes and whose tile outgrows the lattice row; one of 10 240 owners (several stages per
+    window, a tile remainder), split over 8 / 4 / 2 lanes in the forward and 4 / 2 / 1 in the backward at 1 / 2 / 4 lanes per owner;
+    and one of 81 920, where nothing is split (148 SMs x 256 threads of owners' lanes are, with two owners a lane, 75 776 owners).
+    Float32 against the oracle on the float32 tables for the last sample, tolerances as above."""
     from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
 
     nlat, nlon, reach, heads, batch = shape
     c = make_case(nlat, nlon, reach * math.pi / nlat, head, heads, dtype=np.float32)
-    q, k, v, g = seeded((batch * c.n_nodes, c.width), 56, np.float32, 4)
+    q, k, v, g = seeded((c.n_nodes, c.width), 56, np.float32, 4)
     _, lat = tables_for(c)
-    Q, K, V, G = cuda(q), cuda(k), cuda(v), cuda(g)
+    sample = slice((batch - 1) * c.n_nodes, batch * c.n_nodes)
+    generator = torch.Generator(device="cuda").manual_seed(57)
+    others = [torch.randn(batch * c.n_nodes, c.width, device="cuda", generator=generator) for _ in range(4)]
+    for field, values in zip(others, (q, k, v, g)):
+        field[sample] = cuda(values)
+    Q, K, V, G = others
     out, lse = lattice_attention_forward(Q, K, V, lat)
     got = lattice_attention_backward(G, Q, K, V, out, lse, lat)
-    sample = slice((batch - 1) * c.n_nodes, batch * c.n_nodes)
     args = (c.transport, c.bias, c.inside, c.desc, c.row_ptr, c.source, c.heads, c.scale, 1)
-    want = O.attention_forward(q[sample], k[sample], v[sample], *args)
-    grads = O.attention_backward(g[sample], q[sample], k[sample], v[sample], *args)
+    want = O.attention_forward(q, k, v, *args)
+    grads = O.attention_backward(g, q, k, v, *args)
     assert_close(out[sample].cpu().numpy(), want, 1e-5, 1e-6 * max(1.0, np.abs(want).max()), "out")
     for name, a, b in zip(("dq", "dk", "dv"), got, grads):
         assert_close(a[sample].cpu().numpy(), b, 1e-5, 1e-5 * max(1.0, np.abs(b).max()), name)
