@@ -369,10 +369,12 @@ DRIVER_CASES = [
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 @pytest.mark.parametrize("field_in, field_out, bias", DRIVER_CASES)
-def test_pairs_driver_matches_the_pair_loop(field_in, field_out, bias, dtype):
-    """``forward_general`` (one launch per term, blocked readout gradient) against the plain-PyTorch pair loop on the
-    same device: values and every gradient (input field, trunk, both heads), the logic of the reference's
-    ``tests/nn/test_fused_pairs.py:73-93``.  float64 1e-11 / 1e-10; float32 1e-5 relative to the tensor's magnitude."""
+@pytest.mark.parametrize("level", ["node", "edge"])
+def test_pairs_driver_matches_the_pair_loop(monkeypatch, level, field_in, field_out, bias, dtype):
+    """``forward_general`` against the plain-PyTorch pair loop on the same device, on a node field (the factored form) and
+    on the field gathered onto the edges (one launch per term, blocked readout gradient): values and every gradient (input
+    field, trunk, both heads), the logic of the reference's ``tests/nn/test_fused_pairs.py:73-93``.  float64 1e-11 / 1e-10;
+    float32 1e-5 relative to the tensor's magnitude."""
     from gm_attention_b200.fields import FeatureField
     from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
     from gm_attention_b200.nn import fused_pairs as fp
@@ -386,15 +388,20 @@ def test_pairs_driver_matches_the_pair_loop(field_in, field_out, bias, dtype):
     kernel = StandInKernel(field_in, field_out, cutoff, trunk=16, bias=bias, dtype=dtype).to(dev)
     flat0 = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, generator=torch.Generator().manual_seed(5), dtype=dtype).to(dev)
 
+    taken = []
+    recognise = fp._factored_inputs
+    monkeypatch.setattr(fp, "_factored_inputs", lambda *a: taken.append(recognise(*a)) or taken[-1])
+
     def run(fused: bool):
         flat = flat0.clone().requires_grad_(True)
-        x = FeatureField.from_flat(kernel.field_type_in, flat)
+        x = FeatureField.from_flat(kernel.field_type_in, flat if level == "node" else flat.index_select(0, edges.source_index))
         out = fp.forward_general(kernel, x, edges).coefficients if fused else kernel.pair_loop(x, edges)
         loss = sum((out[m] * torch.linspace(0.1, 1.0, out[m].numel(), dtype=dtype, device=dev).reshape(out[m].shape)).sum() for m in out)
         return {m: v.detach() for m, v in out.items()}, [g.detach() for g in torch.autograd.grad(loss, [flat, *kernel.parameters()])]
 
     y_plain, g_plain = run(False)
     y_fused, g_fused = run(True)
+    assert [found is not None for found in taken] == [level == "node"]
     tol_y, tol_g = (1e-11, 1e-10) if dtype == torch.float64 else (1e-5, 1e-5)
     for m in y_plain:
         scale = max(1.0, float(y_plain[m].abs().max()))
