@@ -6,15 +6,15 @@
 // w = (r/c)^{2n} e^{2 i n phi}, and summed with the edge's aggregation weight.  On a lattice whose frames turn with the
 // longitude every one of those quantities depends on (target row, source row, longitude offset) only, and
 // z -> A z + w B conj(z) is a real-linear map of the plane, so the whole edge collapses into ONE real 2 x 2 matrix per
-// (table entry, complex copy) and one real factor per (entry, scalar channel); the caller folds the coefficients into
-// that table (gm_attention_b200/nn/lattice_depthwise.py: fold; plain tensor algebra on ~45 000 entries, differentiable), and the
-// kernels here are
+// (table entry, complex copy) and one real factor per (entry, scalar channel).  The kernels here are
 //
+//   fold        the entries' coefficients, phases and weights -> that table, and its gradient -> the coefficients'
+//               (gm_attention_b200/nn/lattice_depthwise.py: FoldTable; fold there is the same in tensor algebra)
 //   apply       y[i, l] = sum over entries (j, d) of row i   M[entry] x[j, l + lo + d]      (forward; with the transposed
 //               windows and M^T it is the gradient with respect to the node field)
 //   table_grad  dM[entry] = sum over longitudes l and samples  dy[i, l] (x) x[j, l + lo + d]
 //
-// Both are FMA-bound, not HBM-bound (4 multiply-adds per complex copy, edge and sample against 0.01 bytes of compulsory
+// apply and table_grad are FMA-bound, not HBM-bound (4 multiply-adds per complex copy, edge and sample against 0.01 bytes of compulsory
 // traffic), and neither has a contraction over channels, so there is nothing for the tensor cores here.  A thread owns
 // one item -- a complex copy, or a pair of scalar channels -- so a warp reads 32 neighbouring items of a node as one
 // 128-byte line; it keeps 8 longitudes x 2 samples of accumulators in registers and slides a register window of 8
@@ -27,7 +27,7 @@ namespace gmb {
 namespace {
 
 constexpr int LON = 8;  // longitudes (apply) / longitude offsets (table_grad) per thread
-constexpr int THREADS = 160;  // at most; three CTAs per SM (136 registers per thread); more items than threads are looped over
+constexpr int THREADS = 160;  // at most; three CTAs per SM (128 registers per thread); more items than threads are looped over
 
 struct ConvArgs {
   const void* x;        // (batch, rows * nlon, width) node field
@@ -514,7 +514,7 @@ __global__ void __launch_bounds__(128) conv_fold_kernel(const FoldArgs a) {
 }
 
 // Tiles, offsets per stage and samples per thread of the staged apply kernel; returns the samples, 0 where it cannot run.
-// Two samples and two CTAs of 320 threads per SM (102 registers) measured 4.5 ms against 4.7 for four samples and one CTA,
+// Two samples and two CTAs of 320 threads per SM (88 to 95 registers) measured 4.5 ms against 4.7 for four samples and one CTA,
 // 5.8 to 6.0 for CTAs of one tile (256 x 512, batch 4, 64 x (m <= 2), bf16).  A stage should hold the equator's windows
 // whole: where half of the shared memory holds fewer than 8 offsets (float32 rows of 320 columns: 3) a CTA takes all of it.
 // Tiles: as many as 320 threads take, fewer while the launch has less than two CTAs per SM (a small lattice waits for

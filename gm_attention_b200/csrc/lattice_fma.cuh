@@ -22,7 +22,7 @@
 // The neighbour rows of one lattice row are copied by cp.async, all of a stage in flight together, into 16-byte chunks
 // laid out [chunk][position]: lanes of consecutive owners then read consecutive 16-byte words, without bank conflicts.
 // Ragged heads (copies not a multiple of C) are padded with zeros there, so every layout runs the same inner loop.
-// The forward has one buffer (its 128 owners x 2 fields fill it; three CTAs per SM overlap copy and compute), the
+// The forward has one buffer (its 128 owners x 2 fields fill it; the SM's other CTAs compute while one copies), the
 // backward passes two.  On 128 x 256, batch 4, 4 heads of 8 x (m <= 3), float32, the layer's training pass measured
 // 13.06 ms with staging by a loop of dependent loads and 4 / 8 lanes per owner, and 6.2 ms in this form (1.7 + 2.1 + 2.4).
 // Issue slots are 42 % busy: two or three CTAs of 4 warps are what registers and shared memory allow, and 7 to 9 steps per
@@ -96,7 +96,8 @@ struct Tile {
   // 1.72 against 2.09 ms, pass S too: 2.38 against 3.57 ms)
   static constexpr int BY_STATE = STATE <= 72 ? 4 : STATE <= (MODE == MODE_BWD_T ? 140 : 124) ? 3 : 2;
   // ... and no more than shared memory admits (228 KB per SM; 1.5 KB of a CTA's are the system's and the row pairs'):
-  // registers held down for a CTA that cannot come would only cost
+  // registers held down for a CTA that cannot come only cost (pass T of 16 x 3 copies x frequencies held to 165 registers for
+  // nothing: the backward 2.13 ms, 2.04 without; 6 x 4: 1.59, 1.55; 4 x 3, 12 x 3 and 12 x 4 the same within 1 %)
   static constexpr int BY_SMEM = 228 * 1024 / (NBUF * STAGE + 1536);
   static constexpr int CTAS = BY_STATE < BY_SMEM ? BY_STATE : BY_SMEM;
   static __device__ __forceinline__ int idx(int p) { return TT == 2 ? (p >> 1) + (p & 1) * HALF : p; }

@@ -108,9 +108,13 @@ def plan(kernel: Any) -> Plan:
     return cached  # type: ignore[no-any-return]
 
 
+def is_on(t: Tensor, device: torch.device) -> bool:
+    return t.device.type == device.type and device.index in (None, t.device.index)
+
+
 def descriptors(kernel: Any, device: torch.device) -> Tensor:
     cache = kernel.__dict__.setdefault("_fused_factored_descriptors", {})
-    if str(device) not in cache:
+    if str(device) not in cache or not is_on(cache[str(device)], device):  # a kernel loaded from a file may bring others
         cache[str(device)] = torch.tensor([b.row() for b in plan(kernel).blocks], dtype=torch.int32, device=device).reshape(-1, DESC)
     return cache[str(device)]  # type: ignore[no-any-return]
 

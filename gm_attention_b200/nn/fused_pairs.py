@@ -324,11 +324,19 @@ def _field_fits(kernel: Any, frequencies: list[int], values: list[Tensor], n_nod
     return True
 
 
+def _uploaded(kernel: Any, device: torch.device) -> tuple[Tensor, Tensor] | None:
+    """The kernel's descriptors on ``device``, if they are there: a kernel loaded from a file may bring others' under its name."""
+    from gm_attention_b200.nn import fused_factored as ff
+
+    found = kernel.__dict__.get("_fused_node_descriptors", {}).get(str(device))
+    return found if found is not None and all(ff.is_on(t, device) for t in found) else None
+
+
 def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
     """Whether an earlier call left the kernel's descriptors on the device and grouped these edges by source."""
     from gm_attention_b200.nn import fused_factored as ff
 
-    return str(device) in kernel.__dict__.get("_fused_node_descriptors", {}) and ff.cached_grouping(edges, device) is not None
+    return _uploaded(kernel, device) is not None and ff.cached_grouping(edges, device) is not None
 
 
 def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term], table: Tensor | None) -> tuple | None:
@@ -391,11 +399,12 @@ def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tu
     # the kernels read memory: conjugations and signs that torch has put off are carried out first
     flat = [(torch.view_as_real(v.resolve_conj()) if v.is_complex() else v.resolve_neg()).reshape(n_nodes, -1) for v in values]
     packed = flat[0] if len(flat) == 1 else torch.cat(flat, 1)
-    tables = kernel.__dict__.setdefault("_fused_node_descriptors", {})
-    if str(device) not in tables:
-        tables[str(device)] = (torch.tensor(rows, dtype=torch.int32, device=device).reshape(-1, 8),
-                               torch.tensor([b.row() for b in p.blocks], dtype=torch.int32, device=device).reshape(-1, 8))
-    node_desc, desc = tables[str(device)]
+    uploaded = _uploaded(kernel, device)
+    if uploaded is None:
+        uploaded = (torch.tensor(rows, dtype=torch.int32, device=device).reshape(-1, 8),
+                    torch.tensor([b.row() for b in p.blocks], dtype=torch.int32, device=device).reshape(-1, 8))
+        kernel.__dict__.setdefault("_fused_node_descriptors", {})[str(device)] = uploaded
+    node_desc, desc = uploaded
     params = [q for head in (kernel.complex_head, kernel.real_head) for q in ((None, None) if head is None else (head.weight, head.bias))]
     zc, zr = NodeProducts.apply(packed, *params, node_desc, hidden.shape[1] + 1, p.wc, p.wr)
     source = edges.source_index.contiguous()

@@ -8,9 +8,10 @@ row, source row, longitude offset) only -- 44 920 distinct entries instead of 22
 
 1. the radial network runs on the ENTRIES (:class:`RadialCoefficients`: the reference's Gaussian basis, trunk and two
    read-outs, ``nn/kernels.py:191-240``, ``nn/depthwise.py:60-121``; ordinary PyTorch, ordinary autograd);
-2. :func:`fold` turns an entry's coefficients, phases and weight into one real 2 x 2 matrix per complex copy and one
-   real factor per scalar channel (``z -> A tau z + w B conj(tau z)`` is a real-linear map of the plane; also ordinary
-   tensor algebra, so autograd carries the table's gradient back to the network);
+2. :class:`FoldTable` turns an entry's coefficients, phases and weight into one real 2 x 2 matrix per complex copy and
+   one real factor per scalar channel (``z -> A tau z + w B conj(tau z)`` is a real-linear map of the plane): one launch
+   forward, one back to the coefficients' gradients (``gm_lattice_conv_fold``), once differentiable like the rest of the
+   chain; :func:`fold` is the same in tensor algebra, for coefficients or tables that are not laid out as the kernel reads;
 3. :class:`LatticeDepthwise` applies the table (``gm_lattice_conv_apply``) and, backward, forms the field's gradient
    (the same kernel on the transposed windows) and the table's gradient (``gm_lattice_conv_table_grad``).
 

@@ -226,7 +226,9 @@ int gm_lattice_attention_backward(const void* dout, const void* q, const void* k
  *   zc         (n_nodes, k, wc, 2), zr (n_nodes, k, wr)   node-side mixes
  *   angular, transport (n_edges, n_f, 2); rho (n_edges)
  *   desc       (n_blocks, 8) int32    rows (kind, z_off, b_m, ang, trn, power, out_off, take_real),
- *                                     sorted by out_off
+ *                                     sorted by out_off; blocks that share an out_off share b_m and
+ *                                     the kind of their columns (real, or (re, im) pairs), and columns
+ *                                     that no block names are left undefined in out
  *   order (n_edges), group_ptr (n_groups + 1), group_source (n_groups) int64:
  *              the edges sorted by source, each source's run, the sources
  *   out / rows (n_edges, d_out)

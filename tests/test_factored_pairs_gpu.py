@@ -867,3 +867,42 @@ def test_node_level_route_only_for_tensors_its_kernels_can_read(monkeypatch):
     short = {name: getattr(edges, name)[:-1] for name in ("angular_phases", "transport_phases")}
     assert not takes(over=dataclasses.replace(edges, **short))
     assert not takes(over=dataclasses.replace(edges, edge_index=edges.edge_index.int()))
+
+
+def test_kernel_saved_after_a_call_and_loaded_elsewhere():
+    """A kernel saved after a call, loaded with its tensors on the host and moved back, gives what it gave before, from the
+    pair driver and from the factored one: the descriptors it kept are uploaded again."""
+    import io
+
+    from gm_attention_b200.fields import FeatureField
+    from gm_attention_b200.geometry import compute_edge_geometry, midpoint_lattice
+    from gm_attention_b200.nn import fused_factored as ff
+    from gm_attention_b200.nn import fused_pairs as fp
+    from tests.helpers import StandInKernel
+
+    dev = torch.device("cuda", 0)
+    lattice = midpoint_lattice(9, 22, dev)
+    cutoff = 1.9 * math.pi / 9
+    edges = compute_edge_geometry(lattice, lattice.frames, cutoff, max_frequency=4, dtype=torch.float32)
+    kernel = StandInKernel({0: 2, 1: 2}, {0: 2, 1: 2}, cutoff, dtype=torch.float32).to(dev)
+    flat = torch.randn(lattice.n_nodes, kernel.field_type_in.dimension, device=dev)
+    kernel.plan_of_blocks = blocks_for({0: 2, 1: 2}, {0: 2, 1: 2})[0]
+    products = {b: torch.randn(lattice.n_nodes, 9, 2, device=dev, dtype=torch.float32 if b[2] == "real" else torch.complex64) for b in kernel.plan_of_blocks}
+
+    def results(kernel):
+        kernel._blocks = lambda: kernel.plan_of_blocks
+        kernel._trunk_hidden = lambda e: kernel.radial_trunk(kernel.radial_basis(e.distances))
+        with torch.no_grad():
+            out = fp.forward_general(kernel, FeatureField.from_flat(kernel.field_type_in, flat), edges).coefficients
+            out = [*out.values(), ff.forward(kernel, None, edges, dict(products))]
+        del kernel._blocks, kernel._trunk_hidden
+        return out
+
+    want = results(kernel)
+    file = io.BytesIO()
+    torch.save(kernel, file)
+    file.seek(0)
+    loaded = torch.load(file, map_location="cpu", weights_only=False).to(dev)
+    assert loaded.__dict__["_fused_node_descriptors"][str(dev)][0].device.type == "cpu"
+    for a, b in zip(results(loaded), want, strict=True):
+        assert torch.equal(a, b)
