@@ -7,9 +7,15 @@
 // phase * sum_t h~_t(e) Z_t(source(e)), the form factored_ops.cu evaluates: an edge then costs trunk * b multiply-adds per
 // block instead of trunk * a * b, and the readout's gradient is a sum over nodes instead of edges.
 //
-// The work is small (nodes * trunk * a * b per block); what matters is that weights are read once per NODES nodes (8 192
-// nodes, {8, 8, 8} -> {4, 4, 4}, trunk 16: 4 / 8 / 16 nodes take 145 / 99 / 135 us forward, 230 / 200 / 336 for dx) and that
+// The work is small (nodes * trunk * a * b per block); what matters is that weights are read once per NODES nodes and that
 // the readout's gradient, a sum over all nodes, is cut into chunks of nodes whose partial sums the caller adds: no atomics.
+//
+// NODES = 4 / 8 / 16, us forward, then backward (dx, the readout's gradient and the sum of its parts), float32:
+//   {8, 8, 8} -> {4, 4, 4}, trunk 16    8 192 nodes 127 / 87 / 137, 428 / 396 / 498    30 000 nodes 300 / 288 / 434, 1 680 / 1 659 / 1 762
+//   {16, 16} -> {8, 8}, trunk 16        8 192 nodes 134 / 85 / 154, 491 / 470 / 577    30 000 nodes 301 / 255 / 466, 2 025 / 1 997 / 2 181
+//   {2, 2} -> {8, 8}, trunk 16          8 192 nodes  52 / 40 /  53, 145 / 141 / 176    30 000 nodes 135 / 162 / 199,   478 /   490 /   572
+// On 1 000 nodes 4 wins (46 / 51, 166 / 219 for the first), where a pass of some 700 us waits for its launches; float64 leans
+// to 4 on 30 000 nodes (409 / 459 / 698, 1 974 / 2 145 / 2 806 for the first) and to 8 on 8 192 (153 / 125 / 173, 584 / 581 / 764).
 #include "common.cuh"
 
 namespace gmb {
