@@ -258,51 +258,71 @@ class NodeProducts(torch.autograd.Function):
         return (dx, *grads, None, None, None, None)
 
 
-def _node_blocks(kernel: Any, terms: list[Term]) -> tuple[Any, list[list[int]], dict[bool, int] | None]:
-    """The factored plan of the kernel's terms, the descriptor rows of their node products, and the readout rows they read
-    of the real (True) and complex (False) head -- ``None`` where a term's rows are no plain run (cached on the kernel)."""
-    cached = kernel.__dict__.get("_fused_node_plan")
-    if cached is not None:
-        return cached  # type: ignore[no-any-return]
-    from gm_attention_b200.fields import FieldType
-    from gm_attention_b200.nn import fused_factored
+@dataclass(frozen=True)
+class NodePlan:
+    """What the node-level route knows of a kernel from its terms alone."""
 
+    served: bool  # the terms are within the bounds of the pair terms and of the route's kernels, their readout rows plain runs
+    factored: Any = None  # the factored plan of the terms
+    rows: tuple = ()  # descriptor rows of the node products
+    inputs: tuple = ()  # (frequency, multiplicity) of the input type, in its order
+    needed: tuple = ()  # (real head?, readout rows its terms read)
+    width: int = 0  # packed columns of the products, padded to whole 16-byte vectors
+    order: int = 0  # highest order of the phase tables
+    power: int = 0  # highest column of the radial table
+
+
+def _node_plan(kernel: Any, terms: list[Term]) -> NodePlan:
+    """The kernel's :class:`NodePlan`, kept on it like the terms."""
+    cached = kernel.__dict__.get("_fused_node_plan")
+    if cached is None:
+        cached = kernel.__dict__["_fused_node_plan"] = _built_node_plan(kernel, terms)
+    return cached  # type: ignore[no-any-return]
+
+
+def _built_node_plan(kernel: Any, terms: list[Term]) -> NodePlan:
+    from gm_attention_b200.fields import FieldType
+    from gm_attention_b200.nn import fused_factored as ff
+
+    # the pair terms' own bounds first: what they refuse is refused on any graph
+    if not terms or any(not (1 <= t.a <= MAX_MULT and 1 <= t.b <= MAX_MULT) for t in terms):
+        return NodePlan(False)
     # the rows' layout is this route's own: what the kernel's field type is asked is what the pair terms ask
-    p = fused_factored.plan_blocks([(t.n, t.m, t.role) for t in terms], FieldType({t.m: t.b for t in terms}),
-                                   {(t.n, t.m, t.role): t.power for t in terms if t.power is not None})
+    p = ff.plan_blocks([(t.n, t.m, t.role) for t in terms], FieldType({t.m: t.b for t in terms}),
+                       {(t.n, t.m, t.role): t.power for t in terms if t.power is not None})
+    inputs = tuple((n, kernel.field_type_in.multiplicity(n)) for n in kernel.field_type_in.frequencies)
     offsets, at = {}, 0
-    for n in kernel.field_type_in.frequencies:
+    for n, copies in inputs:
         offsets[n] = at
-        at += kernel.field_type_in.multiplicity(n) * (1 if n == 0 else 2)
+        at += copies * (1 if n == 0 else 2)
     by_block = {(t.n, t.m, t.role): t for t in terms}
     rows = []
     for b in p.blocks:
         t = by_block[b.block]
         operand = 0 if t.flags & U_REAL else (2 if t.flags & CONJ_U else 1)
-        rows.append([b.kind, b.z_offset, t.b, t.a, offsets[t.n], operand, t.rows.start or 0, 0])
-    needed: dict[bool, int] | None = {}
+        rows.append((b.kind, b.z_offset, t.b, t.a, offsets[t.n], operand, t.rows.start or 0, 0))
+    needed: dict[bool, int] = {}
+    plain = True
     for t in terms:
         start, width = t.rows.start or 0, t.a * t.b * (2 if t.flags & MATRIX_COMPLEX else 1)
-        if needed is None or start < 0 or t.rows.stop != start + width or t.rows.step not in (None, 1):
-            needed = None
-        else:
-            needed[t.real_head] = max(needed.get(t.real_head, 0), start + width)
-    kernel.__dict__["_fused_node_plan"] = (p, rows, needed)
-    return p, rows, needed
+        plain = plain and start >= 0 and t.rows.stop == start + width and t.rows.step in (None, 1)
+        needed[t.real_head] = max(needed.get(t.real_head, 0), start + width)
+    powers = [b.power for b in p.blocks]
+    served = plain and at <= MAX_NODE_WIDTH and p.d_out <= ff.MAX_OUT and p.max_bm <= ff.MAX_BM and min(powers) >= 0
+    return NodePlan(served, p, tuple(rows), inputs, tuple(needed.items()), -(-(2 * p.wc + p.wr) // 4) * 4,
+                    max(max(abs(b.angular), abs(b.transport)) for b in p.blocks), max(powers))
 
 
-def _readouts_fit(kernel: Any, needed: dict[bool, int] | None, hidden: Tensor) -> bool:
+def _readouts_fit(kernel: Any, needed: tuple, hidden: Tensor) -> bool:
     """Whether both heads hold, in the trunk's dtype and place, the rows their terms read."""
-    if needed is None:
-        return False
-    for real, rows in needed.items():
+    for real, rows in needed:
         head = kernel.real_head if real else kernel.complex_head
         weight, bias = getattr(head, "weight", None), getattr(head, "bias", None)
         if weight is None or weight.dim() != 2 or weight.shape[0] < rows or weight.shape[1] != hidden.shape[1]:
             return False
-        if bias is not None and bias.shape != weight.shape[:1]:
+        if weight.dtype != hidden.dtype or weight.device != hidden.device:
             return False
-        if any(t.dtype != hidden.dtype or t.device != hidden.device for t in (weight, bias) if t is not None):
+        if bias is not None and (bias.shape != weight.shape[:1] or bias.dtype != hidden.dtype or bias.device != hidden.device):
             return False
     return True
 
@@ -315,11 +335,14 @@ def _products_repaid(n_nodes: int, n_edges: int) -> bool:
     return n_edges >= (4 if n_nodes <= 8192 else 10) * n_nodes
 
 
-def _field_fits(kernel: Any, frequencies: list[int], values: list[Tensor], n_nodes: int) -> bool:
-    """Whether the coefficients are ``(N, a_0)`` reals and ``(N, a_n)`` complex numbers or ``(N, a_n, 2)`` pairs."""
-    for n, v in zip(frequencies, values, strict=True):
-        pairs = () if n == 0 or v.is_complex() else (2,)
-        if (n == 0 and v.is_complex()) or v.shape != (n_nodes, kernel.field_type_in.multiplicity(n), *pairs):
+def _field_fits(inputs: tuple, values: list[Tensor], n_nodes: int, like: Tensor) -> bool:
+    """Whether the coefficients are ``(N, a_0)`` reals and ``(N, a_n)`` complex numbers or ``(N, a_n, 2)`` pairs, in ``like``'s
+    real dtype and place."""
+    for (n, copies), v in zip(inputs, values, strict=True):
+        as_complex = v.is_complex()
+        if v.device != like.device or v.dtype != (_complex_of(like.dtype) if as_complex else like.dtype):
+            return False
+        if (n == 0 and as_complex) or v.shape != ((n_nodes, copies) if n == 0 or as_complex else (n_nodes, copies, 2)):
             return False
     return True
 
@@ -342,72 +365,61 @@ def _prepared(kernel: Any, edges: Any, device: torch.device) -> bool:
 def _factored_inputs(kernel: Any, x: Any, edges: Any, hidden: Tensor, terms: list[Term], table: Tensor | None) -> tuple | None:
     """What the factored form needs of this call, or ``None`` where the pair terms serve it: an edge-level or mixed field,
     too few edges per node (:func:`_products_repaid`), phase tables that are not plain per-edge
-    ``angular_phases`` / ``transport_phases`` of one width or that want gradients, sizes beyond the factored kernels."""
-    frequencies = list(kernel.field_type_in.frequencies)
-    values = [x[n] for n in frequencies]
-    nodes = {int(v.shape[0]) for v in values}
-    n_edges = int(edges.n_edges)
+    ``angular_phases`` / ``transport_phases`` of one width or that want gradients, sizes beyond the factored kernels, and any
+    tensor that does not have the shape, dtype or place the kernels read it with."""
     from gm_attention_b200.nn import fused_factored as ff
 
-    if hidden.device.type != "cuda" or hidden.dtype not in (torch.float32, torch.float64) or hidden.dim() != 2 or len(nodes) != 1 or not terms:
+    device, dtype = hidden.device, hidden.dtype
+    if device.type != "cuda" or dtype not in (torch.float32, torch.float64) or hidden.dim() != 2 or not 1 <= hidden.shape[1] <= MAX_TRUNK:
         return None
-    n_nodes = nodes.pop()
-    if n_nodes == n_edges or n_nodes == 0 or not _products_repaid(n_nodes, n_edges):
+    node = _node_plan(kernel, terms)
+    k = hidden.shape[1] + 1
+    if not node.served or k > ff.MAX_K or k * node.width > ff.MAX_KC:
+        return None
+    values = [x[n] for n, _ in node.inputs]
+    n_nodes, n_edges = int(values[0].shape[0]), int(edges.n_edges)
+    if n_nodes == n_edges or n_nodes == 0 or not _products_repaid(n_nodes, n_edges) or not _field_fits(node.inputs, values, n_nodes, hidden):
         return None
     angular, transport = getattr(edges, "angular_phases", None), getattr(edges, "transport_phases", None)
-    if angular is None or transport is None or angular.shape != transport.shape or any(not hasattr(edges, x) for x in ("edge_index", "row_ptr")):
+    if angular is None or transport is None or not hasattr(edges, "edge_index") or not hasattr(edges, "row_ptr"):
         return None
-    source = edges.source_index
-    if edges.edge_index is not edges.edge_index or ff.version(source) < 0 or source.untyped_storage().data_ptr() != edges.edge_index.untyped_storage().data_ptr():
+    for phases in (angular, transport):
+        if phases.dim() != 2 or phases.shape != angular.shape or phases.dtype != _complex_of(dtype) or phases.device != device or phases.requires_grad:
+            return None
+    source, index = edges.source_index, edges.edge_index
+    if source.shape != (n_edges,) or source.dtype != torch.int64 or source.device != device:
+        return None
+    if index is not edges.edge_index or ff.version(source) < 0 or source.untyped_storage().data_ptr() != index.untyped_storage().data_ptr():
         return None  # no grouping to keep, or one whose key could not tell other indices: an edge_index formed on every access,
         # inference tensors, sources kept apart from edge_index
-    if angular.dtype != _complex_of(hidden.dtype) or transport.dtype != angular.dtype or angular.requires_grad or transport.requires_grad:
-        return None
-    if any(v.device != hidden.device or (v.real if v.is_complex() else v).dtype != hidden.dtype for v in (*values, angular, transport)):
-        return None
-    # the pair terms' own bounds: what they refuse is refused on any graph
-    if not 1 <= hidden.shape[1] <= MAX_TRUNK or any(not (1 <= t.a <= MAX_MULT and 1 <= t.b <= MAX_MULT) for t in terms):
-        return None
-    if sum(kernel.field_type_in.multiplicity(n) * (2 if n else 1) for n in frequencies) > MAX_NODE_WIDTH:
-        return None
-    if not _field_fits(kernel, frequencies, values, n_nodes) or angular.dim() != 2 or len({n_edges, *(t.shape[0] for t in (hidden, angular, source))}) != 1:
-        return None
-    if source.dim() != 1 or source.dtype != torch.int64 or source.device != hidden.device:
-        return None
-    p, rows, needed = _node_blocks(kernel, terms)
-    if not _readouts_fit(kernel, needed, hidden):
-        return None
-    k = hidden.shape[1] + 1
-    if k > ff.MAX_K or p.d_out > ff.MAX_OUT or p.max_bm > ff.MAX_BM or k * (-(-(2 * p.wc + p.wr) // 4) * 4) > ff.MAX_KC:
-        return None
-    if max((max(abs(b.angular), abs(b.transport)) for b in p.blocks), default=0) >= angular.shape[1]:
+    if hidden.shape[0] != n_edges or angular.shape[0] != n_edges or node.order >= angular.shape[1] or not _readouts_fit(kernel, node.needed, hidden):
         return None
     scales = hidden.new_ones(n_edges, 1) if table is None else table.detach()  # table None: no block has a scale
-    powers = [b.power for b in p.blocks]
-    if scales.dim() != 2 or scales.shape[0] != n_edges or min(powers) < 0 or max(powers) >= scales.shape[1] or scales.dtype != hidden.dtype or scales.device != hidden.device:
+    if scales.dim() != 2 or scales.shape[0] != n_edges or scales.shape[1] <= node.power or scales.dtype != dtype or scales.device != device:
         return None
-    if torch.cuda.is_current_stream_capturing() and not _prepared(kernel, edges, hidden.device):
+    if torch.cuda.is_current_stream_capturing() and not _prepared(kernel, edges, device):
         return None  # grouping the edges by source and uploading the descriptors synchronise: not while a graph is captured
-    return p, rows, values, angular, transport, scales, n_nodes
+    return node, values, angular, transport, scales, source, n_nodes
 
 
 def _forward_factored(kernel: Any, x: Any, edges: Any, hidden: Tensor, found: tuple) -> Any:
     from gm_attention_b200.nn import fused_factored as ff
 
-    p, rows, values, angular, transport, scales, n_nodes = found
+    node, values, angular, transport, scales, source, n_nodes = found
+    p = node.factored
     device = hidden.device
     # the kernels read memory: conjugations and signs that torch has put off are carried out first
     flat = [(torch.view_as_real(v.resolve_conj()) if v.is_complex() else v.resolve_neg()).reshape(n_nodes, -1) for v in values]
     packed = flat[0] if len(flat) == 1 else torch.cat(flat, 1)
     uploaded = _uploaded(kernel, device)
     if uploaded is None:
-        uploaded = (torch.tensor(rows, dtype=torch.int32, device=device).reshape(-1, 8),
+        uploaded = (torch.tensor(node.rows, dtype=torch.int32, device=device).reshape(-1, 8),
                     torch.tensor([b.row() for b in p.blocks], dtype=torch.int32, device=device).reshape(-1, 8))
         kernel.__dict__.setdefault("_fused_node_descriptors", {})[str(device)] = uploaded
     node_desc, desc = uploaded
     params = [q for head in (kernel.complex_head, kernel.real_head) for q in ((None, None) if head is None else (head.weight, head.bias))]
     zc, zr = NodeProducts.apply(packed, *params, node_desc, hidden.shape[1] + 1, p.wc, p.wr)
-    source = edges.source_index.contiguous()
+    source = source.contiguous()
     order, group_ptr, group_source = ff.grouping_for(edges, source).require_nodes(n_nodes)
     out = ff.Factored.apply(hidden, zc, zr, *(torch.view_as_real(t.resolve_conj().contiguous()) for t in (angular, transport)), scales.resolve_neg().contiguous(),
                             desc, source, order, group_ptr, group_source, p.d_out, p.max_bm, True)
