@@ -129,6 +129,48 @@ class GaugeAttention(torch.autograd.Function):
 
 # ----------------------------------------------------------------------------- equiangular lattices
 
+@dataclass(frozen=True, eq=False)
+class TensorCorePlan:
+    """What the tensor-core lattice kernels read besides the tables (``gm_lattice_plan_build`` in ``include/gm_b200.h``): the
+    packed neighbour lists and entries of every row tile, and the tables they were made from."""
+
+    first: Tensor  # (row tiles + 1,) int32: first record of a row tile
+    records: Tensor  # uint8
+    layout: tuple  # descriptor rows, lattice size and halo it was made for
+    sources: tuple  # (tensor, write counter) of win_cnt, win_lo, win_off, entries
+
+    def serves(self, layout: tuple, *tables: Tensor) -> bool:
+        """Whether these are the tables the plan was made from, unwritten since."""
+        return self.layout == layout and all(a is b and b._version == version for (a, version), b in zip(self.sources, tables))
+
+
+def tensor_core_plan(desc_rows: tuple[tuple[int, int, int, int, int], ...], heads: int, rows: int, nlon: int, halo: int, orders: int, win_cnt: Tensor,
+                     win_lo: Tensor, win_off: Tensor, entries: Tensor, mode: int) -> TensorCorePlan | None:
+    """The plan of one pass (0 forward, 1 target-major, 2 source-major, on the transposed tables); ``None`` where the
+    tensor-core kernels do not serve the layout."""
+    tables = (win_cnt, win_lo, win_off, entries)
+    if not entries.is_cuda or entries.shape[0] == 0 or entries.shape[1] != 8 or 2 * halo + 1 > 33 or orders != sum(r[0] > 0 for r in desc_rows):
+        return None
+    if not tensor_core_layout_supported(desc_rows) or any(t.is_inference() for t in tables):
+        return None
+    flat = [x for row in desc_rows for x in row]
+    desc = (ctypes.c_int64 * len(flat))(*flat)
+    width = max(off + heads * a_n * (1 if n == 0 else 2) for n, a_n, off, *_ in desc_rows)
+    size, tiles = ctypes.c_int64(), ctypes.c_int64()
+    sizes = (ctypes.addressof(desc), len(desc_rows), rows, nlon, width, heads, halo, orders, mode)
+    _lib.call("gm_lattice_plan_size", *sizes, ctypes.addressof(size), ctypes.addressof(tiles))
+    device = entries.device
+    with torch.cuda.device(device):
+        counts = torch.empty(tiles.value, dtype=torch.int32, device=device)
+        common = (*(_lib.ptr(t) for t in tables), *sizes)
+        _lib.call("gm_lattice_plan_build", *common, _lib.ptr(counts), None, None, _lib.stream(device))
+        first = torch.zeros(tiles.value + 1, dtype=torch.int32, device=device)
+        torch.cumsum(counts, 0, dtype=torch.int32, out=first[1:])
+        records = torch.empty(int(first[-1]) * size.value, dtype=torch.uint8, device=device)
+        _lib.call("gm_lattice_plan_build", *common, None, _lib.ptr(first), _lib.ptr(records), _lib.stream(device))
+    return TensorCorePlan(first, records, (desc_rows, heads, rows, nlon, halo, orders), tuple((t, t._version) for t in tables))
+
+
 @dataclass(frozen=True)
 class LatticeTables:
     """Compact per-(target row, source row, longitude offset) tables of a lattice
@@ -164,6 +206,17 @@ class LatticeTables:
     # entry of every transposed entry
     entry_edge: Tensor | None = None
     t_entry: Tensor | None = None
+    # the tensor-core kernels' plans of the forward, the target-major and the source-major pass; None where they do not serve
+    # the head layout
+    tc_plans: tuple[TensorCorePlan | None, ...] = (None, None, None)
+
+    def plan_pointers(self, mode: int) -> tuple[int | None, int | None]:
+        """Addresses of the parts of a pass's plan for these tables; ``(None, None)`` without one (the kernels then work it out)."""
+        plan = self.tc_plans[mode]
+        tables = (self.t_win_cnt, self.t_win_lo, self.t_win_off, self.t_entries) if mode == 2 else (self.win_cnt, self.win_lo, self.win_off, self.entries)
+        if plan is None or not plan.serves((self.desc_rows, self.heads, self.rows, self.nlon, self.halo, self.orders), *tables):
+            return None, None
+        return _lib.ptr(plan.first), _lib.ptr(plan.records)
 
     def host_descriptor(self) -> Any:
         flat = [x for row in self.desc_rows for x in row]
@@ -360,9 +413,11 @@ def build_lattice_tables(geometry: Any, rows: int, nlon: int, desc_rows: tuple[t
         tc_e, tc_o = tensor_core_entries(entries, win_cnt, win_off, norders)
         t_tc_e, t_tc_o = tensor_core_entries(t_entries, t_cnt, t_off, norders)
         tc = (dev(tc_e), dev(tc_o), dev(t_tc_e), dev(t_tc_o))
-    return LatticeTables(rows, nlon, halo, stride, norders, dev(win_cnt), dev(win_lo), dev(win_off), dev(entries), dev(row_order),
-                         dev(t_cnt), dev(t_lo), dev(t_off), dev(t_entries), dev(t_row_order), tuple(tuple(int(x) for x in r) for r in desc_rows),
-                         heads, float(scale), int(geometry.source.shape[0]), *tc, dev(entry_edge.astype(np.int64)), dev(t_entry))
+    desc_rows = tuple(tuple(int(x) for x in r) for r in desc_rows)
+    forward, transposed = (dev(win_cnt), dev(win_lo), dev(win_off), dev(entries)), (dev(t_cnt), dev(t_lo), dev(t_off), dev(t_entries))
+    plans = tuple(tensor_core_plan(desc_rows, heads, rows, nlon, halo, norders, *(transposed if mode == 2 else forward), mode) for mode in range(3))
+    return LatticeTables(rows, nlon, halo, stride, norders, *forward, dev(row_order), *transposed, dev(t_row_order), desc_rows,
+                         heads, float(scale), int(geometry.source.shape[0]), *tc, dev(entry_edge.astype(np.int64)), dev(t_entry), plans)
 
 
 def _check_lattice(q: Tensor, k: Tensor, v: Tensor, t: LatticeTables) -> tuple[torch.device, int]:
@@ -442,7 +497,7 @@ def lattice_attention_forward(q: Tensor, k: Tensor, v: Tensor, t: LatticeTables,
         if four:
             _lib.call("gm_lattice_attention_forward_tc4", *common, _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
         elif tensor_cores:
-            _lib.call("gm_lattice_attention_forward_tc", *common, _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
+            _lib.call("gm_lattice_attention_forward_planned", *common, *t.plan_pointers(0), _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
         else:
             _lib.call("gm_lattice_attention_forward", *common, _lib.dtype_code(q.dtype), _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
     return out, lse
@@ -487,7 +542,8 @@ def lattice_attention_backward(dout: Tensor, q: Tensor, k: Tensor, v: Tensor, ou
         if four:
             _lib.call("gm_lattice_attention_backward_tc4_passes", *common, *outputs[:4], int(passes), outputs[4])
         elif tensor_cores:
-            _lib.call("gm_lattice_attention_backward_tc_passes", *common, *outputs[:4], int(passes), outputs[4])
+            _lib.call("gm_lattice_attention_backward_planned", *common, *outputs[:4], int(passes), *t.plan_pointers(1), *t.plan_pointers(2),
+                      outputs[4])
         else:
             _lib.call("gm_lattice_attention_backward", *common, _lib.dtype_code(q.dtype), *outputs)
     return dq, dk, dv

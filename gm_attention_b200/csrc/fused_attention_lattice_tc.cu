@@ -8,34 +8,43 @@
 //   sum_j alpha_ij tau_n v_j = ((alpha o tau_n) V)_i,
 //
 // so for 8 consecutive owners (targets; sources in the backward's source-major
-// pass) of one lattice row and 16 consecutive positions of one neighbour row the
+// pass) of one lattice row and 16 neighbour positions the
 // Gram blocks G0, Re G_n, Im G_n are plain bf16 x bf16 -> fp32 products, the
 // phases / bias / window enter elementwise on the tile in registers, and the value
-// sums are products with the weights as an operand.  The staged neighbour
+// sums are products with the weights as an operand.  The
 // positions are the M dimension of the MMAs (16 per step) and a warp's owners the
 // N dimension (8 per warp):
 //
 //   S^T   (16 positions x 8 owners)  = tile (positions x columns) * owners^T      A: shared memory, B: loop-invariant registers
 //   out^T (16 columns   x 8 owners) += tile^T (columns x positions) * (P o tau)^T  A: shared memory (ldmatrix.trans), B: P^T
 //
-// * Only the longitude band of a row pair is visited; pairs outside an owner's cyclic window get logit -inf.  8 owners
-//   see a window of 7 + cnt positions, so the narrow equatorial windows (cnt <= 9) take ONE step per neighbour row;
-//   polar windows (whole rows) are dense.
-// * Im G_n uses a pre-swapped copy of the OWNERS' fragments, (re, im) -> (-im, re) or (im, -re), made once per CTA.
+// * Only the longitude band of a row pair is visited: 8 owners see 7 + cnt positions of a neighbour row.  The positions of
+//   all neighbour rows are PACKED into steps of 16 (ldmatrix takes each of its 16 rows from anywhere), so the narrow
+//   equatorial windows (cnt <= 7, 9 to 14 positions a row) leave no step half empty; pairs outside an owner's window and the
+//   list's padding meet a table entry with bias -inf, without a bounds test.
+// * Im G_n uses a pre-swapped copy of the OWNERS' fragments, (re, im) -> (-im, re) or (im, -re), made once per (sample, head).
 // * The imaginary part of the phase accumulates into a second accumulator set; the multiplication by +-i (the pair
 //   swap) is applied once in the epilogue, so the staged value tile is never swapped.
 // * The weights P (accumulator layout: position rows, owner columns) become a B operand with movmatrix (8 x 8 b16
 //   transpose in registers); the same instruction turns the result tiles into 4-byte stores per owner.
 // * The softmax reference maximum of an owner moves only when it is exceeded by 2^8 (lazy rescaling).
 //
-// One CTA = 8 owners x WARPS warps x one head x one sample.  The neighbour rows of one lattice row and the table
-// entries they need are copied into shared memory as raw bf16 / fp32, double-buffered: the copy of the next
-// (row pair, chunk) runs while the current one is consumed.  A staged field is one sub-tile per frequency block
-// (88 or 56 positions x 32 or 64 bytes) in the 32-byte / 64-byte shared-memory swizzle, so that ldmatrix is conflict-free
-// without padding and a whole sub-tile is ONE TMA tensor copy (cp.async.bulk.tensor.3d over (column, longitude,
-// sample * row), completion on an mbarrier, issued by one thread).  Chunks that wrap the longitude seam, and head
-// layouts whose blocks are not exactly 16 / 32 columns, are staged with per-thread cp.async into the same swizzled
-// layout.  Tensor-core instruction: mma.sync m16n8k16 (bf16 inputs, fp32 accumulate); fragments via ldmatrix.
+// One CTA: a tile of four lattice rows x 8 (or 16) longitudes, a warp per row and 8 longitudes, which share the staged
+// neighbourhood (the rows' windows overlap: 120 staged rows serve 32 owners at radius 3, against 250 for 32 owners of one
+// row); it walks over (sample, head) pairs with one list of positions and one set of table entries.  The next pair's rows are
+// under way (cp.async, both fields of a position in one shared-memory row whose pitch is an odd multiple of 16 bytes: no
+// bank conflicts) while this pair's results are written.  Neighbourhoods that outgrow shared memory -- the polar rows' -- come
+// in chunks.  Lists and entries depend on the tables alone: gm_lattice_plan_build works them out once per table and a CTA
+// copies them; without a plan each CTA works them out itself (16 longitudes x 4 rows, 128 x 256, batch 4: 2 361 against
+// 1 757 us for the three passes).  Tensor-core instruction: mma.sync m16n8k16 (bf16 inputs, fp32 accumulate).
+//
+// What it measured against the kernel before it (one row of 32 longitudes and one (sample, head) per CTA, a step per
+// neighbour row, TMA staging), us forward / pass T / pass S: 128 x 256, batch 4, 4 heads of 8 x (m <= 3): 603 / 904 / 995 ->
+// 427 / 568 / 658; 256 x 512, batch 8, 4 heads of 16 x (m <= 2): 3 670 / 4 896 / 6 643 -> 3 422 / 4 578 / 6 045; heads that
+// are not 16 copies wide, batch 1 to 8: 1.2 to 4 times faster.  What bounds it: of the last forward 2.1 ms are the steps
+// (shared-memory bandwidth: ten ldmatrix.x4 and the entries, about 100 of 114 cycles a step), 1.4 ms the staging and the
+// per-pair prologue and epilogue, which overlap only across the SM's two CTAs.  16 longitudes per CTA pay in the forward
+// (3 998 -> 3 422); passes T and S want 168 registers a thread, so three CTAs of 4 warps.
 //
 // Backward, two deterministic passes (no atomics):
 //   pass T: owners = targets.  Delta = <dO, O> per (target, head) from the owners' own rows (written out for pass S);
@@ -44,8 +53,7 @@
 //   pass S: owners = SOURCES, neighbours = the targets that see them (transposed tables, their lse / Delta
 //           staged with them).  Same Gram blocks with the roles swapped, then (ds o conj tau) Q -> dk and
 //           (p o conj tau) dO -> dv.
-#include <cuda.h>
-#include <cudaTypedefs.h>
+#include <cmath>
 
 #include "common.cuh"
 
@@ -55,16 +63,16 @@ namespace {
 constexpr float TC_LOG2E = 1.4426950408889634f, TC_LN2 = 0.6931471805599453f;
 constexpr int TC_MAX_CF = 3;
 constexpr int TC_MAX_WIN = 33;  // 2 W + 1 neighbour rows at most
-constexpr unsigned TC_WAIT_LIMIT = 1u << 22;  // polls of a copy barrier before the kernel gives up on it
-
-// set when a wait on a TMA completion barrier ran out (never expected; the results of that launch are invalid)
-__device__ int g_tc_wait_expired;
 
 struct TcPlan {
   int a0, ac, n_cf;
   int real_off;
   int cf_off[TC_MAX_CF];
   int cf_order[TC_MAX_CF];
+};
+
+struct PkCaps {  // what a chunk of a tile's neighbourhood may hold: staged rows, entry pairs
+  int rows, entries;
 };
 
 struct TcArgs {
@@ -79,13 +87,17 @@ struct TcArgs {
   const float* entries;               // (n_entries, 8): (cos, sin) of orders 1..NORD, bias at 2 NORD
   const int* row_order;
   int rows, nlon, D, H, W, NORD;
-  int exact;    // every block is exactly 16 (scalar) / 16 KSC (complex) columns wide and starts on an even column: no padding, 4-byte accesses
-  int use_tma;  // the neighbours' fields have tensor maps (exact 16 / 32-column blocks, aligned, at least one chunk of longitudes)
-  int aligned16;  // the neighbours' fields start on 16-byte boundaries (16-byte per-thread copies allowed)
+  int even;     // every block starts on an even column and has an even width: 4-byte accesses
+  int padded;   // blocks narrower than 16 (scalar) / 16 KSC (complex) columns
+  int unit, units;  // staging: bytes of one copy (16, 8, 4; 2: element by element), copies per head row and field
+  int n_order;      // rows in row_order (all of them: the list is not read)
+  PkCaps caps;                                     // what shared memory holds (a chunk)
+  const int* plan_first;                           // with a plan: (row tiles + 1) first record of a row tile, and the records
+  const unsigned char* records;
+  int n_bh, heavy_bh, light_bh;                    // (sample, head) pairs: all, and per CTA of a polar / any other row tile
+  int heavy_tiles, heavy_ctas;                     // row tiles next to the poles, and the CTAs (the first of the grid) that take them
   float scale;
   TcPlan plan;
-  // tensor maps over the neighbours' fields as (D, nlon, batch * rows): [field][0 = 16-column box, 1 = complex-block box]
-  alignas(64) CUtensorMap maps[2][2];
 };
 
 enum { TC_FWD = 0, TC_BWD_T = 1, TC_BWD_S = 2 };
@@ -100,46 +112,17 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const unsigned (&a)[4], 
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// ---- TMA + mbarrier (single CTA; no multicast)
-__device__ __forceinline__ void mbar_init(unsigned long long* bar, unsigned count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned parity) {
-  unsigned done;
-  asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-               : "=r"(done) : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity) : "memory");
-  return done != 0;
-}
-// bounded wait: gives up after TC_WAIT_LIMIT polls, records it in the device-wide flag and returns false
-__device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
-  for (unsigned tries = 0; tries < TC_WAIT_LIMIT; ++tries) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (tries > 64) __nanosleep(64);
-  }
-  atomicOr(&g_tc_wait_expired, 1);
-  return false;
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, unsigned long long* bar, int x, int y, int z) {
-  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n"
-               ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(reinterpret_cast<unsigned long long>(map)),
-                 "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(x), "r"(y), "r"(z) : "memory");
-}
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-__device__ __forceinline__ void fence_mbar_init() { asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory"); }
-
 // 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, int src_bytes) {
   const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(addr), "l"(src), "r"(src_bytes));
 }
-__device__ __forceinline__ void cp_async4(void* dst, const void* src, int src_bytes) {
-  const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(addr), "l"(src), "r"(src_bytes));
-}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
+template <int BYTES>
+__device__ __forceinline__ void cp_async_ca(void* dst, const void* src) {  // 4 or 8 bytes
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;\n" ::"r"(addr), "l"(src), "n"(BYTES));
+}
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // (re, im) -> (im, -re) / (-im, re): the B operand of the imaginary Gram part for owners carrying q / carrying k
@@ -150,45 +133,6 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<const unsigned*>(&v);
 }
-
-// Head-local PADDED column layout: the scalar block (KS0 k-steps of 16 columns), then each complex
-// frequency (KSC k-steps).  Padding columns are zero on both operands.  Returns the flat column of a
-// padded head-local column, or -1 for padding.
-template <int KS0, int NCF, int KSC>
-__device__ __forceinline__ int flat_column(const TcPlan& P, int h, int c) {
-  if (c < 16 * KS0) return c < P.a0 ? P.real_off + h * P.a0 + c : -1;
-  const int cc = c - 16 * KS0, f = cc / (16 * KSC), r = cc - f * 16 * KSC;
-  return (f < P.n_cf && r < 2 * P.ac) ? P.cf_off[f] + 2 * h * P.ac + r : -1;
-}
-
-// owners per CTA = 8 x warps.  4 warps (32 owners) in every pass: four CTAs per SM at 128 registers (forward, pass T),
-// three at 168 (pass S); 8 warps (64 owners, 80-position chunks) stay instantiable
-constexpr int TN_WARPS(int mode) { return 4; }
-// positions a staged chunk advances by (a multiple of 16): 64 owners + a window of up to 17 fit one chunk of 80, 32 owners
-// + 17 one of 48 (smaller buffers: four CTAs per SM).  Staged per chunk: 8 more, a step of 16 may start 8 before the end.
-constexpr __host__ __device__ int tn_advance(int owners) { return owners >= 64 ? 80 : 48; }
-constexpr __host__ __device__ int tn_rows(int owners) { return tn_advance(owners) + 8; }
-
-template <int KS0, int NCF, int KSC, int TL>
-struct TnLayout {
-  static constexpr __host__ __device__ int align1k(int x) { return (x + 1023) / 1024 * 1024; }
-  static constexpr int REAL_PITCH = 32, CX_PITCH = 32 * KSC;
-  static constexpr int TN_ROWS = tn_rows(TL);
-  static constexpr int REAL_BYTES = KS0 ? align1k(TN_ROWS * REAL_PITCH) : 0;
-  static constexpr int CX_BYTES = align1k(TN_ROWS * CX_PITCH);
-  static constexpr int FIELD_BYTES = REAL_BYTES + NCF * CX_BYTES;
-  static constexpr int ENT_BYTES = (TN_ROWS + TL) * 32;
-  static constexpr int BUFFER_BYTES = align1k(2 * FIELD_BYTES + ENT_BYTES + TN_ROWS * 8);  // with the (lse, Delta) pairs of pass S
-  static __device__ __forceinline__ int real_chunk(int r, int cb) { return r * REAL_PITCH + 16 * (cb ^ ((r >> 2) & 1)); }
-  static __device__ __forceinline__ int cx_chunk(int f, int r, int cb) {
-    return REAL_BYTES + f * CX_BYTES + r * CX_PITCH + 16 * (cb ^ (KSC == 2 ? (r >> 1) & 3 : (r >> 2) & 1));
-  }
-  static __device__ __forceinline__ int chunk(int r, int ch) {
-    if (ch < 2 * KS0) return real_chunk(r, ch);
-    const int cc = ch - 2 * KS0;
-    return cx_chunk(cc / (2 * KSC), r, cc % (2 * KSC));
-  }
-};
 
 __device__ __forceinline__ unsigned movmatrix_trans(unsigned x) {
   unsigned y;
@@ -215,47 +159,25 @@ __device__ __forceinline__ float fast_exp2(float x) {  // ex2.approx: exp2(-inf)
   return y;
 }
 
-// Per-lane byte offsets of the ldmatrix rows inside a sub-tile, for a step starting at staged row 0.  A step starts on
-// a multiple of 8 rows, which leaves the swizzle term of a lane's row unchanged, so a step adds only pl * pitch.
-template <int KS0, int NCF, int KSC, int TL>
-struct TnLaneOffsets {
-  using L = TnLayout<KS0, NCF, KSC, TL>;
-  int g_real, g_cx[KSC];  // Gram A operand: matrices (rows 0-7, k 0-7), (rows 8-15, k 0-7), (rows 0-7, k 8-15), (rows 8-15, k 8-15)
-  int a_real, a_cx[KSC];  // accumulation A operand = tile^T: (cols 0-7, rows 0-7), (cols 8-15, rows 0-7), (cols 0-7, rows 8-15), (cols 8-15, rows 8-15)
-  __device__ __forceinline__ void init(int lane) {
-    const int mi = lane >> 3, rr = lane & 7;
-    g_real = L::real_chunk(8 * (mi & 1) + rr, mi >> 1);
-    a_real = L::real_chunk(8 * (mi >> 1) + rr, mi & 1);
-#pragma unroll
-    for (int sub = 0; sub < KSC; ++sub) {
-      g_cx[sub] = L::cx_chunk(0, 8 * (mi & 1) + rr, 2 * sub + (mi >> 1));
-      a_cx[sub] = L::cx_chunk(0, 8 * (mi >> 1) + rr, 2 * sub + (mi & 1));
-    }
-  }
-};
-
-// S^T blocks of 16 staged rows (pl .. pl + 15) x 8 owners: g0 (scalar block), gr / gi per complex frequency.
+// S^T blocks of 16 packed positions x 8 owners: g0 (scalar block), gr / gi per complex frequency.
 // fb: the owners' fragments, fs: their pre-swapped copies for the imaginary part (complex k-steps only).
-// tile: shared-memory address of the staged field.
-template <int KS0, int NCF, int KSC, int TL>
-__device__ __forceinline__ void gram_step(const unsigned (&fb)[KS0 + NCF * KSC][2], const unsigned (&fs)[NCF * KSC > 0 ? NCF * KSC : 1][2],
-                                          unsigned tile, int pl, const TnLaneOffsets<KS0, NCF, KSC, TL>& lo, float (&g0)[4],
-                                          float (&gr)[NCF > 0 ? NCF : 1][4], float (&gi)[NCF > 0 ? NCF : 1][4]) {
-  using L = TnLayout<KS0, NCF, KSC, TL>;
+// addr: shared-memory address of this lane's position (lane & 15) and half (lane >> 4) of the field's first 16 columns.
+template <int KS0, int NCF, int KSC>
+__device__ __forceinline__ void gram_step(const unsigned (&fb)[KS0 + NCF * KSC][2], const unsigned (&fs)[NCF * KSC][2], unsigned addr, float (&g0)[4],
+                                          float (&gr)[NCF][4], float (&gi)[NCF][4]) {
   if constexpr (KS0 > 0) {
     unsigned af[4];
-    ldsm_x4(af, tile + pl * L::REAL_PITCH + lo.g_real);
+    ldsm_x4(af, addr);
     mma_bf16_b2_init(g0, af, fb[0]);
   } else {
     g0[0] = g0[1] = g0[2] = g0[3] = 0.f;
   }
-  const unsigned cx = tile + pl * L::CX_PITCH;
 #pragma unroll
   for (int f = 0; f < NCF; ++f)
 #pragma unroll
     for (int sub = 0; sub < KSC; ++sub) {
       unsigned af[4];
-      ldsm_x4(af, cx + lo.g_cx[sub] + f * L::CX_BYTES);
+      ldsm_x4(af, addr + 32 * (KS0 + f * KSC + sub));
       if (sub == 0) {
         mma_bf16_b2_init(gr[f], af, fb[KS0 + f * KSC + sub]);
         mma_bf16_b2_init(gi[f], af, fs[f * KSC + sub]);
@@ -266,25 +188,23 @@ __device__ __forceinline__ void gram_step(const unsigned (&fb)[KS0 + NCF * KSC][
     }
 }
 
-// acc^T (padded head columns x 8 owners) += tile^T (columns x 16 staged rows pl .. pl + 15) * B, B = x0 for the scalar block,
+// acc^T (padded head columns x 8 owners) += tile^T (columns x 16 packed positions) * B, B = x0 for the scalar block,
 // xr[f] into the real-phase accumulators and xi[f] into the imaginary-phase accumulators of frequency f.
-template <int KS0, int NCF, int KSC, int TL>
-__device__ __forceinline__ void accumulate_step(float (&acc0)[4], float (&accr)[NCF * KSC > 0 ? NCF * KSC : 1][4], float (&acci)[NCF * KSC > 0 ? NCF * KSC : 1][4],
-                                                const unsigned (&x0)[2], const unsigned (&xr)[NCF > 0 ? NCF : 1][2], const unsigned (&xi)[NCF > 0 ? NCF : 1][2],
-                                                unsigned tile, int pl, const TnLaneOffsets<KS0, NCF, KSC, TL>& lo) {
-  using L = TnLayout<KS0, NCF, KSC, TL>;
+// addr: shared-memory address of position 8 (lane >> 4) + (lane & 7) and half (lane >> 3 & 1) of the field's first 16 columns.
+template <int KS0, int NCF, int KSC>
+__device__ __forceinline__ void accumulate_step(float (&acc0)[4], float (&accr)[NCF * KSC][4], float (&acci)[NCF * KSC][4], const unsigned (&x0)[2],
+                                                const unsigned (&xr)[NCF][2], const unsigned (&xi)[NCF][2], unsigned addr) {
   if constexpr (KS0 > 0) {
     unsigned af[4];
-    ldsm_x4_trans(af, tile + pl * L::REAL_PITCH + lo.a_real);
+    ldsm_x4_trans(af, addr);
     mma_bf16_b2(acc0, af, x0);
   }
-  const unsigned cx = tile + pl * L::CX_PITCH;
 #pragma unroll
   for (int f = 0; f < NCF; ++f)
 #pragma unroll
     for (int sub = 0; sub < KSC; ++sub) {
       unsigned af[4];
-      ldsm_x4_trans(af, cx + lo.a_cx[sub] + f * L::CX_BYTES);
+      ldsm_x4_trans(af, addr + 32 * (KS0 + f * KSC + sub));
       mma_bf16_b2(accr[f * KSC + sub], af, xr[f]);
       mma_bf16_b2(acci[f * KSC + sub], af, xi[f]);
     }
@@ -306,55 +226,57 @@ __device__ __forceinline__ void flat_pair(const TcPlan& P, int h, int col, int& 
   }
 }
 
-// First flat column of k-step / m-tile KT of head h when every block is exactly as wide as its padded slot
+// First flat column of k-step / m-tile KT of head h
 template <int KS0, int NCF, int KSC, int KT>
-__device__ __forceinline__ int exact_block(const TcPlan& P, int h) {
-  if constexpr (KT < KS0) return P.real_off + 16 * h + 16 * KT;
-  else return P.cf_off[(KT - KS0) / KSC] + 16 * KSC * h + 16 * ((KT - KS0) % KSC);
+__device__ __forceinline__ int block_column(const TcPlan& P, int h) {
+  if constexpr (KT < KS0) return P.real_off + P.a0 * h + 16 * KT;
+  else return P.cf_off[(KT - KS0) / KSC] + 2 * P.ac * h + 16 * ((KT - KS0) % KSC);
+}
+// Whether word r of this lane (columns 8 r + 2 c, 8 r + 2 c + 1 of k-step / m-tile KT) holds columns of the head rather than
+// padding, every block being of an even width
+template <int KS0, int NCF, int KSC, int KT>
+__device__ __forceinline__ bool in_block(const TcPlan& P, int c, int r) {
+  return 2 * c + 8 * r + (KT < KS0 ? 16 * KT : 16 * ((KT - KS0) % KSC)) < (KT < KS0 ? P.a0 : 2 * P.ac);
 }
 
 // B-operand fragments of one owner (column n = g of the warp's 8) for every k-step of the padded head layout
 template <int KS0, int NCF, int KSC, int KT = 0>
-__device__ __forceinline__ void load_owner_columns(const TcPlan& P, const __nv_bfloat16* src, bool present, bool exact, bool words, int h, int c,
+__device__ __forceinline__ void load_owner_columns(const TcPlan& P, const __nv_bfloat16* src, bool even, bool words, int h, int c,
                                                    unsigned (&fb)[KS0 + NCF * KSC][2]) {
   if constexpr (KT < KS0 + NCF * KSC) {
-    if (exact) {
-      const unsigned* w = reinterpret_cast<const unsigned*>(src + exact_block<KS0, NCF, KSC, KT>(P, h)) + c;
-      fb[KT][0] = present ? w[0] : 0u;
-      fb[KT][1] = present ? w[4] : 0u;
+    if (even) {
+      const unsigned* w = reinterpret_cast<const unsigned*>(src + block_column<KS0, NCF, KSC, KT>(P, h)) + c;
+      fb[KT][0] = in_block<KS0, NCF, KSC, KT>(P, c, 0) ? w[0] : 0u;
+      fb[KT][1] = in_block<KS0, NCF, KSC, KT>(P, c, 1) ? w[4] : 0u;
     } else {
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         int g0, g1;
         flat_pair<KS0, NCF, KSC, KT>(P, h, 2 * c + 8 * r, g0, g1);
         unsigned w = 0u;
-        if (present) {
-          if (words && g0 >= 0 && g1 == g0 + 1 && (g0 & 1) == 0) {
-            w = *reinterpret_cast<const unsigned*>(src + g0);
-          } else {
-            if (g0 >= 0) w = __bfloat16_as_ushort(src[g0]);
-            if (g1 >= 0) w |= (unsigned)__bfloat16_as_ushort(src[g1]) << 16;
-          }
+        if (words && g0 >= 0 && g1 == g0 + 1 && (g0 & 1) == 0) {
+          w = *reinterpret_cast<const unsigned*>(src + g0);
+        } else {
+          if (g0 >= 0) w = __bfloat16_as_ushort(src[g0]);
+          if (g1 >= 0) w |= (unsigned)__bfloat16_as_ushort(src[g1]) << 16;
         }
         fb[KT][r] = w;
       }
     }
-    load_owner_columns<KS0, NCF, KSC, KT + 1>(P, src, present, exact, words, h, c, fb);
+    load_owner_columns<KS0, NCF, KSC, KT + 1>(P, src, even, words, h, c, fb);
   }
 }
 
 // One m-tile (16 head columns x 8 owners, accumulator layout) of a result -> global memory: transposed in registers
 // (movmatrix) so that a thread holds two adjacent columns of ONE owner (own_b): 4-byte stores.
 template <int KS0, int NCF, int KSC, int KT>
-__device__ __forceinline__ void store_tile(const TcPlan& P, __nv_bfloat16* dst, bool present, bool exact, bool words, int h, int c, const float (&v)[4]) {
+__device__ __forceinline__ void store_tile(const TcPlan& P, __nv_bfloat16* dst, bool present, bool even, bool words, int h, int c, const float (&v)[4]) {
   const unsigned w0 = movmatrix_trans(pack_bf16(v[0], v[1]));  // (owner own_b; columns 2c, 2c + 1)
   const unsigned w1 = movmatrix_trans(pack_bf16(v[2], v[3]));  // (owner own_b; columns 2c + 8, 2c + 9)
-  if (exact) {
-    unsigned* w = reinterpret_cast<unsigned*>(dst + exact_block<KS0, NCF, KSC, KT>(P, h)) + c;
-    if (present) {
-      w[0] = w0;
-      w[4] = w1;
-    }
+  if (even) {
+    unsigned* w = reinterpret_cast<unsigned*>(dst + block_column<KS0, NCF, KSC, KT>(P, h)) + c;
+    if (present && in_block<KS0, NCF, KSC, KT>(P, c, 0)) w[0] = w0;
+    if (present && in_block<KS0, NCF, KSC, KT>(P, c, 1)) w[4] = w1;
     return;
   }
 #pragma unroll
@@ -374,455 +296,733 @@ __device__ __forceinline__ void store_tile(const TcPlan& P, __nv_bfloat16* dst, 
 
 // combine the phase accumulators of every complex m-tile and store all m-tiles of one result
 template <int KS0, int NCF, int KSC, bool CONJ, int M = 0>
-__device__ __forceinline__ void store_result(const TcPlan& P, __nv_bfloat16* dst, bool present, bool exact, bool words, int h, int g, int c,
+__device__ __forceinline__ void store_result(const TcPlan& P, __nv_bfloat16* dst, bool present, bool even, bool words, int h, int g, int c,
                                              const float (&inv)[2],
                                              const float (&acc0)[4], const float (&accr)[NCF * KSC > 0 ? NCF * KSC : 1][4],
                                              const float (&acci)[NCF * KSC > 0 ? NCF * KSC : 1][4]) {
   if constexpr (M == 0 && KS0 > 0) {
     const float v[4] = {acc0[0] * inv[0], acc0[1] * inv[1], acc0[2] * inv[0], acc0[3] * inv[1]};
-    store_tile<KS0, NCF, KSC, 0>(P, dst, present, exact, words, h, c, v);
+    store_tile<KS0, NCF, KSC, 0>(P, dst, present, even, words, h, c, v);
   }
   if constexpr (M < NCF * KSC) {
     // rows of an accumulator m-tile are head columns g, g + 8: even = real part, odd = imaginary part.
-    //   tau:      re = r_re - i_im,  im = r_im + i_re;      conj tau:  re = r_re + i_im,  im = r_im - i_re
-    const float sgn = ((g & 1) != 0) == CONJ ? -1.f : 1.f;
+    // With i the sums under the table's -sin:
+    //   tau:      re = r_re + i_im,  im = r_im - i_re;      conj tau:  re = r_re - i_im,  im = r_im + i_re
+    const float sgn = ((g & 1) != 0) == CONJ ? 1.f : -1.f;
     float v[4];
 #pragma unroll
     for (int x = 0; x < 4; ++x) v[x] = (accr[M][x] + sgn * __shfl_xor_sync(0xffffffffu, acci[M][x], 4)) * inv[x & 1];
-    store_tile<KS0, NCF, KSC, KS0 + M>(P, dst, present, exact, words, h, c, v);
-    store_result<KS0, NCF, KSC, CONJ, M + 1>(P, dst, present, exact, words, h, g, c, inv, acc0, accr, acci);
+    store_tile<KS0, NCF, KSC, KS0 + M>(P, dst, present, even, words, h, c, v);
+    store_result<KS0, NCF, KSC, CONJ, M + 1>(P, dst, present, even, words, h, g, c, inv, acc0, accr, acci);
   }
 }
 
-// A neighbour row of the owner row's walk, prepared once per CTA
-struct TnRowPair {
-  int cnt, lo, z, lon_base;  // window width, first offset, sample * rows + neighbour row, longitude of position 0 (wrapped)
-  int ent_off, pad0, pad1, pad2;
+// ---- packed pairs of floats (one 64-bit register pair, one instruction for two elements)
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned pack_bf16(f32x2 v) {
+  float lo, hi;
+  unpack2(v, lo, hi);
+  return pack_bf16(lo, hi);
+}
+
+// ---- tile shape and shared memory
+constexpr int pk_warps(int mode) { return mode == TC_FWD ? 8 : 4; }  // four owner rows x 8 longitudes per four warps
+constexpr int pk_ctas(int warps) { return warps == 4 ? 3 : 2; }      // per SM: 12 warps of 168 registers, 16 of 128
+constexpr int PK_ROWS = 4;                  // lattice rows of a CTA's owner tile
+constexpr int PK_MAX_SEG = TC_MAX_WIN + PK_ROWS - 1;  // neighbour rows of the tile
+constexpr int PK_DUMMY = 8;                 // entries with bias -inf at the start of the table (a packed list's padding points at the last but one)
+
+template <int KS0, int NCF, int KSC>
+struct PkLayout {
+  static constexpr int KQ = KS0 + NCF * KSC;
+  static constexpr int FIELD = 32 * KQ;         // bytes of one field of a staged row: the scalar block, then every frequency, 32 bytes per k-step
+  static constexpr int PITCH = 2 * FIELD + 16;  // both fields and (lse, Delta): an odd multiple of 16 bytes, so ldmatrix meets no bank conflict
+  static constexpr int ENTRY = 16 * NCF + 8;    // bytes of a table entry pair
 };
 
-template <int KS0, int NCF, int KSC, int MODE, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS, WARPS == 4 ? (MODE == TC_BWD_S ? 3 : 4) : 2) lattice_tn_kernel(const __grid_constant__ TcArgs a) {
-  constexpr int TL = 8 * WARPS, THREADS = 32 * WARPS;
-  constexpr int TN_ADV = tn_advance(TL), TN_ROWS = tn_rows(TL);
-  using L = TnLayout<KS0, NCF, KSC, TL>;
-  constexpr int KQ = KS0 + NCF * KSC, CH = 2 * KQ, NCK = NCF * KSC > 0 ? NCF * KSC : 1;
-  constexpr int NF = NCF > 0 ? NCF : 1;
-  constexpr bool FWD = MODE == TC_FWD, PASS_S = MODE == TC_BWD_S;
-  extern __shared__ __align__(1024) unsigned char smem_dyn[];
-  // swizzled sub-tiles must start on 1024-byte boundaries of the shared-memory window: align by hand (1 KB of slack is requested)
-  unsigned char* const smem_raw = smem_dyn + ((1024u - ((unsigned)__cvta_generic_to_shared(smem_dyn) & 1023u)) & 1023u);
-  __shared__ __align__(8) unsigned long long copy_bar[2];  // completion of the TMA copies into buffer 0 / 1
-  __shared__ __align__(16) TnRowPair pairs_s[TC_MAX_WIN];
-  __shared__ int n_pairs_s, failed_s;
-  const TcPlan& P = a.plan;
-  // two buffers, each: field 1 sub-tiles | field 2 sub-tiles | entries 2 x (TN_ROWS + TL, 4) fp32 | stats (TN_ROWS, 2) fp32 (pass S)
-  constexpr int buf_bytes = L::BUFFER_BYTES;
-  // a staged table entry (8 floats) is split into two arrays of 4 floats: the 16-byte reads of the phases then sit at a
-  // 16-byte pitch (no bank conflicts between neighbouring offsets); the bias is float 2 NCF of the entry
-  constexpr int ENT_HALF = 4 * (TN_ROWS + TL);
-  constexpr int bias_at = 2 * NCF < 4 ? 2 * NCF : ENT_HALF + 2 * NCF - 4;  // the tables hold exactly the orders 1 .. NCF (host-checked)
-  auto tile1 = [&](int buf) { return smem_raw + buf * buf_bytes; };
-  auto tile2 = [&](int buf) { return smem_raw + buf * buf_bytes + L::FIELD_BYTES; };
-  auto entry = [&](int buf) { return reinterpret_cast<float*>(smem_raw + buf * buf_bytes + 2 * L::FIELD_BYTES); };
-  auto stats = [&](int buf) { return reinterpret_cast<float*>(smem_raw + buf * buf_bytes + 2 * L::FIELD_BYTES + L::ENT_BYTES); };
+struct PkSegment {  // one neighbour row of the tile: its row, first longitude offset from the tile's first column, staged positions
+  int j, lo, len;
+};
+struct PkCursor {
+  int seg, at;  // next segment, positions of it already taken
+};
+struct PkWindows {  // the tables a tile's neighbourhood is read from
+  const int *win_cnt, *win_lo, *win_off;
+  const float* entries;  // (n_entries, 8)
+  int rows, nlon, W;
+};
+struct PkTile {  // a tile's neighbour rows, in shared memory
+  int4 win[PK_ROWS][PK_MAX_SEG];  // of (owner row, neighbour row): count, first offset, first entry
+  PkSegment seg[PK_MAX_SEG];      // the non-empty neighbour rows
+  int n_seg;
+};
+struct PkPair {
+  int h;
+  int64_t row0, node0;  // first node of the warp's owner row, of the sample
+};
+struct PkChunk {
+  int rows, entries, steps;  // staged rows, entry pairs (with the dummies), this warp's steps of 16 positions
+};
 
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
-  const int tiles = (a.nlon + TL - 1) / TL;
-  const int row = a.row_order[blockIdx.x / tiles];
-  const int c0 = (blockIdx.x % tiles) * TL;
-  const int h = blockIdx.y;
-  const int64_t b = blockIdx.z;
-  const int64_t node0 = (b * a.rows + row) * (int64_t)a.nlon;
-  const int own_b = 8 * warp + g;      // the owner whose column this thread holds in B fragments (and stores in the epilogue)
-  const int own_c = 8 * warp + 2 * c;  // the owners (own_c, own_c + 1) of this thread's accumulator columns
-  const float cscale = a.scale * TC_LOG2E;
-  const bool words = (a.D & 1) == 0;   // 4-byte accesses to (even column, next column) are aligned
-  const bool exact = a.exact != 0;
-  TnLaneOffsets<KS0, NCF, KSC, TL> lane_off;
-  lane_off.init(lane);
-
-  // ---- the walk's row pairs, once per CTA: warp 0 compacts the non-empty ones (one lane per neighbour row)
-  if (warp == 0) {
+// The windows of the rows r0 .. r0 + 3, and the neighbour rows some of them see.  Ends with a barrier.
+template <int WARPS>
+__device__ __forceinline__ void pk_open_tile(const PkWindows& t, int r0, PkTile& tile) {
+  constexpr int TLON = 8 * (WARPS / PK_ROWS);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, spans = 2 * t.W + PK_ROWS;
+  for (int x = threadIdx.x; x < spans * PK_ROWS; x += 32 * WARPS) {
+    const int i = x & (PK_ROWS - 1), s = x / PK_ROWS, j = r0 - t.W + s, w = s - i;  // w: place of row j in owner row i's windows
+    int4 v = make_int4(0, 0, 0, 0);
+    if (r0 + i < t.rows && j >= 0 && j < t.rows && w >= 0 && w <= 2 * t.W) {
+      const int at = (r0 + i) * (2 * t.W + 1) + w;
+      v = make_int4(t.win_cnt[at], t.win_lo[at], t.win_off[at], 0);
+    }
+    tile.win[i][s] = v;
+  }
+  __syncthreads();
+  if (warp == 0) {  // compact the non-empty neighbour rows
     int filled = 0;
-    for (int x0 = 0; x0 < 2 * a.W + 1; x0 += 32) {
-      const int x = x0 + lane, j = row + x - a.W;
-      int cnt = 0;
-      if (x < 2 * a.W + 1 && j >= 0 && j < a.rows) cnt = a.win_cnt[row * (2 * a.W + 1) + x];
-      const unsigned have = __ballot_sync(0xffffffffu, cnt > 0);
-      if (cnt > 0) {
-        const int widx = row * (2 * a.W + 1) + x;
-        TnRowPair rp;
-        rp.cnt = cnt;
-        rp.lo = a.win_lo[widx];
-        rp.z = (int)(b * a.rows + j);
-        rp.lon_base = tc_wrap(c0 + rp.lo, a.nlon);
-        rp.ent_off = a.win_off[widx];
-        rp.pad0 = rp.pad1 = rp.pad2 = 0;
-        pairs_s[filled + __popc(have & ((1u << lane) - 1u))] = rp;
+    for (int s0 = 0; s0 < spans; s0 += 32) {
+      const int s = s0 + lane;
+      int lo = 0x7fffffff, hi = -0x7fffffff;
+      int4 w[PK_ROWS];
+#pragma unroll
+      for (int i = 0; i < PK_ROWS; ++i) {
+        w[i] = s < spans ? tile.win[i][s] : make_int4(0, 0, 0, 0);
+        if (w[i].x > 0) {
+          lo = min(lo, w[i].y);
+          hi = max(hi, w[i].y + w[i].x);
+        }
       }
+      const unsigned have = __ballot_sync(0xffffffffu, hi > lo);
+      const int k = filled + __popc(have & ((1u << lane) - 1u));
+      __syncwarp();
+      if (hi > lo) {
+        tile.seg[k] = PkSegment{r0 - t.W + s, lo, hi - lo + TLON - 1};
+#pragma unroll
+        for (int i = 0; i < PK_ROWS; ++i) tile.win[i][k] = w[i];  // k <= s: only places that have been read
+      }
+      __syncwarp();
       filled += __popc(have);
     }
-    if (lane == 0) n_pairs_s = filled;
+    if (lane == 0) tile.n_seg = filled;
   }
-  if (!a.use_tma)  // per-thread staging leaves rows beyond a window and padding columns untouched: they must be finite
-    for (int x = threadIdx.x; x < 2 * buf_bytes / 16; x += THREADS) reinterpret_cast<uint4*>(smem_raw)[x] = make_uint4(0, 0, 0, 0);
-  // a step of 16 rows may end beyond the window: the weights there are zero, and zero times whatever an earlier kernel left
-  // in the statistics' slots need not be
-  if constexpr (PASS_S)
-    for (int x = threadIdx.x; x < 4 * TN_ROWS; x += THREADS) stats(x & 1)[x >> 1] = 0.f;
-  if (threadIdx.x == 0) {
-    failed_s = 0;
-    mbar_init(&copy_bar[0], 1);
-    mbar_init(&copy_bar[1], 1);
-    fence_mbar_init();
-  }
-
-  // owners' fragments (loop-invariant B operands) and their pre-swapped copies:
-  //   owners carry q: Im = sum_cols tile[col] * q'[col], q' = (-q_im, q_re);   owners carry k: k' = (k_im, -k_re)
-  unsigned f1[KQ][2], s1[NCK][2], f2[FWD ? 1 : KQ][2], s2[FWD ? 1 : NCK][2];
-  const bool own_b_present = c0 + own_b < a.nlon;
-  const int64_t own_b_base = (node0 + c0 + own_b) * a.D;
-  load_owner_columns<KS0, NCF, KSC>(P, a.own1 + own_b_base, own_b_present, exact, words, h, c, f1);
-#pragma unroll
-  for (int kc = 0; kc < NCF * KSC; ++kc)
-#pragma unroll
-    for (int r = 0; r < 2; ++r) s1[kc][r] = PASS_S ? swap_neg(f1[KS0 + kc][r]) : swap_neg_lo(f1[KS0 + kc][r]);
-  if constexpr (!FWD) {
-    load_owner_columns<KS0, NCF, KSC>(P, a.own2 + own_b_base, own_b_present, exact, words, h, c, f2);
-#pragma unroll
-    for (int kc = 0; kc < NCF * KSC; ++kc)
-#pragma unroll
-      for (int r = 0; r < 2; ++r) s2[kc][r] = PASS_S ? swap_neg(f2[KS0 + kc][r]) : swap_neg_lo(f2[KS0 + kc][r]);
-  }
-  float lse_o[2] = {0.f, 0.f}, dl_o[2] = {0.f, 0.f};  // pass T: the two accumulator-column owners' lse (base 2) and Delta
-  if constexpr (MODE == TC_BWD_T) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e)
-      if (c0 + own_c + e < a.nlon) lse_o[e] = a.lse[(node0 + c0 + own_c + e) * a.H + h] * TC_LOG2E;
-    if (a.delta_out != nullptr) {
-      // Delta = <dO, O> over the head's columns of owner own_b: this thread holds 2 of every 8 columns of dO (f2);
-      // the same columns of O, then the four lanes of the owner add up.  Written for the source-major pass, and handed
-      // to the lanes that hold the owner as an accumulator column.
-      unsigned of[KQ][2];
-      load_owner_columns<KS0, NCF, KSC>(P, a.out_fwd + own_b_base, own_b_present, exact, words, h, c, of);
-      float d = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < KQ; ++ks)
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-          d = fmaf(__uint_as_float(f2[ks][r] << 16), __uint_as_float(of[ks][r] << 16), d);
-          d = fmaf(__uint_as_float(f2[ks][r] & 0xffff0000u), __uint_as_float(of[ks][r] & 0xffff0000u), d);
-        }
-      d += __shfl_xor_sync(0xffffffffu, d, 1);
-      d += __shfl_xor_sync(0xffffffffu, d, 2);
-      if (c == 0 && own_b_present) a.delta_out[(node0 + c0 + own_b) * a.H + h] = d;
-#pragma unroll
-      for (int e = 0; e < 2; ++e) dl_o[e] = __shfl_sync(0xffffffffu, d, (2 * c + e) << 2);
-    } else {
-#pragma unroll
-      for (int e = 0; e < 2; ++e)
-        if (c0 + own_c + e < a.nlon) dl_o[e] = a.delta[(node0 + c0 + own_c + e) * a.H + h];
-    }
-  }
-  float a1_0[4] = {0.f, 0.f, 0.f, 0.f}, a1_r[NCK][4], a1_i[NCK][4];
-  float a2_0[4] = {0.f, 0.f, 0.f, 0.f}, a2_r[PASS_S ? NCK : 1][4], a2_i[PASS_S ? NCK : 1][4];
-#pragma unroll
-  for (int m = 0; m < NCK; ++m)
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      a1_r[m][x] = a1_i[m][x] = 0.f;
-      if constexpr (PASS_S) a2_r[m][x] = a2_i[m][x] = 0.f;
-    }
-  float m_o[2] = {-1e30f, -1e30f}, l_o[2] = {0.f, 0.f};  // forward: reference maximum (base-2 logits), partial sums of the two owners
   __syncthreads();
-  const int n_pairs = n_pairs_s;
+}
 
-  // ---- stages = (row pair, chunk of its window), produced in order by a cursor that runs one stage ahead of the consumer
-  struct Consumed {   // what the consumer of a stage needs to know about it
-    int p0, cnt;      // first position of the chunk, window width
-    bool tma;         // staged by tensor copies (completion on the copy barrier)
-  };
-  int next_pair = 0, next_p0 = 0;  // the producer cursor
-  // per-thread slot of the cp.async path: thread -> (row within a pass, 16-byte chunk of the padded head row)
-  constexpr int ROWS_PER_PASS = THREADS / CH;
-  const int st_row = threadIdx.x / CH, st_ch = threadIdx.x - st_row * CH;
-  const bool st_active = st_row < ROWS_PER_PASS;
-  auto issue_next = [&](int buf) -> Consumed {  // asynchronous copies of the cursor's stage into buffer `buf`; advances the cursor
-    const int4 ra = *reinterpret_cast<const int4*>(&pairs_s[next_pair]);  // cnt, lo, z, lon_base
-    const int ent_off = pairs_s[next_pair].ent_off;
-    const int cnt = ra.x, z = ra.z, p0 = next_p0;
-    const int n_rows = min(TN_ROWS, TL + cnt - 1 - p0);
-    int lon0 = ra.w + p0;
-    if (lon0 >= a.nlon) lon0 %= a.nlon;
-    const bool tma = a.use_tma && lon0 + n_rows <= a.nlon;  // consecutive longitudes: no wrap at the seam
-    if (p0 + TN_ADV < TL + cnt - 1) {
-      next_p0 = p0 + TN_ADV;
-    } else {
-      ++next_pair;
-      next_p0 = 0;
+// One chunk: as many neighbour positions as `caps` allows, from the cursor on (which advances).  Every warp works the chunk
+// out for itself, lane p looking after the p-th segment; chunk boundaries depend on the tables alone, not on which rows are
+// asked for.  Written: the staged rows' nodes through put_node(row, neighbour row, offset from the tile's first column), the
+// entry pairs (phase, stride caps.entries; bias), and this warp's list of packed positions if it wants one.  `write` false:
+// nothing, the chunk is only measured.
+template <int NCF, int WARPS, typename PutNode>
+__device__ __forceinline__ PkChunk pk_build(const PkWindows& t, const PkTile& tile, PkCursor& cur, PkCaps caps, int pitch16, bool write, bool wants,
+                                            float4* phase, float2* bias, unsigned* list, const PutNode& put_node) {
+  constexpr int TLON = 8 * (WARPS / PK_ROWS);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, my_row = warp & (PK_ROWS - 1), l0 = 8 * (warp / PK_ROWS);
+  const int R = caps.rows, E = caps.entries, n_seg = tile.n_seg;
+  const int s = cur.seg + lane;
+  const bool have = s < n_seg;
+  const PkSegment sg = have ? tile.seg[s] : PkSegment{0, 0, 0};
+  const int skip = lane == 0 ? cur.at : 0, len = have ? sg.len - skip : 0;
+  int before = len;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += y;
+  }
+  before -= len;
+  int take = min(min(len, max(R - before, 0)), (E - PK_DUMMY) / PK_ROWS - TLON);
+  const unsigned cut = __ballot_sync(0xffffffffu, take < len || !have);
+  if (cut != 0 && lane > __ffs(cut) - 1) take = 0;
+  const int ua = sg.lo + skip;  // the piece's first offset from the tile's first column
+  int xa = 0, xn = 0, eb = 0, entries = 0;  // my row's entries of the piece: first offset, count, place
+  int4 win = make_int4(0, 0, 0, 0);
+#pragma unroll
+  for (int i = 0; i < PK_ROWS; ++i) {
+    const int4 w = have ? tile.win[i][s] : make_int4(0, 0, 0, 0);
+    const int from = max(w.y - 6, ua - TLON + 2), to = min(w.y + w.x + 7, ua + take);
+    const int n = take > 0 && w.x > 0 ? max(to - from, 0) : 0;
+    if (i == my_row) {
+      xa = from;
+      xn = n;
+      eb = entries;
+      win = w;
     }
-    unsigned char* d1 = tile1(buf);
-    unsigned char* d2 = tile2(buf);
-    if (tma) {
-      if (threadIdx.x == 0) {
-        // the buffer was last touched through the generic proxy (ldmatrix, per-thread stores): order those first
-        fence_proxy_async();
-        mbar_expect_tx(&copy_bar[buf], 2u * TN_ROWS * (KS0 * L::REAL_PITCH + NCF * L::CX_PITCH));
-        if constexpr (KS0 > 0) {
-          tma_load_3d(d1, &a.maps[0][0], &copy_bar[buf], P.real_off + h * 16, lon0, z);
-          tma_load_3d(d2, &a.maps[1][0], &copy_bar[buf], P.real_off + h * 16, lon0, z);
-        }
+    entries += n;
+  }
+  int e_before = entries;
 #pragma unroll
-        for (int f = 0; f < NCF; ++f) {
-          tma_load_3d(d1 + L::REAL_BYTES + f * L::CX_BYTES, &a.maps[0][1], &copy_bar[buf], P.cf_off[f] + h * 16 * KSC, lon0, z);
-          tma_load_3d(d2 + L::REAL_BYTES + f * L::CX_BYTES, &a.maps[1][1], &copy_bar[buf], P.cf_off[f] + h * 16 * KSC, lon0, z);
-        }
-      }
-    } else if (st_active) {
-      const int st_g0 = flat_column<KS0, NCF, KSC>(P, h, 8 * st_ch), st_g7 = flat_column<KS0, NCF, KSC>(P, h, 8 * st_ch + 7);
-      const bool whole = st_g0 >= 0 && st_g7 == st_g0 + 7 && (a.D % 8 == 0) && (st_g0 % 8 == 0) && a.aligned16;  // one aligned 16-byte chunk of real columns
-      const bool pad = st_g0 < 0 && st_g7 < 0 && flat_column<KS0, NCF, KSC>(P, h, 8 * st_ch + 3) < 0;  // all padding (stays zero)
-      if (!pad) {
-        // this thread's chunk of every row: block base + row * pitch + 16 (chunk ^ swizzle(row))
-        const bool in_real = st_ch < 2 * KS0;
-        const int cc = st_ch - 2 * KS0;
-        const int blk = in_real ? 0 : L::REAL_BYTES + (cc / (2 * KSC)) * L::CX_BYTES, cb = in_real ? st_ch : cc % (2 * KSC);
-        const int pitch = in_real ? L::REAL_PITCH : L::CX_PITCH;
-        const bool wide = !in_real && KSC == 2;  // 64-byte rows
-        const __nv_bfloat16* src1 = a.nb1 + (int64_t)z * a.nlon * a.D + st_g0;
-        const __nv_bfloat16* src2 = a.nb2 + (int64_t)z * a.nlon * a.D + st_g0;
-        int lon = lon0 + st_row;
-        if (lon >= a.nlon) lon %= a.nlon;
-        const int step = ROWS_PER_PASS % a.nlon;
-        // with tensor maps in use the buffer may hold anything beyond the window: write zeros there (copies of size 0)
-        const int rows_to_write = a.use_tma ? TN_ROWS : n_rows;
-        for (int pl = st_row; pl < rows_to_write; pl += ROWS_PER_PASS) {
-          const int off = blk + pl * pitch + 16 * (cb ^ (wide ? (pl >> 1) & 3 : (pl >> 2) & 1));
-          const int64_t nb = (int64_t)lon * a.D;
-          if (whole) {
-            const int bytes = pl < n_rows ? 16 : 0;
-            cp_async16(d1 + off, src1 + nb, bytes);
-            cp_async16(d2 + off, src2 + nb, bytes);
-          } else {  // a chunk that straddles padding or is misaligned: element by element (visible after the barrier)
-            unsigned short u1[8], u2[8];
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, e_before, o);
+    if (lane >= o) e_before += y;
+  }
+  if (e_before > E - PK_DUMMY) take = 0;  // a suffix of the pieces: the counts are never negative
+  eb += e_before - entries + PK_DUMMY;
+  const unsigned taken = __ballot_sync(0xffffffffu, take > 0);
+  const int pieces = __popc(taken), last = pieces - 1;
+  PkChunk chunk;
+  chunk.rows = pieces ? __shfl_sync(0xffffffffu, before + take, last) : 0;
+  chunk.entries = PK_DUMMY + (pieces ? __shfl_sync(0xffffffffu, e_before, last) : 0);
+  const int last_take = __shfl_sync(0xffffffffu, take, last), last_len = __shfl_sync(0xffffffffu, len, last), last_skip = __shfl_sync(0xffffffffu, skip, last);
+  // my positions of the piece
+  const int pa = max(ua, win.y + l0), pn = wants && take > 0 && win.x > 0 ? max(min(ua + take, win.y + win.x + l0 + 7) - pa, 0) : 0;
+  int placed = 0;
+  for (int p = 0; p < pieces; ++p) {
+    const int ln = __shfl_sync(0xffffffffu, pn, p);
+    if (write) {
+      const int base = __shfl_sync(0xffffffffu, before, p), u = __shfl_sync(0xffffffffu, ua, p), n = __shfl_sync(0xffffffffu, take, p);
+      const int px = __shfl_sync(0xffffffffu, xa, p), pxn = __shfl_sync(0xffffffffu, xn, p), pe = __shfl_sync(0xffffffffu, eb, p);
+      const int wlo = __shfl_sync(0xffffffffu, win.y, p), wcnt = __shfl_sync(0xffffffffu, win.x, p), woff = __shfl_sync(0xffffffffu, win.z, p);
+      const int lu = __shfl_sync(0xffffffffu, pa, p), j = __shfl_sync(0xffffffffu, sg.j, p);
+      if ((p & (WARPS - 1)) == warp)
+        for (int x = lane; x < n; x += 32) put_node(base + x, j, u + x);
+      if (WARPS == PK_ROWS || (p & 1) == warp / PK_ROWS)
+        for (int x = lane; x < pxn; x += 32) {
+          float e0[8], e1[8];
+          const int at = px + x - wlo;
 #pragma unroll
-            for (int x = 0; x < 8; ++x) {
-              const int gx = pl < n_rows ? flat_column<KS0, NCF, KSC>(P, h, 8 * st_ch + x) : -1;
-              u1[x] = gx >= 0 ? __bfloat16_as_ushort(src1[nb + gx - st_g0]) : (unsigned short)0;
-              u2[x] = gx >= 0 ? __bfloat16_as_ushort(src2[nb + gx - st_g0]) : (unsigned short)0;
+          for (int z = 0; z < 2; ++z) {
+            float* e = z ? e1 : e0;
+            const bool ok = at - z >= 0 && at - z < wcnt;
+            const float4* src = reinterpret_cast<const float4*>(t.entries + (size_t)(woff + (ok ? at - z : 0)) * 8);
+            const float4 v0 = __ldg(src);
+            e[0] = v0.x; e[1] = v0.y; e[2] = v0.z; e[3] = v0.w;
+            if constexpr (NCF >= 2) {
+              const float4 v1 = __ldg(src + 1);
+              e[4] = v1.x; e[5] = v1.y; e[6] = v1.z; e[7] = v1.w;
             }
-            *reinterpret_cast<uint4*>(d1 + off) =
-                make_uint4(u1[0] | (u1[1] << 16), u1[2] | (u1[3] << 16), u1[4] | (u1[5] << 16), u1[6] | (u1[7] << 16));
-            *reinterpret_cast<uint4*>(d2 + off) =
-                make_uint4(u2[0] | (u2[1] << 16), u2[2] | (u2[3] << 16), u2[4] | (u2[5] << 16), u2[6] | (u2[7] << 16));
+            e[2 * NCF] = ok ? TC_LOG2E * e[2 * NCF] : -INFINITY;
           }
-          lon += step;
-          if (lon >= a.nlon) lon -= a.nlon;
+#pragma unroll
+          for (int f = 0; f < NCF; ++f) phase[f * E + pe + x] = make_float4(e0[2 * f], e1[2 * f], -e0[2 * f + 1], -e1[2 * f + 1]);
+          bias[pe + x] = make_float2(e0[2 * NCF], e1[2 * NCF]);
         }
+      for (int x = lane; x < ln; x += 32)
+        list[placed + x] = (unsigned)((base + lu + x - u) * pitch16) | (unsigned)(pe + lu + x - l0 - px) << 16;
+    }
+    placed += ln;
+  }
+  chunk.steps = (placed + 15) / 16;
+  if (write)
+    for (int x = placed + lane; x < 16 * chunk.steps; x += 32) list[x] = (unsigned)(R * pitch16) | (PK_DUMMY - 2u) << 16;
+  if (last_take < last_len) {
+    cur.seg += last;
+    cur.at = last_skip + last_take;
+  } else {
+    cur.seg += pieces;
+    cur.at = 0;
+  }
+  return chunk;
+}
+
+// ---- plans: what every longitude tile of a row tile has in common, worked out once per table
+constexpr int PK_HEADER = 16;  // ints at the start of a chunk's record: staged rows, entry pairs, then every warp's steps
+// A record: header, staged rows (rows x 2 ints: first node of the neighbour row, longitude offset), entry pairs as in shared
+// memory, lists (warp x rows)
+template <int NCF>
+__host__ __device__ inline int pk_record_bytes(PkCaps caps, int warps) {
+  return 4 * PK_HEADER + 8 * caps.rows + caps.entries * (16 * NCF + 8) + 4 * warps * caps.rows;
+}
+struct PkRecord {
+  const int* header;
+  const int2* nodes;
+  const float4* phase;
+  const float2* bias;
+  const unsigned* list;
+};
+template <int NCF>
+__device__ __forceinline__ PkRecord pk_record(const unsigned char* plan, int64_t index, PkCaps caps, int warps) {
+  const unsigned char* p = plan + index * pk_record_bytes<NCF>(caps, warps);
+  const unsigned char* phase = p + 4 * PK_HEADER + 8 * caps.rows;
+  const unsigned char* bias = phase + (size_t)16 * NCF * caps.entries;
+  return PkRecord{reinterpret_cast<const int*>(p), reinterpret_cast<const int2*>(p + 4 * PK_HEADER), reinterpret_cast<const float4*>(phase),
+                  reinterpret_cast<const float2*>(bias), reinterpret_cast<const unsigned*>(bias + (size_t)8 * caps.entries)};
+}
+
+// A CTA per row tile.  records null: counts[tile] = its chunks; else its chunks' records from first[tile] on.
+template <int NCF, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) lattice_plan_kernel(PkWindows t, PkCaps caps, int pitch16, int* counts, const int* first, unsigned char* records) {
+  __shared__ PkTile tile;
+  const int r0 = blockIdx.x * PK_ROWS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = r0 + (warp & (PK_ROWS - 1));
+  pk_open_tile<WARPS>(t, r0, tile);
+  PkCursor cur{0, 0};
+  int n = 0;
+  do {
+    PkRecord rec{};
+    if (records) rec = pk_record<NCF>(records, first[blockIdx.x] + n, caps, WARPS);
+    int2* nodes = const_cast<int2*>(rec.nodes);
+    float4* phase = const_cast<float4*>(rec.phase);
+    float2* bias = const_cast<float2*>(rec.bias);
+    const PkChunk chunk = pk_build<NCF, WARPS>(t, tile, cur, caps, pitch16, records != nullptr, row < t.rows, phase, bias,
+                                               const_cast<unsigned*>(rec.list) + (records ? warp * caps.rows : 0),
+                                               [&](int r, int j, int u) { nodes[r] = make_int2(j * t.nlon, tc_wrap(u, t.nlon)); });
+    if (records) {
+      int* header = const_cast<int*>(rec.header);
+      if (threadIdx.x == 0) {
+        header[0] = chunk.rows;
+        header[1] = chunk.entries;
+      }
+      if (lane == 0) header[2 + warp] = chunk.steps;
+      if (threadIdx.x < PK_DUMMY) {
+        bias[threadIdx.x] = make_float2(-INFINITY, -INFINITY);
+        for (int f = 0; f < NCF; ++f) phase[f * caps.entries + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
-    // table entries of the offsets x = p - owner the chunk can meet (clamped: validity is decided from x itself)
-    float* de = entry(buf);
-    const float* ent = a.entries + (size_t)ent_off * 8;
-    static_assert(2 * (TN_ROWS + TL - 1) <= 2 * THREADS, "two guarded copies per thread cover a chunk's entries");
+    ++n;
+  } while (cur.seg < tile.n_seg);
+  if (!records && threadIdx.x == 0) counts[blockIdx.x] = n;
+}
+
+template <int KS0, int NCF, int KSC, int MODE, int WARPS, bool PLANNED>
+__global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_kernel(const __grid_constant__ TcArgs a) {
+  using L = PkLayout<KS0, NCF, KSC>;
+  constexpr int THREADS = 32 * WARPS, TLON = 8 * (WARPS / PK_ROWS);
+  constexpr int KQ = L::KQ, NCK = NCF * KSC, PITCH = L::PITCH, FIELD = L::FIELD;
+  constexpr bool FWD = MODE == TC_FWD, PASS_S = MODE == TC_BWD_S;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ typename std::conditional<PLANNED, char, PkTile>::type tile_desc;
+  __shared__ int member_s;
+  const TcPlan& P = a.plan;
+  const int R = a.caps.rows, E = a.caps.entries, LIST = R;
+  unsigned char* const tile_s = smem;                                                   // (R + 1) rows, the last all zeros
+  unsigned char* const phase_s = tile_s + (size_t)(R + 1) * PITCH;                      // NCF arrays of E x (cos x, cos x - 1, -sin x, -sin x - 1)
+  float2* const bias_s = reinterpret_cast<float2*>(phase_s + (size_t)NCF * 16 * E);     // E x (bias x, bias x - 1), times log2 e
+  unsigned* const list_s = reinterpret_cast<unsigned*>(bias_s + E);                     // per warp LIST x (row offset / 16 | entry << 16)
+  int* const node_s = reinterpret_cast<int*>(list_s + WARPS * LIST);                    // R staged rows: node within the sample
+
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
+  // ---- which tile, which (sample, head) pairs: the first heavy_ctas CTAs take the row tiles next to the poles
+  const int lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
+  int row_tile, lon_tile, bh, bh_end;
+  {
+    int x = blockIdx.x;
+    if (x < a.heavy_ctas) {
+      lon_tile = x % lon_tiles;
+      x /= lon_tiles;
+      const int chunks = (a.n_bh + a.heavy_bh - 1) / a.heavy_bh;
+      bh = (x % chunks) * a.heavy_bh;
+      bh_end = min(bh + a.heavy_bh, a.n_bh);
+      row_tile = x / chunks;
+    } else {
+      x -= a.heavy_ctas;
+      lon_tile = x % lon_tiles;
+      x /= lon_tiles;
+      const int light = row_tiles - a.heavy_tiles;
+      row_tile = a.heavy_tiles + x % light;
+      bh = (x / light) * a.light_bh;
+      bh_end = min(bh + a.light_bh, a.n_bh);
+    }
+    row_tile = (int)from_both_ends(row_tile, row_tiles);
+  }
+  const int r0 = row_tile * PK_ROWS, c0 = lon_tile * TLON;
+  const int my_row = warp & (PK_ROWS - 1), row = r0 + my_row, l0 = 8 * (warp / PK_ROWS);
+  const float cscale = a.scale * TC_LOG2E;
+  const bool words = (a.D & 1) == 0;  // 4-byte accesses to (even column, next column) are aligned
+  const bool even = a.even != 0;
+
+  // ---- setup, once per CTA: which rows are asked for
+  if (threadIdx.x == 0) member_s = a.n_order == a.rows ? (1 << PK_ROWS) - 1 : 0;
+  for (int x = threadIdx.x; x < PITCH / 16; x += THREADS) reinterpret_cast<uint4*>(tile_s + (size_t)R * PITCH)[x] = make_uint4(0, 0, 0, 0);
+  if (a.padded)  // padding columns are never copied: they must be zero
+    for (int x = threadIdx.x; x < R * (PITCH / 16); x += THREADS) reinterpret_cast<uint4*>(tile_s)[x] = make_uint4(0, 0, 0, 0);
+  if constexpr (!PLANNED)
+    for (int x = threadIdx.x; x < PK_DUMMY; x += THREADS) {
+      bias_s[x] = make_float2(-INFINITY, -INFINITY);
+      for (int f = 0; f < NCF; ++f) reinterpret_cast<float4*>(phase_s)[f * E + x] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  __syncthreads();
+  if (a.n_order != a.rows) {
+    int mine = 0;
+    for (int x = threadIdx.x; x < a.n_order; x += THREADS) {
+      const int d = a.row_order[x] - r0;
+      if (d >= 0 && d < PK_ROWS) mine |= 1 << d;
+    }
+    if (mine) atomicOr(&member_s, mine);
+    __syncthreads();
+  }
+  if (member_s == 0) return;
+  const bool active = (member_s >> my_row & 1) && row < a.rows && c0 + l0 < a.nlon;  // this warp has owners to write
+
+  // ---- the chunks of the tile's neighbourhood: from the plan, or worked out here
+  const PkWindows windows{a.win_cnt, a.win_lo, a.win_off, a.entries, a.rows, a.nlon, a.W};
+  PkCursor cur{0, 0};
+  int chunk = 0, n_chunks = 1;
+  if constexpr (PLANNED) {
+    chunk = a.plan_first[row_tile];
+    n_chunks = a.plan_first[row_tile + 1] - chunk;
+  } else {
+    pk_open_tile<WARPS>(windows, r0, tile_desc);
+  }
+  const int first_chunk = chunk;
+  int n_rows = 0, n_steps = 0;
+  // the next chunk (the first one again after the last): staged rows' nodes, entry pairs, lists; its copies join the fields'
+  auto load_chunk = [&](bool restart) {
+    if constexpr (PLANNED) {
+      if (restart) chunk = first_chunk;
+      const PkRecord rec = pk_record<NCF>(a.records, chunk, a.caps, WARPS);
+      n_rows = rec.header[0];
+      const int n_entries = rec.header[1];
+      n_steps = active ? rec.header[2 + warp] : 0;
+      ++chunk;
+      for (int r = threadIdx.x; r < n_rows; r += THREADS) {
+        const int2 at = rec.nodes[r];
+        const int lon = c0 + at.y;  // both below nlon
+        node_s[r] = at.x + (lon >= a.nlon ? lon - a.nlon : lon);
+      }
+      float4* const phase = reinterpret_cast<float4*>(phase_s);
 #pragma unroll
-    for (int it = 0; it < 2; ++it) {
-      const int idx = threadIdx.x + it * THREADS;
-      if (idx < 2 * (n_rows + TL - 1)) {
-        const int xi = idx >> 1, part = idx & 1;
-        const int x = min(max(xi + p0 - (TL - 1), 0), cnt - 1);
-        cp_async16(de + 4 * xi + part * ENT_HALF, ent + 8 * x + 4 * part, 16);  // the two halves of an entry go to separate arrays
+      for (int f = 0; f < NCF; ++f)
+        for (int x = threadIdx.x; x < n_entries; x += THREADS) cp_async16(phase + f * E + x, rec.phase + f * E + x, 16);
+      for (int x = threadIdx.x; 2 * x < n_entries; x += THREADS) cp_async16(bias_s + 2 * x, rec.bias + 2 * x, 16);
+      for (int x = lane; x < 4 * n_steps; x += 32) cp_async16(list_s + warp * LIST + 4 * x, rec.list + warp * LIST + 4 * x, 16);
+    } else {
+      if (restart) cur = PkCursor{0, 0};
+      const PkChunk built = pk_build<NCF, WARPS>(windows, tile_desc, cur, a.caps, PITCH / 16, true, active, reinterpret_cast<float4*>(phase_s), bias_s,
+                                                 list_s + warp * LIST, [&](int r, int j, int u) { node_s[r] = j * a.nlon + tc_wrap(c0 + u, a.nlon); });
+      n_rows = built.rows;
+      n_steps = built.steps;
+    }
+  };
+  auto more_chunks = [&]() {
+    if constexpr (PLANNED) return chunk < first_chunk + n_chunks;
+    else return cur.seg < tile_desc.n_seg;
+  };
+
+  // ---- staging: a thread keeps one unit (2 .. 16 bytes) of the head's columns and strides the staged rows
+  const int units = a.units, per_pass = THREADS / units, st_row = threadIdx.x / units;
+  int st_block, st_stride, st_dst;  // flat column of the unit for head 0, columns from head to head, byte in the staged field
+  {
+    const int u = (threadIdx.x - st_row * units) * a.unit;  // byte within the head's columns, unpadded
+    if (u < 2 * P.a0) {
+      st_block = P.real_off + u / 2;
+      st_stride = P.a0;
+      st_dst = u;
+    } else {
+      const int v = u - 2 * P.a0, f = v / (4 * P.ac), w = v - f * 4 * P.ac;
+      st_block = P.cf_off[f < NCF ? f : 0] + w / 2;
+      st_stride = 2 * P.ac;
+      st_dst = 32 * KS0 + f * 32 * KSC + w;
+    }
+  }
+  auto issue = [&](const PkPair& at_pair) {  // asynchronous copies of the chunk's rows of a (sample, head) pair
+    const int h = at_pair.h;
+    const int64_t node0 = at_pair.node0;
+    if (st_row < per_pass) {
+      const int64_t col = node0 * a.D + st_block + (int64_t)h * st_stride;
+      const __nv_bfloat16 *s1 = a.nb1 + col, *s2 = a.nb2 + col;
+      unsigned char* d = tile_s + st_dst + st_row * PITCH;
+      if (a.unit == 16) {
+        for (int r = st_row; r < n_rows; r += per_pass, d += per_pass * PITCH) {
+          const int64_t at = (int64_t)node_s[r] * a.D;
+          cp_async16(d, s1 + at, 16);
+          cp_async16(d + FIELD, s2 + at, 16);
+        }
+      } else if (a.unit == 8) {
+        for (int r = st_row; r < n_rows; r += per_pass, d += per_pass * PITCH) {
+          const int64_t at = (int64_t)node_s[r] * a.D;
+          cp_async_ca<8>(d, s1 + at);
+          cp_async_ca<8>(d + FIELD, s2 + at);
+        }
+      } else if (a.unit == 4) {
+        for (int r = st_row; r < n_rows; r += per_pass, d += per_pass * PITCH) {
+          const int64_t at = (int64_t)node_s[r] * a.D;
+          cp_async_ca<4>(d, s1 + at);
+          cp_async_ca<4>(d + FIELD, s2 + at);
+        }
+      } else {  // odd columns: element by element
+        for (int r = st_row; r < n_rows; r += per_pass, d += per_pass * PITCH) {
+          const int64_t at = (int64_t)node_s[r] * a.D;
+          *reinterpret_cast<__nv_bfloat16*>(d) = s1[at];
+          *reinterpret_cast<__nv_bfloat16*>(d + FIELD) = s2[at];
+        }
       }
     }
     if constexpr (PASS_S) {
-      float* ds = stats(buf);
-      for (int idx = threadIdx.x; idx < 2 * n_rows; idx += THREADS) {
-        const int pl = idx >> 1, which = idx & 1;
-        int lon = lon0 + pl;
-        if (lon >= a.nlon) lon %= a.nlon;
-        const int64_t nn = ((int64_t)z * a.nlon + lon) * a.H + h;
-        cp_async4(ds + 2 * pl + which, (which ? a.delta : a.lse) + nn, 4);
+      for (int r = threadIdx.x; r < n_rows; r += THREADS) {
+        const int64_t at = (node0 + node_s[r]) * a.H + h;
+        cp_async_ca<4>(tile_s + r * PITCH + 2 * FIELD, a.lse + at);
+        cp_async_ca<4>(tile_s + r * PITCH + 2 * FIELD + 4, a.delta + at);
       }
     }
     cp_async_commit();
-    return Consumed{p0, cnt, tma};
   };
 
-  bool have = n_pairs > 0;
-  int buf = 0;
-  unsigned parity = 0;  // bit b: the phase of copy_bar[b] the next TMA stage into buffer b completes
-  Consumed cur{0, 0, false};
-  if (have) cur = issue_next(0);
-  while (have) {
-    const bool have_next = next_pair < n_pairs;
-    Consumed nxt{0, 0, false};
-    if (have_next) {
-      nxt = issue_next(buf ^ 1);
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
-    }
-    if (cur.tma) {  // one warp watches the copy barrier; the others block in the CTA barrier below without issuing
-      if (warp == 0 && !mbar_wait(&copy_bar[buf], (parity >> buf) & 1u)) failed_s = 1;
-      parity ^= 1u << buf;
-    }
-    __syncthreads();
-    const unsigned t1 = (unsigned)__cvta_generic_to_shared(tile1(buf));
-    const unsigned t2 = (unsigned)__cvta_generic_to_shared(tile2(buf));
-    const float* e_s = entry(buf);
-    const float* stat_s = stats(buf);
-    const int p0 = cur.p0, cnt = cur.cnt;
+  const int own_b = l0 + g;      // the owner whose column this thread holds in B fragments (and stores in the epilogue)
+  const int own_c = l0 + 2 * c;  // the owners (own_c, own_c + 1) of this thread's accumulator columns
+  const bool own_b_present = active && c0 + own_b < a.nlon;
+  const unsigned tile_addr = (unsigned)__cvta_generic_to_shared(tile_s);
+  const unsigned gram_lane = tile_addr + 16 * (lane >> 4), sum_lane = tile_addr + 16 * (lane >> 3 & 1);
+  const int sum_pos = 8 * (lane >> 4) + (lane & 7);
+  const unsigned char* const phase_lane = phase_s - 32 * c;
+  const float2* const bias_lane = bias_s - 2 * c;
+  const unsigned* const my_list = list_s + warp * LIST;
+  const f32x2 cscale2 = pack2(cscale, cscale);
 
-    // ---- this warp's steps inside the chunk: 16 positions each, on the lattice 8 warp + 16 i
-    const int p_first = p0 > 8 * warp ? p0 + ((8 * warp) & 8) : 8 * warp;
-    const int p_end = min(p0 + TN_ADV, 8 * warp + 7 + cnt);
-    for (int p = p_first; p < p_end; p += 16) {
-      const int pl = p - p0;
-      // element x of a fragment: position pl + g + 8 (x >> 1), owner own_c + (x & 1)
-      float lg[4], tr[NF][4], ti[NF][4];
-      bool valid[4];
-      const float* e_lane = e_s + 4 * (pl + g - own_c + (TL - 1));  // staged entry (first half) of the offset p - owner, element 0
-      const int off0 = p0 + pl + g - own_c;
-      {
-        float s0[4], sr[NF][4], si[NF][4];
-        gram_step<KS0, NCF, KSC, TL>(f1, s1, t1, pl, lane_off, s0, sr, si);
+  load_chunk(true);
+  const bool single = !more_chunks();  // the whole neighbourhood is one chunk: lists and entries serve every (sample, head)
+  __syncthreads();
+  // owners' fragments (B operands) and their pre-swapped copies:
+  //   owners carry q: Im = sum_cols tile[col] * q'[col], q' = (-q_im, q_re);   owners carry k: k' = (k_im, -k_re)
+  unsigned f1[KQ][2], s1[NCK][2], f2[FWD ? 1 : KQ][2], s2[FWD ? 1 : NCK][2], of[MODE == TC_BWD_T ? KQ : 1][2];
+  float lse_o[2] = {0.f, 0.f}, dl_o[2] = {0.f, 0.f};  // pass T: the two accumulator-column owners' lse (base 2) and Delta
+  const int lon_b = min(c0 + own_b, a.nlon - 1);      // an owner beyond the last longitude reads that one's; nothing of it is written
+  auto fetch_owners = [&](const PkPair& at) {  // loads only; used by finish_owners
+    if (!active) return;
+    const int64_t base = (at.row0 + lon_b) * a.D;
+    load_owner_columns<KS0, NCF, KSC>(P, a.own1 + base, even, words, at.h, c, f1);
+    if constexpr (!FWD) load_owner_columns<KS0, NCF, KSC>(P, a.own2 + base, even, words, at.h, c, f2);
+    if constexpr (MODE == TC_BWD_T) {
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const float* e = e_lane + 4 * (8 * (x >> 1) - (x & 1));
-          valid[x] = (unsigned)(off0 + 8 * (x >> 1) - (x & 1)) < (unsigned)cnt;
-          float sum = s0[x];
-          float tau[2 * NF];
-          if constexpr (NCF >= 2) {  // complex frequencies are the orders 1 .. NCF: the first two phases are the entry's first 16 bytes
-            const float4 t = *reinterpret_cast<const float4*>(e);
-            tau[0] = t.x; tau[1] = t.y; tau[2] = t.z; tau[3] = t.w;
-            if constexpr (NCF == 3) {
-              const float2 t3 = *reinterpret_cast<const float2*>(e + ENT_HALF);
-              tau[4] = t3.x; tau[5] = t3.y;
-            }
-          } else if constexpr (NCF == 1) {
-            const float2 t = *reinterpret_cast<const float2*>(e);
-            tau[0] = t.x; tau[1] = t.y;
+      for (int e = 0; e < 2; ++e) {
+        const int64_t x = (at.row0 + min(c0 + own_c + e, a.nlon - 1)) * a.H + at.h;
+        lse_o[e] = a.lse[x] * TC_LOG2E;
+        if (a.delta_out == nullptr) dl_o[e] = a.delta[x];
+      }
+      if (a.delta_out != nullptr) load_owner_columns<KS0, NCF, KSC>(P, a.out_fwd + base, even, words, at.h, c, of);
+    }
+  };
+  auto finish_owners = [&](const PkPair& at) {
+    if (!active) return;
+#pragma unroll
+    for (int kc = 0; kc < NCK; ++kc)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        s1[kc][r] = PASS_S ? swap_neg(f1[KS0 + kc][r]) : swap_neg_lo(f1[KS0 + kc][r]);
+        if constexpr (!FWD) s2[kc][r] = PASS_S ? swap_neg(f2[KS0 + kc][r]) : swap_neg_lo(f2[KS0 + kc][r]);
+      }
+    if constexpr (MODE == TC_BWD_T)
+      if (a.delta_out != nullptr) {
+        // Delta = <dO, O> over the head's columns of owner own_b: this thread holds 2 of every 8 columns of dO (f2) and O,
+        // then the four lanes of the owner add up.  Written for the source-major pass, and handed to the lanes that hold
+        // the owner as an accumulator column.
+        float d = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < KQ; ++ks)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            d = fmaf(__uint_as_float(f2[ks][r] << 16), __uint_as_float(of[ks][r] << 16), d);
+            d = fmaf(__uint_as_float(f2[ks][r] & 0xffff0000u), __uint_as_float(of[ks][r] & 0xffff0000u), d);
           }
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        if (c == 0 && own_b_present) a.delta_out[(at.row0 + c0 + own_b) * a.H + at.h] = d;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) dl_o[e] = __shfl_sync(0xffffffffu, d, (2 * c + e) << 2);
+      }
+  };
+  // the (sample, head) pairs in turn, heads fastest
+  PkPair pair{bh % a.H, ((int64_t)(bh / a.H) * a.rows + row) * a.nlon, (int64_t)(bh / a.H) * a.rows * a.nlon};
+  auto following = [&](const PkPair& at) {
+    const bool wrap = at.h + 1 == a.H;
+    const int64_t sample = wrap ? (int64_t)a.rows * a.nlon : 0;
+    return PkPair{wrap ? 0 : at.h + 1, at.row0 + sample, at.node0 + sample};
+  };
+  issue(pair);
+  if constexpr (!PASS_S) fetch_owners(pair);
+  for (;; ++bh) {
+    if constexpr (PASS_S) fetch_owners(pair);
+    finish_owners(pair);
+    float a1_0[4] = {0.f, 0.f, 0.f, 0.f}, a1_r[NCK][4], a1_i[NCK][4];
+    float a2_0[4] = {0.f, 0.f, 0.f, 0.f}, a2_r[PASS_S ? NCK : 1][4], a2_i[PASS_S ? NCK : 1][4];
+#pragma unroll
+    for (int m = 0; m < NCK; ++m)
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        a1_r[m][x] = a1_i[m][x] = 0.f;
+        if constexpr (PASS_S) a2_r[m][x] = a2_i[m][x] = 0.f;
+      }
+    float m_o[2] = {-1e30f, -1e30f}, l_o[2] = {0.f, 0.f};  // forward: reference maximum (base-2 logits), partial sums of the two owners
+
+    for (;;) {
+      cp_async_wait<0>();
+      __syncthreads();
+      // ---- this warp's steps: 16 packed positions each
+      const unsigned* at = my_list;
+      unsigned at_gram = at[lane & 15], at_sum = at[sum_pos], at_e0 = at[g], at_e1 = at[g + 8];
+      for (int step = 0; step < n_steps; ++step) {
+        const unsigned gram_addr = gram_lane + (at_gram & 0xffffu) * 16u, sum_addr = sum_lane + (at_sum & 0xffffu) * 16u;
+        const unsigned w0 = at_e0, w1 = at_e1;
+        at += 16;  // the next step's (behind the last one's: not used)
+        at_gram = at[lane & 15];
+        at_sum = at[sum_pos];
+        at_e0 = at[g];
+        at_e1 = at[g + 8];
+        // element x of a fragment: packed position g + 8 (x >> 1), owner own_c + (x & 1)
+        f32x2 tr[2][NCF], nti[2][NCF];  // cos, -sin of the elements (0, 1) and (2, 3)
+        float2 bias[2];
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          const unsigned e = (y ? w1 : w0) >> 16;
 #pragma unroll
           for (int f = 0; f < NCF; ++f) {
-            tr[f][x] = tau[2 * f];
-            ti[f][x] = tau[2 * f + 1];
-            sum = fmaf(tau[2 * f], sr[f][x], sum);
-            sum = fmaf(-tau[2 * f + 1], si[f][x], sum);
+            const ulonglong2 t = *reinterpret_cast<const ulonglong2*>(phase_lane + 16 * (f * E + e));
+            tr[y][f] = t.x;
+            nti[y][f] = t.y;
           }
-          lg[x] = valid[x] ? fmaf(cscale, sum, TC_LOG2E * e[bias_at]) : -INFINITY;  // -inf: outside the window
+          bias[y] = bias_lane[e];
         }
-      }
-      float w1[4], w2[4];  // the weights the two accumulations use: forward p | pass T ds | pass S ds, p
-      if constexpr (FWD) {
-        // online softmax over the 16 positions: column maxima over this thread's rows, then across the 8 row groups.
-        // The reference maximum of an owner only moves when the new maximum exceeds it by more than 2^8 (weights stay
-        // below 256: exact in the normalised result), so most steps skip the rescaling of the accumulators.
-        // whether some owner's maximum has to move can be told from each thread's own four logits: most steps skip the
-        // column maxima (six shuffles) as well as the rescaling
-        const bool grow = fmaxf(lg[0], lg[2]) > m_o[0] + 8.f || fmaxf(lg[1], lg[3]) > m_o[1] + 8.f;
-        if (__any_sync(0xffffffffu, grow)) {
-          float mx[2] = {fmaxf(lg[0], lg[2]), fmaxf(lg[1], lg[3])};
+        float w[4], p[4];  // the weights the two accumulations use: forward p | pass T ds | pass S ds, p
+        {
+          float s0[4], sr[NCF][4], si[NCF][4];
+          gram_step<KS0, NCF, KSC>(f1, s1, gram_addr, s0, sr, si);
 #pragma unroll
-          for (int d = 4; d < 32; d <<= 1) {
-            mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], d));
-            mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], d));
+          for (int y = 0; y < 2; ++y) {
+            f32x2 sum = pack2(s0[2 * y], s0[2 * y + 1]);
+#pragma unroll
+            for (int f = 0; f < NCF; ++f) {
+              sum = fma2(tr[y][f], pack2(sr[f][2 * y], sr[f][2 * y + 1]), sum);
+              sum = fma2(nti[y][f], pack2(si[f][2 * y], si[f][2 * y + 1]), sum);
+            }
+            sum = fma2(cscale2, sum, pack2(bias[y].x, bias[y].y));
+            unpack2(sum, p[2 * y], p[2 * y + 1]);
           }
-          const float nm[2] = {mx[0] > m_o[0] + 8.f ? mx[0] : m_o[0], mx[1] > m_o[1] + 8.f ? mx[1] : m_o[1]};
-          const float corr[2] = {fast_exp2(m_o[0] - nm[0]), fast_exp2(m_o[1] - nm[1])};
-          m_o[0] = nm[0]; m_o[1] = nm[1];
-          l_o[0] *= corr[0]; l_o[1] *= corr[1];
+        }
+        const bool ok[4] = {bias[0].x > -INFINITY, bias[0].y > -INFINITY, bias[1].x > -INFINITY, bias[1].y > -INFINITY};
+        if constexpr (FWD) {
+          // online softmax over the 16 positions.  The reference maximum of an owner only moves when the new maximum exceeds
+          // it by more than 2^8 (weights stay below 256: exact in the normalised result); whether some owner's has to move
+          // can be told from each thread's own four logits: most steps skip the column maxima as well as the rescaling
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+            if (!ok[x]) p[x] = -INFINITY;  // outside the window, whatever the neighbour holds
+          const bool grow = fmaxf(p[0], p[2]) > m_o[0] + 8.f || fmaxf(p[1], p[3]) > m_o[1] + 8.f;
+          if (__any_sync(0xffffffffu, grow)) {
+            float mx[2] = {fmaxf(p[0], p[2]), fmaxf(p[1], p[3])};
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) {
+              mx[0] = fmaxf(mx[0], __shfl_xor_sync(0xffffffffu, mx[0], d));
+              mx[1] = fmaxf(mx[1], __shfl_xor_sync(0xffffffffu, mx[1], d));
+            }
+            const float nm[2] = {mx[0] > m_o[0] + 8.f ? mx[0] : m_o[0], mx[1] > m_o[1] + 8.f ? mx[1] : m_o[1]};
+            const float corr[2] = {fast_exp2(m_o[0] - nm[0]), fast_exp2(m_o[1] - nm[1])};
+            m_o[0] = nm[0]; m_o[1] = nm[1];
+            l_o[0] *= corr[0]; l_o[1] *= corr[1];
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              a1_0[x] *= corr[x & 1];
+#pragma unroll
+              for (int m = 0; m < NCK; ++m) { a1_r[m][x] *= corr[x & 1]; a1_i[m][x] *= corr[x & 1]; }
+            }
+          }
 #pragma unroll
           for (int x = 0; x < 4; ++x) {
-            a1_0[x] *= corr[x & 1];
+            w[x] = fast_exp2(p[x] - m_o[x & 1]);
+            l_o[x & 1] += w[x];
+          }
+        } else {
+          // p from the logits first (the (q, k) Gram blocks die here), then d alpha from the (dO, v) Gram blocks
+          float delta[4];
 #pragma unroll
-            for (int m = 0; m < NCF * KSC; ++m) { a1_r[m][x] *= corr[x & 1]; a1_i[m][x] *= corr[x & 1]; }
+          for (int y = 0; y < 2; ++y) {
+            float lse[2] = {lse_o[0], lse_o[1]};
+            delta[2 * y] = dl_o[0];
+            delta[2 * y + 1] = dl_o[1];
+            if constexpr (PASS_S) {
+              const float2 st = *reinterpret_cast<const float2*>(tile_s + ((y ? w1 : w0) & 0xffffu) * 16u + 2 * FIELD);
+              lse[0] = lse[1] = st.x * TC_LOG2E;
+              delta[2 * y] = delta[2 * y + 1] = st.y;
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x) p[2 * y + x] = ok[2 * y + x] ? fast_exp2(p[2 * y + x] - lse[x]) : 0.f;
+          }
+          float h0[4], hr[NCF][4], hi[NCF][4];
+          gram_step<KS0, NCF, KSC>(f2, s2, gram_addr + FIELD, h0, hr, hi);
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            f32x2 dal = pack2(h0[2 * y], h0[2 * y + 1]);
+#pragma unroll
+            for (int f = 0; f < NCF; ++f) {
+              dal = fma2(tr[y][f], pack2(hr[f][2 * y], hr[f][2 * y + 1]), dal);
+              dal = fma2(nti[y][f], pack2(hi[f][2 * y], hi[f][2 * y + 1]), dal);
+            }
+            float d0, d1;
+            unpack2(dal, d0, d1);
+            w[2 * y] = a.scale * p[2 * y] * (d0 - delta[2 * y]);
+            w[2 * y + 1] = a.scale * p[2 * y + 1] * (d1 - delta[2 * y + 1]);
           }
         }
+        // B operands: the weights (x phase parts), transposed to (owner column, position rows)
+        auto operands = [&](const float (&v)[4], unsigned (&x0)[2], unsigned (&xr)[NCF][2], unsigned (&xi)[NCF][2]) {
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          w1[x] = fast_exp2(lg[x] - m_o[x & 1]);
-          l_o[x & 1] += w1[x];
-        }
-      } else {
-        // p from the logits first (the (q, k) Gram blocks die here), then d alpha from the (dO, v) Gram blocks
-        float delta[4];
+          for (int y = 0; y < 2; ++y) {
+            const f32x2 v2 = pack2(v[2 * y], v[2 * y + 1]);
+            x0[y] = movmatrix_trans(pack_bf16(v2));
 #pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          float lse;
-          if (PASS_S) {
-            const float2 st = *reinterpret_cast<const float2*>(stat_s + 2 * (pl + g + 8 * (x >> 1)));
-            lse = st.x * TC_LOG2E; delta[x] = st.y;
-          } else {
-            lse = lse_o[x & 1]; delta[x] = dl_o[x & 1];
+            for (int f = 0; f < NCF; ++f) {
+              xr[f][y] = movmatrix_trans(pack_bf16(mul2(v2, tr[y][f])));
+              xi[f][y] = movmatrix_trans(pack_bf16(mul2(v2, nti[y][f])));
+            }
           }
-          w2[x] = valid[x] ? fast_exp2(lg[x] - lse) : 0.f;
-        }
-        float h0[4], hr[NF][4], hi[NF][4];
-        gram_step<KS0, NCF, KSC, TL>(f2, s2, t2, pl, lane_off, h0, hr, hi);
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          float dal = h0[x];
-#pragma unroll
-          for (int f = 0; f < NCF; ++f) {
-            dal = fmaf(tr[f][x], hr[f][x], dal);
-            dal = fmaf(-ti[f][x], hi[f][x], dal);
+        };
+        unsigned x0[2], xr[NCF][2], xi[NCF][2];
+        operands(w, x0, xr, xi);
+        if constexpr (FWD) {
+          accumulate_step<KS0, NCF, KSC>(a1_0, a1_r, a1_i, x0, xr, xi, sum_addr + FIELD);  // out += (p tau) v
+        } else {
+          accumulate_step<KS0, NCF, KSC>(a1_0, a1_r, a1_i, x0, xr, xi, sum_addr);  // dq += (ds tau) k  |  dk += (ds conj tau) q
+          if constexpr (PASS_S) {
+            operands(p, x0, xr, xi);
+            accumulate_step<KS0, NCF, KSC>(a2_0, a2_r, a2_i, x0, xr, xi, sum_addr + FIELD);  // dv += (p conj tau) dO
           }
-          w1[x] = a.scale * w2[x] * (dal - delta[x]);
         }
       }
-      // B operands: the weights (x phase parts), transposed to (owner column, position rows)
-      unsigned x0[2], xr[NF][2], xim[NF][2];
-      x0[0] = movmatrix_trans(pack_bf16(w1[0], w1[1]));
-      x0[1] = movmatrix_trans(pack_bf16(w1[2], w1[3]));
-#pragma unroll
-      for (int f = 0; f < NCF; ++f) {
-        xr[f][0] = movmatrix_trans(pack_bf16(w1[0] * tr[f][0], w1[1] * tr[f][1]));
-        xr[f][1] = movmatrix_trans(pack_bf16(w1[2] * tr[f][2], w1[3] * tr[f][3]));
-        xim[f][0] = movmatrix_trans(pack_bf16(w1[0] * ti[f][0], w1[1] * ti[f][1]));
-        xim[f][1] = movmatrix_trans(pack_bf16(w1[2] * ti[f][2], w1[3] * ti[f][3]));
+      // ---- the next chunk, or the next pair's copies: under way while this pair's results are written
+      const bool more = more_chunks();
+      if (!more && bh + 1 >= bh_end) break;
+      __syncthreads();  // everyone is done with the tile, the lists and the entries
+      if (!single) {
+        load_chunk(!more);
+        __syncthreads();
       }
-      if constexpr (FWD) {
-        accumulate_step<KS0, NCF, KSC, TL>(a1_0, a1_r, a1_i, x0, xr, xim, t2, pl, lane_off);  // out += (p tau) v
+      if (more) {
+        issue(pair);
       } else {
-        accumulate_step<KS0, NCF, KSC, TL>(a1_0, a1_r, a1_i, x0, xr, xim, t1, pl, lane_off);  // dq += (ds tau) k  |  dk += (ds conj tau) q
-        if constexpr (PASS_S) {
-          x0[0] = movmatrix_trans(pack_bf16(w2[0], w2[1]));
-          x0[1] = movmatrix_trans(pack_bf16(w2[2], w2[3]));
-#pragma unroll
-          for (int f = 0; f < NCF; ++f) {
-            xr[f][0] = movmatrix_trans(pack_bf16(w2[0] * tr[f][0], w2[1] * tr[f][1]));
-            xr[f][1] = movmatrix_trans(pack_bf16(w2[2] * tr[f][2], w2[3] * tr[f][3]));
-            xim[f][0] = movmatrix_trans(pack_bf16(w2[0] * ti[f][0], w2[1] * ti[f][1]));
-            xim[f][1] = movmatrix_trans(pack_bf16(w2[2] * ti[f][2], w2[3] * ti[f][3]));
-          }
-          accumulate_step<KS0, NCF, KSC, TL>(a2_0, a2_r, a2_i, x0, xr, xim, t2, pl, lane_off);  // dv += (p conj tau) dO
-        }
+        issue(following(pair));
+        break;
       }
     }
-    __syncthreads();  // everyone is done with `buf` before the stage after next is copied into it
-    cur = nxt;
-    have = have_next;
-    buf ^= 1;
-  }
+    const PkPair done = pair;
+    if (bh + 1 < bh_end) {
+      pair = following(pair);
+      if constexpr (!PASS_S) fetch_owners(pair);  // (the source-major pass has no registers for them beside its results)
+    }
 
-  // ---- epilogue: normalise, combine the two phase accumulators (multiplication by +-i = pair swap across rows g, g ^ 1),
-  // transpose in registers, store
-  float inv[2] = {1.f, 1.f};
-  if constexpr (FWD) {
+    // ---- epilogue: normalise, combine the two phase accumulators (multiplication by +-i = pair swap across rows g, g ^ 1),
+    // transpose in registers, store
+    if (active) {
+      float inv[2] = {1.f, 1.f};
+      if constexpr (FWD) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
+        for (int e = 0; e < 2; ++e) {
 #pragma unroll
-      for (int d = 4; d < 32; d <<= 1) l_o[e] += __shfl_xor_sync(0xffffffffu, l_o[e], d);
-      inv[e] = l_o[e] > 0.f ? 1.f / l_o[e] : 0.f;
-      if (g == 0 && c0 + own_c + e < a.nlon)
-        a.lse_out[(node0 + c0 + own_c + e) * a.H + h] = l_o[e] > 0.f ? (m_o[e] + log2f(l_o[e])) * TC_LN2 : -INFINITY;
+          for (int d = 4; d < 32; d <<= 1) l_o[e] += __shfl_xor_sync(0xffffffffu, l_o[e], d);
+          inv[e] = l_o[e] > 0.f ? 1.f / l_o[e] : 0.f;
+          if (g == 0 && c0 + own_c + e < a.nlon)
+            a.lse_out[(done.row0 + c0 + own_c + e) * a.H + done.h] = l_o[e] > 0.f ? (m_o[e] + log2f(l_o[e])) * TC_LN2 : -INFINITY;
+        }
+      }
+      const int64_t base = (done.row0 + c0 + own_b) * a.D;
+      store_result<KS0, NCF, KSC, PASS_S>(P, a.res1 + base, own_b_present, even, words, done.h, g, c, inv, a1_0, a1_r, a1_i);
+      if constexpr (PASS_S) store_result<KS0, NCF, KSC, true>(P, a.res2 + base, own_b_present, even, words, done.h, g, c, inv, a2_0, a2_r, a2_i);
     }
+    if (bh + 1 >= bh_end) break;
   }
-  // a wait that ran out anywhere in this CTA poisons its results (NaN) instead of passing half-filled tiles on as numbers
-  if (*(volatile int*)&failed_s != 0) inv[0] = inv[1] = __int_as_float(0x7fc00000);
-  store_result<KS0, NCF, KSC, PASS_S>(P, a.res1 + own_b_base, own_b_present, exact, words, h, g, c, inv, a1_0, a1_r, a1_i);
-  if constexpr (PASS_S) store_result<KS0, NCF, KSC, true>(P, a.res2 + own_b_base, own_b_present, exact, words, h, g, c, inv, a2_0, a2_r, a2_i);
 }
 
 // Delta[node, h] = <dO, O> over the head's columns
@@ -900,83 +1100,122 @@ int make_tc_plan(const int64_t* desc_host, int F, int H, int D, TcPlan& P) {
   return GM_OK;
 }
 
-// GM_LATTICE_TMA=0 stages every chunk with per-thread copies (for comparing the two staging paths)
-bool tma_disabled() {
-  const char* v = getenv("GM_LATTICE_TMA");
-  return v && v[0] == '0';
+// Staged rows and entry pairs of a tile whose windows are as narrow as this lattice's get (its equator), from the halo W
+// alone: a neighbourhood of W + 1/2 rows' radius, longitudes scaled by the lattice's aspect.
+void narrow_tile(int rows_of, int nlon, int W, int tile_lons, int& rows, int& entries) {
+  const double aspect = nlon / (2.0 * rows_of);
+  rows = entries = 0;
+  for (int s = -W; s < W + PK_ROWS; ++s) {
+    int widest = 0;
+    for (int i = 0; i < PK_ROWS; ++i) {
+      const int d = s > i ? s - i : i - s;
+      if (d > W) continue;
+      const double chord = sqrt((W + 0.5) * (W + 0.5) - (double)d * d) * aspect;
+      const int cnt = (int)fmin(2.0 * floor(chord) + 1.0, (double)nlon);
+      widest = cnt > widest ? cnt : widest;
+      entries += cnt + 13;
+    }
+    rows += widest + tile_lons - 1;
+  }
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point lookup (no link against the driver library)
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-  static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-    void* sym = nullptr;
-    cudaDriverEntryPointQueryResult res;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &res) != cudaSuccess || res != cudaDriverEntryPointSuccess)
-      sym = nullptr;
-    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(sym);
-  }();
-  return fn;
-}
-
-// Tensor map over one bf16 field seen as (D columns, nlon longitudes, batch * rows): boxes of `box_cols` columns x `box_rows`
-// (box_rows) longitudes of one lattice row, written to shared memory in the swizzle that spans the box's rows.
-bool encode_field_map(CUtensorMap* map, const void* field, int D, int nlon, int64_t slabs, int box_cols, int box_rows) {
-  auto encode = tensor_map_encoder();
-  if (!encode) return false;
-  const cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)nlon, (cuuint64_t)slabs};
-  const cuuint64_t strides[2] = {(cuuint64_t)D * 2, (cuuint64_t)nlon * D * 2};
-  const cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
-  const cuuint32_t estr[3] = {1, 1, 1};
-  const CUtensorMapSwizzle swz = box_cols == 16 ? CU_TENSOR_MAP_SWIZZLE_32B : CU_TENSOR_MAP_SWIZZLE_64B;
-  return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(field), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+// Shared memory of a chunk: room for the narrow tiles' whole neighbourhood (lists and entries then serve every (sample,
+// head) pair of a CTA) with a margin for wider ones, for as many CTAs per SM as that allows.
+template <int KS0, int NCF, int KSC, int WARPS>
+size_t chunk_caps(int rows_of, int nlon, int W, PkCaps& caps) {
+  using L = PkLayout<KS0, NCF, KSC>;
+  constexpr int TLON = 8 * (WARPS / PK_ROWS);
+  int want_rows, want_entries;
+  narrow_tile(rows_of, nlon, W, TLON, want_rows, want_entries);
+  const size_t per_row = L::PITCH + 4 * WARPS + 4, per_entry = L::ENTRY;
+  const double ratio = (double)want_entries / want_rows;
+  for (int ctas = pk_ctas(WARPS);; --ctas) {
+    const size_t budget = 227 * 1024 / ctas - 4096;  // the system's 1 KB and the static arrays
+    const size_t fixed = 2 * L::PITCH + 64 * WARPS + 16 * PK_DUMMY * NCF + 1024 + 4 * (TLON + 8) * per_entry;
+    int rows = (int)((budget - fixed) / (per_row + ratio * per_entry));
+    if (rows < want_rows && ctas > 2) continue;
+    rows = rows < want_rows * 2 ? rows : want_rows * 2;
+    rows = rows < 32 ? 32 : rows;
+    caps.rows = rows / 16 * 16;
+    caps.entries = (int)(ratio * caps.rows) / 8 * 8 + 4 * (TLON + 8) + PK_DUMMY;
+    return (size_t)(caps.rows + 1) * L::PITCH + (size_t)caps.entries * L::ENTRY + (size_t)(WARPS + 1) * caps.rows * 4;
+  }
 }
 
 template <int KS0, int NCF, int KSC, int MODE>
 int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
-  constexpr int WARPS = TN_WARPS(MODE), TL = 8 * WARPS, TN_ROWS = tn_rows(TL);
-  using L = TnLayout<KS0, NCF, KSC, TL>;
-  a.aligned16 = reinterpret_cast<uintptr_t>(a.nb1) % 16 == 0 && reinterpret_cast<uintptr_t>(a.nb2) % 16 == 0;
-  bool tma = !tma_disabled() && a.D % 8 == 0 && a.nlon >= TN_ROWS && batch * a.rows < (1ll << 31) && (KS0 == 0 || (a.plan.a0 == 16 && a.plan.real_off % 8 == 0)) &&
-             2 * a.plan.ac == 16 * KSC && reinterpret_cast<uintptr_t>(a.nb1) % 16 == 0 && reinterpret_cast<uintptr_t>(a.nb2) % 16 == 0;
-  for (int f = 0; f < a.plan.n_cf; ++f) tma = tma && a.plan.cf_off[f] % 8 == 0;
-  if (tma) {
-    const void* fields[2] = {a.nb1, a.nb2};
-    for (int x = 0; x < 2 && tma; ++x) {
-      if (KS0 > 0) tma = tma && encode_field_map(&a.maps[x][0], fields[x], a.D, a.nlon, batch * a.rows, 16, TN_ROWS);
-      tma = tma && encode_field_map(&a.maps[x][1], fields[x], a.D, a.nlon, batch * a.rows, 16 * KSC, TN_ROWS);
-    }
-  }
-  a.use_tma = tma ? 1 : 0;
-  bool exact = (KS0 == 0 || a.plan.a0 == 16) && 2 * a.plan.ac == 16 * KSC && a.D % 2 == 0 && (KS0 == 0 || a.plan.real_off % 2 == 0);
-  for (int f = 0; f < a.plan.n_cf; ++f) exact = exact && a.plan.cf_off[f] % 2 == 0;
+  constexpr int WARPS = pk_warps(MODE), TLON = 8 * (WARPS / PK_ROWS);
   const void* ptrs[6] = {a.own1, a.own2, a.nb1, a.nb2, a.res1, a.res2};
-  for (const void* q : ptrs) exact = exact && reinterpret_cast<uintptr_t>(q) % 4 == 0;
-  a.exact = exact ? 1 : 0;
-  const size_t smem = 2 * (size_t)L::BUFFER_BYTES + 1024;
-  auto kernel = lattice_tn_kernel<KS0, NCF, KSC, MODE, WARPS>;
-  int st = allow_smem(kernel, smem, "gm_lattice_attention (tensor cores)");
-  if (st != GM_OK) return st;
-  const int tiles = (a.nlon + TL - 1) / TL;
-  dim3 grid((unsigned)(n_order_rows * tiles), (unsigned)a.H, (unsigned)batch);
-  kernel<<<grid, 32 * WARPS, smem, stream>>>(a);
-  return launch_status("gm_lattice_attention (tensor cores)");
+  uint64_t all = (uint64_t)a.D * 2 | (uint64_t)a.plan.a0 * 2 | (KS0 ? (uint64_t)a.plan.real_off * 2 : 0);  // in bytes
+  for (int f = 0; f < a.plan.n_cf; ++f) all |= (uint64_t)a.plan.cf_off[f] * 2;
+  for (const void* q : ptrs) all |= reinterpret_cast<uintptr_t>(q);
+  if (MODE == TC_BWD_T && a.delta_out) all |= reinterpret_cast<uintptr_t>(a.out_fwd);
+  a.even = all % 4 == 0;
+  a.padded = (KS0 && a.plan.a0 != 16) || 2 * a.plan.ac != 16 * KSC;
+  // the widest copy that every block of every head is made of: all that is added to the fields' addresses, in bytes
+  uint64_t bits = reinterpret_cast<uintptr_t>(a.nb1) | reinterpret_cast<uintptr_t>(a.nb2) | (uint64_t)a.D * 2 | (uint64_t)a.plan.a0 * 2 |
+                  (uint64_t)a.plan.ac * 4 | (KS0 ? (uint64_t)a.plan.real_off * 2 : 0);
+  for (int f = 0; f < a.plan.n_cf; ++f) bits |= (uint64_t)a.plan.cf_off[f] * 2;
+  a.unit = 16;
+  while (a.unit > 2 && bits % a.unit) a.unit /= 2;
+  a.units = (2 * a.plan.a0 + NCF * 4 * a.plan.ac) / a.unit;
+  a.n_order = n_order_rows;
+  const size_t smem = chunk_caps<KS0, NCF, KSC, WARPS>(a.rows, a.nlon, a.W, a.caps);
+  // Polar rows see whole rings: their tiles start first and hold few (sample, head) pairs each.  Elsewhere a CTA takes as
+  // many pairs as leave a few waves of CTAs, up to 16: lists and entries are made once for all of them.
+  const int64_t lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
+  const int64_t n_bh = (int64_t)a.H * batch, slots = (int64_t)sm_count() * pk_ctas(WARPS);
+  GM_REQUIRE(n_bh < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_attention (tensor cores): too many (sample, head) pairs");
+  int64_t heavy_tiles = 2 * ((2 * a.W + 2 + PK_ROWS - 1) / PK_ROWS);
+  if (heavy_tiles > row_tiles) heavy_tiles = row_tiles;
+  const int64_t light_tiles = (row_tiles - heavy_tiles) * lon_tiles;
+  auto pairs_per_cta = [&](int64_t tiles, int64_t waves, int64_t most) {
+    int64_t n = tiles * n_bh / (slots * waves);
+    n = n < 1 ? 1 : n > most ? most : n;
+    const int64_t chunks = (n_bh + n - 1) / n;
+    return (int)((n_bh + chunks - 1) / chunks);
+  };
+  a.n_bh = (int)n_bh;
+  a.light_bh = pairs_per_cta(light_tiles, 6, 16);
+  a.heavy_bh = pairs_per_cta(light_tiles + heavy_tiles * lon_tiles, 24, 2);
+  a.heavy_tiles = (int)heavy_tiles;
+  const int64_t heavy = heavy_tiles * lon_tiles * ((n_bh + a.heavy_bh - 1) / a.heavy_bh);
+  const int64_t light = light_tiles * ((n_bh + a.light_bh - 1) / a.light_bh);
+  GM_REQUIRE(heavy + light < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_attention (tensor cores): %lld tiles exceed a grid", (long long)(heavy + light));
+  a.heavy_ctas = (int)heavy;
+  auto go = [&](auto kernel) {
+    const int st = allow_smem(kernel, smem, "gm_lattice_attention (tensor cores)");
+    if (st != GM_OK) return st;
+    kernel<<<(unsigned)(heavy + light), 32 * WARPS, smem, stream>>>(a);
+    return launch_status("gm_lattice_attention (tensor cores)");
+  };
+  return a.records ? go(lattice_packed_kernel<KS0, NCF, KSC, MODE, WARPS, true>) : go(lattice_packed_kernel<KS0, NCF, KSC, MODE, WARPS, false>);
+}
+
+// f(KS0, NCF, KSC) as integral constants for the layouts that have kernels
+template <typename F>
+int for_layout(const TcPlan& plan, int NORD, const F& f) {
+  const int ks0 = plan.a0 > 0 ? 1 : 0, ksc = plan.ac > 8 ? 2 : 1, ncf = plan.n_cf;
+  for (int x = 0; x < ncf; ++x)
+    GM_REQUIRE(plan.cf_order[x] == x + 1, GM_ERR_UNSUPPORTED, "gm_lattice_attention (tensor cores): complex frequencies must be the orders 1 .. %d", ncf);
+  GM_REQUIRE(NORD == ncf, GM_ERR_UNSUPPORTED, "gm_lattice_attention (tensor cores): the tables must hold exactly the orders 1 .. %d (they hold %d)", ncf, NORD);
+  using std::integral_constant;
+  auto with = [&](auto a, auto b, auto c) { return f(a, b, c); };
+#define GM_LAYOUT(A, B, C) \
+  if (ks0 == A && ncf == B && ksc == C) return with(integral_constant<int, A>(), integral_constant<int, B>(), integral_constant<int, C>());
+  GM_LAYOUT(1, 2, 2)
+  GM_LAYOUT(1, 2, 1)
+  GM_LAYOUT(1, 3, 1)
+  GM_LAYOUT(1, 1, 2)
+  GM_LAYOUT(1, 1, 1)
+  GM_LAYOUT(0, 2, 1)
+#undef GM_LAYOUT
+  return fail(GM_ERR_UNSUPPORTED, "gm_lattice_attention (tensor cores): no kernel for this head layout (a0=%d, %d x %d complex)", plan.a0, ncf, plan.ac);
 }
 
 template <int MODE>
 int dispatch_tc(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t cs) {
-  const int ks0 = a.plan.a0 > 0 ? 1 : 0, ksc = a.plan.ac > 8 ? 2 : 1, ncf = a.plan.n_cf;
-  for (int f = 0; f < ncf; ++f)
-    GM_REQUIRE(a.plan.cf_order[f] == f + 1, GM_ERR_UNSUPPORTED, "gm_lattice_attention (tensor cores): complex frequencies must be the orders 1 .. %d", ncf);
-  GM_REQUIRE(a.NORD == ncf, GM_ERR_UNSUPPORTED, "gm_lattice_attention (tensor cores): the tables must hold exactly the orders 1 .. %d (they hold %d)", ncf, a.NORD);
-  if (ks0 == 1 && ncf == 2 && ksc == 2) return launch_tn<1, 2, 2, MODE>(a, n_order_rows, batch, cs);
-  if (ks0 == 1 && ncf == 2 && ksc == 1) return launch_tn<1, 2, 1, MODE>(a, n_order_rows, batch, cs);
-  if (ks0 == 1 && ncf == 3 && ksc == 1) return launch_tn<1, 3, 1, MODE>(a, n_order_rows, batch, cs);
-  if (ks0 == 1 && ncf == 1 && ksc == 2) return launch_tn<1, 1, 2, MODE>(a, n_order_rows, batch, cs);
-  if (ks0 == 1 && ncf == 1 && ksc == 1) return launch_tn<1, 1, 1, MODE>(a, n_order_rows, batch, cs);
-  if (ks0 == 0 && ncf == 2 && ksc == 1) return launch_tn<0, 2, 1, MODE>(a, n_order_rows, batch, cs);
-  return fail(GM_ERR_UNSUPPORTED, "gm_lattice_attention (tensor cores): no kernel for this head layout (a0=%d, %d x %d complex)",
-              a.plan.a0, ncf, a.plan.ac);
+  return for_layout(a.plan, a.NORD, [&](auto ks0, auto ncf, auto ksc) { return launch_tn<ks0.value, ncf.value, ksc.value, MODE>(a, n_order_rows, batch, cs); });
 }
 
 int fill_tc_args(TcArgs& a, const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H, int W, int ES, int NORD,
@@ -1000,12 +1239,54 @@ int fill_tc_args(TcArgs& a, const int64_t* desc_host, int F, int rows, int nlon,
 
 using namespace gmb;
 
-extern "C" int gm_lattice_attention_forward_tc(const void* q, const void* k, const void* v, const int* win_cnt, const int* win_lo,
+// ---- plans.  gm_lattice_plan_size: bytes of one record and the number of row tiles; _count: chunks per row tile; _fill: the
+// records, row tile x's from first[x] on (first: the running sum of the counts, row tiles + 1 numbers).
+extern "C" int gm_lattice_plan_size(const int64_t* desc_host, int F, int rows, int nlon, int D, int H, int W, int NORD, int mode,
+                                    int64_t* record_bytes, int64_t* row_tiles) {
+  GM_REQUIRE(record_bytes && row_tiles, GM_ERR_ARGUMENT, "gm_lattice_plan_size: null pointer");
+  TcArgs a{};
+  int status = fill_tc_args(a, desc_host, F, rows, nlon, 1, D, H, W, 8, NORD, 1.0);
+  if (status != GM_OK) return status;
+  *row_tiles = (rows + PK_ROWS - 1) / PK_ROWS;
+  return for_layout(a.plan, NORD, [&](auto ks0, auto ncf, auto ksc) {
+    auto size = [&](auto warps) {
+      PkCaps caps;
+      chunk_caps<ks0.value, ncf.value, ksc.value, warps.value>(rows, nlon, W, caps);
+      *record_bytes = pk_record_bytes<ncf.value>(caps, warps.value);
+      return (int)GM_OK;
+    };
+    return mode == TC_FWD ? size(std::integral_constant<int, pk_warps(TC_FWD)>()) : size(std::integral_constant<int, pk_warps(TC_BWD_S)>());
+  });
+}
+
+extern "C" int gm_lattice_plan_build(const int* win_cnt, const int* win_lo, const int* win_off, const float* entries, const int64_t* desc_host, int F,
+                                     int rows, int nlon, int D, int H, int W, int NORD, int mode, int* counts, const int* first, void* records, void* stream) {
+  GM_REQUIRE(win_cnt && win_lo && win_off && entries && (records ? first != nullptr : counts != nullptr), GM_ERR_ARGUMENT, "gm_lattice_plan_build: null pointer");
+  TcArgs a{};
+  int status = fill_tc_args(a, desc_host, F, rows, nlon, 1, D, H, W, 8, NORD, 1.0);
+  if (status != GM_OK) return status;
+  return for_layout(a.plan, NORD, [&](auto ks0, auto ncf, auto ksc) {
+    auto build = [&](auto warps) {
+      PkCaps caps;
+      chunk_caps<ks0.value, ncf.value, ksc.value, warps.value>(rows, nlon, W, caps);
+      const PkWindows t{win_cnt, win_lo, win_off, entries, rows, nlon, W};
+      lattice_plan_kernel<ncf.value, warps.value><<<(unsigned)((rows + PK_ROWS - 1) / PK_ROWS), 32 * warps.value, 0, (cudaStream_t)stream>>>(
+          t, caps, PkLayout<ks0.value, ncf.value, ksc.value>::PITCH / 16, counts, first, (unsigned char*)records);
+      return launch_status("gm_lattice_plan_build");
+    };
+    return mode == TC_FWD ? build(std::integral_constant<int, pk_warps(TC_FWD)>()) : build(std::integral_constant<int, pk_warps(TC_BWD_S)>());
+  });
+}
+
+extern "C" int gm_lattice_attention_forward_planned(const void* q, const void* k, const void* v, const int* win_cnt, const int* win_lo,
                                                const int* win_off, const float* entries, const int* row_order, int n_order_rows,
                                                const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H, int W,
-                                               int ES, int NORD, double scale, void* out, float* lse, void* stream) {
+                                               int ES, int NORD, double scale, const int* plan_first, const void* plan_records, void* out, float* lse,
+                                               void* stream) {
   using B = __nv_bfloat16;
   TcArgs a{};
+  GM_REQUIRE(!plan_records || (plan_first && reinterpret_cast<uintptr_t>(plan_records) % 16 == 0), GM_ERR_ARGUMENT, "gm_lattice_attention_forward_planned: bad plan");
+  a.plan_first = plan_first; a.records = (const unsigned char*)plan_records;
   int status = fill_tc_args(a, desc_host, F, rows, nlon, batch, D, H, W, ES, NORD, scale);
   if (status != GM_OK) return status;
   GM_REQUIRE(q && k && v && win_cnt && win_lo && win_off && entries && row_order && out && lse, GM_ERR_ARGUMENT,
@@ -1014,6 +1295,14 @@ extern "C" int gm_lattice_attention_forward_tc(const void* q, const void* k, con
   a.own1 = (const B*)q; a.nb1 = (const B*)k; a.nb2 = (const B*)v; a.res1 = (B*)out; a.lse_out = lse;
   a.win_cnt = win_cnt; a.win_lo = win_lo; a.win_off = win_off; a.entries = entries; a.row_order = row_order;
   return dispatch_tc<TC_FWD>(a, n_order_rows, batch, (cudaStream_t)stream);
+}
+
+extern "C" int gm_lattice_attention_forward_tc(const void* q, const void* k, const void* v, const int* win_cnt, const int* win_lo,
+                                               const int* win_off, const float* entries, const int* row_order, int n_order_rows,
+                                               const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H, int W,
+                                               int ES, int NORD, double scale, void* out, float* lse, void* stream) {
+  return gm_lattice_attention_forward_planned(q, k, v, win_cnt, win_lo, win_off, entries, row_order, n_order_rows, desc_host, F, rows, nlon, batch, D, H,
+                                              W, ES, NORD, scale, nullptr, nullptr, out, lse, stream);
 }
 
 extern "C" int gm_lattice_attention_backward_tc_passes(const void* dout, const void* q, const void* k, const void* v, const void* out,
@@ -1040,14 +1329,15 @@ extern "C" int gm_lattice_attention_backward_tc(const void* dout, const void* q,
 // passes: bit 0 = Delta, bit 1 = the target-major pass (dq), bit 2 = the source-major pass (dk, dv).  Running a
 // subset is for timing the passes separately.  Bits 0 and 1 together: pass T forms Delta itself; without bit 0 the
 // passes read the Delta an earlier call left in `delta`.
-extern "C" int gm_lattice_attention_backward_tc_passes(const void* dout, const void* q, const void* k, const void* v, const void* out,
+extern "C" int gm_lattice_attention_backward_planned(const void* dout, const void* q, const void* k, const void* v, const void* out,
                                                        const float* lse, const int* win_cnt, const int* win_lo, const int* win_off,
                                                        const float* entries, const int* row_order, int n_order_rows,
                                                        const int* t_win_cnt, const int* t_win_lo, const int* t_win_off,
                                                        const float* t_entries, const int* t_row_order, int t_n_order_rows,
                                                        const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H,
                                                        int W, int ES, int NORD, double scale, void* dq, void* dk, void* dv, float* delta,
-                                                       int passes, void* stream) {
+                                                       int passes, const int* plan_first, const void* plan_records,
+                                                       const int* t_plan_first, const void* t_plan_records, void* stream) {
   using B = __nv_bfloat16;
   cudaStream_t cs = (cudaStream_t)stream;
   TcArgs a{};
@@ -1056,6 +1346,9 @@ extern "C" int gm_lattice_attention_backward_tc_passes(const void* dout, const v
   GM_REQUIRE(dout && q && k && v && out && lse && win_cnt && win_lo && win_off && entries && row_order && t_win_cnt && t_win_lo &&
                  t_win_off && t_entries && t_row_order && dq && dk && dv && delta,
              GM_ERR_ARGUMENT, "gm_lattice_attention_backward_tc: null pointer");
+  GM_REQUIRE((!plan_records || (plan_first && reinterpret_cast<uintptr_t>(plan_records) % 16 == 0)) &&
+                 (!t_plan_records || (t_plan_first && reinterpret_cast<uintptr_t>(t_plan_records) % 16 == 0)),
+             GM_ERR_ARGUMENT, "gm_lattice_attention_backward_planned: bad plan");
   const int64_t n_nodes = batch * rows * (int64_t)nlon;
   bool chunked = D % 8 == 0 && D <= 512 && a.plan.a0 % 8 == 0 && (2 * a.plan.ac) % 8 == 0 && a.plan.real_off % 8 == 0 &&
                  reinterpret_cast<uintptr_t>(dout) % 16 == 0 && reinterpret_cast<uintptr_t>(out) % 16 == 0;
@@ -1074,6 +1367,7 @@ extern "C" int gm_lattice_attention_backward_tc_passes(const void* dout, const v
     a.own1 = (const B*)q; a.own2 = (const B*)dout; a.nb1 = (const B*)k; a.nb2 = (const B*)v; a.res1 = (B*)dq; a.res2 = nullptr;
     a.out_fwd = (const B*)out; a.delta_out = (passes & 1) ? delta : nullptr;
     a.win_cnt = win_cnt; a.win_lo = win_lo; a.win_off = win_off; a.entries = entries; a.row_order = row_order;
+    a.plan_first = plan_first; a.records = (const unsigned char*)plan_records;
     status = dispatch_tc<TC_BWD_T>(a, n_order_rows, batch, cs);
     if (status != GM_OK) return status;
   }
@@ -1081,13 +1375,27 @@ extern "C" int gm_lattice_attention_backward_tc_passes(const void* dout, const v
     a.own1 = (const B*)k; a.own2 = (const B*)v; a.nb1 = (const B*)q; a.nb2 = (const B*)dout; a.res1 = (B*)dk; a.res2 = (B*)dv;
     a.out_fwd = nullptr; a.delta_out = nullptr;
     a.win_cnt = t_win_cnt; a.win_lo = t_win_lo; a.win_off = t_win_off; a.entries = t_entries; a.row_order = t_row_order;
+    a.plan_first = t_plan_first; a.records = (const unsigned char*)t_plan_records;
     status = dispatch_tc<TC_BWD_S>(a, t_n_order_rows, batch, cs);
   }
   return status;
 }
 
+extern "C" int gm_lattice_attention_backward_tc_passes(const void* dout, const void* q, const void* k, const void* v, const void* out,
+                                                       const float* lse, const int* win_cnt, const int* win_lo, const int* win_off,
+                                                       const float* entries, const int* row_order, int n_order_rows,
+                                                       const int* t_win_cnt, const int* t_win_lo, const int* t_win_off,
+                                                       const float* t_entries, const int* t_row_order, int t_n_order_rows,
+                                                       const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H,
+                                                       int W, int ES, int NORD, double scale, void* dq, void* dk, void* dv, float* delta,
+                                                       int passes, void* stream) {
+  return gm_lattice_attention_backward_planned(dout, q, k, v, out, lse, win_cnt, win_lo, win_off, entries, row_order, n_order_rows, t_win_cnt, t_win_lo,
+                                               t_win_off, t_entries, t_row_order, t_n_order_rows, desc_host, F, rows, nlon, batch, D, H, W, ES, NORD,
+                                               scale, dq, dk, dv, delta, passes, nullptr, nullptr, nullptr, nullptr, stream);
+}
+
 extern "C" int gm_lattice_attention_tc_wait_expired(int* expired) {
   GM_REQUIRE(expired, GM_ERR_ARGUMENT, "gm_lattice_attention_tc_wait_expired: null pointer");
-  GM_CUDA(cudaMemcpyFromSymbol(expired, g_tc_wait_expired, sizeof(int)));
+  *expired = 0;
   return GM_OK;
 }

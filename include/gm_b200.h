@@ -314,9 +314,7 @@ int gm_node_products_backward(const void* x, const void* cw, const void* cb, con
  * tables, same results within bf16 rounding of the attention weights): the
  * per-frequency Gram blocks and the (alpha o tau) V sums run as m16n8k16 bf16
  * matrix products on (16 source positions x 8 targets) tiles of the longitude
- * band; neighbour rows are staged with TMA tensor copies where the head's
- * blocks are exactly 16 / 32 columns wide, with per-thread copies otherwise
- * (environment GM_LATTICE_TMA=0 forces the latter; same results bit for bit).
+ * band, the positions of all neighbour rows packed into tiles of 16.
  * Head layouts: an optional scalar block of <= 16 copies and one to three complex
  * frequencies of orders 1, 2, 3 sharing one multiplicity <= 16; otherwise
  * GM_ERR_UNSUPPORTED (use gm_lattice_attention_forward).
@@ -341,11 +339,39 @@ int gm_lattice_attention_backward_tc_passes(const void* dout, const void* q, con
                                             int D, int H, int W, int ES, int NORD, double scale, void* dq, void* dk, void* dv,
                                             float* delta, int passes, void* stream);
 
-/* Health flag of the tensor-core lattice kernels (no counterpart in the reference).  Their waits on the
- * completion barriers of the TMA copies are bounded; a wait that runs out sets a per-device flag and the
- * launch's results are invalid.  Writes the flag of the current device to *expired (0: never happened);
- * synchronises the device. */
+/* Health flag of the tensor-core lattice kernels (no counterpart in the reference): whether a wait for a copy ever ran out.
+ * The kernels wait with cp.async groups only, which cannot run out: *expired = 0. */
 int gm_lattice_attention_tc_wait_expired(int* expired);
+
+/* Plans of the tensor-core lattice kernels: what every longitude tile of a row tile (four lattice rows) has in common -- the
+ * packed list of its neighbour positions and their table entries, in chunks of the kernels' shared memory -- worked out once
+ * per (tables, head layout) instead of once per CTA.  gm_lattice_plan_size: bytes of a chunk's record and the number of row
+ * tiles.  gm_lattice_plan_build with records == NULL: counts[row tile] = its chunks; with records: fills them, row tile x's
+ * from record first[x] on (first: row tiles + 1 running sums).  records starts on a 16-byte boundary.  A plan belongs to the
+ * contents of win_cnt / win_lo / win_off / entries it was built from, to the descriptor and to the lattice's size; mode: 0
+ * for the forward (whose CTAs are wider), 1 for the target-major pass (the same tables), 2 for the source-major pass (the
+ * transposed ones). */
+int gm_lattice_plan_size(const int64_t* desc_host, int F, int rows, int nlon, int D, int H, int W, int NORD, int mode,
+                         int64_t* record_bytes, int64_t* row_tiles);
+int gm_lattice_plan_build(const int* win_cnt, const int* win_lo, const int* win_off, const float* entries, const int64_t* desc_host, int F,
+                          int rows, int nlon, int D, int H, int W, int NORD, int mode, int* counts, const int* first, void* records,
+                          void* stream);
+
+/* gm_lattice_attention_forward_tc / _backward_tc_passes with the plans of modes 0 / 1 and 2
+ * (plan_records == NULL: without one, bit-identical results). */
+int gm_lattice_attention_forward_planned(const void* q, const void* k, const void* v, const int* win_cnt, const int* win_lo,
+                                         const int* win_off, const float* entries, const int* row_order, int n_order_rows,
+                                         const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H, int W, int ES,
+                                         int NORD, double scale, const int* plan_first, const void* plan_records, void* out, float* lse,
+                                         void* stream);
+int gm_lattice_attention_backward_planned(const void* dout, const void* q, const void* k, const void* v, const void* out, const float* lse,
+                                          const int* win_cnt, const int* win_lo, const int* win_off, const float* entries,
+                                          const int* row_order, int n_order_rows, const int* t_win_cnt, const int* t_win_lo,
+                                          const int* t_win_off, const float* t_entries, const int* t_row_order, int t_n_order_rows,
+                                          const int64_t* desc_host, int F, int rows, int nlon, int64_t batch, int D, int H, int W, int ES,
+                                          int NORD, double scale, void* dq, void* dk, void* dv, float* delta, int passes,
+                                          const int* plan_first, const void* plan_records, const int* t_plan_first,
+                                          const void* t_plan_records, void* stream);
 
 int gm_lattice_attention_forward_tc(const void* q, const void* k, const void* v, const int* win_cnt, const int* win_lo,
                                     const int* win_off, const float* entries, const int* row_order, int n_order_rows,

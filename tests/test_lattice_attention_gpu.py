@@ -373,3 +373,47 @@ def test_layer_split_around_a_halo_exchange_equals_one_call():
     lattice_attention_backward(G, Q, K, V, out2, lse2, split.owned_sources, passes=4, workspace=ws)
     for a, b in zip(want, (out2, lse2, *ws[:3])):
         assert torch.equal(a, b)
+
+
+# tiles of 4 rows x 8 or 16 longitudes with remainders both ways, copies of 2 / 8 / 16 bytes at a time, windows cut into
+# chunks, more neighbour rows than a warp has lanes, a lattice narrower than a tile
+PACKED_CASES = [
+    (5, 8, 2 * math.pi / 5, {0: 5, 1: 5}, 3, "hard", 2),
+    (7, 30, 2.5 * math.pi / 7, {0: 4, 1: 4, 2: 4}, 2, "quartic", 1),
+    (33, 40, 3 * math.pi / 33, {0: 8, 1: 8, 2: 8, 3: 8}, 1, "hard", 2),
+    (4, 320, 1.6 * math.pi / 4, {0: 16, 1: 16, 2: 16}, 1, "hard", 1),
+    (40, 12, 15.5 * math.pi / 40, {1: 6, 2: 6}, 1, "hard", 1),
+]
+
+
+@pytest.mark.parametrize("case", PACKED_CASES)
+def test_packed_tensor_core_kernels(case):
+    """The tensor-core kernels with a plan, without one (every CTA packs its own lists) and after the tables were written in
+    place (the plan is theirs no longer), against the oracle on the rounded inputs; bf16 storage: 2e-2 of the magnitude."""
+    import dataclasses
+
+    from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
+
+    batch = case[6]
+    c = make_case(*case[:5], dtype=np.float32, window=case[5])
+    rounded = [torch.from_numpy(x).bfloat16() for x in seeded((batch * c.n_nodes, c.width), 63, np.float32, 4)]
+    q, k, v, g = (x.float().numpy() for x in rounded)
+    Q, K, V, G = (x.cuda() for x in rounded)
+    _, lat = tables_for(c)
+    assert all(plan is not None for plan in lat.tc_plans) and all(lat.plan_pointers(mode)[1] for mode in range(3))
+
+    def run(t):
+        out, lse = lattice_attention_forward(Q, K, V, t, tensor_cores=True)
+        return out, lse, *lattice_attention_backward(G, Q, K, V, out, lse, t, tensor_cores=True)
+
+    planned = run(lat)
+    for a, b in zip(planned, run(dataclasses.replace(lat, tc_plans=(None, None, None)))):
+        assert torch.equal(a, b)
+    want = O.attention_forward(q, k, v, c.transport, c.bias, c.inside, c.desc, c.row_ptr, c.source, c.heads, c.scale, batch)
+    grads = O.attention_backward(g, q, k, v, c.transport, c.bias, c.inside, c.desc, c.row_ptr, c.source, c.heads, c.scale, batch)
+    for name, a, b in zip(("out", "dq", "dk", "dv"), (planned[0], *planned[2:]), (want, *grads)):
+        assert float(np.abs(a.float().cpu().numpy() - b).max()) < 2e-2 * max(1.0, np.abs(b).max()), name
+    lat.entries[:, :2 * lat.orders].mul_(-1.0)
+    assert lat.plan_pointers(0) == lat.plan_pointers(1) == (None, None) and lat.plan_pointers(2)[1]
+    turned = run(lat)
+    assert torch.equal(turned[0], run(dataclasses.replace(lat, tc_plans=(None, None, None)))[0]) and not torch.equal(turned[0], planned[0])
