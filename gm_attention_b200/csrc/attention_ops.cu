@@ -113,13 +113,19 @@ __global__ void __launch_bounds__(SM_THREADS) softmax_forward_kernel(SoftmaxArgs
 // the group reduces with log2(L) xor-shuffles, and all H logits of the edge appear at once.  The raw logits go to
 // alpha, the row is then normalised in place by the same warp (masked edges never enter the shift or the sum).
 // NF: the number of descriptor rows when known at compile time (3 or 4 frequencies: the usual head types), 0 = up to MAX_F
+//
+// SCORE_PARTS warps share a target, four edges of it in turn each: 883 us with one, 762 with two, 808 with four (128 x 256,
+// radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32; half of the targets have fewer than 30 edges, the polar ones a thousand).
+constexpr int SCORE_PARTS = 2;
+
 template <typename T, int R, int NF>
 __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArgs<T> a) {
-  constexpr int FN = NF ? NF : MAX_F;
-  const int lane = threadIdx.x & 31;
-  const int64_t x = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (x >= a.n_nodes) return;
-  const int64_t i = from_both_ends(x, a.n_nodes);
+  constexpr int FN = NF ? NF : MAX_F, PARTS = SCORE_PARTS, TARGETS = 4 / PARTS;
+  __shared__ T max_s[TARGETS][PARTS][MAX_H], sum_s[TARGETS][PARTS][MAX_H];
+  const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % PARTS, mine = (threadIdx.x >> 5) / PARTS;
+  const int64_t x = (int64_t)blockIdx.x * TARGETS + mine;
+  const bool present = x < a.n_nodes;
+  const int64_t i = present ? from_both_ends(x, a.n_nodes) : 0;
   const int L = 32 / a.H, h = lane / L, s = lane % L;
   int col[FN][R], order[FN];
   T qr[FN][R], qi[FN][R];
@@ -142,7 +148,7 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
       }
     }
   }
-  const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
+  const int64_t e0 = a.row_ptr[i], e1 = present ? a.row_ptr[i + 1] : e0;
   T m = neg_inf<T>();
   // this lane's share of <q_i, tau k_j> for one edge
   auto dot = [&](const T* k_j, const T* tau) -> T {
@@ -170,36 +176,46 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
     if (s == 0) a.alpha[e * a.H + h] = lw;
   };
   constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together (8: 0.96 ms against 0.88)
-  int64_t e = e0;
-  for (; e + U <= e1; e += U) {
-    const T* k_j[U];
-    T part[U];
+  for (int64_t e = e0 + U * part; e < e1; e += U * PARTS) {
+    if (e + U <= e1) {
+      const T* k_j[U];
+      T part_sum[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) k_j[u] = a.k + a.source[e + u] * a.D;
+      for (int u = 0; u < U; ++u) k_j[u] = a.k + a.source[e + u] * a.D;
 #pragma unroll
-    for (int u = 0; u < U; ++u) part[u] = dot(k_j[u], a.transport + (e + u) * a.orders * 2);
-    for (int o = L >> 1; o > 0; o >>= 1) {
+      for (int u = 0; u < U; ++u) part_sum[u] = dot(k_j[u], a.transport + (e + u) * a.orders * 2);
+      for (int o = L >> 1; o > 0; o >>= 1) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) part[u] += __shfl_xor_sync(0xffffffffu, part[u], o);
+        for (int u = 0; u < U; ++u) part_sum[u] += __shfl_xor_sync(0xffffffffu, part_sum[u], o);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) finish(e + u, part_sum[u]);
+    } else {
+      for (int64_t t = e; t < e1; ++t) {
+        T one = dot(a.k + a.source[t] * a.D, a.transport + t * a.orders * 2);
+        for (int o = L >> 1; o > 0; o >>= 1) one += __shfl_xor_sync(0xffffffffu, one, o);
+        finish(t, one);
+      }
     }
+  }
+  if (s == 0) max_s[mine][part][h] = m;
+  __syncthreads();
 #pragma unroll
-    for (int u = 0; u < U; ++u) finish(e + u, part[u]);
-  }
-  for (; e < e1; ++e) {
-    T part = dot(a.k + a.source[e] * a.D, a.transport + e * a.orders * 2);
-    for (int o = L >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    finish(e, part);
-  }
-  __syncwarp();
+  for (int p = 0; p < PARTS; ++p) m = max_s[mine][p][h] > m ? max_s[mine][p][h] : m;
   // normalise: the group's lanes stride the row's edges for their head
   T sum = T(0);
-  for (int64_t e = e0 + s; e < e1; e += L) {
+  for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) {
     const T u = a.inside[e] ? gm_exp(a.alpha[e * a.H + h] - m) : T(0);
     a.alpha[e * a.H + h] = u;
     sum += u;
   }
   for (int o = L >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  for (int64_t e = e0 + s; e < e1; e += L) a.alpha[e * a.H + h] /= sum;
+  if (s == 0) sum_s[mine][part][h] = sum;
+  __syncthreads();
+  sum = T(0);
+#pragma unroll
+  for (int p = 0; p < PARTS; ++p) sum += sum_s[mine][p][h];
+  for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) a.alpha[e * a.H + h] /= sum;
 }
 
 // ------------------------------------------------------------------ depthwise conv
@@ -251,6 +267,21 @@ __device__ __forceinline__ void store_pair(T* p, T x, T y) {
   } else {
     p[0] = x; p[1] = y;
   }
+}
+
+// p[0] += x, p[1] += y.  A float pair on an 8-byte boundary is one vector reduction: half as many operations for the L2
+// units.  128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32: 1 098 -> 897 us for the scores' backward.  (The
+// depthwise backward and the fused layer's on general graphs lose by it, 1 045 -> 1 190 and 363 -> 394 us.)
+template <typename T>
+__device__ __forceinline__ void add_pair(T* p, T x, T y) {
+  if constexpr (std::is_same<T, float>::value) {
+    if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(x), "f"(y));
+      return;
+    }
+  }
+  atomicAdd(p, x);
+  atomicAdd(p + 1, y);
 }
 
 // One (head, frequency, copy) of the scores' backward: a scalar column or a (re, im) column pair of one head
@@ -327,8 +358,7 @@ __global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
           const T ds = a.scale * al * (da - total);
           dq_r += ds * (tr * kr - ti * ki);  // (tau k)
           dq_i += ds * (tr * ki + ti * kr);
-          atomicAdd(a.dk + j * a.D + it.col, ds * (tr * q_r + ti * q_i));  // conj(tau) q
-          atomicAdd(a.dk + j * a.D + it.col + 1, ds * (tr * q_i - ti * q_r));
+          add_pair(a.dk + j * a.D + it.col, ds * (tr * q_r + ti * q_i), ds * (tr * q_i - ti * q_r));  // conj(tau) q
         };
         int64_t e = e0;
         for (; e + U <= e1; e += U) {
@@ -577,7 +607,7 @@ int softmax_forward_t(SoftmaxArgs<T> a, int64_t deg_max, int max_mult, cudaStrea
   // head-group kernel when the heads split a warp evenly and every lane owns at most 4 copies per frequency
   if ((a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8) && max_mult > 0 && max_mult <= 4 * (32 / a.H)) {
     const int per_lane = (max_mult + 32 / a.H - 1) / (32 / a.H);
-    const unsigned blocks = (unsigned)((a.n_nodes + 3) / 4);
+    const unsigned blocks = (unsigned)((a.n_nodes * SCORE_PARTS + 3) / 4);
     if (per_lane <= 1 && a.F == 3) softmax_forward_grouped_kernel<T, 1, 3><<<blocks, 128, 0, stream>>>(a);
     else if (per_lane <= 1 && a.F == 4) softmax_forward_grouped_kernel<T, 1, 4><<<blocks, 128, 0, stream>>>(a);
     else if (per_lane <= 1) softmax_forward_grouped_kernel<T, 1, 0><<<blocks, 128, 0, stream>>>(a);
