@@ -21,27 +21,15 @@
 // source longitudes (apply) or 8 target longitudes (table_grad) past them, so every loaded value is used for 8 x 4
 // multiply-adds without shared memory.  apply has a second form that stages both operands and packs the arithmetic, taken
 // wherever a stage fits.  Results do not depend on the launch geometry: no atomics.
-#include "common.cuh"
+#include "lattice_conv.cuh"
 
 namespace gmb {
 namespace {
 
+using lconv::ConvArgs;
+
 constexpr int LON = 8;  // longitudes (apply) / longitude offsets (table_grad) per thread
 constexpr int THREADS = 160;  // at most; three CTAs per SM (128 registers per thread); more items than threads are looped over
-
-struct ConvArgs {
-  const void* x;        // (batch, rows * nlon, width) node field
-  const void* g;        // table_grad: the output gradient, same layout
-  const float* table;   // (entries, table_width)
-  const int* items;     // (n_items, 3): kind (0 complex copy, 1 pair of scalar channels), field column, table column
-  const int* win_cnt;   // (rows, 2 * halo + 1)
-  const int* win_lo;
-  const int* win_off;
-  const int* order;     // apply: target rows, heaviest first; table_grad: (blocks, 2) = window index, first offset
-  void* y;              // apply: (batch, rows * nlon, width)
-  float* dtable;        // table_grad: (entries, table_width)
-  int n_items, rows, nlon, batch, width, halo, table_width, transpose;
-};
 
 // Two neighbouring elements of a node's row: loaded as one word (bf16) or two (float), unpacked when used, so that a
 // value in flight between its load and its use costs one register per bf16 pair.
@@ -576,6 +564,7 @@ extern "C" int gm_lattice_conv_apply(const void* x, const float* table, const in
   a.n_items = n_items; a.rows = rows; a.nlon = nlon; a.batch = batch; a.width = width; a.halo = halo; a.table_width = table_width;
   a.transpose = transpose;
   cudaStream_t cs = (cudaStream_t)stream;
+  if (dtype == GM_BF16 && lconv::tensor_cores_take(a)) return lconv::apply_tc(a, n_order, cs);
   const int elem = dtype == GM_F32 ? 4 : 2;
   StagedShape sh{};
   const int nb = staged_shape(a, elem, n_order, sh);
@@ -627,6 +616,7 @@ extern "C" int gm_lattice_conv_table_grad(const void* g, const void* x, const in
   const int threads = min(THREADS, (n_items + 31) / 32 * 32);
   const int nb = batch >= 2 ? 2 : 1;  // four samples' windows would take every register a thread can have
   cudaStream_t cs = (cudaStream_t)stream;
+  if (dtype == GM_BF16 && lconv::tensor_cores_take(a)) return lconv::table_grad_tc(a, n_blocks, cs);
 #define GM_GRAD(S, NB) conv_table_grad_kernel<S, NB><<<(unsigned)n_blocks, threads, 0, cs>>>(a)
   if (dtype == GM_F32) {
     if (nb == 2) GM_GRAD(float, 2); else GM_GRAD(float, 1);

@@ -1,0 +1,464 @@
+// Lattice convolution of bfloat16 fields on the tensor cores (the operation and its table: lattice_conv.cu).
+//
+// A window's correlation along the longitudes has no contraction over channels, but it becomes a matrix product per
+// channel pair (a complex copy, or two scalar channels) when the longitudes are cut into tiles of 8, l = 8 t + s:
+//
+//   apply       y[8 t + s] = sum over r  T[s, r] x[8 t + r],   T[s, r] = M[r - s]  (0 outside the window)
+//               rows m = (s, component), columns t, contraction over (r, component): m16n8k16, 8 positions r per k-step
+//   table_grad  P[s, r] = sum over t  g[8 t + s] x[8 t + r],   dM[d] = sum over s  P[s, s + d]
+//               rows m = (s, component of g), columns (r, component of x), contraction over t, 16 tiles per k-step
+//
+// Of the (s, r) pairs of a window of cnt offsets 8 cnt in 8 (7 + cnt), rounded up to 8, are wanted: half at cnt = 8.
+// Precision: field values are bfloat16 as they are and the products accumulate in float32.  The table is float32, so
+// apply writes each of its numbers as a sum of three bfloat16 (8 + 8 + 8 bits: exact) and takes three products.
+//
+// In shared memory a node's 32 columns (64 bytes) sit at [position % 8][position / 8], rows of 80 bytes: a lane reads four
+// channel pairs of one position with one 16-byte load, the lanes of a load on different banks.  The (re, im) words are B
+// fragments of apply as they are; table_grad contracts over positions and pairs the words of t and t + 1 with two byte
+// permutations.
+#include "lattice_conv.cuh"
+
+namespace gmb {
+namespace lconv {
+namespace {
+
+constexpr int TC_THREADS = 256;         // 8 warps: 4 groups of 4 channel pairs x 2
+constexpr int TC_COLS = 32;             // columns of the field per CTA
+constexpr int TC_PAIRS = TC_COLS / 2;   // channel pairs
+constexpr int TC_PITCH = 5;             // 16-byte words per staged position (4 and one of padding)
+
+__device__ __forceinline__ void mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// d += a * b with the addition to d rounded to nearest (the accumulator of a long chain of mma would be cut off every time)
+__device__ __forceinline__ void mma_add(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+  float p[4];
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+#pragma unroll
+  for (int x = 0; x < 4; ++x) d[x] += p[x];
+}
+// 16 bytes global -> shared, asynchronously; bytes = 0 writes zeros
+__device__ __forceinline__ void copy16(uint4* dst, const void* src, int bytes) {
+  const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(addr), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N> __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
+
+// Staged copies of `count` positions from longitude `lon` of a row (cyclic) on: position q to [q % 8][q / 8], SP 16-byte words
+// between the eight.  Columns beyond the field's are zeros.
+template <int SP>
+__device__ __forceinline__ void stage_positions(uint4* dst, const unsigned char* row, int lon, int count, int nlon, int row_bytes, int col_byte) {
+  const int k = threadIdx.x & 3, byte = col_byte + 16 * k;
+  const bool in = byte < row_bytes;
+  const unsigned char* src = row + (in ? byte : 0);
+  int at = lon + ((int)threadIdx.x >> 2);
+  while (at >= nlon) at -= nlon;
+  const int step = (TC_THREADS / 4) % nlon;
+  for (int q = threadIdx.x >> 2; q < count; q += TC_THREADS / 4) {
+    copy16(dst + (q & 7) * SP + (q >> 3) * TC_PITCH + k, src + (size_t)at * row_bytes, in ? 16 : 0);
+    at += step;
+    if (at >= nlon) at -= nlon;
+  }
+}
+
+struct PairItem {
+  int kind, fcol;  // -1: no item on these columns
+};
+__device__ __forceinline__ void find_items(const ConvArgs& a, int col0, PairItem* pairs_s) {
+  if (threadIdx.x < TC_PAIRS) pairs_s[threadIdx.x] = PairItem{-1, 0};
+  __syncthreads();
+  for (int x = threadIdx.x; x < a.n_items; x += TC_THREADS) {
+    const int col = a.items[3 * x + 1] - col0;
+    if (col >= 0 && col < TC_COLS) pairs_s[col >> 1] = PairItem{a.items[3 * x], a.items[3 * x + 2]};
+  }
+  __syncthreads();
+}
+
+// ----------------------------------------------------------------------------------------------------------- table_grad
+constexpr int TG_TILES = 32;                      // tiles t per stage: two k-steps
+constexpr int TG_SPG = TG_TILES * TC_PITCH + 1;   // odd: the lanes' eight s fall on different banks beside their four t
+constexpr int TG_SPX = (TG_TILES + 4) * TC_PITCH + 1;
+constexpr int TG_STAGE = 8 * (TG_SPG + TG_SPX);   // 16-byte words
+constexpr int TG_PS = 18;                         // floats between the s of a P block
+constexpr int TG_BLOCK = 8 * TG_PS;               // floats of a P block: 8 s x 16 r
+constexpr int TG_MERGE = 3;                       // blocks of 8 offsets one CTA takes: 24 + 7 positions are four groups of 8
+static_assert(2 * TC_PAIRS * 4 * TG_BLOCK * 4 <= 2 * TG_STAGE * 16, "the P blocks reuse the stages");
+
+// One CTA: up to three consecutive blocks (of 8 offsets) of one window, 32 columns.  A window with up to 9 offsets has one or
+// two groups of 8 positions: the two warps of a channel group then split the contraction; with more they split the groups.
+__global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const ConvArgs a, int n_blocks) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ PairItem pairs_s[TC_PAIRS];
+  const int block = blockIdx.x, w = a.order[2 * block], d0 = a.order[2 * block + 1], b8 = d0 / 8;
+  auto is = [&](int x, int d) { return a.order[2 * x] == w && a.order[2 * x + 1] == d; };
+  if (b8 % TG_MERGE != 0 && block > 0 && is(block - 1, d0 - 8)) return;  // an earlier block's CTA takes this one too
+  int merged = 1;
+  while ((b8 + merged) % TG_MERGE != 0 && block + merged < n_blocks && is(block + merged, d0 + 8 * merged)) ++merged;
+  const int span = 2 * a.halo + 1, row = w / span, j = row + w % span - a.halo;
+  const int valid = min(8 * merged, a.win_cnt[w] - d0), groups = (7 + valid + 7) / 8;
+  const int col0 = blockIdx.y * TC_COLS, row_bytes = 2 * a.width;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3, half = warp >> 2;
+  const bool split_k = groups <= 2;
+  const int first_group = split_k ? 0 : 2 * half, mine = min(groups - first_group, 2);
+  const int T = a.nlon / 8, chunks = (T + TG_TILES - 1) / TG_TILES, stages = chunks * a.batch;
+  find_items(a, col0, pairs_s);
+  int shift = (a.win_lo[w] + d0) % a.nlon;
+  if (shift < 0) shift += a.nlon;
+  const size_t sample = (size_t)a.rows * a.nlon * row_bytes;
+  const unsigned char* grow = static_cast<const unsigned char*>(a.g) + (size_t)row * a.nlon * row_bytes;
+  const unsigned char* xrow = static_cast<const unsigned char*>(a.x) + (size_t)j * a.nlon * row_bytes;
+  uint4* const stage_s = reinterpret_cast<uint4*>(smem);
+  auto issue = [&](int s) {
+    const int b = s / chunks, t0 = (s - b * chunks) * TG_TILES, tl = min(TG_TILES, T - t0);
+    uint4* dst = stage_s + (s & 1) * TG_STAGE;
+    stage_positions<TG_SPG>(dst, grow + b * sample, 8 * t0, 8 * tl, a.nlon, row_bytes, 2 * col0);
+    stage_positions<TG_SPX>(dst + 8 * TG_SPG, xrow + b * sample, shift + 8 * t0, 8 * (tl + groups - 1), a.nlon, row_bytes, 2 * col0);
+    commit();
+  };
+  float acc[4][2][2][4];  // channel pair, group, component of x: rows (s = g: component 0 of g, g + 8: 1), columns r = 2 c, 2 c + 1
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) acc[p][n][q][x] = 0.f;
+
+  issue(0);
+  int k_index = 0;
+  for (int s = 0; s < stages; ++s) {
+    if (s + 1 < stages) {
+      issue(s + 1);
+      wait_copies<1>();
+    } else {
+      wait_copies<0>();
+    }
+    __syncthreads();
+    const int t0 = (s % chunks) * TG_TILES, tl = min(TG_TILES, T - t0);
+    const uint4* gs = stage_s + (s & 1) * TG_STAGE + g * TG_SPG + cg;
+    const uint4* xs = stage_s + (s & 1) * TG_STAGE + 8 * TG_SPG + g * TG_SPX + first_group * TC_PITCH + cg;
+    for (int k0 = 0; k0 < tl; k0 += 16, ++k_index) {
+      if (split_k && (k_index & 1) != half) continue;
+      const bool ragged = k0 + 16 > tl;
+      // the words of tile t = k0 + 2 c (+ 1, + 8, + 9); both operands are zero beyond the last tile
+      auto word = [&](const uint4* base, int t, int n) {
+        uint4 v = base[(t + n) * TC_PITCH];
+        if (ragged && t >= tl) v = make_uint4(0, 0, 0, 0);
+        return v;
+      };
+      const int t = k0 + 2 * c;
+      unsigned fa[4][4];
+      {
+        const uint4 v0 = word(gs, t, 0), v1 = word(gs, t + 1, 0), v8 = word(gs, t + 8, 0), v9 = word(gs, t + 9, 0);
+        const unsigned w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+        const unsigned w8[4] = {v8.x, v8.y, v8.z, v8.w}, w9[4] = {v9.x, v9.y, v9.z, v9.w};
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          fa[p][0] = __byte_perm(w0[p], w1[p], 0x5410);
+          fa[p][1] = __byte_perm(w0[p], w1[p], 0x7632);
+          fa[p][2] = __byte_perm(w8[p], w9[p], 0x5410);
+          fa[p][3] = __byte_perm(w8[p], w9[p], 0x7632);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 2; ++n) {
+        if (n >= mine) break;
+        const uint4 v0 = word(xs, t, n), v1 = word(xs, t + 1, n), v8 = word(xs, t + 8, n), v9 = word(xs, t + 9, n);
+        const unsigned w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+        const unsigned w8[4] = {v8.x, v8.y, v8.z, v8.w}, w9[4] = {v9.x, v9.y, v9.z, v9.w};
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          mma_add(acc[p][n][0], fa[p], __byte_perm(w0[p], w1[p], 0x5410), __byte_perm(w8[p], w9[p], 0x5410));
+          mma_add(acc[p][n][1], fa[p], __byte_perm(w0[p], w1[p], 0x7632), __byte_perm(w8[p], w9[p], 0x7632));
+        }
+      }
+    }
+    __syncthreads();
+  }
+
+  // ---- P blocks (half, channel pair, components) to shared memory, then the sums along their diagonals, always in one order
+  float* const p_s = reinterpret_cast<float*>(smem);
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int n = 0; n < 2; ++n)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        float* at = p_s + ((size_t)(half * TC_PAIRS + 4 * cg + p) * 4 + q) * TG_BLOCK + g * TG_PS + 8 * n + 2 * c;
+        *reinterpret_cast<float2*>(at) = make_float2(acc[p][n][q][0], acc[p][n][q][1]);                 // component 0 of g
+        *reinterpret_cast<float2*>(at + 2 * TG_BLOCK) = make_float2(acc[p][n][q][2], acc[p][n][q][3]);  // component 1
+      }
+  __syncthreads();
+  for (int x = threadIdx.x; x < TC_PAIRS * valid; x += TC_THREADS) {
+    const int p = x % TC_PAIRS, d = x / TC_PAIRS;
+    const PairItem it = pairs_s[p];
+    if (it.kind < 0) continue;
+    float v[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float sum = 0.f;
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const int r = s + d;
+        const float* at = p_s + ((size_t)p * 4 + q) * TG_BLOCK + s * TG_PS;
+        constexpr int OTHER = TC_PAIRS * 4 * TG_BLOCK;
+        if (split_k) sum += at[r] + at[r + OTHER];
+        else sum += r < 16 ? at[r] : at[r - 16 + OTHER];
+      }
+      v[q] = sum;
+    }
+    float* out = a.dtable + (size_t)(a.win_off[w] + d0 + d) * a.table_width + it.fcol;
+    if (it.kind == 0) *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+    else *reinterpret_cast<float2*>(out) = make_float2(v[0], v[3]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------------------------- apply
+constexpr int AP_TILES = 64;                              // tiles of 8 longitudes per CTA
+constexpr int AP_OFFSETS = 17;                            // offsets per stage: 17 + 7 positions are three k-steps
+constexpr int AP_SP = (AP_TILES + 2) * TC_PITCH;          // = 2 mod 8: the lanes' four r fall on different banks beside their two t
+static_assert(AP_SP % 8 == 2, "conflict-free 16-byte loads");
+constexpr int AP_SLOTS = 32;                              // offsets -7 .. 24 of a split table row, 8 bytes each
+constexpr int AP_PAIR = 3 * AP_SLOTS + 1;                 // 8-byte words per channel pair
+constexpr int AP_STAGE = 8 * AP_SP + (TC_PAIRS * AP_PAIR * 8 + 15) / 16;  // 16-byte words
+
+// One output of the sums by themselves: a sum that is not finite may owe it to a value outside its window (0 x Inf) or to
+// another component, so such outputs are formed again from their own neighbours alone.
+__device__ __noinline__ float2 apply_one(const ConvArgs& a, const __nv_bfloat16* x, int row, int l, int col, PairItem it) {
+  float2 y = make_float2(0.f, 0.f);
+  const int span = 2 * a.halo + 1;
+  for (int c = 0; c < span; ++c) {
+    const int j = row + c - a.halo;
+    if (j < 0 || j >= a.rows) continue;
+    const int cnt = a.win_cnt[row * span + c];
+    int lon = (l + (cnt ? a.win_lo[row * span + c] : 0)) % a.nlon;
+    if (lon < 0) lon += a.nlon;
+    for (int d = 0; d < cnt; ++d) {
+      const float* f = a.table + (size_t)(a.win_off[row * span + c] + d) * a.table_width + it.fcol;
+      const __nv_bfloat16* v = x + ((size_t)j * a.nlon + lon) * a.width + col;
+      const float vx = __bfloat162float(v[0]), vy = __bfloat162float(v[1]);
+      if (it.kind == 0) {
+        const float my = a.transpose ? f[2] : f[1], mz = a.transpose ? f[1] : f[2];
+        y.x = fmaf(f[0], vx, fmaf(my, vy, y.x));
+        y.y = fmaf(mz, vx, fmaf(f[3], vy, y.y));
+      } else {
+        y.x = fmaf(f[0], vx, y.x);
+        y.y = fmaf(f[1], vy, y.y);
+      }
+      lon = lon + 1 == a.nlon ? 0 : lon + 1;
+    }
+  }
+  return y;
+}
+
+// (x, y) = sum of three bfloat16 pairs, largest first
+__device__ __forceinline__ void split3(float x, float y, unsigned (&w)[3]) {
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+    w[s] = *reinterpret_cast<const unsigned*>(&h);
+    x -= __uint_as_float(w[s] << 16);
+    y -= __uint_as_float(w[s] & 0xffff0000u);
+  }
+}
+
+__global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const ConvArgs a, int col_blocks, int lon_blocks) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ PairItem pairs_s[TC_PAIRS];
+  int x = blockIdx.x;
+  const int cb = x % col_blocks;
+  x /= col_blocks;
+  const int lb = x % lon_blocks;
+  x /= lon_blocks;
+  const int b = x % a.batch, row = a.order[x / a.batch];  // heaviest rows first
+  const int col0 = cb * TC_COLS, row_bytes = 2 * a.width, span = 2 * a.halo + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3, half = warp >> 2;
+  const int T = a.nlon / 8, t0 = lb * AP_TILES, tl = min(AP_TILES, T - t0), tiles = (tl + 7) / 8;
+  find_items(a, col0, pairs_s);
+  const unsigned char* field = static_cast<const unsigned char*>(a.x) + (size_t)b * a.rows * a.nlon * row_bytes;
+  uint4* const stage_s = reinterpret_cast<uint4*>(smem);
+
+  // stages: offsets [d, d + n) of window w of this row
+  struct Stage { int w, d, n, cnt; };
+  auto first_of = [&](int w) {
+    for (; w < span; ++w) {
+      const int j = row + w - a.halo;
+      if (j < 0 || j >= a.rows) continue;
+      const int cnt = a.win_cnt[row * span + w];
+      if (cnt > 0) return Stage{w, 0, min(AP_OFFSETS, cnt), cnt};
+    }
+    return Stage{span, 0, 0, 0};
+  };
+  auto next_of = [&](const Stage& s) {
+    const int d = s.d + s.n;
+    return d < s.cnt ? Stage{s.w, d, min(AP_OFFSETS, s.cnt - d), s.cnt} : first_of(s.w + 1);
+  };
+  auto issue = [&](int buf, const Stage& s) {
+    int lon = (8 * t0 + a.win_lo[row * span + s.w] + s.d) % a.nlon;
+    if (lon < 0) lon += a.nlon;
+    const int steps = (7 + s.n + 7) / 8;
+    stage_positions<AP_SP>(stage_s + buf * AP_STAGE, field + (size_t)(row + s.w - a.halo) * a.nlon * row_bytes, lon, 8 * (tl + steps - 1), a.nlon, row_bytes, 2 * col0);
+    commit();
+  };
+  // this thread's two slots of the split table: a channel pair and the offsets slot - 7
+  const int tp = threadIdx.x & (TC_PAIRS - 1), ts = threadIdx.x / TC_PAIRS;
+  const PairItem item = pairs_s[tp];
+  auto fetch = [&](const Stage& s, float4 (&m)[2]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int d = ts + 16 * i - 7;
+      m[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (d >= 0 && d < s.n && item.kind >= 0) {
+        const float* f = a.table + (size_t)(a.win_off[row * span + s.w] + s.d + d) * a.table_width + item.fcol;
+        if (item.kind == 0) {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(f));
+          m[i] = a.transpose ? make_float4(v.x, v.z, v.y, v.w) : v;
+        } else {
+          const float2 v = __ldg(reinterpret_cast<const float2*>(f));
+          m[i] = make_float4(v.x, 0.f, 0.f, v.y);
+        }
+      }
+    }
+  };
+  auto place = [&](int buf, const float4 (&m)[2]) {
+    uint2* dst = reinterpret_cast<uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + tp * AP_PAIR + ts;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      unsigned w0[3], w1[3];
+      split3(m[i].x, m[i].y, w0);
+      split3(m[i].z, m[i].w, w1);
+#pragma unroll
+      for (int s = 0; s < 3; ++s) dst[s * AP_SLOTS + 16 * i] = make_uint2(w0[s], w1[s]);
+    }
+  };
+
+  float acc[4][4][4];  // channel pair, tile of 8 t: rows (s = g: component 0, g + 8: component 1), columns t = 2 c, 2 c + 1
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[p][i][v] = 0.f;
+
+  Stage cur = first_of(0);
+  float4 m[2];
+  if (cur.w < span) {
+    issue(0, cur);
+    fetch(cur, m);
+    place(0, m);
+  }
+  int buf = 0;
+  while (cur.w < span) {
+    const Stage nxt = next_of(cur);
+    const bool more = nxt.w < span;
+    if (more) {
+      issue(buf ^ 1, nxt);
+      fetch(nxt, m);
+      wait_copies<1>();
+    } else {
+      wait_copies<0>();
+    }
+    __syncthreads();
+    const uint4* xs = stage_s + buf * AP_STAGE + c * AP_SP + cg;
+    const uint2* ms = reinterpret_cast<const uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + 4 * cg * AP_PAIR + 7 + c - g;
+    const int steps = (7 + cur.n + 7) / 8;
+    for (int k = 0; k < steps; ++k) {
+      unsigned fb[4][2][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int tile = half + 2 * i;
+        if (tile >= tiles) break;
+        const uint4* at = xs + (8 * tile + g + k) * TC_PITCH;
+        const uint4 v0 = at[0], v4 = at[4 * AP_SP];
+        fb[i][0][0] = v0.x; fb[i][0][1] = v0.y; fb[i][0][2] = v0.z; fb[i][0][3] = v0.w;
+        fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
+      }
+#pragma unroll
+      for (int s = 0; s < 3; ++s)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          const uint2* f = ms + p * AP_PAIR + s * AP_SLOTS + 8 * k;
+          const uint2 a01 = f[0], a23 = f[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if (half + 2 * i >= tiles) break;
+            mma(acc[p][i], a01.x, a01.y, a23.x, a23.y, fb[i][0][p], fb[i][1][p]);
+          }
+        }
+    }
+    if (more) place(buf ^ 1, m);
+    __syncthreads();
+    cur = nxt;
+    buf ^= 1;
+  }
+
+  // ---- four channel pairs of a position are 16 bytes of its row
+  const int col = col0 + 8 * cg;
+  if (col >= a.width) return;
+  __nv_bfloat16* y = static_cast<__nv_bfloat16*>(a.y) + ((size_t)b * a.rows + row) * a.nlon * a.width + col;
+  const __nv_bfloat16* xf = reinterpret_cast<const __nv_bfloat16*>(field);
+  bool whole = true;
+#pragma unroll
+  for (int p = 0; p < 4; ++p) whole = whole && pairs_s[4 * cg + p].kind >= 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int t = 8 * (half + 2 * i) + 2 * c + e;
+      if (t >= tl) continue;
+      const int l = 8 * (t0 + t) + g;
+      unsigned word[4];
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+        float2 v = make_float2(acc[p][i][e], acc[p][i][2 + e]);
+        const PairItem it = pairs_s[4 * cg + p];
+        if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && it.kind >= 0) v = apply_one(a, xf, row, l, col + 2 * p, it);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+        word[p] = *reinterpret_cast<const unsigned*>(&h);
+      }
+      __nv_bfloat16* at = y + (size_t)l * a.width;
+      if (whole) {
+        *reinterpret_cast<uint4*>(at) = make_uint4(word[0], word[1], word[2], word[3]);
+      } else {
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+          if (pairs_s[4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(at + 2 * p) = word[p];
+      }
+    }
+}
+
+}  // namespace
+
+bool tensor_cores_take(const ConvArgs& a) {
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.y);
+  return a.nlon % 8 == 0 && a.width % 8 == 0 && bits % 16 == 0;
+}
+
+int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream) {
+  const int col_blocks = (a.width + TC_COLS - 1) / TC_COLS, lon_blocks = (a.nlon / 8 + AP_TILES - 1) / AP_TILES;
+  const int64_t ctas = (int64_t)col_blocks * lon_blocks * a.batch * n_order;
+  GM_REQUIRE(ctas < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_conv_apply: too many tiles");
+  const size_t smem = 2 * (size_t)AP_STAGE * 16;
+  const int st = allow_smem(conv_apply_tc_kernel, smem, "gm_lattice_conv_apply");
+  if (st != GM_OK) return st;
+  conv_apply_tc_kernel<<<(unsigned)ctas, TC_THREADS, smem, stream>>>(a, col_blocks, lon_blocks);
+  return launch_status("gm_lattice_conv_apply");
+}
+
+int table_grad_tc(const ConvArgs& a, int64_t n_blocks, cudaStream_t stream) {
+  const int col_blocks = (a.width + TC_COLS - 1) / TC_COLS;
+  const size_t smem = 2 * (size_t)TG_STAGE * 16;
+  const int st = allow_smem(conv_table_grad_tc_kernel, smem, "gm_lattice_conv_table_grad");
+  if (st != GM_OK) return st;
+  conv_table_grad_tc_kernel<<<dim3((unsigned)n_blocks, col_blocks), TC_THREADS, smem, stream>>>(a, (int)n_blocks);
+  return launch_status("gm_lattice_conv_table_grad");
+}
+
+}  // namespace lconv
+}  // namespace gmb

@@ -80,7 +80,7 @@ def conv_tables(geometry: Any, distances: Tensor, weights: Tensor, rows: Sequenc
     device = edge.device
     cnt = lat.win_cnt.cpu().numpy().reshape(-1)
     blocks = [(w, d) for w in np.flatnonzero(cnt > 0) for d in range(0, int(cnt[w]), OFFSETS_PER_BLOCK)]
-    blocks.sort(key=lambda wd: -min(OFFSETS_PER_BLOCK, int(cnt[wd[0]]) - wd[1]))  # full blocks first
+    blocks.sort(key=lambda wd: -min(OFFSETS_PER_BLOCK, int(cnt[wd[0]])))  # windows with a full block first, a window's blocks together
     rho = geometry.rho.index_select(0, edge).float()
     tau = [torch.view_as_complex(geometry.transport.index_select(0, edge)[:, n].float().contiguous()) for n, *_ in complex_rows]
     omega = []

@@ -161,6 +161,92 @@ def test_apply_against_the_host_loops(nlat, nlon, reach, head, batch, storage):
         assert_close(got, want, 2.0 ** -8 if storage == "bf16" else 1e-5, atol, "transposed" if transposed else "forward")
 
 
+# bfloat16 rows of a multiple of 16 bytes: tensor cores.  One tile of 8 longitudes; column blocks of 32 partly filled; more
+# than 64 tiles (two CTAs along a row, chunks of 32 tiles with a remainder); windows of one to several stages
+TENSOR_CORE_CASES = [
+    (5, 8, 1.5, {0: 2, 1: 1, 2: 2}, 1),
+    (6, 24, 2.0, {0: 8, 1: 8}, 3),
+    (4, 560, 1.3, {0: 8, 1: 8, 2: 8}, 2),
+    (12, 136, 3.0, {0: 4, 1: 14}, 1),
+]
+
+
+def tensor_core_case(nlat, nlon, reach, head):
+    from types import SimpleNamespace
+
+    from gm_attention_b200.nn.lattice_depthwise import conv_tables
+
+    c = make_case(nlat, nlon, reach * math.pi / nlat, head, 1, dtype=np.float32)
+    geometry = SimpleNamespace(transport=cuda(c.transport), angular=cuda(c.angular), rho=cuda(c.rho), bias=cuda(c.bias), inside=cuda(c.inside),
+                               row_ptr=cuda(c.row_ptr), source=cuda(c.source))
+    return c, conv_tables(geometry, cuda(c.rho * np.float32(c.radius)), cuda(c.weights), descriptor_rows(c.head_type, 1), nlat, nlon)
+
+
+@pytest.mark.parametrize("nlat, nlon, reach, head, batch", TENSOR_CORE_CASES)
+def test_tensor_core_kernels_against_the_host_loops(nlat, nlon, reach, head, batch):
+    """apply (one rounding to bf16, 2^-9, and 1e-5 of the largest for the float32 sums), transposed and not, and the table
+    gradient (float32 sums over nlon x batch products of bf16 values: 1e-5 of the largest) against float64, whatever order
+    the blocks come in."""
+    import dataclasses
+
+    from gm_attention_b200.nn.lattice_depthwise import _apply, _table_gradient
+    from tests.test_lattice_depthwise_cpu import _apply_on_the_host
+
+    c, t = tensor_core_case(nlat, nlon, reach, head)
+    lat = t.lattice
+    assert c.width % 8 == 0
+    table, = seeded((t.n_entries, t.table_width), 71, np.float32)
+    x, g = (torch.from_numpy(v).bfloat16() for v in seeded((batch * c.n_nodes, c.width), 72, np.float32, 2))
+    items = t.items.cpu().numpy().tolist()
+    sample = slice((batch - 1) * c.n_nodes, batch * c.n_nodes)
+    for transposed in (False, True):
+        windows = (lat.t_win_cnt, lat.t_win_lo, lat.t_win_off) if transposed else (lat.win_cnt, lat.win_lo, lat.win_off)
+        used = table[lat.t_entry.cpu().numpy()] if transposed else table
+        want = _apply_on_the_host(x[sample].double().numpy(), used.astype(np.float64), *(w.cpu().numpy() for w in windows), items, nlat, nlon, lat.halo,
+                                  transposed)
+        got = _apply(x.cuda(), cuda(used), t, transposed)[sample].float().cpu().numpy()
+        assert_close(got, want, 2.0 ** -8, 1e-5 * np.abs(want).max(), "transposed" if transposed else "forward")
+    cnt, lo, off = (w.cpu().numpy() for w in (lat.win_cnt, lat.win_lo, lat.win_off))
+    X, G = (v.double().numpy().reshape(batch, nlat, nlon, c.width) for v in (x, g))
+    want = np.zeros((t.n_entries, t.table_width))
+    for i in range(nlat):
+        for w in range(2 * lat.halo + 1):
+            for d in range(int(cnt[i, w])):
+                xs = np.roll(X[:, i + w - lat.halo], -(int(lo[i, w]) + d), axis=1)
+                for kind, col, fcol in items:
+                    m = np.einsum("bla,blc->ac", G[:, i, :, col:col + 2], xs[:, :, col:col + 2])
+                    want[off[i, w] + d, fcol:fcol + (4 if kind == 0 else 2)] = m.reshape(-1) if kind == 0 else (m[0, 0], m[1, 1])
+    order = torch.randperm(t.blocks.shape[0], generator=torch.Generator().manual_seed(5))
+    for blocks in (t.blocks, t.blocks[order.to(t.blocks.device)].contiguous()):
+        got = _table_gradient(g.cuda(), x.cuda(), dataclasses.replace(t, blocks=blocks))
+        assert_close(got.cpu().numpy(), want, 1e-5, 1e-5 * np.abs(want).max(), "table gradient")
+
+
+def test_tensor_core_apply_touches_only_true_neighbours():
+    """An Inf, a NaN and a value whose products overflow reach exactly the targets that see their nodes, in their own channel."""
+    from gm_attention_b200.nn.lattice_depthwise import _apply
+
+    c, t = tensor_core_case(16, 64, 3.0, {0: 4, 1: 6})
+    table, = seeded((t.n_entries, t.table_width), 73, np.float32)
+    v, = seeded((c.n_nodes, c.width), 74, np.float32)
+    clean = torch.from_numpy(v).bfloat16().cuda()
+    want = _apply(clean, cuda(table), t, False)
+    dirty = clean.clone()
+    nodes = [(5 * c.nlon + 63, 5, float("inf")), (9 * c.nlon + 20, 2, float("nan")), (0, 9, 3e38)]
+    for node, col, value in nodes:
+        dirty[node, col] = value
+    got = _apply(dirty, cuda(table), t, False)
+    touched = torch.zeros_like(got, dtype=torch.bool)
+    for node, col, value in nodes:
+        seen_by = torch.from_numpy(np.unique(c.target[c.source == node])).cuda()
+        first = col if col < 4 else col - col % 2  # scalar channels stand alone, (re, im) go together
+        for x in range(first, first + (1 if col < 4 else 2)):
+            touched[seen_by, x] = True
+            if value != 3e38:
+                assert not torch.isfinite(got[seen_by, x].float()).any()
+    assert torch.equal(got[~touched], want[~touched])
+
+
 @pytest.mark.parametrize("head", [{0: 2, 1: 1}, {0: 6, 1: 5, 2: 7}, {1: 3}, {0: 130, 1: 130}, {0: 4}])
 def test_fold_kernel_equals_the_tensor_algebra(head):
     """One launch each way against :func:`fold` and its autograd gradients: a handful of float32 products per value, 2e-6 of
