@@ -86,8 +86,9 @@ constexpr int TG_SPX = (TG_TILES + 4) * TC_PITCH + 1;
 constexpr int TG_STAGE = 8 * (TG_SPG + TG_SPX);   // 16-byte words
 constexpr int TG_PS = 18;                         // floats between the s of a P block
 constexpr int TG_BLOCK = 8 * TG_PS;               // floats of a P block: 8 s x 16 r
+constexpr int TG_PAIR = 4 * TG_BLOCK + 2;         // floats of a channel pair's four: the pairs start on different banks
 constexpr int TG_MERGE = 3;                       // blocks of 8 offsets one CTA takes: 24 + 7 positions are four groups of 8
-static_assert(2 * TC_PAIRS * 4 * TG_BLOCK * 4 <= 2 * TG_STAGE * 16, "the P blocks reuse the stages");
+static_assert(2 * TC_PAIRS * TG_PAIR * 4 <= 2 * TG_STAGE * 16, "the P blocks reuse the stages");
 
 // One CTA: up to three consecutive blocks (of 8 offsets) of one window, 32 columns.  A window with up to 9 offsets has one or
 // two groups of 8 positions: the two warps of a channel group then split the contraction; with more they split the groups.
@@ -143,13 +144,11 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const
     const int t0 = (s % chunks) * TG_TILES, tl = min(TG_TILES, T - t0);
     const uint4* gs = stage_s + (s & 1) * TG_STAGE + g * TG_SPG + cg;
     const uint4* xs = stage_s + (s & 1) * TG_STAGE + 8 * TG_SPG + g * TG_SPX + first_group * TC_PITCH + cg;
-    for (int k0 = 0; k0 < tl; k0 += 16, ++k_index) {
-      if (split_k && (k_index & 1) != half) continue;
-      const bool ragged = k0 + 16 > tl;
-      // the words of tile t = k0 + 2 c (+ 1, + 8, + 9); both operands are zero beyond the last tile
+    // the words of tile t = k0 + 2 c (+ 1, + 8, + 9); both operands are zero beyond the last tile
+    auto step = [&](int k0, auto is_ragged) {
       auto word = [&](const uint4* base, int t, int n) {
         uint4 v = base[(t + n) * TC_PITCH];
-        if (ragged && t >= tl) v = make_uint4(0, 0, 0, 0);
+        if (decltype(is_ragged)::value && t >= tl) v = make_uint4(0, 0, 0, 0);
         return v;
       };
       const int t = k0 + 2 * c;
@@ -168,16 +167,22 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const
       }
 #pragma unroll
       for (int n = 0; n < 2; ++n) {
-        if (n >= mine) break;
-        const uint4 v0 = word(xs, t, n), v1 = word(xs, t + 1, n), v8 = word(xs, t + 8, n), v9 = word(xs, t + 9, n);
-        const unsigned w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
-        const unsigned w8[4] = {v8.x, v8.y, v8.z, v8.w}, w9[4] = {v9.x, v9.y, v9.z, v9.w};
+        if (n < mine) {
+          const uint4 v0 = word(xs, t, n), v1 = word(xs, t + 1, n), v8 = word(xs, t + 8, n), v9 = word(xs, t + 9, n);
+          const unsigned w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
+          const unsigned w8[4] = {v8.x, v8.y, v8.z, v8.w}, w9[4] = {v9.x, v9.y, v9.z, v9.w};
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          mma_add(acc[p][n][0], fa[p], __byte_perm(w0[p], w1[p], 0x5410), __byte_perm(w8[p], w9[p], 0x5410));
-          mma_add(acc[p][n][1], fa[p], __byte_perm(w0[p], w1[p], 0x7632), __byte_perm(w8[p], w9[p], 0x7632));
+          for (int p = 0; p < 4; ++p) {
+            mma_add(acc[p][n][0], fa[p], __byte_perm(w0[p], w1[p], 0x5410), __byte_perm(w8[p], w9[p], 0x5410));
+            mma_add(acc[p][n][1], fa[p], __byte_perm(w0[p], w1[p], 0x7632), __byte_perm(w8[p], w9[p], 0x7632));
+          }
         }
       }
+    };
+    for (int k0 = 0; k0 < tl; k0 += 16, ++k_index) {
+      if (split_k && (k_index & 1) != half) continue;
+      if (k0 + 16 <= tl) step(k0, std::false_type{});
+      else step(k0, std::true_type{});
     }
     __syncthreads();
   }
@@ -190,7 +195,7 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const
     for (int n = 0; n < 2; ++n)
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        float* at = p_s + ((size_t)(half * TC_PAIRS + 4 * cg + p) * 4 + q) * TG_BLOCK + g * TG_PS + 8 * n + 2 * c;
+        float* at = p_s + (half * TC_PAIRS + 4 * cg + p) * TG_PAIR + q * TG_BLOCK + g * TG_PS + 8 * n + 2 * c;
         *reinterpret_cast<float2*>(at) = make_float2(acc[p][n][q][0], acc[p][n][q][1]);                 // component 0 of g
         *reinterpret_cast<float2*>(at + 2 * TG_BLOCK) = make_float2(acc[p][n][q][2], acc[p][n][q][3]);  // component 1
       }
@@ -206,8 +211,8 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const
 #pragma unroll
       for (int s = 0; s < 8; ++s) {
         const int r = s + d;
-        const float* at = p_s + ((size_t)p * 4 + q) * TG_BLOCK + s * TG_PS;
-        constexpr int OTHER = TC_PAIRS * 4 * TG_BLOCK;
+        const float* at = p_s + p * TG_PAIR + q * TG_BLOCK + s * TG_PS;
+        constexpr int OTHER = TC_PAIRS * TG_PAIR;
         if (split_k) sum += at[r] + at[r + OTHER];
         else sum += r < 16 ? at[r] : at[r - 16 + OTHER];
       }
@@ -368,30 +373,31 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const Conv
     const uint4* xs = stage_s + buf * AP_STAGE + c * AP_SP + cg;
     const uint2* ms = reinterpret_cast<const uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + 4 * cg * AP_PAIR + 7 + c - g;
     const int steps = (7 + cur.n + 7) / 8;
-    for (int k = 0; k < steps; ++k) {
-      unsigned fb[4][2][4];
+    auto walk = [&](auto mine) {  // tiles half, half + 2, ... of the CTA's (a tile too many reads what a stage left behind: its own columns)
+      constexpr int MINE = decltype(mine)::value;
+      for (int k = 0; k < steps; ++k) {
+        unsigned fb[MINE][2][4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int tile = half + 2 * i;
-        if (tile >= tiles) break;
-        const uint4* at = xs + (8 * tile + g + k) * TC_PITCH;
-        const uint4 v0 = at[0], v4 = at[4 * AP_SP];
-        fb[i][0][0] = v0.x; fb[i][0][1] = v0.y; fb[i][0][2] = v0.z; fb[i][0][3] = v0.w;
-        fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
-      }
-#pragma unroll
-      for (int s = 0; s < 3; ++s)
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const uint2* f = ms + p * AP_PAIR + s * AP_SLOTS + 8 * k;
-          const uint2 a01 = f[0], a23 = f[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if (half + 2 * i >= tiles) break;
-            mma(acc[p][i], a01.x, a01.y, a23.x, a23.y, fb[i][0][p], fb[i][1][p]);
-          }
+        for (int i = 0; i < MINE; ++i) {
+          const uint4* at = xs + (8 * (half + 2 * i) + g + k) * TC_PITCH;
+          const uint4 v0 = at[0], v4 = at[4 * AP_SP];
+          fb[i][0][0] = v0.x; fb[i][0][1] = v0.y; fb[i][0][2] = v0.z; fb[i][0][3] = v0.w;
+          fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
         }
-    }
+#pragma unroll
+        for (int s = 0; s < 3; ++s)
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            const uint2* f = ms + p * AP_PAIR + s * AP_SLOTS + 8 * k;
+            const uint2 a01 = f[0], a23 = f[4];
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) mma(acc[p][i], a01.x, a01.y, a23.x, a23.y, fb[i][0][p], fb[i][1][p]);
+          }
+      }
+    };
+    if (tiles > 4) walk(std::integral_constant<int, 4>());
+    else if (tiles > 2) walk(std::integral_constant<int, 2>());
+    else walk(std::integral_constant<int, 1>());
     if (more) place(buf ^ 1, m);
     __syncthreads();
     cur = nxt;
