@@ -405,7 +405,7 @@ __device__ __forceinline__ int build_conv_items(const int64_t* desc, int F, Conv
 // Depthwise conv, forward: a warp per target node, a lane per item (scalar items and complex items in separate
 // passes, so a pass never diverges); the node's edges are walked in order -- same summation order per output as a
 // sequential loop -- four at a time, with the four edges' loads issued before their arithmetic.
-constexpr int CONV_UNROLL = 4;
+constexpr int CONV_UNROLL = 4, CONV_BACKWARD_UNROLL = 3;  // (backward: 1 033 us with four, 950 with three, 1 083 with two; forward 682, 714, 856)
 
 template <typename T>
 __global__ void conv_forward_kernel(ConvArgs<T> a) {
@@ -506,18 +506,18 @@ __global__ void conv_backward_kernel(ConvArgs<T> a) {
       const ConvItem it = items_s[t0 + lane];
       const T dy = a.g[i * a.D + it.col];
       int64_t e = e0;
-      for (; e + CONV_UNROLL <= e1; e += CONV_UNROLL) {
-        T w[CONV_UNROLL], r[CONV_UNROLL], x[CONV_UNROLL];
-        int64_t j[CONV_UNROLL];
+      for (; e + CONV_BACKWARD_UNROLL <= e1; e += CONV_BACKWARD_UNROLL) {
+        T w[CONV_BACKWARD_UNROLL], r[CONV_BACKWARD_UNROLL], x[CONV_BACKWARD_UNROLL];
+        int64_t j[CONV_BACKWARD_UNROLL];
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) {
+        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u) {
           j[u] = a.source[e + u];
           w[u] = a.weights[e + u];
           r[u] = a.rc[(e + u) * a.A0 + it.coef];
           x[u] = a.v[j[u] * a.D + it.col];
         }
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) {
+        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u) {
           const T dm = w[u] * dy;
           a.drc[(e + u) * a.A0 + it.coef] = dm * x[u];
           atomicAdd(a.dv + j[u] * a.D + it.col, dm * r[u]);
@@ -556,12 +556,12 @@ __global__ void conv_backward_kernel(ConvArgs<T> a) {
         atomicAdd(a.dv + j * a.D + it.col + 1, tr * dzi - ti * dzr);
       };
       int64_t e = e0;
-      for (; e + CONV_UNROLL <= e1; e += CONV_UNROLL) {
-        T w[CONV_UNROLL], rho[CONV_UNROLL], tr[CONV_UNROLL], ti[CONV_UNROLL], vr[CONV_UNROLL], vi[CONV_UNROLL];
-        T Ar[CONV_UNROLL], Ai[CONV_UNROLL], Br[CONV_UNROLL], Bi[CONV_UNROLL], ar[CONV_UNROLL], ai[CONV_UNROLL];
-        int64_t j[CONV_UNROLL];
+      for (; e + CONV_BACKWARD_UNROLL <= e1; e += CONV_BACKWARD_UNROLL) {
+        T w[CONV_BACKWARD_UNROLL], rho[CONV_BACKWARD_UNROLL], tr[CONV_BACKWARD_UNROLL], ti[CONV_BACKWARD_UNROLL], vr[CONV_BACKWARD_UNROLL], vi[CONV_BACKWARD_UNROLL];
+        T Ar[CONV_BACKWARD_UNROLL], Ai[CONV_BACKWARD_UNROLL], Br[CONV_BACKWARD_UNROLL], Bi[CONV_BACKWARD_UNROLL], ar[CONV_BACKWARD_UNROLL], ai[CONV_BACKWARD_UNROLL];
+        int64_t j[CONV_BACKWARD_UNROLL];
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) {
+        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u) {
           const int64_t eu = e + u;
           j[u] = a.source[eu];
           w[u] = a.weights[eu];
@@ -574,7 +574,7 @@ __global__ void conv_backward_kernel(ConvArgs<T> a) {
           load_pair(co + 2 * it.mult, Br[u], Bi[u]);
         }
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u)
+        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u)
           edge(e + u, j[u], w[u], rho[u], tr[u], ti[u], vr[u], vi[u], Ar[u], Ai[u], Br[u], Bi[u], ar[u], ai[u]);
       }
       for (; e < e1; ++e) {
@@ -594,9 +594,11 @@ __global__ void conv_backward_kernel(ConvArgs<T> a) {
 
 constexpr int CONV_THREADS = 128;  // 4 target nodes per CTA
 
-int conv_grid(int64_t n_nodes) {  // a few CTAs per SM, each striding the nodes: the item table is built once per CTA
+int conv_grid(int64_t n_nodes) {  // CTAs stride the nodes, so that the item table is built once for several: up to 64
+  // per SM (16, all resident at once, leave the polar rows' nodes to few of them: depthwise 682 + 1 033 us against
+  // 675 + 989, the scores' backward 897 against 796)
   const int64_t want = (n_nodes + CONV_THREADS / 32 - 1) / (CONV_THREADS / 32);
-  const int64_t cap = (int64_t)sm_count() * 16;
+  const int64_t cap = (int64_t)sm_count() * 64;
   return (int)(want < cap ? (want < 1 ? 1 : want) : cap);
 }
 
