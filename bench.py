@@ -540,11 +540,11 @@ def run_ours(args: argparse.Namespace, cfg: dict) -> None:
                 b_ev.record()
             torch.cuda.synchronize()
             per_pass[name] = statistics.mean(x.elapsed_time(y) for x, y in ev[1:])
-        top_kernel = "lattice_tn_kernel<1,2,2,TC_BWD_S,4> (source-major backward pass: dk, dv)"
+        top_kernel = "lattice_packed_kernel<1,2,2,TC_BWD_S,4> (source-major backward pass: dk, dv)"
         top_ms = per_pass["pass_s"]
         top_bytes = 6 * n_rows_local * D * elem + 2 * n_rows_local * heads * 4
         # DRAM read + write of this kernel per node, from the ncu capture on the 128x256x4 workload (profiles/), scaled by nodes
-        top_traffic = int(4926 * n_rows_local)
+        top_traffic = int(3861 * n_rows_local)
         del out0, lse0, ws
     else:
         per_pass = None
@@ -656,7 +656,7 @@ def run_ours(args: argparse.Namespace, cfg: dict) -> None:
                "job_bytes_per_direction": total_bytes, "band_cuts": e2e_cuts,
                "last_step_phases_ms_slowest_rank": phases}
 
-    # a wait on a TMA completion barrier that ran out is recorded by the kernels instead of hanging: results would be invalid
+    # a wait for a copy that ran out would be recorded by the kernels instead of hanging: results would be invalid
     import ctypes
     expired = ctypes.c_int(0)
     _lib.call("gm_lattice_attention_tc_wait_expired", ctypes.byref(expired))
