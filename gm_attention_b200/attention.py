@@ -149,7 +149,7 @@ def tensor_core_plan(desc_rows: tuple[tuple[int, int, int, int, int], ...], head
     """The plan of one pass (0 forward, 1 target-major, 2 source-major, on the transposed tables); ``None`` where the
     tensor-core kernels do not serve the layout."""
     tables = (win_cnt, win_lo, win_off, entries)
-    if not entries.is_cuda or entries.shape[0] == 0 or entries.shape[1] != 8 or 2 * halo + 1 > 33 or orders != sum(r[0] > 0 for r in desc_rows):
+    if not entries.is_cuda or entries.shape[0] == 0 or entries.shape[1] != 8 or 2 * halo + 1 > 33 or [r[0] for r in desc_rows if r[0]] != list(range(1, orders + 1)):
         return None
     if not tensor_core_layout_supported(desc_rows) or any(t.is_inference() for t in tables):
         return None
@@ -168,6 +168,7 @@ def tensor_core_plan(desc_rows: tuple[tuple[int, int, int, int, int], ...], head
         torch.cumsum(counts, 0, dtype=torch.int32, out=first[1:])
         records = torch.empty(int(first[-1]) * size.value, dtype=torch.uint8, device=device)
         _lib.call("gm_lattice_plan_build", *common, None, _lib.ptr(first), _lib.ptr(records), _lib.stream(device))
+        torch.cuda.current_stream(device).synchronize()  # like the tables themselves, complete for whichever stream uses it
     return TensorCorePlan(first, records, (desc_rows, heads, rows, nlon, halo, orders), tuple((t, t._version) for t in tables))
 
 

@@ -417,3 +417,18 @@ def test_packed_tensor_core_kernels(case):
     assert lat.plan_pointers(0) == lat.plan_pointers(1) == (None, None) and lat.plan_pointers(2)[1]
     turned = run(lat)
     assert torch.equal(turned[0], run(dataclasses.replace(lat, tc_plans=(None, None, None)))[0]) and not torch.equal(turned[0], planned[0])
+
+
+def test_tables_without_a_plan():
+    """Head layouts the tensor-core kernels do not take (orders out of turn) still make tables for the others."""
+    from gm_attention_b200.attention import AttentionTables, build_lattice_tables, lattice_attention_forward
+
+    c = make_case(6, 16, 2 * math.pi / 6, {0: 2, 1: 2, 2: 2}, 1, dtype=np.float32)
+    rows = [tuple(int(x) for x in row) for row in c.desc]
+    general = AttentionTables(cuda(c.transport), cuda(c.bias), cuda(c.inside), cuda(c.row_ptr), cuda(c.source), tuple(rows), c.heads, c.scale)
+    q, k, v = (cuda(x) for x in seeded((c.n_nodes, c.width), 64, np.float32, 3))
+    want, _ = lattice_attention_forward(q, k, v, build_lattice_tables(general, c.nlat, c.nlon, tuple(rows), c.heads, c.scale))
+    turned = build_lattice_tables(general, c.nlat, c.nlon, (rows[0], rows[2], rows[1]), c.heads, c.scale)
+    assert turned.tc_plans == (None, None, None)
+    got, _ = lattice_attention_forward(q, k, v, turned)
+    assert float((got - want).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
