@@ -35,6 +35,11 @@ constexpr int FDESC = 8;
 constexpr int FTHREADS = 128;
 constexpr int MAX_TILE = 64;       // edges per tile, at most (a power of two; less where shared memory is short)
 constexpr int MAX_OWNED = 64;      // K * C <= 64 * 128 in the backward
+// A tile of 64 edges while six CTAs of it share an SM, 32 beyond: a wide packed row (13 blocks to {4, 4, 4}: 100 columns, 53 KB at
+// 64 edges) leaves four CTAs' warps to hide the barriers, a narrow one (18 columns) pays them twice as often for nothing.
+// 128 x 256, radius 3 pi / 128, 100 columns: forward 1 309 us with 64 edges, 1 034 with 32, 1 122 with 16; backward 2 494, 2 460, 3 076.
+// Narrow rows lose with 32: 118 x 236, radius 4 pi / 118, 18 columns, the pass 4.08 -> 4.50 ms.
+constexpr size_t FSMEM_SIXTH = 227 * 1024 / 6 - 1024;
 constexpr size_t FSMEM_MOST = 224 * 1024;  // dynamic shared memory a CTA may ask for, beside the static arrays
 constexpr int TP = 5;              // rows t of a dZ patch (4 columns wide)
 
@@ -657,11 +662,14 @@ extern "C" int gm_factored_forward_scaled(const void* h, const void* zc, const v
     a.out = (T*)out;
     const int C = 2 * wc + wr;
     const size_t extra = (size_t)(n_blocks * FDESC) * sizeof(int32_t) + (size_t)(n_blocks + d_out) * sizeof(int4);
-    // 64 edges per tile; fewer where the packed width or the phase tables leave no room for them
+    // 64 or 32 edges per tile; fewer where the packed width or the phase tables leave no room for them
     int tile = MAX_TILE;
+    if (ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra > FSMEM_SIXTH) tile /= 2;
     while (tile > 8 && ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra > 200 * 1024) tile /= 2;
     size_t smem = ForwardLayout<T>(k, C, n_f, n_scales, n_blocks, d_out, tile).total * sizeof(T) + extra;
-    const int64_t cap = (int64_t)sm_count() * 16;  // the CTAs stride the sources: the column list is built once per CTA
+    // the CTAs stride the sources, so that the column list is built once for several; with the smaller tiles more of them pay
+    // (16 per SM 1 149 us, 64 1 034; with 64 edges 1 309 and 1 330)
+    const int64_t cap = (int64_t)sm_count() * (tile < MAX_TILE ? 64 : 16);
     const unsigned blocks = (unsigned)(n_groups < cap ? n_groups : cap);
     auto go = [&](auto kernel, int x) {
       const int st = allow_smem(kernel, smem, "gm_factored_forward");
@@ -722,9 +730,10 @@ extern "C" int gm_factored_backward_scaled(const void* g, const int64_t* target,
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.g = (const T*)g; a.target = target; a.weights = aggregated ? (const T*)weights : nullptr; a.rows = aggregated ? (const T*)rows : nullptr;
     a.dh = (T*)dh; a.dzc = (T*)dzc; a.dzr = (T*)dzr; a.dweights = aggregated ? (T*)dweights : nullptr;
-    // 64 edges per tile; fewer where the packed width is so large that 64 rows of it do not fit shared memory
+    // 64 or 32 edges per tile; fewer where the packed width is so large that they do not fit shared memory
     int tile = MAX_TILE;
     auto layout = [&](bool staged) { return BackwardLayout<T>(k, C, n_f, n_scales, d_out, tile, staged); };
+    if (layout(true).total * sizeof(T) > FSMEM_SIXTH) tile /= 2;
     while (tile > 8 && layout(true).total * sizeof(T) > 200 * 1024) tile /= 2;
     const bool staged = layout(true).total * sizeof(T) <= FSMEM_MOST;
     const BackwardLayout<T> L = layout(staged);
