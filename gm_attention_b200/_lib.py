@@ -39,6 +39,7 @@ SIGNATURES: dict[str, list[Any]] = {
     "gm_lattice_attention_backward_tc_passes": [_P] * 11 + [_I] + [_P] * 5 + [_I, _P, _I, _I, _I, _L, _I, _I, _I, _I, _I, _D, _P, _P, _P, _P, _I, _P],
     "gm_lattice_plan_size": [_P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "gm_lattice_plan_build": [_P] * 5 + [_I] * 8 + [_P] * 4,
+    "gm_lattice_plan_refresh": [_P] * 5 + [_I] * 8 + [_L, _P, _L, _P, _P],
     "gm_lattice_attention_forward_planned": [_P] * 8 + [_I, _P, _I, _I, _I, _L, _I, _I, _I, _I, _I, _D, _P, _P, _P, _P, _P],
     "gm_lattice_attention_backward_planned": [_P] * 11 + [_I] + [_P] * 5 + [_I, _P, _I, _I, _I, _L, _I, _I, _I, _I, _I, _D, _P, _P, _P, _P, _I]
     + [_P] * 5,

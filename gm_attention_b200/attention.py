@@ -17,7 +17,7 @@ from __future__ import annotations
 
 import ctypes
 import os
-from dataclasses import dataclass
+from dataclasses import dataclass, replace
 from typing import Any
 
 import torch
@@ -129,47 +129,77 @@ class GaugeAttention(torch.autograd.Function):
 
 # ----------------------------------------------------------------------------- equiangular lattices
 
+#: (node, sample, head) triples from which a pass takes its plan.  Refreshing it and looking for row tiles it does not fit are two
+#: launches, about 10 us a pass; below, a CTA's own packing costs less.  Forward / target-major / source-major, us with the plan and
+#: without: 45 x 90, 4 heads (16 200) 38 / 44 / 52 against 34 / 41 / 47; 64 x 128, 4 heads (32 768) 48 / 58 / 65 against 45 / 60 / 68;
+#: 91 x 180, batch 3, 4 heads (196 560) 159 / 214 / 267 against 188 / 260 / 299.
+PLANNED_FROM = 32768
+#: format of the records ``gm_lattice_plan_build`` writes; a plan that was saved with another one is not used
+PLAN_FORMAT = 2
+
+
 @dataclass(frozen=True, eq=False)
 class TensorCorePlan:
     """What the tensor-core lattice kernels read besides the tables (``gm_lattice_plan_build`` in ``include/gm_b200.h``): the
-    packed neighbour lists and entries of every row tile, and the tables they were made from."""
+    packed neighbour lists of every row tile, with the windows they were made from.  Every pass reads the tables anew: the
+    entries are fetched, and the windows compared, by a launch in front of it (``gm_lattice_plan_refresh``), so a plan cannot be
+    out of date."""
 
     first: Tensor  # (row tiles + 1,) int32: first record of a row tile
-    records: Tensor  # uint8
-    layout: tuple  # descriptor rows, lattice size and halo it was made for
-    sources: tuple  # (tensor, write counter) of win_cnt, win_lo, win_off, entries
-
-    def serves(self, layout: tuple, *tables: Tensor) -> bool:
-        """Whether these are the tables the plan was made from, unwritten since."""
-        return self.layout == layout and all(a is b and b._version == version for (a, version), b in zip(self.sources, tables))
+    records: Tensor  # (records, bytes of one) uint8
+    layout: tuple  # record format, descriptor rows, heads, lattice size, halo and orders it was made for
 
 
-def tensor_core_plan(desc_rows: tuple[tuple[int, int, int, int, int], ...], heads: int, rows: int, nlon: int, halo: int, orders: int, win_cnt: Tensor,
-                     win_lo: Tensor, win_off: Tensor, entries: Tensor, mode: int) -> TensorCorePlan | None:
-    """The plan of one pass (0 forward, 1 target-major, 2 source-major, on the transposed tables); ``None`` where the
-    tensor-core kernels do not serve the layout."""
-    tables = (win_cnt, win_lo, win_off, entries)
-    if not entries.is_cuda or entries.shape[0] == 0 or entries.shape[1] != 8 or 2 * halo + 1 > 33 or [r[0] for r in desc_rows if r[0]] != list(range(1, orders + 1)):
-        return None
-    if not tensor_core_layout_supported(desc_rows) or any(t.is_inference() for t in tables):
-        return None
-    flat = [x for row in desc_rows for x in row]
-    desc = (ctypes.c_int64 * len(flat))(*flat)
-    width = max(off + heads * a_n * (1 if n == 0 else 2) for n, a_n, off, *_ in desc_rows)
-    size, tiles = ctypes.c_int64(), ctypes.c_int64()
-    sizes = (ctypes.addressof(desc), len(desc_rows), rows, nlon, width, heads, halo, orders, mode)
-    _lib.call("gm_lattice_plan_size", *sizes, ctypes.addressof(size), ctypes.addressof(tiles))
-    device = entries.device
+def _plan_shape(t: LatticeTables, mode: int, desc: Any) -> tuple:
+    width = max(off + t.heads * a_n * (1 if n == 0 else 2) for n, a_n, off, *_ in t.desc_rows)
+    return ctypes.addressof(desc), len(t.desc_rows), t.rows, t.nlon, width, t.heads, t.halo, t.orders, mode
+
+
+def _plan_tables(t: LatticeTables, mode: int) -> tuple:
+    """Windows and entries a pass reads (0 forward, 1 target-major, 2 source-major: the transposed ones)."""
+    return tuple(_lib.ptr(x) for x in ((t.t_win_cnt, t.t_win_lo, t.t_win_off, t.t_entries) if mode == 2 else (t.win_cnt, t.win_lo, t.win_off, t.entries)))
+
+
+def tensor_core_plans(t: LatticeTables) -> tuple[TensorCorePlan | None, ...]:
+    """The plans of the forward, the target-major and the source-major pass; ``None`` where the tensor-core kernels do not
+    serve the layout."""
+    entries = t.entries
+    if not entries.is_cuda or entries.shape[0] == 0 or entries.shape[1] != 8 or 2 * t.halo + 1 > 33 or [r[0] for r in t.desc_rows if r[0]] != list(range(1, t.orders + 1)):
+        return (None, None, None)
+    if not tensor_core_layout_supported(t.desc_rows):
+        return (None, None, None)
+    device, desc, shapes, sizes = entries.device, t.host_descriptor(), [], []
+    for mode in range(3):
+        size, tiles = ctypes.c_int64(), ctypes.c_int64()
+        shapes.append(_plan_shape(t, mode, desc))
+        _lib.call("gm_lattice_plan_size", *shapes[mode], ctypes.addressof(size), ctypes.addressof(tiles))
+        sizes.append(size.value)
     with torch.cuda.device(device):
-        counts = torch.empty(tiles.value, dtype=torch.int32, device=device)
-        common = (*(_lib.ptr(t) for t in tables), *sizes)
-        _lib.call("gm_lattice_plan_build", *common, _lib.ptr(counts), None, None, _lib.stream(device))
-        first = torch.zeros(tiles.value + 1, dtype=torch.int32, device=device)
-        torch.cumsum(counts, 0, dtype=torch.int32, out=first[1:])
-        records = torch.empty(int(first[-1]) * size.value, dtype=torch.uint8, device=device)
-        _lib.call("gm_lattice_plan_build", *common, None, _lib.ptr(first), _lib.ptr(records), _lib.stream(device))
-        torch.cuda.current_stream(device).synchronize()  # like the tables themselves, complete for whichever stream uses it
-    return TensorCorePlan(first, records, (desc_rows, heads, rows, nlon, halo, orders), tuple((t, t._version) for t in tables))
+        first = torch.zeros((3, tiles.value + 1), dtype=torch.int32, device=device)
+        counts = torch.empty((3, tiles.value), dtype=torch.int32, device=device)
+        for mode in range(3):
+            _lib.call("gm_lattice_plan_build", *_plan_tables(t, mode), *shapes[mode], _lib.ptr(counts[mode]), None, None, _lib.stream(device))
+        torch.cumsum(counts, 1, dtype=torch.int32, out=first[:, 1:])
+        plans = []
+        for mode, total in enumerate(first[:, -1].tolist()):
+            records = torch.empty((total, sizes[mode]), dtype=torch.uint8, device=device)
+            _lib.call("gm_lattice_plan_build", *_plan_tables(t, mode), *shapes[mode], None, _lib.ptr(first[mode]), _lib.ptr(records), _lib.stream(device))
+            plans.append(TensorCorePlan(first[mode], records, t.plan_layout()))
+        torch.cuda.current_stream(device).synchronize()  # like the tables themselves, complete for whichever stream uses them
+    return tuple(plans)
+
+
+def _refreshed_plan(t: LatticeTables, mode: int, desc: Any, batch: int) -> tuple[int | None, Tensor | None]:
+    """First records (address) and records of a pass's plan with the entries the tables hold now, on the current stream;
+    ``None`` without a plan for this layout, or where the pass is too small for one (the kernels then work it out)."""
+    plan = t.tc_plans[mode]
+    if batch * t.rows * t.nlon * t.heads < PLANNED_FROM or plan is None or plan.layout != t.plan_layout() or plan.records.device != t.entries.device:
+        return None, None
+    records = torch.empty_like(plan.records)
+    entries = (t.t_entries if mode == 2 else t.entries).shape[0]
+    _lib.call("gm_lattice_plan_refresh", *_plan_tables(t, mode), *_plan_shape(t, mode, desc), entries, _lib.ptr(plan.records), records.shape[0],
+              _lib.ptr(records), _lib.stream(records.device))
+    return _lib.ptr(plan.first), records
 
 
 @dataclass(frozen=True)
@@ -211,13 +241,9 @@ class LatticeTables:
     # the head layout
     tc_plans: tuple[TensorCorePlan | None, ...] = (None, None, None)
 
-    def plan_pointers(self, mode: int) -> tuple[int | None, int | None]:
-        """Addresses of the parts of a pass's plan for these tables; ``(None, None)`` without one (the kernels then work it out)."""
-        plan = self.tc_plans[mode]
-        tables = (self.t_win_cnt, self.t_win_lo, self.t_win_off, self.t_entries) if mode == 2 else (self.win_cnt, self.win_lo, self.win_off, self.entries)
-        if plan is None or not plan.serves((self.desc_rows, self.heads, self.rows, self.nlon, self.halo, self.orders), *tables):
-            return None, None
-        return _lib.ptr(plan.first), _lib.ptr(plan.records)
+    def plan_layout(self) -> tuple:
+        """What a plan depends on besides the windows."""
+        return PLAN_FORMAT, self.desc_rows, self.heads, self.rows, self.nlon, self.halo, self.orders
 
     def host_descriptor(self) -> Any:
         flat = [x for row in self.desc_rows for x in row]
@@ -303,12 +329,13 @@ def window_is_hard(geometry: Any, e0: Tensor, o0: Tensor, e1: Tensor) -> bool:
 
 
 def build_lattice_tables(geometry: Any, rows: int, nlon: int, desc_rows: tuple[tuple[int, int, int, int, int], ...], heads: int,
-                         scale: float) -> LatticeTables:
+                         scale: float, plans: bool = True) -> LatticeTables:
     """Collapse per-edge tables (``transport``, ``bias``, ``inside``, ``row_ptr``, ``source`` of a
     :class:`gm_attention_b200.nn.fused_attention.Geometry` or :class:`AttentionTables`) of a
     ``rows x nlon`` lattice into compact ones, reading the edges of the targets in column 0.
     Raises ``ValueError`` when a neighbourhood is not a cyclic run of longitudes per source row
-    (the lattice / frames are then not longitude-symmetric: use the general kernels)."""
+    (the lattice / frames are then not longitude-symmetric: use the general kernels).
+    ``plans=False`` leaves out the tensor-core kernels' plans: for tables that no bf16 attention reads."""
     import numpy as np
 
     device = geometry.row_ptr.device
@@ -416,9 +443,9 @@ def build_lattice_tables(geometry: Any, rows: int, nlon: int, desc_rows: tuple[t
         tc = (dev(tc_e), dev(tc_o), dev(t_tc_e), dev(t_tc_o))
     desc_rows = tuple(tuple(int(x) for x in r) for r in desc_rows)
     forward, transposed = (dev(win_cnt), dev(win_lo), dev(win_off), dev(entries)), (dev(t_cnt), dev(t_lo), dev(t_off), dev(t_entries))
-    plans = tuple(tensor_core_plan(desc_rows, heads, rows, nlon, halo, norders, *(transposed if mode == 2 else forward), mode) for mode in range(3))
-    return LatticeTables(rows, nlon, halo, stride, norders, *forward, dev(row_order), *transposed, dev(t_row_order), desc_rows,
-                         heads, float(scale), int(geometry.source.shape[0]), *tc, dev(entry_edge.astype(np.int64)), dev(t_entry), plans)
+    tables = LatticeTables(rows, nlon, halo, stride, norders, *forward, dev(row_order), *transposed, dev(t_row_order), desc_rows,
+                         heads, float(scale), int(geometry.source.shape[0]), *tc, dev(entry_edge.astype(np.int64)), dev(t_entry))
+    return replace(tables, tc_plans=tensor_core_plans(tables)) if plans else tables
 
 
 def _check_lattice(q: Tensor, k: Tensor, v: Tensor, t: LatticeTables) -> tuple[torch.device, int]:
@@ -497,7 +524,8 @@ def lattice_attention_forward(q: Tensor, k: Tensor, v: Tensor, t: LatticeTables,
         if four:
             _lib.call("gm_lattice_attention_forward_tc4", *common, _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
         elif tensor_cores:
-            _lib.call("gm_lattice_attention_forward_planned", *common, *t.plan_pointers(0), _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
+            first, records = _refreshed_plan(t, 0, desc, batch)
+            _lib.call("gm_lattice_attention_forward_planned", *common, first, _lib.ptr(records), _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
         else:
             _lib.call("gm_lattice_attention_forward", *common, _lib.dtype_code(q.dtype), _lib.ptr(out), _lib.ptr(lse), _lib.stream(device))
     return out, lse
@@ -542,8 +570,10 @@ def lattice_attention_backward(dout: Tensor, q: Tensor, k: Tensor, v: Tensor, ou
         if four:
             _lib.call("gm_lattice_attention_backward_tc4_passes", *common, *outputs[:4], int(passes), outputs[4])
         elif tensor_cores:
-            _lib.call("gm_lattice_attention_backward_planned", *common, *outputs[:4], int(passes), *t.plan_pointers(1), *t.plan_pointers(2),
-                      outputs[4])
+            first, records = _refreshed_plan(t, 1, desc, batch) if passes & 2 else (None, None)
+            t_first, t_records = _refreshed_plan(t, 2, desc, batch) if passes & 4 else (None, None)
+            _lib.call("gm_lattice_attention_backward_planned", *common, *outputs[:4], int(passes), first, _lib.ptr(records), t_first,
+                      _lib.ptr(t_records), outputs[4])
         else:
             _lib.call("gm_lattice_attention_backward", *common, _lib.dtype_code(q.dtype), *outputs)
     return dq, dk, dv

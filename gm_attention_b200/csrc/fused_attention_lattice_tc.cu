@@ -34,17 +34,18 @@
 // row); it walks over (sample, head) pairs with one list of positions and one set of table entries.  The next pair's rows are
 // under way (cp.async, both fields of a position in one shared-memory row whose pitch is an odd multiple of 16 bytes: no
 // bank conflicts) while this pair's results are written.  Neighbourhoods that outgrow shared memory -- the polar rows' -- come
-// in chunks.  Lists and entries depend on the tables alone: gm_lattice_plan_build works them out once per table and a CTA
-// copies them; without a plan each CTA works them out itself (16 longitudes x 4 rows, 128 x 256, batch 4: 2 361 against
-// 1 757 us for the three passes).  Tensor-core instruction: mma.sync m16n8k16 (bf16 inputs, fp32 accumulate).
+// in chunks.  The lists depend on the windows alone: gm_lattice_plan_build works them out once per table, gm_lattice_plan_refresh
+// adds the entries in front of every pass, and a CTA copies both; a row tile whose windows are no longer the plan's, and every CTA
+// without a plan, works them out itself (128 x 256, batch 4, 8 x (m <= 3): 2 050 against 1 731 us for the three passes).
+// Tensor-core instruction: mma.sync m16n8k16 (bf16 inputs, fp32 accumulate).
 //
 // What it measured against the kernel before it (one row of 32 longitudes and one (sample, head) per CTA, a step per
 // neighbour row, TMA staging), us forward / pass T / pass S: 128 x 256, batch 4, 4 heads of 8 x (m <= 3): 603 / 904 / 995 ->
-// 427 / 568 / 658; 256 x 512, batch 8, 4 heads of 16 x (m <= 2): 3 670 / 4 896 / 6 643 -> 3 422 / 4 578 / 6 045; heads that
+// 436 / 595 / 700; 256 x 512, batch 8, 4 heads of 16 x (m <= 2): 3 670 / 4 896 / 6 643 -> 3 370 / 4 609 / 6 152; heads that
 // are not 16 copies wide, batch 1 to 8: 1.2 to 4 times faster.  What bounds it: of the last forward 2.1 ms are the steps
 // (shared-memory bandwidth: ten ldmatrix.x4 and the entries, about 100 of 114 cycles a step), 1.4 ms the staging and the
 // per-pair prologue and epilogue, which overlap only across the SM's two CTAs.  16 longitudes per CTA pay in the forward
-// (3 998 -> 3 422); passes T and S want 168 registers a thread, so three CTAs of 4 warps.
+// (3 998 -> 3 422 us at first); passes T and S want 168 registers a thread, so three CTAs of 4 warps.
 //
 // Backward, two deterministic passes (no atomics):
 //   pass T: owners = targets.  Delta = <dO, O> per (target, head) from the owners' own rows (written out for pass S);
@@ -53,6 +54,7 @@
 //   pass S: owners = SOURCES, neighbours = the targets that see them (transposed tables, their lse / Delta
 //           staged with them).  Same Gram blocks with the roles swapped, then (ds o conj tau) Q -> dk and
 //           (p o conj tau) dO -> dv.
+#include <algorithm>
 #include <cmath>
 
 #include "common.cuh"
@@ -94,6 +96,7 @@ struct TcArgs {
   PkCaps caps;                                     // what shared memory holds (a chunk)
   const int* plan_first;                           // with a plan: (row tiles + 1) first record of a row tile, and the records
   const unsigned char* records;
+  int64_t record_bytes;
   int n_bh, heavy_bh, light_bh;                    // (sample, head) pairs: all, and per CTA of a polar / any other row tile
   int heavy_tiles, heavy_ctas;                     // row tiles next to the poles, and the CTAs (the first of the grid) that take them
   float scale;
@@ -364,7 +367,6 @@ struct PkCursor {
 };
 struct PkWindows {  // the tables a tile's neighbourhood is read from
   const int *win_cnt, *win_lo, *win_off;
-  const float* entries;  // (n_entries, 8)
   int rows, nlon, W;
 };
 struct PkTile {  // a tile's neighbour rows, in shared memory
@@ -428,11 +430,11 @@ __device__ __forceinline__ void pk_open_tile(const PkWindows& t, int r0, PkTile&
 // One chunk: as many neighbour positions as `caps` allows, from the cursor on (which advances).  Every warp works the chunk
 // out for itself, lane p looking after the p-th segment; chunk boundaries depend on the tables alone, not on which rows are
 // asked for.  Written: the staged rows' nodes through put_node(row, neighbour row, offset from the tile's first column), the
-// entry pairs (phase, stride caps.entries; bias), and this warp's list of packed positions if it wants one.  `write` false:
-// nothing, the chunk is only measured.
-template <int NCF, int WARPS, typename PutNode>
-__device__ __forceinline__ PkChunk pk_build(const PkWindows& t, const PkTile& tile, PkCursor& cur, PkCaps caps, int pitch16, bool write, bool wants,
-                                            float4* phase, float2* bias, unsigned* list, const PutNode& put_node) {
+// entry pairs (x, x - 1) through put_pair(place, index of entry x, index of entry x - 1), -1 outside the window, and this warp's
+// list of packed positions if it wants one.  `write` false: nothing, the chunk is only measured.
+template <int WARPS, typename PutNode, typename PutPair>
+__device__ __forceinline__ PkChunk pk_build(const PkTile& tile, PkCursor& cur, PkCaps caps, int pitch16, bool write, bool wants, unsigned* list,
+                                            const PutNode& put_node, const PutPair& put_pair) {
   constexpr int TLON = 8 * (WARPS / PK_ROWS);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, my_row = warp & (PK_ROWS - 1), l0 = 8 * (warp / PK_ROWS);
   const int R = caps.rows, E = caps.entries, n_seg = tile.n_seg;
@@ -494,24 +496,8 @@ __device__ __forceinline__ PkChunk pk_build(const PkWindows& t, const PkTile& ti
         for (int x = lane; x < n; x += 32) put_node(base + x, j, u + x);
       if (WARPS == PK_ROWS || (p & 1) == warp / PK_ROWS)
         for (int x = lane; x < pxn; x += 32) {
-          float e0[8], e1[8];
           const int at = px + x - wlo;
-#pragma unroll
-          for (int z = 0; z < 2; ++z) {
-            float* e = z ? e1 : e0;
-            const bool ok = at - z >= 0 && at - z < wcnt;
-            const float4* src = reinterpret_cast<const float4*>(t.entries + (size_t)(woff + (ok ? at - z : 0)) * 8);
-            const float4 v0 = __ldg(src);
-            e[0] = v0.x; e[1] = v0.y; e[2] = v0.z; e[3] = v0.w;
-            if constexpr (NCF >= 2) {
-              const float4 v1 = __ldg(src + 1);
-              e[4] = v1.x; e[5] = v1.y; e[6] = v1.z; e[7] = v1.w;
-            }
-            e[2 * NCF] = ok ? TC_LOG2E * e[2 * NCF] : -INFINITY;
-          }
-#pragma unroll
-          for (int f = 0; f < NCF; ++f) phase[f * E + pe + x] = make_float4(e0[2 * f], e1[2 * f], -e0[2 * f + 1], -e1[2 * f + 1]);
-          bias[pe + x] = make_float2(e0[2 * NCF], e1[2 * NCF]);
+          put_pair(pe + x, at >= 0 && at < wcnt ? woff + at : -1, at >= 1 && at <= wcnt ? woff + at - 1 : -1);
         }
       for (int x = lane; x < ln; x += 32)
         list[placed + x] = (unsigned)((base + lu + x - u) * pitch16) | (unsigned)(pe + lu + x - l0 - px) << 16;
@@ -531,33 +517,69 @@ __device__ __forceinline__ PkChunk pk_build(const PkWindows& t, const PkTile& ti
   return chunk;
 }
 
-// ---- plans: what every longitude tile of a row tile has in common, worked out once per table
-constexpr int PK_HEADER = 16;  // ints at the start of a chunk's record: staged rows, entry pairs, then every warp's steps
-// A record: header, staged rows (rows x 2 ints: first node of the neighbour row, longitude offset), entry pairs as in shared
-// memory, lists (warp x rows)
+// The entry pair at place x: phase (stride E) x (cos x, cos x - 1, -sin x, -sin x - 1), bias x (bias x, bias x - 1) times log2 e,
+// from entries i0 and i1 of the table; -1: outside the window, no weight.
 template <int NCF>
-__host__ __device__ inline int pk_record_bytes(PkCaps caps, int warps) {
-  return 4 * PK_HEADER + 8 * caps.rows + caps.entries * (16 * NCF + 8) + 4 * warps * caps.rows;
-}
-struct PkRecord {
-  const int* header;
-  const int2* nodes;
-  const float4* phase;
-  const float2* bias;
-  const unsigned* list;
-};
-template <int NCF>
-__device__ __forceinline__ PkRecord pk_record(const unsigned char* plan, int64_t index, PkCaps caps, int warps) {
-  const unsigned char* p = plan + index * pk_record_bytes<NCF>(caps, warps);
-  const unsigned char* phase = p + 4 * PK_HEADER + 8 * caps.rows;
-  const unsigned char* bias = phase + (size_t)16 * NCF * caps.entries;
-  return PkRecord{reinterpret_cast<const int*>(p), reinterpret_cast<const int2*>(p + 4 * PK_HEADER), reinterpret_cast<const float4*>(phase),
-                  reinterpret_cast<const float2*>(bias), reinterpret_cast<const unsigned*>(bias + (size_t)8 * caps.entries)};
+__device__ __forceinline__ void pk_put_entries(const float* entries, int i0, int i1, float4* phase, float2* bias, int E, int x) {
+  float e0[8], e1[8];
+#pragma unroll
+  for (int z = 0; z < 2; ++z) {
+    float* e = z ? e1 : e0;
+    const int i = z ? i1 : i0;
+    const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4* src = reinterpret_cast<const float4*>(entries + (size_t)(i < 0 ? 0 : i) * 8);
+    const float4 v0 = i < 0 ? none : __ldg(src);
+    e[0] = v0.x; e[1] = v0.y; e[2] = v0.z; e[3] = v0.w;
+    if constexpr (NCF >= 2) {
+      const float4 v1 = i < 0 ? none : __ldg(src + 1);
+      e[4] = v1.x; e[5] = v1.y; e[6] = v1.z; e[7] = v1.w;
+    }
+    e[2 * NCF] = i < 0 ? -INFINITY : TC_LOG2E * e[2 * NCF];
+  }
+#pragma unroll
+  for (int f = 0; f < NCF; ++f) phase[f * E + x] = make_float4(e0[2 * f], e1[2 * f], -e0[2 * f + 1], -e1[2 * f + 1]);
+  bias[x] = make_float2(e0[2 * NCF], e1[2 * NCF]);
 }
 
-// A CTA per row tile.  records null: counts[tile] = its chunks; else its chunks' records from first[tile] on.
+// ---- plans: what every longitude tile of a row tile has in common.  The packed lists follow from the windows and are worked out
+// once per table; the entries are read in every launch (lattice_plan_refresh_kernel).
+constexpr int PK_HEADER = 16;  // ints at the start of a chunk's record
+enum { PK_HAS_ROWS = 0, PK_HAS_PAIRS = 1, PK_HAS_STEPS = 2, PK_ROW_TILE = 14, PK_READY = 15 };  // staged rows, entry pairs, every warp's steps; its row tile; refreshed
+constexpr int pk_window_words(int W) { return 3 * PK_ROWS * (2 * W + 1); }  // count, first offset and first entry of a row tile's windows
+// A record: header, staged rows (rows x 2 ints: first node of the neighbour row, longitude offset), entry pairs as in shared
+// memory (before it is refreshed the pairs' indices are in the biases' place), lists (warp x rows), the windows it was made from
+inline int pk_record_bytes(PkCaps caps, int warps, int W, int ncf) {
+  return 4 * PK_HEADER + 8 * caps.rows + caps.entries * (16 * ncf + 8) + 4 * warps * caps.rows + 4 * pk_window_words(W);
+}
+struct PkRecord {
+  int* header;
+  int2* nodes;
+  float4* phase;
+  float2* bias;
+  unsigned* list;
+  __device__ __forceinline__ int2* pairs() const { return reinterpret_cast<int2*>(bias); }
+  __device__ __forceinline__ int* windows(PkCaps caps, int warps) const { return reinterpret_cast<int*>(list + warps * caps.rows); }
+};
+// bytes: of a record
+template <int NCF>
+__device__ __forceinline__ PkRecord pk_record(const unsigned char* plan, int64_t index, int64_t bytes, PkCaps caps) {
+  unsigned char* p = const_cast<unsigned char*>(plan) + index * bytes;
+  unsigned char* phase = p + 4 * PK_HEADER + 8 * caps.rows;
+  unsigned char* bias = phase + (size_t)16 * NCF * caps.entries;
+  return PkRecord{reinterpret_cast<int*>(p), reinterpret_cast<int2*>(p + 4 * PK_HEADER), reinterpret_cast<float4*>(phase), reinterpret_cast<float2*>(bias),
+                  reinterpret_cast<unsigned*>(bias + (size_t)8 * caps.entries)};
+}
+// Word x of the windows of a row tile (rows beyond the lattice's last: 0)
+__device__ __forceinline__ int pk_window_word(const PkWindows& t, int row_tile, int x) {
+  const int span = 2 * t.W + 1, kind = x / (PK_ROWS * span), at = row_tile * PK_ROWS * span + x - kind * PK_ROWS * span;
+  if (at >= t.rows * span) return 0;
+  return (kind == 0 ? t.win_cnt : kind == 1 ? t.win_lo : t.win_off)[at];
+}
+
+// A CTA per row tile.  records null: counts[tile] = its chunks; else its chunks' records from first[tile] on, not refreshed.
 template <int NCF, int WARPS>
-__global__ void __launch_bounds__(32 * WARPS) lattice_plan_kernel(PkWindows t, PkCaps caps, int pitch16, int* counts, const int* first, unsigned char* records) {
+__global__ void __launch_bounds__(32 * WARPS) lattice_plan_kernel(PkWindows t, PkCaps caps, int pitch16, int bytes, int* counts, const int* first,
+                                                                  unsigned char* records) {
   __shared__ PkTile tile;
   const int r0 = blockIdx.x * PK_ROWS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, row = r0 + (warp & (PK_ROWS - 1));
   pk_open_tile<WARPS>(t, r0, tile);
@@ -565,32 +587,60 @@ __global__ void __launch_bounds__(32 * WARPS) lattice_plan_kernel(PkWindows t, P
   int n = 0;
   do {
     PkRecord rec{};
-    if (records) rec = pk_record<NCF>(records, first[blockIdx.x] + n, caps, WARPS);
-    int2* nodes = const_cast<int2*>(rec.nodes);
-    float4* phase = const_cast<float4*>(rec.phase);
-    float2* bias = const_cast<float2*>(rec.bias);
-    const PkChunk chunk = pk_build<NCF, WARPS>(t, tile, cur, caps, pitch16, records != nullptr, row < t.rows, phase, bias,
-                                               const_cast<unsigned*>(rec.list) + (records ? warp * caps.rows : 0),
-                                               [&](int r, int j, int u) { nodes[r] = make_int2(j * t.nlon, tc_wrap(u, t.nlon)); });
+    if (records) rec = pk_record<NCF>(records, first[blockIdx.x] + n, bytes, caps);
+    const PkChunk chunk = pk_build<WARPS>(tile, cur, caps, pitch16, records != nullptr, row < t.rows, rec.list + (records ? warp * caps.rows : 0),
+                                          [&](int r, int j, int u) { rec.nodes[r] = make_int2(j * t.nlon, tc_wrap(u, t.nlon)); },
+                                          [&](int x, int i0, int i1) { rec.pairs()[x] = make_int2(i0, i1); });
     if (records) {
-      int* header = const_cast<int*>(rec.header);
       if (threadIdx.x == 0) {
-        header[0] = chunk.rows;
-        header[1] = chunk.entries;
+        rec.header[PK_HAS_ROWS] = chunk.rows;
+        rec.header[PK_HAS_PAIRS] = chunk.entries;
+        rec.header[PK_ROW_TILE] = blockIdx.x;
+        rec.header[PK_READY] = 0;
       }
-      if (lane == 0) header[2 + warp] = chunk.steps;
-      if (threadIdx.x < PK_DUMMY) {
-        bias[threadIdx.x] = make_float2(-INFINITY, -INFINITY);
-        for (int f = 0; f < NCF; ++f) phase[f * caps.entries + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
-      }
+      if (lane == 0) rec.header[PK_HAS_STEPS + warp] = chunk.steps;
+      if (threadIdx.x < PK_DUMMY) rec.pairs()[threadIdx.x] = make_int2(-1, -1);
+      for (int x = threadIdx.x; x < pk_window_words(t.W); x += 32 * WARPS) rec.windows(caps, WARPS)[x] = pk_window_word(t, blockIdx.x, x);
     }
     ++n;
   } while (cur.seg < tile.n_seg);
   if (!records && threadIdx.x == 0) counts[blockIdx.x] = n;
 }
 
+// A CTA per record: the plan's record with the entries the table holds now; an empty one that is not ready where the row tile's
+// windows are no longer those it was made from.  Runs in front of every pass that has a plan: a pass that kept a copy of the
+// entries from call to call would not see a write into the table.
+// Latency bound, so all that can is loaded at once: the entries do not wait for the windows (their indices are only kept below
+// the table's end).
+constexpr int PK_REFRESH_THREADS = 512;
+template <int NCF>
+__global__ void __launch_bounds__(PK_REFRESH_THREADS) lattice_plan_refresh_kernel(PkWindows t, const float* entries, int64_t n_entries, PkCaps caps, int warps,
+                                                                                  int bytes, const unsigned char* plan, unsigned char* records) {
+  const PkRecord from = pk_record<NCF>(plan, blockIdx.x, bytes, caps), to = pk_record<NCF>(records, blockIdx.x, bytes, caps);
+  const int x0 = threadIdx.x, row_tile = __ldg(from.header + PK_ROW_TILE), n_pairs = __ldg(from.header + PK_HAS_PAIRS);
+  const int2 first_pair = x0 < caps.entries ? __ldg(from.pairs() + x0) : make_int2(-1, -1);  // beyond n_pairs: whatever was there, not used
+  uint4* const lists_to = reinterpret_cast<uint4*>(to.list);
+  const uint4* const lists_from = reinterpret_cast<const uint4*>(from.list);
+  for (int x = x0; x < caps.rows; x += PK_REFRESH_THREADS) to.nodes[x] = __ldg(from.nodes + x);
+  for (int x = x0; x < warps * caps.rows / 4; x += PK_REFRESH_THREADS) lists_to[x] = __ldg(lists_from + x);
+  int same = 1;
+  for (int x = x0; x < pk_window_words(t.W); x += PK_REFRESH_THREADS) same &= __ldg(from.windows(caps, warps) + x) == pk_window_word(t, row_tile, x);
+  for (int x = x0; x < n_pairs; x += PK_REFRESH_THREADS) {
+    const int2 at = x == x0 ? first_pair : __ldg(from.pairs() + x);
+    pk_put_entries<NCF>(entries, at.x < n_entries ? at.x : -1, at.y < n_entries ? at.y : -1, to.phase, to.bias, caps.entries, x);
+  }
+  same = __syncthreads_and(same);
+  if (x0 < PK_HEADER) to.header[x0] = x0 == PK_READY ? same : same ? __ldg(from.header + x0) : 0;
+}
+
+template <int NCF>
+__device__ __forceinline__ bool pk_ready(const TcArgs& a, int row_tile) {
+  return pk_record<NCF>(a.records, a.plan_first[row_tile], a.record_bytes, a.caps).header[PK_READY] != 0;
+}
+
+// One tile of owners: PK_ROWS rows x TLON longitudes, (sample, head) pairs [bh, bh_end)
 template <int KS0, int NCF, int KSC, int MODE, int WARPS, bool PLANNED>
-__global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_kernel(const __grid_constant__ TcArgs a) {
+__device__ __forceinline__ void pk_cta(const TcArgs& a, int row_tile, int lon_tile, int bh, int bh_end) {
   using L = PkLayout<KS0, NCF, KSC>;
   constexpr int THREADS = 32 * WARPS, TLON = 8 * (WARPS / PK_ROWS);
   constexpr int KQ = L::KQ, NCK = NCF * KSC, PITCH = L::PITCH, FIELD = L::FIELD;
@@ -607,28 +657,10 @@ __global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_ker
   int* const node_s = reinterpret_cast<int*>(list_s + WARPS * LIST);                    // R staged rows: node within the sample
 
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3;
-  // ---- which tile, which (sample, head) pairs: the first heavy_ctas CTAs take the row tiles next to the poles
-  const int lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
-  int row_tile, lon_tile, bh, bh_end;
-  {
-    int x = blockIdx.x;
-    if (x < a.heavy_ctas) {
-      lon_tile = x % lon_tiles;
-      x /= lon_tiles;
-      const int chunks = (a.n_bh + a.heavy_bh - 1) / a.heavy_bh;
-      bh = (x % chunks) * a.heavy_bh;
-      bh_end = min(bh + a.heavy_bh, a.n_bh);
-      row_tile = x / chunks;
-    } else {
-      x -= a.heavy_ctas;
-      lon_tile = x % lon_tiles;
-      x /= lon_tiles;
-      const int light = row_tiles - a.heavy_tiles;
-      row_tile = a.heavy_tiles + x % light;
-      bh = (x / light) * a.light_bh;
-      bh_end = min(bh + a.light_bh, a.n_bh);
-    }
-    row_tile = (int)from_both_ends(row_tile, row_tiles);
+  int chunk = 0, n_chunks = 1;
+  if constexpr (PLANNED) {
+    chunk = a.plan_first[row_tile];
+    n_chunks = a.plan_first[row_tile + 1] - chunk;
   }
   const int r0 = row_tile * PK_ROWS, c0 = lon_tile * TLON;
   const int my_row = warp & (PK_ROWS - 1), row = r0 + my_row, l0 = 8 * (warp / PK_ROWS);
@@ -660,25 +692,18 @@ __global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_ker
   const bool active = (member_s >> my_row & 1) && row < a.rows && c0 + l0 < a.nlon;  // this warp has owners to write
 
   // ---- the chunks of the tile's neighbourhood: from the plan, or worked out here
-  const PkWindows windows{a.win_cnt, a.win_lo, a.win_off, a.entries, a.rows, a.nlon, a.W};
   PkCursor cur{0, 0};
-  int chunk = 0, n_chunks = 1;
-  if constexpr (PLANNED) {
-    chunk = a.plan_first[row_tile];
-    n_chunks = a.plan_first[row_tile + 1] - chunk;
-  } else {
-    pk_open_tile<WARPS>(windows, r0, tile_desc);
-  }
+  if constexpr (!PLANNED) pk_open_tile<WARPS>(PkWindows{a.win_cnt, a.win_lo, a.win_off, a.rows, a.nlon, a.W}, r0, tile_desc);
   const int first_chunk = chunk;
   int n_rows = 0, n_steps = 0;
   // the next chunk (the first one again after the last): staged rows' nodes, entry pairs, lists; its copies join the fields'
   auto load_chunk = [&](bool restart) {
     if constexpr (PLANNED) {
       if (restart) chunk = first_chunk;
-      const PkRecord rec = pk_record<NCF>(a.records, chunk, a.caps, WARPS);
-      n_rows = rec.header[0];
-      const int n_entries = rec.header[1];
-      n_steps = active ? rec.header[2 + warp] : 0;
+      const PkRecord rec = pk_record<NCF>(a.records, chunk, a.record_bytes, a.caps);
+      n_rows = rec.header[PK_HAS_ROWS];
+      const int n_entries = rec.header[PK_HAS_PAIRS];
+      n_steps = active ? rec.header[PK_HAS_STEPS + warp] : 0;
       ++chunk;
       for (int r = threadIdx.x; r < n_rows; r += THREADS) {
         const int2 at = rec.nodes[r];
@@ -693,8 +718,9 @@ __global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_ker
       for (int x = lane; x < 4 * n_steps; x += 32) cp_async16(list_s + warp * LIST + 4 * x, rec.list + warp * LIST + 4 * x, 16);
     } else {
       if (restart) cur = PkCursor{0, 0};
-      const PkChunk built = pk_build<NCF, WARPS>(windows, tile_desc, cur, a.caps, PITCH / 16, true, active, reinterpret_cast<float4*>(phase_s), bias_s,
-                                                 list_s + warp * LIST, [&](int r, int j, int u) { node_s[r] = j * a.nlon + tc_wrap(c0 + u, a.nlon); });
+      const PkChunk built = pk_build<WARPS>(tile_desc, cur, a.caps, PITCH / 16, true, active, list_s + warp * LIST,
+                                            [&](int r, int j, int u) { node_s[r] = j * a.nlon + tc_wrap(c0 + u, a.nlon); },
+                                            [&](int x, int i0, int i1) { pk_put_entries<NCF>(a.entries, i0, i1, reinterpret_cast<float4*>(phase_s), bias_s, E, x); });
       n_rows = built.rows;
       n_steps = built.steps;
     }
@@ -1025,6 +1051,50 @@ __global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_ker
   }
 }
 
+template <int KS0, int NCF, int KSC, int MODE, int WARPS, bool PLANNED>
+__global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_kernel(const __grid_constant__ TcArgs a) {
+  constexpr int TLON = 8 * (WARPS / PK_ROWS);
+  // which tile, which (sample, head) pairs: the first heavy_ctas CTAs take the row tiles next to the poles
+  const int lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
+  int row_tile, lon_tile, bh, bh_end, x = blockIdx.x;
+  if (x < a.heavy_ctas) {
+    lon_tile = x % lon_tiles;
+    x /= lon_tiles;
+    const int chunks = (a.n_bh + a.heavy_bh - 1) / a.heavy_bh;
+    bh = (x % chunks) * a.heavy_bh;
+    bh_end = min(bh + a.heavy_bh, a.n_bh);
+    row_tile = x / chunks;
+  } else {
+    x -= a.heavy_ctas;
+    lon_tile = x % lon_tiles;
+    x /= lon_tiles;
+    const int light = row_tiles - a.heavy_tiles;
+    row_tile = a.heavy_tiles + x % light;
+    bh = (x / light) * a.light_bh;
+    bh_end = min(bh + a.light_bh, a.n_bh);
+  }
+  pk_cta<KS0, NCF, KSC, MODE, WARPS, PLANNED>(a, (int)from_both_ends(row_tile, row_tiles), lon_tile, bh, bh_end);
+}
+
+// The row tiles whose windows are not the ones the plan was made from, behind the planned launch (to which their records were
+// empty: it wrote zeros); none as a rule, which each of a few CTAs finds out for itself.
+template <int KS0, int NCF, int KSC, int MODE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_stale_kernel(const __grid_constant__ TcArgs a) {
+  constexpr int TLON = 8 * (WARPS / PK_ROWS);
+  const int lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
+  int stale = 0;
+  for (int x = threadIdx.x; x < row_tiles; x += 32 * WARPS) stale |= !pk_ready<NCF>(a, x);
+  if (!__syncthreads_or(stale)) return;
+  for (int row_tile = 0; row_tile < row_tiles; ++row_tile) {
+    if (pk_ready<NCF>(a, row_tile)) continue;
+    for (int64_t x = blockIdx.x; x < (int64_t)lon_tiles * a.n_bh; x += gridDim.x) {
+      const int bh = (int)(x / lon_tiles);
+      pk_cta<KS0, NCF, KSC, MODE, WARPS, false>(a, row_tile, (int)(x % lon_tiles), bh, bh + 1);
+      __syncthreads();
+    }
+  }
+}
+
 // Delta[node, h] = <dO, O> over the head's columns
 __global__ void tc_delta_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ out, float* __restrict__ delta,
                                 int64_t n_nodes, int D, int H, TcPlan P) {
@@ -1161,6 +1231,7 @@ int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
   a.units = (2 * a.plan.a0 + NCF * 4 * a.plan.ac) / a.unit;
   a.n_order = n_order_rows;
   const size_t smem = chunk_caps<KS0, NCF, KSC, WARPS>(a.rows, a.nlon, a.W, a.caps);
+  a.record_bytes = pk_record_bytes(a.caps, WARPS, a.W, NCF);
   // Polar rows see whole rings: their tiles start first and hold few (sample, head) pairs each.  Elsewhere a CTA takes as
   // many pairs as leave a few waves of CTAs, up to 16: lists and entries are made once for all of them.
   const int64_t lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
@@ -1183,13 +1254,15 @@ int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
   const int64_t light = light_tiles * ((n_bh + a.light_bh - 1) / a.light_bh);
   GM_REQUIRE(heavy + light < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_attention (tensor cores): %lld tiles exceed a grid", (long long)(heavy + light));
   a.heavy_ctas = (int)heavy;
-  auto go = [&](auto kernel) {
+  auto go = [&](auto kernel, int64_t ctas) {
     const int st = allow_smem(kernel, smem, "gm_lattice_attention (tensor cores)");
     if (st != GM_OK) return st;
-    kernel<<<(unsigned)(heavy + light), 32 * WARPS, smem, stream>>>(a);
+    kernel<<<(unsigned)ctas, 32 * WARPS, smem, stream>>>(a);
     return launch_status("gm_lattice_attention (tensor cores)");
   };
-  return a.records ? go(lattice_packed_kernel<KS0, NCF, KSC, MODE, WARPS, true>) : go(lattice_packed_kernel<KS0, NCF, KSC, MODE, WARPS, false>);
+  if (!a.records) return go(lattice_packed_kernel<KS0, NCF, KSC, MODE, WARPS, false>, heavy + light);
+  const int st = go(lattice_packed_kernel<KS0, NCF, KSC, MODE, WARPS, true>, heavy + light);
+  return st != GM_OK ? st : go(lattice_packed_stale_kernel<KS0, NCF, KSC, MODE, WARPS>, std::min<int64_t>(slots, heavy + light));
 }
 
 // f(KS0, NCF, KSC) as integral constants for the layouts that have kernels
@@ -1252,7 +1325,7 @@ extern "C" int gm_lattice_plan_size(const int64_t* desc_host, int F, int rows, i
     auto size = [&](auto warps) {
       PkCaps caps;
       chunk_caps<ks0.value, ncf.value, ksc.value, warps.value>(rows, nlon, W, caps);
-      *record_bytes = pk_record_bytes<ncf.value>(caps, warps.value);
+      *record_bytes = pk_record_bytes(caps, warps.value, W, ncf.value);
       return (int)GM_OK;
     };
     return mode == TC_FWD ? size(std::integral_constant<int, pk_warps(TC_FWD)>()) : size(std::integral_constant<int, pk_warps(TC_BWD_S)>());
@@ -1269,12 +1342,34 @@ extern "C" int gm_lattice_plan_build(const int* win_cnt, const int* win_lo, cons
     auto build = [&](auto warps) {
       PkCaps caps;
       chunk_caps<ks0.value, ncf.value, ksc.value, warps.value>(rows, nlon, W, caps);
-      const PkWindows t{win_cnt, win_lo, win_off, entries, rows, nlon, W};
+      const PkWindows t{win_cnt, win_lo, win_off, rows, nlon, W};
       lattice_plan_kernel<ncf.value, warps.value><<<(unsigned)((rows + PK_ROWS - 1) / PK_ROWS), 32 * warps.value, 0, (cudaStream_t)stream>>>(
-          t, caps, PkLayout<ks0.value, ncf.value, ksc.value>::PITCH / 16, counts, first, (unsigned char*)records);
+          t, caps, PkLayout<ks0.value, ncf.value, ksc.value>::PITCH / 16, pk_record_bytes(caps, warps.value, W, ncf.value), counts, first, (unsigned char*)records);
       return launch_status("gm_lattice_plan_build");
     };
     return mode == TC_FWD ? build(std::integral_constant<int, pk_warps(TC_FWD)>()) : build(std::integral_constant<int, pk_warps(TC_BWD_S)>());
+  });
+}
+
+extern "C" int gm_lattice_plan_refresh(const int* win_cnt, const int* win_lo, const int* win_off, const float* entries, const int64_t* desc_host, int F,
+                                       int rows, int nlon, int D, int H, int W, int NORD, int mode, int64_t n_entries, const void* plan,
+                                       int64_t n_records, void* records, void* stream) {
+  GM_REQUIRE(win_cnt && win_lo && win_off && entries && plan && records, GM_ERR_ARGUMENT, "gm_lattice_plan_refresh: null pointer");
+  GM_REQUIRE(n_entries >= 1, GM_ERR_ARGUMENT, "gm_lattice_plan_refresh: empty table");
+  GM_REQUIRE(n_records >= 1 && n_records < (1ll << 31) && (reinterpret_cast<uintptr_t>(plan) | reinterpret_cast<uintptr_t>(records)) % 16 == 0, GM_ERR_ARGUMENT,
+             "gm_lattice_plan_refresh: bad records");
+  TcArgs a{};
+  int status = fill_tc_args(a, desc_host, F, rows, nlon, 1, D, H, W, 8, NORD, 1.0);
+  if (status != GM_OK) return status;
+  return for_layout(a.plan, NORD, [&](auto ks0, auto ncf, auto ksc) {
+    auto refresh = [&](auto warps) {
+      PkCaps caps;
+      chunk_caps<ks0.value, ncf.value, ksc.value, warps.value>(rows, nlon, W, caps);
+      lattice_plan_refresh_kernel<ncf.value><<<(unsigned)n_records, PK_REFRESH_THREADS, 0, (cudaStream_t)stream>>>(
+          PkWindows{win_cnt, win_lo, win_off, rows, nlon, W}, entries, n_entries, caps, warps.value, pk_record_bytes(caps, warps.value, W, ncf.value), (const unsigned char*)plan, (unsigned char*)records);
+      return launch_status("gm_lattice_plan_refresh");
+    };
+    return mode == TC_FWD ? refresh(std::integral_constant<int, pk_warps(TC_FWD)>()) : refresh(std::integral_constant<int, pk_warps(TC_BWD_S)>());
   });
 }
 

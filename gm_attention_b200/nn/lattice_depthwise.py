@@ -65,7 +65,7 @@ def conv_tables(geometry: Any, distances: Tensor, weights: Tensor, rows: Sequenc
     a_0 = scalar[0][1] if scalar else 0
     if a_0 % 2:
         raise ValueError("the lattice depthwise kernels pair the scalar channels: their number must be even")
-    lat = build_lattice_tables(geometry, n_rows, nlon, rows, 1, 1.0)
+    lat = build_lattice_tables(geometry, n_rows, nlon, rows, 1, 1.0, plans=False)
     edge = lat.entry_edge
     complex_rows = [r for r in rows if r[0] > 0]
     padded = -(-a_0 // 4) * 4

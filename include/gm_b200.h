@@ -344,20 +344,27 @@ int gm_lattice_attention_backward_tc_passes(const void* dout, const void* q, con
 int gm_lattice_attention_tc_wait_expired(int* expired);
 
 /* Plans of the tensor-core lattice kernels: what every longitude tile of a row tile (four lattice rows) has in common -- the
- * packed list of its neighbour positions and their table entries, in chunks of the kernels' shared memory -- worked out once
- * per (tables, head layout) instead of once per CTA.  gm_lattice_plan_size: bytes of a chunk's record and the number of row
- * tiles.  gm_lattice_plan_build with records == NULL: counts[row tile] = its chunks; with records: fills them, row tile x's
- * from record first[x] on (first: row tiles + 1 running sums).  records starts on a 16-byte boundary.  A plan belongs to the
- * contents of win_cnt / win_lo / win_off / entries it was built from, to the descriptor and to the lattice's size; mode: 0
- * for the forward (whose CTAs are wider), 1 for the target-major pass (the same tables), 2 for the source-major pass (the
- * transposed ones). */
+ * packed list of its neighbour positions and their table entries, in chunks of the kernels' shared memory.  The lists follow
+ * from the windows and are worked out once per (tables, head layout) instead of once per CTA; the entries are fetched for every
+ * pass.
+ *   gm_lattice_plan_size: bytes of a chunk's record and the number of row tiles.
+ *   gm_lattice_plan_build with records == NULL: counts[row tile] = its chunks; with records: fills them, row tile x's from record
+ *     first[x] on (first: row tiles + 1 running sums).
+ *   gm_lattice_plan_refresh: the n_records records at `plan` with the n_entries entries of the table as they are now, to
+ *     `records` (as many bytes), which a pass in the same stream then takes.  A row tile whose windows are no longer those the plan was made from
+ *     is worked out without it, and so is one whose records were not refreshed.
+ * All records start on a 16-byte boundary.  A plan belongs to the descriptor and to the lattice's size; mode: 0 for the forward
+ * (whose CTAs are wider), 1 for the target-major pass (the same tables), 2 for the source-major pass (the transposed ones). */
 int gm_lattice_plan_size(const int64_t* desc_host, int F, int rows, int nlon, int D, int H, int W, int NORD, int mode,
                          int64_t* record_bytes, int64_t* row_tiles);
 int gm_lattice_plan_build(const int* win_cnt, const int* win_lo, const int* win_off, const float* entries, const int64_t* desc_host, int F,
                           int rows, int nlon, int D, int H, int W, int NORD, int mode, int* counts, const int* first, void* records,
                           void* stream);
+int gm_lattice_plan_refresh(const int* win_cnt, const int* win_lo, const int* win_off, const float* entries, const int64_t* desc_host, int F,
+                            int rows, int nlon, int D, int H, int W, int NORD, int mode, int64_t n_entries, const void* plan,
+                            int64_t n_records, void* records, void* stream);
 
-/* gm_lattice_attention_forward_tc / _backward_tc_passes with the plans of modes 0 / 1 and 2
+/* gm_lattice_attention_forward_tc / _backward_tc_passes with the refreshed plans of modes 0 / 1 and 2
  * (plan_records == NULL: without one, bit-identical results). */
 int gm_lattice_attention_forward_planned(const void* q, const void* k, const void* v, const int* win_cnt, const int* win_lo,
                                          const int* win_off, const float* entries, const int* row_order, int n_order_rows,

@@ -387,20 +387,22 @@ PACKED_CASES = [
 
 
 @pytest.mark.parametrize("case", PACKED_CASES)
-def test_packed_tensor_core_kernels(case):
+def test_packed_tensor_core_kernels(case, monkeypatch):
     """The tensor-core kernels with a plan, without one (every CTA packs its own lists) and after the tables were written in
-    place (the plan is theirs no longer), against the oracle on the rounded inputs; bf16 storage: 2e-2 of the magnitude."""
+    place (the entries are read in every launch; windows that are not the plan's are packed anew), against the oracle on the rounded inputs; bf16 storage: 2e-2 of the magnitude."""
     import dataclasses
 
+    from gm_attention_b200 import attention
     from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
 
+    monkeypatch.setattr(attention, "PLANNED_FROM", 0)
     batch = case[6]
     c = make_case(*case[:5], dtype=np.float32, window=case[5])
     rounded = [torch.from_numpy(x).bfloat16() for x in seeded((batch * c.n_nodes, c.width), 63, np.float32, 4)]
     q, k, v, g = (x.float().numpy() for x in rounded)
     Q, K, V, G = (x.cuda() for x in rounded)
     _, lat = tables_for(c)
-    assert all(plan is not None for plan in lat.tc_plans) and all(lat.plan_pointers(mode)[1] for mode in range(3))
+    assert all(plan is not None for plan in lat.tc_plans)
 
     def run(t):
         out, lse = lattice_attention_forward(Q, K, V, t, tensor_cores=True)
@@ -414,7 +416,6 @@ def test_packed_tensor_core_kernels(case):
     for name, a, b in zip(("out", "dq", "dk", "dv"), (planned[0], *planned[2:]), (want, *grads)):
         assert float(np.abs(a.float().cpu().numpy() - b).max()) < 2e-2 * max(1.0, np.abs(b).max()), name
     lat.entries[:, :2 * lat.orders].mul_(-1.0)
-    assert lat.plan_pointers(0) == lat.plan_pointers(1) == (None, None) and lat.plan_pointers(2)[1]
     turned = run(lat)
     assert torch.equal(turned[0], run(dataclasses.replace(lat, tc_plans=(None, None, None)))[0]) and not torch.equal(turned[0], planned[0])
 
@@ -432,3 +433,61 @@ def test_tables_without_a_plan():
     assert turned.tc_plans == (None, None, None)
     got, _ = lattice_attention_forward(q, k, v, turned)
     assert float((got - want).abs().max()) < 1e-5 * max(1.0, float(want.abs().max()))
+
+
+def test_kernels_read_the_tables_in_every_launch(monkeypatch):
+    """Writes into the tables show at once: by a captured graph's replay, past the tensors' write counters, and where they
+    change the windows that the plans were made from (some row tiles, then all); bit for bit as without plans.  Copies keep
+    their plans."""
+    import copy
+    import dataclasses
+
+    from gm_attention_b200 import attention
+    from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
+
+    monkeypatch.setattr(attention, "PLANNED_FROM", 0)
+
+    c = make_case(13, 40, 2.5 * math.pi / 13, {0: 8, 1: 8}, 2, dtype=np.float32)
+    Q, K, V, G = (torch.from_numpy(x).bfloat16().cuda() for x in seeded((c.n_nodes, c.width), 65, np.float32, 4))
+    _, lat = tables_for(c)
+    bare = dataclasses.replace(lat, tc_plans=(None, None, None))
+    out, lse = torch.empty_like(Q), torch.empty((c.n_nodes, c.heads), device="cuda")
+    grads = [torch.empty_like(Q) for _ in range(3)] + [torch.empty_like(lse)]
+
+    def run(t, out, lse, grads):
+        lattice_attention_forward(Q, K, V, t, tensor_cores=True, out=out, lse=lse)
+        lattice_attention_backward(G, Q, K, V, out, lse, t, tensor_cores=True, workspace=tuple(grads))
+
+    run(lat, out, lse, grads)  # loads the kernels before the capture
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        run(lat, out, lse, grads)
+    results = []
+
+    def compare():
+        for x in (out, lse, *grads):
+            x.fill_(float("nan"))
+        graph.replay()
+        other = [torch.empty_like(x) for x in (out, lse, *grads)]
+        run(bare, other[0], other[1], other[2:])
+        eager = [torch.empty_like(x) for x in (out, lse, *grads)]
+        run(copy.deepcopy(lat), eager[0], eager[1], eager[2:])
+        for a, b, x in zip((out, lse, *grads), other, eager):
+            assert torch.equal(a, b) and torch.equal(x, b)
+        results.append([x.clone() for x in (out, *grads[:3])])
+        for earlier in results[:-1]:
+            assert not torch.equal(earlier[0], out)
+
+    assert all(plan.layout == lat.plan_layout() for plan in copy.deepcopy(lat).tc_plans)
+    compare()
+    lat.entries[:, :2].mul_(-1.0)
+    compare()
+    lat.entries.data[:, 2].add_(torch.linspace(0.0, 1.0, lat.entries.shape[0], device="cuda"))
+    lat.t_entries.data[:, :2].mul_(-1.0)
+    compare()
+    assert not torch.equal(results[2][2], results[1][2])  # dk: the transposed entries
+    lat.win_cnt.data[6].clamp_(max=3)  # one row of one tile
+    compare()
+    lat.win_lo.data.add_(1)
+    lat.t_win_cnt.data.clamp_(max=4)
+    compare()
