@@ -89,7 +89,8 @@ struct TcArgs {
   const float* entries;               // (n_entries, 8): (cos, sin) of orders 1..NORD, bias at 2 NORD
   const int* row_order;
   int rows, nlon, D, H, W, NORD;
-  int even;     // every block starts on an even column and has an even width: 4-byte accesses
+  int words;    // rows and owners' / result fields are whole 4-byte words: 4-byte accesses to (even column, next column)
+  int even;     // and every block starts on an even column and has an even width: 4-byte accesses throughout
   int padded;   // blocks narrower than 16 (scalar) / 16 KSC (complex) columns
   int unit, units;  // staging: bytes of one copy (16, 8, 4; 2: element by element), copies per head row and field
   int n_order;      // rows in row_order (all of them: the list is not read)
@@ -665,7 +666,7 @@ __device__ __forceinline__ void pk_cta(const TcArgs& a, int row_tile, int lon_ti
   const int r0 = row_tile * PK_ROWS, c0 = lon_tile * TLON;
   const int my_row = warp & (PK_ROWS - 1), row = r0 + my_row, l0 = 8 * (warp / PK_ROWS);
   const float cscale = a.scale * TC_LOG2E;
-  const bool words = (a.D & 1) == 0;  // 4-byte accesses to (even column, next column) are aligned
+  const bool words = a.words != 0;
   const bool even = a.even != 0;
 
   // ---- setup, once per CTA: which rows are asked for
@@ -1216,10 +1217,12 @@ template <int KS0, int NCF, int KSC, int MODE>
 int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
   constexpr int WARPS = pk_warps(MODE), TLON = 8 * (WARPS / PK_ROWS);
   const void* ptrs[6] = {a.own1, a.own2, a.nb1, a.nb2, a.res1, a.res2};
-  uint64_t all = (uint64_t)a.D * 2 | (uint64_t)a.plan.a0 * 2 | (KS0 ? (uint64_t)a.plan.real_off * 2 : 0);  // in bytes
-  for (int f = 0; f < a.plan.n_cf; ++f) all |= (uint64_t)a.plan.cf_off[f] * 2;
+  uint64_t all = (uint64_t)a.D * 2;  // in bytes
   for (const void* q : ptrs) all |= reinterpret_cast<uintptr_t>(q);
   if (MODE == TC_BWD_T && a.delta_out) all |= reinterpret_cast<uintptr_t>(a.out_fwd);
+  a.words = all % 4 == 0;
+  all |= (uint64_t)a.plan.a0 * 2 | (KS0 ? (uint64_t)a.plan.real_off * 2 : 0);
+  for (int f = 0; f < a.plan.n_cf; ++f) all |= (uint64_t)a.plan.cf_off[f] * 2;
   a.even = all % 4 == 0;
   a.padded = (KS0 && a.plan.a0 != 16) || 2 * a.plan.ac != 16 * KSC;
   // the widest copy that every block of every head is made of: all that is added to the fields' addresses, in bytes

@@ -491,3 +491,36 @@ def test_kernels_read_the_tables_in_every_launch(monkeypatch):
     lat.win_lo.data.add_(1)
     lat.t_win_cnt.data.clamp_(max=4)
     compare()
+
+
+@pytest.mark.parametrize("head", [{0: 8, 1: 8}, {0: 5, 1: 6, 2: 6}])
+def test_fields_on_odd_addresses(head):
+    """bf16 fields that start on a 2-byte boundary only (contiguous views at an odd element offset), each alone and all
+    together: bit for bit the aligned call's results."""
+    from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
+
+    c = make_case(6, 24, 2 * math.pi / 6, head, 2, dtype=np.float32)
+    _, lat = tables_for(c)
+    aligned = [torch.from_numpy(x).bfloat16().cuda() for x in seeded((c.n_nodes, c.width), 66, np.float32, 4)]
+    results = [torch.empty_like(aligned[0]) for _ in range(4)]
+
+    def odd(x):
+        view = torch.empty(x.numel() + 1, dtype=x.dtype, device="cuda")[1:].view(x.shape)
+        view.copy_(x)
+        assert view.data_ptr() % 4 == 2 and view.is_contiguous()
+        return view
+
+    def run(fields, results):
+        q, k, v, g = fields
+        out, dq, dk, dv = results
+        _, lse = lattice_attention_forward(q, k, v, lat, tensor_cores=True, out=out)
+        delta = torch.empty_like(lse)
+        lattice_attention_backward(g, q, k, v, out, lse, lat, tensor_cores=True, workspace=(dq, dk, dv, delta))
+        return [x.clone() for x in (*results, lse, delta)]
+
+    want = run(aligned, results)
+    for moved in [{x} for x in range(8)] + [set(range(8))]:
+        fields = [odd(x) if i in moved else x for i, x in enumerate(aligned)]
+        places = [odd(x) if i + 4 in moved else x for i, x in enumerate(results)]
+        for a, b in zip(run(fields, places), want):
+            assert torch.equal(a, b), moved
