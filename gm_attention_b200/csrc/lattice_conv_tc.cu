@@ -9,8 +9,13 @@
 //               rows m = (s, component of g), columns (r, component of x), contraction over t, 16 tiles per k-step
 //
 // Of the (s, r) pairs of a window of cnt offsets 8 cnt in 8 (7 + cnt), rounded up to 8, are wanted: half at cnt = 8.
-// Precision: field values are bfloat16 as they are and the products accumulate in float32.  The table is float32, so
-// apply writes each of its numbers as a sum of three bfloat16 (8 + 8 + 8 bits: exact) and takes three products.
+// Precision: field values are bfloat16 as they are.  The table is float32, so apply writes each of its numbers as a sum of three
+// bfloat16 (8 + 8 + 8 bits: exact) and takes three products, smallest first.  An mma cuts its sum off instead of rounding it, so
+// no chain is longer than one k-step (8 positions): its sum is added in float32, rounded to nearest.  Root mean square error
+// against float64 of sums of N(0, 1) terms that cancel, one chain through all windows / this way / the FMA kernel's single
+// additions: rings of 512, terms in order of size 9.5e-4 / 4.9e-5 / 1.3e-4, in random order 1.3e-4 / 6.0e-6 / 1.7e-5; 24 x 48, radius
+// 2.5 pi / 24, 6.4e-6 / 1.1e-6 / 3.2e-6 and 2.1e-6 / 4.3e-7 / 1.1e-6.  It costs a fifth of apply's time (256 x 512, radius
+// 2 pi / 256, 64 x (m <= 2): 322 -> 406 us; by the FMA kernel 469).
 //
 // In shared memory a node's 32 columns (64 bytes) sit at [position % 8][position / 8], rows of 80 bytes: a lane reads four
 // channel pairs of one position with one 16-byte load, the lanes of a load on different banks.  The (re, im) words are B
@@ -32,12 +37,15 @@ __device__ __forceinline__ void mma(float (&d)[4], unsigned a0, unsigned a1, uns
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// d += a * b with the addition to d rounded to nearest (the accumulator of a long chain of mma would be cut off every time)
+__device__ __forceinline__ void mma_first(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {  // d = a * b
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+// d += a * b with the addition to d rounded to nearest
 __device__ __forceinline__ void mma_add(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
   float p[4];
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
-               : "=f"(p[0]), "=f"(p[1]), "=f"(p[2]), "=f"(p[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
+  mma_first(p, a[0], a[1], a[2], a[3], b0, b1);
 #pragma unroll
   for (int x = 0; x < 4; ++x) d[x] += p[x];
 }
@@ -385,14 +393,21 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const Conv
           fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
         }
 #pragma unroll
-        for (int s = 0; s < 3; ++s)
+        for (int p = 0; p < 4; ++p) {
+          const uint2* f = ms + p * AP_PAIR + 8 * k;
+          const uint2 l01 = f[2 * AP_SLOTS], l23 = f[2 * AP_SLOTS + 4], m01 = f[AP_SLOTS], m23 = f[AP_SLOTS + 4], h01 = f[0], h23 = f[4];
+          float sum[MINE][4];
 #pragma unroll
-          for (int p = 0; p < 4; ++p) {
-            const uint2* f = ms + p * AP_PAIR + s * AP_SLOTS + 8 * k;
-            const uint2 a01 = f[0], a23 = f[4];
+          for (int i = 0; i < MINE; ++i) mma_first(sum[i], l01.x, l01.y, l23.x, l23.y, fb[i][0][p], fb[i][1][p]);
 #pragma unroll
-            for (int i = 0; i < MINE; ++i) mma(acc[p][i], a01.x, a01.y, a23.x, a23.y, fb[i][0][p], fb[i][1][p]);
-          }
+          for (int i = 0; i < MINE; ++i) mma(sum[i], m01.x, m01.y, m23.x, m23.y, fb[i][0][p], fb[i][1][p]);
+#pragma unroll
+          for (int i = 0; i < MINE; ++i) mma(sum[i], h01.x, h01.y, h23.x, h23.y, fb[i][0][p], fb[i][1][p]);
+#pragma unroll
+          for (int i = 0; i < MINE; ++i)
+#pragma unroll
+            for (int v = 0; v < 4; ++v) acc[p][i][v] += sum[i][v];
+        }
       }
     };
     if (tiles > 4) walk(std::integral_constant<int, 4>());

@@ -247,6 +247,53 @@ def test_tensor_core_apply_touches_only_true_neighbours():
     assert torch.equal(got[~touched], want[~touched])
 
 
+@pytest.mark.parametrize("order", ["random", "sorted"])
+@pytest.mark.parametrize("nlat, nlon, reach", [(6, 512, 2), (32, 256, 4), (24, 48, 2.5)])
+def test_tensor_core_apply_rounds_no_worse_than_the_fma_kernel(nlat, nlon, reach, order):
+    """Sums that cancel show the rounding of the accumulation, which the bf16 result hides otherwise: along a longitude the
+    field is constant and the last entry of every window takes away the sum of the others.  In float64 what is left is
+    about 2^-24 of a term, so the result is the error.  Bound: the FMA kernel's (a field on an 8-byte boundary takes it)."""
+    from gm_attention_b200.nn.lattice_depthwise import _apply
+
+    c = make_case(nlat, nlon, reach * math.pi / nlat, {0: 8, 1: 8}, 1, dtype=np.float32)
+    t, _ = package_tables(c, None, False)
+    lat, D = t.lattice, 24
+    gen = np.random.default_rng(7)
+    table = gen.standard_normal((t.n_entries, t.table_width)).astype(np.float32)
+    cnt, off = (x.cpu().numpy().reshape(-1) for x in (lat.win_cnt, lat.win_off))
+    sums = np.zeros((cnt.size, t.table_width))
+    for w in np.flatnonzero(cnt > 0):
+        rows = slice(off[w], off[w] + cnt[w])
+        if order == "sorted":  # partial sums of the size of the window, and back
+            table[rows] = -np.sort(-table[rows], axis=0)
+        last = off[w] + cnt[w] - 1
+        table[last] = -table[rows][:-1].astype(np.float64).sum(0)
+        sums[w] = table[rows].astype(np.float64).sum(0)
+    ring = torch.from_numpy(gen.standard_normal((nlat, D)).astype(np.float32)).bfloat16()
+    x = ring.float().double().numpy()
+    want = np.zeros((nlat, D))
+    items, span = t.items.cpu().numpy(), 2 * lat.halo + 1
+    for i in range(nlat):
+        for w in range(span):
+            j = i + w - lat.halo
+            if 0 <= j < nlat and cnt[i * span + w]:
+                for kind, col, fcol in items:
+                    m = sums[i * span + w, fcol:fcol + 4]
+                    m = m.reshape(2, 2) if kind == 0 else np.diag(m[:2])
+                    want[i, col:col + 2] += m @ x[j, col:col + 2]
+    field = ring[:, None, :].expand(nlat, nlon, D).reshape(nlat * nlon, D).contiguous().cuda()
+    shifted = torch.empty(field.numel() + 4, dtype=field.dtype, device="cuda")[4:].view(field.shape)
+    shifted.copy_(field)
+    assert field.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 == 8
+    table = cuda(table)
+    error = []
+    for v in (field, shifted):
+        got = _apply(v, table, t, False).float().double().cpu().numpy().reshape(nlat, nlon, D)
+        error.append((float(np.sqrt(((got - want[:, None]) ** 2).mean())), float(np.abs(got - want[:, None]).max())))
+    print(nlat, nlon, order, "tensor cores", error[0], "fma", error[1])
+    assert error[0][0] <= error[1][0] and error[0][1] <= error[1][1]
+
+
 @pytest.mark.parametrize("head", [{0: 2, 1: 1}, {0: 6, 1: 5, 2: 7}, {1: 3}, {0: 130, 1: 130}, {0: 4}])
 def test_fold_kernel_equals_the_tensor_algebra(head):
     """One launch each way against :func:`fold` and its autograd gradients: a handful of float32 products per value, 2e-6 of
