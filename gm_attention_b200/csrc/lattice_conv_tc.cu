@@ -241,33 +241,128 @@ constexpr int AP_SLOTS = 32;                              // offsets -7 .. 24 of
 constexpr int AP_PAIR = 3 * AP_SLOTS + 1;                 // 8-byte words per channel pair
 constexpr int AP_STAGE = 8 * AP_SP + (TC_PAIRS * AP_PAIR * 8 + 15) / 16;  // 16-byte words
 
-// One output of the sums by themselves: a sum that is not finite may owe it to a value outside its window (0 x Inf) or to
-// another component, so such outputs are formed again from their own neighbours alone.
-__device__ __noinline__ float2 apply_one(const ConvArgs& a, const __nv_bfloat16* x, int row, int l, int col, PairItem it) {
-  float2 y = make_float2(0.f, 0.f);
+// What a CTA works on: 32 columns of a target row's longitudes 8 t0 .. 8 (t0 + tl) - 1, one sample (`field`)
+struct ApplyTile {
+  const unsigned char* field;
+  int row, t0, tl, col0;
+};
+// Stages: offsets [d, d + n) of a window of the row
+struct ApplyStage {
+  int w, d, n, cnt;  // w = 2 halo + 1: past the last
+};
+__device__ __forceinline__ ApplyStage first_stage(const ConvArgs& a, int row, int w) {  // of the windows from w on
   const int span = 2 * a.halo + 1;
-  for (int c = 0; c < span; ++c) {
-    const int j = row + c - a.halo;
+  for (; w < span; ++w) {
+    const int j = row + w - a.halo;
     if (j < 0 || j >= a.rows) continue;
-    const int cnt = a.win_cnt[row * span + c];
-    int lon = (l + (cnt ? a.win_lo[row * span + c] : 0)) % a.nlon;
-    if (lon < 0) lon += a.nlon;
-    for (int d = 0; d < cnt; ++d) {
-      const float* f = a.table + (size_t)(a.win_off[row * span + c] + d) * a.table_width + it.fcol;
-      const __nv_bfloat16* v = x + ((size_t)j * a.nlon + lon) * a.width + col;
-      const float vx = __bfloat162float(v[0]), vy = __bfloat162float(v[1]);
-      if (it.kind == 0) {
-        const float my = a.transpose ? f[2] : f[1], mz = a.transpose ? f[1] : f[2];
-        y.x = fmaf(f[0], vx, fmaf(my, vy, y.x));
-        y.y = fmaf(mz, vx, fmaf(f[3], vy, y.y));
-      } else {
-        y.x = fmaf(f[0], vx, y.x);
-        y.y = fmaf(f[1], vy, y.y);
-      }
-      lon = lon + 1 == a.nlon ? 0 : lon + 1;
-    }
+    const int cnt = a.win_cnt[row * span + w];
+    if (cnt > 0) return ApplyStage{w, 0, min(AP_OFFSETS, cnt), cnt};
   }
-  return y;
+  return ApplyStage{span, 0, 0, 0};
+}
+__device__ __forceinline__ ApplyStage next_stage(const ConvArgs& a, int row, const ApplyStage& s) {
+  const int d = s.d + s.n;
+  return d < s.cnt ? ApplyStage{s.w, d, min(AP_OFFSETS, s.cnt - d), s.cnt} : first_stage(a, row, s.w + 1);
+}
+__device__ __forceinline__ void issue_stage(const ConvArgs& a, const ApplyTile& t, const ApplyStage& s, uint4* dst) {
+  int lon = (8 * t.t0 + a.win_lo[t.row * (2 * a.halo + 1) + s.w] + s.d) % a.nlon;
+  if (lon < 0) lon += a.nlon;
+  const int steps = (7 + s.n + 7) / 8, row_bytes = 2 * a.width;
+  stage_positions<AP_SP>(dst, t.field + (size_t)(t.row + s.w - a.halo) * a.nlon * row_bytes, lon, 8 * (t.tl + steps - 1), a.nlon, row_bytes, 2 * t.col0);
+  commit();
+}
+// The matrix of channel pair `it` at offset d of the stage
+__device__ __forceinline__ float4 table_matrix(const ConvArgs& a, int row, const ApplyStage& s, int d, PairItem it) {
+  const float* f = a.table + (size_t)(a.win_off[row * (2 * a.halo + 1) + s.w] + s.d + d) * a.table_width + it.fcol;
+  if (it.kind == 0) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(f));
+    return a.transpose ? make_float4(v.x, v.z, v.y, v.w) : v;
+  }
+  const float2 v = __ldg(reinterpret_cast<const float2*>(f));
+  return make_float4(v.x, 0.f, 0.f, v.y);
+}
+// Column col of the tile's row in the result
+__device__ __forceinline__ __nv_bfloat16* apply_output(const ConvArgs& a, const ApplyTile& t, int b, int col) {
+  return static_cast<__nv_bfloat16*>(a.y) + ((size_t)b * a.rows + t.row) * a.nlon * a.width + col;
+}
+
+// The CTA's outputs whose sums were not finite, by themselves: such a sum may owe it to a value outside its window (0 x Inf) or
+// to another component, so it is formed again from its own neighbours alone, on the FMA pipe from the staged positions.  A warp
+// leaves out the channel pairs that have no such output, or none that is not NaN already (and stays so).  `bad`: bit
+// 8 p + 2 i + e = channel pair p at longitude 8 (8 (half + 2 i) + 2 c + e) + g.  128 x 256, radius 4 pi / 128, batch 2, 32 x (m <= 2): a
+// field of NaN 324 us, one Inf in a polar row (whose rings all see it) 567, nothing 264; the FMA kernel 344 whatever it meets, each
+// output by its own thread from global memory 9 058 and 1 196.
+__device__ __noinline__ void apply_again(const ConvArgs& a, const ApplyTile& tile, int b, uint4* stage_s, const PairItem* pairs_s, unsigned bad) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3, half = warp >> 2;
+  float2 y[4][4][2];
+  bool open[4];  // pairs the warp still works on
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    open[p] = __any_sync(0xffffffffu, bad >> 8 * p & 0xff);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) y[p][i][0] = y[p][i][1] = make_float2(0.f, 0.f);
+  }
+  ApplyStage s = first_stage(a, tile.row, 0);
+  if (s.w <= 2 * a.halo) issue_stage(a, tile, s, stage_s);
+  int buf = 0;
+  while (s.w <= 2 * a.halo) {
+    const ApplyStage nxt = next_stage(a, tile.row, s);
+    if (nxt.w <= 2 * a.halo) {
+      issue_stage(a, tile, nxt, stage_s + (buf ^ 1) * AP_STAGE);
+      wait_copies<1>();
+    } else {
+      wait_copies<0>();
+    }
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      if (!open[p]) continue;
+      const PairItem it = pairs_s[4 * cg + p];
+      const unsigned* words = reinterpret_cast<const unsigned*>(stage_s + buf * AP_STAGE + cg) + p;
+      float4 next = table_matrix(a, tile.row, s, 0, it);
+      for (int d = 0; d < s.n; ++d) {
+        const float4 m = next;
+        next = table_matrix(a, tile.row, s, min(d + 1, s.n - 1), it);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int q = 8 * (8 * (half + 2 * i) + 2 * c + e) + g + d;
+            const unsigned w = words[4 * ((q & 7) * AP_SP + (q >> 3) * TC_PITCH)];
+            const float vx = __uint_as_float(w << 16), vy = __uint_as_float(w & 0xffff0000u);
+            float2& out = y[p][i][e];
+            if (it.kind == 0) {
+              out.x = fmaf(m.x, vx, fmaf(m.y, vy, out.x));
+              out.y = fmaf(m.z, vx, fmaf(m.w, vy, out.y));
+            } else {
+              out.x = fmaf(m.x, vx, out.x);
+              out.y = fmaf(m.w, vy, out.y);
+            }
+          }
+      }
+      bool undecided = false;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) undecided = undecided || ((bad >> (8 * p + 2 * i + e) & 1) && !(isnan(y[p][i][e].x) && isnan(y[p][i][e].y)));
+      open[p] = __any_sync(0xffffffffu, undecided);
+    }
+    if (!__syncthreads_or(open[0] || open[1] || open[2] || open[3])) break;
+    s = nxt;
+    buf ^= 1;
+  }
+  wait_copies<0>();
+  __nv_bfloat16* at = apply_output(a, tile, b, tile.col0 + 8 * cg);
+#pragma unroll
+  for (int p = 0; p < 4; ++p)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (bad >> (8 * p + 2 * i + e) & 1) {
+          const int l = 8 * (tile.t0 + 8 * (half + 2 * i) + 2 * c + e) + g;
+          *reinterpret_cast<__nv_bfloat162*>(at + (size_t)l * a.width + 2 * p) = __floats2bfloat162_rn(y[p][i][e].x, y[p][i][e].y);
+        }
 }
 
 // (x, y) = sum of three bfloat16 pairs, largest first
@@ -281,7 +376,7 @@ __device__ __forceinline__ void split3(float x, float y, unsigned (&w)[3]) {
   }
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const ConvArgs a, int col_blocks, int lon_blocks) {
+__global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const __grid_constant__ ConvArgs a, int col_blocks, int lon_blocks) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ PairItem pairs_s[TC_PAIRS];
   int x = blockIdx.x;
@@ -297,46 +392,15 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const Conv
   const unsigned char* field = static_cast<const unsigned char*>(a.x) + (size_t)b * a.rows * a.nlon * row_bytes;
   uint4* const stage_s = reinterpret_cast<uint4*>(smem);
 
-  // stages: offsets [d, d + n) of window w of this row
-  struct Stage { int w, d, n, cnt; };
-  auto first_of = [&](int w) {
-    for (; w < span; ++w) {
-      const int j = row + w - a.halo;
-      if (j < 0 || j >= a.rows) continue;
-      const int cnt = a.win_cnt[row * span + w];
-      if (cnt > 0) return Stage{w, 0, min(AP_OFFSETS, cnt), cnt};
-    }
-    return Stage{span, 0, 0, 0};
-  };
-  auto next_of = [&](const Stage& s) {
-    const int d = s.d + s.n;
-    return d < s.cnt ? Stage{s.w, d, min(AP_OFFSETS, s.cnt - d), s.cnt} : first_of(s.w + 1);
-  };
-  auto issue = [&](int buf, const Stage& s) {
-    int lon = (8 * t0 + a.win_lo[row * span + s.w] + s.d) % a.nlon;
-    if (lon < 0) lon += a.nlon;
-    const int steps = (7 + s.n + 7) / 8;
-    stage_positions<AP_SP>(stage_s + buf * AP_STAGE, field + (size_t)(row + s.w - a.halo) * a.nlon * row_bytes, lon, 8 * (tl + steps - 1), a.nlon, row_bytes, 2 * col0);
-    commit();
-  };
+  const ApplyTile tile{field, row, t0, tl, col0};
   // this thread's two slots of the split table: a channel pair and the offsets slot - 7
   const int tp = threadIdx.x & (TC_PAIRS - 1), ts = threadIdx.x / TC_PAIRS;
   const PairItem item = pairs_s[tp];
-  auto fetch = [&](const Stage& s, float4 (&m)[2]) {
+  auto fetch = [&](const ApplyStage& s, float4 (&m)[2]) {
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int d = ts + 16 * i - 7;
-      m[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (d >= 0 && d < s.n && item.kind >= 0) {
-        const float* f = a.table + (size_t)(a.win_off[row * span + s.w] + s.d + d) * a.table_width + item.fcol;
-        if (item.kind == 0) {
-          const float4 v = __ldg(reinterpret_cast<const float4*>(f));
-          m[i] = a.transpose ? make_float4(v.x, v.z, v.y, v.w) : v;
-        } else {
-          const float2 v = __ldg(reinterpret_cast<const float2*>(f));
-          m[i] = make_float4(v.x, 0.f, 0.f, v.y);
-        }
-      }
+      m[i] = d >= 0 && d < s.n && item.kind >= 0 ? table_matrix(a, row, s, d, item) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
   auto place = [&](int buf, const float4 (&m)[2]) {
@@ -359,19 +423,19 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const Conv
 #pragma unroll
       for (int v = 0; v < 4; ++v) acc[p][i][v] = 0.f;
 
-  Stage cur = first_of(0);
+  ApplyStage cur = first_stage(a, row, 0);
   float4 m[2];
   if (cur.w < span) {
-    issue(0, cur);
+    issue_stage(a, tile, cur, stage_s);
     fetch(cur, m);
     place(0, m);
   }
   int buf = 0;
   while (cur.w < span) {
-    const Stage nxt = next_of(cur);
+    const ApplyStage nxt = next_stage(a, row, cur);
     const bool more = nxt.w < span;
     if (more) {
-      issue(buf ^ 1, nxt);
+      issue_stage(a, tile, nxt, stage_s + (buf ^ 1) * AP_STAGE);
       fetch(nxt, m);
       wait_copies<1>();
     } else {
@@ -421,37 +485,37 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const Conv
 
   // ---- four channel pairs of a position are 16 bytes of its row
   const int col = col0 + 8 * cg;
-  if (col >= a.width) return;
-  __nv_bfloat16* y = static_cast<__nv_bfloat16*>(a.y) + ((size_t)b * a.rows + row) * a.nlon * a.width + col;
-  const __nv_bfloat16* xf = reinterpret_cast<const __nv_bfloat16*>(field);
-  bool whole = true;
+  unsigned bad = 0;  // outputs whose sums are not finite
+  if (col < a.width) {
+    __nv_bfloat16* y = apply_output(a, tile, b, col);
+    bool whole = true;
 #pragma unroll
-  for (int p = 0; p < 4; ++p) whole = whole && pairs_s[4 * cg + p].kind >= 0;
+    for (int p = 0; p < 4; ++p) whole = whole && pairs_s[4 * cg + p].kind >= 0;
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int t = 8 * (half + 2 * i) + 2 * c + e;
-      if (t >= tl) continue;
-      const int l = 8 * (t0 + t) + g;
-      unsigned word[4];
+      for (int e = 0; e < 2; ++e) {
+        const int t = 8 * (half + 2 * i) + 2 * c + e;
+        if (t >= tl) continue;
+        unsigned word[4];
 #pragma unroll
-      for (int p = 0; p < 4; ++p) {
-        float2 v = make_float2(acc[p][i][e], acc[p][i][2 + e]);
-        const PairItem it = pairs_s[4 * cg + p];
-        if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && it.kind >= 0) v = apply_one(a, xf, row, l, col + 2 * p, it);
-        const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
-        word[p] = *reinterpret_cast<const unsigned*>(&h);
+        for (int p = 0; p < 4; ++p) {
+          const float2 v = make_float2(acc[p][i][e], acc[p][i][2 + e]);
+          if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && pairs_s[4 * cg + p].kind >= 0) bad |= 1u << (8 * p + 2 * i + e);
+          const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+          word[p] = *reinterpret_cast<const unsigned*>(&h);
+        }
+        __nv_bfloat16* at = y + (size_t)(8 * (t0 + t) + g) * a.width;
+        if (whole) {
+          *reinterpret_cast<uint4*>(at) = make_uint4(word[0], word[1], word[2], word[3]);
+        } else {
+#pragma unroll
+          for (int p = 0; p < 4; ++p)
+            if (pairs_s[4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(at + 2 * p) = word[p];
+        }
       }
-      __nv_bfloat16* at = y + (size_t)l * a.width;
-      if (whole) {
-        *reinterpret_cast<uint4*>(at) = make_uint4(word[0], word[1], word[2], word[3]);
-      } else {
-#pragma unroll
-        for (int p = 0; p < 4; ++p)
-          if (pairs_s[4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(at + 2 * p) = word[p];
-      }
-    }
+  }
+  if (__syncthreads_or(bad != 0)) apply_again(a, tile, b, stage_s, pairs_s, bad);
 }
 
 }  // namespace

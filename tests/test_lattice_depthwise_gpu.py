@@ -294,6 +294,33 @@ def test_tensor_core_apply_rounds_no_worse_than_the_fma_kernel(nlat, nlon, reach
     assert error[0][0] <= error[1][0] and error[0][1] <= error[1][1]
 
 
+@pytest.mark.parametrize("share", [3e-4, 1e-2, 1.0])
+@pytest.mark.parametrize("head, nlon", [({0: 8, 1: 8}, 88), ({0: 4, 1: 10, 2: 12}, 552)])
+def test_tensor_core_apply_of_non_finite_fields(head, nlon, share):
+    """Infinities and NaNs everywhere or here and there, with zeros in the table: the same outputs are NaN, infinite and finite
+    as by the FMA kernel (a field on an 8-byte boundary takes it); finite ones to the bf16 storage's 2^-7."""
+    from gm_attention_b200.nn.lattice_depthwise import _apply
+
+    c = make_case(7, nlon, 2 * math.pi / 7, head, 1, dtype=np.float32)
+    t, _ = package_tables(c, None, False)
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    table = torch.randn(t.n_entries, t.table_width, generator=gen, device="cuda")
+    table[torch.rand(table.shape, generator=gen, device="cuda") < 0.2] = 0.0
+    x = torch.randn(2 * c.n_nodes, c.width, generator=gen, device="cuda")
+    odd = torch.rand(x.shape, generator=gen, device="cuda") < share
+    values = torch.tensor([math.nan, math.inf, -math.inf], device="cuda")[torch.randint(3, x.shape, generator=gen, device="cuda")]
+    field = torch.where(odd, values, x).bfloat16()
+    shifted = torch.empty(field.numel() + 4, dtype=field.dtype, device="cuda")[4:].view(field.shape)
+    shifted.copy_(field)
+    assert c.width % 8 == 0 and field.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 == 8
+    got, want = (_apply(v, table, t, False).float() for v in (field, shifted))
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
+    assert bool(want.isnan().any()) and (share == 1.0 or bool(want.isfinite().any()))
+    finite = want.isfinite()
+    if bool(finite.any()):
+        assert float((got - want)[finite].abs().max()) <= 2.0 ** -7 * float(want[finite].abs().max())
+
+
 @pytest.mark.parametrize("head", [{0: 2, 1: 1}, {0: 6, 1: 5, 2: 7}, {1: 3}, {0: 130, 1: 130}, {0: 4}])
 def test_fold_kernel_equals_the_tensor_algebra(head):
     """One launch each way against :func:`fold` and its autograd gradients: a handful of float32 products per value, 2e-6 of
