@@ -66,6 +66,8 @@ SIGNATURES: dict[str, list[Any]] = {
     "gm_halo_move": [_I, _P, _I, _L, _L, _L, _P, _I, _P],
     "gm_lattice_conv_apply": [_P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "gm_lattice_conv_table_grad": [_P, _P, _P, _I, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "gm_lattice_conv_apply_tc": [_P, _P, _P, _I, _P, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _I, _P, _P],
+    "gm_lattice_conv_table_grad_tc": [_P, _P, _P, _I, _P, _P, _P, _P, _L, _I, _I, _I, _I, _I, _I, _I, _P, _P],
     "gm_lattice_conv_fold": [_P] * 7 + [_L, _I, _I, _I, _I] + [_P] * 4,
     "gm_peer_alloc": [_L, _P, _P],
     "gm_peer_free": [_P],

@@ -551,9 +551,9 @@ using namespace gmb;
 
 // y = table applied along the windows.  order: n_order target rows (any subset, any order).  transpose != 0 applies the
 // transposed matrices (the windows and the table are then the transposed ones: gradient with respect to the field).
-extern "C" int gm_lattice_conv_apply(const void* x, const float* table, const int32_t* items, int n_items, const int32_t* win_cnt,
-                                     const int32_t* win_lo, const int32_t* win_off, const int32_t* order, int n_order, int rows, int nlon,
-                                     int batch, int width, int halo, int table_width, int transpose, int dtype, void* y, void* stream) {
+static int conv_apply(bool tensor_cores, const void* x, const float* table, const int32_t* items, int n_items, const int32_t* win_cnt, const int32_t* win_lo,
+                      const int32_t* win_off, const int32_t* order, int n_order, int rows, int nlon, int batch, int width, int halo, int table_width,
+                      int transpose, int dtype, void* y, void* stream) {
   if (n_order == 0) return GM_OK;
   if (int status = check_common("gm_lattice_conv_apply", x, table, items, n_items, win_cnt, win_lo, win_off, rows, nlon, batch, width, halo,
                                 table_width, dtype))
@@ -564,7 +564,9 @@ extern "C" int gm_lattice_conv_apply(const void* x, const float* table, const in
   a.n_items = n_items; a.rows = rows; a.nlon = nlon; a.batch = batch; a.width = width; a.halo = halo; a.table_width = table_width;
   a.transpose = transpose;
   cudaStream_t cs = (cudaStream_t)stream;
-  if (dtype == GM_BF16 && lconv::tensor_cores_take(a)) return lconv::apply_tc(a, n_order, cs);
+  GM_REQUIRE(!tensor_cores || (dtype == GM_BF16 && lconv::tensor_cores_can(a)), GM_ERR_UNSUPPORTED,
+             "gm_lattice_conv_apply_tc: bfloat16 fields whose rows are whole 16-byte words on 16-byte boundaries");
+  if (tensor_cores || (dtype == GM_BF16 && lconv::tensor_cores_apply(a))) return lconv::apply_tc(a, n_order, cs);
   const int elem = dtype == GM_F32 ? 4 : 2;
   StagedShape sh{};
   const int nb = staged_shape(a, elem, n_order, sh);
@@ -599,12 +601,26 @@ extern "C" int gm_lattice_conv_apply(const void* x, const float* table, const in
   return launch_status("gm_lattice_conv_apply");
 }
 
+extern "C" int gm_lattice_conv_apply(const void* x, const float* table, const int32_t* items, int n_items, const int32_t* win_cnt, const int32_t* win_lo,
+                                     const int32_t* win_off, const int32_t* order, int n_order, int rows, int nlon, int batch, int width, int halo,
+                                     int table_width, int transpose, int dtype, void* y, void* stream) {
+  return conv_apply(false, x, table, items, n_items, win_cnt, win_lo, win_off, order, n_order, rows, nlon, batch, width, halo, table_width, transpose,
+                    dtype, y, stream);
+}
+
+extern "C" int gm_lattice_conv_apply_tc(const void* x, const float* table, const int32_t* items, int n_items, const int32_t* win_cnt, const int32_t* win_lo,
+                                        const int32_t* win_off, const int32_t* order, int n_order, int rows, int nlon, int batch, int width, int halo,
+                                        int table_width, int transpose, int dtype, void* y, void* stream) {
+  return conv_apply(true, x, table, items, n_items, win_cnt, win_lo, win_off, order, n_order, rows, nlon, batch, width, halo, table_width, transpose,
+                    dtype, y, stream);
+}
+
 // dtable[entry] = sum over longitudes and samples of g (target) (x) x (source).  blocks: (n_blocks, 2) int32 = (window
 // index = target row * (2 * halo + 1) + source row - target row + halo, first offset), 8 offsets each; entries no block
 // covers are left untouched.
-extern "C" int gm_lattice_conv_table_grad(const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt,
-                                          const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows,
-                                          int nlon, int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream) {
+static int conv_table_grad(bool tensor_cores, const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt, const int32_t* win_lo,
+                           const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows, int nlon, int batch, int width, int halo,
+                           int table_width, int dtype, float* dtable, void* stream) {
   if (n_blocks == 0) return GM_OK;
   if (int status = check_common("gm_lattice_conv_table_grad", x, dtable, items, n_items, win_cnt, win_lo, win_off, rows, nlon, batch, width,
                                 halo, table_width, dtype))
@@ -616,7 +632,9 @@ extern "C" int gm_lattice_conv_table_grad(const void* g, const void* x, const in
   const int threads = min(THREADS, (n_items + 31) / 32 * 32);
   const int nb = batch >= 2 ? 2 : 1;  // four samples' windows would take every register a thread can have
   cudaStream_t cs = (cudaStream_t)stream;
-  if (dtype == GM_BF16 && lconv::tensor_cores_take(a)) return lconv::table_grad_tc(a, n_blocks, cs);
+  GM_REQUIRE(!tensor_cores || (dtype == GM_BF16 && lconv::tensor_cores_can(a)), GM_ERR_UNSUPPORTED,
+             "gm_lattice_conv_table_grad_tc: bfloat16 fields whose rows are whole 16-byte words on 16-byte boundaries");
+  if (tensor_cores || (dtype == GM_BF16 && lconv::tensor_cores_table_grad(a))) return lconv::table_grad_tc(a, n_blocks, cs);
 #define GM_GRAD(S, NB) conv_table_grad_kernel<S, NB><<<(unsigned)n_blocks, threads, 0, cs>>>(a)
   if (dtype == GM_F32) {
     if (nb == 2) GM_GRAD(float, 2); else GM_GRAD(float, 1);
@@ -625,6 +643,20 @@ extern "C" int gm_lattice_conv_table_grad(const void* g, const void* x, const in
   }
 #undef GM_GRAD
   return launch_status("gm_lattice_conv_table_grad");
+}
+
+extern "C" int gm_lattice_conv_table_grad(const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt,
+                                          const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows, int nlon,
+                                          int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream) {
+  return conv_table_grad(false, g, x, items, n_items, win_cnt, win_lo, win_off, blocks, n_blocks, rows, nlon, batch, width, halo, table_width, dtype,
+                         dtable, stream);
+}
+
+extern "C" int gm_lattice_conv_table_grad_tc(const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt,
+                                             const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows, int nlon,
+                                             int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream) {
+  return conv_table_grad(true, g, x, items, n_items, win_cnt, win_lo, win_off, blocks, n_blocks, rows, nlon, batch, width, halo, table_width, dtype,
+                         dtable, stream);
 }
 
 // The table of per-entry coefficients (dtable null: forward, writes table) or the coefficients' gradients from the table's

@@ -19,8 +19,11 @@ struct ConvArgs {
   int n_items, rows, nlon, batch, width, halo, table_width, transpose;
 };
 
-// Tensor-core forms for bfloat16 fields: whether the sizes and addresses allow them, and the launches.
-bool tensor_cores_take(const ConvArgs& a);
+// Tensor-core forms for bfloat16 fields: whether the sizes and addresses allow them, whether they are the faster ones, and the
+// launches.
+bool tensor_cores_can(const ConvArgs& a);
+bool tensor_cores_apply(const ConvArgs& a);
+bool tensor_cores_table_grad(const ConvArgs& a);
 int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream);
 int table_grad_tc(const ConvArgs& a, int64_t n_blocks, cudaStream_t stream);
 

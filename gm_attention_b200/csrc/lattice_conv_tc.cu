@@ -520,9 +520,28 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const __gr
 
 }  // namespace
 
-bool tensor_cores_take(const ConvArgs& a) {
+bool tensor_cores_can(const ConvArgs& a) {
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.y);
   return a.nlon % 8 == 0 && a.width % 8 == 0 && bits % 16 == 0;
+}
+
+// The FMA kernels stay the faster ones where a launch is short or its tiles are mostly padding.  96 shapes from 24 x 24 to
+// 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores:
+//   apply        up to 8 tiles of 8 longitudes leave half of a CTA's warps without one (64 x 64, batch 4, width 320: 53 / 143; 32 x 64,
+//                batch 1, width 40: 39 / 47); with one sample and a narrow field the launch is the polar rows' chain of stages, which is
+//                longer here (256 x 512, width 40: 367 / 526; 128 x 512, width 96: 371 / 489), from two samples on it is not (91 x 184,
+//                width 96: 259 / 170; 45 x 88, width 40: 72 / 66).  Wide fields fill the chip with one sample, and then it is padding
+//                that decides (256 x 512, width 320: 848 / 604; 64 x 128, batch 2, width 320: 174 / 199).
+//   table_grad   contracts over the tiles, 16 a step: 23 tiles and more are always faster (91 x 184, batch 1, width 80: 75 / 58; 128 x
+//                256, width 24: 99 / 50), 11 with four samples in sequence (45 x 88, width 96: 48 / 32; batch 1, width 160: 30 / 44), fewer
+//                by the shape (100 x 48, batch 4, width 24: 28 / 32; 24 x 48: 26 / 17).
+bool tensor_cores_apply(const ConvArgs& a) {
+  const int tiles = a.nlon / 8;
+  return tensor_cores_can(a) && tiles > 8 && (a.width < 256 ? a.batch >= 2 : tiles >= 32);
+}
+bool tensor_cores_table_grad(const ConvArgs& a) {
+  const int tiles = a.nlon / 8;
+  return tensor_cores_can(a) && (tiles >= 20 || (tiles > 8 && a.batch >= 4));
 }
 
 int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream) {

@@ -80,7 +80,10 @@ def conv_tables(geometry: Any, distances: Tensor, weights: Tensor, rows: Sequenc
     device = edge.device
     cnt = lat.win_cnt.cpu().numpy().reshape(-1)
     blocks = [(w, d) for w in np.flatnonzero(cnt > 0) for d in range(0, int(cnt[w]), OFFSETS_PER_BLOCK)]
-    blocks.sort(key=lambda wd: -min(OFFSETS_PER_BLOCK, int(cnt[wd[0]])))  # windows with a full block first, a window's blocks together
+    # full blocks first; a window's blocks together where the tensor-core kernel, which takes several of them at a time, may run
+    # (32 x 64, batch 2, width 320, by the FMA kernel: 42 us with full blocks first, 48 with windows together)
+    together = nlon // 8 > 8
+    blocks.sort(key=lambda wd: -min(OFFSETS_PER_BLOCK, int(cnt[wd[0]]) - (0 if together else wd[1])))
     rho = geometry.rho.index_select(0, edge).float()
     tau = [torch.view_as_complex(geometry.transport.index_select(0, edge)[:, n].float().contiguous()) for n, *_ in complex_rows]
     omega = []
@@ -168,7 +171,8 @@ def _fold(rc: Tensor | None, cc: Tensor | None, t: ConvTables) -> Tensor:
     return FoldTable.apply(rc.float() if t.a_0 else None, cc.float() if t.complex_width else None, t)  # type: ignore[no-any-return,union-attr]
 
 
-def _apply(x: Tensor, table: Tensor, t: ConvTables, transposed: bool) -> Tensor:
+def _apply(x: Tensor, table: Tensor, t: ConvTables, transposed: bool, tensor_cores: bool = False) -> Tensor:
+    """``tensor_cores``: by those kernels whatever the sizes; otherwise by the faster ones."""
     lat = t.lattice
     device = _lib.require_cuda(x, table)
     nodes = lat.rows * lat.nlon
@@ -182,18 +186,18 @@ def _apply(x: Tensor, table: Tensor, t: ConvTables, transposed: bool) -> Tensor:
     if order.numel() != lat.rows:
         y.zero_()
     with torch.cuda.device(device):
-        _lib.call("gm_lattice_conv_apply", _lib.ptr(x), _lib.ptr(table), _lib.ptr(t.items), t.items.shape[0], _lib.ptr(cnt), _lib.ptr(lo),
+        _lib.call("gm_lattice_conv_apply_tc" if tensor_cores else "gm_lattice_conv_apply", _lib.ptr(x), _lib.ptr(table), _lib.ptr(t.items), t.items.shape[0], _lib.ptr(cnt), _lib.ptr(lo),
                   _lib.ptr(off), _lib.ptr(order), order.numel(), lat.rows, lat.nlon, x.shape[0] // nodes, x.shape[1], lat.halo,
                   t.table_width, int(transposed), _lib.dtype_code(x.dtype), _lib.ptr(y), _lib.stream(device))
     return y
 
 
-def _table_gradient(grad: Tensor, x: Tensor, t: ConvTables) -> Tensor:
+def _table_gradient(grad: Tensor, x: Tensor, t: ConvTables, tensor_cores: bool = False) -> Tensor:
     lat = t.lattice
     device = _lib.require_cuda(grad, x)
     out = torch.zeros((t.n_entries, t.table_width), dtype=torch.float32, device=device)
     with torch.cuda.device(device):
-        _lib.call("gm_lattice_conv_table_grad", _lib.ptr(grad), _lib.ptr(x), _lib.ptr(t.items), t.items.shape[0], _lib.ptr(lat.win_cnt),
+        _lib.call("gm_lattice_conv_table_grad_tc" if tensor_cores else "gm_lattice_conv_table_grad", _lib.ptr(grad), _lib.ptr(x), _lib.ptr(t.items), t.items.shape[0], _lib.ptr(lat.win_cnt),
                   _lib.ptr(lat.win_lo), _lib.ptr(lat.win_off), _lib.ptr(t.blocks), t.blocks.shape[0], lat.rows, lat.nlon,
                   x.shape[0] // (lat.rows * lat.nlon), x.shape[1], lat.halo, t.table_width, _lib.dtype_code(x.dtype), _lib.ptr(out),
                   _lib.stream(device))

@@ -506,6 +506,14 @@ int gm_lattice_conv_apply(const void* x, const float* table, const int32_t* item
 int gm_lattice_conv_table_grad(const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt,
                                const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows,
                                int nlon, int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream);
+/* The same by the tensor-core kernels whatever the sizes: GM_BF16, nlon and width multiples of 8, fields on 16-byte boundaries
+ * (GM_ERR_UNSUPPORTED otherwise).  The calls above take them where they are the faster ones. */
+int gm_lattice_conv_apply_tc(const void* x, const float* table, const int32_t* items, int n_items, const int32_t* win_cnt,
+                             const int32_t* win_lo, const int32_t* win_off, const int32_t* order, int n_order, int rows, int nlon,
+                             int batch, int width, int halo, int table_width, int transpose, int dtype, void* y, void* stream);
+int gm_lattice_conv_table_grad_tc(const void* g, const void* x, const int32_t* items, int n_items, const int32_t* win_cnt,
+                                  const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows,
+                                  int nlon, int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream);
 /* gm_lattice_conv_fold: an entry's coefficients rc (entries, a0), cc (entries, width), weight and phases tau, omega
  * (entries, nf, 2) -> its table row: w rc, zeros up to a multiple of 4, then per complex copy the matrix [[a, b], [c, d]]
  * of z -> w (A tau z + omega B conj(tau z)); items (n_complex, 3) int32: columns of A and B in cc, frequency index.  With

@@ -204,7 +204,7 @@ def test_tensor_core_kernels_against_the_host_loops(nlat, nlon, reach, head, bat
         used = table[lat.t_entry.cpu().numpy()] if transposed else table
         want = _apply_on_the_host(x[sample].double().numpy(), used.astype(np.float64), *(w.cpu().numpy() for w in windows), items, nlat, nlon, lat.halo,
                                   transposed)
-        got = _apply(x.cuda(), cuda(used), t, transposed)[sample].float().cpu().numpy()
+        got = _apply(x.cuda(), cuda(used), t, transposed, tensor_cores=True)[sample].float().cpu().numpy()
         assert_close(got, want, 2.0 ** -8, 1e-5 * np.abs(want).max(), "transposed" if transposed else "forward")
     cnt, lo, off = (w.cpu().numpy() for w in (lat.win_cnt, lat.win_lo, lat.win_off))
     X, G = (v.double().numpy().reshape(batch, nlat, nlon, c.width) for v in (x, g))
@@ -218,7 +218,7 @@ def test_tensor_core_kernels_against_the_host_loops(nlat, nlon, reach, head, bat
                     want[off[i, w] + d, fcol:fcol + (4 if kind == 0 else 2)] = m.reshape(-1) if kind == 0 else (m[0, 0], m[1, 1])
     order = torch.randperm(t.blocks.shape[0], generator=torch.Generator().manual_seed(5))
     for blocks in (t.blocks, t.blocks[order.to(t.blocks.device)].contiguous()):
-        got = _table_gradient(g.cuda(), x.cuda(), dataclasses.replace(t, blocks=blocks))
+        got = _table_gradient(g.cuda(), x.cuda(), dataclasses.replace(t, blocks=blocks), tensor_cores=True)
         assert_close(got.cpu().numpy(), want, 1e-5, 1e-5 * np.abs(want).max(), "table gradient")
 
 
@@ -230,12 +230,12 @@ def test_tensor_core_apply_touches_only_true_neighbours():
     table, = seeded((t.n_entries, t.table_width), 73, np.float32)
     v, = seeded((c.n_nodes, c.width), 74, np.float32)
     clean = torch.from_numpy(v).bfloat16().cuda()
-    want = _apply(clean, cuda(table), t, False)
+    want = _apply(clean, cuda(table), t, False, tensor_cores=True)
     dirty = clean.clone()
     nodes = [(5 * c.nlon + 63, 5, float("inf")), (9 * c.nlon + 20, 2, float("nan")), (0, 9, 3e38)]
     for node, col, value in nodes:
         dirty[node, col] = value
-    got = _apply(dirty, cuda(table), t, False)
+    got = _apply(dirty, cuda(table), t, False, tensor_cores=True)
     touched = torch.zeros_like(got, dtype=torch.bool)
     for node, col, value in nodes:
         seen_by = torch.from_numpy(np.unique(c.target[c.source == node])).cuda()
@@ -252,7 +252,7 @@ def test_tensor_core_apply_touches_only_true_neighbours():
 def test_tensor_core_apply_rounds_no_worse_than_the_fma_kernel(nlat, nlon, reach, order):
     """Sums that cancel show the rounding of the accumulation, which the bf16 result hides otherwise: along a longitude the
     field is constant and the last entry of every window takes away the sum of the others.  In float64 what is left is
-    about 2^-24 of a term, so the result is the error.  Bound: the FMA kernel's (a field on an 8-byte boundary takes it)."""
+    about 2^-24 of a term, so the result is the error.  Bound: the FMA kernel's (which one sample of so narrow a field takes)."""
     from gm_attention_b200.nn.lattice_depthwise import _apply
 
     c = make_case(nlat, nlon, reach * math.pi / nlat, {0: 8, 1: 8}, 1, dtype=np.float32)
@@ -282,23 +282,19 @@ def test_tensor_core_apply_rounds_no_worse_than_the_fma_kernel(nlat, nlon, reach
                     m = m.reshape(2, 2) if kind == 0 else np.diag(m[:2])
                     want[i, col:col + 2] += m @ x[j, col:col + 2]
     field = ring[:, None, :].expand(nlat, nlon, D).reshape(nlat * nlon, D).contiguous().cuda()
-    shifted = torch.empty(field.numel() + 4, dtype=field.dtype, device="cuda")[4:].view(field.shape)
-    shifted.copy_(field)
-    assert field.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 == 8
     table = cuda(table)
     error = []
-    for v in (field, shifted):
-        got = _apply(v, table, t, False).float().double().cpu().numpy().reshape(nlat, nlon, D)
+    for tensor_cores in (True, False):
+        got = _apply(field, table, t, False, tensor_cores=tensor_cores).float().double().cpu().numpy().reshape(nlat, nlon, D)
         error.append((float(np.sqrt(((got - want[:, None]) ** 2).mean())), float(np.abs(got - want[:, None]).max())))
-    print(nlat, nlon, order, "tensor cores", error[0], "fma", error[1])
-    assert error[0][0] <= error[1][0] and error[0][1] <= error[1][1]
+    assert error[0][0] <= error[1][0] and error[0][1] <= error[1][1], error
 
 
 @pytest.mark.parametrize("share", [3e-4, 1e-2, 1.0])
 @pytest.mark.parametrize("head, nlon", [({0: 8, 1: 8}, 88), ({0: 4, 1: 10, 2: 12}, 552)])
 def test_tensor_core_apply_of_non_finite_fields(head, nlon, share):
     """Infinities and NaNs everywhere or here and there, with zeros in the table: the same outputs are NaN, infinite and finite
-    as by the FMA kernel (a field on an 8-byte boundary takes it); finite ones to the bf16 storage's 2^-7."""
+    as by the FMA kernel (which takes a field on an 8-byte boundary); finite ones to the bf16 storage's 2^-7."""
     from gm_attention_b200.nn.lattice_depthwise import _apply
 
     c = make_case(7, nlon, 2 * math.pi / 7, head, 1, dtype=np.float32)
@@ -313,7 +309,7 @@ def test_tensor_core_apply_of_non_finite_fields(head, nlon, share):
     shifted = torch.empty(field.numel() + 4, dtype=field.dtype, device="cuda")[4:].view(field.shape)
     shifted.copy_(field)
     assert c.width % 8 == 0 and field.data_ptr() % 16 == 0 and shifted.data_ptr() % 16 == 8
-    got, want = (_apply(v, table, t, False).float() for v in (field, shifted))
+    got, want = _apply(field, table, t, False, tensor_cores=True).float(), _apply(shifted, table, t, False).float()
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isposinf(), want.isposinf()) and torch.equal(got.isneginf(), want.isneginf())
     assert bool(want.isnan().any()) and (share == 1.0 or bool(want.isfinite().any()))
     finite = want.isfinite()
