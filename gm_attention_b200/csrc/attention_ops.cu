@@ -6,9 +6,9 @@
 // (scores :145-165, softmax :295-316, softmax backward :320-348, depthwise
 // message :174-206, its backward :211-232); the kernels themselves are new:
 //
-//  * scores, head-grouped (H a power of two, the usual case): one warp per target, the lanes split into H head
+//  * scores, head-grouped (H a power of two, the usual case): one or two warps per target, the lanes split into H head
 //    groups, every lane owning a few copies of every frequency; four edges' gathers of k_j are in flight; the raw
-//    logits go to alpha and the same warp normalises the row in place.
+//    logits go to alpha and the same warps normalise the row in place.
 //  * scores, general: one block per target, one WARP per edge with the lanes striding the key row (coalesced
 //    128-byte reads of k_j), per-head sums by warp shuffle; the row's logits live in shared memory (or, for very
 //    large neighbourhoods, in the alpha output itself) and are normalised there.
@@ -107,20 +107,26 @@ __global__ void __launch_bounds__(SM_THREADS) softmax_forward_kernel(SoftmaxArgs
 }
 
 
-// Scores + softmax with the lanes of a warp split into H head groups (H a power of two): one warp per target,
+// Scores + softmax with the lanes of a warp split into H head groups (H a power of two): PARTS warps per target,
 // a group of L = 32 / H lanes owns a head and each lane the copies u = s, s + L, ... of every frequency (at most
 // R per frequency).  Per edge every lane reads its own columns of k_j (the groups together read the whole row once),
 // the group reduces with log2(L) xor-shuffles, and all H logits of the edge appear at once.  The raw logits go to
-// alpha, the row is then normalised in place by the same warp (masked edges never enter the shift or the sum).
+// alpha, the row is then normalised in place by the same warps (masked edges never enter the shift or the sum).
 // NF: the number of descriptor rows when known at compile time (3 or 4 frequencies: the usual head types), 0 = up to MAX_F
 //
-// SCORE_PARTS warps share a target, four edges of it in turn each: 883 us with one, 762 with two, 808 with four (128 x 256,
-// radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32; half of the targets have fewer than 30 edges, the polar ones a thousand).
-constexpr int SCORE_PARTS = 2;
+// PARTS warps share a target, four edges of it in turn each.  Two where the launch is about as long as its longest target's chain
+// of edges (about 1 us for four), one where there are edges enough to hide it: then every warp of a pair only repeats the other's
+// q_i and waits for it.  us with one / two, float32: 128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3) (3 920 edges per edge of the
+// longest target) 883 / 762 (four: 808); 64 x 128, radius 4 pi / 64 (2 120) 575 / 318; 2 562 points of even degree 200 (2 500) 199 / 121;
+// 10 242 points, 4 heads of 8 x (m <= 2), degree 12 (8 400) 39 / 47, degree 200 429 / 432; 163 842, degree 12 457 / 623.  Eight heads' groups of
+// four lanes take longer over an edge: 10 242 points, degree 21 92 / 82, degree 100 356 / 285, degree 11 57 / 57.
+int score_parts(int64_t n_nodes, int64_t n_edges, int64_t deg_max, int H) {
+  return n_edges <= 4096 * deg_max || (H == 8 && n_edges >= 16 * n_nodes) ? 2 : 1;
+}
 
-template <typename T, int R, int NF>
+template <typename T, int R, int NF, int PARTS>
 __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArgs<T> a) {
-  constexpr int FN = NF ? NF : MAX_F, PARTS = SCORE_PARTS, TARGETS = 4 / PARTS;
+  constexpr int FN = NF ? NF : MAX_F, TARGETS = 4 / PARTS;
   __shared__ T max_s[TARGETS][PARTS][MAX_H], sum_s[TARGETS][PARTS][MAX_H];
   const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % PARTS, mine = (threadIdx.x >> 5) / PARTS;
   const int64_t x = (int64_t)blockIdx.x * TARGETS + mine;
@@ -176,45 +182,72 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
     if (s == 0) a.alpha[e * a.H + h] = lw;
   };
   constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together (8: 0.96 ms against 0.88)
-  for (int64_t e = e0 + U * part; e < e1; e += U * PARTS) {
-    if (e + U <= e1) {
-      const T* k_j[U];
-      T part_sum[U];
+  auto several = [&](int64_t e) {
+    const T* k_j[U];
+    T part_sum[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) k_j[u] = a.k + a.source[e + u] * a.D;
+    for (int u = 0; u < U; ++u) k_j[u] = a.k + a.source[e + u] * a.D;
 #pragma unroll
-      for (int u = 0; u < U; ++u) part_sum[u] = dot(k_j[u], a.transport + (e + u) * a.orders * 2);
-      for (int o = L >> 1; o > 0; o >>= 1) {
+    for (int u = 0; u < U; ++u) part_sum[u] = dot(k_j[u], a.transport + (e + u) * a.orders * 2);
+    for (int o = L >> 1; o > 0; o >>= 1) {
 #pragma unroll
-        for (int u = 0; u < U; ++u) part_sum[u] += __shfl_xor_sync(0xffffffffu, part_sum[u], o);
-      }
+      for (int u = 0; u < U; ++u) part_sum[u] += __shfl_xor_sync(0xffffffffu, part_sum[u], o);
+    }
 #pragma unroll
-      for (int u = 0; u < U; ++u) finish(e + u, part_sum[u]);
-    } else {
-      for (int64_t t = e; t < e1; ++t) {
-        T one = dot(a.k + a.source[t] * a.D, a.transport + t * a.orders * 2);
-        for (int o = L >> 1; o > 0; o >>= 1) one += __shfl_xor_sync(0xffffffffu, one, o);
-        finish(t, one);
-      }
+    for (int u = 0; u < U; ++u) finish(e + u, part_sum[u]);
+  };
+  auto rest = [&](int64_t e) {
+    for (; e < e1; ++e) {
+      T one = dot(a.k + a.source[e] * a.D, a.transport + e * a.orders * 2);
+      for (int o = L >> 1; o > 0; o >>= 1) one += __shfl_xor_sync(0xffffffffu, one, o);
+      finish(e, one);
+    }
+  };
+  if constexpr (PARTS == 1 && NF != 4) {  // (four frequencies: the other form is the faster, 40 962 points of degree 12, 8 heads 203 -> 188 us)
+    int64_t e = e0;
+    for (; e + U <= e1; e += U) several(e);
+    rest(e);
+  } else {
+    for (int64_t e = e0 + U * part; e < e1; e += U * PARTS) {
+      if (e + U <= e1) several(e);
+      else rest(e);
     }
   }
-  if (s == 0) max_s[mine][part][h] = m;
-  __syncthreads();
+  if constexpr (PARTS > 1) {
+    if (s == 0) max_s[mine][part][h] = m;
+    __syncthreads();
 #pragma unroll
-  for (int p = 0; p < PARTS; ++p) m = max_s[mine][p][h] > m ? max_s[mine][p][h] : m;
-  // normalise: the group's lanes stride the row's edges for their head
-  T sum = T(0);
-  for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) {
+    for (int p = 0; p < PARTS; ++p) m = max_s[mine][p][h] > m ? max_s[mine][p][h] : m;
+  } else {
+    __syncwarp();
+  }
+  // normalise: the group's lanes stride the row's edges for their head.  The sum is that of two halves (every other L edges),
+  // so that one warp gets the bits of two: a chunk of an edge set may be given to one, the whole set to two
+  auto weigh = [&](int64_t e) {
     const T u = a.inside[e] ? gm_exp(a.alpha[e * a.H + h] - m) : T(0);
     a.alpha[e * a.H + h] = u;
-    sum += u;
+    return u;
+  };
+  T sum = T(0);
+  if constexpr (PARTS > 1) {
+    static_assert(PARTS == 2, "as many halves as there are");
+    for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) sum += weigh(e);
+    for (int o = L >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (s == 0) sum_s[mine][part][h] = sum;
+    __syncthreads();
+    sum = sum_s[mine][0][h] + sum_s[mine][1][h];
+  } else {
+    T other = T(0);
+    for (int64_t e = e0 + s; e < e1; e += 2 * L) {
+      sum += weigh(e);
+      if (e + L < e1) other += weigh(e + L);
+    }
+    for (int o = L >> 1; o > 0; o >>= 1) {
+      sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      other += __shfl_xor_sync(0xffffffffu, other, o);
+    }
+    sum += other;
   }
-  for (int o = L >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if (s == 0) sum_s[mine][part][h] = sum;
-  __syncthreads();
-  sum = T(0);
-#pragma unroll
-  for (int p = 0; p < PARTS; ++p) sum += sum_s[mine][p][h];
   for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) a.alpha[e * a.H + h] /= sum;
 }
 
@@ -272,9 +305,9 @@ __device__ __forceinline__ void store_pair(T* p, T x, T y) {
 // p[0] += x, p[1] += y.  A float pair on an 8-byte boundary is one vector reduction: half as many operations for the L2
 // units.  128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32: 1 098 -> 897 us for the scores' backward.  (The
 // depthwise backward and the fused layer's on general graphs lose by it, 1 045 -> 1 190 and 363 -> 394 us.)
-template <typename T>
+template <bool VECTOR, typename T>
 __device__ __forceinline__ void add_pair(T* p, T x, T y) {
-  if constexpr (std::is_same<T, float>::value) {
+  if constexpr (VECTOR && std::is_same<T, float>::value) {
     if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
       asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(x), "f"(y));
       return;
@@ -292,7 +325,7 @@ struct ScoreItem {
 // Backward of scores + softmax: a warp per target node.  The lanes first reduce sum_e alpha dalpha per head, then
 // every lane owns one item and walks the node's edges in order (dq is a sequential sum per column), four edges'
 // gathers in flight; dk is accumulated atomically.
-template <typename T>
+template <typename T, bool VECTOR>
 __global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ScoreItem* items_s = reinterpret_cast<ScoreItem*>(smem_raw);
@@ -358,7 +391,7 @@ __global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
           const T ds = a.scale * al * (da - total);
           dq_r += ds * (tr * kr - ti * ki);  // (tau k)
           dq_i += ds * (tr * ki + ti * kr);
-          add_pair(a.dk + j * a.D + it.col, ds * (tr * q_r + ti * q_i), ds * (tr * q_i - ti * q_r));  // conj(tau) q
+          add_pair<VECTOR>(a.dk + j * a.D + it.col, ds * (tr * q_r + ti * q_i), ds * (tr * q_i - ti * q_r));  // conj(tau) q
         };
         int64_t e = e0;
         for (; e + U <= e1; e += U) {
@@ -594,9 +627,9 @@ __global__ void conv_backward_kernel(ConvArgs<T> a) {
 
 constexpr int CONV_THREADS = 128;  // 4 target nodes per CTA
 
-int conv_grid(int64_t n_nodes) {  // CTAs stride the nodes, so that the item table is built once for several: up to 64
-  // per SM (16, all resident at once, leave the polar rows' nodes to few of them: depthwise 682 + 1 033 us against
-  // 675 + 989, the scores' backward 897 against 796)
+int conv_grid(int64_t n_nodes) {  // CTAs stride the nodes, so that the item table is built once for several: up to
+  // 64 per SM (16, all resident at once, leave the polar rows' nodes to few of them: depthwise 682 + 1 033 us against
+  // 675 + 989; nodes of even degree: the same, 40 962 of degree 20 221 / 219)
   const int64_t want = (n_nodes + CONV_THREADS / 32 - 1) / (CONV_THREADS / 32);
   const int64_t cap = (int64_t)sm_count() * 64;
   return (int)(want < cap ? (want < 1 ? 1 : want) : cap);
@@ -605,18 +638,22 @@ int conv_grid(int64_t n_nodes) {  // CTAs stride the nodes, so that the item tab
 int grid_for(int64_t n_nodes) { return (int)(n_nodes < (int64_t)1 << 30 ? n_nodes : (int64_t)1 << 30); }
 
 template <typename T>
-int softmax_forward_t(SoftmaxArgs<T> a, int64_t deg_max, int max_mult, cudaStream_t stream) {
+int softmax_forward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, int max_mult, cudaStream_t stream) {
   // head-group kernel when the heads split a warp evenly and every lane owns at most 4 copies per frequency
   if ((a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8) && max_mult > 0 && max_mult <= 4 * (32 / a.H)) {
     const int per_lane = (max_mult + 32 / a.H - 1) / (32 / a.H);
-    const unsigned blocks = (unsigned)((a.n_nodes * SCORE_PARTS + 3) / 4);
-    if (per_lane <= 1 && a.F == 3) softmax_forward_grouped_kernel<T, 1, 3><<<blocks, 128, 0, stream>>>(a);
-    else if (per_lane <= 1 && a.F == 4) softmax_forward_grouped_kernel<T, 1, 4><<<blocks, 128, 0, stream>>>(a);
-    else if (per_lane <= 1) softmax_forward_grouped_kernel<T, 1, 0><<<blocks, 128, 0, stream>>>(a);
-    else if (per_lane <= 2 && a.F == 3) softmax_forward_grouped_kernel<T, 2, 3><<<blocks, 128, 0, stream>>>(a);
-    else if (per_lane <= 2) softmax_forward_grouped_kernel<T, 2, 0><<<blocks, 128, 0, stream>>>(a);
-    else softmax_forward_grouped_kernel<T, 4, 0><<<blocks, 128, 0, stream>>>(a);
-    return launch_status("gm_softmax_forward");
+    auto go = [&](auto parts) {
+      constexpr int P = decltype(parts)::value;
+      const unsigned blocks = (unsigned)((a.n_nodes * P + 3) / 4);
+      if (per_lane <= 1 && a.F == 3) softmax_forward_grouped_kernel<T, 1, 3, P><<<blocks, 128, 0, stream>>>(a);
+      else if (per_lane <= 1 && a.F == 4) softmax_forward_grouped_kernel<T, 1, 4, P><<<blocks, 128, 0, stream>>>(a);
+      else if (per_lane <= 1) softmax_forward_grouped_kernel<T, 1, 0, P><<<blocks, 128, 0, stream>>>(a);
+      else if (per_lane <= 2 && a.F == 3) softmax_forward_grouped_kernel<T, 2, 3, P><<<blocks, 128, 0, stream>>>(a);
+      else if (per_lane <= 2) softmax_forward_grouped_kernel<T, 2, 0, P><<<blocks, 128, 0, stream>>>(a);
+      else softmax_forward_grouped_kernel<T, 4, 0, P><<<blocks, 128, 0, stream>>>(a);
+      return launch_status("gm_softmax_forward");
+    };
+    return score_parts(a.n_nodes, n_edges, deg_max, a.H) == 2 ? go(std::integral_constant<int, 2>()) : go(std::integral_constant<int, 1>());
   }
   // Logits in shared memory when the largest neighbourhood fits ~96 KiB; else kept in alpha.
   const size_t budget = 96 * 1024;
@@ -631,8 +668,14 @@ int softmax_forward_t(SoftmaxArgs<T> a, int64_t deg_max, int max_mult, cudaStrea
 }
 
 template <typename T>
-int softmax_backward_t(SoftmaxArgs<T> a, cudaStream_t stream) {
-  softmax_backward_kernel<T><<<conv_grid(a.n_nodes), CONV_THREADS, a.D * sizeof(ScoreItem), stream>>>(a);
+int softmax_backward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, cudaStream_t stream) {
+  // dk by pairs where targets have many edges, on average or some of them: with few the vector reductions only hold the next
+  // target's loads back.  us by numbers / by pairs: 163 842 points of even degree 12 492 / 552, 40 962 of degree 12 146 / 157, 10 242 of degree 21
+  // 69 / 67, of degree 100 261 / 232; 64 x 128, radius 2 pi / 64 (mean 38, at most 257) 220 / 200; 128 x 256, radius 3 pi / 128 1 051 / 829.
+  const bool pairs = n_edges >= 24 * a.n_nodes || deg_max * a.n_nodes >= 4 * n_edges;
+  auto go = [&](auto kernel) { kernel<<<conv_grid(a.n_nodes), CONV_THREADS, a.D * sizeof(ScoreItem), stream>>>(a); };
+  if (pairs) go(softmax_backward_kernel<T, true>);
+  else go(softmax_backward_kernel<T, false>);
   return launch_status("gm_softmax_backward");
 }
 
@@ -670,7 +713,7 @@ extern "C" int gm_softmax_forward(const void* q, const void* k, const void* tran
     a.q = (const T*)q; a.k = (const T*)k; a.transport = (const T*)transport; a.bias = (const T*)bias;
     a.inside = inside; a.desc = desc; a.row_ptr = row_ptr; a.source = source; a.alpha = (T*)alpha;
     a.n_nodes = n_nodes; a.D = D; a.F = F; a.orders = orders; a.H = H; a.scale = (T)scale;
-    return softmax_forward_t<T>(a, deg_max, max_mult, (cudaStream_t)stream);
+    return softmax_forward_t<T>(a, n_edges, deg_max, max_mult, (cudaStream_t)stream);
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }
@@ -680,7 +723,6 @@ extern "C" int gm_softmax_backward(const void* dalpha, const void* q, const void
                                    const int64_t* source, const void* alpha, int64_t n_nodes, int64_t n_edges, int D,
                                    int F, int orders, int H, double scale, int64_t deg_max, int dtype, void* dq,
                                    void* dk, void* stream) {
-  (void)deg_max;
   int status = check_softmax(q, k, transport, bias, inside, desc, row_ptr, source, n_nodes, n_edges, D, F, orders, H, dtype);
   if (status != GM_OK || n_nodes == 0) return status;
   GM_REQUIRE(dq && dk, GM_ERR_ARGUMENT, "gm_softmax_backward: null output");
@@ -692,7 +734,7 @@ extern "C" int gm_softmax_backward(const void* dalpha, const void* q, const void
     a.inside = inside; a.desc = desc; a.row_ptr = row_ptr; a.source = source;
     a.alpha_in = (const T*)alpha; a.dalpha = (const T*)dalpha; a.dq = (T*)dq; a.dk = (T*)dk;
     a.n_nodes = n_nodes; a.D = D; a.F = F; a.orders = orders; a.H = H; a.scale = (T)scale;
-    return softmax_backward_t<T>(a, (cudaStream_t)stream);
+    return softmax_backward_t<T>(a, n_edges, deg_max, (cudaStream_t)stream);
   };
   return dtype == GM_F32 ? run(float()) : run(double());
 }

@@ -177,6 +177,30 @@ def test_autograd_functions_run_end_to_end(ext):
     assert_close(k.grad.cpu().numpy(), dk_ref, 1e-10, 1e-11, "dk through autograd")
 
 
+@pytest.mark.parametrize("heads, head", [(1, {0: 5}), (2, {0: 4, 1: 4, 2: 4}), (4, {0: 8, 1: 8, 2: 8, 3: 8}), (8, {0: 4, 1: 4, 2: 4, 3: 4}), (4, {0: 20, 1: 16})])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_one_or_two_warps_per_target(ext, heads, head, dtype):
+    """The number of warps that share a target's scores follows the edges per edge of the longest target (a hint to these
+    kernels): both give the same bits, so that chunks equal the whole whatever each is given.  The backward's additions to dk,
+    by numbers or by pairs, agree to the rounding of sums in another order."""
+    c = make_case(24, 40, 3 * math.pi / 24, head, heads, dtype=dtype)
+    q, k = (cuda(x) for x in seeded((c.n_nodes, c.width), 23, dtype, 2))
+    da = cuda(seeded((c.source.shape[0], heads), 24, dtype)[0])
+    tables = [cuda(x) for x in (c.transport, c.bias, c.inside, c.desc, c.row_ptr, c.source)]
+    n_edges = c.source.shape[0]
+    assert 4096 < n_edges <= 4096 * c.max_degree
+    two = ext.softmax_forward(q, k, *tables, heads, c.scale, c.max_degree)
+    one = ext.softmax_forward(q, k, *tables, heads, c.scale, 1)
+    assert torch.equal(one, two) and bool(torch.isfinite(one).all())
+    # a third of the nodes' worth of edges more than 24 a node: by pairs; the same edges as those of many more nodes: by numbers
+    more = torch.cat([tables[4], tables[4][-1:].expand(n_edges)])
+    wide = [torch.cat([x, torch.zeros(n_edges, c.width, dtype=x.dtype, device="cuda")]) for x in (q, k)]
+    pairs = ext.softmax_backward(da, q, k, *tables, two, heads, c.scale, c.max_degree)
+    numbers = ext.softmax_backward(da, *wide, *tables[:4], more, tables[5], two, heads, c.scale, 1)
+    for a, b in zip(pairs, numbers):
+        assert float((a - b[:c.n_nodes]).abs().max()) <= (1e-5 if dtype == np.float32 else 1e-13) * float(a.abs().max())
+
+
 def test_chunked_scores_equal_the_whole_edge_set(ext):
     """Exact chunking over contiguous target ranges (reference ``nn/attention.py:344-402``): every chunk holds whole
     neighbourhoods, its constants are views of the parent's, and the softmax stays a partition of unity inside it --
