@@ -193,7 +193,8 @@ def _refreshed_plan(t: LatticeTables, mode: int, desc: Any, batch: int) -> tuple
     """First records (address) and records of a pass's plan with the entries the tables hold now, on the current stream;
     ``None`` without a plan for this layout, or where the pass is too small for one (the kernels then work it out)."""
     plan = t.tc_plans[mode]
-    if batch * t.rows * t.nlon * t.heads < PLANNED_FROM or plan is None or plan.layout != t.plan_layout() or plan.records.device != t.entries.device:
+    n_rows = (t.t_row_order if mode == 2 else t.row_order).numel()
+    if batch * n_rows * t.nlon * t.heads < PLANNED_FROM or plan is None or plan.layout != t.plan_layout() or plan.records.device != t.entries.device:
         return None, None
     records = torch.empty_like(plan.records)
     entries = (t.t_entries if mode == 2 else t.entries).shape[0]

@@ -89,7 +89,6 @@ struct TcArgs {
   const float* entries;               // (n_entries, 8): (cos, sin) of orders 1..NORD, bias at 2 NORD
   const int* row_order;
   int rows, nlon, D, H, W, NORD;
-  int words;    // rows and owners' / result fields are whole 4-byte words: 4-byte accesses to (even column, next column)
   int even;     // and every block starts on an even column and has an even width: 4-byte accesses throughout
   int padded;   // blocks narrower than 16 (scalar) / 16 KSC (complex) columns
   int unit, units;  // staging: bytes of one copy (16, 8, 4; 2: element by element), copies per head row and field
@@ -102,6 +101,8 @@ struct TcArgs {
   int heavy_tiles, heavy_ctas;                     // row tiles next to the poles, and the CTAs (the first of the grid) that take them
   float scale;
   TcPlan plan;
+  int slots;  // row tiles the grid is made for: all of them, or as many as a short row list can touch
+  int words;    // rows and owners' / result fields are whole 4-byte words: 4-byte accesses to (even column, next column)
 };
 
 enum { TC_FWD = 0, TC_BWD_T = 1, TC_BWD_S = 2 };
@@ -1052,8 +1053,34 @@ __device__ __forceinline__ void pk_cta(const TcArgs& a, int row_tile, int lon_ti
   }
 }
 
+// The x-th row tile, from both ends on, that some row of a short list lies in; -1: there are not that many
+constexpr int PK_LISTED_TILES = 8192;  // lattices with more row tiles have a grid for all of them
+template <int THREADS>
+__device__ __forceinline__ int pk_listed_tile(const int* row_order, int n_order, int row_tiles, int x, unsigned* bits) {
+  const int words = (row_tiles + 31) / 32;
+  for (int w = threadIdx.x; w < words; w += THREADS) bits[w] = 0;
+  __syncthreads();
+  for (int k = threadIdx.x; k < n_order; k += THREADS) {
+    const int row = row_order[k], tile = row / PK_ROWS;
+    if (row < 0 || tile >= row_tiles) continue;
+    const int place = 2 * tile < row_tiles ? 2 * tile : 2 * (row_tiles - 1 - tile) + 1;  // from_both_ends, the other way
+    atomicOr(bits + place / 32, 1u << place % 32);
+  }
+  __syncthreads();
+  int found = -1;
+  for (int w = 0; w < words && found < 0; ++w) {
+    const unsigned have = bits[w];
+    const int n = __popc(have);
+    if (x < n) found = 32 * w + (int)__fns(have, 0, x + 1);
+    x -= n;
+  }
+  __syncthreads();  // the bits' place is used again
+  return found < 0 ? -1 : (int)from_both_ends(found, row_tiles);
+}
+
 template <int KS0, int NCF, int KSC, int MODE, int WARPS, bool PLANNED>
 __global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_kernel(const __grid_constant__ TcArgs a) {
+  extern __shared__ __align__(16) unsigned char smem[];
   constexpr int TLON = 8 * (WARPS / PK_ROWS);
   // which tile, which (sample, head) pairs: the first heavy_ctas CTAs take the row tiles next to the poles
   const int lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
@@ -1069,12 +1096,18 @@ __global__ void __launch_bounds__(32 * WARPS, pk_ctas(WARPS)) lattice_packed_ker
     x -= a.heavy_ctas;
     lon_tile = x % lon_tiles;
     x /= lon_tiles;
-    const int light = row_tiles - a.heavy_tiles;
+    const int light = a.slots - a.heavy_tiles;
     row_tile = a.heavy_tiles + x % light;
     bh = (x / light) * a.light_bh;
     bh_end = min(bh + a.light_bh, a.n_bh);
   }
-  pk_cta<KS0, NCF, KSC, MODE, WARPS, PLANNED>(a, (int)from_both_ends(row_tile, row_tiles), lon_tile, bh, bh_end);
+  if (a.slots == row_tiles) {
+    row_tile = (int)from_both_ends(row_tile, row_tiles);
+  } else {
+    row_tile = pk_listed_tile<32 * WARPS>(a.row_order, a.n_order, row_tiles, row_tile, reinterpret_cast<unsigned*>(smem));
+    if (row_tile < 0) return;
+  }
+  pk_cta<KS0, NCF, KSC, MODE, WARPS, PLANNED>(a, row_tile, lon_tile, bh, bh_end);
 }
 
 // The row tiles whose windows are not the ones the plan was made from, behind the planned launch (to which their records were
@@ -1240,9 +1273,14 @@ int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
   const int64_t lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
   const int64_t n_bh = (int64_t)a.H * batch, slots = (int64_t)sm_count() * pk_ctas(WARPS);
   GM_REQUIRE(n_bh < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_attention (tensor cores): too many (sample, head) pairs");
+  // a list of a few rows (a band's next to its halo): CTAs for the tiles it can touch.  256 x 512, batch 2, 4 heads of 16 x (m <= 2),
+  // three rows, forward / pass T / pass S: 25 / 45 / 45 us (CTAs for all tiles, most of them idle:
+  // 59 / 99 / 125)
+  const int64_t listed = n_order_rows < row_tiles && row_tiles <= PK_LISTED_TILES ? n_order_rows : row_tiles;
+  a.slots = (int)listed;
   int64_t heavy_tiles = 2 * ((2 * a.W + 2 + PK_ROWS - 1) / PK_ROWS);
-  if (heavy_tiles > row_tiles) heavy_tiles = row_tiles;
-  const int64_t light_tiles = (row_tiles - heavy_tiles) * lon_tiles;
+  if (heavy_tiles > listed) heavy_tiles = listed;
+  const int64_t light_tiles = (listed - heavy_tiles) * lon_tiles;
   auto pairs_per_cta = [&](int64_t tiles, int64_t waves, int64_t most) {
     int64_t n = tiles * n_bh / (slots * waves);
     n = n < 1 ? 1 : n > most ? most : n;

@@ -524,3 +524,38 @@ def test_fields_on_odd_addresses(head):
         places = [odd(x) if i + 4 in moved else x for i, x in enumerate(results)]
         for a, b in zip(run(fields, places), want):
             assert torch.equal(a, b), moved
+
+
+@pytest.mark.parametrize("planned_from", [0, 1 << 40])
+def test_short_row_lists(planned_from, monkeypatch):
+    """Lists with fewer rows than the lattice has row tiles (whose grid is made for the tiles they can touch): rows of one tile
+    and of several, out of order, at both poles and in the last, partial tile give the bits of the whole call; other rows
+    keep what they held."""
+    import dataclasses
+
+    from gm_attention_b200 import attention
+    from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
+
+    monkeypatch.setattr(attention, "PLANNED_FROM", planned_from)
+    rows, nlon, batch = 37, 24, 2
+    c = make_case(rows, nlon, 2 * math.pi / rows, {0: 8, 1: 8}, 2, dtype=np.float32)
+    Q, K, V, G = (torch.from_numpy(x).bfloat16().cuda() for x in seeded((batch * c.n_nodes, c.width), 67, np.float32, 4))
+    _, lat = tables_for(c)
+    out, lse = lattice_attention_forward(Q, K, V, lat, tensor_cores=True)
+    whole = lattice_attention_backward(G, Q, K, V, out, lse, lat, tensor_cores=True)
+    banded = lambda x: x.view(batch, rows, nlon, -1)
+    for listed in ([36], [0], [17], [36, 0], [9, 8, 11], [20, 5, 6, 33, 2], [0, 1, 2, 3, 4, 35, 36, 18, 19]):
+        order = torch.tensor(listed, dtype=torch.int32, device="cuda")
+        part = dataclasses.replace(lat, row_order=order, t_row_order=order)
+        got = lattice_attention_forward(Q, K, V, part, tensor_cores=True, out=torch.full_like(out, 7.0), lse=torch.full_like(lse, 7.0))
+        places = tuple(torch.full_like(Q, 7.0) for _ in range(3)) + (torch.full_like(lse, 7.0),)
+        lattice_attention_backward(G, Q, K, V, out, lse, part, tensor_cores=True, passes=3, workspace=places)
+        delta = places[3].clone()
+        full_delta = torch.empty_like(lse)
+        lattice_attention_backward(G, Q, K, V, out, lse, lat, tensor_cores=True, passes=1, workspace=places[:3] + (full_delta,))
+        lattice_attention_backward(G, Q, K, V, out, lse, part, tensor_cores=True, passes=4, workspace=places[:3] + (full_delta,))
+        other = [r for r in range(rows) if r not in listed]
+        for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), (*got, *places[:3]), (out, lse, *whole)):
+            assert torch.equal(banded(a)[:, listed], banded(b)[:, listed]), (name, listed)
+            assert bool((banded(a)[:, other] == 7.0).all()), (name, listed)
+        assert bool((banded(delta)[:, other] == 7.0).all())
