@@ -722,16 +722,12 @@ def row_pair_counts(lattice, radius: float) -> Tensor:
 
 def tensor_core_row_cost(pair_counts: Tensor) -> list[float]:
     """Relative cost of one lattice row under the tensor-core lattice kernels (forward + both backward passes).
-    A warp owns 8 consecutive owners and walks, for every neighbour row, the 7 + cnt positions their windows cover in
-    steps of 16; a CTA stages the neighbour row in chunks and pays a fixed cost per owner tile.  The weights are a
-    fit to measured times of row groups from the pole to the equator of a 256 x 512 lattice (within 15 % for every
-    group; the bands of an 8-way split, each timed alone, come out within 3 % of one another).  Narrow equatorial
-    windows cost several times more PER EDGE than whole-row polar windows, which an edge-count balance ignores.  The constant
-    per row was re-fitted on a 4-way split (bands [0, 40), [40, 128) and their mirror images timed side by side: with the
-    constant at 10 the equatorial bands took 4.08 ms against 3.90 ms for the polar ones)."""
+    A warp owns 8 consecutive owners and walks the 7 + cnt positions their windows cover in every neighbour row, packed into
+    steps of 16; a CTA stages the neighbourhood of four rows and pays a fixed cost per owner tile.  The weights are a fit to
+    measured times of row groups from the pole to the equator of a 256 x 512 lattice (batch 8, 4 heads of 16 x (m <= 2), 8 rows
+    from either end: 4 400 us next to the poles, 1 594, 1 228, 1 066, 972 ... 671 at the equator), within 10 % for every group (18 % for
+    the polar group of a 128 x 256 lattice).  Narrow equatorial windows cost several times more PER EDGE than whole-row polar
+    windows, which an edge-count balance ignores."""
     cnt = pair_counts.to(torch.float64)
-    present = cnt > 0
-    steps = torch.ceil((7 + cnt) / 16)
-    chunks = torch.ceil((63 + cnt) / 80) + torch.ceil((31 + cnt) / 80)
-    cost = torch.where(present, 7.1 * steps + 2.9 * chunks, torch.zeros_like(cnt))
-    return (14.5 + cost.sum(1)).tolist()
+    positions = torch.where(cnt > 0, 7 + cnt, torch.zeros_like(cnt)).sum(1)
+    return (18.4 + 5.3 * positions / 16).tolist()
