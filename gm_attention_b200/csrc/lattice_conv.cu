@@ -14,8 +14,9 @@
 //               windows and M^T it is the gradient with respect to the node field)
 //   table_grad  dM[entry] = sum over longitudes l and samples  dy[i, l] (x) x[j, l + lo + d]
 //
-// apply and table_grad are FMA-bound, not HBM-bound (4 multiply-adds per complex copy, edge and sample against 0.01 bytes of compulsory
-// traffic), and neither has a contraction over channels, so there is nothing for the tensor cores here.  A thread owns
+// apply and table_grad are bound by arithmetic, not HBM (4 multiply-adds per complex copy, edge and sample against 0.01 bytes of
+// compulsory traffic).  bfloat16 fields whose rows are whole 16-byte words have tensor-core kernels (lattice_conv_tc.cu), taken where
+// they are the faster ones; the kernels here, on the FMA pipe, serve everything else.  A thread owns
 // one item -- a complex copy, or a pair of scalar channels -- so a warp reads 32 neighbouring items of a node as one
 // 128-byte line; it keeps 8 longitudes x 2 samples of accumulators in registers and slides a register window of 8
 // source longitudes (apply) or 8 target longitudes (table_grad) past them, so every loaded value is used for 8 x 4

@@ -153,10 +153,10 @@ def test_lattice_through_autograd_and_unsupported_layout():
     assert lattice_layout_supported(lat.desc_rows)
 
 
-#: headline head layout on a lattice wide enough for the TMA staging path: tiles that wrap the longitude seam and
+#: headline head layout on a wide lattice: every unit of staging, tiles that wrap the longitude seam and
 #: tiles that do not, windows from a few positions (one staged chunk) to whole rows (several chunks)
-TMA_CASE = (6, 256, 1.2 * math.pi / 6, {0: 16, 1: 16, 2: 16}, 2, "hard", 2)
-TC_CASES = [CASES[0], CASES[1], CASES[2], CASES[3], CASES[4], (8, 16, 2 * math.pi / 8, {1: 6, 2: 6}, 1, "hard", 2), TMA_CASE]
+STAGING_CASE = (6, 256, 1.2 * math.pi / 6, {0: 16, 1: 16, 2: 16}, 2, "hard", 2)
+TC_CASES = [CASES[0], CASES[1], CASES[2], CASES[3], CASES[4], (8, 16, 2 * math.pi / 8, {1: 6, 2: 6}, 1, "hard", 2), STAGING_CASE]
 
 
 @pytest.fixture(params=["one-head", "four-heads"])
@@ -266,8 +266,8 @@ def test_tensor_core_backward_ignores_stale_shared_memory():
     whatever an earlier kernel left in shared memory (here NaN, on every SM) must not reach the sums."""
     from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
 
-    batch = TMA_CASE[6]
-    c = make_case(*TMA_CASE[:5], dtype=np.float32, window=TMA_CASE[5])
+    batch = STAGING_CASE[6]
+    c = make_case(*STAGING_CASE[:5], dtype=np.float32, window=STAGING_CASE[5])
     _, lat = tables_for(c)
     Q, K, V, G = (torch.from_numpy(x).bfloat16().cuda() for x in seeded((batch * c.n_nodes, c.width), 58, np.float32, 4))
     out, lse = lattice_attention_forward(Q, K, V, lat, tensor_cores=True)
@@ -280,29 +280,25 @@ def test_tensor_core_backward_ignores_stale_shared_memory():
             assert bool(torch.isfinite(got.float()).all()), name
 
 
-def test_tma_staging_equals_per_thread_staging(monkeypatch):
-    """The two staging paths of the tensor-core kernels (TMA tensor copies; per-thread cp.async) feed the same
-    arithmetic: results are bit-identical, and no wait on a copy barrier ever ran out."""
-    import ctypes
-
-    from gm_attention_b200 import _lib
+@pytest.mark.parametrize("offset", [4, 2, 1])
+def test_staging_in_units_of_every_size(offset):
+    """Neighbour rows are staged in copies of 16, 8, 4 or 2 bytes, as the fields' addresses allow (here views at an element
+    offset of 0, 4, 2, 1): the same arithmetic on the same values, bit for bit."""
     from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
 
-    batch = TMA_CASE[6]
-    c = make_case(*TMA_CASE[:5], dtype=np.float32, window=TMA_CASE[5])
+    batch = STAGING_CASE[6]
+    c = make_case(*STAGING_CASE[:5], dtype=np.float32, window=STAGING_CASE[5])
     _, lat = tables_for(c)
-    Q, K, V, G = (torch.from_numpy(x).bfloat16().cuda() for x in seeded((batch * c.n_nodes, c.width), 60, np.float32, 4))
-    results = {}
-    for mode in ("1", "0"):
-        monkeypatch.setenv("GM_LATTICE_TMA", mode)
+    fields = [torch.from_numpy(x).bfloat16().cuda() for x in seeded((batch * c.n_nodes, c.width), 60, np.float32, 4)]
+    moved = [torch.empty(x.numel() + offset, dtype=x.dtype, device="cuda")[offset:].view(x.shape).copy_(x) for x in fields]
+    assert all(x.data_ptr() % 16 == 0 for x in fields) and all(x.data_ptr() % 16 == 2 * offset for x in moved)
+    results = []
+    for Q, K, V, G in (fields, moved):
         out, lse = lattice_attention_forward(Q, K, V, lat, tensor_cores=True)
-        results[mode] = (out, lse, *lattice_attention_backward(G, Q, K, V, out, lse, lat, tensor_cores=True))
-    for a, b in zip(results["1"], results["0"]):
-        assert torch.equal(a, b)
-    assert torch.isfinite(results["1"][0].float()).all()
-    expired = ctypes.c_int(-1)
-    _lib.call("gm_lattice_attention_tc_wait_expired", ctypes.byref(expired))
-    assert expired.value == 0
+        results.append((out, lse, *lattice_attention_backward(G, Q, K, V, out, lse, lat, tensor_cores=True)))
+    for x, y in zip(*results):
+        assert torch.equal(x, y)
+    assert torch.isfinite(results[0][0].float()).all()
 
 
 def test_host_pipeline_equals_the_device_path():
