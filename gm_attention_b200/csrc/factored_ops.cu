@@ -38,7 +38,9 @@ constexpr int MAX_OWNED = 64;      // K * C <= 64 * 128 in the backward
 // A tile of 64 edges while six CTAs of it share an SM, 32 beyond: a wide packed row (13 blocks to {4, 4, 4}: 100 columns, 53 KB at
 // 64 edges) leaves four CTAs' warps to hide the barriers, a narrow one (18 columns) pays them twice as often for nothing.
 // 128 x 256, radius 3 pi / 128, 100 columns: forward 1 309 us with 64 edges, 1 034 with 32, 1 122 with 16; backward 2 494, 2 460, 3 076.
-// Narrow rows lose with 32: 118 x 236, radius 4 pi / 118, 18 columns, the pass 4.08 -> 4.50 ms.
+// Narrow rows lose with 32: 118 x 236, radius 4 pi / 118, 18 columns, the pass 4.08 -> 4.50 ms.  Between: the pass at 64 x 128, radius
+// 3 pi / 64, 13 blocks to {2, 2, 2} (50 columns) 984 -> 988 us, to {8, 8, 8} (200) 2 546 -> 1 874.  float64, whose rows are twice as
+// wide: 18 columns 994 -> 992, 36 3 160 -> 2 497 (radius 4), 50 1 660 -> 1 458, 100 2 637 -> 2 187, 200 5 948 -> 4 220.
 constexpr size_t FSMEM_SIXTH = 227 * 1024 / 6 - 1024;
 constexpr size_t FSMEM_MOST = 224 * 1024;  // dynamic shared memory a CTA may ask for, beside the static arrays
 constexpr int TP = 5;              // rows t of a dZ patch (4 columns wide)

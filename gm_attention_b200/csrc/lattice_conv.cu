@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(THREADS, 3) conv_apply_kernel(const ConvArgs a
 // (the matrix, duplicated into pairs) and 6 NB of loads, conversions and window moves.  Same order of operations per
 // output as conv_apply_kernel: bit-identical results.  256 x 512, radius 4 pi / 256, batch 4, 64 x (m <= 2), bf16: 7.92 ms
 // with conv_apply_kernel, 4.51 in this form (FMA pipe about 40 % busy, 10 warps' barriers and the per-stage set-up beside
-// it); 45 x 88, batch 3, 32 x (m <= 2), float32: 220 us before, 128 now.
+// it; a field of that size takes the tensor cores now); 45 x 88, batch 3, 32 x (m <= 2), float32: 220 us before, 128 now.
 struct StagedShape {
   int tiles, so, threads, stage_bytes, pos_bytes;  // G, SO, G * n_items, bytes of a stage, bytes of one node's row
   int vec16;                                       // rows and bases are multiples of 16 bytes
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(128) conv_fold_kernel(const FoldArgs a) {
 
 // Tiles, offsets per stage and samples per thread of the staged apply kernel; returns the samples, 0 where it cannot run.
 // Two samples and two CTAs of 320 threads per SM (88 to 95 registers) measured 4.5 ms against 4.7 for four samples and one CTA,
-// 5.8 to 6.0 for CTAs of one tile (256 x 512, batch 4, 64 x (m <= 2), bf16).  A stage should hold the equator's windows
+// 5.8 to 6.0 for CTAs of one tile (256 x 512, batch 4, 64 x (m <= 2), bf16, which takes the tensor cores now).  A stage should hold the equator's windows
 // whole: where half of the shared memory holds fewer than 8 offsets (float32 rows of 320 columns: 3) a CTA takes all of it.
 // Tiles: as many as 320 threads take, fewer while the launch has less than two CTAs per SM (a small lattice waits for
 // its polar rows' chains of offsets).
