@@ -36,12 +36,12 @@
 // bank conflicts) while this pair's results are written.  Neighbourhoods that outgrow shared memory -- the polar rows' -- come
 // in chunks.  The lists depend on the windows alone: gm_lattice_plan_build works them out once per table, gm_lattice_plan_refresh
 // adds the entries in front of every pass, and a CTA copies both; a row tile whose windows are no longer the plan's, and every CTA
-// without a plan, works them out itself (128 x 256, batch 4, 8 x (m <= 3): 2 050 against 1 731 us for the three passes).
+// without a plan, works them out itself (128 x 256, batch 4, 8 x (m <= 3): 1 953 against 1 670 us for the three passes).
 // Tensor-core instruction: mma.sync m16n8k16 (bf16 inputs, fp32 accumulate).
 //
 // What it measured against the kernel before it (one row of 32 longitudes and one (sample, head) per CTA, a step per
 // neighbour row, TMA staging), us forward / pass T / pass S: 128 x 256, batch 4, 4 heads of 8 x (m <= 3): 603 / 904 / 995 ->
-// 436 / 595 / 700; 256 x 512, batch 8, 4 heads of 16 x (m <= 2): 3 670 / 4 896 / 6 643 -> 3 370 / 4 609 / 6 152; heads that
+// 433 / 560 / 677; 256 x 512, batch 8, 4 heads of 16 x (m <= 2): 3 670 / 4 896 / 6 643 -> 3 358 / 4 648 / 6 163; heads that
 // are not 16 copies wide, batch 1 to 8: 1.2 to 4 times faster.  What bounds it: of the last forward 2.1 ms are the steps
 // (shared-memory bandwidth: ten ldmatrix.x4 and the entries, about 100 of 114 cycles a step), 1.4 ms the staging and the
 // per-pair prologue and epilogue, which overlap only across the SM's two CTAs.  16 longitudes per CTA pay in the forward
@@ -1269,7 +1269,11 @@ int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
   const size_t smem = chunk_caps<KS0, NCF, KSC, WARPS>(a.rows, a.nlon, a.W, a.caps);
   a.record_bytes = pk_record_bytes(a.caps, WARPS, a.W, NCF);
   // Polar rows see whole rings: their tiles start first and hold few (sample, head) pairs each.  Elsewhere a CTA takes as
-  // many pairs as leave a few waves of CTAs, up to 16: lists and entries are made once for all of them.
+  // many pairs as leave a few waves of CTAs, up to 16: lists and entries are made once for all of them.  Pass T, us, with
+  // 6 waves (24 and at most 2 pairs next to the poles) / 4 (12, 4) / 4 (8, 4) / 2 (12, 2): 128 x 256, batch 4, 8 x (m <= 3) 587 / 560 / 552 / 605;
+  // 91 x 180, batch 3, 16 x (m <= 2) 218 / 206 / 206 / 208; 100 x 200, batch 5, 8 heads 681 / 666 / 667 / 700; 200 x 100, batch 4 237 / 239 / 239 / 239;
+  // 256 x 512, batch 8 4 645 / 4 648 / 4 660 / 4 647; its upper half alone, batch 1, where the polar CTAs' four pairs in turn are the
+  // launch, 351 / 349 / 405; forward at 180 x 360, batch 2 491 / 499 / 493 / 509.
   const int64_t lon_tiles = (a.nlon + TLON - 1) / TLON, row_tiles = (a.rows + PK_ROWS - 1) / PK_ROWS;
   const int64_t n_bh = (int64_t)a.H * batch, slots = (int64_t)sm_count() * pk_ctas(WARPS);
   GM_REQUIRE(n_bh < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_attention (tensor cores): too many (sample, head) pairs");
@@ -1281,6 +1285,7 @@ int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
   int64_t heavy_tiles = 2 * ((2 * a.W + 2 + PK_ROWS - 1) / PK_ROWS);
   if (heavy_tiles > listed) heavy_tiles = listed;
   const int64_t light_tiles = (listed - heavy_tiles) * lon_tiles;
+  const int64_t busy_tiles = std::min<int64_t>(listed, (n_order_rows + PK_ROWS - 1) / PK_ROWS) * lon_tiles;  // of a longer list: about as many have work
   auto pairs_per_cta = [&](int64_t tiles, int64_t waves, int64_t most) {
     int64_t n = tiles * n_bh / (slots * waves);
     n = n < 1 ? 1 : n > most ? most : n;
@@ -1288,8 +1293,8 @@ int launch_tn(TcArgs& a, int n_order_rows, int64_t batch, cudaStream_t stream) {
     return (int)((n_bh + chunks - 1) / chunks);
   };
   a.n_bh = (int)n_bh;
-  a.light_bh = pairs_per_cta(light_tiles, 6, 16);
-  a.heavy_bh = pairs_per_cta(light_tiles + heavy_tiles * lon_tiles, 24, 2);
+  a.light_bh = pairs_per_cta(std::min(light_tiles, busy_tiles), 4, 16);
+  a.heavy_bh = pairs_per_cta(busy_tiles, 12, 4);
   a.heavy_tiles = (int)heavy_tiles;
   const int64_t heavy = heavy_tiles * lon_tiles * ((n_bh + a.heavy_bh - 1) / a.heavy_bh);
   const int64_t light = light_tiles * ((n_bh + a.light_bh - 1) / a.light_bh);
