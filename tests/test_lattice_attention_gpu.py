@@ -555,3 +555,33 @@ def test_short_row_lists(planned_from, monkeypatch):
             assert torch.equal(banded(a)[:, listed], banded(b)[:, listed]), (name, listed)
             assert bool((banded(a)[:, other] == 7.0).all()), (name, listed)
         assert bool((banded(delta)[:, other] == 7.0).all())
+
+
+def test_plans_of_another_format_or_layout_are_not_used(monkeypatch):
+    """Plans that were saved with another record format, or for another head count, lattice or halo, are left alone (their
+    records, here of no use to anyone, are never read): the kernels pack their own lists."""
+    import dataclasses
+
+    from gm_attention_b200 import _lib, attention
+    from gm_attention_b200.attention import lattice_attention_backward, lattice_attention_forward
+
+    monkeypatch.setattr(attention, "PLANNED_FROM", 0)
+    c = make_case(9, 24, 2 * math.pi / 9, {0: 8, 1: 8}, 2, dtype=np.float32)
+    Q, K, V, G = (torch.from_numpy(x).bfloat16().cuda() for x in seeded((c.n_nodes, c.width), 68, np.float32, 4))
+    _, lat = tables_for(c)
+
+    def run(t):
+        before = _lib.CALLS["gm_lattice_plan_refresh"]
+        out, lse = lattice_attention_forward(Q, K, V, t, tensor_cores=True)
+        return (out, lse, *lattice_attention_backward(G, Q, K, V, out, lse, t, tensor_cores=True)), _lib.CALLS["gm_lattice_plan_refresh"] - before
+
+    want, refreshed = run(lat)
+    assert refreshed == 3
+    tag, desc, heads, rows, nlon, halo, orders = lat.plan_layout()
+    for layout in ((tag - 1, desc, heads, rows, nlon, halo, orders), (desc, heads, rows, nlon, halo, orders), (tag, desc, heads + 1, rows, nlon, halo, orders),
+                   (tag, desc, heads, rows, nlon, halo + 1, orders)):
+        other = tuple(dataclasses.replace(p, layout=layout, records=torch.full_like(p.records, 255)) for p in lat.tc_plans)
+        got, refreshed = run(dataclasses.replace(lat, tc_plans=other))
+        assert refreshed == 0
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
