@@ -533,15 +533,18 @@ bool tensor_cores_can(const ConvArgs& a) {
 //                width 96: 259 / 170; 45 x 88, width 40: 72 / 66).  Wide fields fill the chip with one sample, and then it is padding
 //                that decides (256 x 512, width 320: 848 / 604; 64 x 128, batch 2, width 320: 174 / 199).
 //   table_grad   contracts over the tiles, 16 a step: 23 tiles and more are always faster (91 x 184, batch 1, width 80: 75 / 58; 128 x
-//                256, width 24: 99 / 50), 11 with four samples in sequence (45 x 88, width 96: 48 / 32; batch 1, width 160: 30 / 44), fewer
-//                by the shape (100 x 48, batch 4, width 24: 28 / 32; 24 x 48: 26 / 17).
+//                256, width 24: 99 / 50), 16 with four samples in sequence (64 x 128, width 320: 270 / 239; batch 2: 143 / 175), 9 to 15 then
+//                where the field is not wide (45 x 88, width 80: 60 / 57, width 320: 132 / 159; 100 x 104: 105 / 103 and 224 / 307).  One
+//                block of 32 columns, for which the FMA kernel has less than a warp of items, from 8 tiles on (64 x 64: 22 / 20; 45 x 88:
+//                26 / 19); fewer tiles go either way (100 x 48, batch 4: 28 / 32; 24 x 48: 26 / 17).
 bool tensor_cores_apply(const ConvArgs& a) {
   const int tiles = a.nlon / 8;
   return tensor_cores_can(a) && tiles > 8 && (a.width < 256 ? a.batch >= 2 : tiles >= 32);
 }
 bool tensor_cores_table_grad(const ConvArgs& a) {
   const int tiles = a.nlon / 8;
-  return tensor_cores_can(a) && (tiles >= 20 || (tiles > 8 && a.batch >= 4));
+  const bool pays = tiles >= 20 || (tiles >= 8 && a.width <= TC_COLS) || (a.batch >= 4 && (tiles >= 16 || (tiles > 8 && a.width <= 96)));
+  return tensor_cores_can(a) && pays;
 }
 
 int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream) {
