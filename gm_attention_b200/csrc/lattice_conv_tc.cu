@@ -14,40 +14,50 @@
 // no chain is longer than one k-step (8 positions): its sum is added in float32, rounded to nearest.  Root mean square error
 // against float64 of sums of N(0, 1) terms that cancel, one chain through all windows / this way / the FMA kernel's single
 // additions: rings of 512, terms in order of size 9.5e-4 / 4.9e-5 / 1.3e-4, in random order 1.3e-4 / 6.0e-6 / 1.7e-5; 24 x 48, radius
-// 2.5 pi / 24, 6.4e-6 / 1.1e-6 / 3.2e-6 and 2.1e-6 / 4.3e-7 / 1.1e-6.  It costs a fifth of apply's time (256 x 512, radius
-// 2 pi / 256, 64 x (m <= 2): 322 -> 406 us; by the FMA kernel 469).
+// 2.5 pi / 24, 6.4e-6 / 1.1e-6 / 3.2e-6 and 2.1e-6 / 4.3e-7 / 1.1e-6.  It cost a fifth of the time of apply as
+// it was first.
 //
-// In shared memory a node's 32 columns (64 bytes) sit at [position % 8][position / 8], rows of 80 bytes: a lane reads four
-// channel pairs of one position with one 16-byte load, the lanes of a load on different banks.  The (re, im) words are B
-// fragments of apply as they are; table_grad contracts over positions and pairs the words of t and t + 1 with two byte
-// permutations.
+// A CTA is four producer warps and four consumer warps (named barriers, registers 56 / 200 a thread).  The producers copy the
+// positions and, for apply, fetch, split and place the table; the consumers multiply.  With every warp doing both (8 or 12 warps an
+// SM), a CTA's copies, table entries and products followed each other and the tensor pipe stood at 34 %: 256 x 512, radius
+// 4 pi / 256, batch 4, 64 x (m <= 2): apply 3 230 us, 2 475 with stages handed over by one barrier and cut by positions instead of
+// offsets, 2 010 with producers; table_grad 2 440, 2 000 with producers.  128 x 256, batch 2: 502 -> 269 and 439 -> 345; 45 x 88, batch 3, 32 x (m <= 2): 104
+// -> 46 and 75 -> 60.  What bounds them now: the producers alone take 1 490 / 1 420 us, the consumers alone 1 590 / 1 400 (their
+// products 880 / 300, their shared-memory reads 740 / 400), and they share the load / store unit.
+//
+// In shared memory the positions 8 t + e of a plane e follow each other, so that a lane reads four channel pairs of one position
+// with one 16-byte load, the eight lanes of a phase on different banks.  The (re, im) words are B fragments of apply as they are;
+// table_grad contracts over positions and pairs the words of t and t + 1 with two byte permutations.
+#include <algorithm>
+
 #include "lattice_conv.cuh"
 
 namespace gmb {
 namespace lconv {
 namespace {
 
-constexpr int TC_THREADS = 256;         // 8 warps: 4 groups of 4 channel pairs x 2
-constexpr int TC_COLS = 32;             // columns of the field per CTA
-constexpr int TC_PAIRS = TC_COLS / 2;   // channel pairs
-constexpr int TC_PITCH = 5;             // 16-byte words per staged position (4 and one of padding)
-
 __device__ __forceinline__ void mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_first(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {  // d = a * b
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};\n"
+__device__ __forceinline__ void mma_first(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1,
+                                          const float (&zero)[4]) {  // d = a * b
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
                : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(zero[0]), "f"(zero[1]), "f"(zero[2]), "f"(zero[3]));
 }
-// d += a * b with the addition to d rounded to nearest
-__device__ __forceinline__ void mma_add(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  float p[4];
-  mma_first(p, a[0], a[1], a[2], a[3], b0, b1);
-#pragma unroll
-  for (int x = 0; x < 4; ++x) d[x] += p[x];
+// Two float32 sums in one 64-bit register pair
+using f32x2 = unsigned long long;
+__device__ __forceinline__ void add2(f32x2& d, float x, float y) {
+  f32x2 v;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
+  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(v));
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
 }
 // 16 bytes global -> shared, asynchronously; bytes = 0 writes zeros
 __device__ __forceinline__ void copy16(uint4* dst, const void* src, int bytes) {
@@ -57,52 +67,108 @@ __device__ __forceinline__ void copy16(uint4* dst, const void* src, int bytes) {
 __device__ __forceinline__ void commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N> __device__ __forceinline__ void wait_copies() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// Staged copies of `count` positions from longitude `lon` of a row (cyclic) on: position q to [q % 8][q / 8], SP 16-byte words
-// between the eight.  Columns beyond the field's are zeros.
-template <int SP>
+// Where the positions e, 8 + e, 16 + e, ... start, in 16-byte words
+template <int SP, bool SKEW> __device__ __forceinline__ int plane(int e) { return e * SP + (SKEW ? (e & 1) + 2 * (e & 2) : 0); }
+
+// Staged copies of `count` positions from longitude `lon` of a row (cyclic) on, WORDS 16-byte words each: position q to
+// [q % 8][q / 8], SP words between the eight, PITCH between positions.  Columns beyond the field's are zeros.
+template <int THREADS, int WORDS, int SP, int PITCH, bool SKEW>
 __device__ __forceinline__ void stage_positions(uint4* dst, const unsigned char* row, int lon, int count, int nlon, int row_bytes, int col_byte) {
-  const int k = threadIdx.x & 3, byte = col_byte + 16 * k;
+  constexpr int PASS = THREADS / WORDS;
+  const int first = threadIdx.x % THREADS / WORDS, k = threadIdx.x % WORDS, byte = col_byte + 16 * k;
   const bool in = byte < row_bytes;
   const unsigned char* src = row + (in ? byte : 0);
-  int at = lon + ((int)threadIdx.x >> 2);
+  int at = lon + first;
   while (at >= nlon) at -= nlon;
-  const int step = (TC_THREADS / 4) % nlon;
-  for (int q = threadIdx.x >> 2; q < count; q += TC_THREADS / 4) {
-    copy16(dst + (q & 7) * SP + (q >> 3) * TC_PITCH + k, src + (size_t)at * row_bytes, in ? 16 : 0);
+  int step = PASS;
+  while (step >= nlon) step -= nlon;
+  static_assert(PASS % 8 == 0, "a thread's positions lie in one plane");
+  dst += plane<SP, SKEW>(first & 7) + k;
+  for (int q = first; q < count; q += PASS) {
+    copy16(dst + (q >> 3) * PITCH, src + (size_t)at * row_bytes, in ? 16 : 0);
     at += step;
     if (at >= nlon) at -= nlon;
   }
 }
 
+// ---- producers and consumers: a CTA is two groups of 128 threads.  The producers fill stages in shared memory, the consumers
+// multiply; a stage's named barriers say that it is there (the producers arrive, the consumers wait) and that its buffer is free
+// (the other way round).  Both walk the same list of stages, so every arrival is met.
+constexpr int GROUP = 128;
+constexpr int BAR_CONSUMERS = 1, BAR_STAGES = 2;  // ids: the consumers among themselves; then (full, empty) of every buffer
+__device__ __forceinline__ void barrier_sync(int id) { asm volatile("bar.sync %0, %1;\n" ::"r"(id), "n"(2 * GROUP) : "memory"); }
+__device__ __forceinline__ void barrier_arrive(int id) { asm volatile("bar.arrive %0, %1;\n" ::"r"(id), "n"(2 * GROUP) : "memory"); }
+__device__ __forceinline__ int full_barrier(int buf) { return BAR_STAGES + 2 * buf; }
+__device__ __forceinline__ int empty_barrier(int buf) { return BAR_STAGES + 2 * buf + 1; }
+__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync %0, %1;\n" ::"n"(BAR_CONSUMERS), "n"(GROUP) : "memory"); }
+__device__ __forceinline__ bool consumer_or(bool x) {
+  unsigned any;
+  asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 p, %1, 0;\nbar.red.or.pred q, %2, %3, p;\nselp.u32 %0, 1, 0, q;\n}\n"
+               : "=r"(any) : "r"((unsigned)x), "n"(BAR_CONSUMERS), "n"(GROUP) : "memory");
+  return any != 0;
+}
+// The launch's 128 registers a thread (256 threads, two CTAs an SM) split over the groups: 56 + 200
+__device__ __forceinline__ void producer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 56;\n"); }
+__device__ __forceinline__ void consumer_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 200;\n"); }
+// The producers' way through `BUFFERS` stages in turn, up to FLIGHT of them being copied at a time
+template <int BUFFERS, int FLIGHT>
+struct Ring {
+  int n = 0, buf = 0;
+  template <int PENDING>
+  __device__ __forceinline__ void finish() const {  // the stage issued before the PENDING last is complete
+    if (n <= PENDING) return;
+    wait_copies<PENDING>();
+    barrier_arrive(full_barrier(buf > PENDING ? buf - PENDING - 1 : buf + BUFFERS - PENDING - 1));
+  }
+  __device__ __forceinline__ void begin() const {  // hand over the oldest stage, wait for a free buffer
+    finish<FLIGHT - 1>();
+    if (n >= BUFFERS) barrier_sync(empty_barrier(buf));
+  }
+  __device__ __forceinline__ void advance() {
+    ++n;
+    buf = buf == BUFFERS - 1 ? 0 : buf + 1;
+  }
+  __device__ __forceinline__ void drain() const {  // hand over the rest, meet the consumers' last arrivals
+    if constexpr (FLIGHT > 1) finish<1>();
+    finish<0>();
+    const int open = min(n, BUFFERS);
+    for (int x = 0; x < open; ++x) barrier_sync(empty_barrier((n - open + x) % BUFFERS));
+  }
+  static_assert(FLIGHT <= 2 && FLIGHT < BUFFERS + 1, "");
+};
+
 struct PairItem {
   int kind, fcol;  // -1: no item on these columns
 };
+template <int COLS, int THREADS>
 __device__ __forceinline__ void find_items(const ConvArgs& a, int col0, PairItem* pairs_s) {
-  if (threadIdx.x < TC_PAIRS) pairs_s[threadIdx.x] = PairItem{-1, 0};
+  if (threadIdx.x < COLS / 2) pairs_s[threadIdx.x] = PairItem{-1, 0};
   __syncthreads();
-  for (int x = threadIdx.x; x < a.n_items; x += TC_THREADS) {
+  for (int x = threadIdx.x; x < a.n_items; x += THREADS) {
     const int col = a.items[3 * x + 1] - col0;
-    if (col >= 0 && col < TC_COLS) pairs_s[col >> 1] = PairItem{a.items[3 * x], a.items[3 * x + 2]};
+    if (col >= 0 && col < COLS) pairs_s[col >> 1] = PairItem{a.items[3 * x], a.items[3 * x + 2]};
   }
   __syncthreads();
 }
 
 // ----------------------------------------------------------------------------------------------------------- table_grad
-constexpr int TG_TILES = 32;                      // tiles t per stage: two k-steps
-constexpr int TG_SPG = TG_TILES * TC_PITCH + 1;   // odd: the lanes' eight s fall on different banks beside their four t
-constexpr int TG_SPX = (TG_TILES + 4) * TC_PITCH + 1;
+constexpr int TG_COLS = 32;                       // columns of the field at a time: a consumer warp has four channel pairs
+constexpr int TG_PAIRS = TG_COLS / 2;
+constexpr int TG_GROUP = 5;                       // blocks of 32 columns that a CTA works on one after the other, at most
+constexpr int TG_BUFFERS = 4, TG_FLIGHT = 2;
+constexpr int TG_PITCH = 5;                       // 16-byte words per staged position (4 and one of padding)
+constexpr int TG_TILES = 16;                      // tiles t per stage: a k-step
+constexpr int TG_SPG = TG_TILES * TG_PITCH + 1;   // odd: the lanes' eight s fall on different banks beside their four t
+constexpr int TG_SPX = (TG_TILES + 4) * TG_PITCH + 1;
 constexpr int TG_STAGE = 8 * (TG_SPG + TG_SPX);   // 16-byte words
-constexpr int TG_PS = 18;                         // floats between the s of a P block
-constexpr int TG_BLOCK = 8 * TG_PS;               // floats of a P block: 8 s x 16 r
-constexpr int TG_PAIR = 4 * TG_BLOCK + 2;         // floats of a channel pair's four: the pairs start on different banks
 constexpr int TG_MERGE = 3;                       // blocks of 8 offsets one CTA takes: 24 + 7 positions are four groups of 8
-static_assert(2 * TC_PAIRS * TG_PAIR * 4 <= 2 * TG_STAGE * 16, "the P blocks reuse the stages");
+constexpr int TG_PS = 34;                         // floats between the s of a P block: 32 r, and 2 so that rows start on other banks
+constexpr int TG_BLOCK = 8 * TG_PS + 8;           // floats of a P block: 8 s x 32 r
 
-// One CTA: up to three consecutive blocks (of 8 offsets) of one window, 32 columns.  A window with up to 9 offsets has one or
-// two groups of 8 positions: the two warps of a channel group then split the contraction; with more they split the groups.
-__global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const ConvArgs a, int n_blocks) {
+// One CTA: up to three consecutive blocks (of 8 offsets) of one window, 32 columns at a time.
+__global__ void __launch_bounds__(2 * GROUP, 2) conv_table_grad_tc_kernel(const __grid_constant__ ConvArgs a, int n_blocks, int col_blocks, int group) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ PairItem pairs_s[TC_PAIRS];
+  __shared__ PairItem pairs_s[TG_GROUP * TG_PAIRS];
   const int block = blockIdx.x, w = a.order[2 * block], d0 = a.order[2 * block + 1], b8 = d0 / 8;
   auto is = [&](int x, int d) { return a.order[2 * x] == w && a.order[2 * x + 1] == d; };
   if (b8 % TG_MERGE != 0 && block > 0 && is(block - 1, d0 - 8)) return;  // an earlier block's CTA takes this one too
@@ -110,170 +176,192 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_table_grad_tc_kernel(const
   while ((b8 + merged) % TG_MERGE != 0 && block + merged < n_blocks && is(block + merged, d0 + 8 * merged)) ++merged;
   const int span = 2 * a.halo + 1, row = w / span, j = row + w % span - a.halo;
   const int valid = min(8 * merged, a.win_cnt[w] - d0), groups = (7 + valid + 7) / 8;
-  const int col0 = blockIdx.y * TC_COLS, row_bytes = 2 * a.width;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3, half = warp >> 2;
-  const bool split_k = groups <= 2;
-  const int first_group = split_k ? 0 : 2 * half, mine = min(groups - first_group, 2);
-  const int T = a.nlon / 8, chunks = (T + TG_TILES - 1) / TG_TILES, stages = chunks * a.batch;
-  find_items(a, col0, pairs_s);
-  int shift = (a.win_lo[w] + d0) % a.nlon;
-  if (shift < 0) shift += a.nlon;
-  const size_t sample = (size_t)a.rows * a.nlon * row_bytes;
-  const unsigned char* grow = static_cast<const unsigned char*>(a.g) + (size_t)row * a.nlon * row_bytes;
-  const unsigned char* xrow = static_cast<const unsigned char*>(a.x) + (size_t)j * a.nlon * row_bytes;
+  const int cb0 = blockIdx.y * group, n_cb = min(group, col_blocks - cb0), row_bytes = 2 * a.width;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3;
+  const int T = a.nlon / 8, chunks = (T + TG_TILES - 1) / TG_TILES;
   uint4* const stage_s = reinterpret_cast<uint4*>(smem);
-  auto issue = [&](int s) {
-    const int b = s / chunks, t0 = (s - b * chunks) * TG_TILES, tl = min(TG_TILES, T - t0);
-    uint4* dst = stage_s + (s & 1) * TG_STAGE;
-    stage_positions<TG_SPG>(dst, grow + b * sample, 8 * t0, 8 * tl, a.nlon, row_bytes, 2 * col0);
-    stage_positions<TG_SPX>(dst + 8 * TG_SPG, xrow + b * sample, shift + 8 * t0, 8 * (tl + groups - 1), a.nlon, row_bytes, 2 * col0);
-    commit();
-  };
-  float acc[4][2][2][4];  // channel pair, group, component of x: rows (s = g: component 0 of g, g + 8: 1), columns r = 2 c, 2 c + 1
-#pragma unroll
-  for (int p = 0; p < 4; ++p)
-#pragma unroll
-    for (int n = 0; n < 2; ++n)
-#pragma unroll
-      for (int q = 0; q < 2; ++q)
-#pragma unroll
-        for (int x = 0; x < 4; ++x) acc[p][n][q][x] = 0.f;
+  find_items<TG_GROUP * TG_COLS, 2 * GROUP>(a, cb0 * TG_COLS, pairs_s);
 
-  issue(0);
-  int k_index = 0;
-  for (int s = 0; s < stages; ++s) {
-    if (s + 1 < stages) {
-      issue(s + 1);
-      wait_copies<1>();
-    } else {
-      wait_copies<0>();
-    }
-    __syncthreads();
-    const int t0 = (s % chunks) * TG_TILES, tl = min(TG_TILES, T - t0);
-    const uint4* gs = stage_s + (s & 1) * TG_STAGE + g * TG_SPG + cg;
-    const uint4* xs = stage_s + (s & 1) * TG_STAGE + 8 * TG_SPG + g * TG_SPX + first_group * TC_PITCH + cg;
-    // the words of tile t = k0 + 2 c (+ 1, + 8, + 9); both operands are zero beyond the last tile
-    auto step = [&](int k0, auto is_ragged) {
-      auto word = [&](const uint4* base, int t, int n) {
-        uint4 v = base[(t + n) * TC_PITCH];
-        if (decltype(is_ragged)::value && t >= tl) v = make_uint4(0, 0, 0, 0);
-        return v;
-      };
-      const int t = k0 + 2 * c;
-      unsigned fa[4][4];
-      {
-        const uint4 v0 = word(gs, t, 0), v1 = word(gs, t + 1, 0), v8 = word(gs, t + 8, 0), v9 = word(gs, t + 9, 0);
-        const unsigned w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
-        const unsigned w8[4] = {v8.x, v8.y, v8.z, v8.w}, w9[4] = {v9.x, v9.y, v9.z, v9.w};
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          fa[p][0] = __byte_perm(w0[p], w1[p], 0x5410);
-          fa[p][1] = __byte_perm(w0[p], w1[p], 0x7632);
-          fa[p][2] = __byte_perm(w8[p], w9[p], 0x5410);
-          fa[p][3] = __byte_perm(w8[p], w9[p], 0x7632);
+  if (warp >= GROUP / 32) {
+    // ---- producers: the stages are the samples' chunks of tiles, columns by columns
+    producer_registers();
+    int shift = (a.win_lo[w] + d0) % a.nlon;
+    if (shift < 0) shift += a.nlon;
+    const size_t sample = (size_t)a.rows * a.nlon * row_bytes;
+    const unsigned char* grow = static_cast<const unsigned char*>(a.g) + (size_t)row * a.nlon * row_bytes;
+    const unsigned char* xrow = static_cast<const unsigned char*>(a.x) + (size_t)j * a.nlon * row_bytes;
+    Ring<TG_BUFFERS, TG_FLIGHT> ring;
+    for (int cb = 0; cb < n_cb; ++cb)
+      for (int b = 0; b < a.batch; ++b)
+        for (int t0 = 0; t0 < T; t0 += TG_TILES) {
+          const int tl = min(TG_TILES, T - t0), col_byte = 2 * (cb0 + cb) * TG_COLS;
+          ring.begin();
+          uint4* dst = stage_s + ring.buf * TG_STAGE;
+          stage_positions<GROUP, TG_COLS / 8, TG_SPG, TG_PITCH, false>(dst, grow + b * sample, 8 * t0, 8 * tl, a.nlon, row_bytes, col_byte);
+          stage_positions<GROUP, TG_COLS / 8, TG_SPX, TG_PITCH, false>(dst + 8 * TG_SPG, xrow + b * sample, shift + 8 * t0, 8 * (tl + groups - 1),
+                                                                       a.nlon, row_bytes, col_byte);
+          commit();
+          ring.advance();
         }
-      }
+    ring.drain();
+    return;
+  }
+  // ---- consumers
+  consumer_registers();
+  float* const p_s = reinterpret_cast<float*>(stage_s + TG_BUFFERS * TG_STAGE) + warp * 4 * TG_BLOCK;
+  float zero[4];  // zeros that the compiler does not see through: it would clear four registers for every product
 #pragma unroll
-      for (int n = 0; n < 2; ++n) {
-        if (n < mine) {
-          const uint4 v0 = word(xs, t, n), v1 = word(xs, t + 1, n), v8 = word(xs, t + 8, n), v9 = word(xs, t + 9, n);
+  for (int v = 0; v < 4; ++v) zero[v] = __int_as_float(a.nlon >> 31 & (v + 1));
+  int buf = 0;
+  auto columns = [&](auto count, int cb) {
+    constexpr int GROUPS = decltype(count)::value;
+    f32x2 acc[4][GROUPS][2][2];  // channel pair, group, component of x: rows (s = g: component 0 of g, g + 8: 1), columns r = 2 c, 2 c + 1
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+      for (int n = 0; n < GROUPS; ++n)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) acc[p][n][q][0] = acc[p][n][q][1] = 0;
+    for (int s = 0; s < chunks * a.batch; ++s) {
+      const int tl = min(TG_TILES, T - s % chunks * TG_TILES);
+      barrier_sync(full_barrier(buf));
+      const uint4* gs = stage_s + buf * TG_STAGE + g * TG_SPG + cg;
+      const uint4* xs = stage_s + buf * TG_STAGE + 8 * TG_SPG + g * TG_SPX + cg;
+      // the words of tile t = k0 + 2 c (+ 1, + 8, + 9); both operands are zero beyond the last tile
+      auto step = [&](int k0, auto is_ragged) {
+        const int t = k0 + 2 * c;
+        auto words = [&](const uint4* base, int n, unsigned (&lo)[4], unsigned (&hi)[4], int from) {  // tiles t + from, t + from + 1: component 0, 1
+          uint4 v0 = base[(t + from + n) * TG_PITCH], v1 = base[(t + from + 1 + n) * TG_PITCH];
+          if (decltype(is_ragged)::value) {
+            if (t + from >= tl) v0 = make_uint4(0, 0, 0, 0);
+            if (t + from + 1 >= tl) v1 = make_uint4(0, 0, 0, 0);
+          }
           const unsigned w0[4] = {v0.x, v0.y, v0.z, v0.w}, w1[4] = {v1.x, v1.y, v1.z, v1.w};
-          const unsigned w8[4] = {v8.x, v8.y, v8.z, v8.w}, w9[4] = {v9.x, v9.y, v9.z, v9.w};
 #pragma unroll
           for (int p = 0; p < 4; ++p) {
-            mma_add(acc[p][n][0], fa[p], __byte_perm(w0[p], w1[p], 0x5410), __byte_perm(w8[p], w9[p], 0x5410));
-            mma_add(acc[p][n][1], fa[p], __byte_perm(w0[p], w1[p], 0x7632), __byte_perm(w8[p], w9[p], 0x7632));
+            lo[p] = __byte_perm(w0[p], w1[p], 0x5410);
+            hi[p] = __byte_perm(w0[p], w1[p], 0x7632);
           }
+        };
+        unsigned a0[4], a1[4], a2[4], a3[4];
+        words(gs, 0, a0, a1, 0);
+        words(gs, 0, a2, a3, 8);
+#pragma unroll
+        for (int n = 0; n < GROUPS; ++n) {
+          unsigned b00[4], b10[4], b01[4], b11[4];
+          words(xs, n, b00, b10, 0);
+          words(xs, n, b01, b11, 8);
+          float sum[4][2][4];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            mma_first(sum[p][0], a0[p], a1[p], a2[p], a3[p], b00[p], b01[p], zero);
+            mma_first(sum[p][1], a0[p], a1[p], a2[p], a3[p], b10[p], b11[p], zero);
+          }
+#pragma unroll
+          for (int p = 0; p < 4; ++p)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              add2(acc[p][n][q][0], sum[p][q][0], sum[p][q][1]);
+              add2(acc[p][n][q][1], sum[p][q][2], sum[p][q][3]);
+            }
         }
+      };
+      for (int k0 = 0; k0 < tl; k0 += 16) {
+        if (k0 + 16 <= tl) step(k0, std::false_type{});
+        else step(k0, std::true_type{});
       }
-    };
-    for (int k0 = 0; k0 < tl; k0 += 16, ++k_index) {
-      if (split_k && (k_index & 1) != half) continue;
-      if (k0 + 16 <= tl) step(k0, std::false_type{});
-      else step(k0, std::true_type{});
+      barrier_arrive(empty_barrier(buf));
+      buf = buf == TG_BUFFERS - 1 ? 0 : buf + 1;
     }
-    __syncthreads();
-  }
-
-  // ---- P blocks (half, channel pair, components) to shared memory, then the sums along their diagonals, always in one order
-  float* const p_s = reinterpret_cast<float*>(smem);
+    // ---- a channel pair's four P blocks to shared memory, then the sums along their diagonals, a lane per offset
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 4; ++p) {
+      const PairItem it = pairs_s[cb * TG_PAIRS + 4 * cg + p];
+      __syncwarp();
 #pragma unroll
-    for (int n = 0; n < 2; ++n)
+      for (int n = 0; n < GROUPS; ++n)
 #pragma unroll
-      for (int q = 0; q < 2; ++q) {
-        float* at = p_s + (half * TC_PAIRS + 4 * cg + p) * TG_PAIR + q * TG_BLOCK + g * TG_PS + 8 * n + 2 * c;
-        *reinterpret_cast<float2*>(at) = make_float2(acc[p][n][q][0], acc[p][n][q][1]);                 // component 0 of g
-        *reinterpret_cast<float2*>(at + 2 * TG_BLOCK) = make_float2(acc[p][n][q][2], acc[p][n][q][3]);  // component 1
+        for (int q = 0; q < 2; ++q) {
+          float* at = p_s + q * TG_BLOCK + g * TG_PS + 8 * n + 2 * c;
+          *reinterpret_cast<float2*>(at) = unpack2(acc[p][n][q][0]);                 // component 0 of g
+          *reinterpret_cast<float2*>(at + 2 * TG_BLOCK) = unpack2(acc[p][n][q][1]);  // component 1
+        }
+      __syncwarp();
+      if (lane >= valid || it.kind < 0) continue;
+      float v[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float sum = 0.f;
+#pragma unroll
+        for (int s = 0; s < 8; ++s) sum += p_s[q * TG_BLOCK + s * TG_PS + s + lane];
+        v[q] = sum;
       }
-  __syncthreads();
-  for (int x = threadIdx.x; x < TC_PAIRS * valid; x += TC_THREADS) {
-    const int p = x % TC_PAIRS, d = x / TC_PAIRS;
-    const PairItem it = pairs_s[p];
-    if (it.kind < 0) continue;
-    float v[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float sum = 0.f;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const int r = s + d;
-        const float* at = p_s + p * TG_PAIR + q * TG_BLOCK + s * TG_PS;
-        constexpr int OTHER = TC_PAIRS * TG_PAIR;
-        if (split_k) sum += at[r] + at[r + OTHER];
-        else sum += r < 16 ? at[r] : at[r - 16 + OTHER];
-      }
-      v[q] = sum;
+      float* out = a.dtable + (size_t)(a.win_off[w] + d0 + lane) * a.table_width + it.fcol;
+      if (it.kind == 0) *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
+      else *reinterpret_cast<float2*>(out) = make_float2(v[0], v[3]);
     }
-    float* out = a.dtable + (size_t)(a.win_off[w] + d0 + d) * a.table_width + it.fcol;
-    if (it.kind == 0) *reinterpret_cast<float4*>(out) = make_float4(v[0], v[1], v[2], v[3]);
-    else *reinterpret_cast<float2*>(out) = make_float2(v[0], v[3]);
+  };
+  for (int cb = 0; cb < n_cb; ++cb) {
+    if (groups <= 2) columns(std::integral_constant<int, 2>(), cb);
+    else if (groups == 3) columns(std::integral_constant<int, 3>(), cb);
+    else columns(std::integral_constant<int, 4>(), cb);
   }
 }
 
 // ---------------------------------------------------------------------------------------------------------------- apply
-constexpr int AP_TILES = 64;                              // tiles of 8 longitudes per CTA
-constexpr int AP_OFFSETS = 17;                            // offsets per stage: 17 + 7 positions are three k-steps
-constexpr int AP_SP = (AP_TILES + 2) * TC_PITCH;          // = 2 mod 8: the lanes' four r fall on different banks beside their two t
-static_assert(AP_SP % 8 == 2, "conflict-free 16-byte loads");
-constexpr int AP_SLOTS = 32;                              // offsets -7 .. 24 of a split table row, 8 bytes each
+constexpr int AP_GROUP = 5;                              // blocks of 16 columns that a CTA works on one after the other, at most
+constexpr int AP_BUFFERS = 3;                             // stages in shared memory
+constexpr int AP_COLS = 16;                               // columns of the field at a time: 2 groups of 4 channel pairs x 2 sets of tiles
+constexpr int AP_PAIRS = AP_COLS / 2;
+constexpr int AP_TILES = 64;                              // tiles of 8 longitudes per CTA, of one sample or of several
+constexpr int AP_STEPS = 3;                               // k-steps of 8 positions per stage
+constexpr int AP_HALO = AP_STEPS - 1;                     // tiles staged beyond a sample's last
+constexpr int AP_STAGED = 72;                             // staged tiles: the CTA's and the samples' halos
+constexpr int AP_PITCH = 2;                               // 16-byte words per staged position
+// A lane reads position c of tile t, eight lanes (c = 0 .. 3, two t) at a time: the planes of c start 0, 1, 4, 5 words off a
+// multiple of eight, so that their sixteen-byte words 2 t + 0, 1, 4, 5 and 2 (t + 1) + 0, 1, 4, 5 fall on different banks
+constexpr int AP_SP = AP_STAGED * AP_PITCH + 8;
+static_assert(AP_SP % 8 == 0, "conflict-free 16-byte loads");
+constexpr int AP_SLOTS = 32;                              // offsets -7 .. 24 of a stage's first position, 8 bytes each
 constexpr int AP_PAIR = 3 * AP_SLOTS + 1;                 // 8-byte words per channel pair
-constexpr int AP_STAGE = 8 * AP_SP + (TC_PAIRS * AP_PAIR * 8 + 15) / 16;  // 16-byte words
+constexpr int AP_STAGE = 8 * AP_SP + (AP_PAIRS * AP_PAIR * 8 + 15) / 16;  // 16-byte words
+constexpr int AP_MAX_SPAN = 4096;                         // neighbour rows whose windows a CTA lists in shared memory
 
-// What a CTA works on: 32 columns of a target row's longitudes 8 t0 .. 8 (t0 + tl) - 1, one sample (`field`)
+// What a CTA works on: 16 columns of a target row's longitudes 8 t0 .. 8 (t0 + tl) - 1, the samples b0 .. b0 + nb - 1; their
+// tiles, sample by sample, are the columns of its products.
 struct ApplyTile {
-  const unsigned char* field;
-  int row, t0, tl, col0;
+  int row, col0, t0, tl, b0, nb;
 };
-// Stages: offsets [d, d + n) of a window of the row
+struct Window {
+  int cnt, lo, off, row;
+};
+// Stages: positions [r, r + 8 steps) of the cnt + 7 that the eight longitudes of a tile see through a window
 struct ApplyStage {
-  int w, d, n, cnt;  // w = 2 halo + 1: past the last
+  int w, r, steps;
 };
-__device__ __forceinline__ ApplyStage first_stage(const ConvArgs& a, int row, int w) {  // of the windows from w on
-  const int span = 2 * a.halo + 1;
-  for (; w < span; ++w) {
-    const int j = row + w - a.halo;
-    if (j < 0 || j >= a.rows) continue;
-    const int cnt = a.win_cnt[row * span + w];
-    if (cnt > 0) return ApplyStage{w, 0, min(AP_OFFSETS, cnt), cnt};
-  }
-  return ApplyStage{span, 0, 0, 0};
+__device__ __forceinline__ ApplyStage stage_at(const Window* windows, int n_windows, int w, int r) {
+  return ApplyStage{w, r, w < n_windows ? min(AP_STEPS, (windows[w].cnt + 7 - r + 7) / 8) : 0};
 }
-__device__ __forceinline__ ApplyStage next_stage(const ConvArgs& a, int row, const ApplyStage& s) {
-  const int d = s.d + s.n;
-  return d < s.cnt ? ApplyStage{s.w, d, min(AP_OFFSETS, s.cnt - d), s.cnt} : first_stage(a, row, s.w + 1);
+__device__ __forceinline__ ApplyStage next_stage(const Window* windows, int n_windows, const ApplyStage& s) {
+  const int r = s.r + 8 * s.steps;
+  return r < windows[s.w].cnt + 7 ? stage_at(windows, n_windows, s.w, r) : stage_at(windows, n_windows, s.w + 1, 0);
 }
-__device__ __forceinline__ void issue_stage(const ConvArgs& a, const ApplyTile& t, const ApplyStage& s, uint4* dst) {
-  int lon = (8 * t.t0 + a.win_lo[t.row * (2 * a.halo + 1) + s.w] + s.d) % a.nlon;
-  if (lon < 0) lon += a.nlon;
-  const int steps = (7 + s.n + 7) / 8, row_bytes = 2 * a.width;
-  stage_positions<AP_SP>(dst, t.field + (size_t)(t.row + s.w - a.halo) * a.nlon * row_bytes, lon, 8 * (t.tl + steps - 1), a.nlon, row_bytes, 2 * t.col0);
+// Tile n of the CTA's in the staged tiles
+__device__ __forceinline__ int staged_tile(const ApplyTile& t, int n) { return n + AP_HALO * (n / t.tl); }
+
+__device__ __forceinline__ void issue_stage(const ConvArgs& a, const ApplyTile& t, const Window& w, const ApplyStage& s, uint4* dst) {
+  const int row_bytes = 2 * a.width, tiles = t.tl + s.steps - 1;
+  int lon = 8 * t.t0 + w.lo + s.r;
+  while (lon < 0) lon += a.nlon;
+  const size_t sample = (size_t)a.rows * a.nlon * row_bytes;
+  const unsigned char* row = static_cast<const unsigned char*>(a.x) + t.b0 * sample + (size_t)w.row * a.nlon * row_bytes;
+  for (int b = 0; b < t.nb; ++b, row += sample, dst += (t.tl + AP_HALO) * AP_PITCH)
+    stage_positions<GROUP, AP_COLS / 8, AP_SP, AP_PITCH, true>(dst, row, lon, 8 * tiles, a.nlon, row_bytes, 2 * t.col0);
   commit();
 }
-// The matrix of channel pair `it` at offset d of the stage
-__device__ __forceinline__ float4 table_matrix(const ConvArgs& a, int row, const ApplyStage& s, int d, PairItem it) {
-  const float* f = a.table + (size_t)(a.win_off[row * (2 * a.halo + 1) + s.w] + s.d + d) * a.table_width + it.fcol;
+// The matrix of channel pair `it` at offset d of the window
+__device__ __forceinline__ float4 table_matrix(const ConvArgs& a, const Window& w, int d, PairItem it) {
+  const float* f = a.table + (size_t)(w.off + d) * a.table_width + it.fcol;
   if (it.kind == 0) {
     const float4 v = __ldg(reinterpret_cast<const float4*>(f));
     return a.transpose ? make_float4(v.x, v.z, v.y, v.w) : v;
@@ -281,20 +369,21 @@ __device__ __forceinline__ float4 table_matrix(const ConvArgs& a, int row, const
   const float2 v = __ldg(reinterpret_cast<const float2*>(f));
   return make_float4(v.x, 0.f, 0.f, v.y);
 }
-// Column col of the tile's row in the result
-__device__ __forceinline__ __nv_bfloat16* apply_output(const ConvArgs& a, const ApplyTile& t, int b, int col) {
-  return static_cast<__nv_bfloat16*>(a.y) + ((size_t)b * a.rows + t.row) * a.nlon * a.width + col;
+// Longitude s of tile n of the CTA's in the result, column col
+__device__ __forceinline__ __nv_bfloat16* apply_output(const ConvArgs& a, const ApplyTile& t, int n, int s, int col) {
+  const int b = t.b0 + n / t.tl, l = 8 * (t.t0 + n % t.tl) + s;
+  return static_cast<__nv_bfloat16*>(a.y) + (((size_t)b * a.rows + t.row) * a.nlon + l) * a.width + col;
 }
 
 // The CTA's outputs whose sums were not finite, by themselves: such a sum may owe it to a value outside its window (0 x Inf) or
 // to another component, so it is formed again from its own neighbours alone, on the FMA pipe from the staged positions.  A warp
 // leaves out the channel pairs that have no such output, or none that is not NaN already (and stays so).  `bad`: bit
-// 8 p + 2 i + e = channel pair p at longitude 8 (8 (half + 2 i) + 2 c + e) + g.  128 x 256, radius 4 pi / 128, batch 2, 32 x (m <= 2): a
-// field of NaN 324 us, one Inf in a polar row (whose rings all see it) 567, nothing 264; the FMA kernel 344 whatever it meets, each
-// output by its own thread from global memory 9 058 and 1 196.
-__device__ __noinline__ void apply_again(const ConvArgs& a, const ApplyTile& tile, int b, uint4* stage_s, const PairItem* pairs_s, unsigned bad) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3, half = warp >> 2;
+// 8 p + 2 i + e = channel pair p at longitude g of tile 8 (half + 2 i) + 2 c + e.
+__device__ __forceinline__ void apply_again(const ConvArgs& a, const ApplyTile& tile, const Window* windows, int n_windows, uint4* stage_s,
+                                         const PairItem* pairs_s, unsigned bad) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 1, half = warp >> 1;
   float2 y[4][4][2];
+  int at[4][2];  // word of position 0 of the tiles' eight
   bool open[4];  // pairs the warp still works on
 #pragma unroll
   for (int p = 0; p < 4; ++p) {
@@ -302,33 +391,36 @@ __device__ __noinline__ void apply_again(const ConvArgs& a, const ApplyTile& til
 #pragma unroll
     for (int i = 0; i < 4; ++i) y[p][i][0] = y[p][i][1] = make_float2(0.f, 0.f);
   }
-  ApplyStage s = first_stage(a, tile.row, 0);
-  if (s.w <= 2 * a.halo) issue_stage(a, tile, s, stage_s);
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) at[i][e] = 4 * (staged_tile(tile, min(8 * (half + 2 * i) + 2 * c + e, tile.nb * tile.tl - 1)) * AP_PITCH + cg);
+  ApplyStage s = stage_at(windows, n_windows, 0, 0);
+  if (s.w < n_windows) issue_stage(a, tile, windows[s.w], s, stage_s);
   int buf = 0;
-  while (s.w <= 2 * a.halo) {
-    const ApplyStage nxt = next_stage(a, tile.row, s);
-    if (nxt.w <= 2 * a.halo) {
-      issue_stage(a, tile, nxt, stage_s + (buf ^ 1) * AP_STAGE);
-      wait_copies<1>();
-    } else {
-      wait_copies<0>();
-    }
-    __syncthreads();
+  while (s.w < n_windows) {
+    const Window win = windows[s.w];
+    const ApplyStage nxt = next_stage(windows, n_windows, s);
+    wait_copies<0>();
+    consumer_sync();
+    if (nxt.w < n_windows) issue_stage(a, tile, windows[nxt.w], nxt, stage_s + (buf ^ 1) * AP_STAGE);
 #pragma unroll
     for (int p = 0; p < 4; ++p) {
       if (!open[p]) continue;
       const PairItem it = pairs_s[4 * cg + p];
-      const unsigned* words = reinterpret_cast<const unsigned*>(stage_s + buf * AP_STAGE + cg) + p;
-      float4 next = table_matrix(a, tile.row, s, 0, it);
-      for (int d = 0; d < s.n; ++d) {
+      const unsigned* words = reinterpret_cast<const unsigned*>(stage_s + buf * AP_STAGE) + p;
+      // position r of the window is offset r - g of the lane's longitudes
+      auto matrix = [&](int r) { return table_matrix(a, win, min(max(s.r + r - g, 0), win.cnt - 1), it); };
+      float4 next = matrix(0);
+      for (int r = 0; r < 8 * s.steps; ++r) {
         const float4 m = next;
-        next = table_matrix(a, tile.row, s, min(d + 1, s.n - 1), it);
+        next = matrix(min(r + 1, 8 * s.steps - 1));
+        if (s.r + r < g || s.r + r - g >= win.cnt) continue;
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const int q = 8 * (8 * (half + 2 * i) + 2 * c + e) + g + d;
-            const unsigned w = words[4 * ((q & 7) * AP_SP + (q >> 3) * TC_PITCH)];
+            const unsigned w = words[at[i][e] + 4 * (plane<AP_SP, true>(r & 7) + (r >> 3) * AP_PITCH)];
             const float vx = __uint_as_float(w << 16), vy = __uint_as_float(w & 0xffff0000u);
             float2& out = y[p][i][e];
             if (it.kind == 0) {
@@ -347,22 +439,20 @@ __device__ __noinline__ void apply_again(const ConvArgs& a, const ApplyTile& til
         for (int e = 0; e < 2; ++e) undecided = undecided || ((bad >> (8 * p + 2 * i + e) & 1) && !(isnan(y[p][i][e].x) && isnan(y[p][i][e].y)));
       open[p] = __any_sync(0xffffffffu, undecided);
     }
-    if (!__syncthreads_or(open[0] || open[1] || open[2] || open[3])) break;
+    if (!consumer_or(open[0] || open[1] || open[2] || open[3])) break;
     s = nxt;
     buf ^= 1;
   }
   wait_copies<0>();
-  __nv_bfloat16* at = apply_output(a, tile, b, tile.col0 + 8 * cg);
 #pragma unroll
   for (int p = 0; p < 4; ++p)
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 2; ++e)
-        if (bad >> (8 * p + 2 * i + e) & 1) {
-          const int l = 8 * (tile.t0 + 8 * (half + 2 * i) + 2 * c + e) + g;
-          *reinterpret_cast<__nv_bfloat162*>(at + (size_t)l * a.width + 2 * p) = __floats2bfloat162_rn(y[p][i][e].x, y[p][i][e].y);
-        }
+        if (bad >> (8 * p + 2 * i + e) & 1)
+          *reinterpret_cast<__nv_bfloat162*>(apply_output(a, tile, 8 * (half + 2 * i) + 2 * c + e, g, tile.col0 + 8 * cg + 2 * p)) =
+              __floats2bfloat162_rn(y[p][i][e].x, y[p][i][e].y);
 }
 
 // (x, y) = sum of three bfloat16 pairs, largest first
@@ -376,83 +466,139 @@ __device__ __forceinline__ void split3(float x, float y, unsigned (&w)[3]) {
   }
 }
 
-__global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const __grid_constant__ ConvArgs a, int col_blocks, int lon_blocks) {
+
+__global__ void __launch_bounds__(2 * GROUP, 2) conv_apply_tc_kernel(const __grid_constant__ ConvArgs a, int col_blocks, int single_rows, int single_ctas, int group, int lon_blocks,
+                                                                             int samples) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ PairItem pairs_s[TC_PAIRS];
-  int x = blockIdx.x;
-  const int cb = x % col_blocks;
-  x /= col_blocks;
+  __shared__ PairItem pairs_s[AP_GROUP * AP_PAIRS];
+  __shared__ unsigned bad_s[AP_GROUP][GROUP];
+  __shared__ int n_windows_s;
+  int x = blockIdx.x, first_row = 0;
+  if (x < single_ctas) {
+    group = 1;
+  } else {
+    x -= single_ctas;
+    first_row = single_rows;
+  }
+  const int groups = (col_blocks + group - 1) / group, cb0 = x % groups * group, n_cb = min(group, col_blocks - cb0);
+  x /= groups;
   const int lb = x % lon_blocks;
   x /= lon_blocks;
-  const int b = x % a.batch, row = a.order[x / a.batch];  // heaviest rows first
-  const int col0 = cb * TC_COLS, row_bytes = 2 * a.width, span = 2 * a.halo + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 3, half = warp >> 2;
-  const int T = a.nlon / 8, t0 = lb * AP_TILES, tl = min(AP_TILES, T - t0), tiles = (tl + 7) / 8;
-  find_items(a, col0, pairs_s);
-  const unsigned char* field = static_cast<const unsigned char*>(a.x) + (size_t)b * a.rows * a.nlon * row_bytes;
+  const int chunks = (a.batch + samples - 1) / samples, b0 = (x % chunks) * samples, row = a.order[first_row + x / chunks];  // heaviest rows first
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, c = lane & 3, cg = warp & 1, half = warp >> 1 & 1;
+  const int T = a.nlon / 8, per = (T + lon_blocks - 1) / lon_blocks, t0 = lb * per;
+  ApplyTile tile{row, cb0 * AP_COLS, t0, min(per, T - t0), b0, min(samples, a.batch - b0)};
+  const int n_tiles = tile.nb * tile.tl, mine = ((n_tiles + 7) / 8 - half + 1) / 2;  // this warp's eights of tiles: half, half + 2, ...
   uint4* const stage_s = reinterpret_cast<uint4*>(smem);
-
-  const ApplyTile tile{field, row, t0, tl, col0};
-  // this thread's two slots of the split table: a channel pair and the offsets slot - 7
-  const int tp = threadIdx.x & (TC_PAIRS - 1), ts = threadIdx.x / TC_PAIRS;
-  const PairItem item = pairs_s[tp];
-  auto fetch = [&](const ApplyStage& s, float4 (&m)[2]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int d = ts + 16 * i - 7;
-      m[i] = d >= 0 && d < s.n && item.kind >= 0 ? table_matrix(a, row, s, d, item) : make_float4(0.f, 0.f, 0.f, 0.f);
+  Window* const windows = reinterpret_cast<Window*>(stage_s + AP_BUFFERS * AP_STAGE);
+  if (warp == 0) {
+    const int span = 2 * a.halo + 1;
+    int filled = 0;
+    for (int w0 = 0; w0 < span; w0 += 32) {
+      const int w = w0 + lane, j = row + w - a.halo, cnt = w < span && j >= 0 && j < a.rows ? a.win_cnt[row * span + w] : 0;
+      const unsigned have = __ballot_sync(0xffffffffu, cnt > 0);
+      if (cnt > 0) windows[filled + __popc(have & ((1u << lane) - 1u))] = Window{cnt, a.win_lo[row * span + w] % a.nlon, a.win_off[row * span + w], j};
+      filled += __popc(have);
     }
-  };
-  auto place = [&](int buf, const float4 (&m)[2]) {
-    uint2* dst = reinterpret_cast<uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + tp * AP_PAIR + ts;
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      unsigned w0[3], w1[3];
-      split3(m[i].x, m[i].y, w0);
-      split3(m[i].z, m[i].w, w1);
-#pragma unroll
-      for (int s = 0; s < 3; ++s) dst[s * AP_SLOTS + 16 * i] = make_uint2(w0[s], w1[s]);
-    }
-  };
+    if (lane == 0) n_windows_s = filled;
+  }
+  find_items<AP_GROUP * AP_COLS, 2 * GROUP>(a, tile.col0, pairs_s);
+  const int n_windows = n_windows_s;
 
-  float acc[4][4][4];  // channel pair, tile of 8 t: rows (s = g: component 0, g + 8: component 1), columns t = 2 c, 2 c + 1
+  if (warp >= GROUP / 32) {
+    // ---- producers
+    producer_registers();
+    // this thread's two slots of the split table: a channel pair and the offsets slot - 7 from the stage's first position
+    const int tp = threadIdx.x % AP_PAIRS, ts = threadIdx.x % GROUP / AP_PAIRS;
+    PairItem item = pairs_s[tp];
+    // (the loaded words are looked at by place alone, so that a stage's products run while they are under way)
+    auto fetch = [&](const ApplyStage& s, float2 (&m)[2][2]) {
+      const Window w = windows[s.w];
+      const float* f = a.table + (size_t)w.off * a.table_width + item.fcol;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int d = s.r + ts + 16 * i - 7;
+        const bool in = (i == 0 || s.steps > 1) && d >= 0 && d < w.cnt && item.kind >= 0;
+        const float2* from = reinterpret_cast<const float2*>(f + (size_t)d * a.table_width);
+        m[i][0] = m[i][1] = make_float2(0.f, 0.f);
+        if (in) m[i][0] = __ldg(from);
+        if (in && item.kind == 0) m[i][1] = __ldg(from + 1);
+      }
+    };
+    auto place = [&](int buf, const ApplyStage& s, const PairItem& item, const float2 (&m)[2][2]) {
+      uint2* dst = reinterpret_cast<uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + tp * AP_PAIR + ts;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (i == 1 && s.steps == 1) break;  // one k-step reads 15 slots
+        float4 v = make_float4(m[i][0].x, m[i][0].y, m[i][1].x, m[i][1].y);
+        if (item.kind == 1) v = make_float4(v.x, 0.f, 0.f, v.y);
+        else if (a.transpose) v = make_float4(v.x, v.z, v.y, v.w);
+        unsigned w0[3], w1[3];
+        split3(v.x, v.y, w0);
+        split3(v.z, v.w, w1);
+#pragma unroll
+        for (int q = 0; q < 3; ++q) dst[q * AP_SLOTS + 16 * i] = make_uint2(w0[q], w1[q]);
+      }
+    };
+
+    ApplyStage cur = stage_at(windows, n_windows, 0, 0);
+    float2 m[2][2];
+    if (cur.w < n_windows) fetch(cur, m);
+    Ring<AP_BUFFERS, 1> ring;
+    for (int cb = 0; n_windows > 0 && cb < n_cb;) {
+      ring.begin();
+      issue_stage(a, tile, windows[cur.w], cur, stage_s + ring.buf * AP_STAGE);
+      const PairItem placed = item;
+      ApplyStage nxt = next_stage(windows, n_windows, cur);
+      if (nxt.w == n_windows) {  // on to the next columns
+        nxt = stage_at(windows, n_windows, 0, 0);
+        ++cb;
+        tile.col0 += AP_COLS;
+        if (cb < n_cb) item = pairs_s[cb * AP_PAIRS + tp];
+      }
+      float2 ahead[2][2];
+      if (cb < n_cb) fetch(nxt, ahead);
+      place(ring.buf, cur, placed, m);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) { m[i][0] = ahead[i][0]; m[i][1] = ahead[i][1]; }
+      cur = nxt;
+      ring.advance();
+    }
+    ring.drain();
+    return;
+  }
+  // ---- consumers
+  consumer_registers();
+  // (zeros and the identity of a byte permutation that the compiler does not see through: it would clear four registers for every
+  // product that starts a chain, and pair the words of a B operand again for each of its three products)
+  float zero[4];
+#pragma unroll
+  for (int v = 0; v < 4; ++v) zero[v] = __int_as_float(a.nlon >> 31 & (v + 1));
+  const unsigned same = a.nlon > 0 ? 0x3210u : 0u;
+  int at[4];  // 16-byte word of position c of this lane's tiles
+#pragma unroll
+  for (int i = 0; i < 4; ++i) at[i] = plane<AP_SP, true>(c) + staged_tile(tile, min(8 * (half + 2 * i) + g, n_tiles - 1)) * AP_PITCH + cg;
+
+  int buf = 0;
+  for (int cb = 0; cb < n_cb; ++cb, tile.col0 += AP_COLS) {
+  f32x2 acc[4][4][2];  // channel pair, eight of tiles: rows (s = g: component 0, g + 8: component 1), columns t = 2 c, 2 c + 1
 #pragma unroll
   for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int v = 0; v < 4; ++v) acc[p][i][v] = 0.f;
-
-  ApplyStage cur = first_stage(a, row, 0);
-  float4 m[2];
-  if (cur.w < span) {
-    issue_stage(a, tile, cur, stage_s);
-    fetch(cur, m);
-    place(0, m);
-  }
-  int buf = 0;
-  while (cur.w < span) {
-    const ApplyStage nxt = next_stage(a, row, cur);
-    const bool more = nxt.w < span;
-    if (more) {
-      issue_stage(a, tile, nxt, stage_s + (buf ^ 1) * AP_STAGE);
-      fetch(nxt, m);
-      wait_copies<1>();
-    } else {
-      wait_copies<0>();
-    }
-    __syncthreads();
-    const uint4* xs = stage_s + buf * AP_STAGE + c * AP_SP + cg;
+    for (int i = 0; i < 4; ++i) acc[p][i][0] = acc[p][i][1] = 0;
+  ApplyStage cur = stage_at(windows, n_windows, 0, 0);
+  while (cur.w < n_windows) {
+    barrier_sync(full_barrier(buf));
+    const uint4* xs = stage_s + buf * AP_STAGE;
     const uint2* ms = reinterpret_cast<const uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + 4 * cg * AP_PAIR + 7 + c - g;
-    const int steps = (7 + cur.n + 7) / 8;
-    auto walk = [&](auto mine) {  // tiles half, half + 2, ... of the CTA's (a tile too many reads what a stage left behind: its own columns)
-      constexpr int MINE = decltype(mine)::value;
-      for (int k = 0; k < steps; ++k) {
+    auto walk = [&](auto count) {
+      constexpr int MINE = decltype(count)::value;
+      for (int k = 0; k < cur.steps; ++k) {
         unsigned fb[MINE][2][4];
 #pragma unroll
         for (int i = 0; i < MINE; ++i) {
-          const uint4* at = xs + (8 * (half + 2 * i) + g + k) * TC_PITCH;
-          const uint4 v0 = at[0], v4 = at[4 * AP_SP];
+          const uint4* from = xs + at[i] + k * AP_PITCH;
+          const uint4 v0 = from[0], v4 = from[4 * AP_SP];
           fb[i][0][0] = v0.x; fb[i][0][1] = v0.y; fb[i][0][2] = v0.z; fb[i][0][3] = v0.w;
           fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
         }
@@ -461,109 +607,145 @@ __global__ void __launch_bounds__(TC_THREADS, 2) conv_apply_tc_kernel(const __gr
           const uint2* f = ms + p * AP_PAIR + 8 * k;
           const uint2 l01 = f[2 * AP_SLOTS], l23 = f[2 * AP_SLOTS + 4], m01 = f[AP_SLOTS], m23 = f[AP_SLOTS + 4], h01 = f[0], h23 = f[4];
           float sum[MINE][4];
+          unsigned b0[MINE], b1[MINE];
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) mma_first(sum[i], l01.x, l01.y, l23.x, l23.y, fb[i][0][p], fb[i][1][p]);
+          for (int i = 0; i < MINE; ++i) {
+            b0[i] = __byte_perm(fb[i][0][p], 0, same);
+            b1[i] = __byte_perm(fb[i][1][p], 0, same);
+          }
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) mma(sum[i], m01.x, m01.y, m23.x, m23.y, fb[i][0][p], fb[i][1][p]);
+          for (int i = 0; i < MINE; ++i) mma_first(sum[i], l01.x, l01.y, l23.x, l23.y, b0[i], b1[i], zero);
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) mma(sum[i], h01.x, h01.y, h23.x, h23.y, fb[i][0][p], fb[i][1][p]);
+          for (int i = 0; i < MINE; ++i) mma(sum[i], m01.x, m01.y, m23.x, m23.y, b0[i], b1[i]);
 #pragma unroll
-          for (int i = 0; i < MINE; ++i)
+          for (int i = 0; i < MINE; ++i) mma(sum[i], h01.x, h01.y, h23.x, h23.y, b0[i], b1[i]);
 #pragma unroll
-            for (int v = 0; v < 4; ++v) acc[p][i][v] += sum[i][v];
+          for (int i = 0; i < MINE; ++i) {
+            add2(acc[p][i][0], sum[i][0], sum[i][1]);
+            add2(acc[p][i][1], sum[i][2], sum[i][3]);
+          }
         }
       }
     };
-    if (tiles > 4) walk(std::integral_constant<int, 4>());
-    else if (tiles > 2) walk(std::integral_constant<int, 2>());
-    else walk(std::integral_constant<int, 1>());
-    if (more) place(buf ^ 1, m);
-    __syncthreads();
-    cur = nxt;
-    buf ^= 1;
+    if (mine == 4) walk(std::integral_constant<int, 4>());
+    else if (mine == 3) walk(std::integral_constant<int, 3>());
+    else if (mine == 2) walk(std::integral_constant<int, 2>());
+    else if (mine == 1) walk(std::integral_constant<int, 1>());
+    barrier_arrive(empty_barrier(buf));
+    cur = next_stage(windows, n_windows, cur);
+    buf = buf == AP_BUFFERS - 1 ? 0 : buf + 1;
   }
 
   // ---- four channel pairs of a position are 16 bytes of its row
-  const int col = col0 + 8 * cg;
+  const int col = tile.col0 + 8 * cg;
   unsigned bad = 0;  // outputs whose sums are not finite
   if (col < a.width) {
-    __nv_bfloat16* y = apply_output(a, tile, b, col);
     bool whole = true;
 #pragma unroll
-    for (int p = 0; p < 4; ++p) whole = whole && pairs_s[4 * cg + p].kind >= 0;
+    for (int p = 0; p < 4; ++p) whole = whole && pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int t = 8 * (half + 2 * i) + 2 * c + e;
-        if (t >= tl) continue;
+        const int n = 8 * (half + 2 * i) + 2 * c + e;
+        if (n >= n_tiles) continue;
         unsigned word[4];
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-          const float2 v = make_float2(acc[p][i][e], acc[p][i][2 + e]);
-          if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && pairs_s[4 * cg + p].kind >= 0) bad |= 1u << (8 * p + 2 * i + e);
+          const float2 re = unpack2(acc[p][i][0]), im = unpack2(acc[p][i][1]);
+          const float2 v = e ? make_float2(re.y, im.y) : make_float2(re.x, im.x);
+          if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0) bad |= 1u << (8 * p + 2 * i + e);
           const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
           word[p] = *reinterpret_cast<const unsigned*>(&h);
         }
-        __nv_bfloat16* at = y + (size_t)(8 * (t0 + t) + g) * a.width;
+        __nv_bfloat16* out = apply_output(a, tile, n, g, col);
         if (whole) {
-          *reinterpret_cast<uint4*>(at) = make_uint4(word[0], word[1], word[2], word[3]);
+          *reinterpret_cast<uint4*>(out) = make_uint4(word[0], word[1], word[2], word[3]);
         } else {
 #pragma unroll
           for (int p = 0; p < 4; ++p)
-            if (pairs_s[4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(at + 2 * p) = word[p];
+            if (pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(out + 2 * p) = word[p];
         }
       }
   }
-  if (__syncthreads_or(bad != 0)) apply_again(a, tile, b, stage_s, pairs_s, bad);
+  bad_s[cb][threadIdx.x] = bad;
+  }
+  tile.col0 = cb0 * AP_COLS;
+  for (int cb = 0; cb < n_cb; ++cb, tile.col0 += AP_COLS) {
+    const unsigned bad = bad_s[cb][threadIdx.x];
+    if (consumer_or(bad != 0)) apply_again(a, tile, windows, n_windows, stage_s, pairs_s + cb * AP_PAIRS, bad);
+  }
 }
 
 }  // namespace
 
 bool tensor_cores_can(const ConvArgs& a) {
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.y);
-  return a.nlon % 8 == 0 && a.width % 8 == 0 && bits % 16 == 0;
+  return a.nlon % 8 == 0 && a.width % 8 == 0 && bits % 16 == 0 && 2 * (int64_t)a.halo + 1 <= AP_MAX_SPAN;
 }
 
-// The FMA kernels stay the faster ones where a launch is short or its tiles are mostly padding.  96 shapes from 24 x 24 to
-// 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores:
-//   apply        up to 8 tiles of 8 longitudes leave half of a CTA's warps without one (64 x 64, batch 4, width 320: 53 / 143; 32 x 64,
-//                batch 1, width 40: 39 / 47); with one sample and a narrow field the launch is the polar rows' chain of stages, which is
-//                longer here (256 x 512, width 40: 367 / 526; 128 x 512, width 96: 371 / 489), from two samples on it is not (91 x 184,
-//                width 96: 259 / 170; 45 x 88, width 40: 72 / 66).  Wide fields fill the chip with one sample, and then it is padding
-//                that decides (256 x 512, width 320: 848 / 604; 64 x 128, batch 2, width 320: 174 / 199).
-//   table_grad   contracts over the tiles, 16 a step: 23 tiles and more are always faster (91 x 184, batch 1, width 80: 75 / 58; 128 x
-//                256, width 24: 99 / 50), 16 with four samples in sequence (64 x 128, width 320: 270 / 239; batch 2: 143 / 175), 9 to 15 then
-//                where the field is not wide (45 x 88, width 80: 60 / 57, width 320: 132 / 159; 100 x 104: 105 / 103 and 224 / 307).  One
-//                block of 32 columns, for which the FMA kernel has less than a warp of items, from 8 tiles on (64 x 64: 22 / 20; 45 x 88:
-//                26 / 19); fewer tiles go either way (100 x 48, batch 4: 28 / 32; 24 x 48: 26 / 17).
+// How apply cuts a field: blocks of columns, of tiles along a row, and samples that share a CTA: of a short row as many as its
+// tiles hold with their halos
+struct ApplyGrid {
+  int col_blocks, lon_blocks, samples;
+  int64_t per_block;  // CTAs of a row and a block of columns
+};
+static ApplyGrid apply_grid(const ConvArgs& a) {
+  const int T = a.nlon / 8, lon_blocks = (T + AP_TILES - 1) / AP_TILES, per = (T + lon_blocks - 1) / lon_blocks;
+  const int samples = lon_blocks > 1 ? 1 : std::max(1, std::min({a.batch, AP_TILES / per, AP_STAGED / (per + AP_HALO)}));
+  return {(a.width + AP_COLS - 1) / AP_COLS, lon_blocks, samples, (int64_t)lon_blocks * ((a.batch + samples - 1) / samples)};
+}
+
+// The FMA kernels stay the faster ones where the tiles are mostly padding and there are enough of them to fill the chip.  333
+// shapes from 24 x 24 to 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores:
+//   apply        a CTA takes up to 64 tiles of 8 longitudes.  From 32 on it is the faster one (128 x 128, width 320, batch 2: 179 / 179, batch
+//                4: 333 / 237; 256 x 512, width 320: 1 336 / 540), with fewer while the launch has few CTAs and lasts as long as the polar
+//                rows' chains of stages, which are shorter here (64 x 128, batch 1, width 160: 81 / 42, width 320: 78 / 70; 128 x 128, batch
+//                1, width 160: 116 / 81, but width 320: 112 / 154).  With up to 8 tiles a row the FMA kernel's chains are short too (32 x 64:
+//                50 / 25, width 320: 48 / 47; 200 x 48, width 24: 24 / 22, width 40: 24 / 28, width 320: 28 / 116).
+//   table_grad   contracts over the tiles, 16 a step: 23 tiles and more are always faster (91 x 184, width 320: 132 / 128; 256 x 512: 1 701 /
+//                738), 9 to 22 with four samples (45 x 88, width 80: 62 / 46, width 320: 132 / 116), one block of 32 columns (28 / 21), or
+//                two samples of a field that is not wide (45 x 88, width 96: 38 / 38, width 160: 32 / 38; 64 x 128, width 160: 69 / 54, width
+//                320: 97 / 93; 128 x 128, width 320: 175 / 196); 8 tiles with one block of 32 columns and four samples (32 x 64: 32 / 22).
 bool tensor_cores_apply(const ConvArgs& a) {
-  const int tiles = a.nlon / 8;
-  return tensor_cores_can(a) && tiles > 8 && (a.width < 256 ? a.batch >= 2 : tiles >= 32);
+  if (!tensor_cores_can(a)) return false;
+  const int T = a.nlon / 8;
+  const ApplyGrid grid = apply_grid(a);
+  const int64_t ctas = grid.per_block * grid.col_blocks * a.rows, fill = (int64_t)grid.samples * std::min(T, AP_TILES);
+  return T > 8 ? fill >= 32 || ctas <= 80 * fill : T >= 3 && ctas <= 80 * T;
 }
 bool tensor_cores_table_grad(const ConvArgs& a) {
-  const int tiles = a.nlon / 8;
-  const bool pays = tiles >= 20 || (tiles >= 8 && a.width <= TC_COLS) || (a.batch >= 4 && (tiles >= 16 || (tiles > 8 && a.width <= 96)));
+  const int T = a.nlon / 8;
+  const bool narrow = a.width <= TG_COLS;
+  const bool pays = T > 8 ? T >= 20 || narrow || a.batch >= 4 || (a.batch >= 2 && a.width <= (T >= 16 ? 160 : 96)) : T == 8 && narrow && a.batch >= 4;
   return tensor_cores_can(a) && pays;
 }
 
 int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream) {
-  const int col_blocks = (a.width + TC_COLS - 1) / TC_COLS, lon_blocks = (a.nlon / 8 + AP_TILES - 1) / AP_TILES;
-  const int64_t ctas = (int64_t)col_blocks * lon_blocks * a.batch * n_order;
+  const ApplyGrid grid = apply_grid(a);
+  // Light rows take several blocks of columns one after the other while that leaves six waves of CTAs (256 x 512, radius 4 pi / 256,
+  // batch 4, width 320: 2 134 us one, 2 053 two, 2 011 five at a time); the heaviest rows, whose chains of stages a launch could
+  // end in, always one (128 x 256, batch 2: every row five at a time 424 us, one 277).
+  const int single_rows = (n_order + 7) / 8;
+  const int64_t light = grid.per_block * grid.col_blocks * (n_order - single_rows);
+  const int group = (int)std::max<int64_t>(1, std::min<int64_t>({AP_GROUP, grid.col_blocks, light / (12 * sm_count())}));
+  const int64_t singles = grid.per_block * grid.col_blocks * single_rows;
+  const int64_t ctas = singles + grid.per_block * ((grid.col_blocks + group - 1) / group) * (n_order - single_rows);
   GM_REQUIRE(ctas < (1ll << 31), GM_ERR_LIMIT, "gm_lattice_conv_apply: too many tiles");
-  const size_t smem = 2 * (size_t)AP_STAGE * 16;
+  const size_t smem = AP_BUFFERS * (size_t)AP_STAGE * 16 + (2 * (size_t)a.halo + 1) * sizeof(Window);
   const int st = allow_smem(conv_apply_tc_kernel, smem, "gm_lattice_conv_apply");
   if (st != GM_OK) return st;
-  conv_apply_tc_kernel<<<(unsigned)ctas, TC_THREADS, smem, stream>>>(a, col_blocks, lon_blocks);
+  conv_apply_tc_kernel<<<(unsigned)ctas, 2 * GROUP, smem, stream>>>(a, grid.col_blocks, single_rows, (int)singles, group, grid.lon_blocks, grid.samples);
   return launch_status("gm_lattice_conv_apply");
 }
 
 int table_grad_tc(const ConvArgs& a, int64_t n_blocks, cudaStream_t stream) {
-  const int col_blocks = (a.width + TC_COLS - 1) / TC_COLS;
-  const size_t smem = 2 * (size_t)TG_STAGE * 16;
+  const int col_blocks = (a.width + TG_COLS - 1) / TG_COLS;
+  const int group = std::min(TG_GROUP, col_blocks);
+  const size_t smem = TG_BUFFERS * (size_t)TG_STAGE * 16 + (GROUP / 32) * 4 * TG_BLOCK * sizeof(float);
   const int st = allow_smem(conv_table_grad_tc_kernel, smem, "gm_lattice_conv_table_grad");
   if (st != GM_OK) return st;
-  conv_table_grad_tc_kernel<<<dim3((unsigned)n_blocks, col_blocks), TC_THREADS, smem, stream>>>(a, (int)n_blocks);
+  conv_table_grad_tc_kernel<<<dim3((unsigned)n_blocks, (col_blocks + group - 1) / group), 2 * GROUP, smem, stream>>>(a, (int)n_blocks, col_blocks, group);
   return launch_status("gm_lattice_conv_table_grad");
 }
 

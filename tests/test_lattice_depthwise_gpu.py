@@ -168,6 +168,10 @@ TENSOR_CORE_CASES = [
     (6, 24, 2.0, {0: 8, 1: 8}, 3),
     (4, 560, 1.3, {0: 8, 1: 8, 2: 8}, 2),
     (12, 136, 3.0, {0: 4, 1: 14}, 1),
+    (4, 24, 1.4, {0: 8}, 15),                        # 14 samples of 3 tiles share a CTA, one is left; one half of a block of 16 columns
+    (3, 256, 1.2, {0: 8, 1: 8, 2: 8}, 3),            # two samples of 32 tiles fill a CTA, one is left
+    (2, 512, 1.1, {0: 2, 1: 3}, 1),                  # 64 tiles; a window of 519 positions: four groups of 24 offsets and fewer
+    (3, 520, 1.1, {1: 20}, 2),                       # 65 tiles: blocks of 33 and 32
 ]
 
 
@@ -252,7 +256,7 @@ def test_tensor_core_apply_touches_only_true_neighbours():
 def test_tensor_core_apply_rounds_no_worse_than_the_fma_kernel(nlat, nlon, reach, order):
     """Sums that cancel show the rounding of the accumulation, which the bf16 result hides otherwise: along a longitude the
     field is constant and the last entry of every window takes away the sum of the others.  In float64 what is left is
-    about 2^-24 of a term, so the result is the error.  Bound: the FMA kernel's (which one sample of so narrow a field takes)."""
+    about 2^-24 of a term, so the result is the error.  Bound: the FMA kernel's (which takes a field on an 8-byte boundary)."""
     from gm_attention_b200.nn.lattice_depthwise import _apply
 
     c = make_case(nlat, nlon, reach * math.pi / nlat, {0: 8, 1: 8}, 1, dtype=np.float32)
@@ -282,10 +286,12 @@ def test_tensor_core_apply_rounds_no_worse_than_the_fma_kernel(nlat, nlon, reach
                     m = m.reshape(2, 2) if kind == 0 else np.diag(m[:2])
                     want[i, col:col + 2] += m @ x[j, col:col + 2]
     field = ring[:, None, :].expand(nlat, nlon, D).reshape(nlat * nlon, D).contiguous().cuda()
+    shifted = torch.empty(field.numel() + 4, dtype=field.dtype, device="cuda")[4:].view(field.shape)
+    shifted.copy_(field)
     table = cuda(table)
     error = []
     for tensor_cores in (True, False):
-        got = _apply(field, table, t, False, tensor_cores=tensor_cores).float().double().cpu().numpy().reshape(nlat, nlon, D)
+        got = _apply(field if tensor_cores else shifted, table, t, False, tensor_cores=tensor_cores).float().double().cpu().numpy().reshape(nlat, nlon, D)
         error.append((float(np.sqrt(((got - want[:, None]) ** 2).mean())), float(np.abs(got - want[:, None]).max())))
     assert error[0][0] <= error[1][0] and error[0][1] <= error[1][1], error
 
