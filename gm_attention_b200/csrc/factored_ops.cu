@@ -25,13 +25,14 @@
 // bound is shared-memory bandwidth, so both run on register tiles: 2 edges x 4 t over 4 columns per step for dh (6
 // 16-byte reads for 32 multiply-adds), 5 t x 4 columns over 4 edges per step for dZ (9 reads for 80), the latter owned by
 // fixed threads for the whole source.
-#include "common.cuh"
+#include "factored.cuh"
 
 namespace gmb {
 namespace {
 
+using namespace factored;
+
 constexpr int FMAX_K = 20;
-constexpr int FDESC = 8;
 constexpr int FTHREADS = 128;
 constexpr int MAX_TILE = 64;       // edges per tile, at most (a power of two; less where shared memory is short)
 constexpr int MAX_OWNED = 64;      // K * C <= 64 * 128 in the backward
@@ -44,22 +45,6 @@ constexpr int MAX_OWNED = 64;      // K * C <= 64 * 128 in the backward
 constexpr size_t FSMEM_SIXTH = 227 * 1024 / 6 - 1024;
 constexpr size_t FSMEM_MOST = 224 * 1024;  // dynamic shared memory a CTA may ask for, beside the static arrays
 constexpr int TP = 5;              // rows t of a dZ patch (4 columns wide)
-
-template <typename T>
-struct FArgs {
-  int64_t n_edges, n_groups;
-  int k, wc, wr, n_f, n_blocks, d_out;
-  int n_scales;  // 0: rho (n_edges), a block's scale is a power of it; else (SCALED) rho (n_edges, n_scales), its scale a column of it
-  const T *h, *zc, *zr, *angular, *transport, *rho;
-  const int32_t* desc;
-  const int64_t *source, *order, *group_ptr, *group_source;
-  T* out;
-  // backward
-  const T* g;
-  const int64_t* target;
-  const T *weights, *rows;
-  T *dh, *dzc, *dzr, *dweights;
-};
 
 // An edge's record in shared memory: angular phases (n_f, 2), transport phases (n_f, 2), rho or the scales; odd pitch.
 __host__ __device__ inline int record_pitch(int n_f, int n_scales) { return n_scales ? (4 * n_f + n_scales) | 1 : 4 * n_f + 1; }
@@ -134,39 +119,6 @@ __device__ __forceinline__ void block_factor(const T* rec, int n_f, const int32_
   fr *= s;
   fi *= s;
 }
-// ... from the tables themselves.  (Its own body: one over pointers to the three parts, or over accessors, cost the staged
-// kernels registers and 1 to 6 %.)
-template <bool SCALED, typename T>
-__device__ __forceinline__ void table_factor(const FArgs<T>& a, int64_t e, const int32_t* d, T& fr, T& fi) {
-  const T *angular = a.angular + e * a.n_f * 2, *t = a.transport + e * a.n_f * 2, *scale = a.rho + e * (SCALED ? a.n_scales : 1);
-  fr = T(1);
-  fi = T(0);
-  const int ang = d[3], trn = d[4], power = d[5];
-  if (ang != 0) {
-    const int o = ang < 0 ? -ang : ang;
-    const T pr = angular[2 * o], pi = ang < 0 ? -angular[2 * o + 1] : angular[2 * o + 1];
-    const T nr = fr * pr - fi * pi, ni = fr * pi + fi * pr;
-    fr = nr;
-    fi = ni;
-  }
-  if (trn != 0) {
-    const int o = trn < 0 ? -trn : trn;
-    const T pr = t[2 * o], pi = trn < 0 ? -t[2 * o + 1] : t[2 * o + 1];
-    const T nr = fr * pr - fi * pi, ni = fr * pi + fi * pr;
-    fr = nr;
-    fi = ni;
-  }
-  T s = T(1);
-  if constexpr (SCALED) {
-    s = scale[power];
-  } else {
-    const T r = scale[0];
-    for (int x = 0; x < power; ++x) s *= r;
-  }
-  fr *= s;
-  fi *= s;
-}
-
 // Z(j) of one node into shared memory: row t = [zc (wc, 2) | zr (wr)], `pitch` elements apart; asynchronous.
 template <typename T>
 __device__ __forceinline__ void stage_node(const FArgs<T>& a, int64_t j, T* z_s, int pitch) {
@@ -662,6 +614,8 @@ extern "C" int gm_factored_forward_scaled(const void* h, const void* zc, const v
     a.h = (const T*)h; a.zc = (const T*)zc; a.zr = (const T*)zr; a.angular = (const T*)angular; a.transport = (const T*)transport;
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.out = (T*)out;
+    if constexpr (sizeof(T) == 4)
+      if (tensor_cores_forward(a)) return forward_tc(a, (cudaStream_t)stream);
     const int C = 2 * wc + wr;
     const size_t extra = (size_t)(n_blocks * FDESC) * sizeof(int32_t) + (size_t)(n_blocks + d_out) * sizeof(int4);
     // 64 or 32 edges per tile; fewer where the packed width or the phase tables leave no room for them
@@ -732,6 +686,8 @@ extern "C" int gm_factored_backward_scaled(const void* g, const int64_t* target,
     a.rho = (const T*)rho; a.desc = desc; a.source = source; a.order = order; a.group_ptr = group_ptr; a.group_source = group_source;
     a.g = (const T*)g; a.target = target; a.weights = aggregated ? (const T*)weights : nullptr; a.rows = aggregated ? (const T*)rows : nullptr;
     a.dh = (T*)dh; a.dzc = (T*)dzc; a.dzr = (T*)dzr; a.dweights = aggregated ? (T*)dweights : nullptr;
+    if constexpr (sizeof(T) == 4)
+      if (tensor_cores_backward(a)) return backward_tc(a, (cudaStream_t)stream);
     // 64 or 32 edges per tile; fewer where the packed width is so large that they do not fit shared memory
     int tile = MAX_TILE;
     auto layout = [&](bool staged) { return BackwardLayout<T>(k, C, n_f, n_scales, d_out, tile, staged); };

@@ -194,6 +194,49 @@ def test_factored_against_plain_sums(type_in, type_out, k, degrees, dtype):
         assert rel_err(a.cpu().numpy(), b.numpy()) < tolerance, name
 
 
+@pytest.mark.parametrize("scales", [0, 3])
+@pytest.mark.parametrize("type_in, type_out, k, degrees", [
+    ({0: 8, 1: 8, 2: 8}, {0: 4, 1: 4, 2: 4}, 17, [92, 16, 0, 129, 17, 47]),  # full trunk; steps of 16 edges: exact, one more, one less
+    ({0: 2, 1: 2}, {0: 4, 1: 4}, 2, [64, 100]),                            # one trunk output
+    ({0: 2, 1: 2}, {0: 3, 1: 9}, 16, [64, 65, 63, 300]),                   # uneven blocks: a round more than their mean asks for; an odd trunk
+    ({1: 3}, {0: 5, 2: 5}, 6, [130, 200]),                                 # no scalar block; gradient rows of an odd width
+    ({0: 2, 1: 2, 2: 2}, {0: 25, 1: 25, 2: 25}, 11, [90, 33]),             # 91 tiles: three rounds of 32 backward
+])
+def test_factored_tensor_cores_against_float64(type_in, type_out, k, degrees, scales):
+    """Rows, weighted sums' gradients and all others of the float32 kernels that sources of many edges take, against the float64
+    kernels (which the tests above pin) on the same numbers: sums of at most 300 edges x 19 trunk outputs or 575 columns of O(1)
+    terms whose rounding errors of 2^-24 add up like their square root, 2e-6 of each tensor's norm."""
+    from gm_attention_b200.fields import FieldType
+    from gm_attention_b200.nn import fused_factored as ff
+
+    blocks, powers = blocks_for(type_in, type_out)
+    p = ff.plan_blocks(blocks, FieldType(type_out), powers)
+    n_f, n = 8, len(degrees)
+    rng = np.random.default_rng(15)
+    source = rng.permutation(np.repeat(np.arange(n), degrees))
+    e = source.shape[0]
+    phase = np.exp(1j * rng.uniform(0, 6.28, (2, e, n_f)))
+    angular, transport = (np.stack([x.real, x.imag], -1) for x in phase)
+    rho = rng.uniform(0.1, 1.0, (e, scales) if scales else e)
+    desc = np.array([b.row() for b in p.blocks], np.int32).reshape(-1, 8)
+    if scales:
+        desc[:, 5] %= scales
+    values = [x.astype(np.float32) for x in (rng.standard_normal((e, k - 1)), rng.standard_normal((n, k, p.wc, 2)), rng.standard_normal((n, k, p.wr)),
+                                             angular, transport, rho)]
+    targets = np.sort(rng.integers(0, 5, e))
+    g, weights = rng.standard_normal((5, p.d_out)).astype(np.float32), rng.standard_normal(e).astype(np.float32)
+    groups = [x.cuda() for x in ff.source_groups(torch.from_numpy(source))]
+    ext, results = ff.extension(True), []
+    for dtype in (np.float32, np.float64):
+        args = (*(cuda(x.astype(dtype)) for x in values), cuda(desc), cuda(source))
+        rows = ext.forward(*args, *groups, p.d_out, p.max_bm, bool(scales))
+        plain = ext.backward(rows, *args, *groups, bool(scales))
+        summed = [] if scales else ext.backward_aggregated(cuda(g.astype(dtype)), cuda(targets), cuda(weights.astype(dtype)), rows, *args, *groups)
+        results.append((rows, *plain, *summed))
+    for x, (a, b) in enumerate(zip(*results)):
+        assert a.shape == b.shape and (b.numel() == 0 or float((a.double() - b).norm() / b.norm()) < 2e-6), x
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_factored_sources_without_edges(dtype):
     """A grouping that lists every node, most of them with an empty run between two full ones (more runs than the forward
