@@ -25,6 +25,65 @@ constexpr int MAX_H = 8;
 constexpr int MAX_F = 8;
 constexpr int DESC = 5;
 
+template <typename T> struct Pair;
+template <> struct Pair<float> { using type = float2; };
+template <> struct Pair<double> { using type = double2; };
+
+// (x, y) at p: one vector access when the address allows it: decided from the address itself, or (VEC) known by the caller
+template <bool VEC, typename T>
+__device__ __forceinline__ void load_pair(const T* p, T& x, T& y) {
+  if (VEC || (reinterpret_cast<uintptr_t>(p) & (2 * sizeof(T) - 1)) == 0) {
+    const typename Pair<T>::type t = *reinterpret_cast<const typename Pair<T>::type*>(p);
+    x = t.x; y = t.y;
+  } else {
+    x = p[0]; y = p[1];
+  }
+}
+template <bool VEC, typename T>
+__device__ __forceinline__ void store_pair(T* p, T x, T y) {
+  if (VEC || (reinterpret_cast<uintptr_t>(p) & (2 * sizeof(T) - 1)) == 0) {
+    typename Pair<T>::type t;
+    t.x = x; t.y = y;
+    *reinterpret_cast<typename Pair<T>::type*>(p) = t;
+  } else {
+    p[0] = x; p[1] = y;
+  }
+}
+// Whether all of these addresses (as bits set in any of them) are those of pairs
+template <typename T> __device__ __forceinline__ bool whole_pairs(uintptr_t bits) { return (bits & (2 * sizeof(T) - 1)) == 0; }
+template <typename T> __device__ __forceinline__ uintptr_t bits_of(const T* p) { return reinterpret_cast<uintptr_t>(p); }
+
+// f(t, n, j) for the edges t .. t + n - 1 of a node's `degree` and their sources j that are this turn's of `turns`: U at a time,
+// the last ones one at a time; AHEAD: the sources are read while the U edges before them are worked on.
+template <int U, bool AHEAD, typename F>
+__device__ __forceinline__ void for_edges(int turn, int turns, int degree, const int64_t* source, const F& f) {
+  auto single = [&](int t) {
+    for (; t < degree; ++t) f(t, std::integral_constant<int, 1>(), [&](int) { return (unsigned)source[t]; });
+  };
+  if constexpr (AHEAD) {
+    unsigned ahead[U];
+    auto read = [&](int from) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) ahead[u] = (unsigned)source[from + u];
+    };
+    int t = U * turn;
+    if (t + U <= degree) read(t);
+    for (; t + U <= degree; t += U * turns) {
+      unsigned j[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) j[u] = ahead[u];
+      if (t + U * turns + U <= degree) read(t + U * turns);
+      f(t, std::integral_constant<int, U>(), [&](int u) { return j[u]; });
+    }
+    single(t);
+  } else {
+    for (int t = U * turn; t < degree; t += U * turns) {
+      if (t + U <= degree) f(t, std::integral_constant<int, U>(), [&](int u) { return (unsigned)source[t + u]; });
+      else single(t);
+    }
+  }
+}
+
 // ------------------------------------------------------------------ softmax
 
 template <typename T>
@@ -36,6 +95,7 @@ struct SoftmaxArgs {
   int64_t n_nodes;
   int D, F, orders, H;
   int slots;  // shared-memory logit slots per block (0: keep the logits in alpha)
+  int shares;  // grouped scores: groups of a warp's lanes that take a target's edges in turn
   T scale;
 };
 
@@ -124,7 +184,7 @@ int score_parts(int64_t n_nodes, int64_t n_edges, int64_t deg_max, int H) {
   return n_edges <= 4096 * deg_max || (H == 8 && n_edges >= 16 * n_nodes) ? 2 : 1;
 }
 
-template <typename T, int R, int NF, int PARTS>
+template <typename T, int R, int NF, int PARTS, bool SHARED>
 __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArgs<T> a) {
   constexpr int FN = NF ? NF : MAX_F, TARGETS = 4 / PARTS;
   __shared__ T max_s[TARGETS][PARTS][MAX_H], sum_s[TARGETS][PARTS][MAX_H];
@@ -132,8 +192,12 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
   const int64_t x = (int64_t)blockIdx.x * TARGETS + mine;
   const bool present = x < a.n_nodes;
   const int64_t i = present ? from_both_ends(x, a.n_nodes) : 0;
-  const int L = 32 / a.H, h = lane / L, s = lane % L;
+  // narrow heads leave lanes free: a.shares groups of H heads' lanes take the target's edges in turn
+  const int shares = SHARED ? a.shares : 1, full = 32 / a.H, L = full / shares;
+  const int share = SHARED ? lane / (a.H * L) : 0, h = SHARED ? lane / L % a.H : lane / L, s = lane % L;
+  const unsigned group_mask = SHARED ? ((1u << (a.H * L)) - 1u) << (share * a.H * L) : 0xffffffffu;
   int col[FN][R], order[FN];
+  uintptr_t bits = bits_of(a.k) | bits_of(a.transport) | (uintptr_t)a.D * sizeof(T);
   T qr[FN][R], qi[FN][R];
 #pragma unroll
   for (int f = 0; f < FN; ++f) {
@@ -143,6 +207,7 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
     if (NF || f < a.F) {
       const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2];
       order[f] = n;
+      if (n != 0) bits |= (uintptr_t)off * sizeof(T);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int u = s + L * r;
@@ -155,63 +220,61 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
     }
   }
   const int64_t e0 = a.row_ptr[i], e1 = present ? a.row_ptr[i + 1] : e0;
+  const int degree = (int)(e1 - e0);
+  const int64_t* source = a.source + e0;
+  const T *transport = a.transport + e0 * a.orders * 2, *bias = a.bias + e0;
+  const uint8_t* inside = a.inside + e0;
+  T* const alpha = a.alpha + e0 * a.H + h;
   T m = neg_inf<T>();
-  // this lane's share of <q_i, tau k_j> for one edge
-  auto dot = [&](const T* k_j, const T* tau) -> T {
-    T part = T(0);
+  constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together (8: 0.96 ms against 0.88)
+  auto walk = [&](auto is_vec) {  // every (re, im) and phase is read as a pair
+    constexpr bool VEC = decltype(is_vec)::value;
+    // this lane's share of <q_i, tau k_j> for one edge
+    auto dot = [&](int t, unsigned j) -> T {
+      const T *k_j = a.k + (size_t)j * (unsigned)a.D, *tau = transport + (size_t)(unsigned)t * (2u * a.orders);
+      T sum = T(0);
 #pragma unroll
-    for (int f = 0; f < FN; ++f) {
-      if (!NF && order[f] < 0) continue;
-      const T tr = order[f] ? tau[2 * order[f]] : T(1), ti = order[f] ? tau[2 * order[f] + 1] : T(0);
+      for (int f = 0; f < FN; ++f) {
+        if (!NF && order[f] < 0) continue;
+        T tr = T(1), ti = T(0);
+        if (order[f]) load_pair<VEC>(tau + 2 * order[f], tr, ti);
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        if (col[f][r] < 0) continue;
-        if (order[f] == 0) {
-          part += qr[f][r] * k_j[col[f][r]];
-        } else {
-          const T kr = k_j[col[f][r]], ki = k_j[col[f][r] + 1];
-          part += qr[f][r] * (tr * kr - ti * ki) + qi[f][r] * (tr * ki + ti * kr);
+        for (int r = 0; r < R; ++r) {
+          if (col[f][r] < 0) continue;
+          if (order[f] == 0) {
+            sum += qr[f][r] * k_j[col[f][r]];
+          } else {
+            T kr, ki;
+            load_pair<VEC>(k_j + col[f][r], kr, ki);
+            sum += qr[f][r] * (tr * kr - ti * ki) + qi[f][r] * (tr * ki + ti * kr);
+          }
         }
       }
-    }
-    return part;
-  };
-  auto finish = [&](int64_t e, T part) {
-    const T lw = a.scale * part + a.bias[e];
-    if (a.inside[e] && lw > m) m = lw;
-    if (s == 0) a.alpha[e * a.H + h] = lw;
-  };
-  constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together (8: 0.96 ms against 0.88)
-  auto several = [&](int64_t e) {
-    const T* k_j[U];
-    T part_sum[U];
+      return sum;
+    };
+    auto edges = [&](int t, auto count, auto from) {
+      constexpr int N = decltype(count)::value;
+      T sum[N];
 #pragma unroll
-    for (int u = 0; u < U; ++u) k_j[u] = a.k + a.source[e + u] * a.D;
+      for (int u = 0; u < N; ++u) sum[u] = dot(t + u, from(u));
+      for (int o = L >> 1; o > 0; o >>= 1) {
 #pragma unroll
-    for (int u = 0; u < U; ++u) part_sum[u] = dot(k_j[u], a.transport + (e + u) * a.orders * 2);
-    for (int o = L >> 1; o > 0; o >>= 1) {
+        for (int u = 0; u < N; ++u) sum[u] += __shfl_xor_sync(group_mask, sum[u], o);
+      }
 #pragma unroll
-      for (int u = 0; u < U; ++u) part_sum[u] += __shfl_xor_sync(0xffffffffu, part_sum[u], o);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) finish(e + u, part_sum[u]);
+      for (int u = 0; u < N; ++u) {
+        const T lw = a.scale * sum[u] + bias[t + u];
+        if (inside[t + u] && lw > m) m = lw;
+        if (s == 0) alpha[(size_t)(unsigned)(t + u) * (unsigned)a.H] = lw;
+      }
+    };
+    for_edges<U, false>(part * shares + share, PARTS * shares, degree, source, edges);
   };
-  auto rest = [&](int64_t e) {
-    for (; e < e1; ++e) {
-      T one = dot(a.k + a.source[e] * a.D, a.transport + e * a.orders * 2);
-      for (int o = L >> 1; o > 0; o >>= 1) one += __shfl_xor_sync(0xffffffffu, one, o);
-      finish(e, one);
-    }
-  };
-  if constexpr (PARTS == 1 && NF != 4) {  // (four frequencies: the other form is the faster, 40 962 points of degree 12, 8 heads 203 -> 188 us)
-    int64_t e = e0;
-    for (; e + U <= e1; e += U) several(e);
-    rest(e);
-  } else {
-    for (int64_t e = e0 + U * part; e < e1; e += U * PARTS) {
-      if (e + U <= e1) several(e);
-      else rest(e);
-    }
+  if (whole_pairs<T>(bits)) walk(std::true_type());
+  else walk(std::false_type());
+  for (int o = a.H * L; SHARED && o < 32; o <<= 1) {
+    const T other = __shfl_xor_sync(0xffffffffu, m, o);
+    m = other > m ? other : m;
   }
   if constexpr (PARTS > 1) {
     if (s == 0) max_s[mine][part][h] = m;
@@ -221,34 +284,35 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
   } else {
     __syncwarp();
   }
-  // normalise: the group's lanes stride the row's edges for their head.  The sum is that of two halves (every other L edges),
+  // normalise: a head's lanes stride the row's edges.  The sum is that of two halves (every other `full` edges),
   // so that one warp gets the bits of two: a chunk of an edge set may be given to one, the whole set to two
-  auto weigh = [&](int64_t e) {
-    const T u = a.inside[e] ? gm_exp(a.alpha[e * a.H + h] - m) : T(0);
-    a.alpha[e * a.H + h] = u;
+  const int place = s + L * share;
+  auto head_sum = [&](T v) {
+    for (int o = full >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, SHARED && o >= L ? o / L * (a.H * L) : o);
+    return v;
+  };
+  auto weigh = [&](int t) {
+    const T u = inside[t] ? gm_exp(alpha[(size_t)(unsigned)t * (unsigned)a.H] - m) : T(0);
+    alpha[(size_t)(unsigned)t * (unsigned)a.H] = u;
     return u;
   };
   T sum = T(0);
   if constexpr (PARTS > 1) {
     static_assert(PARTS == 2, "as many halves as there are");
-    for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) sum += weigh(e);
-    for (int o = L >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (s == 0) sum_s[mine][part][h] = sum;
+    for (int t = place + full * part; t < degree; t += full * PARTS) sum += weigh(t);
+    sum = head_sum(sum);
+    if (place == 0) sum_s[mine][part][h] = sum;
     __syncthreads();
     sum = sum_s[mine][0][h] + sum_s[mine][1][h];
   } else {
     T other = T(0);
-    for (int64_t e = e0 + s; e < e1; e += 2 * L) {
-      sum += weigh(e);
-      if (e + L < e1) other += weigh(e + L);
+    for (int t = place; t < degree; t += 2 * full) {
+      sum += weigh(t);
+      if (t + full < degree) other += weigh(t + full);
     }
-    for (int o = L >> 1; o > 0; o >>= 1) {
-      sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      other += __shfl_xor_sync(0xffffffffu, other, o);
-    }
-    sum += other;
+    sum = head_sum(sum) + head_sum(other);
   }
-  for (int64_t e = e0 + s + L * part; e < e1; e += L * PARTS) a.alpha[e * a.H + h] /= sum;
+  for (int t = place + full * part; t < degree; t += full * PARTS) alpha[(size_t)(unsigned)t * (unsigned)a.H] /= sum;
 }
 
 // ------------------------------------------------------------------ depthwise conv
@@ -263,9 +327,10 @@ struct ConvArgs {
 };
 
 template <typename T>
-__device__ __forceinline__ T rho_power(T rho, int n) {  // (r / c)^{2n} by repeated multiplication from 1
-  T s = T(1);
-  for (int i = 0; i < 2 * n; ++i) s *= rho;
+__device__ __forceinline__ T rho_power(T rho, int n) {  // (r / c)^{2n} by repeated multiplication from 1 (n >= 1)
+  const T two = rho * rho, four = two * rho * rho;
+  T s = n == 1 ? two : four;
+  for (int i = 2; i < n; ++i) s = s * rho * rho;
   return s;
 }
 
@@ -277,31 +342,21 @@ struct ConvItem {
   int mult;
 };
 
-template <typename T> struct Pair;
-template <> struct Pair<float> { using type = float2; };
-template <> struct Pair<double> { using type = double2; };
-
-// (x, y) at p: one vector access when the address allows it (decided from the address itself), two scalar ones otherwise
-template <typename T>
-__device__ __forceinline__ void load_pair(const T* p, T& x, T& y) {
-  if ((reinterpret_cast<uintptr_t>(p) & (2 * sizeof(T) - 1)) == 0) {
-    const typename Pair<T>::type t = *reinterpret_cast<const typename Pair<T>::type*>(p);
-    x = t.x; y = t.y;
-  } else {
-    x = p[0]; y = p[1];
+// A warp's lanes on up to 32 items: as many groups of lanes as there is room for (4 lanes at least), which take a node's edges in
+// turn.
+struct Lanes {
+  int width, item, group, groups;
+  __device__ __forceinline__ Lanes(int lane, int n) {
+    width = n > 16 ? 32 : n > 8 ? 16 : n > 4 ? 8 : 4;
+    item = lane & (width - 1);
+    group = lane / width;
+    groups = 32 / width;
   }
-}
-template <typename T>
-__device__ __forceinline__ void store_pair(T* p, T x, T y) {
-  if ((reinterpret_cast<uintptr_t>(p) & (2 * sizeof(T) - 1)) == 0) {
-    typename Pair<T>::type t;
-    t.x = x; t.y = y;
-    *reinterpret_cast<typename Pair<T>::type*>(p) = t;
-  } else {
-    p[0] = x; p[1] = y;
+  template <typename T> __device__ __forceinline__ T sum(T v) const {  // over the groups
+    for (int o = width; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
   }
-}
-
+};
 // p[0] += x, p[1] += y.  A float pair on an 8-byte boundary is one vector reduction: half as many operations for the L2
 // units.  128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32: 1 098 -> 897 us for the scores' backward.  (The
 // depthwise backward and the fused layer's on general graphs lose by it, 1 045 -> 1 190 and 363 -> 394 us.)
@@ -323,102 +378,111 @@ struct ScoreItem {
 };
 
 // Backward of scores + softmax: a warp per target node.  The lanes first reduce sum_e alpha dalpha per head, then
-// every lane owns one item and walks the node's edges in order (dq is a sequential sum per column), four edges'
-// gathers in flight; dk is accumulated atomically.
-template <typename T, bool VECTOR>
+// every lane owns one item and walks the node's edges, four edges' gathers in flight; dk is accumulated atomically.
+// VECTOR: pairs of it by one reduction; VEC: every pair is read and written as one.
+template <bool VECTOR, bool VEC, bool AHEAD, typename T>
+__device__ __forceinline__ void softmax_backward_node(const SoftmaxArgs<T>& a, const ScoreItem* items_s, int n_items, int n_real, int64_t i) {
+  const int lane = threadIdx.x & 31;
+  constexpr int U = 4;
+  const int64_t e0 = a.row_ptr[i];
+  const int degree = (int)(a.row_ptr[i + 1] - e0);
+  const T *alpha = a.alpha_in + e0 * a.H, *dalpha = a.dalpha + e0 * a.H, *transport = a.transport + e0 * a.orders * 2;
+  const int64_t* source = a.source + e0;
+  T total_of_lane = T(0);  // lane h < H ends up with sum_e alpha[e, h] dalpha[e, h]
+  for (int h = 0; h < a.H; ++h) {
+    T total = T(0);
+    for (int t = lane; t < degree; t += 32) total += alpha[(size_t)t * a.H + h] * dalpha[(size_t)t * a.H + h];
+    total = warp_sum(total);
+    if (lane == h) total_of_lane = total;
+  }
+  for (int t0 = 0; t0 < n_items;) {
+    // a block of 32 items never mixes scalar and complex items
+    const int t1 = t0 < n_real ? min(t0 + 32, n_real) : min(t0 + 32, n_items);
+    const Lanes lanes(lane, t1 - t0);
+    const bool active = t0 + lanes.item < t1;
+    const ScoreItem it = items_s[active ? t0 + lanes.item : t0];
+    const T total = __shfl_sync(0xffffffffu, total_of_lane, it.head);
+    const T *al_at = alpha + it.head, *da_at = dalpha + it.head, *k_at = a.k + it.col;
+    T* dk_at = a.dk + it.col;
+    if (t0 < n_real) {
+      const T q_c = a.q[i * a.D + it.col];
+      T dq = T(0);
+      if (active)
+        for_edges<U, AHEAD>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+          constexpr int N = decltype(count)::value;
+          size_t j[N];
+          T al[N], da[N], kc[N];
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            j[u] = (size_t)from(u) * (unsigned)a.D;
+            al[u] = al_at[(size_t)(unsigned)(t + u) * (unsigned)a.H];
+            da[u] = da_at[(size_t)(unsigned)(t + u) * (unsigned)a.H];
+            kc[u] = k_at[j[u]];
+          }
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            const T ds = a.scale * al[u] * (da[u] - total);
+            dq += ds * kc[u];
+            atomicAdd(dk_at + j[u], ds * q_c);
+          }
+        });
+      dq = lanes.sum(dq);
+      if (active && lanes.group == 0) a.dq[i * a.D + it.col] = dq;
+    } else {
+      T q_r, q_i;
+      load_pair<VEC>(a.q + i * a.D + it.col, q_r, q_i);
+      T dq_r = T(0), dq_i = T(0);
+      const T* tau_at = transport + it.order * 2;
+      const unsigned tau_step = 2 * a.orders;
+      if (active)
+        for_edges<U, AHEAD>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+          constexpr int N = decltype(count)::value;
+          size_t j[N];
+          T al[N], da[N], tr[N], ti[N], kr[N], ki[N];
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            j[u] = (size_t)from(u) * (unsigned)a.D;
+            al[u] = al_at[(size_t)(unsigned)(t + u) * (unsigned)a.H];
+            da[u] = da_at[(size_t)(unsigned)(t + u) * (unsigned)a.H];
+            load_pair<VEC>(tau_at + (size_t)(unsigned)(t + u) * tau_step, tr[u], ti[u]);
+            load_pair<VEC>(k_at + j[u], kr[u], ki[u]);
+          }
+#pragma unroll
+          for (int u = 0; u < N; ++u) {
+            const T ds = a.scale * al[u] * (da[u] - total);
+            dq_r += ds * (tr[u] * kr[u] - ti[u] * ki[u]);  // (tau k)
+            dq_i += ds * (tr[u] * ki[u] + ti[u] * kr[u]);
+            add_pair<VECTOR>(dk_at + j[u], ds * (tr[u] * q_r + ti[u] * q_i), ds * (tr[u] * q_i - ti[u] * q_r));  // conj(tau) q
+          }
+        });
+      dq_r = lanes.sum(dq_r);
+      dq_i = lanes.sum(dq_i);
+      if (active && lanes.group == 0) store_pair<VEC>(a.dq + i * a.D + it.col, dq_r, dq_i);
+    }
+    t0 = t1;
+  }
+}
+
+template <typename T, bool VECTOR, bool AHEAD>
 __global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ScoreItem* items_s = reinterpret_cast<ScoreItem*>(smem_raw);
   int n_items = 0, n_real = 0;
+  uintptr_t bits = bits_of(a.q) | bits_of(a.k) | bits_of(a.transport) | bits_of(a.dq) | (uintptr_t)a.D * sizeof(T);
   for (int f = 0; f < a.F; ++f) {
     const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2], dim = (int)a.desc[f * DESC + 4];
     for (int x = threadIdx.x; x < a.H * a_n; x += blockDim.x) items_s[n_items + x] = ScoreItem{off + dim * x, n, x / a_n, 0};
     n_items += a.H * a_n;
     if (n == 0) n_real = n_items;  // items are in column order: the scalar block first
+    else bits |= (uintptr_t)off * sizeof(T);
   }
   __syncthreads();
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  constexpr int U = 4;
+  const bool vec = whole_pairs<T>(bits);
+  const int warps = blockDim.x >> 5;
   for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
     const int64_t i = from_both_ends(x, a.n_nodes);
-    const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
-    T total_of_lane = T(0);  // lane h < H ends up with sum_e alpha[e, h] dalpha[e, h]
-    for (int h = 0; h < a.H; ++h) {
-      T total = T(0);
-      for (int64_t e = e0 + lane; e < e1; e += 32) total += a.alpha_in[e * a.H + h] * a.dalpha[e * a.H + h];
-      total = warp_sum(total);
-      if (lane == h) total_of_lane = total;
-    }
-    for (int t0 = 0; t0 < n_items; t0 += 32) {
-      // a block of 32 items never mixes scalar and complex items unless it straddles the boundary: split it there
-      const int t1 = (t0 < n_real && t0 + 32 > n_real) ? n_real : min(t0 + 32, n_items);
-      const bool active = t0 + lane < t1;
-      const ScoreItem it = items_s[active ? t0 + lane : t0];
-      const T total = __shfl_sync(0xffffffffu, total_of_lane, it.head);
-      if (active && it.order == 0) {
-        const T q_c = a.q[i * a.D + it.col];
-        T dq = T(0);
-        int64_t e = e0;
-        for (; e + U <= e1; e += U) {
-          int64_t j[U];
-          T al[U], da[U], kc[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            j[u] = a.source[e + u];
-            al[u] = a.alpha_in[(e + u) * a.H + it.head];
-            da[u] = a.dalpha[(e + u) * a.H + it.head];
-            kc[u] = a.k[j[u] * a.D + it.col];
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            const T ds = a.scale * al[u] * (da[u] - total);
-            dq += ds * kc[u];
-            atomicAdd(a.dk + j[u] * a.D + it.col, ds * q_c);
-          }
-        }
-        for (; e < e1; ++e) {
-          const int64_t j = a.source[e];
-          const T ds = a.scale * a.alpha_in[e * a.H + it.head] * (a.dalpha[e * a.H + it.head] - total);
-          dq += ds * a.k[j * a.D + it.col];
-          atomicAdd(a.dk + j * a.D + it.col, ds * q_c);
-        }
-        a.dq[i * a.D + it.col] = dq;
-      } else if (active) {
-        T q_r, q_i;
-        load_pair(a.q + i * a.D + it.col, q_r, q_i);
-        T dq_r = T(0), dq_i = T(0);
-        auto edge = [&](int64_t j, T al, T da, T tr, T ti, T kr, T ki) {
-          const T ds = a.scale * al * (da - total);
-          dq_r += ds * (tr * kr - ti * ki);  // (tau k)
-          dq_i += ds * (tr * ki + ti * kr);
-          add_pair<VECTOR>(a.dk + j * a.D + it.col, ds * (tr * q_r + ti * q_i), ds * (tr * q_i - ti * q_r));  // conj(tau) q
-        };
-        int64_t e = e0;
-        for (; e + U <= e1; e += U) {
-          int64_t j[U];
-          T al[U], da[U], tr[U], ti[U], kr[U], ki[U];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            j[u] = a.source[e + u];
-            al[u] = a.alpha_in[(e + u) * a.H + it.head];
-            da[u] = a.dalpha[(e + u) * a.H + it.head];
-            load_pair(a.transport + ((e + u) * a.orders + it.order) * 2, tr[u], ti[u]);
-            load_pair(a.k + j[u] * a.D + it.col, kr[u], ki[u]);
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) edge(j[u], al[u], da[u], tr[u], ti[u], kr[u], ki[u]);
-        }
-        for (; e < e1; ++e) {
-          const int64_t j = a.source[e];
-          T tr, ti, kr, ki;
-          load_pair(a.transport + (e * a.orders + it.order) * 2, tr, ti);
-          load_pair(a.k + j * a.D + it.col, kr, ki);
-          edge(j, a.alpha_in[e * a.H + it.head], a.dalpha[e * a.H + it.head], tr, ti, kr, ki);
-        }
-        store_pair(a.dq + i * a.D + it.col, dq_r, dq_i);
-      }
-      if (t1 != min(t0 + 32, n_items)) t0 = t1 - 32;  // resume at the boundary
-    }
+    if (vec) softmax_backward_node<VECTOR, true, AHEAD>(a, items_s, n_items, n_real, i);
+    else softmax_backward_node<VECTOR, false, AHEAD>(a, items_s, n_items, n_real, i);
   }
 }
 
@@ -436,191 +500,193 @@ __device__ __forceinline__ int build_conv_items(const int64_t* desc, int F, Conv
 }
 
 // Depthwise conv, forward: a warp per target node, a lane per item (scalar items and complex items in separate
-// passes, so a pass never diverges); the node's edges are walked in order -- same summation order per output as a
-// sequential loop -- four at a time, with the four edges' loads issued before their arithmetic.
+// passes, so a pass never diverges); the node's edges are walked four at a time, with the four edges' loads issued before their
+// arithmetic.
 constexpr int CONV_UNROLL = 4, CONV_BACKWARD_UNROLL = 3;  // (backward: 1 033 us with four, 950 with three, 1 083 with two; forward 682, 714, 856)
 
-template <typename T>
-__global__ void conv_forward_kernel(ConvArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ConvItem* items_s = reinterpret_cast<ConvItem*>(smem_raw);
-  const int n_items = build_conv_items(a.desc, a.F, items_s);
-  __syncthreads();
-  int n_real = 0;  // items are in column order: the scalar block (frequency 0) first
-  while (n_real < n_items && items_s[n_real].order == 0) ++n_real;
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
-    const int64_t i = from_both_ends(x, a.n_nodes);
-    const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
-    for (int t0 = 0; t0 < n_real; t0 += 32) {
-      if (t0 + lane >= n_real) continue;
-      const ConvItem it = items_s[t0 + lane];
-      T y = T(0);
-      int64_t e = e0;
-      for (; e + CONV_UNROLL <= e1; e += CONV_UNROLL) {
-        T w[CONV_UNROLL], r[CONV_UNROLL], x[CONV_UNROLL];
+template <bool VEC, typename T>
+__device__ __forceinline__ void conv_forward_node(const ConvArgs<T>& a, const ConvItem* items_s, int n_items, int n_real, int64_t i) {
+  const int lane = threadIdx.x & 31;
+  const int64_t e0 = a.row_ptr[i];
+  const int degree = (int)(a.row_ptr[i + 1] - e0);
+  const int64_t* source = a.source + e0;
+  const T* weights = a.weights + e0;
+  for (int t0 = 0; t0 < n_real; t0 += 32) {
+    const Lanes lanes(lane, n_real - t0);
+    const bool active = t0 + lanes.item < n_real;
+    const ConvItem it = items_s[active ? t0 + lanes.item : t0];
+    const T *r_at = a.rc + e0 * a.A0 + it.coef, *v_at = a.v + it.col;
+    T y = T(0);
+    if (active)
+      for_edges<CONV_UNROLL, true>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+        constexpr int N = decltype(count)::value;
+        T w[N], r[N], x[N];
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) {
-          w[u] = a.weights[e + u];
-          r[u] = a.rc[(e + u) * a.A0 + it.coef];
-          x[u] = a.v[a.source[e + u] * a.D + it.col];
+        for (int u = 0; u < N; ++u) {
+          w[u] = weights[t + u];
+          r[u] = r_at[(size_t)(unsigned)(t + u) * (unsigned)a.A0];
+          x[u] = v_at[(size_t)from(u) * (unsigned)a.D];
         }
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) y += w[u] * (r[u] * x[u]);
-      }
-      for (; e < e1; ++e) y += a.weights[e] * (a.rc[e * a.A0 + it.coef] * a.v[a.source[e] * a.D + it.col]);
-      a.out[i * a.D + it.col] = y;
-    }
-    for (int t0 = n_real; t0 < n_items; t0 += 32) {
-      if (t0 + lane >= n_items) continue;
-      const ConvItem it = items_s[t0 + lane];
-      const int n = it.order;
-      T yr = T(0), yi = T(0);
-      auto message = [&](T w_e, T rho, T tr, T ti, T vr, T vi, T Ar, T Ai, T Br, T Bi, T ar, T ai) {
-        const T zr = tr * vr - ti * vi, zi = tr * vi + ti * vr;  // z = tau v
-        const T p = rho_power(rho, n);
-        const T wr = p * ar, wi = p * ai;
-        // m = A z + w (B conj z)
-        const T bzr = Br * zr + Bi * zi, bzi = Bi * zr - Br * zi;
-        const T mr = (Ar * zr - Ai * zi) + (wr * bzr - wi * bzi);
-        const T mi = (Ar * zi + Ai * zr) + (wr * bzi + wi * bzr);
-        yr += w_e * mr;
-        yi += w_e * mi;
-      };
-      int64_t e = e0;
-      for (; e + CONV_UNROLL <= e1; e += CONV_UNROLL) {
-        T w[CONV_UNROLL], rho[CONV_UNROLL], tr[CONV_UNROLL], ti[CONV_UNROLL], vr[CONV_UNROLL], vi[CONV_UNROLL];
-        T Ar[CONV_UNROLL], Ai[CONV_UNROLL], Br[CONV_UNROLL], Bi[CONV_UNROLL], ar[CONV_UNROLL], ai[CONV_UNROLL];
+        for (int u = 0; u < N; ++u) y += w[u] * (r[u] * x[u]);
+      });
+    y = lanes.sum(y);
+    if (active && lanes.group == 0) a.out[i * a.D + it.col] = y;
+  }
+  for (int t0 = n_real; t0 < n_items; t0 += 32) {
+    const Lanes lanes(lane, n_items - t0);
+    const bool active = t0 + lanes.item < n_items;
+    const ConvItem it = items_s[active ? t0 + lanes.item : t0];
+    const int n = it.order;
+    const T *rho_at = a.rho + e0, *v_at = a.v + it.col, *co_at = a.cc + e0 * a.W + it.coef;
+    const T *tau_at = a.transport + (e0 * a.orders + n) * 2, *ang_at = a.angular + (e0 * a.orders + 2 * n) * 2;
+    const unsigned phase_step = 2 * a.orders;
+    const int behind = 2 * it.mult;
+    T yr = T(0), yi = T(0);
+    if (active)
+      for_edges<CONV_UNROLL, true>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+        constexpr int N = decltype(count)::value;
+        T w[N], rho[N], tr[N], ti[N], vr[N], vi[N], Ar[N], Ai[N], Br[N], Bi[N], ar[N], ai[N];
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) {
-          const int64_t eu = e + u;
-          w[u] = a.weights[eu];
-          rho[u] = a.rho[eu];
-          load_pair(a.v + a.source[eu] * a.D + it.col, vr[u], vi[u]);
-          load_pair(a.transport + (eu * a.orders + n) * 2, tr[u], ti[u]);
-          load_pair(a.angular + (eu * a.orders + 2 * n) * 2, ar[u], ai[u]);
-          const T* co = a.cc + eu * a.W + it.coef;
-          load_pair(co, Ar[u], Ai[u]);
-          load_pair(co + 2 * it.mult, Br[u], Bi[u]);
+        for (int u = 0; u < N; ++u) {
+          const unsigned x = t + u;
+          w[u] = weights[x];
+          rho[u] = rho_at[x];
+          load_pair<VEC>(v_at + (size_t)from(u) * (unsigned)a.D, vr[u], vi[u]);
+          load_pair<VEC>(tau_at + (size_t)x * phase_step, tr[u], ti[u]);
+          load_pair<VEC>(ang_at + (size_t)x * phase_step, ar[u], ai[u]);
+          const T* co = co_at + (size_t)x * (unsigned)a.W;
+          load_pair<VEC>(co, Ar[u], Ai[u]);
+          load_pair<VEC>(co + behind, Br[u], Bi[u]);
         }
 #pragma unroll
-        for (int u = 0; u < CONV_UNROLL; ++u) message(w[u], rho[u], tr[u], ti[u], vr[u], vi[u], Ar[u], Ai[u], Br[u], Bi[u], ar[u], ai[u]);
-      }
-      for (; e < e1; ++e) {
-        T tr, ti, vr, vi, Ar, Ai, Br, Bi, ar, ai;
-        load_pair(a.transport + (e * a.orders + n) * 2, tr, ti);
-        load_pair(a.v + a.source[e] * a.D + it.col, vr, vi);
-        const T* co = a.cc + e * a.W + it.coef;
-        load_pair(co, Ar, Ai);
-        load_pair(co + 2 * it.mult, Br, Bi);
-        load_pair(a.angular + (e * a.orders + 2 * n) * 2, ar, ai);
-        message(a.weights[e], a.rho[e], tr, ti, vr, vi, Ar, Ai, Br, Bi, ar, ai);
-      }
-      store_pair(a.out + i * a.D + it.col, yr, yi);
-    }
+        for (int u = 0; u < N; ++u) {
+          const T zr = tr[u] * vr[u] - ti[u] * vi[u], zi = tr[u] * vi[u] + ti[u] * vr[u];  // z = tau v
+          const T p = rho_power(rho[u], n);
+          const T wr = p * ar[u], wi = p * ai[u];
+          // m = A z + w (B conj z)
+          const T bzr = Br[u] * zr + Bi[u] * zi, bzi = Bi[u] * zr - Br[u] * zi;
+          const T mr = (Ar[u] * zr - Ai[u] * zi) + (wr * bzr - wi * bzi);
+          const T mi = (Ar[u] * zi + Ai[u] * zr) + (wr * bzi + wi * bzr);
+          yr += w[u] * mr;
+          yi += w[u] * mi;
+        }
+      });
+    yr = lanes.sum(yr);
+    yi = lanes.sum(yi);
+    if (active && lanes.group == 0) store_pair<VEC>(a.out + i * a.D + it.col, yr, yi);
   }
 }
 
 // Backward: same walk and grouping; the edge-owned coefficient gradients are written once, dv is accumulated atomically.
-template <typename T>
-__global__ void conv_backward_kernel(ConvArgs<T> a) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ConvItem* items_s = reinterpret_cast<ConvItem*>(smem_raw);
-  const int n_items = build_conv_items(a.desc, a.F, items_s);
-  __syncthreads();
-  int n_real = 0;
-  while (n_real < n_items && items_s[n_real].order == 0) ++n_real;
-  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
-    const int64_t i = from_both_ends(x, a.n_nodes);
-    const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
-    for (int t0 = 0; t0 < n_real; t0 += 32) {
-      if (t0 + lane >= n_real) continue;
-      const ConvItem it = items_s[t0 + lane];
-      const T dy = a.g[i * a.D + it.col];
-      int64_t e = e0;
-      for (; e + CONV_BACKWARD_UNROLL <= e1; e += CONV_BACKWARD_UNROLL) {
-        T w[CONV_BACKWARD_UNROLL], r[CONV_BACKWARD_UNROLL], x[CONV_BACKWARD_UNROLL];
-        int64_t j[CONV_BACKWARD_UNROLL];
+template <bool VEC, typename T>
+__device__ __forceinline__ void conv_backward_node(const ConvArgs<T>& a, const ConvItem* items_s, int n_items, int n_real, int64_t i) {
+  const int lane = threadIdx.x & 31;
+  const int64_t e0 = a.row_ptr[i];
+  const int degree = (int)(a.row_ptr[i + 1] - e0);
+  const int64_t* source = a.source + e0;
+  const T* weights = a.weights + e0;
+  for (int t0 = 0; t0 < n_real; t0 += 32) {
+    const Lanes lanes(lane, n_real - t0);
+    if (t0 + lanes.item >= n_real) continue;
+    const ConvItem it = items_s[t0 + lanes.item];
+    const T dy = a.g[i * a.D + it.col];
+    const T *r_at = a.rc + e0 * a.A0 + it.coef, *v_at = a.v + it.col;
+    T *dr_at = a.drc + e0 * a.A0 + it.coef, *dv_at = a.dv + it.col;
+    for_edges<CONV_BACKWARD_UNROLL, false>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+      constexpr int N = decltype(count)::value;
+      T w[N], r[N], x[N];
+      size_t j[N];
 #pragma unroll
-        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u) {
-          j[u] = a.source[e + u];
-          w[u] = a.weights[e + u];
-          r[u] = a.rc[(e + u) * a.A0 + it.coef];
-          x[u] = a.v[j[u] * a.D + it.col];
-        }
+      for (int u = 0; u < N; ++u) {
+        j[u] = (size_t)from(u) * (unsigned)a.D;
+        w[u] = weights[t + u];
+        r[u] = r_at[(size_t)(unsigned)(t + u) * (unsigned)a.A0];
+        x[u] = v_at[j[u]];
+      }
 #pragma unroll
-        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u) {
-          const T dm = w[u] * dy;
-          a.drc[(e + u) * a.A0 + it.coef] = dm * x[u];
-          atomicAdd(a.dv + j[u] * a.D + it.col, dm * r[u]);
-        }
+      for (int u = 0; u < N; ++u) {
+        const T dm = w[u] * dy;
+        dr_at[(size_t)(unsigned)(t + u) * (unsigned)a.A0] = dm * x[u];
+        atomicAdd(dv_at + j[u], dm * r[u]);
       }
-      for (; e < e1; ++e) {
-        const int64_t j = a.source[e];
-        const T dm = a.weights[e] * dy;
-        a.drc[e * a.A0 + it.coef] = dm * a.v[j * a.D + it.col];
-        atomicAdd(a.dv + j * a.D + it.col, dm * a.rc[e * a.A0 + it.coef]);
+    });
+  }
+  for (int t0 = n_real; t0 < n_items; t0 += 32) {
+    const Lanes lanes(lane, n_items - t0);
+    if (t0 + lanes.item >= n_items) continue;
+    const ConvItem it = items_s[t0 + lanes.item];
+    const int n = it.order;
+    T dyr, dyi;
+    load_pair<VEC>(a.g + i * a.D + it.col, dyr, dyi);
+    const T *rho_at = a.rho + e0, *v_at = a.v + it.col, *co_at = a.cc + e0 * a.W + it.coef;
+    const T *tau_at = a.transport + (e0 * a.orders + n) * 2, *ang_at = a.angular + (e0 * a.orders + 2 * n) * 2;
+    T *dco_at = a.dcc + e0 * a.W + it.coef, *dv_at = a.dv + it.col;
+    const unsigned phase_step = 2 * a.orders;
+    const int behind = 2 * it.mult;
+    for_edges<CONV_BACKWARD_UNROLL, false>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+      constexpr int N = decltype(count)::value;
+      T w[N], rho[N], tr[N], ti[N], vr[N], vi[N], Ar[N], Ai[N], Br[N], Bi[N], ar[N], ai[N];
+      size_t j[N];
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const unsigned x = t + u;
+        j[u] = (size_t)from(u) * (unsigned)a.D;
+        w[u] = weights[x];
+        rho[u] = rho_at[x];
+        load_pair<VEC>(v_at + j[u], vr[u], vi[u]);
+        load_pair<VEC>(tau_at + (size_t)x * phase_step, tr[u], ti[u]);
+        load_pair<VEC>(ang_at + (size_t)x * phase_step, ar[u], ai[u]);
+        const T* co = co_at + (size_t)x * (unsigned)a.W;
+        load_pair<VEC>(co, Ar[u], Ai[u]);
+        load_pair<VEC>(co + behind, Br[u], Bi[u]);
       }
-    }
-    for (int t0 = n_real; t0 < n_items; t0 += 32) {
-      if (t0 + lane >= n_items) continue;
-      const ConvItem it = items_s[t0 + lane];
-      const int n = it.order;
-      T dyr, dyi;
-      load_pair(a.g + i * a.D + it.col, dyr, dyi);
-      auto edge = [&](int64_t e, int64_t j, T w_e, T rho, T tr, T ti, T vr, T vi, T Ar, T Ai, T Br, T Bi, T ar, T ai) {
-        const T zr = tr * vr - ti * vi, zi = tr * vi + ti * vr;
-        const T p = rho_power(rho, n);
-        const T wr = p * ar, wi = p * ai;
-        const T dmr = w_e * dyr, dmi = w_e * dyi;
+#pragma unroll
+      for (int u = 0; u < N; ++u) {
+        const T zr = tr[u] * vr[u] - ti[u] * vi[u], zi = tr[u] * vi[u] + ti[u] * vr[u];
+        const T p = rho_power(rho[u], n);
+        const T wr = p * ar[u], wi = p * ai[u];
+        const T dmr = w[u] * dyr, dmi = w[u] * dyi;
         // dA = dm conj(z); dB = (dm conj(w)) z
         const T dAr = dmr * zr + dmi * zi, dAi = dmi * zr - dmr * zi;
         const T cr = dmr * wr + dmi * wi, ci2 = dmi * wr - dmr * wi;
         const T dBr = cr * zr - ci2 * zi, dBi = cr * zi + ci2 * zr;
-        const int64_t ci = e * a.W + it.coef;
-        store_pair(a.dcc + ci, dAr, dAi);
-        store_pair(a.dcc + ci + 2 * it.mult, dBr, dBi);
+        T* dco = dco_at + (size_t)(unsigned)(t + u) * (unsigned)a.W;
+        store_pair<VEC>(dco, dAr, dAi);
+        store_pair<VEC>(dco + behind, dBr, dBi);
         // dz = conj(A) dm + w (B conj(dm)); dv = conj(tau) dz
-        const T bdr = Br * dmr + Bi * dmi, bdi = Bi * dmr - Br * dmi;
-        const T dzr = (Ar * dmr + Ai * dmi) + (wr * bdr - wi * bdi);
-        const T dzi = (Ar * dmi - Ai * dmr) + (wr * bdi + wi * bdr);
-        atomicAdd(a.dv + j * a.D + it.col, tr * dzr + ti * dzi);
-        atomicAdd(a.dv + j * a.D + it.col + 1, tr * dzi - ti * dzr);
-      };
-      int64_t e = e0;
-      for (; e + CONV_BACKWARD_UNROLL <= e1; e += CONV_BACKWARD_UNROLL) {
-        T w[CONV_BACKWARD_UNROLL], rho[CONV_BACKWARD_UNROLL], tr[CONV_BACKWARD_UNROLL], ti[CONV_BACKWARD_UNROLL], vr[CONV_BACKWARD_UNROLL], vi[CONV_BACKWARD_UNROLL];
-        T Ar[CONV_BACKWARD_UNROLL], Ai[CONV_BACKWARD_UNROLL], Br[CONV_BACKWARD_UNROLL], Bi[CONV_BACKWARD_UNROLL], ar[CONV_BACKWARD_UNROLL], ai[CONV_BACKWARD_UNROLL];
-        int64_t j[CONV_BACKWARD_UNROLL];
-#pragma unroll
-        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u) {
-          const int64_t eu = e + u;
-          j[u] = a.source[eu];
-          w[u] = a.weights[eu];
-          rho[u] = a.rho[eu];
-          load_pair(a.v + j[u] * a.D + it.col, vr[u], vi[u]);
-          load_pair(a.transport + (eu * a.orders + n) * 2, tr[u], ti[u]);
-          load_pair(a.angular + (eu * a.orders + 2 * n) * 2, ar[u], ai[u]);
-          const T* co = a.cc + eu * a.W + it.coef;
-          load_pair(co, Ar[u], Ai[u]);
-          load_pair(co + 2 * it.mult, Br[u], Bi[u]);
-        }
-#pragma unroll
-        for (int u = 0; u < CONV_BACKWARD_UNROLL; ++u)
-          edge(e + u, j[u], w[u], rho[u], tr[u], ti[u], vr[u], vi[u], Ar[u], Ai[u], Br[u], Bi[u], ar[u], ai[u]);
+        const T bdr = Br[u] * dmr + Bi[u] * dmi, bdi = Bi[u] * dmr - Br[u] * dmi;
+        const T dzr = (Ar[u] * dmr + Ai[u] * dmi) + (wr * bdr - wi * bdi);
+        const T dzi = (Ar[u] * dmi - Ai[u] * dmr) + (wr * bdi + wi * bdr);
+        atomicAdd(dv_at + j[u], tr[u] * dzr + ti[u] * dzi);
+        atomicAdd(dv_at + j[u] + 1, tr[u] * dzi - ti[u] * dzr);
       }
-      for (; e < e1; ++e) {
-        const int64_t j = a.source[e];
-        T tr, ti, vr, vi, Ar, Ai, Br, Bi, ar, ai;
-        load_pair(a.transport + (e * a.orders + n) * 2, tr, ti);
-        load_pair(a.v + j * a.D + it.col, vr, vi);
-        const T* co = a.cc + e * a.W + it.coef;
-        load_pair(co, Ar, Ai);
-        load_pair(co + 2 * it.mult, Br, Bi);
-        load_pair(a.angular + (e * a.orders + 2 * n) * 2, ar, ai);
-        edge(e, j, a.weights[e], a.rho[e], tr, ti, vr, vi, Ar, Ai, Br, Bi, ar, ai);
-      }
+    });
+  }
+}
+
+template <typename T, bool BACKWARD>
+__global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : BACKWARD ? 7 : 6) conv_kernel(ConvArgs<T> a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ConvItem* items_s = reinterpret_cast<ConvItem*>(smem_raw);
+  const int n_items = build_conv_items(a.desc, a.F, items_s);
+  uintptr_t bits = bits_of(a.v) | bits_of(a.cc) | bits_of(a.transport) | bits_of(a.angular) | bits_of(a.out) | bits_of(a.g) | bits_of(a.dcc) |
+                   (uintptr_t)(a.D | a.W) * sizeof(T);
+  for (int f = 0; f < a.F; ++f)
+    if (a.desc[f * DESC] != 0) bits |= (uintptr_t)(a.desc[f * DESC + 2] | a.desc[f * DESC + 3]) * sizeof(T);
+  __syncthreads();
+  const bool vec = whole_pairs<T>(bits);
+  int n_real = 0;  // items are in column order: the scalar block (frequency 0) first
+  while (n_real < n_items && items_s[n_real].order == 0) ++n_real;
+  const int warps = blockDim.x >> 5;
+  for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
+    const int64_t i = from_both_ends(x, a.n_nodes);
+    if constexpr (BACKWARD) {
+      if (vec) conv_backward_node<true>(a, items_s, n_items, n_real, i);
+      else conv_backward_node<false>(a, items_s, n_items, n_real, i);
+    } else {
+      if (vec) conv_forward_node<true>(a, items_s, n_items, n_real, i);
+      else conv_forward_node<false>(a, items_s, n_items, n_real, i);
     }
   }
 }
@@ -642,15 +708,21 @@ int softmax_forward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, int ma
   // head-group kernel when the heads split a warp evenly and every lane owns at most 4 copies per frequency
   if ((a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8) && max_mult > 0 && max_mult <= 4 * (32 / a.H)) {
     const int per_lane = (max_mult + 32 / a.H - 1) / (32 / a.H);
+    a.shares = 1;
+    while (2 * a.shares * max_mult <= 32 / a.H) a.shares *= 2;
     auto go = [&](auto parts) {
       constexpr int P = decltype(parts)::value;
       const unsigned blocks = (unsigned)((a.n_nodes * P + 3) / 4);
-      if (per_lane <= 1 && a.F == 3) softmax_forward_grouped_kernel<T, 1, 3, P><<<blocks, 128, 0, stream>>>(a);
-      else if (per_lane <= 1 && a.F == 4) softmax_forward_grouped_kernel<T, 1, 4, P><<<blocks, 128, 0, stream>>>(a);
-      else if (per_lane <= 1) softmax_forward_grouped_kernel<T, 1, 0, P><<<blocks, 128, 0, stream>>>(a);
-      else if (per_lane <= 2 && a.F == 3) softmax_forward_grouped_kernel<T, 2, 3, P><<<blocks, 128, 0, stream>>>(a);
-      else if (per_lane <= 2) softmax_forward_grouped_kernel<T, 2, 0, P><<<blocks, 128, 0, stream>>>(a);
-      else softmax_forward_grouped_kernel<T, 4, 0, P><<<blocks, 128, 0, stream>>>(a);
+      auto run = [&](auto kernel) { kernel<<<blocks, 128, 0, stream>>>(a); };
+      if (a.shares > 1 && a.F == 3) run(softmax_forward_grouped_kernel<T, 1, 3, P, true>);
+      else if (a.shares > 1 && a.F == 4) run(softmax_forward_grouped_kernel<T, 1, 4, P, true>);
+      else if (a.shares > 1) run(softmax_forward_grouped_kernel<T, 1, 0, P, true>);
+      else if (per_lane <= 1 && a.F == 3) run(softmax_forward_grouped_kernel<T, 1, 3, P, false>);
+      else if (per_lane <= 1 && a.F == 4) run(softmax_forward_grouped_kernel<T, 1, 4, P, false>);
+      else if (per_lane <= 1) run(softmax_forward_grouped_kernel<T, 1, 0, P, false>);
+      else if (per_lane <= 2 && a.F == 3) run(softmax_forward_grouped_kernel<T, 2, 3, P, false>);
+      else if (per_lane <= 2) run(softmax_forward_grouped_kernel<T, 2, 0, P, false>);
+      else run(softmax_forward_grouped_kernel<T, 4, 0, P, false>);
       return launch_status("gm_softmax_forward");
     };
     return score_parts(a.n_nodes, n_edges, deg_max, a.H) == 2 ? go(std::integral_constant<int, 2>()) : go(std::integral_constant<int, 1>());
@@ -674,8 +746,14 @@ int softmax_backward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, cudaS
   // 69 / 67, of degree 100 261 / 232; 64 x 128, radius 2 pi / 64 (mean 38, at most 257) 220 / 200; 128 x 256, radius 3 pi / 128 1 051 / 829.
   const bool pairs = n_edges >= 24 * a.n_nodes || deg_max * a.n_nodes >= 4 * n_edges;
   auto go = [&](auto kernel) { kernel<<<conv_grid(a.n_nodes), CONV_THREADS, a.D * sizeof(ScoreItem), stream>>>(a); };
-  if (pairs) go(softmax_backward_kernel<T, true>);
-  else go(softmax_backward_kernel<T, false>);
+  // sources read ahead where the launch is a few waves of nodes and lasts as long as its chains of gathers: 64 x 128, radius 4 pi / 64, 4
+  // heads of 8 x (m <= 3) 417 -> 350 us, 50 x 100 76 -> 63; more nodes hide the gathers and want the registers (128 x 256 809 -> 883,
+  // 100 x 200 45 -> 53)
+  const bool ahead = a.n_nodes <= 12288;
+  if (pairs && ahead) go(softmax_backward_kernel<T, true, true>);
+  else if (pairs) go(softmax_backward_kernel<T, true, false>);
+  else if (ahead) go(softmax_backward_kernel<T, false, true>);
+  else go(softmax_backward_kernel<T, false, false>);
   return launch_status("gm_softmax_backward");
 }
 
@@ -784,7 +862,7 @@ extern "C" int gm_conv_forward(const void* v, const void* rc, const void* cc, co
     using T = decltype(tag);
     auto a = conv_args<T>(v, rc, cc, transport, angular, rho, weights, desc, row_ptr, source, n_nodes, D, F, orders, A0, W);
     a.out = (T*)out;
-    conv_forward_kernel<T><<<conv_grid(n_nodes), CONV_THREADS, D * sizeof(ConvItem), (cudaStream_t)stream>>>(a);
+    conv_kernel<T, false><<<conv_grid(n_nodes), CONV_THREADS, D * sizeof(ConvItem), (cudaStream_t)stream>>>(a);
     return launch_status("gm_conv_forward");
   };
   return dtype == GM_F32 ? run(float()) : run(double());
@@ -802,7 +880,7 @@ extern "C" int gm_conv_backward(const void* g, const void* v, const void* rc, co
     using T = decltype(tag);
     auto a = conv_args<T>(v, rc, cc, transport, angular, rho, weights, desc, row_ptr, source, n_nodes, D, F, orders, A0, W);
     a.g = (const T*)g; a.dv = (T*)dv; a.drc = (T*)drc; a.dcc = (T*)dcc;
-    conv_backward_kernel<T><<<conv_grid(n_nodes), CONV_THREADS, D * sizeof(ConvItem), (cudaStream_t)stream>>>(a);
+    conv_kernel<T, true><<<conv_grid(n_nodes), CONV_THREADS, D * sizeof(ConvItem), (cudaStream_t)stream>>>(a);
     return launch_status("gm_conv_backward");
   };
   return dtype == GM_F32 ? run(float()) : run(double());

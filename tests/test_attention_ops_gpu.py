@@ -97,6 +97,62 @@ def test_conv_forward_backward(ext, reference_modules, case, dtype):
     assert_close(dcc.cpu().numpy(), dcc_ref, rtol, atol * magnitude(dcc_ref), "dcc")
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("types, heads", [
+    ({0: 4, 1: 4}, 1),         # four items a pass: eight groups of lanes take a node's edges in turn
+    ({0: 8, 1: 5, 2: 3}, 1),   # eight scalar items, eight complex ones, aligned pairs
+    ({0: 3, 1: 9}, 1),         # pairs at odd offsets: read number by number
+    ({1: 17, 3: 16}, 1),       # 33 complex items: a pass of 32 and one of one; the third frequency's power
+    ({0: 4, 1: 4, 2: 4}, 2),   # scores: two heads of four lanes, four groups
+    ({0: 5, 1: 5, 2: 5}, 4),   # five copies in groups of eight lanes
+    ({0: 2, 1: 2, 2: 2, 3: 2}, 8),
+])
+def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
+    """Neighbourhoods of 0 to 130 edges -- fewer than the groups, one more than they take at a time, many turns -- against the oracle
+    in float64: float64 1e-12 of the largest value, float32 2e-6 (sums of at most 130 terms of O(1) and of 2 x 51 products)."""
+    orders = 2 * max(types) + 1
+    degrees = np.array([0, 1, 3, 4, 5, 17, 130, 33, 2, 64, 0, 12])
+    n, e = len(degrees), int(degrees.sum())
+    rng = np.random.default_rng(3)
+    row_ptr = np.concatenate([[0], np.cumsum(degrees)]).astype(np.int64)
+    source = rng.integers(0, n, e).astype(np.int64)
+    phases = np.exp(1j * rng.uniform(0, 6.28, (2, e, 1)) * np.arange(orders))
+    transport, angular = (np.stack([x.real, x.imag], -1) for x in phases)
+    rho, weights, bias = rng.uniform(0.1, 1.0, e), rng.standard_normal(e), rng.standard_normal(e)
+    inside = (rng.random(e) > 0.2).astype(np.uint8)
+    inside[row_ptr[:-1][degrees > 0]] = 1
+    desc, flat, coef = [], 0, 0
+    for f, a in types.items():
+        dim = 1 if f == 0 else 2
+        desc.append([f, a, flat, coef if f else 0, dim])
+        flat += heads * a * dim
+        coef += 4 * a if f else 0
+    desc = np.array(desc, np.int64)
+    cast = lambda *xs: [x.astype(dtype) for x in xs]
+    tolerance = 1e-12 if dtype == np.float64 else 2e-6
+
+    def compare(got, want, names):
+        for name, a, b in zip(names, got, want):
+            assert_close(a.cpu().numpy(), b.astype(dtype), 0.0, tolerance * magnitude(b), name)
+
+    q, k, da = cast(rng.standard_normal((n, flat)), rng.standard_normal((n, flat)), rng.standard_normal((e, heads)))
+    transport, angular, rho, weights, bias = cast(transport, angular, rho, weights, bias)
+    wide = lambda *xs: [x.astype(np.float64) for x in xs]
+    alpha = O.softmax_forward(*wide(q, k, transport, bias), inside, desc, row_ptr, source, heads, 0.3)
+    tables = [cuda(x) for x in (transport, bias, inside, desc, row_ptr, source)]
+    compare([ext.softmax_forward(cuda(q), cuda(k), *tables, heads, 0.3, 130)], [alpha], ["alpha"])
+    want = O.softmax_backward(*wide(da, q, k, transport), desc, row_ptr, source, alpha, heads, 0.3)
+    compare(ext.softmax_backward(cuda(da), cuda(q), cuda(k), *tables, cuda(alpha.astype(dtype)), heads, 0.3, 130), want, ["dq", "dk"])
+    if heads == 1:
+        a0 = types.get(0, 0)
+        rc, cc = cast(rng.standard_normal((e, a0)), rng.standard_normal((e, coef)))
+        edge = [rc, cc, transport, angular, rho, weights]
+        dev = [cuda(x) for x in (*edge, desc, row_ptr, source)]
+        compare([ext.conv_forward(cuda(q), *dev, a0, coef)], [O.conv_forward(*wide(q, *edge), desc, row_ptr, source, a0, coef)], ["out"])
+        want = O.conv_backward(*wide(k, q, *edge), desc, row_ptr, source, a0, coef)
+        compare(ext.conv_backward(cuda(k), cuda(q), *dev, a0, coef), want, ["dv", "drc", "dcc"])
+
+
 def test_softmax_large_neighbourhood_spills_to_global(ext):
     """A row whose logits exceed the shared-memory budget keeps them in alpha."""
     n, deg, heads, d = 3, 30000, 2, 4
