@@ -70,6 +70,7 @@ __device__ __forceinline__ double gm_exp(double x) { return exp(x); }
 __device__ __forceinline__ float gm_log(float x) { return logf(x); }
 __device__ __forceinline__ double gm_log(double x) { return log(x); }
 template <typename T> __device__ __forceinline__ T neg_inf() { return -(T)INFINITY; }
+template <typename T> __device__ __forceinline__ T lowest() { return sizeof(T) == 4 ? -(T)3.402823466e+38 : -(T)1.7976931348623157e+308; }
 
 // The x-th of n items taken from both ends of the list in turn: 0, n - 1, 1, n - 2, ...  On a lattice the nodes of large
 // degree are the polar rows, at the two ends of the node list; in plain order the last of them start when everything else

@@ -17,6 +17,8 @@
 // dO / dq.  Per edge the group reduces its partial dot products with log2(L)
 // xor-shuffles, so all heads' logits appear at once; the softmax is online
 // (running max / sum), the transport rho(n theta) is applied in registers.
+// Heads with few copies need fewer lanes: then several such groups take the
+// target's edges in turn and add up their sums at the end.
 //
 // The geometry (row_ptr, source, tables) describes ONE sample of n_nodes
 // points; the node fields hold `batch` samples back to back and every sample
@@ -37,6 +39,7 @@ constexpr int MAX_F = 8;
 
 struct SlotPlan {
   int n_slots;
+  int form;  // scalar slots where these come first and pairs follow, else 0
   int off[MAX_SLOTS];    // flat offset of the slot's frequency block (all heads)
   int mult[MAX_SLOTS];   // a_n per head
   int order[MAX_SLOTS];  // n (0: scalar)
@@ -55,98 +58,24 @@ struct FusedArgs {
   void *dk, *dv;  // S*, or float* accumulators when S is bf16
   int64_t n_nodes, batch;
   int D, orders, H;
+  int shares;  // groups of a warp's lanes that take a target's edges in turn
   C scale;
   SlotPlan plan;
 };
 
-template <typename T>
-__device__ __forceinline__ T group_sum(T v, int L) {
-  for (int o = L >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-template <typename S, int NS>
-__global__ void __launch_bounds__(256) fused_forward_kernel(FusedArgs<S> a) {
-  using C = typename Compute<S>::type;
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (gw >= a.n_nodes * a.batch) return;
-  const int64_t i = gw / a.batch, b = gw % a.batch;
-  const int L = 32 / a.H, h = lane / L, s = lane % L;
-  const int64_t base = b * a.n_nodes;
-
-  int col[NS];
-  C qr[NS], qi[NS], accr[NS], acci[NS];
-  const S* q_i = a.q + (base + i) * a.D;
-#pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    col[t] = -1;
-    qr[t] = qi[t] = accr[t] = acci[t] = C(0);
-    if (t < a.plan.n_slots) {
-      const int u = s + L * a.plan.round[t], a_n = a.plan.mult[t];
-      if (u < a_n) {
-        const int dim = a.plan.order[t] == 0 ? 1 : 2;
-        col[t] = a.plan.off[t] + dim * (h * a_n + u);
-        qr[t] = ld<C>(q_i + col[t]);
-        if (dim == 2) qi[t] = ld<C>(q_i + col[t] + 1);
-      }
-    }
-  }
-  C m = neg_inf<C>(), l = C(0);
-  const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
-  for (int64_t e = e0; e < e1; ++e) {
-    if (!a.inside[e]) continue;
-    const int64_t j = base + a.source[e];
-    const S* k_j = a.k + j * a.D;
-    const S* v_j = a.v + j * a.D;
-    const C* tau = a.transport + e * a.orders * 2;
-    C part = C(0);
-    C tvr[NS], tvi[NS];
-#pragma unroll
-    for (int t = 0; t < NS; ++t) {
-      tvr[t] = tvi[t] = C(0);
-      if (col[t] >= 0) {
-        const int n = a.plan.order[t];
-        if (n == 0) {
-          part += qr[t] * ld<C>(k_j + col[t]);
-          tvr[t] = ld<C>(v_j + col[t]);
-        } else {
-          const C tr = tau[2 * n], ti = tau[2 * n + 1];
-          const C kr = ld<C>(k_j + col[t]), ki = ld<C>(k_j + col[t] + 1);
-          part += qr[t] * (tr * kr - ti * ki) + qi[t] * (tr * ki + ti * kr);
-          const C vr = ld<C>(v_j + col[t]), vi = ld<C>(v_j + col[t] + 1);
-          tvr[t] = tr * vr - ti * vi;
-          tvi[t] = tr * vi + ti * vr;
-        }
-      }
-    }
-    const C logit = a.scale * group_sum(part, L) + a.bias[e];
-    if (logit > m) {
-      const C corr = gm_exp(m - logit);
-      l *= corr;
-#pragma unroll
-      for (int t = 0; t < NS; ++t) { accr[t] *= corr; acci[t] *= corr; }
-      m = logit;
-    }
-    const C p = gm_exp(logit - m);
-    l += p;
-#pragma unroll
-    for (int t = 0; t < NS; ++t) { accr[t] += p * tvr[t]; acci[t] += p * tvi[t]; }
-  }
-  const C inv = l > C(0) ? C(1) / l : C(0);
-  S* out_i = a.out + (base + i) * a.D;
-#pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    if (col[t] >= 0) {
-      st<S>(out_i + col[t], accr[t] * inv);
-      if (a.plan.order[t] != 0) st<S>(out_i + col[t] + 1, acci[t] * inv);
-    }
-  }
-  if (s == 0) a.lse[(base + i) * a.H + h] = l > C(0) ? m + gm_log(l) : neg_inf<C>();
-}
-
 template <typename A, typename C>
 __device__ __forceinline__ void accumulate(A* p, C v) { atomicAdd(p, (A)v); }
+
+// VEC: p sits on a 2-element boundary, one addition for the pair
+template <bool VEC, typename A, typename C>
+__device__ __forceinline__ void accumulate_pair(A* p, C x, C y) {
+  if constexpr (VEC && std::is_same<A, float>::value) {
+    asm volatile("red.relaxed.gpu.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"((float)x), "f"((float)y) : "memory");
+  } else {
+    accumulate(p, x);
+    accumulate(p + 1, y);
+  }
+}
 
 // (re, im) at p as compute values; VEC: p sits on a 2-element boundary, one load
 template <typename C, bool VEC, typename S>
@@ -165,32 +94,192 @@ __device__ __forceinline__ void load_pair(const S* p, C& x, C& y) {
   }
 }
 
-// Whether every (re, im) pair a warp's lanes read (columns col of the rows at base pointers, D apart; the transport table)
-// sits on a 2-element boundary.  The backward then issues one load where it issued two: 407 -> 363 us on 10 242 points of
-// degree ~37, batch 2, 4 heads of 8 x (m <= 2), float32 (what is left are the atomic additions to dk and dv; the forward,
-// 240 us, gained nothing from it or from two edges in flight).
+// Whether every (re, im) pair a warp's lanes read (columns col of the rows at base pointers, D apart; the transport table;
+// the gradients' sums) sits on a 2-element boundary: one load or addition then where there would be two.
 template <typename S, int NS>
-__device__ __forceinline__ bool pairs_aligned(const FusedArgs<S>& a, const int (&col)[NS], const void* p0, const void* p1) {
+__device__ __forceinline__ bool pairs_aligned(const FusedArgs<S>& a, const int (&col)[NS]) {
   using C = typename Compute<S>::type;
-  bool ok = a.D % 2 == 0 && ((reinterpret_cast<uintptr_t>(p0) | reinterpret_cast<uintptr_t>(p1)) & (2 * sizeof(S) - 1)) == 0 &&
+  bool ok = a.D % 2 == 0 && ((reinterpret_cast<uintptr_t>(a.k) | reinterpret_cast<uintptr_t>(a.v)) & (2 * sizeof(S) - 1)) == 0 &&
+            ((reinterpret_cast<uintptr_t>(a.dk) | reinterpret_cast<uintptr_t>(a.dv)) & (2 * sizeof(C) - 1)) == 0 &&
             (reinterpret_cast<uintptr_t>(a.transport) & (2 * sizeof(C) - 1)) == 0;
 #pragma unroll
   for (int t = 0; t < NS; ++t) ok = ok && (col[t] < 0 || a.plan.order[t] == 0 || col[t] % 2 == 0);
   return __all_sync(0xffffffffu, ok);
 }
 
-template <typename S, int NS>
-__global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
+// A lane's place: head, lane of the head, and (SHARED: heads so narrow that H heads' lanes fit a warp several times) which of
+// the groups that take a target's edges in turn.
+template <bool SHARED>
+struct Place {
+  int L, H, h, s, share, shares;
+  unsigned mask;  // of the group
+  __device__ __forceinline__ Place(int lane, int H_, int shares_) {
+    H = H_;
+    shares = SHARED ? shares_ : 1;
+    L = 32 / H / shares;
+    share = SHARED ? lane / (H * L) : 0;
+    h = SHARED ? lane / L % H : lane / L;
+    s = lane % L;
+    mask = SHARED ? ((1u << (H * L)) - 1u) << (share * H * L) : 0xffffffffu;
+  }
+  template <typename T> __device__ __forceinline__ T over_shares(T v) const {
+    for (int o = H * L; SHARED && o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+};
+// f(e, source, bias) of each edge in the window in a group's turn; nothing is asked of a masked edge's source.  AHEAD: what is read
+// of one is asked for a turn ahead of its gathers (registers that the kernels without FORM do not have: 8 % on their forward).
+template <bool AHEAD, typename C, typename Place, typename F>
+__device__ __forceinline__ void for_edges(const Place& at, int degree, const int64_t* source, const uint8_t* inside, const C* bias, F f) {
+  if constexpr (!AHEAD) {
+    for (int e = at.share; e < degree; e += at.shares)
+      if (inside[e]) f((unsigned)e, (unsigned)source[e], bias[e]);
+    return;
+  }
+  if (at.share >= degree) return;
+  unsigned e = at.share;
+  int64_t src = source[e];
+  uint8_t in = inside[e];
+  C w = bias[e];
+  while (true) {
+    const unsigned next = e + at.shares, ahead = min(next, (unsigned)degree - 1);
+    const int64_t src_next = source[ahead];
+    const uint8_t in_next = inside[ahead];
+    const C w_next = bias[ahead];
+    if (in) f(e, (unsigned)src, w);
+    if (next >= degree) return;
+    e = next; src = src_next; in = in_next; w = w_next;
+  }
+}
+// FORM: the first FORM slots are scalars, the other NS - FORM pairs, all of them in the plan; a lane without a copy in one computes
+// with zeros.  0: as the plan has them, each looked up and branched around.
+template <typename S, int NS, int FORM>
+__device__ __forceinline__ bool is_scalar(const FusedArgs<S>& a, int t) { return FORM ? t < FORM : a.plan.order[t] == 0; }
+
+// Both kernels wait for their gathers (a target's k and v rows come from L2) in the time that issuing leaves over; the backward
+// also for its atomic additions.  10 242 points of degree ~37, batch 2, 4 heads of 8 x (m <= 2), float32: forward 240 -> 159 us with
+// slots whose kind the compiler knows (FORM), one load for a pair and the next edge's source asked for early; backward 363 -> 333
+// likewise, 304 with four CTAs to an SM (64 registers; five spill: 381),
+// 261 with one addition for a pair; of 8 x (m <= 3) three CTAs (80 registers) are better than two, 350 and 402.  Two edges' gathers in
+// flight cost registers: 239 -> 275 and 402 -> 413 before FORM.  Groups of lanes in turn on the edges (SHARED): 1 head of 8 x (m <= 3)
+// on 3 000 points, batch 4, 138 -> 41 and 197 -> 75; 2 heads of 5 x (m <= 2) on 5 000, batch 3, 194 -> 85 and 270 -> 110.
+template <typename S, int NS, int FORM, bool SHARED>
+__global__ void __launch_bounds__(256, !FORM && NS <= 4 && !SHARED ? 3 : 0) fused_forward_kernel(const __grid_constant__ FusedArgs<S> a) {
+  using C = typename Compute<S>::type;
+  const int lane = threadIdx.x & 31;
+  const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (gw >= a.n_nodes * a.batch) return;
+  const int64_t i = gw / a.batch, b = gw % a.batch;
+  const Place<SHARED> at(lane, a.H, a.shares);
+  const int64_t base = b * a.n_nodes;
+
+  int col[NS];
+  C qr[NS], qi[NS], accr[NS], acci[NS];
+  const S* q_i = a.q + (base + i) * a.D;
+#pragma unroll
+  for (int t = 0; t < NS; ++t) {
+    col[t] = -1;
+    qr[t] = qi[t] = accr[t] = acci[t] = C(0);
+    if (t < a.plan.n_slots) {
+      const int u = at.s + at.L * a.plan.round[t], a_n = a.plan.mult[t];
+      if (u < a_n) {
+        const int dim = a.plan.order[t] == 0 ? 1 : 2;
+        col[t] = a.plan.off[t] + dim * (at.h * a_n + u);
+        qr[t] = ld<C>(q_i + col[t]);
+        if (dim == 2) qi[t] = ld<C>(q_i + col[t] + 1);
+      }
+    }
+  }
+  C m = lowest<C>(), l = C(0);  // (not minus infinity: an edge of bias minus infinity counts nothing, wherever it stands)
+  const int64_t e0 = a.row_ptr[i];
+  const int degree = (int)(a.row_ptr[i + 1] - e0);
+  const int64_t* source = a.source + e0;
+  const uint8_t* inside = a.inside + e0;
+  const C *bias = a.bias + e0, *transport = a.transport + e0 * a.orders * 2;
+  const S *k = a.k + base * a.D, *v = a.v + base * a.D;
+  const unsigned D = a.D, tau_step = 2 * a.orders;
+  auto walk = [&](auto vec) {
+    constexpr bool VEC = decltype(vec)::value;
+    for_edges<FORM != 0>(at, degree, source, inside, bias, [&](unsigned e, unsigned src, C w) {
+      const C* tau = transport + (size_t)e * tau_step;
+      C part = C(0), tvr[NS], tvi[NS];
+#pragma unroll
+      for (int t = 0; t < NS; ++t) {
+        tvr[t] = tvi[t] = C(0);
+        if (FORM || col[t] >= 0) {
+          const size_t x = FORM ? (size_t)(src * D + (unsigned)col[t]) : (size_t)src * D + col[t];
+          if (is_scalar<S, NS, FORM>(a, t)) {
+            C kr = C(0);
+            if (!FORM || col[t] >= 0) { kr = ld<C>(k + x); tvr[t] = ld<C>(v + x); }
+            part += qr[t] * kr;
+          } else {
+            C tr = C(0), ti = C(0), kr = C(0), ki = C(0), vr = C(0), vi = C(0);
+            if (!FORM || col[t] >= 0) {
+              load_pair<C, VEC>(tau + 2 * a.plan.order[t], tr, ti);
+              load_pair<C, VEC>(k + x, kr, ki);
+              load_pair<C, VEC>(v + x, vr, vi);
+            }
+            part += qr[t] * (tr * kr - ti * ki) + qi[t] * (tr * ki + ti * kr);
+            tvr[t] = tr * vr - ti * vi;
+            tvi[t] = tr * vi + ti * vr;
+          }
+        }
+      }
+      for (int o = at.L >> 1; o > 0; o >>= 1) part += __shfl_xor_sync(at.mask, part, o);
+      const C logit = a.scale * part + w;
+      if (logit > m) {
+        const C corr = gm_exp(m - logit);
+        l *= corr;
+#pragma unroll
+        for (int t = 0; t < NS; ++t) { accr[t] *= corr; acci[t] *= corr; }
+        m = logit;
+      }
+      const C p = gm_exp(logit - m);
+      l += p;
+#pragma unroll
+      for (int t = 0; t < NS; ++t) { accr[t] += p * tvr[t]; acci[t] += p * tvi[t]; }
+    });
+  };
+  if (FORM && pairs_aligned<S, NS>(a, col)) walk(std::true_type{});
+  else walk(std::false_type{});
+  if constexpr (SHARED) {  // the groups' sums, each against its own maximum
+    C top = m;
+    for (int o = at.H * at.L; o < 32; o <<= 1) {
+      const C other = __shfl_xor_sync(0xffffffffu, top, o);
+      top = other > top ? other : top;
+    }
+    const C corr = gm_exp(m - top);
+    m = top;
+    l = at.over_shares(l * corr);
+#pragma unroll
+    for (int t = 0; t < NS; ++t) {
+      accr[t] = at.over_shares(accr[t] * corr);
+      acci[t] = at.over_shares(acci[t] * corr);
+    }
+    if (at.share != 0) return;
+  }
+  const C inv = l > C(0) ? C(1) / l : C(0);
+  S* out_i = a.out + (base + i) * a.D;
+#pragma unroll
+  for (int t = 0; t < NS; ++t) {
+    if (col[t] >= 0) {
+      st<S>(out_i + col[t], accr[t] * inv);
+      if (a.plan.order[t] != 0) st<S>(out_i + col[t] + 1, acci[t] * inv);
+    }
+  }
+  if (at.s == 0) a.lse[(base + i) * a.H + at.h] = l > C(0) ? m + gm_log(l) : neg_inf<C>();
+}
+
+template <typename S, int NS, int FORM, bool SHARED>
+__global__ void __launch_bounds__(256, FORM == 1 && sizeof(S) <= 4 ? (NS <= 3 ? 4 : 3) : 1) fused_backward_kernel(const __grid_constant__ FusedArgs<S> a) {
   using C = typename Compute<S>::type;
   using A = typename std::conditional<std::is_same<S, __nv_bfloat16>::value, float, S>::type;
   const int lane = threadIdx.x & 31;
   const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (gw >= a.n_nodes * a.batch) return;
   const int64_t i = gw / a.batch, b = gw % a.batch;
-  const int L = 32 / a.H, h = lane / L, s = lane % L;
+  const Place<SHARED> at(lane, a.H, a.shares);
   const int64_t base = b * a.n_nodes;
-  A* dk = reinterpret_cast<A*>(a.dk);
-  A* dv = reinterpret_cast<A*>(a.dv);
 
   int col[NS];
   C qr[NS], qi[NS], gr[NS], gi[NS], dqr[NS], dqi[NS];
@@ -203,10 +292,10 @@ __global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
     col[t] = -1;
     qr[t] = qi[t] = gr[t] = gi[t] = dqr[t] = dqi[t] = C(0);
     if (t < a.plan.n_slots) {
-      const int u = s + L * a.plan.round[t], a_n = a.plan.mult[t];
+      const int u = at.s + at.L * a.plan.round[t], a_n = a.plan.mult[t];
       if (u < a_n) {
         const int dim = a.plan.order[t] == 0 ? 1 : 2;
-        col[t] = a.plan.off[t] + dim * (h * a_n + u);
+        col[t] = a.plan.off[t] + dim * (at.h * a_n + u);
         qr[t] = ld<C>(q_i + col[t]);
         gr[t] = ld<C>(g_i + col[t]);
         delta += gr[t] * ld<C>(o_i + col[t]);
@@ -218,34 +307,38 @@ __global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
       }
     }
   }
-  delta = group_sum(delta, L);
-  const C lse = a.lse_in[(base + i) * a.H + h];
-  const int64_t e0 = a.row_ptr[i], e1 = a.row_ptr[i + 1];
+  for (int o = at.L >> 1; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
+  const C lse = a.lse_in[(base + i) * a.H + at.h];
+  const int64_t e0 = a.row_ptr[i];
+  const int degree = (int)(a.row_ptr[i + 1] - e0);
+  const int64_t* source = a.source + e0;
+  const uint8_t* inside = a.inside + e0;
+  const C *bias = a.bias + e0, *transport = a.transport + e0 * a.orders * 2;
+  const S *k = a.k + base * a.D, *v = a.v + base * a.D;
+  A *dk = reinterpret_cast<A*>(a.dk) + base * a.D, *dv = reinterpret_cast<A*>(a.dv) + base * a.D;
+  const unsigned D = a.D, tau_step = 2 * a.orders;
   auto walk = [&](auto vec) {
     constexpr bool VEC = decltype(vec)::value;
-    for (int64_t e = e0; e < e1; ++e) {
-      if (!a.inside[e]) continue;
-      const int64_t j = base + a.source[e];
-      const S* k_j = a.k + j * a.D;
-      const S* v_j = a.v + j * a.D;
-      const C* tau = a.transport + e * a.orders * 2;
-      C part = C(0), dpart = C(0);
-      C tkr[NS], tki[NS];
+    for_edges<FORM != 0>(at, degree, source, inside, bias, [&](unsigned e, unsigned src, C w) {
+      const C* tau = transport + (size_t)e * tau_step;
+      C part = C(0), dpart = C(0), tkr[NS], tki[NS];
 #pragma unroll
       for (int t = 0; t < NS; ++t) {
         tkr[t] = tki[t] = C(0);
-        if (col[t] >= 0) {
-          const int n = a.plan.order[t];
-          if (n == 0) {
-            tkr[t] = ld<C>(k_j + col[t]);
+        if (FORM || col[t] >= 0) {
+          const size_t x = FORM ? (size_t)(src * D + (unsigned)col[t]) : (size_t)src * D + col[t];
+          if (is_scalar<S, NS, FORM>(a, t)) {
+            C vr = C(0);
+            if (!FORM || col[t] >= 0) { tkr[t] = ld<C>(k + x); vr = ld<C>(v + x); }
             part += qr[t] * tkr[t];
-            dpart += gr[t] * ld<C>(v_j + col[t]);
+            dpart += gr[t] * vr;
           } else {
-            C tr, ti;
-            load_pair<C, VEC>(tau + 2 * n, tr, ti);
-            C kr, ki, vr, vi;
-            load_pair<C, VEC>(k_j + col[t], kr, ki);
-            load_pair<C, VEC>(v_j + col[t], vr, vi);
+            C tr = C(0), ti = C(0), kr = C(0), ki = C(0), vr = C(0), vi = C(0);
+            if (!FORM || col[t] >= 0) {
+              load_pair<C, VEC>(tau + 2 * a.plan.order[t], tr, ti);
+              load_pair<C, VEC>(k + x, kr, ki);
+              load_pair<C, VEC>(v + x, vr, vi);
+            }
             tkr[t] = tr * kr - ti * ki;
             tki[t] = tr * ki + ti * kr;
             part += qr[t] * tkr[t] + qi[t] * tki[t];
@@ -254,41 +347,46 @@ __global__ void __launch_bounds__(256) fused_backward_kernel(FusedArgs<S> a) {
         }
       }
       // one shuffle tree for both sums
-      for (int o = L >> 1; o > 0; o >>= 1) {
-        part += __shfl_xor_sync(0xffffffffu, part, o);
-        dpart += __shfl_xor_sync(0xffffffffu, dpart, o);
+      for (int o = at.L >> 1; o > 0; o >>= 1) {
+        part += __shfl_xor_sync(at.mask, part, o);
+        dpart += __shfl_xor_sync(at.mask, dpart, o);
       }
-      const C p = gm_exp(a.scale * part + a.bias[e] - lse);
+      const C p = gm_exp(a.scale * part + w - lse);
       const C ds = a.scale * p * (dpart - delta);
-      A* dk_j = dk + j * a.D;
-      A* dv_j = dv + j * a.D;
 #pragma unroll
       for (int t = 0; t < NS; ++t) {
-        if (col[t] >= 0) {
-          const int n = a.plan.order[t];
+        if (FORM || col[t] >= 0) {
+          const size_t x = FORM ? (size_t)(src * D + (unsigned)col[t]) : (size_t)src * D + col[t];
           dqr[t] += ds * tkr[t];
-          if (n == 0) {
-            accumulate(dk_j + col[t], ds * qr[t]);
-            accumulate(dv_j + col[t], p * gr[t]);
+          if (is_scalar<S, NS, FORM>(a, t)) {
+            if (!FORM || col[t] >= 0) {
+              accumulate(dk + x, ds * qr[t]);
+              accumulate(dv + x, p * gr[t]);
+            }
           } else {
             dqi[t] += ds * tki[t];
-            C tr, ti;
-            load_pair<C, VEC>(tau + 2 * n, tr, ti);
-            // conj(tau) x = (tr xr + ti xi, tr xi - ti xr)
-            accumulate(dk_j + col[t], ds * (tr * qr[t] + ti * qi[t]));
-            accumulate(dk_j + col[t] + 1, ds * (tr * qi[t] - ti * qr[t]));
-            accumulate(dv_j + col[t], p * (tr * gr[t] + ti * gi[t]));
-            accumulate(dv_j + col[t] + 1, p * (tr * gi[t] - ti * gr[t]));
+            if (!FORM || col[t] >= 0) {
+              C tr, ti;
+              load_pair<C, VEC>(tau + 2 * a.plan.order[t], tr, ti);
+              // conj(tau) x = (tr xr + ti xi, tr xi - ti xr)
+              accumulate_pair<VEC>(dk + x, ds * (tr * qr[t] + ti * qi[t]), ds * (tr * qi[t] - ti * qr[t]));
+              accumulate_pair<VEC>(dv + x, p * (tr * gr[t] + ti * gi[t]), p * (tr * gi[t] - ti * gr[t]));
+            }
           }
         }
       }
-    }
+    });
   };
-  // 16 slots of float64 leave no registers for two walks in one kernel (988 bytes of spill stores against 420; 4 236 us
-  // against 4 115 on 6 000 points, batch 2, 8 heads of 16 x (m <= 3); at 8 slots the vector form wins, 1 817 against 1 837)
+  // (16 slots of float64 leave no registers for two walks in one kernel: 988 bytes of spill stores against 420)
   if constexpr (std::is_same<S, double>::value && NS > 8) walk(std::false_type{});
-  else if (pairs_aligned<S, NS>(a, col, a.k, a.v)) walk(std::true_type{});
+  else if (pairs_aligned<S, NS>(a, col)) walk(std::true_type{});
   else walk(std::false_type{});
+#pragma unroll
+  for (int t = 0; t < NS; ++t) {
+    dqr[t] = at.over_shares(dqr[t]);
+    dqi[t] = at.over_shares(dqi[t]);
+  }
+  if (SHARED && at.share != 0) return;
   S* dq_i = a.dq + (base + i) * a.D;
 #pragma unroll
   for (int t = 0; t < NS; ++t) {
@@ -304,16 +402,19 @@ __global__ void narrow_to_bf16_kernel(const float* __restrict__ src, __nv_bfloat
     dst[x] = __float2bfloat16_rn(src[x]);
 }
 
-int make_plan(const int64_t* desc_host, int F, int H, int D, SlotPlan& plan) {
+// shares: as many groups of lanes as have a lane for every copy of a head
+int make_plan(const int64_t* desc_host, int F, int H, int D, SlotPlan& plan, int& shares) {
   GM_REQUIRE(H == 1 || H == 2 || H == 4 || H == 8, GM_ERR_UNSUPPORTED, "gm_attention: heads must be 1, 2, 4 or 8 (got %d)", H);
   GM_REQUIRE(F >= 1 && F <= MAX_F, GM_ERR_ARGUMENT, "gm_attention: 1 <= F <= %d descriptor rows", MAX_F);
   const int L = 32 / H;
   plan.n_slots = 0;
+  int widest = 1;
   for (int f = 0; f < F; ++f) {
     const int n = (int)desc_host[f * 5 + 0], a_n = (int)desc_host[f * 5 + 1], off = (int)desc_host[f * 5 + 2];
     const int dim = n == 0 ? 1 : 2;
     GM_REQUIRE(n >= 0 && a_n >= 1 && off >= 0 && off + H * a_n * dim <= D, GM_ERR_ARGUMENT,
                "gm_attention: descriptor row %d (n=%d, a_n=%d, off=%d) leaves the width D=%d", f, n, a_n, off, D);
+    widest = a_n > widest ? a_n : widest;
     for (int r = 0; r * L < a_n; ++r) {
       GM_REQUIRE(plan.n_slots < MAX_SLOTS, GM_ERR_LIMIT, "gm_attention: a lane would own more than %d slots (D=%d, H=%d)", MAX_SLOTS, D, H);
       plan.off[plan.n_slots] = off;
@@ -323,6 +424,12 @@ int make_plan(const int64_t* desc_host, int F, int H, int D, SlotPlan& plan) {
       ++plan.n_slots;
     }
   }
+  plan.form = 0;
+  while (plan.form < plan.n_slots && plan.order[plan.form] == 0) ++plan.form;
+  for (int t = plan.form; t < plan.n_slots; ++t)
+    if (plan.order[t] == 0) plan.form = 0;
+  shares = 1;
+  while (2 * shares * widest <= L) shares *= 2;
   return GM_OK;
 }
 
@@ -335,7 +442,7 @@ int fill_args(FusedArgs<S>& a, const void* q, const void* k, const void* v, cons
   a.transport = (const C*)transport; a.bias = (const C*)bias; a.inside = inside;
   a.row_ptr = row_ptr; a.source = source;
   a.n_nodes = n_nodes; a.batch = batch; a.D = D; a.orders = orders; a.H = H; a.scale = (C)scale;
-  int status = make_plan(desc_host, F, H, D, a.plan);
+  int status = make_plan(desc_host, F, H, D, a.plan, a.shares);
   if (status != GM_OK) return status;
   for (int t = 0; t < a.plan.n_slots; ++t)
     GM_REQUIRE(a.plan.order[t] < orders, GM_ERR_ARGUMENT, "gm_attention: transport table has %d orders, frequency %d needs more", orders, a.plan.order[t]);
@@ -355,26 +462,47 @@ int check_common(const void* q, const void* k, const void* v, const void* transp
   return GM_OK;
 }
 
-template <typename S, template <typename, int> class Launcher>
+template <int N> using Int = std::integral_constant<int, N>;
+
+template <typename S, template <typename, int, int> class Launcher>
 int dispatch_slots(const FusedArgs<S>& a, cudaStream_t stream) {
   const int64_t warps = a.n_nodes * a.batch;
   const int threads = 256, per_block = threads / 32;
   const int64_t blocks = (warps + per_block - 1) / per_block;
   GM_REQUIRE(blocks < ((int64_t)1 << 31), GM_ERR_LIMIT, "gm_attention: too many (node, sample) pairs");
-  if (a.plan.n_slots <= 4) Launcher<S, 4>::run(a, (int)blocks, threads, stream);
-  else if (a.plan.n_slots <= 8) Launcher<S, 8>::run(a, (int)blocks, threads, stream);
-  else Launcher<S, 16>::run(a, (int)blocks, threads, stream);
+  const int n = (int)blocks;
+  const auto wide = [&](auto slots, auto form) {
+    Launcher<S, decltype(slots)::value, decltype(form)::value>::template run<false>(a, n, threads, stream);
+  };
+  const auto narrow = [&](auto slots, auto form) {
+    if (a.shares > 1) Launcher<S, decltype(slots)::value, decltype(form)::value>::template run<true>(a, n, threads, stream);
+    else wide(slots, form);
+  };
+  // One scalar frequency and one to three others, a copy a lane or (twice the slots) two: what heads of up to 32 / H and 64 / H
+  // copies have.  2 x 8 000 targets of ~37 edges, float32, 4 heads of 8: 213 + 329 us by the plan, 174 + 244 in the form; 8 heads of
+  // 5, two copies a lane, 422 + 681 and 256 + 432; 4 000 targets, 4 heads of 16: 303 + 442 and 188 + 253.  (32-bit element indices.)
+  const int slots = a.plan.n_slots;
+  const int form = a.n_nodes * a.D < ((int64_t)1 << 31) ? a.plan.form : 0;
+  if (form == 1 && slots == 2) narrow(Int<2>{}, Int<1>{});
+  else if (form == 1 && slots == 3) narrow(Int<3>{}, Int<1>{});
+  else if (form == 1 && slots == 4) narrow(Int<4>{}, Int<1>{});
+  else if (form == 2 && slots == 4 && a.shares == 1) wide(Int<4>{}, Int<2>{});
+  else if (form == 2 && slots == 6 && a.shares == 1) wide(Int<6>{}, Int<2>{});
+  else if (form == 2 && slots == 8 && a.shares == 1) wide(Int<8>{}, Int<2>{});
+  else if (slots <= 4) narrow(Int<4>{}, Int<0>{});
+  else if (slots <= 8) narrow(Int<8>{}, Int<0>{});
+  else wide(Int<16>{}, Int<0>{});  // (several copies a lane)
   return launch_status("gm_attention");
 }
 
-template <typename S, int NS> struct ForwardLauncher {
-  static void run(const FusedArgs<S>& a, int blocks, int threads, cudaStream_t stream) {
-    fused_forward_kernel<S, NS><<<blocks, threads, 0, stream>>>(a);
+template <typename S, int NS, int FORM> struct ForwardLauncher {
+  template <bool SHARED> static void run(const FusedArgs<S>& a, int blocks, int threads, cudaStream_t stream) {
+    fused_forward_kernel<S, NS, FORM, SHARED><<<blocks, threads, 0, stream>>>(a);
   }
 };
-template <typename S, int NS> struct BackwardLauncher {
-  static void run(const FusedArgs<S>& a, int blocks, int threads, cudaStream_t stream) {
-    fused_backward_kernel<S, NS><<<blocks, threads, 0, stream>>>(a);
+template <typename S, int NS, int FORM> struct BackwardLauncher {
+  template <bool SHARED> static void run(const FusedArgs<S>& a, int blocks, int threads, cudaStream_t stream) {
+    fused_backward_kernel<S, NS, FORM, SHARED><<<blocks, threads, 0, stream>>>(a);
   }
 };
 

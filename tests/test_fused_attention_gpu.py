@@ -123,3 +123,56 @@ def test_one_infinite_value_reaches_its_neighbours_only():
     assert np.array_equal(np.isfinite(out), np.isfinite(want))
     finite = np.isfinite(want)
     assert_close(out[finite], want[finite], 1e-5, 1e-6 * max(1.0, np.abs(want[finite]).max()), "finite entries")
+
+
+# (heads, descriptor (n, copies, offset) in the descriptor's order, row length, degree).  Lane groups share a target's edges when
+# a head's lanes are at least twice its copies; one scalar frequency with one to three others is the form with its own kernels.
+GRAPHS = [
+    (1, [(0, 4, 0), (1, 3, 4)], 10, 33),  # eight groups
+    (1, [(0, 1, 0), (2, 1, 1)], 3, 40),  # 32 groups, odd rows: pairs of numbers
+    (2, [(1, 5, 0), (0, 5, 20)], 30, 9),  # the scalar is not first
+    (4, [(0, 8, 0), (1, 7, 32), (2, 8, 88)], 152, 21),  # one group, lanes without a copy
+    (8, [(0, 2, 0), (1, 2, 16), (2, 1, 48), (3, 2, 64)], 96, 7),
+    (2, [(1, 3, 0), (2, 3, 12), (3, 3, 24), (4, 3, 36), (5, 1, 48)], 52, 18),  # no scalar, five slots
+    (1, [(0, 40, 0), (1, 33, 40)], 106, 5),  # two slots each
+]
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("graph", GRAPHS)
+def test_lane_groups_share_edges(graph, dtype):
+    """Against the oracle on graphs whose targets have none, one and many edges, some outside the window (with a source that
+    no node has) and some of bias minus infinity (which count nothing, also as a target's first or as all that a group has).
+    Tolerances as above."""
+    from gm_attention_b200.attention import AttentionTables, attention_backward, attention_forward
+
+    heads, rows, width, degree = graph
+    n_nodes, batch = 37, 2
+    rng = np.random.default_rng(5)
+    counts = rng.integers(0, 2 * degree + 1, n_nodes)
+    counts[:3] = 0, 1, 2
+    row_ptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    n_edges, orders = int(row_ptr[-1]), 1 + max(n for n, _, _ in rows)
+    desc = np.array([(n, copies, offset, 0, 1 if n == 0 else 2) for n, copies, offset in rows], dtype=np.int64)
+    source = rng.integers(0, n_nodes, n_edges)
+    angle = rng.uniform(-np.pi, np.pi, (n_edges, 1)) * np.arange(orders)
+    transport = np.stack([np.cos(angle), np.sin(angle)], -1).astype(dtype)
+    bias = rng.standard_normal(n_edges).astype(dtype)
+    silent, inside = rng.random(n_edges) < 0.3, (rng.random(n_edges) < 0.8).astype(np.uint8)
+    silent[row_ptr[:-1][counts > 0]] = True  # each target's first
+    last = row_ptr[1:][counts > 0] - 1  # (one edge of each counts)
+    silent[last], inside[last] = False, 1
+    q, k, v, g = seeded((batch * n_nodes, width), 13, dtype, 4)
+    keep = (inside & ~silent).astype(np.uint8)  # what the oracle sees
+    args = (transport, bias, keep, desc, row_ptr, source, heads, 0.3, batch)
+    want = O.attention_forward(q, k, v, *args)
+    grads = O.attention_backward(g, q, k, v, *args)
+    elsewhere = np.where(inside != 0, source, -(1 << 40))
+    bias = np.where(silent, dtype(-np.inf), bias)
+    t = AttentionTables(cuda(transport), cuda(bias), cuda(inside), cuda(row_ptr), cuda(elsewhere), tuple(map(tuple, desc.tolist())), heads, 0.3)
+    Q, K, V, G = map(cuda, (q, k, v, g))
+    out, lse = attention_forward(Q, K, V, t)
+    rtol, atol = (1e-10, 1e-11) if dtype == np.float64 else (1e-5, 1e-6)
+    assert_close(out.cpu().numpy(), want, rtol, atol * max(1.0, np.abs(want).max()), "out")
+    for name, got, ref in zip(("dq", "dk", "dv"), attention_backward(G, Q, K, V, out, lse, t), grads):
+        assert_close(got.cpu().numpy(), ref, rtol, 10 * atol * max(1.0, np.abs(ref).max()), name)
