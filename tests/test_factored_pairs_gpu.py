@@ -949,3 +949,97 @@ def test_kernel_saved_after_a_call_and_loaded_elsewhere():
     assert loaded.__dict__["_fused_node_descriptors"][str(dev)][0].device.type == "cpu"
     for a, b in zip(results(loaded), want, strict=True):
         assert torch.equal(a, b)
+
+
+# (nodes, copies of the input frequencies, of the output ones, k): copies about what a thread holds (16) or sums (8), columns
+# about what is staged together (128), nodes about a tile (32)
+NODE_PRODUCTS = [
+    (1, (1, 1), (1, 2), 2),
+    (33, (8, 9), (4, 3), 17),
+    (31, (16, 17), (2, 5), 5),
+    (70, (33, 3), (40, 31), 6),
+    (300, (7, 8, 4), (3, 4, 2), 17),
+    (40, (2, 5), (150, 1), 3),
+]
+
+
+@pytest.mark.parametrize("aligned", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("case", NODE_PRODUCTS)
+def test_node_products_against_float64(case, dtype, aligned):
+    """``Z_t = M_t x~`` and its gradients against the sums in float64.  A sum of ``n`` products of complex numbers errs by at most
+    ``(2 n + 2)`` roundings of the sum of the terms' magnitudes (a float64 result: of twice that, the oracle's own)."""
+    from gm_attention_b200.nn.fused_pairs import NodeProducts
+
+    n_nodes, ins, outs, k = case
+    offsets = np.concatenate([[0], np.cumsum([a if n == 0 else 2 * a for n, a in enumerate(ins)])])
+    rows, counts, widths = [], [0, 0], [0, 0]
+    for n, a in enumerate(ins):
+        for m, b in enumerate(outs):
+            for mode in (0,) if n == 0 else (1, 2) if m else (2,):
+                c = int(n > 0 or m > 0)
+                rows.append((c, widths[c], b, a, int(offsets[n]), mode, counts[c], 0))
+                widths[c] += b
+                counts[c] += (2 if c else 1) * a * b
+    wr, wc = (w + 3 for w in widths)  # (columns of no block)
+    gen = torch.Generator().manual_seed(3)
+
+    def normal(*shape):
+        return torch.randn(*shape, generator=gen, dtype=torch.float64).to(dtype).cuda()
+
+    x, cw, cb, rw, rb = normal(n_nodes, int(offsets[-1])), normal(counts[1], k - 1), normal(counts[1]), normal(counts[0], k - 1), normal(counts[0])
+    gc, gr = normal(n_nodes, k, wc, 2), normal(n_nodes, k, wr)
+    if not aligned:  # the same numbers one element on
+        gc = torch.cat([gc.new_zeros(1), gc.reshape(-1)])[1:].view(gc.shape)
+    leaves = [t.requires_grad_() for t in (x, cw, cb, rw, rb)]
+    zc, zr = NodeProducts.apply(*leaves, torch.tensor(rows, dtype=torch.int32).cuda(), k, wc, wr)
+    grads = torch.autograd.grad((zc, zr), leaves, (gc, gr))
+
+    def oracle(sign, x, cw, cb, rw, rb, gc, gr):
+        """zc, zr (columns of no block zero) and the gradients, from real parts so that magnitudes can be put through too
+        (they add: ``sign`` 1 in place of -1)."""
+        cm, rm = torch.cat([cb[:, None], cw], 1), torch.cat([rb[:, None], rw], 1)
+        zc, zr = torch.zeros_like(gc), torch.zeros_like(gr)
+        dx, dcm, drm = torch.zeros_like(x), torch.zeros_like(cm), torch.zeros_like(rm)
+        for c, z0, b, a, x0, mode, row0, _ in rows:
+            if mode == 0:
+                xr, xi = x[:, x0 : x0 + a], torch.zeros_like(x[:, x0 : x0 + a])
+            else:
+                xr, xi = x[:, x0 : x0 + 2 * a].view(-1, a, 2).unbind(-1)
+                xi = sign * xi if mode == 2 else xi
+            if c:
+                mr, mi = cm[row0 : row0 + 2 * a * b].view(b, a, 2, k).unbind(2)
+                g_r, g_i = gc[:, :, z0 : z0 + b].unbind(-1)
+            else:
+                mr = rm[row0 : row0 + a * b].view(b, a, k)
+                mi, g_r = torch.zeros_like(mr), gr[:, :, z0 : z0 + b]
+                g_i = torch.zeros_like(g_r)
+            product = lambda m, y: torch.einsum("bak,na->nkb", m, y)
+            z_r, z_i = product(mr, xr) + sign * product(mi, xi), product(mr, xi) + product(mi, xr)
+            back = lambda m, g: torch.einsum("bak,nkb->na", m, g)
+            d_r, d_i = back(mr, g_r) + back(mi, g_i), back(mr, g_i) + sign * back(mi, g_r)
+            outer = lambda g, y: torch.einsum("nkb,na->bak", g, y)
+            w_r, w_i = outer(g_r, xr) + outer(g_i, xi), outer(g_i, xr) + sign * outer(g_r, xi)
+            if c:
+                zc[:, :, z0 : z0 + b] = torch.stack([z_r, z_i], -1)
+                dcm[row0 : row0 + 2 * a * b] = torch.stack([w_r, w_i], 2).reshape(2 * a * b, k)
+            else:
+                zr[:, :, z0 : z0 + b] = z_r
+                drm[row0 : row0 + a * b] = w_r.reshape(a * b, k)
+            if mode == 0:
+                dx[:, x0 : x0 + a] += d_r
+            else:
+                dx[:, x0 : x0 + 2 * a] += torch.stack([d_r, sign * d_i if mode == 2 else d_i], -1).reshape(n_nodes, 2 * a)
+        return zc, zr, dx, dcm[:, 1:], dcm[:, 0], drm[:, 1:], drm[:, 0]
+
+    inputs = [t.detach().double().cpu() for t in (*leaves, gc, gr)]
+    want, size = oracle(-1.0, *inputs), oracle(1.0, *(t.abs() for t in inputs))
+    columns = [torch.zeros(w, dtype=torch.bool) for w in (wr, wc)]
+    for c, z0, b, *_ in rows:
+        columns[c][z0 : z0 + b] = True
+    zc, zr = torch.where(columns[1][:, None], zc.detach().cpu(), 0.0), torch.where(columns[0], zr.detach().cpu(), 0.0)
+    terms = (max(ins), max(ins), k * sum(outs) * 2, n_nodes, n_nodes, n_nodes, n_nodes)
+    unit = torch.finfo(dtype).eps / 2 * (2 if dtype == torch.float64 else 1)
+    for name, got, ref, scale, n in zip(("zc", "zr", "dx", "dcw", "dcb", "drw", "drb"), (zc, zr, *grads), want, size, terms):
+        excess = (got.cpu().double() - ref).abs() - (2 * n + 2) * unit * scale
+        assert got.shape == ref.shape and excess.max() <= 0, (name, float(excess.max()))
