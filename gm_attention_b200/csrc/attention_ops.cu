@@ -179,13 +179,45 @@ __global__ void __launch_bounds__(SM_THREADS) softmax_forward_kernel(SoftmaxArgs
 // q_i and waits for it.  us with one / two, float32: 128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3) (3 920 edges per edge of the
 // longest target) 883 / 762 (four: 808); 64 x 128, radius 4 pi / 64 (2 120) 575 / 318; 2 562 points of even degree 200 (2 500) 199 / 121;
 // 10 242 points, 4 heads of 8 x (m <= 2), degree 12 (8 400) 39 / 47, degree 200 429 / 432; 163 842, degree 12 457 / 623.  Eight heads' groups of
-// four lanes take longer over an edge: 10 242 points, degree 21 92 / 82, degree 100 356 / 285, degree 11 57 / 57.
+// four lanes take longer over an edge: 10 242 points, degree 21 92 / 82, degree 100 356 / 285, degree 11 57 / 57.  (All before the walk
+// below lost its branches.)
+//
+// What bounds it: the issue of what surrounds the gathers.  With every slot of a lane looked up and branched around in the walk the
+// first of these took 740 us, with the kind of a slot known and lanes without a copy reading nothing 511 (two edges in flight 683,
+// two with their sources read ahead 614); 99 x 198, radius 2.5 pi / 99: 8 heads of 8 x (m <= 2) 494 -> 278, of 16 x (m <= 2) 2 014 -> 546,
+// 120 x 200, radius 3 pi / 120, 8 heads of 4 x (m <= 1) 447 -> 262.  CTAs of 8 or 16 warps on neighbouring targets: 583, 566.
 int score_parts(int64_t n_nodes, int64_t n_edges, int64_t deg_max, int H) {
   return n_edges <= 4096 * deg_max || (H == 8 && n_edges >= 16 * n_nodes) ? 2 : 1;
 }
 
+// The logits of a target's edges turn, turn + turns, ... and their maximum, in the descriptor's order and number by number.  Not
+// inlined: in the kernel's body it cost the usual walk 17 % (513 -> 602 us).
+template <typename T>
+__device__ __noinline__ T logits_in_any_order(const SoftmaxArgs<T>* args, int64_t i, int turn, int turns, int h, int s, int L, unsigned group_mask) {
+  const SoftmaxArgs<T>& a = *args;
+  const T* q_i = a.q + i * a.D;
+  T m = neg_inf<T>();
+  for (int64_t e = a.row_ptr[i] + turn; e < a.row_ptr[i + 1]; e += turns) {
+    const T *k_j = a.k + a.source[e] * a.D, *tau = a.transport + e * a.orders * 2;
+    T sum = T(0);
+    for (int f = 0; f < a.F; ++f) {
+      const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2];
+      for (int u = s; u < a_n; u += L) {
+        const int c = off + (n == 0 ? 1 : 2) * (h * a_n + u);
+        if (n == 0) sum += q_i[c] * k_j[c];
+        else sum += q_i[c] * (tau[2 * n] * k_j[c] - tau[2 * n + 1] * k_j[c + 1]) + q_i[c + 1] * (tau[2 * n] * k_j[c + 1] + tau[2 * n + 1] * k_j[c]);
+      }
+    }
+    for (int o = L >> 1; o > 0; o >>= 1) sum += __shfl_xor_sync(group_mask, sum, o);
+    const T lw = a.scale * sum + a.bias[e];
+    if (a.inside[e] && lw > m) m = lw;
+    if (s == 0) a.alpha[e * a.H + h] = lw;
+  }
+  return m;
+}
+
 template <typename T, int R, int NF, int PARTS, bool SHARED>
-__global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArgs<T> a) {
+__global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(const __grid_constant__ SoftmaxArgs<T> a) {
   constexpr int FN = NF ? NF : MAX_F, TARGETS = 4 / PARTS;
   __shared__ T max_s[TARGETS][PARTS][MAX_H], sum_s[TARGETS][PARTS][MAX_H];
   const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % PARTS, mine = (threadIdx.x >> 5) / PARTS;
@@ -198,6 +230,7 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
   const unsigned group_mask = SHARED ? ((1u << (a.H * L)) - 1u) << (share * a.H * L) : 0xffffffffu;
   int col[FN][R], order[FN];
   uintptr_t bits = bits_of(a.k) | bits_of(a.transport) | (uintptr_t)a.D * sizeof(T);
+  bool sorted = true;  // NF: frequency 0 can only be the first
   T qr[FN][R], qi[FN][R];
 #pragma unroll
   for (int f = 0; f < FN; ++f) {
@@ -208,6 +241,7 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
       const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2];
       order[f] = n;
       if (n != 0) bits |= (uintptr_t)off * sizeof(T);
+      else if (NF && f > 0) sorted = false;
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         const int u = s + L * r;
@@ -227,7 +261,7 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
   T* const alpha = a.alpha + e0 * a.H + h;
   T m = neg_inf<T>();
   constexpr int U = 4;  // edges in flight: their gathers of k_j are issued together (8: 0.96 ms against 0.88)
-  auto walk = [&](auto is_vec) {  // every (re, im) and phase is read as a pair
+  auto walk = [&](auto is_vec) {  // VEC: every (re, im) and phase is read as a pair
     constexpr bool VEC = decltype(is_vec)::value;
     // this lane's share of <q_i, tau k_j> for one edge
     auto dot = [&](int t, unsigned j) -> T {
@@ -236,18 +270,18 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
 #pragma unroll
       for (int f = 0; f < FN; ++f) {
         if (!NF && order[f] < 0) continue;
-        T tr = T(1), ti = T(0);
-        if (order[f]) load_pair<VEC>(tau + 2 * order[f], tr, ti);
+        if ((!NF || f == 0) && order[f] == 0) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) sum += qr[f][r] * (col[f][r] >= 0 ? k_j[col[f][r]] : T(0));
+          continue;
+        }
+        T tr = T(0), ti = T(0);
+        if (col[f][0] >= 0) load_pair<VEC>(tau + 2 * order[f], tr, ti);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          if (col[f][r] < 0) continue;
-          if (order[f] == 0) {
-            sum += qr[f][r] * k_j[col[f][r]];
-          } else {
-            T kr, ki;
-            load_pair<VEC>(k_j + col[f][r], kr, ki);
-            sum += qr[f][r] * (tr * kr - ti * ki) + qi[f][r] * (tr * ki + ti * kr);
-          }
+          T kr = T(0), ki = T(0);
+          if (col[f][r] >= 0) load_pair<VEC>(k_j + col[f][r], kr, ki);
+          sum += qr[f][r] * (tr * kr - ti * ki) + qi[f][r] * (tr * ki + ti * kr);
         }
       }
       return sum;
@@ -270,7 +304,8 @@ __global__ void __launch_bounds__(128) softmax_forward_grouped_kernel(SoftmaxArg
     };
     for_edges<U, false>(part * shares + share, PARTS * shares, degree, source, edges);
   };
-  if (whole_pairs<T>(bits)) walk(std::true_type());
+  if (!sorted) m = present ? logits_in_any_order(&a, i, part * shares + share, PARTS * shares, h, s, L, group_mask) : m;
+  else if (whole_pairs<T>(bits)) walk(std::true_type());
   else walk(std::false_type());
   for (int o = a.H * L; SHARED && o < 32; o <<= 1) {
     const T other = __shfl_xor_sync(0xffffffffu, m, o);
@@ -463,8 +498,106 @@ __device__ __forceinline__ void softmax_backward_node(const SoftmaxArgs<T>& a, c
   }
 }
 
-template <typename T, bool VECTOR, bool AHEAD>
-__global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
+// The same with a group of lanes per head, as in the forward: a lane owns its head's copies s, s + L, ... of every frequency, and
+// one walk over the edges serves them all.  Every pair is read as one; frequency 0 can only be the first.
+template <int NF, int R, bool VECTOR, bool AHEAD, typename T>
+__device__ __forceinline__ void softmax_backward_heads(const SoftmaxArgs<T>& a, int shares, int64_t i) {
+  constexpr int U = R == 1 ? (NF == 2 ? 4 : 2) : R == 2 ? 2 : 1;
+  const int lane = threadIdx.x & 31, full = 32 / a.H, L = full / shares;
+  const int share = lane / (a.H * L), h = lane / L % a.H, s = lane % L;
+  int col[NF][R], order[NF];
+  T qr[NF][R], qi[NF][R], dqr[NF][R], dqi[NF][R];
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2];
+    order[f] = n;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int u = s + L * r;
+      col[f][r] = -1;
+      qr[f][r] = qi[f][r] = dqr[f][r] = dqi[f][r] = T(0);
+      if (u < a_n) {
+        col[f][r] = off + (n == 0 ? 1 : 2) * (h * a_n + u);
+        qr[f][r] = a.q[i * a.D + col[f][r]];
+        if (n != 0) qi[f][r] = a.q[i * a.D + col[f][r] + 1];
+      }
+    }
+  }
+  const int64_t e0 = a.row_ptr[i];
+  const int degree = (int)(a.row_ptr[i + 1] - e0);
+  const T *alpha = a.alpha_in + e0 * a.H + h, *dalpha = a.dalpha + e0 * a.H + h, *transport = a.transport + e0 * a.orders * 2;
+  T total = T(0);  // sum_e alpha dalpha of the head
+  for (int t = s + L * share; t < degree; t += full) total += alpha[(size_t)(unsigned)t * (unsigned)a.H] * dalpha[(size_t)(unsigned)t * (unsigned)a.H];
+  for (int o = L >> 1; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  for (int o = a.H * L; o < 32; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  const unsigned D = a.D, tau_step = 2 * a.orders;
+  for_edges<U, AHEAD>(share, shares, degree, a.source + e0, [&](int t, auto count, auto from) {
+    constexpr int N = decltype(count)::value;
+    T ds[N], tr[N][NF], ti[N][NF], kr[N][NF][R], ki[N][NF][R];
+    size_t j[N];
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      const unsigned x = t + u;
+      j[u] = (size_t)from(u) * D;
+      ds[u] = a.scale * alpha[(size_t)x * (unsigned)a.H] * (dalpha[(size_t)x * (unsigned)a.H] - total);
+      const T *k_j = a.k + j[u], *tau = transport + (size_t)x * tau_step;
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        tr[u][f] = ti[u][f] = T(0);
+        const bool scalar = f == 0 && order[0] == 0;
+        if (!scalar && col[f][0] >= 0) load_pair<true>(tau + 2 * order[f], tr[u][f], ti[u][f]);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          kr[u][f][r] = ki[u][f][r] = T(0);
+          if (col[f][r] >= 0) {
+            if (scalar) kr[u][f][r] = k_j[col[f][r]];
+            else load_pair<true>(k_j + col[f][r], kr[u][f][r], ki[u][f][r]);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+      T* dk_j = a.dk + j[u];
+#pragma unroll
+      for (int f = 0; f < NF; ++f) {
+        const bool scalar = f == 0 && order[0] == 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if (scalar) {
+            dqr[f][r] += ds[u] * kr[u][f][r];
+            if (col[f][r] >= 0) atomicAdd(dk_j + col[f][r], ds[u] * qr[f][r]);
+          } else {
+            dqr[f][r] += ds[u] * (tr[u][f] * kr[u][f][r] - ti[u][f] * ki[u][f][r]);  // (tau k)
+            dqi[f][r] += ds[u] * (tr[u][f] * ki[u][f][r] + ti[u][f] * kr[u][f][r]);
+            if (col[f][r] >= 0)  // conj(tau) q
+              add_pair<VECTOR>(dk_j + col[f][r], ds[u] * (tr[u][f] * qr[f][r] + ti[u][f] * qi[f][r]), ds[u] * (tr[u][f] * qi[f][r] - ti[u][f] * qr[f][r]));
+          }
+        }
+      }
+    }
+  });
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      for (int o = a.H * L; o < 32; o <<= 1) {
+        dqr[f][r] += __shfl_xor_sync(0xffffffffu, dqr[f][r], o);
+        dqi[f][r] += __shfl_xor_sync(0xffffffffu, dqi[f][r], o);
+      }
+      if (share == 0 && col[f][r] >= 0) {
+        T* dq = a.dq + i * a.D + col[f][r];
+        if (f == 0 && order[0] == 0) *dq = dqr[f][r];
+        else store_pair<true>(dq, dqr[f][r], dqi[f][r]);
+      }
+    }
+  }
+}
+
+// NF frequencies by heads' lanes, where these hold at most R copies of each and every pair is one; otherwise, and with NF = 0, item
+// by item
+template <typename T, int NF, int R, bool VECTOR, bool AHEAD>
+__global__ void __launch_bounds__(128, R == 1 || sizeof(T) == 8 ? 0 : 4) softmax_backward_kernel(const __grid_constant__ SoftmaxArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ScoreItem* items_s = reinterpret_cast<ScoreItem*>(smem_raw);
   int n_items = 0, n_real = 0;
@@ -479,6 +612,23 @@ __global__ void softmax_backward_kernel(SoftmaxArgs<T> a) {
   __syncthreads();
   const bool vec = whole_pairs<T>(bits);
   const int warps = blockDim.x >> 5;
+  if constexpr (NF > 0) {
+    int most = 1, later_scalars = 0;
+    for (int f = 0; f < NF; ++f) {
+      most = max(most, (int)a.desc[f * DESC + 1]);
+      later_scalars += f > 0 && a.desc[f * DESC] == 0;
+    }
+    const int full = 32 / a.H;
+    if (vec && later_scalars == 0 && most <= R * full) {
+      int shares = 1;
+      while (2 * shares * most <= full) shares *= 2;
+      for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
+        const int64_t i = from_both_ends(x, a.n_nodes);
+        softmax_backward_heads<NF, R, VECTOR, AHEAD>(a, shares, i);
+      }
+      return;
+    }
+  }
   for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
     const int64_t i = from_both_ends(x, a.n_nodes);
     if (vec) softmax_backward_node<VECTOR, true, AHEAD>(a, items_s, n_items, n_real, i);
@@ -714,15 +864,17 @@ int softmax_forward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, int ma
       constexpr int P = decltype(parts)::value;
       const unsigned blocks = (unsigned)((a.n_nodes * P + 3) / 4);
       auto run = [&](auto kernel) { kernel<<<blocks, 128, 0, stream>>>(a); };
-      if (a.shares > 1 && a.F == 3) run(softmax_forward_grouped_kernel<T, 1, 3, P, true>);
-      else if (a.shares > 1 && a.F == 4) run(softmax_forward_grouped_kernel<T, 1, 4, P, true>);
-      else if (a.shares > 1) run(softmax_forward_grouped_kernel<T, 1, 0, P, true>);
-      else if (per_lane <= 1 && a.F == 3) run(softmax_forward_grouped_kernel<T, 1, 3, P, false>);
-      else if (per_lane <= 1 && a.F == 4) run(softmax_forward_grouped_kernel<T, 1, 4, P, false>);
-      else if (per_lane <= 1) run(softmax_forward_grouped_kernel<T, 1, 0, P, false>);
-      else if (per_lane <= 2 && a.F == 3) run(softmax_forward_grouped_kernel<T, 2, 3, P, false>);
-      else if (per_lane <= 2) run(softmax_forward_grouped_kernel<T, 2, 0, P, false>);
-      else run(softmax_forward_grouped_kernel<T, 4, 0, P, false>);
+      auto frequencies = [&](auto nf) {
+        constexpr int NF = decltype(nf)::value;
+        if (a.shares > 1) run(softmax_forward_grouped_kernel<T, 1, NF, P, true>);
+        else if (per_lane <= 1) run(softmax_forward_grouped_kernel<T, 1, NF, P, false>);
+        else if (per_lane <= 2) run(softmax_forward_grouped_kernel<T, 2, NF, P, false>);
+        else run(softmax_forward_grouped_kernel<T, 4, NF, P, false>);
+      };
+      if (a.F == 2) frequencies(std::integral_constant<int, 2>());
+      else if (a.F == 3) frequencies(std::integral_constant<int, 3>());
+      else if (a.F == 4) frequencies(std::integral_constant<int, 4>());
+      else frequencies(std::integral_constant<int, 0>());
       return launch_status("gm_softmax_forward");
     };
     return score_parts(a.n_nodes, n_edges, deg_max, a.H) == 2 ? go(std::integral_constant<int, 2>()) : go(std::integral_constant<int, 1>());
@@ -744,16 +896,40 @@ int softmax_backward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, cudaS
   // dk by pairs where targets have many edges, on average or some of them: with few the vector reductions only hold the next
   // target's loads back.  us by numbers / by pairs: 163 842 points of even degree 12 492 / 552, 40 962 of degree 12 146 / 157, 10 242 of degree 21
   // 69 / 67, of degree 100 261 / 232; 64 x 128, radius 2 pi / 64 (mean 38, at most 257) 220 / 200; 128 x 256, radius 3 pi / 128 1 051 / 829.
-  const bool pairs = n_edges >= 24 * a.n_nodes || deg_max * a.n_nodes >= 4 * n_edges;
+  const bool uneven = deg_max * a.n_nodes >= 4 * n_edges, pairs = n_edges >= 24 * a.n_nodes || uneven;
   auto go = [&](auto kernel) { kernel<<<conv_grid(a.n_nodes), CONV_THREADS, a.D * sizeof(ScoreItem), stream>>>(a); };
+  // By heads where some targets have many more edges than the others: one walk over a polar target's edges instead of one per
+  // frequency and 32 items.  us by items / by heads: 128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3) 820 / 764, 99 x 198, radius 2.5 pi / 99, 8 of
+  // 4 x (m <= 3) 512 / 382, 8 of 8 x (m <= 2) 703 / 512, 2 of 16 x (m <= 3) 442 / 328, 64 x 128, radius 4 pi / 64 329 / 290; where all have 40, 30 000
+  // points, 4 heads of 8 x (m <= 1) 211 / 249, 20 000, 8 of 5 x (m <= 2) 287 / 430, 8 of 16 x (m <= 3) 960 / 1 425.
   // sources read ahead where the launch is a few waves of nodes and lasts as long as its chains of gathers: 64 x 128, radius 4 pi / 64, 4
   // heads of 8 x (m <= 3) 417 -> 350 us, 50 x 100 76 -> 63; more nodes hide the gathers and want the registers (128 x 256 809 -> 883,
   // 100 x 200 45 -> 53)
   const bool ahead = a.n_nodes <= 12288;
-  if (pairs && ahead) go(softmax_backward_kernel<T, true, true>);
-  else if (pairs) go(softmax_backward_kernel<T, true, false>);
-  else if (ahead) go(softmax_backward_kernel<T, false, true>);
-  else go(softmax_backward_kernel<T, false, false>);
+  auto frequencies = [&](auto nf, auto r) {
+    constexpr int NF = decltype(nf)::value, R = decltype(r)::value;
+    if (pairs && ahead) go(softmax_backward_kernel<T, NF, R, true, true>);
+    else if (pairs) go(softmax_backward_kernel<T, NF, R, true, false>);
+    else if (ahead) go(softmax_backward_kernel<T, NF, R, false, true>);
+    else go(softmax_backward_kernel<T, NF, R, false, false>);
+  };
+  // as many copies a lane as a row of equal multiplicities has, the scalars' among them (the kernel sees what there really is)
+  const int lanes = 32 / a.H, copies = a.F > 0 ? (a.D / a.H + 2 * a.F - 2) / (2 * a.F - 1) : 1, each = (copies + lanes - 1) / lanes;
+  int room = lanes * each;
+  while (each == 1 && room >= 2 * copies) room /= 2;
+  auto held = [&](auto nf) {
+    if (each <= 1) frequencies(nf, std::integral_constant<int, 1>());
+    else if (each <= 2) frequencies(nf, std::integral_constant<int, 2>());
+    else frequencies(nf, std::integral_constant<int, 4>());
+  };
+  // (Five copies leave three of a head's eight lanes idle, which a large launch pays for: 120 x 240, radius 2.5 pi / 120, 4 heads of
+  // 5 x (m <= 3) 431 / 523, 60 x 120 155 / 156.)
+  const bool filled = a.n_nodes <= 12288 || 4 * copies >= 3 * room;
+  const bool even = uneven && filled && (a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8);  // heads that split a warp evenly
+  if (even && a.F == 2 && each <= 4) held(std::integral_constant<int, 2>());
+  else if (even && a.F == 3 && each <= 4) held(std::integral_constant<int, 3>());
+  else if (even && a.F == 4 && each <= 4) held(std::integral_constant<int, 4>());
+  else frequencies(std::integral_constant<int, 0>(), std::integral_constant<int, 1>());
   return launch_status("gm_softmax_backward");
 }
 

@@ -106,6 +106,11 @@ def test_conv_forward_backward(ext, reference_modules, case, dtype):
     ({0: 4, 1: 4, 2: 4}, 2),   # scores: two heads of four lanes, four groups
     ({0: 5, 1: 5, 2: 5}, 4),   # five copies in groups of eight lanes
     ({0: 2, 1: 2, 2: 2, 3: 2}, 8),
+    ({0: 8, 1: 8}, 4),         # as many copies as lanes
+    ({0: 5, 1: 6, 2: 5}, 8),   # a second round of copies, pairs at even offsets
+    ({0: 16, 1: 15, 2: 16, 3: 13}, 8),  # four rounds
+    ({1: 17, 2: 3}, 2),        # no scalars
+    ({1: 3, 0: 5}, 2),         # the scalars behind others (scores, forward)
 ])
 def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
     """Neighbourhoods of 0 to 130 edges -- fewer than the groups, one more than they take at a time, many turns -- against the oracle
@@ -141,8 +146,11 @@ def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
     alpha = O.softmax_forward(*wide(q, k, transport, bias), inside, desc, row_ptr, source, heads, 0.3)
     tables = [cuda(x) for x in (transport, bias, inside, desc, row_ptr, source)]
     compare([ext.softmax_forward(cuda(q), cuda(k), *tables, heads, 0.3, 130)], [alpha], ["alpha"])
+    if list(types) != sorted(types):
+        return
     want = O.softmax_backward(*wide(da, q, k, transport), desc, row_ptr, source, alpha, heads, 0.3)
-    compare(ext.softmax_backward(cuda(da), cuda(q), cuda(k), *tables, cuda(alpha.astype(dtype)), heads, 0.3, 130), want, ["dq", "dk"])
+    for largest in (130, 1):  # uneven neighbourhoods: by heads; as if all were alike: by items
+        compare(ext.softmax_backward(cuda(da), cuda(q), cuda(k), *tables, cuda(alpha.astype(dtype)), heads, 0.3, largest), want, ["dq", "dk"])
     if heads == 1:
         a0 = types.get(0, 0)
         rc, cc = cast(rng.standard_normal((e, a0)), rng.standard_normal((e, coef)))
