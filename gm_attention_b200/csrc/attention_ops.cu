@@ -498,106 +498,8 @@ __device__ __forceinline__ void softmax_backward_node(const SoftmaxArgs<T>& a, c
   }
 }
 
-// The same with a group of lanes per head, as in the forward: a lane owns its head's copies s, s + L, ... of every frequency, and
-// one walk over the edges serves them all.  Every pair is read as one; frequency 0 can only be the first.
-template <int NF, int R, bool VECTOR, bool AHEAD, typename T>
-__device__ __forceinline__ void softmax_backward_heads(const SoftmaxArgs<T>& a, int shares, int64_t i) {
-  constexpr int U = R == 1 ? (NF == 2 ? 4 : 2) : R == 2 ? 2 : 1;
-  const int lane = threadIdx.x & 31, full = 32 / a.H, L = full / shares;
-  const int share = lane / (a.H * L), h = lane / L % a.H, s = lane % L;
-  int col[NF][R], order[NF];
-  T qr[NF][R], qi[NF][R], dqr[NF][R], dqi[NF][R];
-#pragma unroll
-  for (int f = 0; f < NF; ++f) {
-    const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2];
-    order[f] = n;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int u = s + L * r;
-      col[f][r] = -1;
-      qr[f][r] = qi[f][r] = dqr[f][r] = dqi[f][r] = T(0);
-      if (u < a_n) {
-        col[f][r] = off + (n == 0 ? 1 : 2) * (h * a_n + u);
-        qr[f][r] = a.q[i * a.D + col[f][r]];
-        if (n != 0) qi[f][r] = a.q[i * a.D + col[f][r] + 1];
-      }
-    }
-  }
-  const int64_t e0 = a.row_ptr[i];
-  const int degree = (int)(a.row_ptr[i + 1] - e0);
-  const T *alpha = a.alpha_in + e0 * a.H + h, *dalpha = a.dalpha + e0 * a.H + h, *transport = a.transport + e0 * a.orders * 2;
-  T total = T(0);  // sum_e alpha dalpha of the head
-  for (int t = s + L * share; t < degree; t += full) total += alpha[(size_t)(unsigned)t * (unsigned)a.H] * dalpha[(size_t)(unsigned)t * (unsigned)a.H];
-  for (int o = L >> 1; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-  for (int o = a.H * L; o < 32; o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-  const unsigned D = a.D, tau_step = 2 * a.orders;
-  for_edges<U, AHEAD>(share, shares, degree, a.source + e0, [&](int t, auto count, auto from) {
-    constexpr int N = decltype(count)::value;
-    T ds[N], tr[N][NF], ti[N][NF], kr[N][NF][R], ki[N][NF][R];
-    size_t j[N];
-#pragma unroll
-    for (int u = 0; u < N; ++u) {
-      const unsigned x = t + u;
-      j[u] = (size_t)from(u) * D;
-      ds[u] = a.scale * alpha[(size_t)x * (unsigned)a.H] * (dalpha[(size_t)x * (unsigned)a.H] - total);
-      const T *k_j = a.k + j[u], *tau = transport + (size_t)x * tau_step;
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        tr[u][f] = ti[u][f] = T(0);
-        const bool scalar = f == 0 && order[0] == 0;
-        if (!scalar && col[f][0] >= 0) load_pair<true>(tau + 2 * order[f], tr[u][f], ti[u][f]);
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          kr[u][f][r] = ki[u][f][r] = T(0);
-          if (col[f][r] >= 0) {
-            if (scalar) kr[u][f][r] = k_j[col[f][r]];
-            else load_pair<true>(k_j + col[f][r], kr[u][f][r], ki[u][f][r]);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < N; ++u) {
-      T* dk_j = a.dk + j[u];
-#pragma unroll
-      for (int f = 0; f < NF; ++f) {
-        const bool scalar = f == 0 && order[0] == 0;
-#pragma unroll
-        for (int r = 0; r < R; ++r) {
-          if (scalar) {
-            dqr[f][r] += ds[u] * kr[u][f][r];
-            if (col[f][r] >= 0) atomicAdd(dk_j + col[f][r], ds[u] * qr[f][r]);
-          } else {
-            dqr[f][r] += ds[u] * (tr[u][f] * kr[u][f][r] - ti[u][f] * ki[u][f][r]);  // (tau k)
-            dqi[f][r] += ds[u] * (tr[u][f] * ki[u][f][r] + ti[u][f] * kr[u][f][r]);
-            if (col[f][r] >= 0)  // conj(tau) q
-              add_pair<VECTOR>(dk_j + col[f][r], ds[u] * (tr[u][f] * qr[f][r] + ti[u][f] * qi[f][r]), ds[u] * (tr[u][f] * qi[f][r] - ti[u][f] * qr[f][r]));
-          }
-        }
-      }
-    }
-  });
-#pragma unroll
-  for (int f = 0; f < NF; ++f) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      for (int o = a.H * L; o < 32; o <<= 1) {
-        dqr[f][r] += __shfl_xor_sync(0xffffffffu, dqr[f][r], o);
-        dqi[f][r] += __shfl_xor_sync(0xffffffffu, dqi[f][r], o);
-      }
-      if (share == 0 && col[f][r] >= 0) {
-        T* dq = a.dq + i * a.D + col[f][r];
-        if (f == 0 && order[0] == 0) *dq = dqr[f][r];
-        else store_pair<true>(dq, dqr[f][r], dqi[f][r]);
-      }
-    }
-  }
-}
-
-// NF frequencies by heads' lanes, where these hold at most R copies of each and every pair is one; otherwise, and with NF = 0, item
-// by item
-template <typename T, int NF, int R, bool VECTOR, bool AHEAD>
-__global__ void __launch_bounds__(128, R == 1 || sizeof(T) == 8 ? 0 : 4) softmax_backward_kernel(const __grid_constant__ SoftmaxArgs<T> a) {
+template <typename T, bool VECTOR, bool AHEAD>
+__global__ void __launch_bounds__(128) softmax_backward_kernel(const __grid_constant__ SoftmaxArgs<T> a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ScoreItem* items_s = reinterpret_cast<ScoreItem*>(smem_raw);
   int n_items = 0, n_real = 0;
@@ -612,23 +514,6 @@ __global__ void __launch_bounds__(128, R == 1 || sizeof(T) == 8 ? 0 : 4) softmax
   __syncthreads();
   const bool vec = whole_pairs<T>(bits);
   const int warps = blockDim.x >> 5;
-  if constexpr (NF > 0) {
-    int most = 1, later_scalars = 0;
-    for (int f = 0; f < NF; ++f) {
-      most = max(most, (int)a.desc[f * DESC + 1]);
-      later_scalars += f > 0 && a.desc[f * DESC] == 0;
-    }
-    const int full = 32 / a.H;
-    if (vec && later_scalars == 0 && most <= R * full) {
-      int shares = 1;
-      while (2 * shares * most <= full) shares *= 2;
-      for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
-        const int64_t i = from_both_ends(x, a.n_nodes);
-        softmax_backward_heads<NF, R, VECTOR, AHEAD>(a, shares, i);
-      }
-      return;
-    }
-  }
   for (int64_t x = (int64_t)blockIdx.x * warps + (threadIdx.x >> 5); x < a.n_nodes; x += (int64_t)gridDim.x * warps) {
     const int64_t i = from_both_ends(x, a.n_nodes);
     if (vec) softmax_backward_node<VECTOR, true, AHEAD>(a, items_s, n_items, n_real, i);
@@ -898,38 +783,16 @@ int softmax_backward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, cudaS
   // 69 / 67, of degree 100 261 / 232; 64 x 128, radius 2 pi / 64 (mean 38, at most 257) 220 / 200; 128 x 256, radius 3 pi / 128 1 051 / 829.
   const bool uneven = deg_max * a.n_nodes >= 4 * n_edges, pairs = n_edges >= 24 * a.n_nodes || uneven;
   auto go = [&](auto kernel) { kernel<<<conv_grid(a.n_nodes), CONV_THREADS, a.D * sizeof(ScoreItem), stream>>>(a); };
-  // By heads where some targets have many more edges than the others: one walk over a polar target's edges instead of one per
-  // frequency and 32 items.  us by items / by heads: 128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3) 820 / 764, 99 x 198, radius 2.5 pi / 99, 8 of
-  // 4 x (m <= 3) 512 / 382, 8 of 8 x (m <= 2) 703 / 512, 2 of 16 x (m <= 3) 442 / 328, 64 x 128, radius 4 pi / 64 329 / 290; where all have 40, 30 000
-  // points, 4 heads of 8 x (m <= 1) 211 / 249, 20 000, 8 of 5 x (m <= 2) 287 / 430, 8 of 16 x (m <= 3) 960 / 1 425.
-  // sources read ahead where the launch is a few waves of nodes and lasts as long as its chains of gathers: 64 x 128, radius 4 pi / 64, 4
-  // heads of 8 x (m <= 3) 417 -> 350 us, 50 x 100 76 -> 63; more nodes hide the gathers and want the registers (128 x 256 809 -> 883,
-  // 100 x 200 45 -> 53)
-  const bool ahead = a.n_nodes <= 12288;
-  auto frequencies = [&](auto nf, auto r) {
-    constexpr int NF = decltype(nf)::value, R = decltype(r)::value;
-    if (pairs && ahead) go(softmax_backward_kernel<T, NF, R, true, true>);
-    else if (pairs) go(softmax_backward_kernel<T, NF, R, true, false>);
-    else if (ahead) go(softmax_backward_kernel<T, NF, R, false, true>);
-    else go(softmax_backward_kernel<T, NF, R, false, false>);
-  };
-  // as many copies a lane as a row of equal multiplicities has, the scalars' among them (the kernel sees what there really is)
-  const int lanes = 32 / a.H, copies = a.F > 0 ? (a.D / a.H + 2 * a.F - 2) / (2 * a.F - 1) : 1, each = (copies + lanes - 1) / lanes;
-  int room = lanes * each;
-  while (each == 1 && room >= 2 * copies) room /= 2;
-  auto held = [&](auto nf) {
-    if (each <= 1) frequencies(nf, std::integral_constant<int, 1>());
-    else if (each <= 2) frequencies(nf, std::integral_constant<int, 2>());
-    else frequencies(nf, std::integral_constant<int, 4>());
-  };
-  // (Five copies leave three of a head's eight lanes idle, which a large launch pays for: 120 x 240, radius 2.5 pi / 120, 4 heads of
-  // 5 x (m <= 3) 431 / 523, 60 x 120 155 / 156.)
-  const bool filled = a.n_nodes <= 12288 || 4 * copies >= 3 * room;
-  const bool even = uneven && filled && (a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8);  // heads that split a warp evenly
-  if (even && a.F == 2 && each <= 4) held(std::integral_constant<int, 2>());
-  else if (even && a.F == 3 && each <= 4) held(std::integral_constant<int, 3>());
-  else if (even && a.F == 4 && each <= 4) held(std::integral_constant<int, 4>());
-  else frequencies(std::integral_constant<int, 0>(), std::integral_constant<int, 1>());
+  // Sources read ahead where the chains of gathers show: some targets' long ones, or few targets.  us without / with: 120 x 240, radius
+  // 2.5 pi / 120, 4 heads of 5 x (m <= 3) 505 / 389, 99 x 198, radius 2.5 pi / 99, 8 of 5 x (m <= 2) 502 / 346, 8 of 16 x (m <= 2) 1 372 / 980, 128 x 256,
+  // radius 3 pi / 128, 4 of 8 x (m <= 3) 822 / 775; points of even degree 40, 30 000, 4 of 8 x (m <= 2) 303 / 319, of 8 x (m <= 1) 207 / 229,
+  // 3 000 85 / 82.  (A group of lanes per head and one walk for all frequencies: 765 and 286 on the lattices of 4 heads of 8 x (m <= 3), but
+  // 1 158 for the 16 copies and 502 for the five, and 1 425 against 957 where 20 000 points have 40 edges each, 8 of 16 x (m <= 3).)
+  const bool ahead = uneven || a.n_nodes <= 12288;
+  if (pairs && ahead) go(softmax_backward_kernel<T, true, true>);
+  else if (pairs) go(softmax_backward_kernel<T, true, false>);
+  else if (ahead) go(softmax_backward_kernel<T, false, true>);
+  else go(softmax_backward_kernel<T, false, false>);
   return launch_status("gm_softmax_backward");
 }
 

@@ -149,7 +149,7 @@ def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
     if list(types) != sorted(types):
         return
     want = O.softmax_backward(*wide(da, q, k, transport), desc, row_ptr, source, alpha, heads, 0.3)
-    for largest in (130, 1):  # uneven neighbourhoods: by heads; as if all were alike: by items
+    for largest in (130, 1):  # uneven neighbourhoods, and as if all were alike
         compare(ext.softmax_backward(cuda(da), cuda(q), cuda(k), *tables, cuda(alpha.astype(dtype)), heads, 0.3, largest), want, ["dq", "dk"])
     if heads == 1:
         a0 = types.get(0, 0)
