@@ -392,13 +392,13 @@ struct Lanes {
     return v;
   }
 };
-// p[0] += x, p[1] += y.  A float pair on an 8-byte boundary is one vector reduction: half as many operations for the L2
-// units.  128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32: 1 098 -> 897 us for the scores' backward.  (The
-// depthwise backward and the fused layer's on general graphs lose by it, 1 045 -> 1 190 and 363 -> 394 us.)
-template <bool VECTOR, typename T>
+// p[0] += x, p[1] += y.  A float pair on an 8-byte boundary (ALIGNED: known to be on one) is one vector reduction: half as many
+// operations for the L2 units.  128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3), float32: 1 098 -> 897 us for the scores' backward.
+// (The depthwise backward lost by it, 1 045 -> 1 190, while every access tested its address; now it gains, 745 -> 712.)
+template <bool VECTOR, bool ALIGNED = false, typename T>
 __device__ __forceinline__ void add_pair(T* p, T x, T y) {
   if constexpr (VECTOR && std::is_same<T, float>::value) {
-    if ((reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+    if (ALIGNED || (reinterpret_cast<uintptr_t>(p) & 7) == 0) {
       asm volatile("red.global.add.v2.f32 [%0], {%1, %2};\n" ::"l"(p), "f"(x), "f"(y));
       return;
     }
@@ -536,8 +536,11 @@ __device__ __forceinline__ int build_conv_items(const int64_t* desc, int F, Conv
 
 // Depthwise conv, forward: a warp per target node, a lane per item (scalar items and complex items in separate
 // passes, so a pass never diverges); the node's edges are walked four at a time, with the four edges' loads issued before their
-// arithmetic.
-constexpr int CONV_UNROLL = 4, CONV_BACKWARD_UNROLL = 3;  // (backward: 1 033 us with four, 950 with three, 1 083 with two; forward 682, 714, 856)
+// arithmetic and the next four's sources read meanwhile.  What bounds it: the latency of the gathers and issue.  128 x 256, radius
+// 3 pi / 128, 16 x (m <= 2), float32, forward and backward: 675 + 940 us with every access testing its address, 504 with sources read
+// ahead and 110 registers, 428 with six CTAs to an SM (five 443; seven 420, but they spill) + 676 with seven; lane groups on narrow
+// fields: 4 x (m <= 1), radius 2.5 pi / 128, 380 + 503 -> 98 + 118.
+constexpr int CONV_UNROLL = 4, CONV_BACKWARD_UNROLL = 3;  // (backward: 710 us with four and five CTAs to an SM, 676 with three and seven)
 
 template <bool VEC, typename T>
 __device__ __forceinline__ void conv_forward_node(const ConvArgs<T>& a, const ConvItem* items_s, int n_items, int n_real, int64_t i) {
@@ -628,7 +631,7 @@ __device__ __forceinline__ void conv_backward_node(const ConvArgs<T>& a, const C
     const T dy = a.g[i * a.D + it.col];
     const T *r_at = a.rc + e0 * a.A0 + it.coef, *v_at = a.v + it.col;
     T *dr_at = a.drc + e0 * a.A0 + it.coef, *dv_at = a.dv + it.col;
-    for_edges<CONV_BACKWARD_UNROLL, false>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+    for_edges<CONV_BACKWARD_UNROLL, true>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
       constexpr int N = decltype(count)::value;
       T w[N], r[N], x[N];
       size_t j[N];
@@ -659,7 +662,7 @@ __device__ __forceinline__ void conv_backward_node(const ConvArgs<T>& a, const C
     T *dco_at = a.dcc + e0 * a.W + it.coef, *dv_at = a.dv + it.col;
     const unsigned phase_step = 2 * a.orders;
     const int behind = 2 * it.mult;
-    for_edges<CONV_BACKWARD_UNROLL, false>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
+    for_edges<CONV_BACKWARD_UNROLL, true>(lanes.group, lanes.groups, degree, source, [&](int t, auto count, auto from) {
       constexpr int N = decltype(count)::value;
       T w[N], rho[N], tr[N], ti[N], vr[N], vi[N], Ar[N], Ai[N], Br[N], Bi[N], ar[N], ai[N];
       size_t j[N];
@@ -693,8 +696,7 @@ __device__ __forceinline__ void conv_backward_node(const ConvArgs<T>& a, const C
         const T bdr = Br[u] * dmr + Bi[u] * dmi, bdi = Bi[u] * dmr - Br[u] * dmi;
         const T dzr = (Ar[u] * dmr + Ai[u] * dmi) + (wr * bdr - wi * bdi);
         const T dzi = (Ar[u] * dmi - Ai[u] * dmr) + (wr * bdi + wi * bdr);
-        atomicAdd(dv_at + j[u], tr[u] * dzr + ti[u] * dzi);
-        atomicAdd(dv_at + j[u] + 1, tr[u] * dzi - ti[u] * dzr);
+        add_pair<VEC, VEC>(dv_at + j[u], tr[u] * dzr + ti[u] * dzi, tr[u] * dzi - ti[u] * dzr);
       }
     });
   }
@@ -705,7 +707,7 @@ __global__ void __launch_bounds__(128, sizeof(T) == 8 ? 4 : BACKWARD ? 7 : 6) co
   extern __shared__ __align__(16) unsigned char smem_raw[];
   ConvItem* items_s = reinterpret_cast<ConvItem*>(smem_raw);
   const int n_items = build_conv_items(a.desc, a.F, items_s);
-  uintptr_t bits = bits_of(a.v) | bits_of(a.cc) | bits_of(a.transport) | bits_of(a.angular) | bits_of(a.out) | bits_of(a.g) | bits_of(a.dcc) |
+  uintptr_t bits = bits_of(a.v) | bits_of(a.cc) | bits_of(a.transport) | bits_of(a.angular) | bits_of(a.out) | bits_of(a.g) | bits_of(a.dcc) | bits_of(a.dv) |
                    (uintptr_t)(a.D | a.W) * sizeof(T);
   for (int f = 0; f < a.F; ++f)
     if (a.desc[f * DESC] != 0) bits |= (uintptr_t)(a.desc[f * DESC + 2] | a.desc[f * DESC + 3]) * sizeof(T);
