@@ -567,7 +567,7 @@ static int conv_apply(bool tensor_cores, const void* x, const float* table, cons
   cudaStream_t cs = (cudaStream_t)stream;
   GM_REQUIRE(!tensor_cores || (dtype == GM_BF16 && lconv::tensor_cores_can(a)), GM_ERR_UNSUPPORTED,
              "gm_lattice_conv_apply_tc: bfloat16 fields whose rows are whole 16-byte words on 16-byte boundaries");
-  if (tensor_cores || (dtype == GM_BF16 && lconv::tensor_cores_apply(a))) return lconv::apply_tc(a, n_order, cs);
+  if (tensor_cores ? lconv::tensor_cores_hold(a) : dtype == GM_BF16 && lconv::tensor_cores_apply(a)) return lconv::apply_tc(a, n_order, cs);
   const int elem = dtype == GM_F32 ? 4 : 2;
   StagedShape sh{};
   const int nb = staged_shape(a, elem, n_order, sh);

@@ -21,7 +21,8 @@ struct ConvArgs {
 
 // Tensor-core forms for bfloat16 fields: whether the sizes and addresses allow them, whether they are the faster ones, and the
 // launches.
-bool tensor_cores_can(const ConvArgs& a);
+bool tensor_cores_can(const ConvArgs& a);   // the fields are such as the kernels read
+bool tensor_cores_hold(const ConvArgs& a);  // apply's list of neighbour rows
 bool tensor_cores_apply(const ConvArgs& a);
 bool tensor_cores_table_grad(const ConvArgs& a);
 int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream);

@@ -681,8 +681,9 @@ __global__ void __launch_bounds__(2 * GROUP, 2) conv_apply_tc_kernel(const __gri
 
 bool tensor_cores_can(const ConvArgs& a) {
   const uintptr_t bits = reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.g) | reinterpret_cast<uintptr_t>(a.y);
-  return a.nlon % 8 == 0 && a.width % 8 == 0 && bits % 16 == 0 && 2 * (int64_t)a.halo + 1 <= AP_MAX_SPAN;
+  return a.nlon % 8 == 0 && a.width % 8 == 0 && bits % 16 == 0;
 }
+bool tensor_cores_hold(const ConvArgs& a) { return 2 * (int64_t)a.halo + 1 <= AP_MAX_SPAN; }
 
 // How apply cuts a field: blocks of columns, of tiles along a row, and samples that share a CTA: of a short row as many as its
 // tiles hold with their halos
@@ -708,7 +709,7 @@ static ApplyGrid apply_grid(const ConvArgs& a) {
 //                two samples of a field that is not wide (45 x 88, width 96: 38 / 38, width 160: 32 / 38; 64 x 128, width 160: 69 / 54, width
 //                320: 97 / 93; 128 x 128, width 320: 175 / 196); 8 tiles with one block of 32 columns and four samples (32 x 64: 32 / 22).
 bool tensor_cores_apply(const ConvArgs& a) {
-  if (!tensor_cores_can(a)) return false;
+  if (!tensor_cores_can(a) || !tensor_cores_hold(a)) return false;
   const int T = a.nlon / 8;
   const ApplyGrid grid = apply_grid(a);
   const int64_t ctas = grid.per_block * grid.col_blocks * a.rows, fill = (int64_t)grid.samples * std::min(T, AP_TILES);

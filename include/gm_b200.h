@@ -507,7 +507,8 @@ int gm_lattice_conv_table_grad(const void* g, const void* x, const int32_t* item
                                const int32_t* win_lo, const int32_t* win_off, const int32_t* blocks, int64_t n_blocks, int rows,
                                int nlon, int batch, int width, int halo, int table_width, int dtype, float* dtable, void* stream);
 /* The same by the tensor-core kernels whatever the sizes: GM_BF16, nlon and width multiples of 8, fields on 16-byte boundaries
- * (GM_ERR_UNSUPPORTED otherwise).  The calls above take them where they are the faster ones. */
+ * (GM_ERR_UNSUPPORTED otherwise); apply with more than 4096 neighbour rows a target row by the others.  The calls above take them
+ * where they are the faster ones. */
 int gm_lattice_conv_apply_tc(const void* x, const float* table, const int32_t* items, int n_items, const int32_t* win_cnt,
                              const int32_t* win_lo, const int32_t* win_off, const int32_t* order, int n_order, int rows, int nlon,
                              int batch, int width, int halo, int table_width, int transpose, int dtype, void* y, void* stream);
