@@ -329,9 +329,10 @@ def _readouts_fit(kernel: Any, needed: tuple, hidden: Tensor) -> bool:
 
 def _products_repaid(n_nodes: int, n_edges: int) -> bool:
     """Whether a node's products serve enough edges.  Forward and backward, float32, trunk 16, ms as factored form / pair
-    terms: {16, 16} -> {8, 8} on 30 000 nodes 3.53 / 2.71 at 4.9 edges per node, 3.63 / 3.63 at 8.6, 3.81 / 5.95 at 17 (the
-    products bound the factored form there); {2, 2} -> {8, 8} 1.97 / 1.90 at 6.8, 2.20 / 2.64 at 17.  Up to 8 192 nodes both
-    wait for their launches, of which the factored form has fewer: 1.32 / 1.42 at 2.6, 1.33 / 1.73 at 4.8."""
+    terms, before the products became two to three times faster: {16, 16} -> {8, 8} on 30 000 nodes 3.53 / 2.71 at 4.9 edges
+    per node, 3.63 / 3.63 at 8.6, 3.81 / 5.95 at 17 (the products bound the factored form there); {2, 2} -> {8, 8}
+    1.97 / 1.90 at 6.8, 2.20 / 2.64 at 17.  Up to 8 192 nodes both wait for their launches, of which the factored form has
+    fewer: 1.32 / 1.42 at 2.6, 1.33 / 1.73 at 4.8."""
     return n_edges >= (4 if n_nodes <= 8192 else 10) * n_nodes
 
 
