@@ -367,19 +367,45 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_wide_kernel(FArgs<T
   }
 }
 
-// out_i = sum over the target's edges of w_e * row_e  (factored.h:337-347): a warp per target, lanes over columns.
-template <typename T>
+// out_i = sum over the target's edges of w_e * row_e  (factored.h:337-347): a warp per target.  What bounds it: the rows' stream, and
+// the polar targets' chains of edges.  Lanes are vectors of V columns, and as many edges at a time as the vectors leave room for, whose
+// sums meet at the end.  128 x 256, radius 3 pi / 128, 20 columns, float32: 45 us (a lane per column, an edge at a time: 120).
+template <typename T, int V>
 __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict__ weights, const int64_t* __restrict__ row_ptr,
                                  int64_t n_targets, int d_out, T* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
+  struct alignas(V * sizeof(T)) Vec { T x[V]; };
+  const int lane = threadIdx.x & 31, vectors = d_out / V;
   const int64_t x = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (x >= n_targets) return;
   const int64_t i = from_both_ends(x, n_targets);
   const int64_t e0 = row_ptr[i], e1 = row_ptr[i + 1];
-  for (int c = lane; c < d_out; c += 32) {
-    T acc = T(0);
-    for (int64_t e = e0; e < e1; ++e) acc += weights[e] * rows[e * d_out + c];
-    out[i * d_out + c] = acc;
+  for (int q0 = 0; q0 < vectors; q0 += 32) {
+    const int width = min(32, vectors - q0), slots = 32 / width, slot = lane / width, c = V * (q0 + lane % width);
+    T acc[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) acc[v] = T(0);
+    if (slot < slots) {
+#pragma unroll 4
+      for (int64_t e = e0 + slot; e < e1; e += slots) {
+        const T w = weights[e];
+        const Vec row = *reinterpret_cast<const Vec*>(rows + e * d_out + c);
+#pragma unroll
+        for (int v = 0; v < V; ++v) acc[v] += w * row.x[v];
+      }
+    }
+    for (int s = 1; s < slots; ++s) {
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const T other = __shfl_sync(0xffffffffu, acc[v], (lane + s * width) & 31);
+        if (slot == 0) acc[v] += other;
+      }
+    }
+    if (slot == 0) {
+      Vec sum;
+#pragma unroll
+      for (int v = 0; v < V; ++v) sum.x[v] = acc[v];
+      *reinterpret_cast<Vec*>(out + i * d_out + c) = sum;
+    }
   }
 }
 
@@ -649,10 +675,15 @@ extern "C" int gm_factored_aggregate(const void* rows, const void* weights, cons
   if (n_targets == 0) return GM_OK;
   GM_REQUIRE(row_ptr && out && (n_edges == 0 || (rows && weights)), GM_ERR_ARGUMENT, "gm_factored_aggregate: null pointer");
   const unsigned blocks = (unsigned)((n_targets + 7) / 8);
-  if (dtype == GM_F32)
-    aggregate_kernel<float><<<blocks, 256, 0, (cudaStream_t)stream>>>((const float*)rows, (const float*)weights, row_ptr, n_targets, d_out, (float*)out);
-  else
-    aggregate_kernel<double><<<blocks, 256, 0, (cudaStream_t)stream>>>((const double*)rows, (const double*)weights, row_ptr, n_targets, d_out, (double*)out);
+  auto run = [&](auto tag) {
+    using T = decltype(tag);
+    constexpr int V = 16 / sizeof(T);
+    auto go = [&](auto kernel) { kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const T*)rows, (const T*)weights, row_ptr, n_targets, d_out, (T*)out); };
+    if (d_out % V == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) go(aggregate_kernel<T, V>);
+    else go(aggregate_kernel<T, 1>);
+  };
+  if (dtype == GM_F32) run(float());
+  else run(double());
   return launch_status("gm_factored_aggregate");
 }
 

@@ -1043,3 +1043,25 @@ def test_node_products_against_float64(case, dtype, aligned):
     for name, got, ref, scale, n in zip(("zc", "zr", "dx", "dcw", "dcb", "drw", "drb"), (zc, zr, *grads), want, size, terms):
         excess = (got.cpu().double() - ref).abs() - (2 * n + 2) * unit * scale
         assert got.shape == ref.shape and excess.max() <= 0, (name, float(excess.max()))
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("d_out", [1, 2, 5, 20, 33, 64, 127, 128])
+def test_aggregate_widths(d_out, dtype, offset):
+    """A target's weighted sum of its rows (0 to 300 of them) against float64: a sum of ``n`` products errs by at most ``n + 1``
+    roundings of the sum of their magnitudes.  ``offset`` 1: rows that do not start on a 16-byte boundary."""
+    from gm_attention_b200.nn import fused_factored as ff
+
+    degrees = torch.tensor([0, 1, 300, 2, 7, 33, 0, 64, 15, 128])
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.int64), degrees.cumsum(0)])
+    n_edges = int(row_ptr[-1])
+    gen = torch.Generator().manual_seed(d_out)
+    rows = torch.randn(n_edges * d_out + offset, generator=gen, dtype=torch.float64).to(dtype).cuda()[offset:].view(n_edges, d_out)
+    weights = torch.randn(n_edges, generator=gen, dtype=torch.float64).to(dtype).cuda()
+    got = ff.extension(True).aggregate(rows, weights, row_ptr.cuda()).cpu().double()
+    terms = weights.cpu().double()[:, None] * rows.cpu().double()
+    target = torch.repeat_interleave(torch.arange(len(degrees)), degrees)
+    want = torch.zeros(len(degrees), d_out, dtype=torch.float64).index_add(0, target, terms)
+    size = torch.zeros_like(want).index_add(0, target, terms.abs())
+    assert ((got - want).abs() <= (degrees[:, None] + 1) * torch.finfo(dtype).eps * size).all()
