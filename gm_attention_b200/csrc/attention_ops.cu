@@ -504,12 +504,28 @@ __global__ void __launch_bounds__(128) softmax_backward_kernel(const __grid_cons
   ScoreItem* items_s = reinterpret_cast<ScoreItem*>(smem_raw);
   int n_items = 0, n_real = 0;
   uintptr_t bits = bits_of(a.q) | bits_of(a.k) | bits_of(a.transport) | bits_of(a.dq) | (uintptr_t)a.D * sizeof(T);
-  for (int f = 0; f < a.F; ++f) {
+  auto list = [&](int f, int at) {  // the items of row f from `at` on; their number
     const int n = (int)a.desc[f * DESC], a_n = (int)a.desc[f * DESC + 1], off = (int)a.desc[f * DESC + 2], dim = (int)a.desc[f * DESC + 4];
-    for (int x = threadIdx.x; x < a.H * a_n; x += blockDim.x) items_s[n_items + x] = ScoreItem{off + dim * x, n, x / a_n, 0};
-    n_items += a.H * a_n;
-    if (n == 0) n_real = n_items;  // items are in column order: the scalar block first
-    else bits |= (uintptr_t)off * sizeof(T);
+    for (int x = threadIdx.x; x < a.H * a_n; x += blockDim.x) items_s[at + x] = ScoreItem{off + dim * x, n, x / a_n, 0};
+    if (n != 0) bits |= (uintptr_t)off * sizeof(T);
+    return a.H * a_n;
+  };
+  bool behind = false;  // scalar items behind others
+  for (int f = 0; f < a.F; ++f) {
+    const int count = list(f, n_items);
+    if (a.desc[f * DESC] == 0) {
+      behind = behind || n_real != n_items;
+      n_real += count;
+    }
+    n_items += count;
+  }
+  if (behind) {  // the walk wants them in front (two passes over the descriptor for everyone: 6 us of 780)
+    __syncthreads();
+    int scalar = 0, other = n_real;
+    for (int f = 0; f < a.F; ++f) {
+      int& at = a.desc[f * DESC] == 0 ? scalar : other;
+      at += list(f, at);
+    }
   }
   __syncthreads();
   const bool vec = whole_pairs<T>(bits);

@@ -110,7 +110,9 @@ def test_conv_forward_backward(ext, reference_modules, case, dtype):
     ({0: 5, 1: 6, 2: 5}, 8),   # a second round of copies, pairs at even offsets
     ({0: 16, 1: 15, 2: 16, 3: 13}, 8),  # four rounds
     ({1: 17, 2: 3}, 2),        # no scalars
-    ({1: 3, 0: 5}, 2),         # the scalars behind others (scores, forward)
+    ({1: 3, 0: 5}, 2),         # the scalars behind others (scores)
+    ({2: 17, 0: 9, 1: 20}, 2),  # ... and between others: 34 and 40 complex items, 18 scalar ones
+    ({3: 2, 2: 1, 0: 3, 1: 4, 4: 1}, 4),  # five rows
 ])
 def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
     """Neighbourhoods of 0 to 130 edges -- fewer than the groups, one more than they take at a time, many turns -- against the oracle
@@ -146,8 +148,6 @@ def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
     alpha = O.softmax_forward(*wide(q, k, transport, bias), inside, desc, row_ptr, source, heads, 0.3)
     tables = [cuda(x) for x in (transport, bias, inside, desc, row_ptr, source)]
     compare([ext.softmax_forward(cuda(q), cuda(k), *tables, heads, 0.3, 130)], [alpha], ["alpha"])
-    if list(types) != sorted(types):
-        return
     want = O.softmax_backward(*wide(da, q, k, transport), desc, row_ptr, source, alpha, heads, 0.3)
     for largest in (130, 1):  # uneven neighbourhoods, and as if all were alike
         compare(ext.softmax_backward(cuda(da), cuda(q), cuda(k), *tables, cuda(alpha.astype(dtype)), heads, 0.3, largest), want, ["dq", "dk"])
