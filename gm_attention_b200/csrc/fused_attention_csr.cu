@@ -308,7 +308,8 @@ __global__ void __launch_bounds__(256, FORM == 1 && sizeof(S) <= 4 ? (NS <= 3 ? 
     }
   }
   for (int o = at.L >> 1; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
-  const C lse = a.lse_in[(base + i) * a.H + at.h];
+  C lse = a.lse_in[(base + i) * a.H + at.h];
+  if (lse == neg_inf<C>()) lse = -lse;  // no edge counted: p = 0 for all of them
   const int64_t e0 = a.row_ptr[i];
   const int degree = (int)(a.row_ptr[i + 1] - e0);
   const int64_t* source = a.source + e0;

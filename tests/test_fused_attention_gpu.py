@@ -176,3 +176,43 @@ def test_lane_groups_share_edges(graph, dtype):
     assert_close(out.cpu().numpy(), want, rtol, atol * max(1.0, np.abs(want).max()), "out")
     for name, got, ref in zip(("dq", "dk", "dv"), attention_backward(G, Q, K, V, out, lse, t), grads):
         assert_close(got.cpu().numpy(), ref, rtol, 10 * atol * max(1.0, np.abs(ref).max()), name)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("graph", GRAPHS)
+def test_targets_whose_edges_all_count_nothing(graph, dtype):
+    """A target all of whose edges in the window have bias minus infinity is one without edges: zeros forward, zeros backward, and
+    its neighbours' gradients are those of the other targets.  Tolerances as above."""
+    from gm_attention_b200.attention import AttentionTables, attention_backward, attention_forward
+
+    heads, rows, width, degree = graph
+    n_nodes, batch = 29, 2
+    rng = np.random.default_rng(6)
+    counts = rng.integers(1, 2 * degree + 1, n_nodes)
+    row_ptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    n_edges, orders = int(row_ptr[-1]), 1 + max(n for n, _, _ in rows)
+    desc = np.array([(n, copies, offset, 0, 1 if n == 0 else 2) for n, copies, offset in rows], dtype=np.int64)
+    source = rng.integers(0, n_nodes, n_edges)
+    angle = rng.uniform(-np.pi, np.pi, (n_edges, 1)) * np.arange(orders)
+    transport = np.stack([np.cos(angle), np.sin(angle)], -1).astype(dtype)
+    bias = rng.standard_normal(n_edges).astype(dtype)
+    inside = (rng.random(n_edges) < 0.8).astype(np.uint8)
+    inside[row_ptr[:-1]] = 1
+    silent = np.repeat(np.arange(n_nodes) % 3 == 0, counts)
+    q, k, v, g = seeded((batch * n_nodes, width), 17, dtype, 4)
+    # what the oracle sees: the other targets' edges
+    ptr = np.concatenate([[0], np.cumsum(np.where(np.arange(n_nodes) % 3 == 0, 0, counts))]).astype(np.int64)
+    args = (transport[~silent], bias[~silent], inside[~silent], desc, ptr, source[~silent], heads, 0.3, batch)
+    want = O.attention_forward(q, k, v, *args)
+    grads = O.attention_backward(g, q, k, v, *args)
+    bias = np.where(silent, dtype(-np.inf), bias)
+    t = AttentionTables(cuda(transport), cuda(bias), cuda(inside), cuda(row_ptr), cuda(source), tuple(map(tuple, desc.tolist())), heads, 0.3)
+    Q, K, V, G = map(cuda, (q, k, v, g))
+    out, lse = attention_forward(Q, K, V, t)
+    dq, dk, dv = attention_backward(G, Q, K, V, out, lse, t)
+    nothing = torch.arange(batch * n_nodes, device="cuda") % n_nodes % 3 == 0
+    assert not out[nothing].any() and not dq[nothing].any() and bool((lse[nothing] == -np.inf).all())
+    rtol, atol = (1e-10, 1e-11) if dtype == np.float64 else (1e-5, 1e-6)
+    assert_close(out.cpu().numpy(), want, rtol, atol * max(1.0, np.abs(want).max()), "out")
+    for name, got, ref in zip(("dq", "dk", "dv"), (dq, dk, dv), grads):
+        assert_close(got.cpu().numpy(), ref, rtol, 10 * atol * max(1.0, np.abs(ref).max()), name)
