@@ -595,8 +595,13 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
         }
         if (warp == warps - 1 && base == 0 && a.dweights) {  // dweights_e = <g_i, row_e>, two lanes per edge
           const float* row = rows + (lane >> 1) * rec.pitch;
-          float s = 0.f;
-          for (int x = lane & 1; x < a.d_out; x += 2) s = fmaf(row[rec.grad + x], row[rec.row + x], s);
+          float part[4] = {0.f, 0.f, 0.f, 0.f};  // every eighth column: the sums, and their order, of the CUDA-core kernel's eight lanes
+          for (int x = lane & 1; x < a.d_out; x += 8) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v)
+              if (x + 2 * v < a.d_out) part[v] = fmaf(row[rec.grad + x + 2 * v], row[rec.row + x + 2 * v], part[v]);
+          }
+          float s = (part[0] + part[2]) + (part[1] + part[3]);
           s += __shfl_xor_sync(0xffffffffu, s, 1);
           if ((lane & 1) == 0 && lane / 2 < n_rows) a.dweights[edge_s[(step & 3) * ROWS + lane / 2]] = s;
         }

@@ -237,6 +237,65 @@ def test_factored_tensor_cores_against_float64(type_in, type_out, k, degrees, sc
         assert a.shape == b.shape and (b.numel() == 0 or float((a.double() - b).norm() / b.norm()) < 2e-6), x
 
 
+def both_factored_kernels(type_in, type_out, k, degrees, scales, spoil=lambda **fields: None, dtypes=(np.float32,)):
+    """Rows, plain gradients and (no ``scales``) aggregated ones by the kernels that sources of many edges take in float32 and by
+    the others, which a grouping with as many empty runs of further nodes as make the mean run short sends the same edges to.
+    ``spoil`` may change the numbers before.  Per dtype a pair of dicts of tensors, rows of edges or of the nodes with edges first."""
+    from gm_attention_b200.fields import FieldType
+    from gm_attention_b200.nn import fused_factored as ff
+
+    blocks, powers = blocks_for(type_in, type_out)
+    p = ff.plan_blocks(blocks, FieldType(type_out), powers)
+    n_f, n, e = 8, len(degrees), sum(degrees)
+    more = e // 24 + 1
+    rng = np.random.default_rng(15)
+    source = rng.permutation(np.repeat(np.arange(n), degrees))
+    phase = np.exp(1j * rng.uniform(0, 6.28, (2, e, n_f)))
+    desc = np.array([b.row() for b in p.blocks], np.int32).reshape(-1, 8)
+    if scales:
+        desc[:, 5] %= scales
+    fields = dict(h=rng.standard_normal((e, k - 1)), zc=rng.standard_normal((n + more, k, p.wc, 2)), zr=rng.standard_normal((n + more, k, p.wr)),
+                  angular=np.stack([phase[0].real, phase[0].imag], -1), transport=np.stack([phase[1].real, phase[1].imag], -1),
+                  rho=rng.uniform(0.1, 1.0, (e, scales) if scales else e))
+    upstream = dict(g=rng.standard_normal((e, p.d_out)), gt=rng.standard_normal((5, p.d_out)), weights=rng.uniform(0.1, 0.5, e))
+    fields, upstream = ({name: x.astype(np.float32) for name, x in d.items()} for d in (fields, upstream))
+    targets = np.sort(rng.integers(0, 5, e))
+    spoil(source=source, targets=targets, **fields, **upstream)
+    order, ptr, nodes = [x.cuda() for x in ff.source_groups(torch.from_numpy(source))]
+    long = (order, torch.cat([ptr, ptr[-1:].expand(more)]), torch.cat([nodes, torch.arange(n, n + more, device="cuda")]))
+    ext, results = ff.extension(True), []
+    for dtype in dtypes:
+        args = (*(cuda(x.astype(dtype)) for x in fields.values()), cuda(desc), cuda(source))
+        g, gt, weights = (cuda(x.astype(dtype)) for x in upstream.values())
+        pair = []
+        for groups in ((order, ptr, nodes), long):
+            rows = ext.forward(*args, *groups, p.d_out, p.max_bm, bool(scales))
+            got = dict(rows=rows, **dict(zip(("dh", "dzc", "dzr"), ext.backward(g, *args, *groups, bool(scales)))))
+            if not scales:
+                # (the same forward rows for both)
+                shared = pair[0]["rows"] if pair else rows
+                got |= dict(zip(("dh_t", "dzc_t", "dzr_t", "dw_t"), ext.backward_aggregated(gt, cuda(targets), weights, shared, *args, *groups)))
+            pair.append({name: x[: n if "z" in name else e] for name, x in got.items() if x.numel()})
+        results.append(pair)
+    return results
+
+
+FACTORED_TENSOR_CORES = [
+    ({0: 8, 1: 8, 2: 8}, {0: 4, 1: 4, 2: 4}, 17, [92, 16, 0, 129, 17, 47]),
+    ({0: 2, 1: 2}, {0: 4, 1: 4}, 2, [64, 100]),
+    ({0: 2, 1: 2}, {0: 3, 1: 9}, 16, [64, 65, 63, 300]),  # two rounds of tiles forward
+    ({1: 3}, {0: 5, 2: 5}, 6, [130, 200]),
+    ({0: 2, 1: 2, 2: 2}, {0: 25, 1: 25, 2: 25}, 11, [90, 33]),  # three rounds backward
+]
+
+
+@pytest.mark.parametrize("case", FACTORED_TENSOR_CORES)
+def test_factored_weights_gradients_are_the_same_sums(case):
+    """An edge's ``<g, row>`` has no matrix product in it: the tensor-core kernel adds it up as the other does."""
+    (tensor_cores, others), = both_factored_kernels(*case, 0)
+    assert torch.equal(tensor_cores["dw_t"], others["dw_t"])
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_factored_sources_without_edges(dtype):
     """A grouping that lists every node, most of them with an empty run between two full ones (more runs than the forward
