@@ -9,7 +9,8 @@
 // the block factors, and the sum over the blocks of one output, are applied to the accumulators in registers.  A real block is a
 // complex one whose imaginary columns are zero.
 //
-// Precision: every float32 operand is the sum of three bfloat16 (8 + 8 + 8 bits: exact), and of the nine products the six that
+// Precision: every float32 operand is the sum of three bfloat16 (8 + 8 + 8 bits: exact from 2^-110 on, below with an error of up to
+// 2^-134), and of the nine products the six that
 // reach 2^-24 of the result are taken, in two chains of three, smallest first; everything that is summed over more than one
 // k-step (the 16 edges of dZ, the two tiles of dh) is added in float32, rounded to nearest.
 // What it measured, 128 x 256, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4}, trunk 16, us on CUDA cores -> here: forward 1 036 -> 734,
@@ -19,7 +20,11 @@
 // eight 2 095 us (the loop over tiles, unrolled for its accumulators, outgrew the instruction cache), two 1 946.  168 registers
 // and twelve warps an SM instead of sixteen: 2 077.  Errors against float64 over the sizes it serves: 0.6 to 1.0 of the CUDA-core
 // kernels' for rows and columns, the same for the trunk's parameters (0.5 to 1.4, sums over every edge by the library).
-// An operand that is infinite makes NaN here where a plain product might stay infinite: in the same places, no others.
+// Infinities and numbers of 2^60 and more do not go through the splits: what they are operands of is formed by single
+// multiply-adds (a step of the forward, a source of the backward), so that infinite and finite results are those of the
+// CUDA-core kernel; NaN spreads as it would there.  128 x 256, 13 blocks to {4, 4, 4}: the test for them takes 1 % of the backward; an
+// infinity in one polar node's Z makes the forward 731 -> 1 042, in one row of the gradient the backward 1 838 -> 3 572, and
+// nothing but infinities 3 400 and 10 807 (CUDA-core kernels 1 040 and 2 470).
 #include <algorithm>
 
 #include "factored.cuh"
@@ -84,6 +89,15 @@ __device__ __forceinline__ void split3(float x, float y, unsigned (&w)[3]) {
     y -= __uint_as_float(w[s] & 0xffff0000u);
   }
 }
+// Operands of 2^60 and more, infinities among them, go to single multiply-adds: of smaller ones no product and no sum here
+// overflows, where parts of opposite signs could make a NaN of an infinity.  (NaN goes where it would go there.)
+// The larger magnitudes of two pairs of bfloat16, under whatever sign, NaN left out
+__device__ __forceinline__ unsigned larger(unsigned x, unsigned y) {
+  unsigned m;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(m) : "r"(x), "r"(y));
+  return m;
+}
+__device__ __forceinline__ bool too_large(unsigned m) { return fmaxf(fabsf(__uint_as_float(m << 16)), fabsf(__uint_as_float(m & 0xffff0000u))) >= 0x1p60f; }
 __device__ __forceinline__ unsigned transposed(unsigned x) {  // of an 8 x 8 matrix of bfloat16, a row's pairs over four lanes
   unsigned y;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
@@ -223,8 +237,8 @@ __device__ __forceinline__ float2 record_factor(const float* rec, const Factor& 
     for (int x = 0; x < f.power; ++x) s *= rho;
   return make_float2(s * (p.x * t.x - pi * ti), s * (p.x * ti + pi * t.x));
 }
-// The trunk's outputs of two edges (their records) as the A operand of 16 edges x 16 outputs
-__device__ __forceinline__ void load_trunk(const float* r0, const float* r1, int n, int c, unsigned (&h)[3][4]) {
+// The trunk's outputs of two edges (their records) as the A operand of 16 edges x 16 outputs; returned: their largest magnitudes
+__device__ __forceinline__ unsigned load_trunk(const float* r0, const float* r1, int n, int c, unsigned (&h)[3][4]) {
 #pragma unroll
   for (int x = 0; x < 4; ++x) {
     const int t = 2 * c + 8 * (x >> 1);
@@ -236,6 +250,7 @@ __device__ __forceinline__ void load_trunk(const float* r0, const float* r1, int
 #pragma unroll
     for (int p = 0; p < 3; ++p) h[p][x] = w[p];
   }
+  return larger(larger(h[0][0], h[0][1]), larger(h[0][2], h[0][3]));
 }
 
 // Shared memory of the forward
@@ -254,8 +269,70 @@ struct ForwardPlan {
   }
 };
 
+// The columns of two edges that a lane's copy c of a tile belongs to: written, or (add) added to
+__device__ __forceinline__ void write_columns(const Tile& tile, int c, float* out0, float* out1, bool in0, bool in1, bool add, float2 y0, float2 y1) {
+  if (c >= tile.flags >> 8) return;
+  const bool real = tile.flags & TILE_REAL_OUT;
+  const int col = tile.output + (real ? c : 2 * c);
+  if (add) {
+    if (in0) y0.x += out0[col];
+    if (in1) y1.x += out1[col];
+    if (!real && in0) y0.y += out0[col + 1];
+    if (!real && in1) y1.y += out1[col + 1];
+  }
+  if (in0) out0[col] = y0.x;
+  if (in1) out1[col] = y1.x;
+  if (!real) {
+    if (in0) out0[col + 1] = y0.y;
+    if (in1) out1[col + 1] = y1.y;
+  }
+}
+
+// A step of the forward where an operand is too large: by single multiply-adds, from the records and the node's own
+// numbers.  (Not inlined: few steps come here.)
+__device__ __noinline__ void forward_step_by_products(const FArgs<float>* args, int64_t j, const Tile* tile_s, int n_tiles, bool later_round, const float* row0,
+                                                    const float* row1, const float2* f_at, int c, float* out0, float* out1, bool in0, bool in1) {
+  const FArgs<float>& a = *args;
+  const float *zc = a.zc + j * a.k * 2 * a.wc, *zr = a.zr + j * a.k * a.wr;
+  float2 y0 = make_float2(0.f, 0.f), y1 = y0;
+  bool continued = later_round && !(tile_s[0].flags & TILE_FIRST);
+#pragma unroll 1
+  for (int x = 0; x < n_tiles; ++x) {
+    const Tile tile = tile_s[x];
+    if (c < (tile.flags & 7)) {
+      const bool real = tile.flags & TILE_REAL;
+      float2 u0 = make_float2(0.f, 0.f), u1 = u0;
+#pragma unroll 2
+      for (int t = 0; t < a.k; ++t) {
+        const float h0 = t ? row0[t - 1] : 1.f, h1 = t ? row1[t - 1] : 1.f;
+        const float* z = real ? zr + t * a.wr + tile.column + c : zc + 2 * (t * a.wc + tile.column + c);
+        u0.x = fmaf(h0, z[0], u0.x);
+        u1.x = fmaf(h1, z[0], u1.x);
+        if (real) continue;
+        u0.y = fmaf(h0, z[1], u0.y);
+        u1.y = fmaf(h1, z[1], u1.y);
+      }
+      if (real) {
+        y0.x += u0.x;
+        y1.x += u1.x;
+      } else {
+        const float2 f0 = f_at[tile.block * ROWS], f1 = f_at[tile.block * ROWS + 8];
+        y0.x = fmaf(-f0.y, u0.y, fmaf(f0.x, u0.x, y0.x));
+        y0.y = fmaf(f0.y, u0.x, fmaf(f0.x, u0.y, y0.y));
+        y1.x = fmaf(-f1.y, u1.y, fmaf(f1.x, u1.x, y1.x));
+        y1.y = fmaf(f1.y, u1.x, fmaf(f1.x, u1.y, y1.y));
+      }
+    }
+    if ((tile.flags & TILE_LAST) || x + 1 == n_tiles) {
+      write_columns(tile, c, out0, out1, in0, in1, continued, y0, y1);
+      continued = false;
+      y0 = y1 = make_float2(0.f, 0.f);
+    }
+  }
+}
+
 template <bool SCALED>
-__global__ void __launch_bounds__(32 * FWD_WARPS) factored_forward_tc_kernel(const __grid_constant__ FArgs<float> a, int tiles) {
+__global__ void __launch_bounds__(32 * FWD_WARPS, 10) factored_forward_tc_kernel(const __grid_constant__ FArgs<float> a, int tiles) {
   extern __shared__ __align__(16) unsigned char raw[];
   const int n_rho = SCALED ? a.n_scales : 1;
   const Record rec(a.k, a.n_f, n_rho, a.d_out, false);
@@ -298,6 +375,7 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) factored_forward_tc_kernel(con
       auto edge = [&](int64_t x) { return (unsigned)a.order[min(x + (lane & 15), last - 1)]; };
       unsigned e = x0 < last ? edge(x0) : 0, e_next = x0 + ROWS * FWD_WARPS < last ? edge(x0 + ROWS * FWD_WARPS) : 0;
       __syncthreads();
+      unsigned largest = 0;
       {  // lane (column n, outputs 2 c, 2 c + 1 (+ 8 for the second warp)) of every tile
         const int n = lane >> 2, t = 1 + 2 * (lane & 3) + 8 * warp;
         const bool in0 = t < a.k, in1 = t + 1 < a.k;
@@ -312,6 +390,7 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) factored_forward_tc_kernel(con
           if (in && in1) v1 = __ldg(z + (real ? a.wr : 2 * a.wc));
           unsigned w[3];
           split3(v0, v1, w);
+          largest = larger(largest, w[0]);
 #pragma unroll
           for (int p = 0; p < 3; ++p) reinterpret_cast<unsigned*>(z_s)[2 * ((x * 3 + p) * 32 + lane) + warp] = w[p];
         }
@@ -327,7 +406,7 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) factored_forward_tc_kernel(con
         reinterpret_cast<float*>(z0_s)[x] = v;
       }
       if (x0 < last) stage(rec_s, e);
-      __syncthreads();
+      const bool large_node = __syncthreads_or(too_large(largest));
       for (int buf = 0; x0 < last; x0 += ROWS * FWD_WARPS, buf ^= 1) {
         const int n_rows = (int)min((int64_t)ROWS, last - x0);
         copy_wait();
@@ -344,12 +423,15 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) factored_forward_tc_kernel(con
           for (int b = lane >> 4; b < a.n_blocks; b += 2) f_s[b * ROWS + (lane & 15)] = record_factor<SCALED>(row, place_s[b], rho);
         }
         unsigned h[3][4];
-        load_trunk(rows + g * rec.pitch, rows + (g + 8) * rec.pitch, a.k - 1, c, h);
-        __syncwarp();
+        const bool large = __any_sync(0xffffffffu, too_large(load_trunk(rows + g * rec.pitch, rows + (g + 8) * rec.pitch, a.k - 1, c, h)) || large_node);
         const bool in0 = g < n_rows, in1 = g + 8 < n_rows;
         float *out0 = a.out + (size_t)e0 * a.d_out, *out1 = a.out + (size_t)e1 * a.d_out;
+        if (large) {
+          forward_step_by_products(&a, j, tile_s, n_tiles, base > 0, rows + g * rec.pitch, rows + (g + 8) * rec.pitch, f_s + g, c, out0, out1, in0, in1);
+          continue;
+        }
         float2 y0 = make_float2(0.f, 0.f), y1 = y0;
-        bool continued = !(tile_s[0].flags & TILE_FIRST);  // a later round's first columns: the sum goes on
+        bool continued = base > 0 && !(tile_s[0].flags & TILE_FIRST);  // a later round's first columns: the sum goes on
         const uint2* z_at = z_s + lane;
         const float2 *z0_at = z0_s + c, *f_at = f_s + g;
 #pragma unroll 2
@@ -367,22 +449,7 @@ __global__ void __launch_bounds__(32 * FWD_WARPS) factored_forward_tc_kernel(con
           y1.x = fmaf(f1.x, u1.x, fmaf(-f1.y, u1.y, y1.x));
           y1.y = fmaf(f1.x, u1.y, fmaf(f1.y, u1.x, y1.y));
           if ((tile.flags & TILE_LAST) || x + 1 == n_tiles) {
-            if (c < (tile.flags >> 8)) {
-              const bool real = tile.flags & TILE_REAL_OUT;
-              const int col = tile.output + (real ? c : 2 * c);
-              if (base > 0 && continued) {
-                if (in0) y0.x += out0[col];
-                if (in1) y1.x += out1[col];
-                if (!real && in0) y0.y += out0[col + 1];
-                if (!real && in1) y1.y += out1[col + 1];
-              }
-              if (in0) out0[col] = y0.x;
-              if (in1) out1[col] = y1.x;
-              if (!real) {
-                if (in0) out0[col + 1] = y0.y;
-                if (in1) out1[col + 1] = y1.y;
-              }
-            }
+            write_columns(tile, c, out0, out1, in0, in1, continued, y0, y1);
             continued = false;
             y0 = y1 = make_float2(0.f, 0.f);
           }
@@ -408,6 +475,84 @@ struct BackwardPlan {
     total = desc + (size_t)n_blocks * FDESC * sizeof(int32_t);
   }
 };
+
+// A source of the backward where an operand is too large: dZ of this round's tiles and dh as it is after this round, again by single
+// multiply-adds.  W of 16 edges and of a round's columns takes the place of Z's fragments.  (Not inlined.)
+constexpr int W_PITCH = ROWS + 1;
+static_assert(4 * W_PITCH * sizeof(float2) <= 3 * 32 * sizeof(uint2), "a tile's W fits where its fragments were");
+template <bool SCALED>
+__device__ __noinline__ void backward_source_by_products(const FArgs<float>* args, int64_t j, int64_t first, int64_t last, int base, int capacity, const int32_t* desc_s,
+                                                       Tile* tile_s, float2* w_s, float* h_s, unsigned* edge_s) {
+  const FArgs<float>& a = *args;
+  const int threads = blockDim.x, n_trunk = a.k - 1;
+  for (int b0 = 0; b0 <= base; b0 += capacity) {
+    __syncthreads();
+    const int n_tiles = min(list_tiles(desc_s, a.n_blocks, b0, capacity, tile_s) - b0, capacity), columns = 4 * n_tiles;
+    for (int64_t x0 = first; x0 < last; x0 += ROWS) {
+      const int n = (int)min((int64_t)ROWS, last - x0);
+      __syncthreads();
+      if (threadIdx.x < ROWS) edge_s[threadIdx.x] = (unsigned)a.order[min(x0 + threadIdx.x, last - 1)];
+      __syncthreads();
+      for (int i = threadIdx.x; i < ROWS * n_trunk; i += threads) h_s[i / n_trunk * DH_PITCH + i % n_trunk] = a.h[(size_t)edge_s[i / n_trunk] * n_trunk + i % n_trunk];
+      for (int i = threadIdx.x; i < columns * ROWS; i += threads) {
+        const Tile tile = tile_s[i / (4 * ROWS)];
+        const int c = i / ROWS & 3, r = i % ROWS;
+        float2 w = make_float2(0.f, 0.f);
+        if (c < (tile.flags & 7) && r < n) {
+          const int64_t e = edge_s[r];
+          const float weight = a.weights ? a.weights[e] : 1.f, *g = a.g + (a.target ? a.target[e] : e) * a.d_out + tile.output;
+          if (tile.flags & TILE_REAL) {
+            w.x = weight * g[c];
+          } else {
+            float fr, fi;
+            table_factor<SCALED>(a, e, desc_s + tile.block * FDESC, fr, fi);
+            const bool real = tile.flags & TILE_REAL_OUT;
+            const float gr = weight * g[real ? c : 2 * c], gi = real ? 0.f : weight * g[2 * c + 1];
+            w = make_float2(gr * fr + gi * fi, gi * fr - gr * fi);
+          }
+        }
+        w_s[i / ROWS * W_PITCH + r] = w;
+      }
+      __syncthreads();
+      for (int i = threadIdx.x; i < ROWS * n_trunk; i += threads) {  // dh
+        const int r = i % ROWS, t = 1 + i / ROWS;
+        if (r >= n) continue;
+        float* to = a.dh + (size_t)edge_s[r] * n_trunk + t - 1;
+        float s = b0 ? *to : 0.f;
+        for (int x = 0; x < n_tiles; ++x) {
+          const Tile tile = tile_s[x];
+          const bool real = tile.flags & TILE_REAL;
+          const float* z = real ? a.zr + (j * a.k + t) * a.wr + tile.column : a.zc + ((j * a.k + t) * a.wc + tile.column) * 2;
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            if (c >= (tile.flags & 7)) continue;
+            const float2 w = w_s[(4 * x + c) * W_PITCH + r];
+            s = fmaf(w.x, z[real ? c : 2 * c], s);
+            if (!real) s = fmaf(w.y, z[2 * c + 1], s);
+          }
+        }
+        *to = s;
+      }
+      for (int i = threadIdx.x; i < a.k * columns; i += threads) {  // dZ; a thread keeps its entries
+        const int t = i / columns, x = i % columns, c = x & 3;
+        const Tile tile = tile_s[x / 4];
+        if (c >= (tile.flags & 7)) continue;
+        const bool real = tile.flags & TILE_REAL;
+        float* to = real ? a.dzr + (j * a.k + t) * a.wr + tile.column + c : a.dzc + ((j * a.k + t) * a.wc + tile.column + c) * 2;
+        float2 s = x0 == first ? make_float2(0.f, 0.f) : make_float2(to[0], real ? 0.f : to[1]);
+#pragma unroll 4
+        for (int r = 0; r < n; ++r) {
+          const float h = t ? h_s[r * DH_PITCH + t - 1] : 1.f;
+          const float2 w = w_s[x * W_PITCH + r];
+          s.x = fmaf(h, w.x, s.x);
+          s.y = fmaf(h, w.y, s.y);
+        }
+        to[0] = s.x;
+        if (!real) to[1] = s.y;
+      }
+    }
+  }
+}
 
 template <bool SCALED>
 __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel(const __grid_constant__ FArgs<float> a) {
@@ -473,6 +618,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
         if (steps > 1) put_edges(1, edge(1));
         if (steps > 2) e_ahead = edge(2);
       }
+      unsigned largest = 0;
       {  // lane (output 8 half + g, columns of copy c of tile 2 pair + r)
         const int n_items = (n_tiles + 1) / 2 * 4;  // (pair, half, r)
 #pragma unroll 4
@@ -481,8 +627,10 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
           const Tile tile = at < n_tiles ? tile_s[at] : Tile{0, 0, 0, 0};
           const bool real = tile.flags & TILE_REAL, in = t < a.k && c < (tile.flags & 7);
           const float* z = real ? a.zr + (j * a.k + t) * a.wr + tile.column + c : a.zc + ((j * a.k + t) * a.wc + tile.column + c) * 2;
+          const float re = in ? __ldg(z) : 0.f, im = in && !real ? __ldg(z + 1) : 0.f;
           unsigned w[3];
-          split3(in ? __ldg(z) : 0.f, in && !real ? __ldg(z + 1) : 0.f, w);
+          split3(re, im, w);
+          largest = larger(largest, w[0]);
 #pragma unroll
           for (int p = 0; p < 3; ++p) reinterpret_cast<unsigned*>(z_s)[2 * (((pair * 2 + half) * 3 + p) * 32 + lane) + r] = w[p];
         }
@@ -535,7 +683,8 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
         unsigned ht[3][4];  // the trunk's outputs as 16 outputs x 16 edges
         {
           unsigned h[3][4];
-          load_trunk(rows + g * rec.pitch, rows + (g + 8) * rec.pitch, a.k - 1, c, h);
+          const unsigned most = load_trunk(rows + g * rec.pitch, rows + (g + 8) * rec.pitch, a.k - 1, c, h);
+          largest = larger(largest, most);
 #pragma unroll
           for (int p = 0; p < 3; ++p) {
             ht[p][0] = transposed(in0 ? h[p][0] : 0u);
@@ -571,6 +720,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
             unsigned s0[3], s1[3];
             split3(w0.x, w0.y, s0);
             split3(w1.x, w1.y, s1);
+            largest = larger(largest, larger(s0[0], s1[0]));
             uint2 wt[3];  // 16 edges x 8 columns as a B operand
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
@@ -596,6 +746,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
         if (warp == warps - 1 && base == 0 && a.dweights) {  // dweights_e = <g_i, row_e>, two lanes per edge
           const float* row = rows + (lane >> 1) * rec.pitch;
           float part[4] = {0.f, 0.f, 0.f, 0.f};  // every eighth column: the sums, and their order, of the CUDA-core kernel's eight lanes
+#pragma unroll 1
           for (int x = lane & 1; x < a.d_out; x += 8) {
 #pragma unroll
             for (int v = 0; v < 4; ++v)
@@ -612,7 +763,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
           *reinterpret_cast<float2*>(mine_s + (g + 8) * DH_PITCH + 8 * half + 2 * c) = unpack2(dh[half][1]);
         }
       }
-      __syncthreads();
+      const bool again = __syncthreads_or(too_large(largest));
       if (steps > 0) write_dh(steps - 1);
       // ---- dZ: rows t from the accumulators, row 0 from the lanes' sums
 #pragma unroll
@@ -640,6 +791,7 @@ __global__ void __launch_bounds__(32 * MAX_WARPS, 2) factored_backward_tc_kernel
           }
         }
       }
+      if (again) backward_source_by_products<SCALED>(&a, j, first, last, base, plan.tiles, desc_s, tile_s, reinterpret_cast<float2*>(z_s), dh_s, edge_s);
     }
   }
 }

@@ -296,6 +296,47 @@ def test_factored_weights_gradients_are_the_same_sums(case):
     assert torch.equal(tensor_cores["dw_t"], others["dw_t"])
 
 
+@pytest.mark.parametrize("scales", [0, 3])
+@pytest.mark.parametrize("case", FACTORED_TENSOR_CORES)
+def test_factored_kernels_agree_on_values_no_bfloat16_holds(case, scales):
+    """Infinities, NaN and finite numbers that round to infinity in bfloat16, in every operand: the tensor-core kernels give
+    infinities, NaN and finite values where the others give them, and the latter to the rounding of sums in another order (1e-5 of a
+    row's largest value: up to 575 terms, of which one may be 1e38 times the others).  Products that overflow are among them."""
+    big = np.float32(3.4e38)  # (the largest bfloat16 is 3.39e38)
+
+    def spoil(source, targets, h, zc, zr, angular, transport, rho, g, gt, weights):
+        # hundredths, so that a product with `big` stays finite
+        for x in (h, zc, zr, g, gt):
+            x *= np.float32(0.01)
+        of = [np.flatnonzero(source == j) for j in range(int(source.max()) + 1)]
+        t = h.shape[1] - 1
+        h[of[0][3], t], h[of[0][40], 0] = np.inf, big
+        zc[1, t + 1, 0, 1], zc[1, 1, -1, 0] = -big, np.inf
+        if zr.shape[-1]:
+            zr[1, 1, 0] = big
+        h[of[1][5], 0], h[of[1][-1], t] = -big, np.nan
+        g[of[0][17], -1], g[of[0][18], 0] = -np.inf, big
+        gt[1, 0], gt[3, -1], weights[of[0][50]] = -np.inf, np.inf, big  # (no two of `big` in a product: whether that overflows hangs on the order)
+        if len(of) > 3:
+            zc[3, 0, 0, 0], zc[3, 1, 1, 0] = np.inf, big  # (the constant feature's)
+            h[of[3][-1], 0] = -np.inf
+        if len(of) > 5:
+            # overflowing sums, in the order of the trunk's outputs (rows) and of a source's edges (dZ)
+            h[of[4]] *= np.float32(1e26)
+            g[of[4]] *= np.float32(1e26)
+            h[of[5]] *= np.float32(1e26)
+            zc[5] *= np.float32(1e26)
+            zr[5] *= np.float32(1e26)
+
+    (tensor_cores, others), = both_factored_kernels(*case, scales, spoil)
+    for name, want in others.items():
+        got = tensor_cores[name]
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()), name
+        assert torch.equal(got[got.isinf()], want[got.isinf()]), name
+        a, b = (torch.where(x.isfinite(), x, 0.0).double().reshape(len(x), -1) for x in (got, want))
+        assert bool(((a - b).abs() <= 1e-5 * b.abs().amax(1, keepdim=True)).all()), name
+
+
 @pytest.mark.parametrize("dtype", [np.float32, np.float64])
 def test_factored_sources_without_edges(dtype):
     """A grouping that lists every node, most of them with an empty run between two full ones (more runs than the forward
