@@ -18,8 +18,8 @@
 // among 1 600 / 4 000 instructions, most of them the splits, the factors and the records' copies.  With the records read where
 // they are (1 245 / 3 225 us) every step waited for its chain of gathers; they are copied a step ahead.  Four tiles a backward warp:
 // eight 2 095 us (the loop over tiles, unrolled for its accumulators, outgrew the instruction cache), two 1 946.  168 registers
-// and twelve warps an SM instead of sixteen: 2 077.  Errors against float64 over the sizes it serves: 0.6 to 1.0 of the CUDA-core
-// kernels' for rows and columns, the same for the trunk's parameters (0.5 to 1.4, sums over every edge by the library).
+// and twelve warps an SM instead of sixteen: 2 077.  Errors against float64: 0.85 to 0.98 of the CUDA-core kernels' for rows
+// (shorter trunks go to those: FWD_LEAST_K), 0.2 to 0.8 for the gradients; weights' gradients are the same.
 // Infinities and numbers of 2^60 and more do not go through the splits: what they are operands of is formed by single
 // multiply-adds (a step of the forward, a source of the backward), so that infinite and finite results are those of the
 // CUDA-core kernel; NaN spreads as it would there.  128 x 256, 13 blocks to {4, 4, 4}: the test for them takes 1 % of the backward; an
@@ -819,7 +819,11 @@ bool pays(const FArgs<float>& a) {
 
 }  // namespace
 
-bool tensor_cores_forward(const FArgs<float>& a) { return pays(a) && forward_plan(a).total <= SMEM_MOST; }
+// Rows: with few trunk outputs the roundings of a column's two chains and of Z_0 weigh more than those of the CUDA-core kernel's single
+// chain.  Error against float64, here over there, by k: 2 1.10 to 1.16, 3 1.12 to 1.19, 5 1.09 to 1.13, 7 1.05 to 1.07, 8 1.03, 9 1.01, 10 0.98,
+// 11 0.96, 13 0.92 to 0.94, 17 0.85 to 0.88 (three field types, powers and scales).  The backward's are 0.2 to 0.8 for any k.
+constexpr int FWD_LEAST_K = 10;
+bool tensor_cores_forward(const FArgs<float>& a) { return a.k >= FWD_LEAST_K && pays(a) && forward_plan(a).total <= SMEM_MOST; }
 bool tensor_cores_backward(const FArgs<float>& a) { return pays(a) && backward_plan(a).total <= SMEM_MOST; }
 
 int forward_tc(const FArgs<float>& a, cudaStream_t stream) {
