@@ -26,6 +26,7 @@
 // infinity in one polar node's Z makes the forward 731 -> 1 042, in one row of the gradient the backward 1 838 -> 3 572, and
 // nothing but infinities 3 400 and 10 807 (CUDA-core kernels 1 040 and 2 470).
 #include <algorithm>
+#include <cmath>
 
 #include "factored.cuh"
 
@@ -806,25 +807,50 @@ int backward_warps(const FArgs<float>& a) { return std::min((std::max(likely_til
 BackwardPlan backward_plan(const FArgs<float>& a) {
   return BackwardPlan(a.n_blocks, Record(a.k, a.n_f, n_rho(a), a.d_out, true), backward_warps(a));
 }
-// The CUDA-core kernels stay the faster ones where a source has few edges (its columns are split once for all of them) or tiles of four
-// copies are half empty.  us forward and backward, CUDA cores / tensor cores, by edges per source and copies per block: 92 edges, 4
-// copies, 13 blocks 1 036 + 2 463 / 734 + 1 811; 80 edges, 8 copies 545 + 864 / 355 + 828; 122 edges, 8 copies, 5 blocks 136 + 320 / 84 + 245; 32 edges, 4
-// copies 35 + 67 / 30 + 60; 33 edges, 3 copies 21 + 42 / 18 + 40; 152 edges, 2 copies, 5 blocks 474 + 1 454 / 367 + 1 312; but 80 edges, 2 copies 176 + 400 / 182
-// + 425 and 15 edges, 3 copies 79 + 172 / 96 + 177.  (Edge indices are 32-bit here.)
-bool pays(const FArgs<float>& a) {
+// Where the tensor-core kernels are the faster ones: 949 timings, lattices from 24 x 48 to 128 x 256, radius 1 to 4 rows (7 to 144 edges per
+// source), k 2 to 17, 5, 13 or 25 blocks of 2 to 8 copies.  A source's columns are split once for all of its edges (few edges: no),
+// tiles of four copies may be part empty, and a step takes as long whatever k is, where the CUDA-core kernels' products grow with
+// it, four trunk outputs (a quad) at a time.  us, CUDA cores / tensor cores:
+//   forward   from 24 edges on (92 edges, 13 blocks of 4 copies, k 17: 1 034 / 734, k 11 873 / 691; 38, 13 of 8: 337 / 259), with part-empty tiles from 4.5 edges a tile on (69 edges, 13 blocks of 3: 55 / 48; 133, 13 of 2: 262 / 246;
+//             but 43 edges, 13 of 3, 1.06 to 1.09 of the time, 92, 13 of 5, 1.07 to 1.16).
+//   backward  k 17: 92 edges, 13 blocks of 4, 2 475 / 1 838; 80, 13 of 3, 495 / 439; 80, 13 of 8, 867 / 838; 133, 13 of 8, 1 319 / 1 196; but 80, 13 of 2,
+//             400 / 432; 38, 13 of 8, 532 / 570.  k 11: 80, 13 of 4, 518 / 437, but 80, 13 of 8, 771 / 825.  k 9: 80, 13 of 8, 602 / 803; 43, 5 of 4, 818 / 594.
+//             Small launches last as long as their longest source's steps, which are longer here.  The lines are fitted to that: at worst
+//             10 % (k 10 on 26 tiles, 45 x 90 with k 2), at k 16 and 17 5 %.  Where the other kernel would pass a source's edges twice (25 blocks of 8:
+//             0.71 to 0.76 of its time) always.
+// (Edge indices are 32-bit here.)
+struct Split {
+  int tiles;
+  double fill, edges;  // share of the tiles' copies that exist, edges per source
+  explicit Split(const FArgs<float>& a)
+      : tiles(std::max(likely_tiles(a.wc, a.wr, a.n_blocks), 1)), fill((double)(a.wc + a.wr) / (4 * tiles)), edges((double)a.n_edges / a.n_groups) {}
+};
+bool serves(const FArgs<float>& a) {
   if (a.k < 2 || a.k > TRUNK + 1 || a.n_blocks < 1 || a.n_edges >= (1ll << 31)) return false;
-  const double fill = (double)(a.wc + a.wr) / (4 * std::max(likely_tiles(a.wc, a.wr, a.n_blocks), 1));
-  return fill * fill * a.n_edges >= 24.0 * a.n_groups;
+  const Split s(a);
+  return s.fill * s.fill * s.edges >= 24;
 }
-
-}  // namespace
 
 // Rows: with few trunk outputs the roundings of a column's two chains and of Z_0 weigh more than those of the CUDA-core kernel's single
 // chain.  Error against float64, here over there, by k: 2 1.10 to 1.16, 3 1.12 to 1.19, 5 1.09 to 1.13, 7 1.05 to 1.07, 8 1.03, 9 1.01, 10 0.98,
 // 11 0.96, 13 0.92 to 0.94, 17 0.85 to 0.88 (three field types, powers and scales).  The backward's are 0.2 to 0.8 for any k.
 constexpr int FWD_LEAST_K = 10;
-bool tensor_cores_forward(const FArgs<float>& a) { return a.k >= FWD_LEAST_K && pays(a) && forward_plan(a).total <= SMEM_MOST; }
-bool tensor_cores_backward(const FArgs<float>& a) { return pays(a) && backward_plan(a).total <= SMEM_MOST; }
+
+}  // namespace
+
+bool tensor_cores_forward(const FArgs<float>& a) {
+  if (a.k < FWD_LEAST_K || !serves(a)) return false;
+  const Split s(a);
+  return (s.fill > 0.999 || s.edges >= 4.5 * s.tiles) && forward_plan(a).total <= SMEM_MOST;
+}
+bool tensor_cores_backward(const FArgs<float>& a) {
+  if (!serves(a)) return false;
+  const Split s(a);
+  const int quads = (a.k + 2) / 4, patches = (a.k + 4) / 5 * ((2 * a.wc + a.wr + 3) / 4);
+  const bool pays = patches > 256 || (quads == 4 && std::pow(s.fill, 3) * s.edges >= 2 * s.tiles) ||
+                    ((quads > 2 || s.tiles <= 5) && quads * std::pow(s.fill, 1.5) * std::pow((double)a.n_edges, 0.25) >= 3.7 * s.tiles);
+  return pays && backward_plan(a).total <= SMEM_MOST;
+}
 
 int forward_tc(const FArgs<float>& a, cudaStream_t stream) {
   const ForwardPlan plan = forward_plan(a);
