@@ -369,8 +369,11 @@ __global__ void __launch_bounds__(FTHREADS) factored_forward_wide_kernel(FArgs<T
 
 // out_i = sum over the target's edges of w_e * row_e  (factored.h:337-347): a warp per target.  What bounds it: the rows' stream, and
 // the polar targets' chains of edges.  Lanes are vectors of V columns, and as many edges at a time as the vectors leave room for, whose
-// sums meet at the end.  128 x 256, radius 3 pi / 128, 20 columns, float32: 45 us (a lane per column, an edge at a time: 120).
-template <typename T, int V>
+// sums meet at the end: one after the other, or (TREE) half of them added to the others at a time.  128 x 256, radius 3 pi / 128, 20
+// columns, float32: 45 us (a lane per column, an edge at a time: 120).  The tree is for rows of one or two vectors (40 000 targets of
+// 37 edges, 4 columns 30 -> 15 us), and for columns one by one (33: 73 -> 56); with it the compiler has fewer rows under way,
+// which longer rows notice (128 columns: 118 -> 129; four rows a step written out: 128 to 141).
+template <typename T, int V, bool TREE>
 __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict__ weights, const int64_t* __restrict__ row_ptr,
                                  int64_t n_targets, int d_out, T* __restrict__ out) {
   struct alignas(V * sizeof(T)) Vec { T x[V]; };
@@ -393,11 +396,23 @@ __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict
         for (int v = 0; v < V; ++v) acc[v] += w * row.x[v];
       }
     }
-    for (int s = 1; s < slots; ++s) {
+    if constexpr (TREE) {
+      for (int n = slots; n > 1;) {
+        const int half = (n + 1) / 2;
 #pragma unroll
-      for (int v = 0; v < V; ++v) {
-        const T other = __shfl_sync(0xffffffffu, acc[v], (lane + s * width) & 31);
-        if (slot == 0) acc[v] += other;
+        for (int v = 0; v < V; ++v) {
+          const T other = __shfl_sync(0xffffffffu, acc[v], (lane + half * width) & 31);
+          if (slot + half < n) acc[v] += other;
+        }
+        n = half;
+      }
+    } else {
+      for (int s = 1; s < slots; ++s) {
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+          const T other = __shfl_sync(0xffffffffu, acc[v], (lane + s * width) & 31);
+          if (slot == 0) acc[v] += other;
+        }
       }
     }
     if (slot == 0) {
@@ -406,6 +421,22 @@ __global__ void aggregate_kernel(const T* __restrict__ rows, const T* __restrict
       for (int v = 0; v < V; ++v) sum.x[v] = acc[v];
       *reinterpret_cast<Vec*>(out + i * d_out + c) = sum;
     }
+  }
+}
+// The same with a lane per column, an edge at a time: for many targets of few edges, whose rows are soon read, so that the division
+// of the lanes and the meeting of their sums would cost more than they save.
+template <typename T>
+__global__ void aggregate_columns_kernel(const T* __restrict__ rows, const T* __restrict__ weights, const int64_t* __restrict__ row_ptr,
+                                         int64_t n_targets, int d_out, T* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
+  const int64_t x = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (x >= n_targets) return;
+  const int64_t i = from_both_ends(x, n_targets);
+  const int64_t e0 = row_ptr[i], e1 = row_ptr[i + 1];
+  for (int c = lane; c < d_out; c += 32) {
+    T acc = T(0);
+    for (int64_t e = e0; e < e1; ++e) acc += weights[e] * rows[e * d_out + c];
+    out[i * d_out + c] = acc;
   }
 }
 
@@ -679,8 +710,16 @@ extern "C" int gm_factored_aggregate(const void* rows, const void* weights, cons
     using T = decltype(tag);
     constexpr int V = 16 / sizeof(T);
     auto go = [&](auto kernel) { kernel<<<blocks, 256, 0, (cudaStream_t)stream>>>((const T*)rows, (const T*)weights, row_ptr, n_targets, d_out, (T*)out); };
-    if (d_out % V == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) go(aggregate_kernel<T, V>);
-    else go(aggregate_kernel<T, 1>);
+    const bool vectors = d_out % V == 0 && ((reinterpret_cast<uintptr_t>(rows) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+    // us by columns / by vectors, 40 000 targets: of 8 edges, 20 columns 9 / 14 (float64 12 / 14), 64 columns 20 / 16; of 16 edges, 20 columns 13 / 16
+    // (float64 35 / 30), 33 columns 22 / 30, 40 columns 29 / 26; of 24, 20 columns 19 / 17, 33 columns 37 / 40.  4 000 targets are too few to
+    // tell (3 us), and of those of 8 x 16 edges the longest take 7 / 4.
+    const bool few = n_targets > 12288 && n_edges < 24 * n_targets &&
+                     ((int64_t)sizeof(T) * n_edges * d_out < 1600 * n_targets || (!vectors && d_out > 32));
+    if (few) go(aggregate_columns_kernel<T>);
+    else if (!vectors) go(aggregate_kernel<T, 1, true>);
+    else if (d_out <= 2 * V) go(aggregate_kernel<T, V, true>);
+    else go(aggregate_kernel<T, V, false>);
   };
   if (dtype == GM_F32) run(float());
   else run(double());

@@ -1182,3 +1182,22 @@ def test_aggregate_widths(d_out, dtype, offset):
     want = torch.zeros(len(degrees), d_out, dtype=torch.float64).index_add(0, target, terms)
     size = torch.zeros_like(want).index_add(0, target, terms.abs())
     assert ((got - want).abs() <= (degrees[:, None] + 1) * torch.finfo(dtype).eps * size).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("d_out", [1, 8, 20, 33, 50])
+def test_aggregate_many_targets_of_few_edges(d_out, dtype):
+    """12 300 targets of 0 to 12 edges, by columns where vectors would cost more; the bound of ``test_aggregate_widths``."""
+    from gm_attention_b200.nn import fused_factored as ff
+
+    gen = torch.Generator().manual_seed(d_out)
+    degrees = torch.randint(0, 13, (12300,), generator=gen)
+    row_ptr = torch.cat([torch.zeros(1, dtype=torch.int64), degrees.cumsum(0)])
+    n_edges = int(row_ptr[-1])
+    rows, weights = (torch.randn(*shape, generator=gen, dtype=torch.float64).to(dtype) for shape in ((n_edges, d_out), (n_edges,)))
+    got = ff.extension(True).aggregate(rows.cuda(), weights.cuda(), row_ptr.cuda()).cpu().double()
+    terms = weights.double()[:, None] * rows.double()
+    target = torch.repeat_interleave(torch.arange(len(degrees)), degrees)
+    want = torch.zeros(len(degrees), d_out, dtype=torch.float64).index_add(0, target, terms)
+    size = torch.zeros_like(want).index_add(0, target, terms.abs())
+    assert ((got - want).abs() <= (degrees[:, None] + 1) * torch.finfo(dtype).eps * size).all()
