@@ -163,8 +163,25 @@ __device__ __forceinline__ bool is_scalar(const FusedArgs<S>& a, int t) { return
 // 261 with one addition for a pair; of 8 x (m <= 3) three CTAs (80 registers) are better than two, 350 and 402.  Two edges' gathers in
 // flight cost registers: 239 -> 275 and 402 -> 413 before FORM.  Groups of lanes in turn on the edges (SHARED): 1 head of 8 x (m <= 3)
 // on 3 000 points, batch 4, 138 -> 41 and 197 -> 75; 2 heads of 5 x (m <= 2) on 5 000, batch 3, 194 -> 85 and 270 -> 110.
+// CTAs to an SM that the registers are held to, where the compiler would take a few registers more and leave one CTA less.  By the
+// plan (FORM 0) 6 000 targets of 20 edges, bfloat16, 4 heads of 20 x (m <= 1) take 85 us forward with two CTAs, 72 with three; 2 000 of 20,
+// float32, 4 heads of 20 scalars 48 backward with three, 31 with four.  Two copies a lane: 40 000 targets of 4 edges, 8 heads of 8 x (m <= 1),
+// float32, 285 backward with two, 206 with three.
 template <typename S, int NS, int FORM, bool SHARED>
-__global__ void __launch_bounds__(256, !FORM && NS <= 4 && !SHARED ? 3 : 0) fused_forward_kernel(const __grid_constant__ FusedArgs<S> a) {
+constexpr int forward_ctas() {
+  if (FORM || SHARED) return 0;
+  if (sizeof(S) == 2) return NS <= 4 ? 4 : NS <= 8 ? 3 : 0;
+  return NS <= 4 ? 3 : 0;
+}
+template <typename S, int NS, int FORM, bool SHARED>
+constexpr int backward_ctas() {
+  if (sizeof(S) > 4) return 1;
+  if (FORM == 1) return NS <= 3 ? 4 : 3;
+  if (FORM == 2 && NS == 4) return 3;
+  return FORM == 0 && !SHARED && NS <= 4 ? 4 : 1;
+}
+template <typename S, int NS, int FORM, bool SHARED>
+__global__ void __launch_bounds__(256, forward_ctas<S, NS, FORM, SHARED>()) fused_forward_kernel(const __grid_constant__ FusedArgs<S> a) {
   using C = typename Compute<S>::type;
   const int lane = threadIdx.x & 31;
   const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -271,7 +288,7 @@ __global__ void __launch_bounds__(256, !FORM && NS <= 4 && !SHARED ? 3 : 0) fuse
 }
 
 template <typename S, int NS, int FORM, bool SHARED>
-__global__ void __launch_bounds__(256, FORM == 1 && sizeof(S) <= 4 ? (NS <= 3 ? 4 : 3) : 1) fused_backward_kernel(const __grid_constant__ FusedArgs<S> a) {
+__global__ void __launch_bounds__(256, backward_ctas<S, NS, FORM, SHARED>()) fused_backward_kernel(const __grid_constant__ FusedArgs<S> a) {
   using C = typename Compute<S>::type;
   using A = typename std::conditional<std::is_same<S, __nv_bfloat16>::value, float, S>::type;
   const int lane = threadIdx.x & 31;
