@@ -7,15 +7,17 @@
 // message :174-206, its backward :211-232); the kernels themselves are new:
 //
 //  * scores, head-grouped (H a power of two, the usual case): one or two warps per target, the lanes split into H head
-//    groups, every lane owning a few copies of every frequency; four edges' gathers of k_j are in flight; the raw
-//    logits go to alpha and the same warps normalise the row in place.
+//    groups (narrow heads: several times over, the groups taking the target's edges in turn), every lane owning a few copies
+//    of every frequency; four edges' gathers of k_j are in flight; the raw logits go to alpha and the same warps normalise
+//    the row in place.
 //  * scores, general: one block per target, one WARP per edge with the lanes striding the key row (coalesced
 //    128-byte reads of k_j), per-head sums by warp shuffle; the row's logits live in shared memory (or, for very
 //    large neighbourhoods, in the alpha output itself) and are normalised there.
 //  * softmax backward, conv forward / backward: one warp per target and one LANE per work item -- a (head,
 //    frequency, copy) or (frequency, copy): a scalar column or a (re, im) column pair -- listed once per CTA in
-//    shared memory; a lane walks the node's edges in order (sequential sums per output) with four edges' loads in
-//    flight, 8-byte accesses for the pairs where the address allows, atomics only for the scattered dk / dv.
+//    shared memory.  Where there are few items, groups of lanes take the node's edges in turn and their sums meet by shuffles.
+//    Four edges' loads are in flight (conv backward: three), pairs are read as pairs where the addresses allow, atomics only for
+//    the scattered dk / dv.
 #include "common.cuh"
 
 namespace gmb {
@@ -762,7 +764,9 @@ int softmax_forward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, int ma
   if ((a.H == 1 || a.H == 2 || a.H == 4 || a.H == 8) && max_mult > 0 && max_mult <= 4 * (32 / a.H)) {
     const int per_lane = (max_mult + 32 / a.H - 1) / (32 / a.H);
     a.shares = 1;
-    while (2 * a.shares * max_mult <= 32 / a.H) a.shares *= 2;
+    // (with fewer edges most groups have none: of 5 edges each 1.13 to 1.19 of the time without groups for one frequency, 8 0.82 to 0.88)
+    if (n_edges >= 7 * a.n_nodes)
+      while (2 * a.shares * max_mult <= 32 / a.H) a.shares *= 2;
     auto go = [&](auto parts) {
       constexpr int P = decltype(parts)::value;
       const unsigned blocks = (unsigned)((a.n_nodes * P + 3) / 4);
@@ -799,14 +803,18 @@ int softmax_backward_t(SoftmaxArgs<T> a, int64_t n_edges, int64_t deg_max, cudaS
   // dk by pairs where targets have many edges, on average or some of them: with few the vector reductions only hold the next
   // target's loads back.  us by numbers / by pairs: 163 842 points of even degree 12 492 / 552, 40 962 of degree 12 146 / 157, 10 242 of degree 21
   // 69 / 67, of degree 100 261 / 232; 64 x 128, radius 2 pi / 64 (mean 38, at most 257) 220 / 200; 128 x 256, radius 3 pi / 128 1 051 / 829.
-  const bool uneven = deg_max * a.n_nodes >= 4 * n_edges, pairs = n_edges >= 24 * a.n_nodes || uneven;
+  // Uneven only where the longest targets' chains are not lost among many short ones: the same with deg_max 8 x the degree at both ends,
+  // as uneven / as even, mean over twelve types against the time before either: 40 000 nodes of 5 edges 1.22 / 0.94, of 16 0.89 / 0.73, 14 000 of 8 0.99 /
+  // 0.87, of 24 0.67 / 0.67, of 40 0.59 / 0.63, 3 000 of 3 0.99 / 0.81, of 8 0.64 / 0.66; but 128 x 256, radius pi / 128 (mean 12, at most 257) 178 / 273 us.
+  const bool few = a.n_nodes <= 12288, uneven = deg_max * a.n_nodes >= (n_edges >= (few ? 6 : 20) * a.n_nodes ? 4 : 12) * n_edges;
+  const bool pairs = n_edges >= 24 * a.n_nodes || uneven;
   auto go = [&](auto kernel) { kernel<<<conv_grid(a.n_nodes), CONV_THREADS, a.D * sizeof(ScoreItem), stream>>>(a); };
   // Sources read ahead where the chains of gathers show: some targets' long ones, or few targets.  us without / with: 120 x 240, radius
   // 2.5 pi / 120, 4 heads of 5 x (m <= 3) 505 / 389, 99 x 198, radius 2.5 pi / 99, 8 of 5 x (m <= 2) 502 / 346, 8 of 16 x (m <= 2) 1 372 / 980, 128 x 256,
   // radius 3 pi / 128, 4 of 8 x (m <= 3) 822 / 775; points of even degree 40, 30 000, 4 of 8 x (m <= 2) 303 / 319, of 8 x (m <= 1) 207 / 229,
   // 3 000 85 / 82.  (A group of lanes per head and one walk for all frequencies: 765 and 286 on the lattices of 4 heads of 8 x (m <= 3), but
   // 1 158 for the 16 copies and 502 for the five, and 1 425 against 957 where 20 000 points have 40 edges each, 8 of 16 x (m <= 3).)
-  const bool ahead = uneven || a.n_nodes <= 12288;
+  const bool ahead = uneven || (few && (sizeof(T) == 4 || n_edges >= 16 * a.n_nodes));  // (float64, 3 000 of 5 edges each: 6 % slower ahead)
   if (pairs && ahead) go(softmax_backward_kernel<T, true, true>);
   else if (pairs) go(softmax_backward_kernel<T, true, false>);
   else if (ahead) go(softmax_backward_kernel<T, false, true>);

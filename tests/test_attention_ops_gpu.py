@@ -161,6 +161,38 @@ def test_ops_with_lanes_that_share_edges(ext, types, heads, dtype):
         compare(ext.conv_backward(cuda(k), cuda(q), *dev, a0, coef), want, ["dv", "drc", "dcc"])
 
 
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n, degree, longest", [
+    (12400, 24, 24),   # pairs of dk at once, sources not read ahead
+    (12400, 5, 5),     # by numbers, not ahead; forward: no groups of lanes
+    (12400, 12, 600),  # uneven: pairs, ahead
+    (700, 8, 8),       # few targets: by numbers, ahead (float64: not)
+    (700, 24, 24),     # pairs, ahead
+])
+def test_scores_by_every_kernel(ext, n, degree, longest, dtype):
+    """Scores and their gradients where each of the kernels' variants is chosen, against the oracle in float64: to 1e-12 of the
+    largest value, in float32 to 2e-6 (a gradient of dk sums about as many terms as a target has edges, up to 600 of dq)."""
+    rng = np.random.default_rng(7)
+    degrees = np.full(n, degree)
+    degrees[:1] = longest
+    row_ptr = np.concatenate([[0], np.cumsum(degrees)]).astype(np.int64)
+    e, heads = int(row_ptr[-1]), 2
+    source = rng.integers(0, n, e).astype(np.int64)
+    desc = np.array([[0, 3, 0, 0, 1], [1, 4, 6, 0, 2]], np.int64)
+    phase = np.exp(1j * rng.uniform(0, 6.28, (e, 1)) * np.arange(2))
+    q, k, da, transport, bias = (x.astype(dtype) for x in (rng.standard_normal((n, 22)), rng.standard_normal((n, 22)), rng.standard_normal((e, heads)),
+                                                           np.stack([phase.real, phase.imag], -1), rng.standard_normal(e)))
+    inside = np.ones(e, np.uint8)
+    wide = lambda *xs: [x.astype(np.float64) for x in xs]
+    alpha = O.softmax_forward(*wide(q, k, transport, bias), inside, desc, row_ptr, source, heads, 0.3)
+    want = O.softmax_backward(*wide(da, q, k, transport), desc, row_ptr, source, alpha, heads, 0.3)
+    tables = [cuda(x) for x in (transport, bias, inside, desc, row_ptr, source)]
+    got = [ext.softmax_forward(cuda(q), cuda(k), *tables, heads, 0.3, longest),
+           *ext.softmax_backward(cuda(da), cuda(q), cuda(k), *tables, cuda(alpha.astype(dtype)), heads, 0.3, longest)]
+    for name, a, b in zip(("alpha", "dq", "dk"), got, (alpha, *want)):
+        assert_close(a.cpu().numpy(), b.astype(dtype), 0.0, (1e-12 if dtype == np.float64 else 2e-6) * magnitude(b), name)
+
+
 def test_softmax_large_neighbourhood_spills_to_global(ext):
     """A row whose logits exceed the shared-memory budget keeps them in alpha."""
     n, deg, heads, d = 3, 30000, 2, 4
