@@ -178,18 +178,18 @@ __global__ void __launch_bounds__(SM_THREADS) softmax_forward_kernel(SoftmaxArgs
 //
 // PARTS warps share a target, four edges of it in turn each.  Two where the launch is about as long as its longest target's chain
 // of edges (about 1 us for four), one where there are edges enough to hide it: then every warp of a pair only repeats the other's
-// q_i and waits for it.  us with one / two, float32: 128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3) (3 920 edges per edge of the
-// longest target) 883 / 762 (four: 808); 64 x 128, radius 4 pi / 64 (2 120) 575 / 318; 2 562 points of even degree 200 (2 500) 199 / 121;
-// 10 242 points, 4 heads of 8 x (m <= 2), degree 12 (8 400) 39 / 47, degree 200 429 / 432; 163 842, degree 12 457 / 623.  Eight heads' groups of
-// four lanes take longer over an edge: 10 242 points, degree 21 92 / 82, degree 100 356 / 285, degree 11 57 / 57.  (All before the walk
-// below lost its branches.)
+// q_i and waits for it.  us with one / two, float32: 128 x 256, radius 3 pi / 128, 4 heads of 8 x (m <= 3) (3 899 edges per edge of the
+// longest target) 584 / 509; 64 x 128, radius 4 pi / 64 (2 126) 338 / 187; 128 x 256, radius 4 pi / 128 (4 931) equal; 2 562 points of even degree 200, 4 of
+// 8 x (m <= 2), 130 / 79; 10 242 points, degree 12 24 / 30, degree 200 334 / 323; 120 000, degree 12 289 / 383.  Eight heads' groups of four lanes take
+// longer over an edge: 10 242 points, degree 40 100 / 91 and 203 / 187, degree 200 534 / 468, but degree 21 56 / 57 and (4 x (m <= 1)) 32 / 36, 40 962 202 / 232.
+// 288 timings: 1.1 % above the better of the two in the mean, one frequency pair of 2 562 points with eight heads 34 % (11 us).
 //
 // What bounds it: the issue of what surrounds the gathers.  With every slot of a lane looked up and branched around in the walk the
 // first of these took 740 us, with the kind of a slot known and lanes without a copy reading nothing 511 (two edges in flight 683,
 // two with their sources read ahead 614); 99 x 198, radius 2.5 pi / 99: 8 heads of 8 x (m <= 2) 494 -> 278, of 16 x (m <= 2) 2 014 -> 546,
 // 120 x 200, radius 3 pi / 120, 8 heads of 4 x (m <= 1) 447 -> 262.  CTAs of 8 or 16 warps on neighbouring targets: 583, 566.
 int score_parts(int64_t n_nodes, int64_t n_edges, int64_t deg_max, int H) {
-  return n_edges <= 4096 * deg_max || (H == 8 && n_edges >= 16 * n_nodes) ? 2 : 1;
+  return n_edges <= 4096 * deg_max || (H == 8 && n_edges >= 32 * n_nodes) ? 2 : 1;
 }
 
 // The logits of a target's edges turn, turn + turns, ... and their maximum, in the descriptor's order and number by number.  Not
