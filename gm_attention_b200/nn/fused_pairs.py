@@ -328,11 +328,12 @@ def _readouts_fit(kernel: Any, needed: tuple, hidden: Tensor) -> bool:
 
 
 def _products_repaid(n_nodes: int, n_edges: int) -> bool:
-    """Whether a node's products serve enough edges.  Forward and backward, float32, trunk 16, ms as factored form / pair
-    terms, before the products became two to three times faster: {16, 16} -> {8, 8} on 30 000 nodes 3.53 / 2.71 at 4.9 edges
-    per node, 3.63 / 3.63 at 8.6, 3.81 / 5.95 at 17 (the products bound the factored form there); {2, 2} -> {8, 8}
-    1.97 / 1.90 at 6.8, 2.20 / 2.64 at 17.  Up to 8 192 nodes both wait for their launches, of which the factored form has
-    fewer: 1.32 / 1.42 at 2.6, 1.33 / 1.73 at 4.8."""
+    """Whether a node's products serve enough edges, so that no kernel measured loses by the factored form, a first pass
+    on an edge set (0.25 to 0.5 ms for its grouping) included.  Forward and backward, float32, trunk 16, ms as factored form /
+    pair terms.  Beyond 8 192 nodes the narrow kernels on many nodes decide: {2, 2} -> {8, 8} on 80 000 nodes 2.91 / 2.24 at
+    4.9 edges per node, 3.16 / 2.90 at 8.8, 3.26 / 3.34 at 10.9; others would gain earlier ({16, 16} -> {8, 8} there 4.03 / 4.88 at
+    4.9, on 30 000 nodes 1.72 / 2.70; {8, 8, 8} -> {4, 4, 4} 1.71 / 2.72).  Up to 8 192 nodes both wait for their launches, of which the
+    factored form has fewer: {2, 2} -> {8, 8} 1.16 / 1.37 from 1 to 8 edges per node, three frequencies 1.24 / 2.05."""
     return n_edges >= (4 if n_nodes <= 8192 else 10) * n_nodes
 
 
