@@ -698,16 +698,17 @@ static ApplyGrid apply_grid(const ConvArgs& a) {
 }
 
 // The FMA kernels stay the faster ones where the tiles are mostly padding and there are enough of them to fill the chip.  333
-// shapes from 24 x 24 to 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores:
+// shapes from 24 x 24 to 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores (apply), 576 (table_grad):
 //   apply        a CTA takes up to 64 tiles of 8 longitudes.  From 32 on it is the faster one (128 x 128, width 320, batch 2: 179 / 179, batch
 //                4: 333 / 237; 256 x 512, width 320: 1 336 / 540), with fewer while the launch has few CTAs and lasts as long as the polar
 //                rows' chains of stages, which are shorter here (64 x 128, batch 1, width 160: 81 / 42, width 320: 78 / 70; 128 x 128, batch
 //                1, width 160: 116 / 81, but width 320: 112 / 154).  With up to 8 tiles a row the FMA kernel's chains are short too (32 x 64:
 //                50 / 25, width 320: 48 / 47; 200 x 48, width 24: 24 / 22, width 40: 24 / 28, width 320: 28 / 116).
-//   table_grad   contracts over the tiles, 16 a step: 23 tiles and more are always faster (91 x 184, width 320: 132 / 128; 256 x 512: 1 701 /
-//                738), 9 to 22 with four samples (45 x 88, width 80: 62 / 46, width 320: 132 / 116), one block of 32 columns (28 / 21), or
-//                two samples of a field that is not wide (45 x 88, width 96: 38 / 38, width 160: 32 / 38; 64 x 128, width 160: 69 / 54, width
-//                320: 97 / 93; 128 x 128, width 320: 175 / 196); 8 tiles with one block of 32 columns and four samples (32 x 64: 32 / 22).
+//   table_grad   contracts over the tiles of all samples, 16 a step; the FMA kernel takes samples by two.  The least tiles by samples and
+//                width are the least at which neither radius 2 nor 4 rows lost (576 timings, 9 to 32 tiles; but 40 columns, one sample, 4 rows: 1.13 at 19): one sample, width 160, radius 2, 22 tiles 38 /
+//                42, 24 0.77 of the time; width 320 24 tiles 73 / 81, 28 0.92; two, width 320, 22 tiles 94 / 103, 24 0.98; width 160 19 tiles 52 / 50;
+//                width 96 11 tiles 1.12, 13 0.89; three, width 320, 11 tiles 61 / 51, 19 133 / 112, radius 4 358 / 231.  One block of 32 columns always
+//                (9 tiles 0.50), 8 tiles with four samples (32 x 64: 32 / 22).  256 x 512: 1 701 / 738.
 bool tensor_cores_apply(const ConvArgs& a) {
   if (!tensor_cores_can(a) || !tensor_cores_hold(a)) return false;
   const int T = a.nlon / 8;
@@ -716,10 +717,11 @@ bool tensor_cores_apply(const ConvArgs& a) {
   return T > 8 ? fill >= 32 || ctas <= 80 * fill : T >= 3 && ctas <= 80 * T;
 }
 bool tensor_cores_table_grad(const ConvArgs& a) {
-  const int T = a.nlon / 8;
   const bool narrow = a.width <= TG_COLS;
-  const bool pays = T > 8 ? T >= 20 || narrow || a.batch >= 4 || (a.batch >= 2 && a.width <= (T >= 16 ? 160 : 96)) : T == 8 && narrow && a.batch >= 4;
-  return tensor_cores_can(a) && pays;
+  const int by_width = a.width <= 96 ? 0 : a.width <= 160 ? 1 : 2;
+  constexpr int ONE[] = {16, 24, 28}, TWO[] = {13, 19, 24};
+  const int least = narrow ? (a.batch >= 4 ? 8 : 9) : a.batch >= 4 ? 9 : a.batch == 3 ? 11 : a.batch == 2 ? TWO[by_width] : ONE[by_width];
+  return tensor_cores_can(a) && a.nlon / 8 >= least;
 }
 
 int apply_tc(const ConvArgs& a, int n_order, cudaStream_t stream) {
