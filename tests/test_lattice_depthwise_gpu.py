@@ -226,6 +226,40 @@ def test_tensor_core_kernels_against_the_host_loops(nlat, nlon, reach, head, bat
         assert_close(got.cpu().numpy(), want, 1e-5, 1e-5 * np.abs(want).max(), "table gradient")
 
 
+@pytest.mark.parametrize("head", [{0: 8, 1: 12, 2: 8}, {0: 16, 1: 40, 2: 40}])
+def test_tensor_core_kernels_with_several_blocks_of_columns_per_cta(head):
+    """Launches of so many CTAs that apply gives one CTA up to 2 of 3 or 5 of 11 blocks of 16 columns, table_grad 5 of 6 blocks of 32,
+    the last of each fewer, against the FMA kernels (which take a field on an 8-byte boundary): apply to two roundings to bf16 (2^-8 each)
+    and 1e-5 of the largest, the table gradient to 1e-5 of the largest.  Infinities and NaN in the first, a middle and the last block of
+    several samples and rows reach the same outputs as there."""
+    from gm_attention_b200.nn.lattice_depthwise import _apply, _table_gradient
+
+    batch = 32
+    c, t = tensor_core_case(24, 520, 1.1, head)
+    gen = torch.Generator(device="cuda").manual_seed(75)
+    x, g = (torch.randn(batch * c.n_nodes, c.width, generator=gen, device="cuda").bfloat16() for _ in range(2))
+    table = torch.randn(t.n_entries, t.table_width, generator=gen, device="cuda")
+    shifted = torch.empty(x.numel() + 4, dtype=x.dtype, device="cuda")[4:].view(x.shape)
+    for node, col, value in [(0, 0, None)] + [(b * c.n_nodes + row * 520 + lon, col, value) for b, row, lon in ((0, 12, 519), (17, 5, 8), (31, 23, 260))
+                                             for col, value in ((3, np.inf), (17, np.nan), (c.width - 1, -np.inf), (c.width // 2, np.nan))]:
+        if value is None:
+            shifted.copy_(x)
+            want, got = _table_gradient(g, shifted, t), _table_gradient(g, x, t, tensor_cores=True)
+            assert_close(got.cpu().numpy(), want.cpu().numpy(), 0.0, 1e-5 * float(want.abs().max()), "table gradient")
+            for transposed in (False, True):
+                want, got = (_apply(v, table, t, transposed, tensor_cores=v is x).float() for v in (shifted, x))
+                assert bool(((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-5 * float(want.abs().max())).all())
+        else:
+            x[node, col] = value
+    shifted.copy_(x)
+    for transposed in (False, True):
+        want, got = (_apply(v, table, t, transposed, tensor_cores=v is x).float() for v in (shifted, x))
+        finite = want.isfinite()
+        assert not bool(finite.all()) and torch.equal(got.isfinite(), finite) and torch.equal(got.isnan(), want.isnan())
+        assert torch.equal(got[want.isinf()], want[want.isinf()])
+        assert bool(((got - want).abs() <= 2.0 ** -7 * want.abs() + 1e-5 * float(want[finite].abs().max()))[finite].all())
+
+
 def test_tensor_core_apply_touches_only_true_neighbours():
     """An Inf, a NaN and a value whose products overflow reach exactly the targets that see their nodes, in their own channel."""
     from gm_attention_b200.nn.lattice_depthwise import _apply
