@@ -9,13 +9,12 @@
 // the block factors, and the sum over the blocks of one output, are applied to the accumulators in registers.  A real block is a
 // complex one whose imaginary columns are zero.
 //
-// Precision: every float32 operand is the sum of three bfloat16 (8 + 8 + 8 bits: exact from 2^-110 on, below with an error of up to
-// 2^-134), and of the nine products the six that
+// Precision: every float32 operand is the sum of three bfloat16 (8 + 8 + 8 bits: exactly, mma.cuh), and of the nine products the six that
 // reach 2^-24 of the result are taken, in two chains of three, smallest first; everything that is summed over more than one
 // k-step (the 16 edges of dZ, the two tiles of dh) is added in float32, rounded to nearest.
-// What it measured, 128 x 256, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4}, trunk 16, us on CUDA cores -> here: forward 1 036 -> 734,
-// backward 2 463 -> 1 811.  Bound by latency and issue (issue 43 / 39 %, tensor pipe 17 / 14 %): a step of 16 edges is 78 / 168 products
-// among 1 600 / 4 000 instructions, most of them the splits, the factors and the records' copies.  With the records read where
+// What it measured, 128 x 256, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4}, trunk 16, us on CUDA cores -> here: forward 1 036 -> 731,
+// backward 2 463 -> 1 830.  Bound by latency and issue (issue 41 / 46 %, tensor pipe 17 / 14 %): a step of 16 edges is 78 / 168 products
+// among 1 600 / 4 400 instructions, most of them the splits, the factors and the records' copies.  With the records read where
 // they are (1 245 / 3 225 us) every step waited for its chain of gathers; they are copied a step ahead.  Four tiles a backward warp:
 // eight 2 095 us (the loop over tiles, unrolled for its accumulators, outgrew the instruction cache), two 1 946.  168 registers
 // and twelve warps an SM instead of sixteen: 2 077.  Errors against float64: 0.85 to 0.98 of the CUDA-core kernels' for rows
@@ -29,6 +28,7 @@
 #include <cmath>
 
 #include "factored.cuh"
+#include "mma.cuh"
 
 namespace gmb {
 namespace factored {
@@ -42,53 +42,21 @@ constexpr int MAX_WARPS = 8;
 constexpr int DH_PITCH = TRUNK + 2;
 constexpr int FWD_CTAS = 64, BWD_CTAS = 64;  // CTAs of the grid per SM
 
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float x, float y) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
-  return v;
-}
-__device__ __forceinline__ void add2(f32x2& d, f32x2 v) { asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(v)); }
-__device__ __forceinline__ void add2(f32x2& d, float x, float y) { add2(d, pack2(x, y)); }
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ void mma(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_first(float (&d)[4], const unsigned (&a)[4], unsigned b0, unsigned b1, const float (&zero)[4]) {  // d = a b
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
-               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(zero[0]), "f"(zero[1]), "f"(zero[2]), "f"(zero[3]));
-}
-// sum = a b (rows g and g + 8, two columns each) of operands in three parts (largest first), in float32; zero: four zeros the compiler does not see through (it would
-// clear four registers for every product)
+// sum = a b (rows g and g + 8, two columns each) of operands in three parts (largest first), in float32
 __device__ __forceinline__ void product(f32x2 (&sum)[2], const unsigned (&a)[3][4], const uint2 (&b)[3], const float (&zero)[4]) {
   float low[4], d[4];
-  mma_first(low, a[2], b[0].x, b[0].y, zero);
-  mma_first(d, a[1], b[0].x, b[0].y, zero);
-  mma(low, a[0], b[2].x, b[2].y);
-  mma(d, a[0], b[1].x, b[1].y);
-  mma(low, a[1], b[1].x, b[1].y);
-  mma(d, a[0], b[0].x, b[0].y);
+  auto first = [&](float (&to)[4], int p, int q) { mma_first(to, a[p][0], a[p][1], a[p][2], a[p][3], b[q].x, b[q].y, zero); };
+  auto next = [&](float (&to)[4], int p, int q) { mma(to, a[p][0], a[p][1], a[p][2], a[p][3], b[q].x, b[q].y); };
+  first(low, 2, 0);
+  first(d, 1, 0);
+  next(low, 0, 2);
+  next(d, 0, 1);
+  next(low, 1, 1);
+  next(d, 0, 0);
   sum[0] = pack2(low[0], low[1]);
   sum[1] = pack2(low[2], low[3]);
   add2(sum[0], d[0], d[1]);
   add2(sum[1], d[2], d[3]);
-}
-// (x, y) as three pairs of bfloat16, largest first
-__device__ __forceinline__ void split3(float x, float y, unsigned (&w)[3]) {
-#pragma unroll
-  for (int s = 0; s < 3; ++s) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    w[s] = *reinterpret_cast<const unsigned*>(&h);
-    x -= __uint_as_float(w[s] << 16);
-    y -= __uint_as_float(w[s] & 0xffff0000u);
-  }
 }
 // Operands of 2^60 and more, infinities among them, go to single multiply-adds: of smaller ones no product and no sum here
 // overflows, where parts of opposite signs could make a NaN of an infinity.  (NaN goes where it would go there.)
@@ -104,7 +72,6 @@ __device__ __forceinline__ unsigned transposed(unsigned x) {  // of an 8 x 8 mat
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
   return y;
 }
-
 
 template <int BYTES>
 __device__ __forceinline__ void copy_async(float* dst, const float* src) {

@@ -31,34 +31,12 @@
 #include <algorithm>
 
 #include "lattice_conv.cuh"
+#include "mma.cuh"
 
 namespace gmb {
 namespace lconv {
 namespace {
 
-__device__ __forceinline__ void mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma_first(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0, unsigned b1,
-                                          const float (&zero)[4]) {  // d = a * b
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};\n"
-               : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(zero[0]), "f"(zero[1]), "f"(zero[2]), "f"(zero[3]));
-}
-// Two float32 sums in one 64-bit register pair
-using f32x2 = unsigned long long;
-__device__ __forceinline__ void add2(f32x2& d, float x, float y) {
-  f32x2 v;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(x), "f"(y));
-  asm("add.rn.f32x2 %0, %0, %1;" : "+l"(d) : "l"(v));
-}
-__device__ __forceinline__ float2 unpack2(f32x2 v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
 // 16 bytes global -> shared, asynchronously; bytes = 0 writes zeros
 __device__ __forceinline__ void copy16(uint4* dst, const void* src, int bytes) {
   const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
@@ -455,20 +433,8 @@ __device__ __forceinline__ void apply_again(const ConvArgs& a, const ApplyTile& 
               __floats2bfloat162_rn(y[p][i][e].x, y[p][i][e].y);
 }
 
-// (x, y) = sum of three bfloat16 pairs, largest first
-__device__ __forceinline__ void split3(float x, float y, unsigned (&w)[3]) {
-#pragma unroll
-  for (int s = 0; s < 3; ++s) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-    w[s] = *reinterpret_cast<const unsigned*>(&h);
-    x -= __uint_as_float(w[s] << 16);
-    y -= __uint_as_float(w[s] & 0xffff0000u);
-  }
-}
-
-
-__global__ void __launch_bounds__(2 * GROUP, 2) conv_apply_tc_kernel(const __grid_constant__ ConvArgs a, int col_blocks, int single_rows, int single_ctas, int group, int lon_blocks,
-                                                                             int samples) {
+__global__ void __launch_bounds__(2 * GROUP, 2) conv_apply_tc_kernel(const __grid_constant__ ConvArgs a, int col_blocks, int single_rows, int single_ctas, int group,
+                                                                     int lon_blocks, int samples) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ PairItem pairs_s[AP_GROUP * AP_PAIRS];
   __shared__ unsigned bad_s[AP_GROUP][GROUP];
@@ -581,94 +547,94 @@ __global__ void __launch_bounds__(2 * GROUP, 2) conv_apply_tc_kernel(const __gri
 
   int buf = 0;
   for (int cb = 0; cb < n_cb; ++cb, tile.col0 += AP_COLS) {
-  f32x2 acc[4][4][2];  // channel pair, eight of tiles: rows (s = g: component 0, g + 8: component 1), columns t = 2 c, 2 c + 1
+    f32x2 acc[4][4][2];  // channel pair, eight of tiles: rows (s = g: component 0, g + 8: component 1), columns t = 2 c, 2 c + 1
 #pragma unroll
-  for (int p = 0; p < 4; ++p)
+    for (int p = 0; p < 4; ++p)
 #pragma unroll
-    for (int i = 0; i < 4; ++i) acc[p][i][0] = acc[p][i][1] = 0;
-  ApplyStage cur = stage_at(windows, n_windows, 0, 0);
-  while (cur.w < n_windows) {
-    barrier_sync(full_barrier(buf));
-    const uint4* xs = stage_s + buf * AP_STAGE;
-    const uint2* ms = reinterpret_cast<const uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + 4 * cg * AP_PAIR + 7 + c - g;
-    auto walk = [&](auto count) {
-      constexpr int MINE = decltype(count)::value;
-      for (int k = 0; k < cur.steps; ++k) {
-        unsigned fb[MINE][2][4];
-#pragma unroll
-        for (int i = 0; i < MINE; ++i) {
-          const uint4* from = xs + at[i] + k * AP_PITCH;
-          const uint4 v0 = from[0], v4 = from[4 * AP_SP];
-          fb[i][0][0] = v0.x; fb[i][0][1] = v0.y; fb[i][0][2] = v0.z; fb[i][0][3] = v0.w;
-          fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const uint2* f = ms + p * AP_PAIR + 8 * k;
-          const uint2 l01 = f[2 * AP_SLOTS], l23 = f[2 * AP_SLOTS + 4], m01 = f[AP_SLOTS], m23 = f[AP_SLOTS + 4], h01 = f[0], h23 = f[4];
-          float sum[MINE][4];
-          unsigned b0[MINE], b1[MINE];
+      for (int i = 0; i < 4; ++i) acc[p][i][0] = acc[p][i][1] = 0;
+    ApplyStage cur = stage_at(windows, n_windows, 0, 0);
+    while (cur.w < n_windows) {
+      barrier_sync(full_barrier(buf));
+      const uint4* xs = stage_s + buf * AP_STAGE;
+      const uint2* ms = reinterpret_cast<const uint2*>(stage_s + buf * AP_STAGE + 8 * AP_SP) + 4 * cg * AP_PAIR + 7 + c - g;
+      auto walk = [&](auto count) {
+        constexpr int MINE = decltype(count)::value;
+        for (int k = 0; k < cur.steps; ++k) {
+          unsigned fb[MINE][2][4];
 #pragma unroll
           for (int i = 0; i < MINE; ++i) {
-            b0[i] = __byte_perm(fb[i][0][p], 0, same);
-            b1[i] = __byte_perm(fb[i][1][p], 0, same);
+            const uint4* from = xs + at[i] + k * AP_PITCH;
+            const uint4 v0 = from[0], v4 = from[4 * AP_SP];
+            fb[i][0][0] = v0.x; fb[i][0][1] = v0.y; fb[i][0][2] = v0.z; fb[i][0][3] = v0.w;
+            fb[i][1][0] = v4.x; fb[i][1][1] = v4.y; fb[i][1][2] = v4.z; fb[i][1][3] = v4.w;
           }
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) mma_first(sum[i], l01.x, l01.y, l23.x, l23.y, b0[i], b1[i], zero);
+          for (int p = 0; p < 4; ++p) {
+            const uint2* f = ms + p * AP_PAIR + 8 * k;
+            const uint2 l01 = f[2 * AP_SLOTS], l23 = f[2 * AP_SLOTS + 4], m01 = f[AP_SLOTS], m23 = f[AP_SLOTS + 4], h01 = f[0], h23 = f[4];
+            float sum[MINE][4];
+            unsigned b0[MINE], b1[MINE];
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) mma(sum[i], m01.x, m01.y, m23.x, m23.y, b0[i], b1[i]);
+            for (int i = 0; i < MINE; ++i) {
+              b0[i] = __byte_perm(fb[i][0][p], 0, same);
+              b1[i] = __byte_perm(fb[i][1][p], 0, same);
+            }
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) mma(sum[i], h01.x, h01.y, h23.x, h23.y, b0[i], b1[i]);
+            for (int i = 0; i < MINE; ++i) mma_first(sum[i], l01.x, l01.y, l23.x, l23.y, b0[i], b1[i], zero);
 #pragma unroll
-          for (int i = 0; i < MINE; ++i) {
-            add2(acc[p][i][0], sum[i][0], sum[i][1]);
-            add2(acc[p][i][1], sum[i][2], sum[i][3]);
+            for (int i = 0; i < MINE; ++i) mma(sum[i], m01.x, m01.y, m23.x, m23.y, b0[i], b1[i]);
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) mma(sum[i], h01.x, h01.y, h23.x, h23.y, b0[i], b1[i]);
+#pragma unroll
+            for (int i = 0; i < MINE; ++i) {
+              add2(acc[p][i][0], sum[i][0], sum[i][1]);
+              add2(acc[p][i][1], sum[i][2], sum[i][3]);
+            }
           }
         }
-      }
-    };
-    if (mine == 4) walk(std::integral_constant<int, 4>());
-    else if (mine == 3) walk(std::integral_constant<int, 3>());
-    else if (mine == 2) walk(std::integral_constant<int, 2>());
-    else if (mine == 1) walk(std::integral_constant<int, 1>());
-    barrier_arrive(empty_barrier(buf));
-    cur = next_stage(windows, n_windows, cur);
-    buf = buf == AP_BUFFERS - 1 ? 0 : buf + 1;
-  }
+      };
+      if (mine == 4) walk(std::integral_constant<int, 4>());
+      else if (mine == 3) walk(std::integral_constant<int, 3>());
+      else if (mine == 2) walk(std::integral_constant<int, 2>());
+      else if (mine == 1) walk(std::integral_constant<int, 1>());
+      barrier_arrive(empty_barrier(buf));
+      cur = next_stage(windows, n_windows, cur);
+      buf = buf == AP_BUFFERS - 1 ? 0 : buf + 1;
+    }
 
-  // ---- four channel pairs of a position are 16 bytes of its row
-  const int col = tile.col0 + 8 * cg;
-  unsigned bad = 0;  // outputs whose sums are not finite
-  if (col < a.width) {
-    bool whole = true;
+    // ---- four channel pairs of a position are 16 bytes of its row
+    const int col = tile.col0 + 8 * cg;
+    unsigned bad = 0;  // outputs whose sums are not finite
+    if (col < a.width) {
+      bool whole = true;
 #pragma unroll
-    for (int p = 0; p < 4; ++p) whole = whole && pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0;
+      for (int p = 0; p < 4; ++p) whole = whole && pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        const int n = 8 * (half + 2 * i) + 2 * c + e;
-        if (n >= n_tiles) continue;
-        unsigned word[4];
+        for (int e = 0; e < 2; ++e) {
+          const int n = 8 * (half + 2 * i) + 2 * c + e;
+          if (n >= n_tiles) continue;
+          unsigned word[4];
 #pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          const float2 re = unpack2(acc[p][i][0]), im = unpack2(acc[p][i][1]);
-          const float2 v = e ? make_float2(re.y, im.y) : make_float2(re.x, im.x);
-          if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0) bad |= 1u << (8 * p + 2 * i + e);
-          const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
-          word[p] = *reinterpret_cast<const unsigned*>(&h);
+          for (int p = 0; p < 4; ++p) {
+            const float2 re = unpack2(acc[p][i][0]), im = unpack2(acc[p][i][1]);
+            const float2 v = e ? make_float2(re.y, im.y) : make_float2(re.x, im.x);
+            if (!(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY) && pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0) bad |= 1u << (8 * p + 2 * i + e);
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
+            word[p] = *reinterpret_cast<const unsigned*>(&h);
+          }
+          __nv_bfloat16* out = apply_output(a, tile, n, g, col);
+          if (whole) {
+            *reinterpret_cast<uint4*>(out) = make_uint4(word[0], word[1], word[2], word[3]);
+          } else {
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+              if (pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(out + 2 * p) = word[p];
+          }
         }
-        __nv_bfloat16* out = apply_output(a, tile, n, g, col);
-        if (whole) {
-          *reinterpret_cast<uint4*>(out) = make_uint4(word[0], word[1], word[2], word[3]);
-        } else {
-#pragma unroll
-          for (int p = 0; p < 4; ++p)
-            if (pairs_s[cb * AP_PAIRS + 4 * cg + p].kind >= 0) *reinterpret_cast<unsigned*>(out + 2 * p) = word[p];
-        }
-      }
-  }
-  bad_s[cb][threadIdx.x] = bad;
+    }
+    bad_s[cb][threadIdx.x] = bad;
   }
   tile.col0 = cb0 * AP_COLS;
   for (int cb = 0; cb < n_cb; ++cb, tile.col0 += AP_COLS) {

@@ -203,8 +203,9 @@ def test_factored_against_plain_sums(type_in, type_out, k, degrees, dtype):
     ({0: 2, 1: 2, 2: 2}, {0: 25, 1: 25, 2: 25}, 11, [90, 33]),             # 91 tiles: three rounds of 32 backward
 ])
 def test_factored_tensor_cores_against_float64(type_in, type_out, k, degrees, scales):
-    """Rows, weighted sums' gradients and all others of the float32 kernels that sources of many edges take, against the float64
-    kernels (which the tests above pin) on the same numbers: sums of at most 300 edges x 19 trunk outputs or 575 columns of O(1)
+    """Rows, weighted sums' gradients and all others of the float32 kernels, against the float64 kernels (which the tests above pin)
+    on the same numbers (rows by the tensor cores from k 10 on, the last graph's gradients too; ``both_factored_kernels`` below has
+    edges enough for the others'): sums of at most 300 edges x 19 trunk outputs or 575 columns of O(1)
     terms whose rounding errors of 2^-24 add up like their square root, 2e-6 of each tensor's norm."""
     from gm_attention_b200.fields import FieldType
     from gm_attention_b200.nn import fused_factored as ff
