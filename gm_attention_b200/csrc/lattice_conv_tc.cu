@@ -664,17 +664,18 @@ static ApplyGrid apply_grid(const ConvArgs& a) {
 }
 
 // The FMA kernels stay the faster ones where the tiles are mostly padding and there are enough of them to fill the chip.  333
-// shapes from 24 x 24 to 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores (apply), 576 (table_grad):
+// shapes from 24 x 24 to 256 x 512, batch 1 to 4, widths 24 to 320, us FMA / tensor cores:
 //   apply        a CTA takes up to 64 tiles of 8 longitudes.  From 32 on it is the faster one (128 x 128, width 320, batch 2: 179 / 179, batch
 //                4: 333 / 237; 256 x 512, width 320: 1 336 / 540), with fewer while the launch has few CTAs and lasts as long as the polar
 //                rows' chains of stages, which are shorter here (64 x 128, batch 1, width 160: 81 / 42, width 320: 78 / 70; 128 x 128, batch
 //                1, width 160: 116 / 81, but width 320: 112 / 154).  With up to 8 tiles a row the FMA kernel's chains are short too (32 x 64:
 //                50 / 25, width 320: 48 / 47; 200 x 48, width 24: 24 / 22, width 40: 24 / 28, width 320: 28 / 116).
 //   table_grad   contracts over the tiles of all samples, 16 a step; the FMA kernel takes samples by two.  The least tiles by samples and
-//                width are the least at which neither radius 2 nor 4 rows lost (576 timings, 9 to 32 tiles; but 40 columns, one sample, 4 rows: 1.13 at 19): one sample, width 160, radius 2, 22 tiles 38 /
-//                42, 24 0.77 of the time; width 320 24 tiles 73 / 81, 28 0.92; two, width 320, 22 tiles 94 / 103, 24 0.98; width 160 19 tiles 52 / 50;
-//                width 96 11 tiles 1.12, 13 0.89; three, width 320, 11 tiles 61 / 51, 19 133 / 112, radius 4 358 / 231.  One block of 32 columns always
-//                (9 tiles 0.50), 8 tiles with four samples (32 x 64: 32 / 22).  256 x 512: 1 701 / 738.
+//                width are where radius 2, 2.5, 3 and 4 rows come out even (736 timings, 9 to 32 tiles; the share of the FMA time for each radius): one
+//                sample, width 320, 22 tiles 1.18, 0.99, 1.08, 0.98, 24 1.11, 0.89, 0.95, 0.90; width 160, 18 tiles 1.29, 1.22, 0.92, 0.95, 20 1.14, 0.86, 0.91,
+//                0.87; two, width 320, 20 tiles 1.14, 1.00, 1.06, 0.96, 22 1.09, 0.95, 0.96, 0.87; width 160, 13 tiles 0.97, 1.01, 1.02, 0.88, 16 0.99, 0.82,
+//                0.81, 0.79; width 96, 11 tiles 1.12, 1.01, 1.27, 1.02, 13 0.89, 0.94, 0.89, 0.81; three, width 96, 9 tiles 0.77, width 320, 11 tiles 0.82 and (radius 4)
+//                0.74.  One block of 32 columns always (9 tiles 0.50), 8 tiles with three samples or four (35 x 64: 23 / 15 us, 32 x 64: 32 / 22).  256 x 512: 1 701 / 738 us.
 bool tensor_cores_apply(const ConvArgs& a) {
   if (!tensor_cores_can(a) || !tensor_cores_hold(a)) return false;
   const int T = a.nlon / 8;
@@ -685,8 +686,8 @@ bool tensor_cores_apply(const ConvArgs& a) {
 bool tensor_cores_table_grad(const ConvArgs& a) {
   const bool narrow = a.width <= TG_COLS;
   const int by_width = a.width <= 96 ? 0 : a.width <= 160 ? 1 : 2;
-  constexpr int ONE[] = {16, 24, 28}, TWO[] = {13, 19, 24};
-  const int least = narrow ? (a.batch >= 4 ? 8 : 9) : a.batch >= 4 ? 9 : a.batch == 3 ? 11 : a.batch == 2 ? TWO[by_width] : ONE[by_width];
+  constexpr int LEAST[4][3] = {{20, 20, 24}, {13, 16, 22}, {9, 11, 11}, {9, 9, 9}};  // samples, width
+  const int least = narrow ? (a.batch >= 3 ? 8 : 9) : LEAST[std::min(a.batch, 4) - 1][by_width];
   return tensor_cores_can(a) && a.nlon / 8 >= least;
 }
 
