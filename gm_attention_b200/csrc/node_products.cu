@@ -431,7 +431,7 @@ extern "C" int gm_node_products_backward(const void* x, const void* cw, const vo
     st = allow_smem(node_products_dw_kernel<T>, smem, "gm_node_products_backward");
     if (st != GM_OK) return st;
     // CTAs in z share an entry's copies, of which a row's width tells the most there can be
-    const dim3 grid((unsigned)((n_nodes + chunk - 1) / chunk), entry_tiles(k, wc, wr), (unsigned)std::clamp(din / (2 * A_SUMMED), 1, 4));
+    const dim3 grid((unsigned)((n_nodes + chunk - 1) / chunk), entry_tiles(k, wc, wr), (unsigned)std::clamp((din + A_SUMMED - 1) / A_SUMMED, 1, 4));
     node_products_dw_kernel<T><<<grid, ENTRY_THREADS, smem, (cudaStream_t)stream>>>(p);
     return launch_status("gm_node_products_backward");
   };
