@@ -297,6 +297,22 @@ def test_one_or_two_warps_per_target(ext, heads, head, dtype):
         assert float((a - b[:c.n_nodes]).abs().max()) <= (1e-5 if dtype == np.float32 else 1e-13) * float(a.abs().max())
 
 
+@pytest.mark.parametrize("heads, head", [(1, {0: 5, 1: 3}), (2, {0: 4, 1: 4, 2: 4}), (4, {0: 4, 1: 2, 2: 3, 3: 4}), (8, {0: 2, 1: 2})])
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+def test_lane_groups_give_the_same_bits(ext, heads, head, dtype):
+    """Groups of lanes that share a target's edges come with seven edges per target and more: the same edges as those of
+    targets enough for none give the same scores bit for bit, as a chunk of few edges per target must."""
+    c = make_case(12, 24, 3 * math.pi / 12, head, heads, dtype=dtype)
+    q, k = (cuda(x) for x in seeded((c.n_nodes, c.width), 29, dtype, 2))
+    tables = [cuda(x) for x in (c.transport, c.bias, c.inside, c.desc, c.row_ptr, c.source)]
+    n_edges = c.source.shape[0]
+    assert n_edges >= 7 * c.n_nodes
+    more = torch.cat([tables[4], tables[4][-1:].expand(n_edges)])
+    wide = [torch.cat([x, torch.zeros(n_edges, c.width, dtype=x.dtype, device="cuda")]) for x in (q, k)]
+    shared = ext.softmax_forward(q, k, *tables, heads, c.scale, c.max_degree)
+    assert torch.equal(ext.softmax_forward(*wide, *tables[:4], more, tables[5], heads, c.scale, c.max_degree), shared)
+
+
 def test_chunked_scores_equal_the_whole_edge_set(ext):
     """Exact chunking over contiguous target ranges (reference ``nn/attention.py:344-402``): every chunk holds whole
     neighbourhoods, its constants are views of the parent's, and the softmax stays a partition of unity inside it --
