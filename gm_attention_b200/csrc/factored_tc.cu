@@ -13,7 +13,7 @@
 // reach 2^-24 of the result are taken, in two chains of three, smallest first; everything that is summed over more than one
 // k-step (the 16 edges of dZ, the two tiles of dh) is added in float32, rounded to nearest.
 // What it measured, 128 x 256, radius 3 pi / 128 (3.0 M edges), 13 blocks to {4, 4, 4}, trunk 16, us on CUDA cores -> here: forward 1 036 -> 731,
-// backward 2 463 -> 1 830.  Bound by latency and issue (issue 41 / 46 %, tensor pipe 17 / 14 %): a step of 16 edges is 78 / 168 products
+// backward 2 463 -> 1 830.  Bound by latency and issue (issue 44 / 46 %, tensor pipe 17 / 14 %): a step of 16 edges is 78 / 168 products
 // among 1 600 / 4 400 instructions, most of them the splits, the factors and the records' copies.  With the records read where
 // they are (1 245 / 3 225 us) every step waited for its chain of gathers; they are copied a step ahead.  Four tiles a backward warp:
 // eight 2 095 us (the loop over tiles, unrolled for its accumulators, outgrew the instruction cache), two 1 946.  168 registers

@@ -80,6 +80,7 @@ int gm_softmax_backward(const void* dalpha, const void* q, const void* k, const 
  *   out        (n_nodes, D)    out
  *   dv         (n_nodes, D)    out, ACCUMULATED (zero it first)
  *   drc, dcc   shaped as rc, cc; every entry written
+ *   desc       rows as above; one of frequency 0 comes first
  * dtype: GM_F32 or GM_F64.
  * ------------------------------------------------------------------------ */
 int gm_conv_forward(const void* v, const void* rc, const void* cc, const void* transport, const void* angular,
@@ -111,6 +112,8 @@ int gm_conv_backward(const void* g, const void* v, const void* rc, const void* c
  *   desc_host   (F, 5) int64 in HOST memory (rows as above)
  *   transport   (n_edges, orders, 2), bias (n_edges): fp32 for GM_F32 / GM_BF16, fp64 for GM_F64
  *   lse         (batch * n_nodes, H)   fp32 (fp64 for GM_F64): log-sum-exp of each row's logits
+ *               (a row without edges in its window, or whose logits are all minus infinity: out 0, lse minus infinity,
+ *               no gradients)
  *   H must be 1, 2, 4 or 8.
  * Backward: dq, dk, dv are fully written (zero-initialised inside).  With
  * GM_BF16 the source-side sums accumulate in fp32 in `scratch`
