@@ -392,6 +392,7 @@ __global__ void __launch_bounds__(32 * FWD_WARPS, 10) factored_forward_tc_kernel
         }
         unsigned h[3][4];
         const bool large = __any_sync(0xffffffffu, too_large(load_trunk(rows + g * rec.pitch, rows + (g + 8) * rec.pitch, a.k - 1, c, h)) || large_node);
+        __syncwarp();  // the factors are there (a vote orders no memory)
         const bool in0 = g < n_rows, in1 = g + 8 < n_rows;
         float *out0 = a.out + (size_t)e0 * a.d_out, *out1 = a.out + (size_t)e1 * a.d_out;
         if (large) {
