@@ -326,7 +326,18 @@ __global__ void __launch_bounds__(256, backward_ctas<S, NS, FORM, SHARED>()) fus
   }
   for (int o = at.L >> 1; o > 0; o >>= 1) delta += __shfl_xor_sync(0xffffffffu, delta, o);
   C lse = a.lse_in[(base + i) * a.H + at.h];
-  if (lse == neg_inf<C>()) lse = -lse;  // no edge counted: p = 0 for all of them
+  // No edge counted: p = 0 for all of them.  (Where the logits were not numbers the forward gives minus infinity as well, but NaN
+  // with it, which the gradients of the target's neighbours are to show.)
+  if (lse == neg_inf<C>()) {  // (a head's lanes come here together)
+    bool number = true;
+#pragma unroll
+    for (int t = 0; t < NS; ++t)
+      if (col[t] >= 0) {
+        const C re = ld<C>(o_i + col[t]), im = a.plan.order[t] == 0 ? C(0) : ld<C>(o_i + col[t] + 1);
+        number = number && re == re && im == im;
+      }
+    if (__all_sync((at.L == 32 ? 0xffffffffu : (1u << at.L) - 1u) << (lane / at.L * at.L), number)) lse = -lse;
+  }
   const int64_t e0 = a.row_ptr[i];
   const int degree = (int)(a.row_ptr[i + 1] - e0);
   const int64_t* source = a.source + e0;

@@ -216,3 +216,37 @@ def test_targets_whose_edges_all_count_nothing(graph, dtype):
     assert_close(out.cpu().numpy(), want, rtol, atol * max(1.0, np.abs(want).max()), "out")
     for name, got, ref in zip(("dq", "dk", "dv"), (dq, dk, dv), grads):
         assert_close(got.cpu().numpy(), ref, rtol, 10 * atol * max(1.0, np.abs(ref).max()), name)
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("graph", GRAPHS)
+def test_what_is_not_a_number_reaches_the_neighbours_gradients(graph, dtype):
+    """A NaN in a target's q and an infinity in a source's k make their targets' outputs NaN, in their head; the gradients are not
+    finite where the oracle's are not: of those targets, and of all that they see."""
+    from gm_attention_b200.attention import AttentionTables, attention_backward, attention_forward
+
+    heads, rows, width, degree = graph
+    n_nodes, batch = 211, 2
+    rng = np.random.default_rng(8)
+    counts = rng.integers(1, 6, n_nodes)
+    counts[7], counts[60] = 2 * degree, degree
+    row_ptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+    n_edges, orders = int(row_ptr[-1]), 1 + max(n for n, _, _ in rows)
+    desc = np.array([(n, copies, offset, 0, 1 if n == 0 else 2) for n, copies, offset in rows], dtype=np.int64)
+    source = rng.integers(0, n_nodes, n_edges)
+    angle = rng.uniform(-np.pi, np.pi, (n_edges, 1)) * np.arange(orders)
+    transport = np.stack([np.cos(angle), np.sin(angle)], -1).astype(dtype)
+    bias, inside = rng.standard_normal(n_edges).astype(dtype), np.ones(n_edges, np.uint8)
+    q, k, v, g = seeded((batch * n_nodes, width), 19, dtype, 4)
+    q[7, rows[0][2]] = np.nan
+    k[n_nodes + source[row_ptr[60]], rows[-1][2]] = np.inf
+    args = (transport, bias, inside, desc, row_ptr, source, heads, 0.3, batch)
+    want = O.attention_forward(q, k, v, *args)
+    grads = O.attention_backward(g, q, k, v, *args)
+    t = AttentionTables(cuda(transport), cuda(bias), cuda(inside), cuda(row_ptr), cuda(source), tuple(map(tuple, desc.tolist())), heads, 0.3)
+    Q, K, V, G = map(cuda, (q, k, v, g))
+    out, lse = attention_forward(Q, K, V, t)
+    seen = np.arange(n_edges)[row_ptr[7]:row_ptr[8]]
+    assert not np.isfinite(grads[2][source[seen]]).all(1).any()
+    for name, got, ref in zip(("out", "dq", "dk", "dv"), (out, *attention_backward(G, Q, K, V, out, lse, t)), (want, *grads)):
+        assert np.array_equal(np.isfinite(got.cpu().numpy()), np.isfinite(ref)), name
